@@ -15,6 +15,11 @@ from .decode import Rwkv7DecodeState
 from .varlen import PackedSequences, generalized_delta_rule_varlen, wkv6_varlen
 from .fused import generalized_delta_rule_fused
 
+from . import _ops
+
+if _ops.built():      # register the operators now, so that tracing finds them; an unbuilt package raises at the first call
+    _ops.load()
+
 __version__ = "0.1"
 
 RWKV7_USE_KERNEL = True

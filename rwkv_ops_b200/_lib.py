@@ -84,7 +84,7 @@ def load() -> ctypes.CDLL:
             f"{LIB_PATH} not found. Build it with `python -m rwkv_ops_b200.build` (needs nvcc); "
             "rwkv_ops_b200 has no CPU or eager fallback."
         )
-    lib = ctypes.CDLL(LIB_PATH)
+    lib = ctypes.CDLL(LIB_PATH, mode=ctypes.RTLD_GLOBAL)      # the torch operators' library resolves against it
     for name, (res, args) in SIGNATURES.items():
         fn = getattr(lib, name)  # AttributeError if the library does not export a declared symbol
         fn.restype = res

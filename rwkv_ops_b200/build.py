@@ -6,7 +6,9 @@ The library is a plain C-ABI shared object (no torch, no pybind): one nvcc
 invocation per ``csrc/*.cu`` into ``csrc/_build/*.o`` and a link step.  A source is
 recompiled only when it or a header is newer than its object.
 
-A second library, ``librwkv_ops_b200_dev.so``, is the same sources with ``-DRWKVB200_DEVTOOLS``: it adds the
+The torch operators (``csrc/torch_ops.cpp``, plain C++) go into ``librwkv_ops_b200_torch.so`` beside it.
+
+Another library, ``librwkv_ops_b200_dev.so``, is the same sources with ``-DRWKVB200_DEVTOOLS``: it adds the
 building-block self-test and the phase-stamp instrumentation that the unit tests of the tensor-core
 primitives use (``include/rwkv_ops_b200_devtools.h``).  The product never loads it.
 """
@@ -25,6 +27,7 @@ CSRC = os.path.join(PKG, "csrc")
 BUILD = os.path.join(CSRC, "_build")
 LIB = os.path.join(PKG, "librwkv_ops_b200.so")
 DEV_LIB = os.path.join(PKG, "librwkv_ops_b200_dev.so")
+TORCH_LIB = os.path.join(PKG, "librwkv_ops_b200_torch.so")
 INCLUDE = os.path.join(os.path.dirname(PKG), "include")
 
 NVCC_FLAGS = [
@@ -49,7 +52,7 @@ def _newest_header() -> float:
 
 
 def build(force: bool = False, verbose: bool = False, dev: bool = False) -> str:
-    """Build the product library, or with ``dev`` the developer build."""
+    """Build the product library and the torch operators, or with ``dev`` the developer build."""
     build_dir = os.path.join(BUILD, "dev") if dev else BUILD
     lib = DEV_LIB if dev else LIB
     flags = NVCC_FLAGS + (["-DRWKVB200_DEVTOOLS"] if dev else [])
@@ -81,11 +84,35 @@ def build(force: bool = False, verbose: bool = False, dev: bool = False) -> str:
     with ThreadPoolExecutor(max_workers=min(8, max(1, len(jobs)))) as ex:
         list(ex.map(compile_one, jobs))
     if jobs or force or not os.path.exists(lib):
-        cmd = [nvcc, "-shared", "-o", lib, *objs, "-lcudart"]
+        # -Bsymbolic: the product library is loaded with global symbols (the torch operators resolve against it), and
+        # the developer build beside it in the same process must keep calling its own functions
+        cmd = [nvcc, "-shared", "-Xlinker", "-Bsymbolic", "-o", lib, *objs, "-lcudart"]
         p = subprocess.run(cmd, capture_output=True, text=True)
         if p.returncode != 0:
             raise RuntimeError("link failed:\n" + p.stdout + p.stderr)
+    if not dev:
+        build_torch(force)
     return lib
+
+
+def build_torch(force: bool = False) -> str:
+    """Build the torch operators (``csrc/torch_ops.cpp``): host code only, linked against torch."""
+    import torch
+
+    src = os.path.join(CSRC, "torch_ops.cpp")
+    newest = max(os.path.getmtime(src), *(os.path.getmtime(h) for h in glob.glob(os.path.join(INCLUDE, "*.h"))))
+    if not force and os.path.exists(TORCH_LIB) and os.path.getmtime(TORCH_LIB) >= newest:
+        return TORCH_LIB
+    cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))), "include")
+    root = os.path.dirname(torch.__file__)
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wno-attributes",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           *(f"-I{os.path.join(root, p)}" for p in ("include", "include/torch/csrc/api/include")), f"-I{cuda}", src, "-o", TORCH_LIB,
+           f"-L{os.path.join(root, 'lib')}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch"]
+    p = subprocess.run(cmd, capture_output=True, text=True)
+    if p.returncode != 0:
+        raise RuntimeError("g++ failed on torch_ops.cpp:\n" + p.stdout + p.stderr)
+    return TORCH_LIB
 
 
 if __name__ == "__main__":

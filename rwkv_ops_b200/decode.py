@@ -13,30 +13,9 @@ from typing import Optional
 
 import torch
 
-from . import _lib
+from . import _lib, _ops
 
 HEAD_SIZE = 64
-
-
-@torch.library.custom_op("rwkv_ops_b200::rwkv7_decode_step", mutates_args=("state",))
-def _decode_step(r: torch.Tensor, w: torch.Tensor, k: torch.Tensor, v: torch.Tensor, a: torch.Tensor,
-                 b: torch.Tensor, state: torch.Tensor) -> torch.Tensor:
-    lib = _lib.load()
-    dev = _lib.require_cuda(r, w, k, v, a, b, state)
-    B, H = state.shape[0], state.shape[1]
-    o = torch.empty_like(r)
-    with torch.cuda.device(dev):
-        rc = lib.rwkvb200_rwkv7_decode_step(r.data_ptr(), w.data_ptr(), k.data_ptr(), v.data_ptr(), a.data_ptr(),
-                                            b.data_ptr(), state.data_ptr(), _lib.dtype_code(state.dtype),
-                                            o.data_ptr(), B, H, HEAD_SIZE, _lib.dtype_code(r.dtype),
-                                            _lib.stream_ptr(dev))
-        _lib.check(rc, "rwkv7_decode_step")
-    return o
-
-
-@_decode_step.register_fake
-def _(r, w, k, v, a, b, state):
-    return torch.empty_like(r)
 
 
 class Rwkv7DecodeState:
@@ -63,20 +42,23 @@ class Rwkv7DecodeState:
         if not self.state.is_cuda:
             raise _lib.RwkvB200Error("Rwkv7DecodeState lives on a CUDA device; there is no CPU fallback.")
 
-    @torch.no_grad()
-    def step(self, r, w, k, v, a, b):
-        shape = r.shape
+    def _check_args(self, r, w, k, v, a, b):
+        """Raise what the interface documents for invalid arguments (the operator itself only says that they are)."""
+        shape = tuple(r.shape)
         B, H = self.state.shape[0], self.state.shape[1]
-        if tuple(shape) not in ((B, 1, H, HEAD_SIZE), (B, H, HEAD_SIZE)):
-            raise ValueError(f"expected token tensors [{B}, 1, {H}, 64] or [{B}, {H}, 64], got {tuple(shape)}")
-        dt = r.dtype if r.dtype in (torch.float32, torch.bfloat16, torch.float16) else torch.float32
-        args = []
-        for name, x in (("r", r), ("w", w), ("k", k), ("v", v), ("a", a), ("b", b)):
-            if x.shape != shape:
-                raise ValueError(f"{name} has shape {tuple(x.shape)}, expected {tuple(shape)}")
-            args.append(x.to(dt).contiguous().view(B, H, HEAD_SIZE))
-        o = _decode_step(*args, self.state)
-        return o.view(shape).to(r.dtype)
+        if shape not in ((B, 1, H, HEAD_SIZE), (B, H, HEAD_SIZE)):
+            raise ValueError(f"expected token tensors [{B}, 1, {H}, 64] or [{B}, {H}, 64], got {shape}")
+        for name, x in (("w", w), ("k", k), ("v", v), ("a", a), ("b", b)):
+            if x.shape != r.shape:
+                raise ValueError(f"{name} has shape {tuple(x.shape)}, expected {shape}")
+        _lib.require_cuda(r, w, k, v, a, b, self.state)
+
+    def step(self, r, w, k, v, a, b):
+        try:
+            return _ops.load().rwkv7_decode_step(r, w, k, v, a, b, self.state)
+        except Exception as e:
+            self._check_args(r, w, k, v, a, b)
+            raise _ops.failed(e)
 
     def final_state(self) -> torch.Tensor:
         """The state as the operator would return it (float32 copy)."""
