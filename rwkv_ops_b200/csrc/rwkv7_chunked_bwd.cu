@@ -15,17 +15,6 @@ using namespace tc;
 typedef __nv_bfloat16 bf16;
 
 // decay sums are kept in units of log 2 (tc::ex2), as in the forward kernels; nothing is clamped
-constexpr int NROW = 68;
-
-__device__ __forceinline__ void store_row32_global(bf16* dst, const float* x) {
-#pragma unroll
-  for (int j = 0; j < 32; j += 8) {
-    uint4 u;
-    u.x = pack_bf16(x[j], x[j + 1]); u.y = pack_bf16(x[j + 2], x[j + 3]);
-    u.z = pack_bf16(x[j + 4], x[j + 5]); u.w = pack_bf16(x[j + 6], x[j + 7]);
-    *reinterpret_cast<uint4*>(dst + j) = u;
-  }
-}
 
 // ---------------------------------------------------------------------------------------------
 // 3. B2 = Ainv^T b~ and P2 = Ainv^T (A_qb^T do): persistent CTAs of 128 threads over the chunk-heads
@@ -329,35 +318,37 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
 // ---------------------------------------------------------------------------------------------
 // 5. all token gradients of one chunk: persistent CTAs of 256 threads over the B*H*NT chunk-heads
 // ---------------------------------------------------------------------------------------------
+// What bounds it: per chunk-head about 14 k warp instructions in phases that wait for one another (tiles ->
+// products -> read-out -> products -> read-out -> prefix sums).  With one CTA per SM (213 KB of shared memory) the
+// SM issued 1.0 instruction per cycle; two CTAs per SM fill each other's waits.  To fit two, a chunk-head lives in
+// twelve tiles whose space is used over again (names below: what is loaded, then what replaces it) and one fp32
+// array, and an accumulator that does not need the dA tiles is issued with the first MMA group, which frees its
+// operands.  TMEM: dA columns 0..127, [dq~; da~] 128..191, dv 192..255 (lower lane halves); [dk~; db~] 0..63 once
+// dA has been read.
 struct FinalSmem {
-  // loaded per chunk, group A (free again once MMA group 2 has completed)
-  unsigned char dout[TILE_BYTES], dz[TILE_BYTES];                 // [do; dz]
-  unsigned char v[TILE_BYTES], sa[TILE_BYTES];                    // [v; sa]
-  unsigned char aqk[TILE_BYTES], aak[TILE_BYTES];                 // adjacent workspace slots; aqk later stages dv
-  unsigned char h0[TILE_BYTES], dhh[TILE_BYTES];
-  // loaded per chunk, group B (read by the last epilogue, free after it)
-  unsigned char qt[TILE_BYTES], at[TILE_BYTES], kt[TILE_BYTES], bt[TILE_BYTES];
-  // computed
-  unsigned char daqk[TILE_BYTES], daak[TILE_BYTES], daqb[TILE_BYTES], daab[TILE_BYTES];
-  unsigned char red_pad[2048];    // the two fp32 scratch arrays that later overlay the dA tiles need 34 KB
-  unsigned char dge[TILE_BYTES];  // da~ a~ as bf16
-  unsigned char stage[5][TILE_BYTES];   // dq, dk, da, db, dw rows staged for TMA stores
-  float gs[L * NROW];       // (gi - gref) log2(e): inclusive prefix of g inside the chunk, relative to the reference point
-  float gg[L * NROW];       // g log2(e)
-  float qtot[4][64];        // sums of g over the four quarters of the chunk
-  float rqtot[4][64];       // sums of the decay-gradient terms over the four quarters
-  float dgl[64];            // dglast
-  uint64_t bar_lda, bar_ldb, bar_m1, bar_m2;
+  unsigned char dout[TILE_BYTES], dz[TILE_BYTES];       // [do; dz]   then dA_qk, dA_ak   then red1 (fp32)
+  unsigned char aqk[TILE_BYTES], aak[TILE_BYTES];       // A_qk, A_ak then dA_qb, dA_ab   then red2 (fp32)
+  unsigned char h0[TILE_BYTES];                         // h~0        then dv rows        then dw rows
+  unsigned char dhh[TILE_BYTES];                        // dh^
+  unsigned char v[TILE_BYTES], sa[TILE_BYTES];          // [v; sa]    (sa) then da~ a~ as bf16
+  unsigned char qt[TILE_BYTES], at[TILE_BYTES];         // q~, a~     then dq, da rows
+  unsigned char kt[TILE_BYTES], bt[TILE_BYTES];         // k~, b~     then dk, db rows
+  float gs[L * 64];         // g log2(e), then (gi - gref) log2(e): inclusive prefix inside the chunk (sw64)
+  float quart[3][64];       // sums over quarters of the chunk; [2] between the prefix sum and the epilogue: -gref
+  uint64_t bar_l0, bar_l1, bar_l2, bar_m1, bar_m2;
   uint32_t tmem_base;
 };
+// two CTAs per SM: 228 KB shared by both, 1 KB of each reserved by the system
+static_assert(sizeof(FinalSmem) <= 115712, "two CTAs per SM");
 
-// Persistent: one CTA per SM walks over chunk-heads ch = blockIdx.x, blockIdx.x + gridDim.x, ...; the
-// tiles of the next chunk-head are requested as soon as the current one no longer needs them, and its w
-// rows wait in registers, so only the first chunk-head of a CTA pays the load latency.
+// index of (row, channel) in a 64 x 64 fp32 array whose 16-byte pieces are permuted by the row, so that threads that
+// own a row and threads that own a channel both access it without bank conflicts
+__device__ __forceinline__ int sw64(int row, int c) { return row * 64 + ((((c >> 2) ^ (row & 7)) << 2) | (c & 3)); }
+
 // 256 threads: warp w reads TMEM lanes 32*(w&3).. (its row), and the two warps that share a lane
 // window split the columns (hsel = w>>2), so every elementwise phase is spread over 8 warps.
 template <bool PACKED, bool FUSED>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtensorMap tmap_do,
                      const __grid_constant__ CUtensorMap tmap_v, const unsigned char* __restrict__ ws_tiles,
                      int tiles_per_chunk, const __grid_constant__ CUtensorMap tmap_dq,
@@ -368,19 +359,24 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
                      bf16* __restrict__ dv_rows, bf16* __restrict__ da_rows, bf16* __restrict__ db_rows,
                      SeqView sv, int H, int NT, int n_ch, TokLayout lay, int* status, long long* dbg) {
 #ifdef RWKVB200_DEVTOOLS
-#define R7C_STAMP(n) do { if (dbg && tid == 0 && blockIdx.x == gridDim.x / 2 && it == 30) dbg[n] = clock64(); } while (0)
+#define R7C_STAMP(n) do { if (dbg && tid == 0 && blockIdx.x == gridDim.x / 2 && it == 15) dbg[n] = clock64(); } while (0)
 #else
 #define R7C_STAMP(n) do {} while (0)
 #endif
-  extern __shared__ unsigned char smem_raw[];
-  FinalSmem& sm = *reinterpret_cast<FinalSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  FinalSmem& sm = *reinterpret_cast<FinalSmem*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int wq = warp & 3, hsel = warp >> 2;
+  if (smem_u32(smem_raw) & 1023u) {      // the swizzled tiles need this alignment; there is no room to align by hand
+    if (tid == 0) atomicCAS(status, 0, 320);
+    return;
+  }
 
   if (tid == 0) {
-    // each MMA group is issued by two threads (threads 0 and 32), one accumulator each, and completes with
-    // the arrival of both: one thread issues an MMA about every 80 cycles, the tensor pipe takes them faster
-    mbar_init(&sm.bar_lda, 1); mbar_init(&sm.bar_ldb, 1); mbar_init(&sm.bar_m1, 2); mbar_init(&sm.bar_m2, 2);
+    // an MMA group is issued by several threads, one accumulator each, and completes with the arrival of all: one
+    // thread issues an MMA about every 80 cycles, the tensor pipe takes them faster
+    mbar_init(&sm.bar_l0, 1); mbar_init(&sm.bar_l1, 1); mbar_init(&sm.bar_l2, 1);
+    mbar_init(&sm.bar_m1, 3); mbar_init(&sm.bar_m2, 2);
     fence_mbar_init();
   }
   if (warp == 0) tmem_alloc(&sm.tmem_base, 256);
@@ -388,53 +384,52 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
   __syncthreads();
   tc_fence_after();
   const uint32_t tm = sm.tmem_base;
+  const bool st_thread = tid == 96;      // requests the tiles, stores the results
 
-  auto coords = [&](const ChunkPos& p, int& bi, int& hi, int& t0) { bi = p.bi; hi = p.hi; t0 = p.c * L; };
-  auto load_group_a = [&](const ChunkPos& p) {     // tid 0
-    int bi, hi, t0; coords(p, bi, hi, t0);
+  // the tiles of a chunk-head in the order in which their space becomes free
+  auto load_0 = [&](const ChunkPos& p) {      // dh^, v
     const unsigned char* tiles = ws_tiles + (size_t)p.ch * tiles_per_chunk * TILE_BYTES;
-    mbar_expect_tx(&sm.bar_lda, 8 * TILE_BYTES);
-    tma_load_4d(sm.dout, &tmap_do, &sm.bar_lda, 0, sv.first<PACKED>(bi) + t0, hi, sv.row<PACKED>(bi));
-    tma_load_4d(sm.v, &tmap_v, &sm.bar_lda, 0, sv.first<PACKED>(bi) + t0, hi, sv.row<PACKED>(bi));
-    bulk_load(sm.dz, tiles + S_DZ * TILE_BYTES, TILE_BYTES, &sm.bar_lda);
-    bulk_load(sm.sa, tiles + S_SA * TILE_BYTES, TILE_BYTES, &sm.bar_lda);
-    bulk_load(sm.aqk, tiles + S_AQK * TILE_BYTES, 2 * TILE_BYTES, &sm.bar_lda);
-    bulk_load(sm.h0, tiles + S_H0 * TILE_BYTES, TILE_BYTES, &sm.bar_lda);
-    bulk_load(sm.dhh, tiles + S_DHH * TILE_BYTES, TILE_BYTES, &sm.bar_lda);
+    mbar_expect_tx(&sm.bar_l0, 2 * TILE_BYTES);
+    bulk_load(sm.dhh, tiles + S_DHH * TILE_BYTES, TILE_BYTES, &sm.bar_l0);
+    tma_load_4d(sm.v, &tmap_v, &sm.bar_l0, 0, sv.first<PACKED>(p.bi) + p.c * L, p.hi, sv.row<PACKED>(p.bi));
   };
-  auto load_group_b = [&](const ChunkPos& p) {     // tid 0
+  auto load_1a = [&](const ChunkPos& p) {     // the other operands of MMA group 1, but for k~ and h~0
     const unsigned char* tiles = ws_tiles + (size_t)p.ch * tiles_per_chunk * TILE_BYTES;
-    mbar_expect_tx(&sm.bar_ldb, 4 * TILE_BYTES);
-    bulk_load(sm.qt, tiles + S_QT * TILE_BYTES, TILE_BYTES, &sm.bar_ldb);
-    bulk_load(sm.at, tiles + S_AT * TILE_BYTES, TILE_BYTES, &sm.bar_ldb);
-    bulk_load(sm.kt, tiles + S_KT * TILE_BYTES, TILE_BYTES, &sm.bar_ldb);
-    bulk_load(sm.bt, tiles + S_BT * TILE_BYTES, TILE_BYTES, &sm.bar_ldb);
+    mbar_expect_tx(&sm.bar_l1, 7 * TILE_BYTES);
+    tma_load_4d(sm.dout, &tmap_do, &sm.bar_l1, 0, sv.first<PACKED>(p.bi) + p.c * L, p.hi, sv.row<PACKED>(p.bi));
+    bulk_load(sm.dz, tiles + S_DZ * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
+    bulk_load(sm.sa, tiles + S_SA * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
+    bulk_load(sm.aqk, tiles + S_AQK * TILE_BYTES, 2 * TILE_BYTES, &sm.bar_l1);
   };
-  // Ask for everything a chunk-head will load to be brought into L2 (issued one chunk-head ahead of the
+  auto load_2 = [&](const ChunkPos& p) {      // k~; q~, a~, b~ (MMA group 2 and the epilogue)
+    const unsigned char* tiles = ws_tiles + (size_t)p.ch * tiles_per_chunk * TILE_BYTES;
+    bulk_load(sm.kt, tiles + S_KT * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
+    mbar_expect_tx(&sm.bar_l2, 3 * TILE_BYTES);
+    bulk_load(sm.qt, tiles + S_QT * TILE_BYTES, TILE_BYTES, &sm.bar_l2);
+    bulk_load(sm.at, tiles + S_AT * TILE_BYTES, TILE_BYTES, &sm.bar_l2);
+    bulk_load(sm.bt, tiles + S_BT * TILE_BYTES, TILE_BYTES, &sm.bar_l2);
+  };
+  auto load_1b = [&](const ChunkPos& p) {     // h~0
+    const unsigned char* tiles = ws_tiles + (size_t)p.ch * tiles_per_chunk * TILE_BYTES;
+    bulk_load(sm.h0, tiles + S_H0 * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
+  };
+  // Ask for everything a chunk-head will load to be brought into L2 (issued most of a chunk-head ahead of the
   // loads themselves, which then take an L2 round trip instead of a DRAM one).
   auto prefetch_l2 = [&](const ChunkPos& p) {      // one warp
-    int bi, hi, t0; coords(p, bi, hi, t0);
+    const int t0 = p.c * L;
     const unsigned char* tiles = ws_tiles + (size_t)p.ch * tiles_per_chunk * TILE_BYTES;
     if (lane == 0) {
-      tma_prefetch_4d(&tmap_do, 0, sv.first<PACKED>(bi) + t0, hi, sv.row<PACKED>(bi));
-      tma_prefetch_4d(&tmap_v, 0, sv.first<PACKED>(bi) + t0, hi, sv.row<PACKED>(bi));
+      tma_prefetch_4d(&tmap_do, 0, sv.first<PACKED>(p.bi) + t0, p.hi, sv.row<PACKED>(p.bi));
+      tma_prefetch_4d(&tmap_v, 0, sv.first<PACKED>(p.bi) + t0, p.hi, sv.row<PACKED>(p.bi));
       bulk_prefetch_l2(tiles + S_QT * TILE_BYTES, 3 * TILE_BYTES);     // q~, k~, b~
       bulk_prefetch_l2(tiles + S_AT * TILE_BYTES, 3 * TILE_BYTES);     // a~, A_qk, A_ak
       bulk_prefetch_l2(tiles + S_SA * TILE_BYTES, 3 * TILE_BYTES);     // sa, h~0, X
       bulk_prefetch_l2(tiles + S_DZ * TILE_BYTES, 2 * TILE_BYTES);     // dz, dh^
     }
-    const int Tn = sv.length<PACKED>(bi);
-    const long long base = sv.row<PACKED>(bi) * lay.sb + hi * lay.sh + sv.first<PACKED>(bi) * lay.st;
-#pragma unroll
-    for (int n = 0; n < 2; ++n) {
-      const int tok = t0 + lane + 32 * n;
-      if (tok < Tn) asm volatile("prefetch.global.L2 [%0];" ::"l"(w + base + (long long)tok * lay.st));
-    }
   };
   auto load_w = [&](const ChunkPos& p, uint4 (&rw)[2]) {   // all threads: 2 x 8 channels of the chunk's w rows
-    int bi, hi, t0; coords(p, bi, hi, t0);
-    const int Tn = sv.length<PACKED>(bi);
-    const long long base = sv.row<PACKED>(bi) * lay.sb + hi * lay.sh + sv.first<PACKED>(bi) * lay.st;
+    const int t0 = p.c * L, Tn = sv.length<PACKED>(p.bi);
+    const long long base = sv.row<PACKED>(p.bi) * lay.sb + p.hi * lay.sh + sv.first<PACKED>(p.bi) * lay.st;
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
       const int e = tid + 256 * n, row = e >> 3, cc = e & 7, tok = t0 + row;
@@ -454,28 +449,27 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
   };
   ChunkPos cur = chunk_pos(blockIdx.x, NT, H);
   if (cur.ch < n_ch && empty(cur)) cur = advance(cur);
-  ChunkPos nxt = cur;     // the chunk-head after `cur`, and the one after that (found once per iteration)
-  if (cur.ch < n_ch) nxt = advance(cur);
 
   uint4 rw[2];
   if (cur.ch < n_ch) {
-    if (tid == 0) { load_group_a(cur); load_group_b(cur); }
+    if (st_thread) { load_0(cur); load_1a(cur); load_2(cur); load_1b(cur); }
     load_w(cur, rw);
-    if (warp == 1 && nxt.ch < n_ch) prefetch_l2(nxt);
   }
 
   bool ok = true;
   int it = 0;
-  for (ChunkPos aft = nxt; cur.ch < n_ch && ok; cur = nxt, nxt = aft, ++it) {
-    const int ch = cur.ch, next = nxt.ch;
-    int bi, hi, t0; coords(cur, bi, hi, t0);
+  for (ChunkPos nxt; cur.ch < n_ch && ok; cur = nxt, ++it) {
+    const int bi = cur.bi, hi = cur.hi, t0 = cur.c * L;
     const int Tn = sv.length<PACKED>(bi);
     // in a packed batch the last rows of a sequence's last chunk belong to the next sequence: such a chunk
     // is stored row by row instead of by TMA boxes
     const bool row_stores = PACKED && t0 + L > Tn;
     const long long out_base = sv.row<PACKED>(bi) * lay.sb + hi * lay.sh + (long long)(sv.first<PACKED>(bi) + t0) * lay.st;
-    const unsigned char* tiles = ws_tiles + (size_t)ch * tiles_per_chunk * TILE_BYTES;
+    const int tt = sv.first<PACKED>(bi) + t0, br = sv.row<PACKED>(bi);
+    const unsigned char* tiles = ws_tiles + (size_t)cur.ch * tiles_per_chunk * TILE_BYTES;
     const uint32_t par = it & 1;
+    nxt = advance(cur);
+    const bool more = nxt.ch < n_ch;
     R7C_STAMP(16);
 
     // ---- g of every (token, channel), from the w rows already in registers
@@ -495,59 +489,60 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
         g[2 * m] = valid ? -LOG2E * ex2(LOG2E * w0) : 0.f;
         g[2 * m + 1] = valid ? -LOG2E * ex2(LOG2E * w1) : 0.f;
       }
-      *reinterpret_cast<float4*>(&sm.gg[row * NROW + 8 * cc]) = make_float4(g[0], g[1], g[2], g[3]);
-      *reinterpret_cast<float4*>(&sm.gg[row * NROW + 8 * cc + 4]) = make_float4(g[4], g[5], g[6], g[7]);
+      *reinterpret_cast<float4*>(&sm.gs[sw64(row, 8 * cc)]) = make_float4(g[0], g[1], g[2], g[3]);
+      *reinterpret_cast<float4*>(&sm.gs[sw64(row, 8 * cc + 4)]) = make_float4(g[4], g[5], g[6], g[7]);
     }
-    if (tid == 0) bulk_wait_read();    // the TMA stores of the previous chunk-head have left the staging tiles
     R7C_STAMP(17);
-    ok = mbar_wait(&sm.bar_lda, par, status, 321) && ok;
-    ok = mbar_wait(&sm.bar_ldb, par, status, 324) && ok;
+    // ---- MMA group 1: all four dA products; dv; the state part of [dq~; da~]
+    if (lane == 0 && warp < 3) {
+      ok = mbar_wait(&sm.bar_l0, par, status, 321) && ok;
+      ok = mbar_wait(&sm.bar_l1, par, status, 324) && ok;
+      if (ok) {
+        tc_fence_after();
+        if (warp == 0) {
+          umma_tile<128, 128, 0, 0>(tmem_addr(tm, 0, 0), smem_u32(sm.dout), smem_u32(sm.v), false);        // [do;dz] [v;sa]^T
+        } else if (warp == 1) {
+          umma_tile<64, 64, 1, 1, 8>(tmem_addr(tm, 0, 192), smem_u32(sm.aqk), smem_u32(sm.dout), false);   // A_qk^T do + A_ak^T dz
+          umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 192), smem_u32(sm.kt), smem_u32(sm.dhh), true);         // + k~ dh^
+        } else {
+          umma_tile<128, 64, 0, 0>(tmem_addr(tm, 0, 128), smem_u32(sm.dout), smem_u32(sm.h0), false);      // [do;dz] h~0^T
+        }
+        umma_commit(&sm.bar_m1);
+      }
+    }
     ok = __syncthreads_and(ok);
     R7C_STAMP(18);
-
-    // ---- MMA group 1: all four dA products, and dv
-    if (tid == 0 && ok) {
-      tc_fence_after();
-      umma_tile<128, 128, 0, 0>(tmem_addr(tm, 0, 0), smem_u32(sm.dout), smem_u32(sm.v), false);        // [do;dz] [v;sa]^T
-      umma_commit(&sm.bar_m1);
-    }
-    if (tid == 32 && ok) {
-      tc_fence_after();
-      umma_tile<64, 64, 1, 1, 8>(tmem_addr(tm, 0, 128), smem_u32(sm.aqk), smem_u32(sm.dout), false);   // A_qk^T do + A_ak^T dz
-      umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 128), smem_u32(sm.kt), smem_u32(sm.dhh), true);         // + k~ dh^
-      umma_commit(&sm.bar_m1);
-    }
+    if (warp == 3 && more) prefetch_l2(nxt);
     // ---- meanwhile: prefix sums of g over tokens, thread = (channel, quarter of the chunk)
+    float dglast = 0.f;       // threads of the last quarter: sum_v dh^[c][v] X[c][v]
     {
       const int c = tid & 63, quarter = tid >> 6;
       float gv[16];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) gv[j] = sm.gg[(16 * quarter + j) * NROW + c];
+      for (int j = 0; j < 16; ++j) gv[j] = sm.gs[sw64(16 * quarter + j, c)];
       float run = 0.f;
 #pragma unroll
       for (int j = 0; j < 16; ++j) { run += gv[j]; gv[j] = run; }
-      sm.qtot[quarter][c] = run;
+      if (quarter == 1 || quarter == 2) sm.quart[quarter - 1][c] = run;
       __syncthreads();
       // gi - gref: the prefix inside the half; the first half lies before the reference point, the end of that half
-      const float add = quarter == 0 ? -(run + sm.qtot[1][c]) : quarter == 1 ? -run : quarter == 3 ? sm.qtot[2][c] : 0.f;
+      const float add = quarter == 0 ? -(run + sm.quart[0][c]) : quarter == 1 ? -run : quarter == 3 ? sm.quart[1][c] : 0.f;
+      if (quarter == 0) sm.quart[2][c] = add;      // -gref: the exclusive prefix of the first token
 #pragma unroll
-      for (int j = 0; j < 16; ++j) sm.gs[(16 * quarter + j) * NROW + c] = gv[j] + add;
-    }
-    // dglast[c] = sum_v dh^[c][v] X[c][v]  (X straight from the workspace)
-    if (tid >= 128 && tid < 192 && ok) {
-      const int c = tid - 128;
-      float s_ = 0.f;
-      const uint4* xr = reinterpret_cast<const uint4*>(tiles + S_X * TILE_BYTES);
+      for (int j = 0; j < 16; ++j) sm.gs[sw64(16 * quarter + j, c)] = gv[j] + add;
+      if (quarter == 3 && ok) {      // X straight from the workspace
+        ok = mbar_wait(&sm.bar_l0, par, status, 325) && ok;
+        const uint4* xr = reinterpret_cast<const uint4*>(tiles + S_X * TILE_BYTES);
 #pragma unroll
-      for (int cchunk = 0; cchunk < 8; ++cchunk) {
-        const uint4 xa = __ldg(xr + (tile_chunk_off(c, cchunk) >> 4));
-        const uint4 da_ = *reinterpret_cast<const uint4*>(sm.dhh + tile_chunk_off(c, cchunk));
-        s_ += bf16_lo(xa.x) * bf16_lo(da_.x) + bf16_hi(xa.x) * bf16_hi(da_.x);
-        s_ += bf16_lo(xa.y) * bf16_lo(da_.y) + bf16_hi(xa.y) * bf16_hi(da_.y);
-        s_ += bf16_lo(xa.z) * bf16_lo(da_.z) + bf16_hi(xa.z) * bf16_hi(da_.z);
-        s_ += bf16_lo(xa.w) * bf16_lo(da_.w) + bf16_hi(xa.w) * bf16_hi(da_.w);
+        for (int cchunk = 0; cchunk < 8; ++cchunk) {
+          const uint4 xa = __ldg(xr + (tile_chunk_off(c, cchunk) >> 4));
+          const uint4 da_ = *reinterpret_cast<const uint4*>(sm.dhh + tile_chunk_off(c, cchunk));
+          dglast += bf16_lo(xa.x) * bf16_lo(da_.x) + bf16_hi(xa.x) * bf16_hi(da_.x);
+          dglast += bf16_lo(xa.y) * bf16_lo(da_.y) + bf16_hi(xa.y) * bf16_hi(da_.y);
+          dglast += bf16_lo(xa.z) * bf16_lo(da_.z) + bf16_hi(xa.z) * bf16_hi(da_.z);
+          dglast += bf16_lo(xa.w) * bf16_lo(da_.w) + bf16_hi(xa.w) * bf16_hi(da_.w);
+        }
       }
-      sm.dgl[c] = s_;
     }
     ok = mbar_wait(&sm.bar_m1, par, status, 322) && ok;
     tc_fence_after();
@@ -559,7 +554,8 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
       // the same for the whole warp: left of the diagonal block every element is kept, right of it every element
       // is zero (TMEM is not read), and only the diagonal block takes a per-element choice.
       const int ihalf = wq & 1;
-      unsigned char* dst = lower ? (hsel ? sm.daab : sm.daak) : (hsel ? sm.daqb : sm.daqk);
+      // dA tiles, in the order dA_qk, dA_ak, dA_qb, dA_ab, over the operands of group 1
+      unsigned char* dst = sm.dout + ((lower ? 1 : 0) + 2 * hsel) * TILE_BYTES;
 #pragma unroll
       for (int pp = 0; pp < 2; ++pp) {
         const int part = 2 * hsel + pp;   // hsel 0: products with v (dA_qk / dA_ak); hsel 1: with sa (dA_qb / dA_ab)
@@ -587,17 +583,16 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
           tile_store_row32(dst, i, j0, x);
         }
       }
-      // dv rows sit on the lower lane halves of columns 128..191; each warp of a pair takes 32 columns.
-      // Staged in the A_qk tile (dead: MMA group 1 has completed), stored by TMA below.
+      // dv rows sit on the lower lane halves of columns 192..255; each warp of a pair takes 32 columns
       const int row = 16 * wq + (lane & 15);
       uint32_t rr[32];
-      tmem_ld32(tmem_addr(tm, 32 * wq, 128 + 32 * hsel), rr);
+      tmem_ld32(tmem_addr(tm, 32 * wq, 192 + 32 * hsel), rr);
       tmem_ld_wait();
       if (lane < 16) {
         float x[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
-        tile_store_row32(sm.aqk, row, 32 * hsel, x);
+        tile_store_row32(sm.h0, row, 32 * hsel, x);
       }
     }
     fence_async_smem();
@@ -605,135 +600,157 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     ok = __syncthreads_and(ok);
     R7C_STAMP(20);
 
-    // ---- MMA group 2: [dq~; da~] (columns 0..63) and [dk~; db~] (columns 64..127)
-    if (tid == 32 && ok) {
-      tc_fence_after();
-      umma_tile<128, 64, 1, 1>(tmem_addr(tm, 0, 64), smem_u32(sm.daqk), smem_u32(sm.qt), false, 2 * TILE_BYTES);  // [dA_qk|dA_qb]^T q~
-      umma_tile<128, 64, 1, 1>(tmem_addr(tm, 0, 64), smem_u32(sm.daak), smem_u32(sm.at), true, 2 * TILE_BYTES);   // + [dA_ak|dA_ab]^T a~
-      umma_tile<128, 64, 0, 0>(tmem_addr(tm, 0, 64), smem_u32(sm.v), smem_u32(sm.dhh), true);          // + [v;sa] dh^^T
-      umma_commit(&sm.bar_m2);
-    }
-    if (tid == 0 && ok) {
-      tc_fence_after();
-      umma_tile<128, 64, 0, 0>(tmem_addr(tm, 0, 0), smem_u32(sm.dout), smem_u32(sm.h0), false);        // [do;dz] h~0^T
-      umma_tile<128, 64, 0, 1>(tmem_addr(tm, 0, 0), smem_u32(sm.daqk), smem_u32(sm.kt), true);         // + [dA_qk;dA_ak] k~
-      umma_tile<128, 64, 0, 1>(tmem_addr(tm, 0, 0), smem_u32(sm.daqb), smem_u32(sm.bt), true);         // + [dA_qb;dA_ab] b~
-      umma_commit(&sm.bar_m2);
-      if (!row_stores) {
-        tma_store_4d(&tmap_dv, sm.aqk, 0, sv.first<PACKED>(bi) + t0, hi, sv.row<PACKED>(bi));
-        bulk_commit();
+    // ---- MMA group 2: [dq~; da~] completed (columns 128..191), and [dk~; db~] (columns 0..63)
+    if (lane == 0 && warp < 2 && ok) {
+      ok = mbar_wait(&sm.bar_l2, par, status, 326);
+      if (ok) {
+        tc_fence_after();
+        if (warp == 0) {
+          umma_tile<128, 64, 0, 1>(tmem_addr(tm, 0, 128), smem_u32(sm.dout), smem_u32(sm.kt), true);         // + [dA_qk;dA_ak] k~
+          umma_tile<128, 64, 0, 1>(tmem_addr(tm, 0, 128), smem_u32(sm.aqk), smem_u32(sm.bt), true);          // + [dA_qb;dA_ab] b~
+        } else {
+          umma_tile<128, 64, 0, 0>(tmem_addr(tm, 0, 0), smem_u32(sm.v), smem_u32(sm.dhh), false);            // [v;sa] dh^^T
+          umma_tile<128, 64, 1, 1>(tmem_addr(tm, 0, 0), smem_u32(sm.dout), smem_u32(sm.qt), true, 2 * TILE_BYTES);  // + [dA_qk|dA_qb]^T q~
+          umma_tile<128, 64, 1, 1>(tmem_addr(tm, 0, 0), smem_u32(sm.dz), smem_u32(sm.at), true, 2 * TILE_BYTES);    // + [dA_ak|dA_ab]^T a~
+        }
+        umma_commit(&sm.bar_m2);
       }
     }
-    if (row_stores && ok) {
-      store_tile_rows<256>(dv_rows + out_base, lay.st, sm.aqk, Tn - t0, tid);
-      __syncthreads();      // the A_qk tile is loaded again below
+    if (st_thread && ok && !row_stores) {
+      tma_store_4d(&tmap_dv, sm.h0, 0, tt, hi, br);
+      bulk_commit();
     }
+    if (row_stores && ok) store_tile_rows<256>(dv_rows + out_base, lay.st, sm.h0, Tn - t0, tid);
+    if (more) load_w(nxt, rw);
     ok = mbar_wait(&sm.bar_m2, par, status, 323) && ok;
+    ok = mbar_wait(&sm.bar_l2, par, status, 327) && ok;      // the epilogue reads q~, a~, b~ (and k~, which came with group 1)
+    ok = mbar_wait(&sm.bar_l1, par, status, 328) && ok;
     tc_fence_after();
     R7C_STAMP(21);
-    // group A tiles are free: request the next chunk-head's, and fetch its w rows
-    if (next < n_ch) {
-      if (tid == 0 && ok) { bulk_wait_read(); load_group_a(nxt); }
-      load_w(nxt, rw);
-      aft = advance(nxt);
-      if (warp == 1 && aft.ch < n_ch) prefetch_l2(aft);
+    if (st_thread && ok) {
+      if (more) load_0(nxt);      // dh^ and v have been read for the last time
+      bulk_wait_read();           // the copy of dv has left its tile, which will hold dw
     }
 
     // ---- epilogue.  Row r < 64 holds dq~_i and dk~_i (token i = r), row r >= 64 holds da~_i, db~_i; the
-    // two warps of a lane window take 32 channels each.  Row owners read and write the fp32 scratch
-    // arrays as float4 (conflict-free with the padded rows).  red1 = dq~ q~ - dk~ k~ and
-    // red2 = da~ a~ - db~ b~ overlay the dA tiles (dead once MMA group 2 has completed).
-    float* red1 = reinterpret_cast<float*>(sm.daqk);
-    float* red2 = red1 + L * NROW;
+    // two warps of a lane window take 32 channels each.  red1 = dq~ q~ - dk~ k~ and red2 = da~ a~ - db~ b~ overlay
+    // the dA tiles (dead once MMA group 2 has completed); the results replace q~, k~ / a~, b~ row by row.
+    float* red1 = reinterpret_cast<float*>(sm.dout);
+    float* red2 = reinterpret_cast<float*>(sm.aqk);
     if (ok) {
       const int r = 32 * wq + lane, i = r & 63;
       const bool second = r >= 64;
       float* red = second ? red2 : red1;
-      const int c0 = 32 * hsel;
-      uint32_t r1[32], r2[32];
-      tmem_ld32(tmem_addr(tm, 32 * wq, c0), r1);          // dq~ / da~
-      tmem_ld32(tmem_addr(tm, 32 * wq, 64 + c0), r2);     // dk~ / db~
-      tmem_ld_wait();
-      float t1[32], t2[32], o1[32], o2[32], ge[32];
-      tile_load_row32(second ? sm.at : sm.qt, i, c0, t1);
-      tile_load_row32(second ? sm.bt : sm.kt, i, c0, t2);
+      unsigned char* tile1 = second ? sm.at : sm.qt;
+      unsigned char* tile2 = second ? sm.bt : sm.kt;
+      // exponents of the first factor: inclusive prefix for q~, exclusive (the previous token's) for a~
+      const float* grow = second ? (i ? sm.gs + 64 * (i - 1) : sm.quart[2]) : sm.gs + 64 * i;
+      const int gkey = second ? (i ? (i - 1) & 7 : 0) : i & 7;
 #pragma unroll
-      for (int j4 = 0; j4 < 32; j4 += 4) {
-        const int c = c0 + j4;
-        const float4 gs4 = *reinterpret_cast<const float4*>(&sm.gs[i * NROW + c]);
-        const float4 gg4 = *reinterpret_cast<const float4*>(&sm.gg[i * NROW + c]);
-        const float gsv[4] = {gs4.x, gs4.y, gs4.z, gs4.w}, ggv[4] = {gg4.x, gg4.y, gg4.z, gg4.w};
-        float rd[4];
+      for (int half = 0; half < 2; ++half) {
+        const int c0 = 32 * hsel + 16 * half;
+        uint32_t r1[16], r2[16];
+        tmem_ld16(tmem_addr(tm, 32 * wq, 128 + c0), r1);    // dq~ / da~
+        tmem_ld16(tmem_addr(tm, 32 * wq, c0), r2);          // dk~ / db~
+        tmem_ld_wait();
+        float t1[16], t2[16];
+        tile_load_row<16>(tile1, i, c0, t1);
+        tile_load_row<16>(tile2, i, c0, t2);
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          const int j = j4 + m;
-          const float d1 = gsv[m];                                       // gi - gref
-          const float x1 = __uint_as_float(r1[j]), x2 = __uint_as_float(r2[j]);
-          o2[j] = x2 * ex2(-d1);                                         // dk / db
-          o1[j] = x1 * ex2(second ? d1 - ggv[m] : d1);                   // da / dq
-          ge[j] = x1 * t1[j];
-          rd[m] = ge[j] - x2 * t2[j];
+        for (int j4 = 0; j4 < 16; j4 += 4) {
+          const int c = c0 + j4;
+          const float4 gs4 = *reinterpret_cast<const float4*>(&sm.gs[sw64(i, c)]);
+          const float4 ge4 = *reinterpret_cast<const float4*>(grow + (((c >> 2) ^ gkey) << 2));
+          const float gsv[4] = {gs4.x, gs4.y, gs4.z, gs4.w}, gev[4] = {ge4.x, ge4.y, ge4.z, ge4.w};
+          float rd[4];
+#pragma unroll
+          for (int m = 0; m < 4; ++m) {
+            const int j = j4 + m;
+            const float x1 = __uint_as_float(r1[j]), x2 = __uint_as_float(r2[j]);
+            const float e1 = x1 * t1[j];
+            rd[m] = e1 - x2 * t2[j];
+            t1[j] = x1 * ex2(gev[m]);                                      // dq / da
+            t2[j] = x2 * ex2(-gsv[m]);                                     // dk / db
+            r1[j] = __float_as_uint(e1);
+          }
+          *reinterpret_cast<float4*>(&red[sw64(i, c)]) = make_float4(rd[0], rd[1], rd[2], rd[3]);
         }
-        *reinterpret_cast<float4*>(&red[i * NROW + c]) = make_float4(rd[0], rd[1], rd[2], rd[3]);
+        tile_store_row<16>(tile1, i, c0, t1);
+        tile_store_row<16>(tile2, i, c0, t2);
+        if (second) {      // da~ a~
+#pragma unroll
+          for (int j = 0; j < 16; ++j) t1[j] = __uint_as_float(r1[j]);
+          tile_store_row<16>(sm.sa, i, c0, t1);
+        }
       }
-      if (second) tile_store_row32(sm.dge, i, c0, ge);
-      tile_store_row32(sm.stage[second ? 2 : 0], i, c0, o1);    // da / dq
-      tile_store_row32(sm.stage[second ? 3 : 1], i, c0, o2);    // db / dk
     }
     fence_async_smem();
     ok = __syncthreads_and(ok);
     R7C_STAMP(22);
     if (row_stores && ok) {
-      store_tile_rows<256>(dq_rows + out_base, lay.st, sm.stage[0], Tn - t0, tid);
-      store_tile_rows<256>(dk_rows + out_base, lay.st, sm.stage[1], Tn - t0, tid);
-      store_tile_rows<256>(da_rows + out_base, lay.st, sm.stage[2], Tn - t0, tid);
-      store_tile_rows<256>(db_rows + out_base, lay.st, sm.stage[3], Tn - t0, tid);
+      store_tile_rows<256>(dq_rows + out_base, lay.st, sm.qt, Tn - t0, tid);
+      store_tile_rows<256>(dk_rows + out_base, lay.st, sm.kt, Tn - t0, tid);
+      store_tile_rows<256>(da_rows + out_base, lay.st, sm.at, Tn - t0, tid);
+      store_tile_rows<256>(db_rows + out_base, lay.st, sm.bt, Tn - t0, tid);
     }
-    if (tid == 0 && ok) {
-      if (!row_stores) {
-        const int tt = sv.first<PACKED>(bi) + t0, br = sv.row<PACKED>(bi);
-        tma_store_4d(&tmap_dq, sm.stage[0], 0, tt, hi, br);
-        tma_store_4d(&tmap_dk, sm.stage[1], 0, tt, hi, br);
-        tma_store_4d(&tmap_da, sm.stage[2], 0, tt, hi, br);
-        tma_store_4d(&tmap_db, sm.stage[3], 0, tt, hi, br);
-        bulk_commit();
-      }
-      if (next < n_ch) load_group_b(nxt);       // q~, a~, k~, b~ were last read by the epilogue above
+    if (st_thread && ok && !row_stores) {
+      tma_store_4d(&tmap_dq, sm.qt, 0, tt, hi, br);
+      tma_store_4d(&tmap_dk, sm.kt, 0, tt, hi, br);
+      tma_store_4d(&tmap_da, sm.at, 0, tt, hi, br);
+      tma_store_4d(&tmap_db, sm.bt, 0, tt, hi, br);
+      bulk_commit();
     }
     // reverse inclusive prefix over tokens, per channel; thread = (channel, quarter)
     {
       const int c = tid & 63, quarter = tid >> 6;
       float rv[16];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) rv[j] = red1[(16 * quarter + j) * NROW + c] + red2[(16 * quarter + j) * NROW + c];
-      float run = 0.f;
+      for (int j = 0; j < 16; ++j) rv[j] = red1[sw64(16 * quarter + j, c)] + red2[sw64(16 * quarter + j, c)];
+      float run = dglast;
 #pragma unroll
       for (int j = 15; j >= 0; --j) { run += rv[j]; rv[j] = run; }
-      sm.rqtot[quarter][c] = run;
+      const float gfirst = quarter ? sm.gs[sw64(16 * quarter - 1, c)] : sm.quart[2][c];
+      __syncthreads();      // -gref has been read
+      if (quarter) sm.quart[quarter - 1][c] = run;      // the last quarter's sum carries dglast
       __syncthreads();
-      float add = sm.dgl[c];
-      for (int q2 = quarter + 1; q2 < 4; ++q2) add += sm.rqtot[q2][c];
+      float add = 0.f;
+      for (int q2 = quarter; q2 < 3; ++q2) add += sm.quart[q2][c];
+      float gprev = gfirst;
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         const int ii = 16 * quarter + j;
-        const float e_ = __bfloat162float(*reinterpret_cast<const bf16*>(sm.dge + tile_off(ii, c)));
+        const float e_ = __bfloat162float(*reinterpret_cast<const bf16*>(sm.sa + tile_off(ii, c)));
         const float dg = rv[j] + add - e_;
-        // dw = dg g, with g = gg ln 2 (gg is in units of log 2)
-        *reinterpret_cast<bf16*>(sm.stage[4] + tile_off(ii, c)) = __float2bfloat16_rn(dg * (LN2 * sm.gg[ii * NROW + c]));
+        // dw = dg g; g is the difference of neighbouring prefix sums (in units of log 2)
+        const float gi = sm.gs[sw64(ii, c)];
+        *reinterpret_cast<bf16*>(sm.h0 + tile_off(ii, c)) = __float2bfloat16_rn(dg * (LN2 * (gi - gprev)));
+        gprev = gi;
       }
     }
     fence_async_smem();
     tc_fence_before();
     ok = __syncthreads_and(ok);
     if (row_stores) {
-      if (ok) store_tile_rows<256>(dw_rows + out_base, lay.st, sm.stage[4], Tn - t0, tid);
-    } else if (tid == 0 && ok) {
-      tma_store_4d(&tmap_dw, sm.stage[4], 0, sv.first<PACKED>(bi) + t0, hi, sv.row<PACKED>(bi));
-      bulk_commit();
+      if (ok) store_tile_rows<256>(dw_rows + out_base, lay.st, sm.h0, Tn - t0, tid);
+      fence_async_smem();
+      __syncthreads();      // the rows are read before their space is loaded again
+    }
+    if (st_thread && ok) {
+      if (!row_stores) {
+        tma_store_4d(&tmap_dw, sm.h0, 0, tt, hi, br);
+        bulk_commit();
+      }
+      if (more) {
+        load_1a(nxt);
+        bulk_wait_read_1();       // dq, dk, da, db have left their tiles
+        load_2(nxt);
+        bulk_wait_read();         // and dw
+        load_1b(nxt);
+      }
     }
     R7C_STAMP(23);
   }
-  if (tid == 0) bulk_wait_all();
+  if (st_thread) bulk_wait_all();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tm, 256);
@@ -885,13 +902,13 @@ int launch_rwkv7_chunked_bwd(const void* r, const void* w, const void* k, const 
     return e;
   }
   {
-    const int smem = (int)sizeof(FinalSmem) + 1024;
+    const int smem = (int)sizeof(FinalSmem);
     ProfScope prof("r7c_bwd_final_kernel", st);
     const int n_ch = B * H * NT;
     int dev = 0, sms = 0;
     if (cuda_ok(cudaGetDevice(&dev)) || cuda_ok(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)))
       return RWKVB200_E_CUDA;
-    const int grid = n_ch < sms ? n_ch : sms;     // persistent: one CTA per SM
+    const int grid = n_ch < 2 * sms ? n_ch : 2 * sms;     // persistent: two CTAs per SM
 #define R7C_LAUNCH_FINAL(P, F)                                                                                    \
     do {                                                                                                          \
       if (cuda_ok(cudaFuncSetAttribute(r7c_bwd_final_kernel<P, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem))) \
