@@ -32,10 +32,6 @@
 //     dk~ = dA_qk^T q~ + dA_ak^T a~ + v dh^^T     db~ = dA_qb^T q~ + dA_ab^T a~ + sa dh^^T
 //     dq = dq~ e^{gi-gref} ...;  dgi = dq~ q~ - dk~ k~ - db~ b~;  dge = da~ a~;  dglast = sum_v dh_L h_L
 //     dg_j = sum_{i>=j} (dgi_i + dge_i) - dge_j + dglast;   dw = dg g
-// dglast contains the state parts of dk~ k~ and db~ b~ of the whole chunk, X = (v dh^^T) k~ + (sa dh^^T) b~, and the sum
-// over i >= j takes them away again: with large states (long runs without decay) that difference lost most of its
-// digits.  So they are summed where they remain, dgi without them (dgi', from inside the chunk):
-//     dg_j = sum_{i>=j} (dgi'_i + dge_i) - dge_j + sum_{i<j} X_i + sum_v dh^ h~0
 // (reference: chunk_o_bwd.py:111-113,246-277,364-381, chunk_h_bwd.py:141-157, wy_fast_bwd.py:99-193,
 // chunk_A_bwd.py:146-250,318-320 under rwkv_ops/rwkv7_kernel/triton_kernel/).
 // These are the chunk equations of the reference's kernels (rwkv_ops/rwkv7_kernel/triton_kernel/
@@ -64,7 +60,7 @@ enum Slot { // what the two scans read: Q, P, N (float32, two slots), O' -- one 
             S_G = FWD_TILES, S_B2, S_W, S_U, S_QT, S_AT, S_KT, S_BT, S_AQK, S_AAK,
             // h~0, written by the forward scan; dh^, written by the backward scan
             S_H0, S_DHH, ALL_TILES };
-// per chunk: e^{gref}[64], e^{glast-gref}[64] (intra kernel), sum_v dh^ h~0 [64] (backward scan)
+// per chunk: e^{gref}[64], e^{glast-gref}[64] (intra kernel), dglast[64] (backward scan)
 constexpr int AUX_FLOATS = 192;
 // Index of (row, channel) in a 64 x 64 float32 array whose 16-byte pieces are permuted by the row, so that threads that
 // own a row and threads that own a channel both access it without bank conflicts (N is stored like this as well).
@@ -143,6 +139,7 @@ struct Workspace {
   unsigned char* tiles;   // [n_chunks_total][tiles_per_chunk][8192]
   float* aux;             // [n_chunks_total][AUX_FLOATS]
   int* flags;             // [B*H] nonzero: the unit's decay left the range of the scaled operands (DECAY_LIMIT)
+  unsigned char* fin;     // [B*H][8192] final state as bf16 tiles (kept for the backward)
   int tiles_per_chunk;
 };
 
@@ -165,7 +162,7 @@ inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 inline size_t fwd_workspace_bytes(int B, int T, int H, int tiles_per_chunk) {
   const size_t n = (size_t)B * H * num_chunks(T);
   return align256(n * tiles_per_chunk * tc::TILE_BYTES) + align256(n * AUX_FLOATS * sizeof(float)) +
-         align256((size_t)B * H * sizeof(int)) + 1024;
+         align256((size_t)B * H * sizeof(int)) + (tiles_per_chunk == ALL_TILES ? (size_t)B * H * tc::TILE_BYTES : 0) + 1024;
 }
 
 inline Workspace carve(void* ws, int B, int T, int H, int tiles_per_chunk) {
@@ -175,6 +172,8 @@ inline Workspace carve(void* ws, int B, int T, int H, int tiles_per_chunk) {
   w.tiles = reinterpret_cast<unsigned char*>(p);
   w.aux = reinterpret_cast<float*>(p + align256(n * tiles_per_chunk * tc::TILE_BYTES));
   w.flags = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(w.aux) + align256(n * AUX_FLOATS * sizeof(float)));
+  w.fin = tiles_per_chunk == ALL_TILES
+              ? reinterpret_cast<unsigned char*>(w.flags) + align256((size_t)B * H * sizeof(int)) : nullptr;
   w.tiles_per_chunk = tiles_per_chunk;
   return w;
 }

@@ -2,7 +2,7 @@
 //
 // Launch sequence (all on the caller's stream, tiles exchanged through the workspace):
 //   1. forward intra kernel with keep_for_bwd (P, Q and the tiles the final kernel reads), forward scan (h~0)
-//   2. r7c_bwd_scan_kernel   (one CTA per (b,h), chunks in reverse)  dh^ and sum_v dh^ h~0 per chunk, d initial state
+//   2. r7c_bwd_scan_kernel   (one CTA per (b,h), chunks in reverse)  dh^ and dglast per chunk, d initial state
 //   3. r7c_bwd_final_kernel  (parallel over chunks)   dq, dk, dv, da, db, dw
 // (1. only where the forward call has not left its tiles)
 #include "rwkv7_chunked.cuh"
@@ -25,14 +25,14 @@ typedef __nv_bfloat16 bf16;
 struct BScanStage {
   unsigned char q[TILE_BYTES], p[TILE_BYTES];     // adjacent workspace slots: one bulk copy
   unsigned char dout[TILE_BYTES];
-  unsigned char h0[TILE_BYTES];                   // h~0
+  unsigned char hn[TILE_BYTES];                   // h~0 of the next chunk, or the final state
 };
 template <int STAGES>
 struct BScanSmem {
   BScanStage st[STAGES];
   unsigned char dh[TILE_BYTES];       // dh as bf16, [k][v]
   unsigned char dhh[2][TILE_BYTES];   // dh^ as bf16 (kept for the final kernel)
-  float part[2][2][64];               // sum_v dh^ h~0 of a chunk, by column half
+  float part[2][2][64];               // dglast of a chunk, by column half
   uint64_t bar_ld[STAGES], bar_m[2];
   uint32_t tmem_base;
 };
@@ -41,7 +41,7 @@ static_assert(sizeof(BScanSmem<2>) + 1024 <= 115712, "two CTAs per SM");
 template <int STAGES, bool PACKED>
 __global__ void __launch_bounds__(256, STAGES == 2 ? 2 : 1)
 r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* __restrict__ ws_tiles,
-                    float* __restrict__ ws_aux, int tiles_per_chunk,
+                    float* __restrict__ ws_aux, const unsigned char* __restrict__ fin_tiles, int tiles_per_chunk,
                     const float* __restrict__ d_ht, float* __restrict__ d_h0, SeqView sv, int H, int NT_slots,
                     int* status) {
   extern __shared__ unsigned char smem_raw[];
@@ -76,7 +76,8 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
     mbar_expect_tx(bar, sizeof(BScanStage));
     bulk_load(g.q, tiles + S_Q * TILE_BYTES, 2 * TILE_BYTES, bar);
     tma_load_4d(g.dout, &tmap_do, bar, 0, tb + c * L, hi, brow);
-    bulk_load(g.h0, tiles + S_H0 * TILE_BYTES, TILE_BYTES, bar);
+    bulk_load(g.hn, n == 0 ? fin_tiles + (size_t)unit * TILE_BYTES
+                           : tiles + ((size_t)tiles_per_chunk + S_H0) * TILE_BYTES, TILE_BYTES, bar);
   };
   if (ld_thread)
     for (int n = 0; n < STAGES && n < NT; ++n) issue_load(n);
@@ -93,7 +94,7 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
   }
 
   // the decay factors of a chunk are fetched one chunk ahead
-  float eg_next = 1.f, dl_next = 1.f;
+  float eg_next = 1.f, dl_next = 1.f, eg_after = 1.f;
   if (state_lane) {
     eg_next = ws_aux[(ch0 + NT - 1) * AUX_FLOATS + row];
     dl_next = ws_aux[(ch0 + NT - 1) * AUX_FLOATS + 64 + row];
@@ -134,23 +135,24 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
     }
     // the stage of the chunk before has been read: by its products, and its h~0 by every thread before the barrier
     if (ld_thread && n > 0 && n - 1 + STAGES < NT) issue_load(n - 1 + STAGES);
-    if (n > 0) {      // what the chunk before left: its dh^ tile and its sum_v dh^ h~0
+    if (n > 0) {      // what the chunk before left: its dh^ tile and its dglast
       if (st_thread) {
         bulk_store(tiles + ((size_t)tiles_per_chunk + S_DHH) * TILE_BYTES, sm.dhh[t ^ 1], TILE_BYTES);
         bulk_commit();
       }
       if (tid >= 192) ws_aux[(ch0 + c + 1) * AUX_FLOATS + 128 + tid - 192] = sm.part[t ^ 1][0][tid - 192] + sm.part[t ^ 1][1][tid - 192];
     }
-    // under the product: dh^ = e^{glast-gref} dh, and sum_v dh^ h~0
+    // under the product: dh^ = e^{glast-gref} dh, and dglast = sum_v dh h_L with h_L = h~0 / e^{gref} of the next chunk
     ok = ok && mbar_wait(&sm.bar_ld[s], sp, status, 314);
     if (state_lane && ok) {
       float y[32], h[32];
-      tile_load_row32(sm.st[s].h0, row, c0, h);
+      tile_load_row32(sm.st[s].hn, row, c0, h);
       float acc = 0.f;
 #pragma unroll
-      for (int j = 0; j < 32; ++j) { y[j] = dh[j] * dl; acc += y[j] * h[j]; }
+      for (int j = 0; j < 32; ++j) { acc += dh[j] * h[j]; y[j] = dh[j] * dl; }
       tile_store_row32(sm.dhh[t], row, c0, y);
-      sm.part[t][hsel][row] = acc;
+      sm.part[t][hsel][row] = n == 0 ? acc : acc / eg_after;
+      eg_after = eg;
     }
     ok = ok && mbar_wait(&sm.bar_m[t], tp, status, 312);
     tc_fence_after();
@@ -192,30 +194,22 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
 // twelve tiles whose space is used over again (names below: what is loaded, then what replaces it) and one fp32
 // array, and an accumulator that does not need the dA tiles is issued with the first MMA group, which frees its
 // operands.  TMEM: sa | dz columns 192..255, then dv there (lower lane halves); dA 0..127, [dq~; da~] 128..191;
-// [dk~; db~] once dA has been read, their parts from inside the chunk in 0..63 and from the state in 64..127.
-// Sums over tokens run in (channel, quarter of the chunk) threads, the quarters of a channel in one warp.
+// [dk~; db~] 0..63 once dA has been read.
 struct FinalSmem {
   unsigned char dout[TILE_BYTES], dz[TILE_BYTES];       // [do; dz]   (dz: W before)   then dA_qk, dA_ak   then red1 (fp32)
   unsigned char aqk[TILE_BYTES], aak[TILE_BYTES];       // A_qk, A_ak                  then dA_qb, dA_ab   then red2 (fp32)
   unsigned char h0[TILE_BYTES];                         // h~0                         then dv rows        then dw rows
-  unsigned char dhh[TILE_BYTES];                        // dh^                          then (sa dh^^T) b~ as bf16
-  unsigned char v[TILE_BYTES], sa[TILE_BYTES];          // [v; sa]    (sa: G before)   then (v dh^^T) k~ and da~ a~ as bf16
+  unsigned char dhh[TILE_BYTES];                        // dh^
+  unsigned char v[TILE_BYTES], sa[TILE_BYTES];          // [v; sa]    (sa: G before)   then (sa) da~ a~ as bf16
   unsigned char qt[TILE_BYTES], at[TILE_BYTES];         // q~, a~     (a~: B2 before)  then dq, da rows
   unsigned char kt[TILE_BYTES], bt[TILE_BYTES];         // k~, b~     (b~: U before)   then dk, db rows
-  float gs[L * 64];         // g log2(e), then (gi - gref) log2(e): inclusive prefix inside the chunk (swq)
-  float gex0[64];           // -gref log2(e): the exclusive prefix of the first token
-  uint64_t bar_l1, bar_l2, bar_m0, bar_m1, bar_m2;
+  float gs[L * 64];         // g log2(e), then (gi - gref) log2(e): inclusive prefix inside the chunk (sw64)
+  float quart[3][64];       // sums over quarters of the chunk; [2] between the prefix sum and the epilogue: -gref
+  uint64_t bar_l0, bar_l1, bar_l2, bar_m0, bar_m1, bar_m2;
   uint32_t tmem_base;
 };
 // two CTAs per SM: 228 KB shared by both, 1 KB of each reserved by the system
 static_assert(sizeof(FinalSmem) <= 115712, "two CTAs per SM");
-
-// Swizzles of the arrays that threads owning a row and (channel, quarter) threads share: 16-byte pieces permuted by the
-// row and by its quarter, which keeps both free of bank conflicts.  swq: 64 x 64 fp32; bfq: 64 x 64 bf16, byte offset of
-// a 16-byte piece.
-__device__ __forceinline__ int rowkey(int row) { return (row ^ ((row >> 4) << 1)) & 7; }
-__device__ __forceinline__ int swq(int row, int c) { return row * 64 + ((((c >> 2) ^ rowkey(row)) << 2) | (c & 3)); }
-__device__ __forceinline__ int bfq(int row, int piece) { return row * 128 + ((piece ^ rowkey(row)) << 4); }
 
 // 256 threads: warp w reads TMEM lanes 32*(w&3).. (its row), and the two warps that share a lane
 // window split the columns (hsel = w>>2), so every elementwise phase is spread over 8 warps.
@@ -247,8 +241,8 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
   if (tid == 0) {
     // an MMA group is issued by several threads, one accumulator each, and completes with the arrival of all: one
     // thread issues an MMA about every 80 cycles, the tensor pipe takes them faster
-    mbar_init(&sm.bar_l1, 1); mbar_init(&sm.bar_l2, 1);
-    mbar_init(&sm.bar_m0, 2); mbar_init(&sm.bar_m1, 3); mbar_init(&sm.bar_m2, 3);
+    mbar_init(&sm.bar_l0, 1); mbar_init(&sm.bar_l1, 1); mbar_init(&sm.bar_l2, 1);
+    mbar_init(&sm.bar_m0, 2); mbar_init(&sm.bar_m1, 3); mbar_init(&sm.bar_m2, 2);
     fence_mbar_init();
   }
   if (warp == 0) tmem_alloc(&sm.tmem_base, 256);
@@ -257,15 +251,18 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
   tc_fence_after();
   const uint32_t tm = sm.tmem_base;
   const bool st_thread = tid == 96;      // requests the tiles, stores the results
-  const int ch_c = 8 * warp + (lane & 7), quarter = lane >> 3;      // (channel, quarter) role
 
   // the tiles of a chunk-head in the order in which their space becomes free
+  auto load_0 = [&](const ChunkPos& p) {      // dh^, v
+    const unsigned char* tiles = ws_tiles + (size_t)p.ch * tiles_per_chunk * TILE_BYTES;
+    mbar_expect_tx(&sm.bar_l0, 2 * TILE_BYTES);
+    bulk_load(sm.dhh, tiles + S_DHH * TILE_BYTES, TILE_BYTES, &sm.bar_l0);
+    tma_load_4d(sm.v, &tmap_v, &sm.bar_l0, 0, sv.first<PACKED>(p.bi) + p.c * L, p.hi, sv.row<PACKED>(p.bi));
+  };
   auto load_1a = [&](const ChunkPos& p) {     // the other operands of MMA groups 0 and 1, but for those below
     const unsigned char* tiles = ws_tiles + (size_t)p.ch * tiles_per_chunk * TILE_BYTES;
-    mbar_expect_tx(&sm.bar_l1, 11 * TILE_BYTES);
+    mbar_expect_tx(&sm.bar_l1, 9 * TILE_BYTES);
     tma_load_4d(sm.dout, &tmap_do, &sm.bar_l1, 0, sv.first<PACKED>(p.bi) + p.c * L, p.hi, sv.row<PACKED>(p.bi));
-    tma_load_4d(sm.v, &tmap_v, &sm.bar_l1, 0, sv.first<PACKED>(p.bi) + p.c * L, p.hi, sv.row<PACKED>(p.bi));
-    bulk_load(sm.dhh, tiles + S_DHH * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
     bulk_load(sm.dz, tiles + S_W * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
     bulk_load(sm.sa, tiles + S_G * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
     bulk_load(sm.aqk, tiles + S_AQK * TILE_BYTES, 2 * TILE_BYTES, &sm.bar_l1);
@@ -324,7 +321,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
 
   uint4 rw[2];
   if (cur.ch < n_ch) {
-    if (st_thread) { load_1a(cur); load_1b(cur); load_1c(cur); }
+    if (st_thread) { load_0(cur); load_1a(cur); load_1b(cur); load_1c(cur); }
     load_w(cur, rw);
   }
 
@@ -360,12 +357,13 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
         g[2 * m] = valid ? -LOG2E * ex2(LOG2E * w0) : 0.f;
         g[2 * m + 1] = valid ? -LOG2E * ex2(LOG2E * w1) : 0.f;
       }
-      *reinterpret_cast<float4*>(&sm.gs[swq(row, 8 * cc)]) = make_float4(g[0], g[1], g[2], g[3]);
-      *reinterpret_cast<float4*>(&sm.gs[swq(row, 8 * cc + 4)]) = make_float4(g[4], g[5], g[6], g[7]);
+      *reinterpret_cast<float4*>(&sm.gs[sw64(row, 8 * cc)]) = make_float4(g[0], g[1], g[2], g[3]);
+      *reinterpret_cast<float4*>(&sm.gs[sw64(row, 8 * cc + 4)]) = make_float4(g[4], g[5], g[6], g[7]);
     }
     R7C_STAMP(17);
     // ---- MMA group 0: sa = W h~0 (+ U) | dz = G^T do + B2 dh^
     if (lane == 0 && warp < 2) {
+      ok = mbar_wait(&sm.bar_l0, par, status, 321) && ok;
       ok = mbar_wait(&sm.bar_l1, par, status, 324) && ok;
       if (ok) {
         tc_fence_after();
@@ -382,20 +380,24 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     R7C_STAMP(18);
     if (warp == 3 && more) prefetch_l2(nxt);
     // ---- meanwhile: prefix sums of g over tokens, thread = (channel, quarter of the chunk)
-    const float dstate = __ldg(ws_aux + (size_t)cur.ch * AUX_FLOATS + 128 + ch_c);      // sum_v dh^ h~0, from the reverse scan
+    float dglast = 0.f;       // threads of the last quarter: from the reverse scan
+    float gfirst = 0.f;       // threads of the first quarter: -gref, the exclusive prefix of the first token
     {
+      const int c = tid & 63, quarter = tid >> 6;
+      if (quarter == 3) dglast = __ldg(ws_aux + (size_t)cur.ch * AUX_FLOATS + 128 + c);
       float gv[16];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) gv[j] = sm.gs[swq(16 * quarter + j, ch_c)];
+      for (int j = 0; j < 16; ++j) gv[j] = sm.gs[sw64(16 * quarter + j, c)];
       float run = 0.f;
 #pragma unroll
       for (int j = 0; j < 16; ++j) { run += gv[j]; gv[j] = run; }
-      const float q1 = __shfl_sync(0xffffffffu, run, (lane & 7) + 8), q2 = __shfl_sync(0xffffffffu, run, (lane & 7) + 16);
+      if (quarter == 1 || quarter == 2) sm.quart[quarter - 1][c] = run;
+      __syncthreads();
       // gi - gref: the prefix inside the half; the first half lies before the reference point, the end of that half
-      const float add = quarter == 0 ? -(run + q1) : quarter == 1 ? -run : quarter == 3 ? q2 : 0.f;
-      if (quarter == 0) sm.gex0[ch_c] = add;
+      const float add = quarter == 0 ? -(run + sm.quart[0][c]) : quarter == 1 ? -run : quarter == 3 ? sm.quart[1][c] : 0.f;
+      if (quarter == 0) { gfirst = add; sm.quart[2][c] = add; }
 #pragma unroll
-      for (int j = 0; j < 16; ++j) sm.gs[swq(16 * quarter + j, ch_c)] = gv[j] + add;
+      for (int j = 0; j < 16; ++j) sm.gs[sw64(16 * quarter + j, c)] = gv[j] + add;
     }
     ok = mbar_wait(&sm.bar_l1, par, status, 325) && ok;      // U
     ok = ok && mbar_wait(&sm.bar_m0, par, status, 329);
@@ -489,19 +491,18 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     ok = __syncthreads_and(ok);
     R7C_STAMP(20);
 
-    // ---- MMA group 2: [dq~; da~] completed (columns 128..191), and the two parts of [dk~; db~] (columns 0..127)
-    if (lane == 0 && warp < 3 && ok) {
+    // ---- MMA group 2: [dq~; da~] completed (columns 128..191), and [dk~; db~] (columns 0..63)
+    if (lane == 0 && warp < 2 && ok) {
       ok = mbar_wait(&sm.bar_l2, par, status, 326);
       if (ok) {
         tc_fence_after();
         if (warp == 0) {
           umma_tile<128, 64, 0, 1>(tmem_addr(tm, 0, 128), smem_u32(sm.dout), smem_u32(sm.kt), true);         // + [dA_qk;dA_ak] k~
           umma_tile<128, 64, 0, 1>(tmem_addr(tm, 0, 128), smem_u32(sm.aqk), smem_u32(sm.bt), true);          // + [dA_qb;dA_ab] b~
-        } else if (warp == 1) {
-          umma_tile<128, 64, 1, 1>(tmem_addr(tm, 0, 0), smem_u32(sm.dout), smem_u32(sm.qt), false, 2 * TILE_BYTES); // [dA_qk|dA_qb]^T q~
-          umma_tile<128, 64, 1, 1>(tmem_addr(tm, 0, 0), smem_u32(sm.dz), smem_u32(sm.at), true, 2 * TILE_BYTES);    // + [dA_ak|dA_ab]^T a~
         } else {
-          umma_tile<128, 64, 0, 0>(tmem_addr(tm, 0, 64), smem_u32(sm.v), smem_u32(sm.dhh), false);           // [v;sa] dh^^T
+          umma_tile<128, 64, 0, 0>(tmem_addr(tm, 0, 0), smem_u32(sm.v), smem_u32(sm.dhh), false);            // [v;sa] dh^^T
+          umma_tile<128, 64, 1, 1>(tmem_addr(tm, 0, 0), smem_u32(sm.dout), smem_u32(sm.qt), true, 2 * TILE_BYTES);  // + [dA_qk|dA_qb]^T q~
+          umma_tile<128, 64, 1, 1>(tmem_addr(tm, 0, 0), smem_u32(sm.dz), smem_u32(sm.at), true, 2 * TILE_BYTES);    // + [dA_ak|dA_ab]^T a~
         }
         umma_commit(&sm.bar_m2);
       }
@@ -517,12 +518,14 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     ok = mbar_wait(&sm.bar_l1, par, status, 328) && ok;
     tc_fence_after();
     R7C_STAMP(21);
-    if (st_thread && ok) bulk_wait_read();      // the copy of dv has left its tile, which will hold dw
+    if (st_thread && ok) {
+      if (more) load_0(nxt);      // dh^ and v have been read for the last time
+      bulk_wait_read();           // the copy of dv has left its tile, which will hold dw
+    }
 
     // ---- epilogue.  Row r < 64 holds dq~_i and dk~_i (token i = r), row r >= 64 holds da~_i, db~_i; the
-    // two warps of a lane window take 32 channels each.  With dk~, db~ from inside the chunk, red1 = dq~ q~ - dk~ k~ and
-    // red2 = da~ a~ - db~ b~ overlay the dA tiles (dead once MMA group 2 has completed); the state parts (v dh^^T) k~ and
-    // (sa dh^^T) b~ go over v and dh^; the results replace q~, k~ / a~, b~ row by row.
+    // two warps of a lane window take 32 channels each.  red1 = dq~ q~ - dk~ k~ and red2 = da~ a~ - db~ b~ overlay
+    // the dA tiles (dead once MMA group 2 has completed); the results replace q~, k~ / a~, b~ row by row.
     float* red1 = reinterpret_cast<float*>(sm.dout);
     float* red2 = reinterpret_cast<float*>(sm.aqk);
     if (ok) {
@@ -531,56 +534,44 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
       float* red = second ? red2 : red1;
       unsigned char* tile1 = second ? sm.at : sm.qt;
       unsigned char* tile2 = second ? sm.bt : sm.kt;
-      unsigned char* tilex = second ? sm.dhh : sm.v;
       // exponents of the first factor: inclusive prefix for q~, exclusive (the previous token's) for a~
-      const float* grow = second ? (i ? sm.gs + 64 * (i - 1) : sm.gex0) : sm.gs + 64 * i;
-      const int gkey = second ? (i ? rowkey(i - 1) : 0) : rowkey(i);
+      const float* grow = second ? (i ? sm.gs + 64 * (i - 1) : sm.quart[2]) : sm.gs + 64 * i;
+      const int gkey = second ? (i ? (i - 1) & 7 : 0) : i & 7;
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         const int c0 = 32 * hsel + 16 * half;
-        uint32_t r1[16], r2[16], r3[16];
+        uint32_t r1[16], r2[16];
         tmem_ld16(tmem_addr(tm, 32 * wq, 128 + c0), r1);    // dq~ / da~
-        tmem_ld16(tmem_addr(tm, 32 * wq, c0), r2);          // dk~ / db~ from inside the chunk
-        tmem_ld16(tmem_addr(tm, 32 * wq, 64 + c0), r3);     // and from the state
+        tmem_ld16(tmem_addr(tm, 32 * wq, c0), r2);          // dk~ / db~
         tmem_ld_wait();
-        float t1[16], t2[16], xs[16];
+        float t1[16], t2[16];
         tile_load_row<16>(tile1, i, c0, t1);
         tile_load_row<16>(tile2, i, c0, t2);
 #pragma unroll
         for (int j4 = 0; j4 < 16; j4 += 4) {
           const int c = c0 + j4;
-          const float4 gs4 = *reinterpret_cast<const float4*>(&sm.gs[swq(i, c)]);
+          const float4 gs4 = *reinterpret_cast<const float4*>(&sm.gs[sw64(i, c)]);
           const float4 ge4 = *reinterpret_cast<const float4*>(grow + (((c >> 2) ^ gkey) << 2));
           const float gsv[4] = {gs4.x, gs4.y, gs4.z, gs4.w}, gev[4] = {ge4.x, ge4.y, ge4.z, ge4.w};
           float rd[4];
 #pragma unroll
-          for (int m = 0; m < 4; m += 2) {
+          for (int m = 0; m < 4; ++m) {
             const int j = j4 + m;
-            const float x10 = __uint_as_float(r1[j]), x11 = __uint_as_float(r1[j + 1]);
-            const float x20 = __uint_as_float(r2[j]), x21 = __uint_as_float(r2[j + 1]);
-            const float x30 = __uint_as_float(r3[j]), x31 = __uint_as_float(r3[j + 1]);
-            float e10, e11;
-            mul2(e10, e11, x10, x11, t1[j], t1[j + 1]);
-            mul2(xs[j], xs[j + 1], x30, x31, t2[j], t2[j + 1]);
-            fma2(rd[m], rd[m + 1], -x20, -x21, t2[j], t2[j + 1], e10, e11);
-            mul2(t1[j], t1[j + 1], x10, x11, ex2(gev[m]), ex2(gev[m + 1]));                          // dq / da
-            mul2(t2[j], t2[j + 1], x20 + x30, x21 + x31, ex2(-gsv[m]), ex2(-gsv[m + 1]));            // dk / db
-            r1[j] = __float_as_uint(e10); r1[j + 1] = __float_as_uint(e11);
+            const float x1 = __uint_as_float(r1[j]), x2 = __uint_as_float(r2[j]);
+            const float e1 = x1 * t1[j];
+            rd[m] = e1 - x2 * t2[j];
+            t1[j] = x1 * ex2(gev[m]);                                      // dq / da
+            t2[j] = x2 * ex2(-gsv[m]);                                     // dk / db
+            r1[j] = __float_as_uint(e1);
           }
-          *reinterpret_cast<float4*>(&red[swq(i, c)]) = make_float4(rd[0], rd[1], rd[2], rd[3]);
+          *reinterpret_cast<float4*>(&red[sw64(i, c)]) = make_float4(rd[0], rd[1], rd[2], rd[3]);
         }
         tile_store_row<16>(tile1, i, c0, t1);
         tile_store_row<16>(tile2, i, c0, t2);
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
-          *reinterpret_cast<uint4*>(tilex + bfq(i, (c0 >> 3) + q)) =
-              make_uint4(pack_bf16(xs[8 * q], xs[8 * q + 1]), pack_bf16(xs[8 * q + 2], xs[8 * q + 3]),
-                         pack_bf16(xs[8 * q + 4], xs[8 * q + 5]), pack_bf16(xs[8 * q + 6], xs[8 * q + 7]));
         if (second) {      // da~ a~
-          auto e = [&](int j) { return pack_bf16(__uint_as_float(r1[j]), __uint_as_float(r1[j + 1])); };
 #pragma unroll
-          for (int q = 0; q < 2; ++q)
-            *reinterpret_cast<uint4*>(sm.sa + bfq(i, (c0 >> 3) + q)) = make_uint4(e(8 * q), e(8 * q + 2), e(8 * q + 4), e(8 * q + 6));
+          for (int j = 0; j < 16; ++j) t1[j] = __uint_as_float(r1[j]);
+          tile_store_row<16>(sm.sa, i, c0, t1);
         }
       }
     }
@@ -600,40 +591,28 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
       tma_store_4d(&tmap_db, sm.bt, 0, tt, hi, br);
       bulk_commit();
     }
-    // ---- decay gradient, thread = (channel, quarter): sums over i >= j of red1 + red2, over i < j of the state parts
+    // reverse inclusive prefix over tokens, per channel; thread = (channel, quarter)
     {
-      float rv[16], xv[16];
-      auto bf = [&](const unsigned char* t, int row) {
-        return __uint_as_float((uint32_t)*reinterpret_cast<const unsigned short*>(t + bfq(row, ch_c >> 3) + 2 * (ch_c & 7)) << 16);
-      };
-      float run = 0.f, xrun = 0.f;
+      const int c = tid & 63, quarter = tid >> 6;
+      float rv[16];
 #pragma unroll
-      for (int j = 15; j >= 0; --j) {
-        const int ii = 16 * quarter + j;
-        run += red1[swq(ii, ch_c)] + red2[swq(ii, ch_c)];
-        rv[j] = run;
-      }
+      for (int j = 0; j < 16; ++j) rv[j] = red1[sw64(16 * quarter + j, c)] + red2[sw64(16 * quarter + j, c)];
+      float run = dglast;
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const int ii = 16 * quarter + j;
-        xv[j] = xrun;
-        xrun += bf(sm.v, ii) + bf(sm.dhh, ii);
-      }
-      float add = dstate;
-#pragma unroll
-      for (int q2 = 0; q2 < 4; ++q2) {
-        const float rt = __shfl_sync(0xffffffffu, run, (lane & 7) + 8 * q2), xt = __shfl_sync(0xffffffffu, xrun, (lane & 7) + 8 * q2);
-        if (q2 > quarter) add += rt;
-        if (q2 < quarter) add += xt;
-      }
-      float gprev = quarter ? sm.gs[swq(16 * quarter - 1, ch_c)] : sm.gex0[ch_c];
+      for (int j = 15; j >= 0; --j) { run += rv[j]; rv[j] = run; }
+      if (quarter) sm.quart[quarter - 1][c] = run;      // the last quarter's sum carries dglast
+      __syncthreads();
+      float add = 0.f;
+      for (int q2 = quarter; q2 < 3; ++q2) add += sm.quart[q2][c];
+      float gprev = quarter ? sm.gs[sw64(16 * quarter - 1, c)] : gfirst;
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         const int ii = 16 * quarter + j;
-        const float dg = (rv[j] + xv[j]) + (add - bf(sm.sa, ii));
+        const float e_ = __bfloat162float(*reinterpret_cast<const bf16*>(sm.sa + tile_off(ii, c)));
+        const float dg = rv[j] + add - e_;
         // dw = dg g; g is the difference of neighbouring prefix sums (in units of log 2)
-        const float gi = sm.gs[swq(ii, ch_c)];
-        *reinterpret_cast<bf16*>(sm.h0 + tile_off(ii, ch_c)) = __float2bfloat16_rn(dg * (LN2 * (gi - gprev)));
+        const float gi = sm.gs[sw64(ii, c)];
+        *reinterpret_cast<bf16*>(sm.h0 + tile_off(ii, c)) = __float2bfloat16_rn(dg * (LN2 * (gi - gprev)));
         gprev = gi;
       }
     }
@@ -770,8 +749,8 @@ int launch_rwkv7_chunked_bwd(const void* r, const void* w, const void* k, const 
       const int smem = (int)sizeof(BScanSmem<S>) + 1024;                                                          \
       if (cuda_ok(cudaFuncSetAttribute(r7c_bwd_scan_kernel<S, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem))) \
         return RWKVB200_E_CUDA;                                                                                   \
-      r7c_bwd_scan_kernel<S, P><<<B * H, 256, smem, st>>>(tmap_do, ws.tiles, ws.aux, ALL_TILES, d_ht, d_h0, sv,  \
-                                                           H, NT, status);                                     \
+      r7c_bwd_scan_kernel<S, P><<<B * H, 256, smem, st>>>(tmap_do, ws.tiles, ws.aux, ws.fin, ALL_TILES, d_ht, d_h0, \
+                                                          sv, H, NT, status);                                     \
     } while (0)
     if (B * H > sms) { if (seq_start) R7C_LAUNCH_BSCAN(2, true); else R7C_LAUNCH_BSCAN(2, false); }
     else             { if (seq_start) R7C_LAUNCH_BSCAN(4, true); else R7C_LAUNCH_BSCAN(4, false); }

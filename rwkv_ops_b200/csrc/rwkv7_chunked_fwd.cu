@@ -607,7 +607,8 @@ static_assert(sizeof(ScanSmem<2>) <= 115712, "two CTAs per SM");
 template <int STAGES, bool PACKED>
 __global__ void __launch_bounds__(256, STAGES == 2 ? 2 : 1)
 r7c_scan_fwd_kernel(const unsigned char* __restrict__ ws_tiles, const float* __restrict__ ws_aux, int tiles_per_chunk,
-                    unsigned char* __restrict__ bwd_tiles, const float* __restrict__ h0, int n_state, const __grid_constant__ CUtensorMap tmap_o,
+                    unsigned char* __restrict__ bwd_tiles, unsigned char* __restrict__ fin_tiles,
+                    const float* __restrict__ h0, int n_state, const __grid_constant__ CUtensorMap tmap_o,
                     int write_o, float* __restrict__ ht, bf16* __restrict__ o_rows, SeqView sv, int H, int NT_slots,
                     TokLayout lay, int* status) {
   extern __shared__ __align__(1024) unsigned char smem_al[];
@@ -706,17 +707,20 @@ r7c_scan_fwd_kernel(const unsigned char* __restrict__ ws_tiles, const float* __r
         if (lane == 0) mbar_arrive(&sm.bar_free[s]);
       }
     }
+    // ---- the final state: fp32 for the caller, a bf16 tile for the backward
     if (ok && ht) {
       float* S = ht + (size_t)unit * 4096;
 #pragma unroll
       for (int j = 0; j < 32; ++j) S[(c0 + j) * 64 + row] = x[j];
     }
-    if (bwd_tiles) {      // h~0 of the last chunk
+    if (bwd_tiles) {
+      if (ok) tile_store_row32(sm.ht, row, c0, x);
       fence_async_smem();
       ok = bar_sync_and(1, 128, ok);
       if (tid == 96) {
         if (ok) {
           bulk_store(bwd_tiles + ((ch0 + NT - 1) * (size_t)tiles_per_chunk + S_H0) * TILE_BYTES, sm.hs[(NT - 1) & 1], TILE_BYTES);
+          bulk_store(fin_tiles + (size_t)unit * TILE_BYTES, sm.ht, TILE_BYTES);
           bulk_commit();
         }
         bulk_wait_all();
@@ -838,7 +842,7 @@ int launch_rwkv7_chunked_fwd(const void* r, const void* w, const void* k, const 
       if (cuda_ok(cudaFuncSetAttribute(r7c_scan_fwd_kernel<S, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem))) \
         return RWKVB200_E_CUDA;                                                                                    \
       r7c_scan_fwd_kernel<S, P><<<B * H, 256, smem, st>>>(ws.tiles, ws.aux, tpc, keep_for_bwd ? ws.tiles : nullptr, \
-          h0, n_state, tmap_o, o ? 1 : 0, ht, (bf16*)o, sv, H, NT, lay, status);                           \
+          ws.fin, h0, n_state, tmap_o, o ? 1 : 0, ht, (bf16*)o, sv, H, NT, lay, status);                           \
     } while (0)
     if (B * H > sms) { if (seq_start) R7C_LAUNCH_SCAN(2, true); else R7C_LAUNCH_SCAN(2, false); }
     else             { if (seq_start) R7C_LAUNCH_SCAN(4, true); else R7C_LAUNCH_SCAN(4, false); }
