@@ -17,7 +17,7 @@
 //     P   = diag(e^{glast-gref}) b~^T W^,    N  = diag(e^{glast-gref}) (k~^T v + b~^T U)     (N stays float32)
 //     Q   = q~ diag(e^{gref}) + A_qb W^,     O' = A_qk v + A_qb U
 //     h_L = diag(e^{glast}) h0 + P h0 + N,   o  = Q h0 + O'
-// i.e. ONE 128x64x64 product [Q; P] h0 per chunk, and the chain from chunk to chunk is one product, its read-out and
+// i.e. ONE 128x64x64 product [P; Q] h0 per chunk, and the chain from chunk to chunk is one product, its read-out and
 // a barrier.  Before, the scan formed sa first and then h_L from it: five 64^3 products in two dependent groups
 // and eight operand tiles per chunk (2.3 us per chunk with one sequence per SM; 0.264 ms for 64 chunks of 256
 // sequences).
@@ -53,18 +53,17 @@ namespace r7c {
 
 constexpr int L = 64;                 // chunk length
 // tiles of one chunk in the workspace, in this order
-// (tiles that are adjacent in the shared memory of a kernel are adjacent here, so that one copy moves them)
-enum Slot { // what the two scans read: Q, P, N (float32, two slots), O' -- one copy of 40 KB
-            S_Q = 0, S_P, S_N, S_O = S_N + 2, FWD_TILES,
+enum Slot { // what the two scans read: P, Q, N (float32, two slots), O' -- one copy of 40 KB
+            S_P = 0, S_Q, S_N, S_O = S_N + 2, FWD_TILES,
             // kept for the backward by the intra kernel
-            S_G = FWD_TILES, S_B2, S_W, S_U, S_QT, S_AT, S_KT, S_BT, S_AQK, S_AAK,
+            S_QT = FWD_TILES, S_KT, S_BT, S_AT, S_AQK, S_AAK, S_G, S_B2, S_W, S_U,
             // h~0, written by the forward scan; dh^, written by the backward scan
             S_H0, S_DHH, ALL_TILES };
 // per chunk: e^{gref}[64], e^{glast-gref}[64] (intra kernel), dglast[64] (backward scan)
 constexpr int AUX_FLOATS = 192;
-// Index of (row, channel) in a 64 x 64 float32 array whose 16-byte pieces are permuted by the row, so that threads that
-// own a row and threads that own a channel both access it without bank conflicts (N is stored like this as well).
-__device__ __forceinline__ int sw64(int row, int c) { return row * 64 + ((((c >> 2) ^ (row & 7)) << 2) | (c & 3)); }
+// N: 64 x 64 float32, row k of 256 bytes, its 16-byte pieces permuted by the row so that threads that own a row
+// access it without bank conflicts
+__device__ __forceinline__ uint32_t n_piece_off(int row, int piece) { return row * 256 + ((piece ^ (row & 7)) << 4); }
 
 inline int num_chunks(int T) { return (T + L - 1) / L; }
 

@@ -23,7 +23,7 @@ typedef __nv_bfloat16 bf16;
 // one of two accumulators.  The chain is: dh (fp32, registers) -> bf16 tile -> P^T dh -> read-out -> dh.
 // STAGES as in the forward scan: 2 with two CTAs per SM, 4 with one.
 struct BScanStage {
-  unsigned char q[TILE_BYTES], p[TILE_BYTES];     // adjacent workspace slots: one bulk copy
+  unsigned char p[TILE_BYTES], q[TILE_BYTES];     // adjacent workspace slots: one bulk copy
   unsigned char dout[TILE_BYTES];
   unsigned char hn[TILE_BYTES];                   // h~0 of the next chunk, or the final state
 };
@@ -74,7 +74,7 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
     uint64_t* bar = &sm.bar_ld[n % STAGES];
     const unsigned char* tiles = ws_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES;
     mbar_expect_tx(bar, sizeof(BScanStage));
-    bulk_load(g.q, tiles + S_Q * TILE_BYTES, 2 * TILE_BYTES, bar);
+    bulk_load(g.p, tiles + S_P * TILE_BYTES, 2 * TILE_BYTES, bar);
     tma_load_4d(g.dout, &tmap_do, bar, 0, tb + c * L, hi, brow);
     bulk_load(g.hn, n == 0 ? fin_tiles + (size_t)unit * TILE_BYTES
                            : tiles + ((size_t)tiles_per_chunk + S_H0) * TILE_BYTES, TILE_BYTES, bar);
@@ -211,6 +211,10 @@ struct FinalSmem {
 // two CTAs per SM: 228 KB shared by both, 1 KB of each reserved by the system
 static_assert(sizeof(FinalSmem) <= 115712, "two CTAs per SM");
 
+// index of (row, channel) in a 64 x 64 fp32 array whose 16-byte pieces are permuted by the row, so that threads that
+// own a row and threads that own a channel both access it without bank conflicts
+__device__ __forceinline__ int sw64(int row, int c) { return row * 64 + ((((c >> 2) ^ (row & 7)) << 2) | (c & 3)); }
+
 // 256 threads: warp w reads TMEM lanes 32*(w&3).. (its row), and the two warps that share a lane
 // window split the columns (hsel = w>>2), so every elementwise phase is spread over 8 warps.
 template <bool PACKED, bool FUSED>
@@ -292,8 +296,8 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     if (lane == 0) {
       tma_prefetch_4d(&tmap_do, 0, sv.first<PACKED>(p.bi) + t0, p.hi, sv.row<PACKED>(p.bi));
       tma_prefetch_4d(&tmap_v, 0, sv.first<PACKED>(p.bi) + t0, p.hi, sv.row<PACKED>(p.bi));
-      // everything from G to dh^ (the slots are adjacent and all of them are read)
-      bulk_prefetch_l2(tiles + S_G * TILE_BYTES, (S_DHH + 1 - S_G) * TILE_BYTES);
+      // everything from q~ to dh^ (the slots are adjacent and all of them are read)
+      bulk_prefetch_l2(tiles + S_QT * TILE_BYTES, (S_DHH + 1 - S_QT) * TILE_BYTES);
     }
   };
   auto load_w = [&](const ChunkPos& p, uint4 (&rw)[2]) {   // all threads: 2 x 8 channels of the chunk's w rows

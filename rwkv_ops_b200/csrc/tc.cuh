@@ -212,17 +212,15 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
 // majors.  A 128-row K-major operand is two tiles adjacent in shared memory; a 128-wide MN-major operand
 // is two tiles `a_lbo` / `b_lbo` bytes apart; an MN-major operand with KSTEPS = 8 continues into the
 // tile that follows it (contraction rows 64..127).
-// K0: the first of the KSTEPS steps, for products whose operands are zero outside a range of the contraction index.
-template <int M, int N, int A_MN, int B_MN, int KSTEPS = 4, int K0 = 0>
+template <int M, int N, int A_MN, int B_MN, int KSTEPS = 4>
 __device__ __forceinline__ void umma_tile(uint32_t tmem_d, uint32_t a_addr, uint32_t b_addr, bool accumulate,
                                           uint32_t a_lbo = TILE_BYTES, uint32_t b_lbo = TILE_BYTES) {
-  static_assert(K0 + KSTEPS <= 4 || (A_MN && B_MN), "a K-major operand holds 64 contraction elements");
+  static_assert(KSTEPS == 4 || (A_MN && B_MN), "a K-major operand holds 64 contraction elements");
   constexpr uint32_t id = idesc_bf16(M, N, A_MN, B_MN);
   // lower descriptor words of step 0; a K=16 step advances the start address by 32 B (K-major) or 2048 B
   // (MN-major), i.e. the word by 2 or 128 (no carry out of the 14-bit field: shared addresses stay below 256 KB)
+  const uint32_t a0 = umma_desc_lo(a_addr, A_MN ? a_lbo : 16u), b0 = umma_desc_lo(b_addr, B_MN ? b_lbo : 16u);
   constexpr uint32_t a_step = A_MN ? 128u : 2u, b_step = B_MN ? 128u : 2u;
-  const uint32_t a0 = umma_desc_lo(a_addr, A_MN ? a_lbo : 16u) + a_step * K0;
-  const uint32_t b0 = umma_desc_lo(b_addr, B_MN ? b_lbo : 16u) + b_step * K0;
   if (accumulate) umma_lo<true>(tmem_d, a0, b0, id); else umma_lo<false>(tmem_d, a0, b0, id);
 #pragma unroll
   for (int ks = 1; ks < KSTEPS; ++ks) umma_lo<true>(tmem_d, a0 + a_step * ks, b0 + b_step * ks, id);
@@ -286,24 +284,6 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
-// Two float32 operations in one instruction (the same roundings as two single ones).
-__device__ __forceinline__ void mul2(float& o0, float& o1, float a0, float a1, float b0, float b1) {
-  asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
-      "mul.rn.f32x2 c, a, b;\n\tmov.b64 {%0, %1}, c;\n\t}"
-      : "=f"(o0), "=f"(o1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
-}
-__device__ __forceinline__ void fma2(float& o0, float& o1, float a0, float a1, float b0, float b1, float c0, float c1) {
-  asm("{\n\t.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
-      "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
-      : "=f"(o0), "=f"(o1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1), "f"(c0), "f"(c1));
-}
-
-// 1 / x to within an ulp or so, in one instruction
-__device__ __forceinline__ float rcp(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 // ---------------------------------------------------------------------------------------------
 // small helpers for moving rows between registers and swizzled tiles
 // ---------------------------------------------------------------------------------------------
