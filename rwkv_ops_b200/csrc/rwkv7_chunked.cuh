@@ -6,31 +6,21 @@
 //   glast = gi at token 63.
 //   q~ = q e^{gi-gref}   k~ = k e^{gref-gi}   a~ = a e^{ge-gref}   b~ = b e^{gref-gi}
 //   A_qk = tril(q~ k~^T)  A_qb = tril(q~ b~^T)  A_ak = stril(a~ k~^T)  A_ab = stril(a~ b~^T)
-//   Ainv = (I - A_ab)^-1,  W = Ainv a~,  U = Ainv A_ak v
+//   Ainv = (I - A_ab)^-1,  W = Ainv a~,  U = Ainv A_ak v,  O1 = A_qk v
 //   with h~0 = diag(e^{gref}) h0:
 //     sa  = W h~0 + U                       (rows a_i^T h_{i-1})
-//     o   = q~ h~0 + A_qk v + A_qb sa
+//     o   = q~ h~0 + O1 + A_qb sa
 //     h_L = diag(e^{glast-gref}) (h~0 + k~^T v + b~^T sa)
-// Everything but the state itself is known before the scan, so the scan gets one matrix per chunk for the state
-// and one for the output (all exponents of what follows are <= 0: nothing can overflow):
-//     W^  = W diag(e^{gref})
-//     P   = diag(e^{glast-gref}) b~^T W^,    N  = diag(e^{glast-gref}) (k~^T v + b~^T U)     (N stays float32)
-//     Q   = q~ diag(e^{gref}) + A_qb W^,     O' = A_qk v + A_qb U
-//     h_L = diag(e^{glast}) h0 + P h0 + N,   o  = Q h0 + O'
-// i.e. ONE 128x64x64 product [P; Q] h0 per chunk, and the chain from chunk to chunk is one product, its read-out and
-// a barrier.  Before, the scan formed sa first and then h_L from it: five 64^3 products in two dependent groups
-// and eight operand tiles per chunk (2.3 us per chunk with one sequence per SM; 0.264 ms for 64 chunks of 256
-// sequences).
 // Backward (do = grad of o, dh_L = grad of the state after the chunk, gref held constant: the result
 // does not depend on it):
-//     dh0  = diag(e^{glast}) dh_L + P^T dh_L + Q^T do            (the scan: the transposes of the same two matrices)
 //     dh^  = diag(e^{glast-gref}) dh_L
-//     dz   = Ainv^T (A_qb^T do + b~ dh^)  = G^T do + B2 dh^      (G = A_qb Ainv, B2 = Ainv^T b~;  z = a~ h~0 + A_ak v,  sa = Ainv z)
+//     dz   = Ainv^T (A_qb^T do + b~ dh^)  = P2 + B2 dh^          (z = a~ h~0 + A_ak v,  sa = Ainv z)
+//     dh~0 = q~^T do + a~^T dz + dh^,   dh0 = diag(e^{gref}) dh~0
 //     dv   = A_qk^T do + A_ak^T dz + k~ dh^
 //     dA_qk = tril(do v^T)  dA_qb = tril(do sa^T)  dA_ak = stril(dz v^T)  dA_ab = stril(dz sa^T)
 //     dq~ = do h~0^T + dA_qk k~ + dA_qb b~        da~ = dz h~0^T + dA_ak k~ + dA_ab b~
 //     dk~ = dA_qk^T q~ + dA_ak^T a~ + v dh^^T     db~ = dA_qb^T q~ + dA_ab^T a~ + sa dh^^T
-//     dq = dq~ e^{gi-gref} ...;  dgi = dq~ q~ - dk~ k~ - db~ b~;  dge = da~ a~;  dglast = sum_v dh_L h_L
+//     dq = dq~ e^{gi-gref} ...;  dgi = dq~ q~ - dk~ k~ - db~ b~;  dge = da~ a~;  dglast = sum_v dh^ X
 //     dg_j = sum_{i>=j} (dgi_i + dge_i) - dge_j + dglast;   dw = dg g
 // (reference: chunk_o_bwd.py:111-113,246-277,364-381, chunk_h_bwd.py:141-157, wy_fast_bwd.py:99-193,
 // chunk_A_bwd.py:146-250,318-320 under rwkv_ops/rwkv7_kernel/triton_kernel/).
@@ -39,10 +29,10 @@
 // rewritten around one reference point per chunk so that all four A matrices come out of a single
 // 128x128x64 tensor-core product of pre-scaled bf16 operands.
 //
-// Two kernels per direction: an "intra" / "final" kernel, parallel over (batch, head, chunk), for everything that
-// does not depend on the neighbouring chunks, and a "scan" kernel, one CTA per (batch, head), that walks the
-// chunks in order with the fp32 state (or its gradient) in registers.  Tiles travel between them through the
-// caller's workspace as raw 8 KB images of the swizzled shared-memory layout (tc.cuh), moved by bulk copies.
+// Two kernels per direction: an "intra" kernel, parallel over (batch, head, chunk), that produces the
+// state-independent tiles, and a "scan" kernel, one CTA per (batch, head), that walks the chunks in
+// order with the fp32 state resident in TMEM.  Tiles travel between them through the caller's
+// workspace as raw 8 KB images of the swizzled shared-memory layout (tc.cuh), moved by bulk copies.
 #pragma once
 
 #include "common.cuh"
@@ -52,18 +42,15 @@ namespace rwkvb200 {
 namespace r7c {
 
 constexpr int L = 64;                 // chunk length
-// tiles of one chunk in the workspace, in this order
-enum Slot { // what the two scans read: P, Q, N (float32, two slots), O' -- one copy of 40 KB
-            S_P = 0, S_Q, S_N, S_O = S_N + 2, FWD_TILES,
-            // kept for the backward by the intra kernel
-            S_QT = FWD_TILES, S_KT, S_BT, S_AT, S_AQK, S_AAK, S_G, S_B2, S_W, S_U,
-            // h~0, written by the forward scan; dh^, written by the backward scan
-            S_H0, S_DHH, ALL_TILES };
-// per chunk: e^{gref}[64], e^{glast-gref}[64] (intra kernel), dglast[64] (backward scan)
-constexpr int AUX_FLOATS = 192;
-// N: 64 x 64 float32, row k of 256 bytes, its 16-byte pieces permuted by the row so that threads that own a row
-// access it without bank conflicts
-__device__ __forceinline__ uint32_t n_piece_off(int row, int piece) { return row * 256 + ((piece ^ (row & 7)) << 4); }
+// tiles of one chunk in the workspace, in this order (the first FWD_TILES feed the forward scan)
+enum Slot { S_QT = 0, S_KT, S_BT, S_AQB, S_O1, S_W, S_U, FWD_TILES,
+            // kept for the backward: a~, A_qk, A_ak, Ainv (intra kernel); sa, h~0 and
+            // X = h~0 + k~^T v + b~^T sa (forward scan)
+            S_AT = FWD_TILES, S_AQK, S_AAK, S_AINV, S_SA, S_H0, S_X,
+            // backward intermediates: B2 = Ainv^T b~, P2 = Ainv^T A_qb^T do (adjacent), then
+            // dz = Ainv^T dsa and dh^ = e^{glast-gref} dh_L written by the reverse scan
+            S_B2, S_P2, S_DZ, S_DHH, ALL_TILES };
+constexpr int AUX_FLOATS = 128;       // per chunk: e^{gref}[64], e^{glast-gref}[64]
 
 inline int num_chunks(int T) { return (T + L - 1) / L; }
 
@@ -136,9 +123,8 @@ __device__ __noinline__ void store_tile_rows(__nv_bfloat16* dst, long long st, c
 
 struct Workspace {
   unsigned char* tiles;   // [n_chunks_total][tiles_per_chunk][8192]
-  float* aux;             // [n_chunks_total][AUX_FLOATS]
+  float* aux;             // [n_chunks_total][128]
   int* flags;             // [B*H] nonzero: the unit's decay left the range of the scaled operands (DECAY_LIMIT)
-  unsigned char* fin;     // [B*H][8192] final state as bf16 tiles (kept for the backward)
   int tiles_per_chunk;
 };
 
@@ -161,7 +147,7 @@ inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 inline size_t fwd_workspace_bytes(int B, int T, int H, int tiles_per_chunk) {
   const size_t n = (size_t)B * H * num_chunks(T);
   return align256(n * tiles_per_chunk * tc::TILE_BYTES) + align256(n * AUX_FLOATS * sizeof(float)) +
-         align256((size_t)B * H * sizeof(int)) + (tiles_per_chunk == ALL_TILES ? (size_t)B * H * tc::TILE_BYTES : 0) + 1024;
+         align256((size_t)B * H * sizeof(int)) + 1024;
 }
 
 inline Workspace carve(void* ws, int B, int T, int H, int tiles_per_chunk) {
@@ -171,8 +157,6 @@ inline Workspace carve(void* ws, int B, int T, int H, int tiles_per_chunk) {
   w.tiles = reinterpret_cast<unsigned char*>(p);
   w.aux = reinterpret_cast<float*>(p + align256(n * tiles_per_chunk * tc::TILE_BYTES));
   w.flags = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(w.aux) + align256(n * AUX_FLOATS * sizeof(float)));
-  w.fin = tiles_per_chunk == ALL_TILES
-              ? reinterpret_cast<unsigned char*>(w.flags) + align256((size_t)B * H * sizeof(int)) : nullptr;
   w.tiles_per_chunk = tiles_per_chunk;
   return w;
 }
@@ -183,7 +167,7 @@ inline Workspace carve(void* ws, int B, int T, int H, int tiles_per_chunk) {
 // a sequence over several GPUs runs the state-independent phase on every GPU at once and only the scans one GPU
 // after the other (the workspace carries everything from one phase to the next).
 //   forward:  PREPARE = intra-chunk kernel;            SCAN = state scan over the chunks (+ exact fallback)
-//   backward: PREPARE = forward recomputation, where the forward kept nothing;
+//   backward: PREPARE = (forward recomputation and) the state-independent products of the reverse scan;
 //             SCAN = reverse scan (gradient of the state);   FINISH = token gradients (+ exact fallback)
 enum Phase { PHASE_PREPARE = 1, PHASE_SCAN = 2, PHASE_FINISH = 4, PHASE_ALL = 7 };
 

@@ -1,10 +1,11 @@
 // Chunked RWKV7 backward on tcgen05 (bf16 token tensors).  Equations in rwkv7_chunked.cuh.
 //
 // Launch sequence (all on the caller's stream, tiles exchanged through the workspace):
-//   1. forward intra kernel with keep_for_bwd (P, Q and the tiles the final kernel reads), forward scan (h~0)
-//   2. r7c_bwd_scan_kernel   (one CTA per (b,h), chunks in reverse)  dh^ and dglast per chunk, d initial state
-//   3. r7c_bwd_final_kernel  (parallel over chunks)   dq, dk, dv, da, db, dw
-// (1. only where the forward call has not left its tiles)
+//   1. forward intra kernel with keep_for_bwd (q~, k~, b~, a~, A_qk, A_ak, A_qb, Ainv, W, U, decay factors)
+//   2. forward scan without output, keeping sa, h~0 and X of every chunk
+//   3. r7c_bwd_pre_kernel    (parallel over chunks)   B2 = Ainv^T b~,  P2 = Ainv^T A_qb^T do
+//   4. r7c_bwd_scan_kernel   (one CTA per (b,h), chunks in reverse)  dz, dh^ per chunk, d initial state
+//   5. r7c_bwd_final_kernel  (parallel over chunks)   dq, dk, dv, da, db, dw
 #include "rwkv7_chunked.cuh"
 
 namespace rwkvb200 {
@@ -16,50 +17,33 @@ typedef __nv_bfloat16 bf16;
 // decay sums are kept in units of log 2 (tc::ex2), as in the forward kernels; nothing is clamped
 
 // ---------------------------------------------------------------------------------------------
-// 2. reverse scan: grid = B*H, 256 threads: dh <- e^{glast} dh + P^T dh + Q^T do
+// 3. B2 = Ainv^T b~ and P2 = Ainv^T (A_qb^T do): persistent CTAs of 128 threads over the chunk-heads
 // ---------------------------------------------------------------------------------------------
-// Both products of a chunk add up in one M = 64 accumulator (row k on the lower lane halves; the two warps of a lane
-// window take 32 columns each).  Q^T do does not wait for the chain: it is issued a chunk ahead, into the other
-// one of two accumulators.  The chain is: dh (fp32, registers) -> bf16 tile -> P^T dh -> read-out -> dh.
-// STAGES as in the forward scan: 2 with two CTAs per SM, 4 with one.
-struct BScanStage {
-  unsigned char p[TILE_BYTES], q[TILE_BYTES];     // adjacent workspace slots: one bulk copy
-  unsigned char dout[TILE_BYTES];
-  unsigned char hn[TILE_BYTES];                   // h~0 of the next chunk, or the final state
+struct PreStage {
+  unsigned char ainv[TILE_BYTES], bt[TILE_BYTES], aqb[TILE_BYTES], dout[TILE_BYTES];
 };
-template <int STAGES>
-struct BScanSmem {
-  BScanStage st[STAGES];
-  unsigned char dh[TILE_BYTES];       // dh as bf16, [k][v]
-  unsigned char dhh[2][TILE_BYTES];   // dh^ as bf16 (kept for the final kernel)
-  float part[2][2][64];               // dglast of a chunk, by column half
-  uint64_t bar_ld[STAGES], bar_m[2];
+struct PreSmem {
+  PreStage st[2];             // the operand tiles of this chunk-head and of the next one
+  unsigned char p1[TILE_BYTES], b2[TILE_BYTES], p2[TILE_BYTES];
+  uint64_t bar_ld[2], bar_m1, bar_m2;
   uint32_t tmem_base;
 };
-static_assert(sizeof(BScanSmem<2>) + 1024 <= 115712, "two CTAs per SM");
 
-template <int STAGES, bool PACKED>
-__global__ void __launch_bounds__(256, STAGES == 2 ? 2 : 1)
-r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* __restrict__ ws_tiles,
-                    float* __restrict__ ws_aux, const unsigned char* __restrict__ fin_tiles, int tiles_per_chunk,
-                    const float* __restrict__ d_ht, float* __restrict__ d_h0, SeqView sv, int H, int NT_slots,
-                    int* status) {
+// Two CTAs per SM walk over chunk-heads ch = blockIdx.x, blockIdx.x + gridDim.x, ...; the four operand tiles
+// of the next chunk-head are requested before the current one is worked on, so that loads, the two dependent
+// MMAs and the copies of the results overlap.
+template <bool PACKED>
+__global__ void __launch_bounds__(128)
+r7c_bwd_pre_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* __restrict__ ws_tiles,
+                   int tiles_per_chunk, SeqView sv, int H, int NT, int n_ch, int* status) {
   extern __shared__ unsigned char smem_raw[];
-  BScanSmem<STAGES>& sm =
-      *reinterpret_cast<BScanSmem<STAGES>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  PreSmem& sm = *reinterpret_cast<PreSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int unit = blockIdx.x, bi = unit / H, hi = unit % H;
-  const size_t ch0 = (size_t)unit * NT_slots;
-  const int NT = (sv.length<PACKED>(bi) + L - 1) / L;      // chunks of this sequence
-  const int tb = sv.first<PACKED>(bi), brow = sv.row<PACKED>(bi);
-  const int wq = warp & 3, hsel = warp >> 2, c0 = 32 * hsel;
-  const int row = 16 * wq + (lane & 15);
-  const bool state_lane = lane < 16;
-  const bool st_thread = tid == 32, ld_thread = tid == 64;
+  const int row = 16 * warp + (lane & 15);
+  const bool lo = lane < 16;
 
   if (tid == 0) {
-    for (int s = 0; s < STAGES; ++s) mbar_init(&sm.bar_ld[s], 1);
-    mbar_init(&sm.bar_m[0], 1); mbar_init(&sm.bar_m[1], 1);
+    mbar_init(&sm.bar_ld[0], 1); mbar_init(&sm.bar_ld[1], 1); mbar_init(&sm.bar_m1, 1); mbar_init(&sm.bar_m2, 1);
     fence_mbar_init();
   }
   if (warp == 0) tmem_alloc(&sm.tmem_base, 128);
@@ -68,22 +52,165 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
   tc_fence_after();
   const uint32_t tm = sm.tmem_base;
 
-  auto issue_load = [&](int n) {     // n-th chunk in reverse order
-    const int c = NT - 1 - n;
-    BScanStage& g = sm.st[n % STAGES];
-    uint64_t* bar = &sm.bar_ld[n % STAGES];
-    const unsigned char* tiles = ws_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES;
-    mbar_expect_tx(bar, sizeof(BScanStage));
-    bulk_load(g.p, tiles + S_P * TILE_BYTES, 2 * TILE_BYTES, bar);
-    tma_load_4d(g.dout, &tmap_do, bar, 0, tb + c * L, hi, brow);
-    bulk_load(g.hn, n == 0 ? fin_tiles + (size_t)unit * TILE_BYTES
-                           : tiles + ((size_t)tiles_per_chunk + S_H0) * TILE_BYTES, TILE_BYTES, bar);
+  auto empty = [&](const ChunkPos& p) {
+    if constexpr (!PACKED) return false;
+    return p.c * L >= sv.length<PACKED>(p.bi);      // a chunk slot past the end of a packed sequence
   };
-  if (ld_thread)
-    for (int n = 0; n < STAGES && n < NT; ++n) issue_load(n);
+  auto advance = [&](ChunkPos p) {
+    do { chunk_step(p, gridDim.x, NT, H); } while (p.ch < n_ch && empty(p));
+    return p;
+  };
+  auto issue_loads = [&](const ChunkPos& p, int s) {      // tid 0
+    const unsigned char* tiles = ws_tiles + (size_t)p.ch * tiles_per_chunk * TILE_BYTES;
+    PreStage& g = sm.st[s];
+    mbar_expect_tx(&sm.bar_ld[s], 4 * TILE_BYTES);
+    bulk_load(g.ainv, tiles + S_AINV * TILE_BYTES, TILE_BYTES, &sm.bar_ld[s]);
+    bulk_load(g.bt, tiles + S_BT * TILE_BYTES, TILE_BYTES, &sm.bar_ld[s]);
+    bulk_load(g.aqb, tiles + S_AQB * TILE_BYTES, TILE_BYTES, &sm.bar_ld[s]);
+    tma_load_4d(g.dout, &tmap_do, &sm.bar_ld[s], 0, sv.first<PACKED>(p.bi) + p.c * L, p.hi, sv.row<PACKED>(p.bi));
+  };
+  ChunkPos cur = chunk_pos(blockIdx.x, NT, H);
+  if (cur.ch < n_ch && empty(cur)) cur = advance(cur);
+  if (cur.ch < n_ch && tid == 0) issue_loads(cur, 0);
 
-  // gradient of the state after the current chunk, row k of dh[k][v] = d_ht[v][k], columns c0 .. c0 + 31
-  float dh[32];
+  bool ok = true;
+  int it = 0;
+  for (ChunkPos nxt; cur.ch < n_ch && ok; cur = nxt, ++it) {
+    const int s = it & 1;
+    const uint32_t par = it & 1;
+    PreStage& g = sm.st[s];
+    unsigned char* tiles = ws_tiles + (size_t)cur.ch * tiles_per_chunk * TILE_BYTES;
+    nxt = advance(cur);
+    // the other stage was last read by the MMAs of the previous chunk-head, which have completed
+    if (tid == 0 && nxt.ch < n_ch) issue_loads(nxt, s ^ 1);
+    ok = mbar_wait(&sm.bar_ld[s], (it >> 1) & 1, status, 301);
+    if (tid == 0 && ok) {
+      bulk_wait_read();      // the copies of the previous B2 / P2 have left their tiles, which are rewritten below
+      tc_fence_after();
+      umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 0), smem_u32(g.aqb), smem_u32(g.dout), false);   // A_qb^T do
+      umma_tile<64, 64, 1, 1>(tmem_addr(tm, 16, 0), smem_u32(g.ainv), smem_u32(g.bt), false);   // Ainv^T b~
+      umma_commit(&sm.bar_m1);
+    }
+    ok = mbar_wait(&sm.bar_m1, par, status, 302) && ok;
+    tc_fence_after();
+    if (ok) {
+#pragma unroll
+      for (int part = 0; part < 2; ++part) {
+        uint32_t r[32];
+        tmem_ld32(tmem_addr(tm, 32 * warp, 32 * part), r);
+        tmem_ld_wait();
+        float x[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(r[j]);
+        tile_store_row32(lo ? sm.p1 : sm.b2, row, 32 * part, x);
+      }
+    }
+    fence_async_smem();
+    tc_fence_before();
+    ok = __syncthreads_and(ok);
+    if (tid == 0 && ok) {
+      tc_fence_after();
+      umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 64), smem_u32(g.ainv), smem_u32(sm.p1), false);   // Ainv^T P1
+      umma_commit(&sm.bar_m2);
+      bulk_store(tiles + S_B2 * TILE_BYTES, sm.b2, TILE_BYTES);
+      bulk_commit();
+    }
+    ok = mbar_wait(&sm.bar_m2, par, status, 303) && ok;
+    tc_fence_after();
+    if (ok) {
+#pragma unroll
+      for (int part = 0; part < 2; ++part) {
+        uint32_t r[32];
+        tmem_ld32(tmem_addr(tm, 32 * warp, 64 + 32 * part), r);
+        tmem_ld_wait();
+        if (lo) {
+          float x[32];
+#pragma unroll
+          for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(r[j]);
+          tile_store_row32(sm.p2, row, 32 * part, x);
+        }
+      }
+    }
+    fence_async_smem();
+    tc_fence_before();
+    ok = __syncthreads_and(ok);
+    if (tid == 0 && ok) {
+      bulk_store(tiles + S_P2 * TILE_BYTES, sm.p2, TILE_BYTES);
+      bulk_commit();
+    }
+  }
+  if (tid == 0) bulk_wait_all();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tm, 128);
+}
+
+// ---------------------------------------------------------------------------------------------
+// 4. reverse scan: grid = B*H, 256 threads (the two warps of a TMEM lane window take 32 columns each)
+// ---------------------------------------------------------------------------------------------
+struct BScanStage {
+  unsigned char b2[TILE_BYTES], p2[TILE_BYTES];   // adjacent workspace slots: one bulk copy
+  unsigned char at[TILE_BYTES], qt[TILE_BYTES], dout[TILE_BYTES];
+};
+struct BScanSmem {
+  BScanStage st[2];
+  unsigned char dhh[TILE_BYTES];    // dh^ as bf16, [k][v]
+  unsigned char dz[TILE_BYTES];     // dz as bf16, [token][v]
+  uint64_t bar_full[2], bar_m1, bar_m2;
+  uint32_t tmem_base;
+};
+
+template <bool PACKED>
+__global__ void __launch_bounds__(256, 2)
+r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* __restrict__ ws_tiles,
+                    const float* __restrict__ ws_aux, int tiles_per_chunk, const float* __restrict__ d_ht,
+                    float* __restrict__ d_h0, SeqView sv, int H, int NT_slots, int spread, int* status) {
+  extern __shared__ unsigned char smem_raw[];
+  BScanSmem& sm = *reinterpret_cast<BScanSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int unit = blockIdx.x, bi = unit / H, hi = unit % H;
+  const size_t ch0 = (size_t)unit * NT_slots;
+  const int NT = (sv.length<PACKED>(bi) + L - 1) / L;      // chunks of this sequence
+  const int tb = sv.first<PACKED>(bi), brow = sv.row<PACKED>(bi);
+  const int wq = warp & 3, hsel = warp >> 2, c0 = 32 * hsel;
+  const int row = 16 * wq + (lane & 15);
+  const bool state_lane = lane < 16;
+  // single-thread jobs side by side: thread 0 issues the MMAs (thread 96 one product of the first group, when
+  // the CTA has the SM to itself), st_thread copies dh^ and dz out (and waits for
+  // its own bulk-copy groups), ld_thread requests the operand tiles of the chunk after the next
+  // (they share the SM with a second CTA when there are more sequences than SMs, and then stay with thread 0)
+  const bool st_thread = tid == (spread ? 32 : 0), ld_thread = tid == (spread ? 64 : 0);
+
+  if (tid == 0) {
+    mbar_init(&sm.bar_full[0], 1); mbar_init(&sm.bar_full[1], 1);
+    // with one CTA per SM the two products of the first MMA group have an issuing thread each
+    mbar_init(&sm.bar_m1, spread ? 2 : 1); mbar_init(&sm.bar_m2, 1);
+    fence_mbar_init();
+  }
+  if (warp == 0) tmem_alloc(&sm.tmem_base, 64);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tm = sm.tmem_base;
+  const uint32_t tm_w = tmem_addr(tm, 32 * wq, c0);
+
+  auto issue_loads = [&](int n) {     // n-th chunk in reverse order
+    const int c = NT - 1 - n;
+    BScanStage& s = sm.st[n & 1];
+    unsigned char* tiles = ws_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES;
+    mbar_expect_tx(&sm.bar_full[n & 1], 5 * TILE_BYTES);
+    bulk_load(s.b2, tiles + S_B2 * TILE_BYTES, 2 * TILE_BYTES, &sm.bar_full[n & 1]);
+    bulk_load(s.at, tiles + S_AT * TILE_BYTES, TILE_BYTES, &sm.bar_full[n & 1]);
+    bulk_load(s.qt, tiles + S_QT * TILE_BYTES, TILE_BYTES, &sm.bar_full[n & 1]);
+    tma_load_4d(s.dout, &tmap_do, &sm.bar_full[n & 1], 0, tb + c * L, hi, brow);
+  };
+  if (tid == 0) {
+    issue_loads(0);
+    if (NT > 1) issue_loads(1);
+  }
+
+  // gradient of the state after the current chunk, row k of dh[k][v] = d_ht[v][k]
+  float dh[32];        // columns c0 .. c0 + 31
   if (state_lane && d_ht) {
     const float* S = d_ht + (size_t)unit * 4096;
 #pragma unroll
@@ -93,119 +220,122 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
     for (int vv = 0; vv < 32; ++vv) dh[vv] = 0.f;
   }
 
-  // the decay factors of a chunk are fetched one chunk ahead
-  float eg_next = 1.f, dl_next = 1.f, eg_after = 1.f;
+  // the two decay factors of a chunk are fetched one chunk ahead: they head the chain of a chunk
+  float dc_next = 1.f, e0_next = 1.f;
   if (state_lane) {
-    eg_next = ws_aux[(ch0 + NT - 1) * AUX_FLOATS + row];
-    dl_next = ws_aux[(ch0 + NT - 1) * AUX_FLOATS + 64 + row];
+    dc_next = ws_aux[(ch0 + NT - 1) * AUX_FLOATS + 64 + row];
+    e0_next = ws_aux[(ch0 + NT - 1) * AUX_FLOATS + row];
   }
-  bool ok = true;
-  bool ahead = false;      // thread 0: Q^T do of this chunk has been issued already
-  for (int n = 0; n < NT; ++n) {
-    const int c = NT - 1 - n, s = n % STAGES, t = n & 1;
-    const uint32_t sp = (n / STAGES) & 1, tp = (n >> 1) & 1;
+  bool ok = true;          // the same in every thread at the loop's head: the result of the last barrier
+  bool tail_ok = true;     // this thread's wait at the end of the previous chunk
+  for (int n = 0; n < NT && ok; ++n) {
+    const int c = NT - 1 - n;
+    BScanStage& s = sm.st[n & 1];
     unsigned char* tiles = ws_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES;
-    const float eg = eg_next, dl = dl_next;
+    const float dc = dc_next, e0 = e0_next;
     if (state_lane) {
-      tile_store_row32(sm.dh, row, c0, dh);
+#pragma unroll
+      for (int vv = 0; vv < 32; ++vv) dh[vv] *= dc;      // dh^ = e^{glast-gref} dh_L
+      tile_store_row32(sm.dhh, row, c0, dh);
       if (c > 0) {
-        eg_next = ws_aux[(ch0 + c - 1) * AUX_FLOATS + row];
-        dl_next = ws_aux[(ch0 + c - 1) * AUX_FLOATS + 64 + row];
+        dc_next = ws_aux[(ch0 + c - 1) * AUX_FLOATS + 64 + row];
+        e0_next = ws_aux[(ch0 + c - 1) * AUX_FLOATS + row];
       }
     }
-    if (st_thread) bulk_wait_read();    // the dh^ tile about to be rewritten has left shared memory
+    ok = tail_ok && mbar_wait(&sm.bar_full[n & 1], (n >> 1) & 1, status, 311);
+    if (st_thread) bulk_wait_read();    // the copy of the previous chunk's dz has left its tile, rewritten below
     fence_async_smem();
     tc_fence_before();
-    ok = __syncthreads_and(ok);         // the one place where the loop may be left: by all threads or none
-    if (!ok) break;
-    if (tid == 0) {
-      ok = mbar_wait(&sm.bar_ld[s], sp, status, 311);
+    ok = __syncthreads_and(ok);
+    if (tid == 0 && ok) {
       tc_fence_after();
-      if (!ahead)
-        umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 64 * t), smem_u32(sm.st[s].q), smem_u32(sm.st[s].dout), false);    // Q^T do
-      umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 64 * t), smem_u32(sm.st[s].p), smem_u32(sm.dh), true);               // + P^T dh
-      umma_commit(&sm.bar_m[t]);
-      // the other accumulator was read before the barrier above: the next chunk's Q^T do, if its tiles are there
-      ahead = false;
-      if (n + 1 < NT && mbar_try_wait(&sm.bar_ld[(n + 1) % STAGES], ((n + 1) / STAGES) & 1)) {
-        BScanStage& g = sm.st[(n + 1) % STAGES];
-        umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 64 * (t ^ 1)), smem_u32(g.q), smem_u32(g.dout), false);
-        ahead = true;
-      }
+      umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 0), smem_u32(s.b2), smem_u32(sm.dhh), false);   // B2 dh^
+      if (!spread) umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 0), smem_u32(s.qt), smem_u32(s.dout), false);    // q~^T do
+      umma_commit(&sm.bar_m1);
     }
-    // the stage of the chunk before has been read: by its products, and its h~0 by every thread before the barrier
-    if (ld_thread && n > 0 && n - 1 + STAGES < NT) issue_load(n - 1 + STAGES);
-    if (n > 0) {      // what the chunk before left: its dh^ tile and its dglast
-      if (st_thread) {
-        bulk_store(tiles + ((size_t)tiles_per_chunk + S_DHH) * TILE_BYTES, sm.dhh[t ^ 1], TILE_BYTES);
-        bulk_commit();
-      }
-      if (tid >= 192) ws_aux[(ch0 + c + 1) * AUX_FLOATS + 128 + tid - 192] = sm.part[t ^ 1][0][tid - 192] + sm.part[t ^ 1][1][tid - 192];
+    if (spread && tid == 96 && ok) {
+      tc_fence_after();
+      umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 0), smem_u32(s.qt), smem_u32(s.dout), false);    // q~^T do
+      umma_commit(&sm.bar_m1);
     }
-    // under the product: dh^ = e^{glast-gref} dh, and dglast = sum_v dh h_L with h_L = h~0 / e^{gref} of the next chunk
-    ok = ok && mbar_wait(&sm.bar_ld[s], sp, status, 314);
-    if (state_lane && ok) {
-      float y[32], h[32];
-      tile_load_row32(sm.st[s].hn, row, c0, h);
-      float acc = 0.f;
-#pragma unroll
-      for (int j = 0; j < 32; ++j) { acc += dh[j] * h[j]; y[j] = dh[j] * dl; }
-      tile_store_row32(sm.dhh[t], row, c0, y);
-      sm.part[t][hsel][row] = n == 0 ? acc : acc / eg_after;
-      eg_after = eg;
+    if (st_thread && ok) {
+      bulk_store(tiles + S_DHH * TILE_BYTES, sm.dhh, TILE_BYTES);
+      bulk_commit();
     }
-    ok = ok && mbar_wait(&sm.bar_m[t], tp, status, 312);
+    ok = ok && mbar_wait(&sm.bar_m1, n & 1, status, 312);
     tc_fence_after();
     if (ok) {
       uint32_t r[32];
-      tmem_ld32(tmem_addr(tm, 32 * wq, 64 * t + c0), r);
+      tmem_ld32(tm_w, r);
       tmem_ld_wait();
-      const float et = eg * dl;
+      if (!state_lane) {      // dz = P2 + B2 dh^
+        float x[32], p[32];
+        tile_load_row32(s.p2, row, c0, p);
 #pragma unroll
-      for (int j = 0; j < 32; ++j) dh[j] = et * dh[j] + __uint_as_float(r[j]);
+        for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(r[j]) + p[j];
+        tile_store_row32(sm.dz, row, c0, x);
+      }
     }
+    if (st_thread) bulk_wait_read();    // the copy of dh^ has left its tile, rewritten at the top of the next chunk
+    fence_async_smem();
+    tc_fence_before();
+    ok = __syncthreads_and(ok);
+    if (tid == 0 && ok) {
+      tc_fence_after();
+      umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 0), smem_u32(s.at), smem_u32(sm.dz), true);      // += a~^T dz
+      umma_commit(&sm.bar_m2);
+    }
+    if (st_thread && ok) {
+      bulk_store(tiles + S_DZ * TILE_BYTES, sm.dz, TILE_BYTES);
+      bulk_commit();
+    }
+    tail_ok = ok && mbar_wait(&sm.bar_m2, n & 1, status, 313);
+    tc_fence_after();
+    // this stage has been read: p2 by every thread before the last barrier, the rest by the two MMA groups
+    if (ld_thread && tail_ok && n + 2 < NT) issue_loads(n + 2);
+    if (tail_ok) {
+      uint32_t r[32];
+      tmem_ld32(tm_w, r);
+      tmem_ld_wait();
+      if (state_lane) {       // dh0 = e^{gref} (q~^T do + a~^T dz + dh^)
+#pragma unroll
+        for (int j = 0; j < 32; ++j) dh[j] = e0 * (__uint_as_float(r[j]) + dh[j]);
+      }
+    }
+    // no barrier here: the next one (after dh^ of the next chunk is in its tile) orders these TMEM reads
+    // before the MMAs that overwrite the accumulators
   }
-  if (state_lane && d_h0 && ok) {
+  if (state_lane && d_h0 && ok && tail_ok) {
     float* S = d_h0 + (size_t)unit * 4096;
 #pragma unroll
     for (int vv = 0; vv < 32; ++vv) S[(c0 + vv) * 64 + row] = dh[vv];
   }
-  fence_async_smem();
-  tc_fence_before();
-  ok = __syncthreads_and(ok);
-  if (ok) {      // what the last chunk left
-    const int t = (NT - 1) & 1;
-    if (st_thread) {
-      bulk_store(ws_tiles + (ch0 * tiles_per_chunk + S_DHH) * TILE_BYTES, sm.dhh[t], TILE_BYTES);
-      bulk_commit();
-    }
-    if (tid >= 192) ws_aux[ch0 * AUX_FLOATS + 128 + tid - 192] = sm.part[t][0][tid - 192] + sm.part[t][1][tid - 192];
-  }
   if (st_thread) bulk_wait_all();
-  if (warp == 0) tmem_dealloc(tm, 128);
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tm, 64);
 }
 
 // ---------------------------------------------------------------------------------------------
-// 3. all token gradients of one chunk: persistent CTAs of 256 threads over the B*H*NT chunk-heads
+// 5. all token gradients of one chunk: persistent CTAs of 256 threads over the B*H*NT chunk-heads
 // ---------------------------------------------------------------------------------------------
 // What bounds it: per chunk-head about 14 k warp instructions in phases that wait for one another (tiles ->
 // products -> read-out -> products -> read-out -> prefix sums).  With one CTA per SM (213 KB of shared memory) the
 // SM issued 1.0 instruction per cycle; two CTAs per SM fill each other's waits.  To fit two, a chunk-head lives in
 // twelve tiles whose space is used over again (names below: what is loaded, then what replaces it) and one fp32
 // array, and an accumulator that does not need the dA tiles is issued with the first MMA group, which frees its
-// operands.  TMEM: sa | dz columns 192..255, then dv there (lower lane halves); dA 0..127, [dq~; da~] 128..191;
-// [dk~; db~] 0..63 once dA has been read.
+// operands.  TMEM: dA columns 0..127, [dq~; da~] 128..191, dv 192..255 (lower lane halves); [dk~; db~] 0..63 once
+// dA has been read.
 struct FinalSmem {
-  unsigned char dout[TILE_BYTES], dz[TILE_BYTES];       // [do; dz]   (dz: W before)   then dA_qk, dA_ak   then red1 (fp32)
-  unsigned char aqk[TILE_BYTES], aak[TILE_BYTES];       // A_qk, A_ak                  then dA_qb, dA_ab   then red2 (fp32)
-  unsigned char h0[TILE_BYTES];                         // h~0                         then dv rows        then dw rows
+  unsigned char dout[TILE_BYTES], dz[TILE_BYTES];       // [do; dz]   then dA_qk, dA_ak   then red1 (fp32)
+  unsigned char aqk[TILE_BYTES], aak[TILE_BYTES];       // A_qk, A_ak then dA_qb, dA_ab   then red2 (fp32)
+  unsigned char h0[TILE_BYTES];                         // h~0        then dv rows        then dw rows
   unsigned char dhh[TILE_BYTES];                        // dh^
-  unsigned char v[TILE_BYTES], sa[TILE_BYTES];          // [v; sa]    (sa: G before)   then (sa) da~ a~ as bf16
-  unsigned char qt[TILE_BYTES], at[TILE_BYTES];         // q~, a~     (a~: B2 before)  then dq, da rows
-  unsigned char kt[TILE_BYTES], bt[TILE_BYTES];         // k~, b~     (b~: U before)   then dk, db rows
+  unsigned char v[TILE_BYTES], sa[TILE_BYTES];          // [v; sa]    (sa) then da~ a~ as bf16
+  unsigned char qt[TILE_BYTES], at[TILE_BYTES];         // q~, a~     then dq, da rows
+  unsigned char kt[TILE_BYTES], bt[TILE_BYTES];         // k~, b~     then dk, db rows
   float gs[L * 64];         // g log2(e), then (gi - gref) log2(e): inclusive prefix inside the chunk (sw64)
   float quart[3][64];       // sums over quarters of the chunk; [2] between the prefix sum and the epilogue: -gref
-  uint64_t bar_l0, bar_l1, bar_l2, bar_m0, bar_m1, bar_m2;
+  uint64_t bar_l0, bar_l1, bar_l2, bar_m1, bar_m2;
   uint32_t tmem_base;
 };
 // two CTAs per SM: 228 KB shared by both, 1 KB of each reserved by the system
@@ -221,7 +351,7 @@ template <bool PACKED, bool FUSED>
 __global__ void __launch_bounds__(256, 2)
 r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtensorMap tmap_do,
                      const __grid_constant__ CUtensorMap tmap_v, const unsigned char* __restrict__ ws_tiles,
-                     const float* __restrict__ ws_aux, int tiles_per_chunk, const __grid_constant__ CUtensorMap tmap_dq,
+                     int tiles_per_chunk, const __grid_constant__ CUtensorMap tmap_dq,
                      const __grid_constant__ CUtensorMap tmap_dw, const __grid_constant__ CUtensorMap tmap_dk,
                      const __grid_constant__ CUtensorMap tmap_dv, const __grid_constant__ CUtensorMap tmap_da,
                      const __grid_constant__ CUtensorMap tmap_db,
@@ -246,7 +376,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     // an MMA group is issued by several threads, one accumulator each, and completes with the arrival of all: one
     // thread issues an MMA about every 80 cycles, the tensor pipe takes them faster
     mbar_init(&sm.bar_l0, 1); mbar_init(&sm.bar_l1, 1); mbar_init(&sm.bar_l2, 1);
-    mbar_init(&sm.bar_m0, 2); mbar_init(&sm.bar_m1, 3); mbar_init(&sm.bar_m2, 2);
+    mbar_init(&sm.bar_m1, 3); mbar_init(&sm.bar_m2, 2);
     fence_mbar_init();
   }
   if (warp == 0) tmem_alloc(&sm.tmem_base, 256);
@@ -263,30 +393,25 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     bulk_load(sm.dhh, tiles + S_DHH * TILE_BYTES, TILE_BYTES, &sm.bar_l0);
     tma_load_4d(sm.v, &tmap_v, &sm.bar_l0, 0, sv.first<PACKED>(p.bi) + p.c * L, p.hi, sv.row<PACKED>(p.bi));
   };
-  auto load_1a = [&](const ChunkPos& p) {     // the other operands of MMA groups 0 and 1, but for those below
+  auto load_1a = [&](const ChunkPos& p) {     // the other operands of MMA group 1, but for k~ and h~0
     const unsigned char* tiles = ws_tiles + (size_t)p.ch * tiles_per_chunk * TILE_BYTES;
-    mbar_expect_tx(&sm.bar_l1, 9 * TILE_BYTES);
+    mbar_expect_tx(&sm.bar_l1, 7 * TILE_BYTES);
     tma_load_4d(sm.dout, &tmap_do, &sm.bar_l1, 0, sv.first<PACKED>(p.bi) + p.c * L, p.hi, sv.row<PACKED>(p.bi));
-    bulk_load(sm.dz, tiles + S_W * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
-    bulk_load(sm.sa, tiles + S_G * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
+    bulk_load(sm.dz, tiles + S_DZ * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
+    bulk_load(sm.sa, tiles + S_SA * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
     bulk_load(sm.aqk, tiles + S_AQK * TILE_BYTES, 2 * TILE_BYTES, &sm.bar_l1);
   };
-  auto load_1b = [&](const ChunkPos& p) {     // B2, U, k~; q~ (MMA group 2 and the epilogue)
+  auto load_2 = [&](const ChunkPos& p) {      // k~; q~, a~, b~ (MMA group 2 and the epilogue)
     const unsigned char* tiles = ws_tiles + (size_t)p.ch * tiles_per_chunk * TILE_BYTES;
-    bulk_load(sm.at, tiles + S_B2 * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
-    bulk_load(sm.bt, tiles + S_U * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
     bulk_load(sm.kt, tiles + S_KT * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
     mbar_expect_tx(&sm.bar_l2, 3 * TILE_BYTES);
     bulk_load(sm.qt, tiles + S_QT * TILE_BYTES, TILE_BYTES, &sm.bar_l2);
-  };
-  auto load_1c = [&](const ChunkPos& p) {     // h~0
-    const unsigned char* tiles = ws_tiles + (size_t)p.ch * tiles_per_chunk * TILE_BYTES;
-    bulk_load(sm.h0, tiles + S_H0 * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
-  };
-  auto load_2 = [&](const ChunkPos& p) {      // a~, b~ over B2, U
-    const unsigned char* tiles = ws_tiles + (size_t)p.ch * tiles_per_chunk * TILE_BYTES;
     bulk_load(sm.at, tiles + S_AT * TILE_BYTES, TILE_BYTES, &sm.bar_l2);
     bulk_load(sm.bt, tiles + S_BT * TILE_BYTES, TILE_BYTES, &sm.bar_l2);
+  };
+  auto load_1b = [&](const ChunkPos& p) {     // h~0
+    const unsigned char* tiles = ws_tiles + (size_t)p.ch * tiles_per_chunk * TILE_BYTES;
+    bulk_load(sm.h0, tiles + S_H0 * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
   };
   // Ask for everything a chunk-head will load to be brought into L2 (issued most of a chunk-head ahead of the
   // loads themselves, which then take an L2 round trip instead of a DRAM one).
@@ -296,8 +421,10 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     if (lane == 0) {
       tma_prefetch_4d(&tmap_do, 0, sv.first<PACKED>(p.bi) + t0, p.hi, sv.row<PACKED>(p.bi));
       tma_prefetch_4d(&tmap_v, 0, sv.first<PACKED>(p.bi) + t0, p.hi, sv.row<PACKED>(p.bi));
-      // everything from q~ to dh^ (the slots are adjacent and all of them are read)
-      bulk_prefetch_l2(tiles + S_QT * TILE_BYTES, (S_DHH + 1 - S_QT) * TILE_BYTES);
+      bulk_prefetch_l2(tiles + S_QT * TILE_BYTES, 3 * TILE_BYTES);     // q~, k~, b~
+      bulk_prefetch_l2(tiles + S_AT * TILE_BYTES, 3 * TILE_BYTES);     // a~, A_qk, A_ak
+      bulk_prefetch_l2(tiles + S_SA * TILE_BYTES, 3 * TILE_BYTES);     // sa, h~0, X
+      bulk_prefetch_l2(tiles + S_DZ * TILE_BYTES, 2 * TILE_BYTES);     // dz, dh^
     }
   };
   auto load_w = [&](const ChunkPos& p, uint4 (&rw)[2]) {   // all threads: 2 x 8 channels of the chunk's w rows
@@ -325,7 +452,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
 
   uint4 rw[2];
   if (cur.ch < n_ch) {
-    if (st_thread) { load_0(cur); load_1a(cur); load_1b(cur); load_1c(cur); }
+    if (st_thread) { load_0(cur); load_1a(cur); load_2(cur); load_1b(cur); }
     load_w(cur, rw);
   }
 
@@ -339,6 +466,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     const bool row_stores = PACKED && t0 + L > Tn;
     const long long out_base = sv.row<PACKED>(bi) * lay.sb + hi * lay.sh + (long long)(sv.first<PACKED>(bi) + t0) * lay.st;
     const int tt = sv.first<PACKED>(bi) + t0, br = sv.row<PACKED>(bi);
+    const unsigned char* tiles = ws_tiles + (size_t)cur.ch * tiles_per_chunk * TILE_BYTES;
     const uint32_t par = it & 1;
     nxt = advance(cur);
     const bool more = nxt.ch < n_ch;
@@ -365,30 +493,30 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
       *reinterpret_cast<float4*>(&sm.gs[sw64(row, 8 * cc + 4)]) = make_float4(g[4], g[5], g[6], g[7]);
     }
     R7C_STAMP(17);
-    // ---- MMA group 0: sa = W h~0 (+ U) | dz = G^T do + B2 dh^
-    if (lane == 0 && warp < 2) {
+    // ---- MMA group 1: all four dA products; dv; the state part of [dq~; da~]
+    if (lane == 0 && warp < 3) {
       ok = mbar_wait(&sm.bar_l0, par, status, 321) && ok;
       ok = mbar_wait(&sm.bar_l1, par, status, 324) && ok;
       if (ok) {
         tc_fence_after();
         if (warp == 0) {
-          umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 192), smem_u32(sm.dz), smem_u32(sm.h0), false);         // W h~0
+          umma_tile<128, 128, 0, 0>(tmem_addr(tm, 0, 0), smem_u32(sm.dout), smem_u32(sm.v), false);        // [do;dz] [v;sa]^T
+        } else if (warp == 1) {
+          umma_tile<64, 64, 1, 1, 8>(tmem_addr(tm, 0, 192), smem_u32(sm.aqk), smem_u32(sm.dout), false);   // A_qk^T do + A_ak^T dz
+          umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 192), smem_u32(sm.kt), smem_u32(sm.dhh), true);         // + k~ dh^
         } else {
-          umma_tile<64, 64, 1, 1>(tmem_addr(tm, 16, 192), smem_u32(sm.sa), smem_u32(sm.dout), false);      // G^T do
-          umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 192), smem_u32(sm.at), smem_u32(sm.dhh), true);        // + B2 dh^
+          umma_tile<128, 64, 0, 0>(tmem_addr(tm, 0, 128), smem_u32(sm.dout), smem_u32(sm.h0), false);      // [do;dz] h~0^T
         }
-        umma_commit(&sm.bar_m0);
+        umma_commit(&sm.bar_m1);
       }
     }
     ok = __syncthreads_and(ok);
     R7C_STAMP(18);
     if (warp == 3 && more) prefetch_l2(nxt);
     // ---- meanwhile: prefix sums of g over tokens, thread = (channel, quarter of the chunk)
-    float dglast = 0.f;       // threads of the last quarter: from the reverse scan
-    float gfirst = 0.f;       // threads of the first quarter: -gref, the exclusive prefix of the first token
+    float dglast = 0.f;       // threads of the last quarter: sum_v dh^[c][v] X[c][v]
     {
       const int c = tid & 63, quarter = tid >> 6;
-      if (quarter == 3) dglast = __ldg(ws_aux + (size_t)cur.ch * AUX_FLOATS + 128 + c);
       float gv[16];
 #pragma unroll
       for (int j = 0; j < 16; ++j) gv[j] = sm.gs[sw64(16 * quarter + j, c)];
@@ -399,46 +527,23 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
       __syncthreads();
       // gi - gref: the prefix inside the half; the first half lies before the reference point, the end of that half
       const float add = quarter == 0 ? -(run + sm.quart[0][c]) : quarter == 1 ? -run : quarter == 3 ? sm.quart[1][c] : 0.f;
-      if (quarter == 0) { gfirst = add; sm.quart[2][c] = add; }
+      if (quarter == 0) sm.quart[2][c] = add;      // -gref: the exclusive prefix of the first token
 #pragma unroll
       for (int j = 0; j < 16; ++j) sm.gs[sw64(16 * quarter + j, c)] = gv[j] + add;
-    }
-    ok = mbar_wait(&sm.bar_l1, par, status, 325) && ok;      // U
-    ok = ok && mbar_wait(&sm.bar_m0, par, status, 329);
-    tc_fence_after();
-    if (ok) {      // sa (lower lane halves) and dz (upper): the two upper rows of the operands of group 1
-      const int i = 16 * wq + (lane & 15), c0 = 32 * hsel;
-      uint32_t rr[32];
-      tmem_ld32(tmem_addr(tm, 32 * wq, 192 + c0), rr);
-      tmem_ld_wait();
-      float x[32];
-      if (lane < 16) {
-        tile_load_row32(sm.bt, i, c0, x);
+      if (quarter == 3 && ok) {      // X straight from the workspace
+        ok = mbar_wait(&sm.bar_l0, par, status, 325) && ok;
+        const uint4* xr = reinterpret_cast<const uint4*>(tiles + S_X * TILE_BYTES);
 #pragma unroll
-        for (int j = 0; j < 32; ++j) x[j] += __uint_as_float(rr[j]);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
+        for (int cchunk = 0; cchunk < 8; ++cchunk) {
+          const uint4 xa = __ldg(xr + (tile_chunk_off(c, cchunk) >> 4));
+          const uint4 da_ = *reinterpret_cast<const uint4*>(sm.dhh + tile_chunk_off(c, cchunk));
+          dglast += bf16_lo(xa.x) * bf16_lo(da_.x) + bf16_hi(xa.x) * bf16_hi(da_.x);
+          dglast += bf16_lo(xa.y) * bf16_lo(da_.y) + bf16_hi(xa.y) * bf16_hi(da_.y);
+          dglast += bf16_lo(xa.z) * bf16_lo(da_.z) + bf16_hi(xa.z) * bf16_hi(da_.z);
+          dglast += bf16_lo(xa.w) * bf16_lo(da_.w) + bf16_hi(xa.w) * bf16_hi(da_.w);
+        }
       }
-      tile_store_row32(lane < 16 ? sm.sa : sm.dz, i, c0, x);
     }
-    fence_async_smem();
-    tc_fence_before();
-    ok = __syncthreads_and(ok);
-    // ---- MMA group 1: all four dA products; dv; the state part of [dq~; da~]
-    if (lane == 0 && warp < 3 && ok) {
-      tc_fence_after();
-      if (warp == 0) {
-        umma_tile<128, 128, 0, 0>(tmem_addr(tm, 0, 0), smem_u32(sm.dout), smem_u32(sm.v), false);        // [do;dz] [v;sa]^T
-      } else if (warp == 1) {
-        umma_tile<64, 64, 1, 1, 8>(tmem_addr(tm, 0, 192), smem_u32(sm.aqk), smem_u32(sm.dout), false);   // A_qk^T do + A_ak^T dz
-        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 192), smem_u32(sm.kt), smem_u32(sm.dhh), true);         // + k~ dh^
-      } else {
-        umma_tile<128, 64, 0, 0>(tmem_addr(tm, 0, 128), smem_u32(sm.dout), smem_u32(sm.h0), false);      // [do;dz] h~0^T
-      }
-      umma_commit(&sm.bar_m1);
-    }
-    if (st_thread && ok) load_2(cur);      // a~, b~ over B2, U, which have been read
     ok = mbar_wait(&sm.bar_m1, par, status, 322) && ok;
     tc_fence_after();
     R7C_STAMP(19);
@@ -604,11 +709,13 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
       float run = dglast;
 #pragma unroll
       for (int j = 15; j >= 0; --j) { run += rv[j]; rv[j] = run; }
+      const float gfirst = quarter ? sm.gs[sw64(16 * quarter - 1, c)] : sm.quart[2][c];
+      __syncthreads();      // -gref has been read
       if (quarter) sm.quart[quarter - 1][c] = run;      // the last quarter's sum carries dglast
       __syncthreads();
       float add = 0.f;
       for (int q2 = quarter; q2 < 3; ++q2) add += sm.quart[q2][c];
-      float gprev = quarter ? sm.gs[sw64(16 * quarter - 1, c)] : gfirst;
+      float gprev = gfirst;
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         const int ii = 16 * quarter + j;
@@ -636,9 +743,9 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
       if (more) {
         load_1a(nxt);
         bulk_wait_read_1();       // dq, dk, da, db have left their tiles
-        load_1b(nxt);
+        load_2(nxt);
         bulk_wait_read();         // and dw
-        load_1c(nxt);
+        load_1b(nxt);
       }
     }
     R7C_STAMP(23);
@@ -651,7 +758,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
 }
 
 // ---------------------------------------------------------------------------------------------
-// 4. fused producers, backward: one 64-channel row per 8 threads (16 bytes each), in place
+// 6. fused producers, backward: one 64-channel row per 8 threads (16 bytes each), in place
 //      dp = dw W_SCALE s_p (1 - s_p),  s_p = sigmoid(p)
 //      dkk = -da + db s_q,  s_q = sigmoid(q);   dq = db kk s_q (1 - s_q)
 //      du = (dkk - kk (kk . dkk)) / |u|,  kk = u / |u|
@@ -743,28 +850,39 @@ int launch_rwkv7_chunked_bwd(const void* r, const void* w, const void* k, const 
   const int NT = num_chunks(Tn);
   Workspace ws = carve(workspace, B, Tn, H, ALL_TILES);
   TokLayout lay(mapT, H, head_first);
+  // every kernel exists for dense batches and for packed variable-length ones
+#define R7C_DISPATCH_PACKED(...) do { if (seq_start) { constexpr bool P = true; __VA_ARGS__; } else { constexpr bool P = false; __VA_ARGS__; } } while (0)
+  if (phases & PHASE_PREPARE) {
+    const int smem = (int)sizeof(PreSmem) + 1024;
+    int dev = 0, sms = 0;
+    if (cuda_ok(cudaGetDevice(&dev)) || cuda_ok(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)))
+      return RWKVB200_E_CUDA;
+    const int pre_grid = B * H * NT < 2 * sms ? B * H * NT : 2 * sms;     // persistent: two CTAs per SM
+    ProfScope prof("r7c_bwd_pre_kernel", st);
+    R7C_DISPATCH_PACKED(
+      if (cuda_ok(cudaFuncSetAttribute(r7c_bwd_pre_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)))
+        return RWKVB200_E_CUDA;
+      r7c_bwd_pre_kernel<P><<<pre_grid, 128, smem, st>>>(tmap_do, ws.tiles, ALL_TILES, sv, H, NT, B * H * NT, status));
+  }
+  e = check_launch();
+  if (e) return e;
   if (phases & PHASE_SCAN) {
+    const int smem = (int)sizeof(BScanSmem) + 1024;
     int dev = 0, sms = 0;
     if (cuda_ok(cudaGetDevice(&dev)) || cuda_ok(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)))
       return RWKVB200_E_CUDA;
     ProfScope prof("r7c_bwd_scan_kernel", st);
-#define R7C_LAUNCH_BSCAN(S, P)                                                                                    \
-    do {                                                                                                          \
-      const int smem = (int)sizeof(BScanSmem<S>) + 1024;                                                          \
-      if (cuda_ok(cudaFuncSetAttribute(r7c_bwd_scan_kernel<S, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem))) \
-        return RWKVB200_E_CUDA;                                                                                   \
-      r7c_bwd_scan_kernel<S, P><<<B * H, 256, smem, st>>>(tmap_do, ws.tiles, ws.aux, ws.fin, ALL_TILES, d_ht, d_h0, \
-                                                          sv, H, NT, status);                                     \
-    } while (0)
-    if (B * H > sms) { if (seq_start) R7C_LAUNCH_BSCAN(2, true); else R7C_LAUNCH_BSCAN(2, false); }
-    else             { if (seq_start) R7C_LAUNCH_BSCAN(4, true); else R7C_LAUNCH_BSCAN(4, false); }
-#undef R7C_LAUNCH_BSCAN
+    R7C_DISPATCH_PACKED(
+      if (cuda_ok(cudaFuncSetAttribute(r7c_bwd_scan_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)))
+        return RWKVB200_E_CUDA;
+      r7c_bwd_scan_kernel<P><<<B * H, 256, smem, st>>>(tmap_do, ws.tiles, ws.aux, ALL_TILES, d_ht, d_h0, sv, H, NT,
+                                                       B * H <= sms ? 1 : 0, status));
   }
   e = check_launch();
   if (e) return e;
   // Units the forward marked (decay beyond the range of the scaled operands, or a very short sequence): their
   // gradients come from the float32 recurrence instead.  Its state checkpoints (16 KB per 8 tokens = 128 KB per
-  // chunk) go into the unit's own tile region of the workspace (136 KB per chunk), whose contents are void for
+  // chunk) go into the unit's own tile region of the workspace (144 KB per chunk), whose contents are void for
   // such a unit.
   auto exact_units = [&]() -> int {
     const long long unit_floats = (long long)NT * ALL_TILES * TILE_BYTES / (long long)sizeof(float);
@@ -795,7 +913,7 @@ int launch_rwkv7_chunked_bwd(const void* r, const void* w, const void* k, const 
     do {                                                                                                          \
       if (cuda_ok(cudaFuncSetAttribute(r7c_bwd_final_kernel<P, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem))) \
         return RWKVB200_E_CUDA;                                                                                   \
-      r7c_bwd_final_kernel<P, F><<<grid, 256, smem, st>>>((const bf16*)w, tmap_do, tmap_v, ws.tiles, ws.aux, ALL_TILES, \
+      r7c_bwd_final_kernel<P, F><<<grid, 256, smem, st>>>((const bf16*)w, tmap_do, tmap_v, ws.tiles, ALL_TILES,   \
           tmap_out[0], tmap_out[1], tmap_out[2], tmap_out[3], tmap_out[4], tmap_out[5], (bf16*)dr, (bf16*)dw,     \
           (bf16*)dk, (bf16*)dv, (bf16*)da, (bf16*)db, sv, H, NT, n_ch, lay, status, debug_stamp_buffer());        \
     } while (0)
@@ -804,6 +922,7 @@ int launch_rwkv7_chunked_bwd(const void* r, const void* w, const void* k, const 
     else R7C_LAUNCH_FINAL(false, false);
 #undef R7C_LAUNCH_FINAL
   }
+#undef R7C_DISPATCH_PACKED
   if (fused) {      // dw, da, db -> gradients of the pre-activations, in place
     e = check_launch();
     if (e) return e;

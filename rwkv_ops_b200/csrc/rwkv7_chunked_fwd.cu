@@ -18,30 +18,27 @@ constexpr float EXP2_FLOOR = -126.f;      // 2^x below this is flushed to zero a
 // ---------------------------------------------------------------------------------------------
 constexpr int NROW = 68;   // padded row of the fp32 copy of A_ab (keeps float4 alignment)
 
-// Eleven tiles whose space is used over again; each line says what a tile holds in turn.
 struct IntraSmem {
   unsigned char qt[TILE_BYTES], at[TILE_BYTES];     // [q~; a~]  (128-row A operand)
   unsigned char kt[TILE_BYTES], bt[TILE_BYTES];     // [k~; b~]  (128-row B operand)
-  unsigned char aqk[TILE_BYTES], aak[TILE_BYTES];   // A_qk, A_ak; the inverse's Q, T; W^, U; N (fp32, both)
-  unsigned char aqb[TILE_BYTES];                    // A_qb; P
-  unsigned char v[TILE_BYTES];                      // v (TMA)
-  unsigned char ainv[TILE_BYTES];                   // Ainv; G; Q
-  unsigned char y[TILE_BYTES];                      // raw w (TMA); Y = A_ak v; W
-  unsigned char x1[TILE_BYTES];                     // B2; O'
-  float nmat[L * NROW];                             // g, then its prefix sums; stril(A_ab) in fp32
+  unsigned char aqk[TILE_BYTES], aak[TILE_BYTES];   // [A_qk; A_ak] (128-row A operand); aak later holds W
+  unsigned char o1[TILE_BYTES];                     // A_qk v
+  unsigned char aqb[TILE_BYTES];
+  unsigned char v[TILE_BYTES];                      // TMA; later U
+  unsigned char ainv[TILE_BYTES];
+  unsigned char y[TILE_BYTES];                      // A_ak v
+  float nmat[L * NROW];                             // stril(A_ab) in fp32
   float qtot[4][64];                                // sums of g over the four quarters of the chunk
-  float vec[2][64];                                 // e^{gref}, e^{glast-gref}
-  uint64_t bar_v, bar_w, bar_in, bar_dr, bar_m1, bar_m2, bar_m3, bar_m4, bar_m5, bar_m6;
+  uint64_t bar_v, bar_w, bar_in, bar_ia, bar_m1, bar_m2, bar_m3, bar_m4, bar_m5;
   uint32_t tmem_base;
 };
 
-// Persistent: CTAs (two per SM) walk over chunk-heads ch = blockIdx.x, blockIdx.x + gridDim.x, ...  The raw tiles of
-// the next chunk-head are requested by TMA as soon as the tiles they land in are free: k and v after MMA 2, a after
-// MMA 3, w and b after MMA 4, q at the end; and its rows are asked into L2 before that.
-// TMEM: columns 0..127 MMA 1; then (M = 64 accumulators pair up on the two lane halves)
-//   0..63 G | B2, then P | Q;   64..127 N | O' (from MMA 2 on);   128..191 Y | the inverse's T, P T;   192..255 W | U.
+// Persistent: CTAs (two per SM) walk over chunk-heads ch = blockIdx.x, blockIdx.x + gridDim.x, ...  The
+// raw q, k, a, b, w tiles of the next chunk-head are requested by TMA as soon as the tiles they land in
+// (q~, k~, a~, b~, which are then scaled in place, and O1) have been copied out, its v tile as soon as
+// MMA 2 has read the current one, and the rows of the one after that are asked into L2.
 // 256 threads: warp w reads TMEM lanes 32*(w&3).. and the two warps that share a lane window split
-// the columns (hsel = w>>2).
+// the columns (hsel = w>>2); the triangular solve runs on warps 0-1 while the other warps drain MMA 2.
 template <bool PACKED, bool FUSED>
 __global__ void __launch_bounds__(256, 2)
 r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, const bf16* __restrict__ k,
@@ -53,7 +50,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
                      float* __restrict__ ws_aux, int* __restrict__ ws_flags, int tiles_per_chunk,
                      int keep_for_bwd, SeqView sv, int H, int NT, int n_ch, TokLayout lay, int* status, long long* dbg) {
 #ifdef RWKVB200_DEVTOOLS
-#define R7C_STAMP(n) do { if (dbg && tid == 0 && blockIdx.x == gridDim.x / 2 && it == 15) dbg[n] = clock64(); } while (0)
+#define R7C_STAMP(n) do { if (dbg && tid == 0 && blockIdx.x == gridDim.x / 2 && it == 30) dbg[n] = clock64(); } while (0)
 #else
 #define R7C_STAMP(n) do {} while (0)
 #endif
@@ -61,12 +58,10 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
   IntraSmem& sm = *reinterpret_cast<IntraSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int wq = warp & 3, hsel = warp >> 2;
-  const bool st_thread = tid == 64;      // requests raw tiles, copies results out
 
   if (tid == 0) {
-    mbar_init(&sm.bar_v, 1); mbar_init(&sm.bar_w, 1); mbar_init(&sm.bar_in, 1); mbar_init(&sm.bar_dr, 1);
-    mbar_init(&sm.bar_m1, 1); mbar_init(&sm.bar_m2, 1); mbar_init(&sm.bar_m3, 2); mbar_init(&sm.bar_m4, 1);
-    mbar_init(&sm.bar_m5, 1); mbar_init(&sm.bar_m6, 2);
+    mbar_init(&sm.bar_v, 1); mbar_init(&sm.bar_w, 1); mbar_init(&sm.bar_in, 1); mbar_init(&sm.bar_ia, 1); mbar_init(&sm.bar_m1, 1); mbar_init(&sm.bar_m2, 1); mbar_init(&sm.bar_m3, 1);
+    mbar_init(&sm.bar_m4, 1); mbar_init(&sm.bar_m5, 1);
     fence_mbar_init();
   }
   if (warp == 0) tmem_alloc(&sm.tmem_base, 256);
@@ -75,17 +70,32 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
   tc_fence_after();
   const uint32_t tm = sm.tmem_base;
 
-  // The raw tiles of a chunk-head (rows past the end of the sequence arrive as zeros); all of st_thread
-  auto load = [&](unsigned char* dst, const CUtensorMap* map, uint64_t* bar, const ChunkPos& p) {
-    tma_load_4d(dst, map, bar, 0, sv.first<PACKED>(p.bi) + p.c * L, p.hi, sv.row<PACKED>(p.bi));
+  auto coords = [&](const ChunkPos& p, int& bi, int& hi, int& t0) { bi = p.bi; hi = p.hi; t0 = p.c * L; };
+  // The raw tiles of a chunk-head (rows past the end of the sequence arrive as zeros).  w, needed first,
+  // lands in the A_qk tile, free from the end of the triangular inverse to the first epilogue of the next
+  // chunk-head; q, k, a, b, needed only after the prefix sums, land in the tiles that will hold their
+  // scaled versions once those have been copied out.
+  auto load_w = [&](const ChunkPos& p) {       // tid 0
+    int bi, hi, t0; coords(p, bi, hi, t0);
+    mbar_expect_tx(&sm.bar_w, TILE_BYTES);
+    tma_load_4d(sm.aqk, &tmap_w, &sm.bar_w, 0, sv.first<PACKED>(bi) + t0, hi, sv.row<PACKED>(bi));
   };
-  auto load_w = [&](const ChunkPos& p) { mbar_expect_tx(&sm.bar_w, TILE_BYTES); load(sm.y, &tmap_w, &sm.bar_w, p); };
-  auto load_v = [&](const ChunkPos& p) { mbar_expect_tx(&sm.bar_v, TILE_BYTES); load(sm.v, &tmap_v, &sm.bar_v, p); };
-  // q, k, a, b share a barrier; k comes first
-  auto load_k = [&](const ChunkPos& p) { mbar_expect_tx(&sm.bar_in, 4 * TILE_BYTES); load(sm.kt, &tmap_k, &sm.bar_in, p); };
-  auto load_q = [&](const ChunkPos& p) { load(sm.qt, &tmap_q, &sm.bar_in, p); };
-  auto load_a = [&](const ChunkPos& p) { load(sm.at, &tmap_a, &sm.bar_in, p); };
-  auto load_b = [&](const ChunkPos& p) { load(sm.bt, &tmap_b, &sm.bar_in, p); };
+  // q, k, b land in tiles that only MMA 1 reads and are requested as soon as MMA 2 has completed (their
+  // copies to the workspace have left shared memory by then); a lands in the tile MMA 3 reads and is requested
+  // after it: both are on their way most of a chunk-head before the next one needs them.
+  auto load_qkb = [&](const ChunkPos& p) {     // tid 0
+    int bi, hi, t0; coords(p, bi, hi, t0);
+    const int tt = sv.first<PACKED>(bi) + t0, br = sv.row<PACKED>(bi);
+    mbar_expect_tx(&sm.bar_in, 3 * TILE_BYTES);
+    tma_load_4d(sm.qt, &tmap_q, &sm.bar_in, 0, tt, hi, br);
+    tma_load_4d(sm.kt, &tmap_k, &sm.bar_in, 0, tt, hi, br);
+    tma_load_4d(sm.bt, &tmap_b, &sm.bar_in, 0, tt, hi, br);
+  };
+  auto load_a = [&](const ChunkPos& p) {       // tid 0
+    int bi, hi, t0; coords(p, bi, hi, t0);
+    mbar_expect_tx(&sm.bar_ia, TILE_BYTES);
+    tma_load_4d(sm.at, &tmap_a, &sm.bar_ia, 0, sv.first<PACKED>(bi) + t0, hi, sv.row<PACKED>(bi));
+  };
   // chunk slots past the end of a (packed) sequence are skipped
   auto empty = [&](const ChunkPos& p) {
     if constexpr (!PACKED) return false;      // a dense batch has no empty slots
@@ -96,42 +106,56 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
     return p;
   };
   // Ask for a chunk-head's token rows to be brought into L2, ahead of the TMA loads above.
-  auto prefetch_rows = [&](const ChunkPos& p) {      // one thread
-    const int tt = sv.first<PACKED>(p.bi) + p.c * L, br = sv.row<PACKED>(p.bi);
-    tma_prefetch_4d(&tmap_k, 0, tt, p.hi, br);
-    tma_prefetch_4d(&tmap_v, 0, tt, p.hi, br);
-    tma_prefetch_4d(&tmap_a, 0, tt, p.hi, br);
-    tma_prefetch_4d(&tmap_w, 0, tt, p.hi, br);
-    tma_prefetch_4d(&tmap_b, 0, tt, p.hi, br);
-    tma_prefetch_4d(&tmap_q, 0, tt, p.hi, br);
+  auto prefetch_rows = [&](const ChunkPos& p) {
+    int bi, hi, t0; coords(p, bi, hi, t0);
+    const int Tn = sv.length<PACKED>(bi);
+    const long long base = sv.row<PACKED>(bi) * lay.sb + hi * lay.sh + sv.first<PACKED>(bi) * lay.st;
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      const int e = tid + 256 * n, row = e >> 3, cc = e & 7, tok = t0 + row;
+      if (tok < Tn && cc == 0) {      // one 128-byte row per request
+        const long long off = base + (long long)tok * lay.st;
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(w + off));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(q + off));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(k + off));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(a + off));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(b + off));
+      }
+    }
+  };
+  auto load_v = [&](const ChunkPos& p) {   // tid 0
+    int bi, hi, t0; coords(p, bi, hi, t0);
+    mbar_expect_tx(&sm.bar_v, TILE_BYTES);
+    tma_load_4d(sm.v, &tmap_v, &sm.bar_v, 0, sv.first<PACKED>(bi) + t0, hi, sv.row<PACKED>(bi));
   };
   ChunkPos cur = chunk_pos(blockIdx.x, NT, H);
   if (cur.ch < n_ch && empty(cur)) cur = advance(cur);
-  if (cur.ch < n_ch && st_thread) { load_w(cur); load_k(cur); load_q(cur); load_a(cur); load_b(cur); load_v(cur); }
+  if (cur.ch < n_ch && tid == 0) { load_w(cur); load_qkb(cur); load_a(cur); load_v(cur); }
   // The two CTAs that share an SM would otherwise run their phases in lockstep and compete for the
   // same unit (shared-memory pipe during the triangular solve); start every other CTA half a
-  // chunk-head late, where there is more than one chunk-head per CTA.
-  if ((blockIdx.x & 1) && n_ch > 2 * gridDim.x) __nanosleep(6000);
+  // chunk-head late.
+  if (blockIdx.x & 1) __nanosleep(6000);
 
   bool ok = true;
   int it = 0;
   for (ChunkPos nxt; cur.ch < n_ch && ok; cur = nxt, ++it) {
-    const int ch = cur.ch, bi = cur.bi, hi = cur.hi, t0 = cur.c * L;
+    const int ch = cur.ch;
+    int bi, hi, t0; coords(cur, bi, hi, t0);
     const int Tn = sv.length<PACKED>(bi);
     unsigned char* out_tiles = ws_tiles + (size_t)ch * tiles_per_chunk * TILE_BYTES;
     const uint32_t par = it & 1;
     nxt = advance(cur);
-    const bool more = nxt.ch < n_ch;
+    const int next = nxt.ch;
 
     R7C_STAMP(0);
-    if (more && tid == 96) prefetch_rows(nxt);
+    if (next < n_ch) prefetch_rows(nxt);
     // this thread's 2 x 16 bytes (8 channels of one token) of the raw w tile
     uint4 rw[2];
     ok = mbar_wait(&sm.bar_w, par, status, 206) && ok;
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
       const int e = tid + 256 * n;
-      rw[n] = *reinterpret_cast<const uint4*>(sm.y + tile_chunk_off(e >> 3, e & 7));
+      rw[n] = *reinterpret_cast<const uint4*>(sm.aqk + tile_chunk_off(e >> 3, e & 7));
     }
     // ---- phase A: decay prefix sums (in units of log 2) and the four scaled operands; the prefix sum over tokens goes
     // through shared memory (the fp32 area that later holds A_ab).
@@ -176,17 +200,16 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
       __syncthreads();
       if (tid < 64) {
         const float tot0 = sm.qtot[0][tid] + sm.qtot[1][tid], tot1 = sm.qtot[2][tid] + sm.qtot[3][tid];
-        const float eg = ex2(fmaxf(tot0, EXP2_FLOOR)), dl = ex2(fmaxf(tot1, EXP2_FLOOR));
-        sm.vec[0][tid] = eg;                                   // e^{gref}
-        sm.vec[1][tid] = dl;                                   // e^{glast-gref}
-        ws_aux[(size_t)ch * AUX_FLOATS + tid] = eg;
-        ws_aux[(size_t)ch * AUX_FLOATS + 64 + tid] = dl;
+        ws_aux[(size_t)ch * AUX_FLOATS + tid] = ex2(fmaxf(tot0, EXP2_FLOOR));        // e^{gref}
+        ws_aux[(size_t)ch * AUX_FLOATS + 64 + tid] = ex2(fmaxf(tot1, EXP2_FLOOR));   // e^{glast-gref}
         // a half-chunk decay sum beyond the limit: the unit is recomputed by the float32 recurrence
         if (fminf(tot0, tot1) < -DECAY_LIMIT * LOG2E || Tn < SHORT_SEQ) ws_flags[bi * H + hi] = 1;
       }
-      // the raw q, k, a, b: each thread scales its own 2 x 16 bytes in place
+      // the raw q, k, a, b: each thread scales its own 2 x 16 bytes in place (the previous chunk-head's W, U,
+      // A_qb, O1 copies may still be reading their tiles: those are rewritten only after MMA 1)
       uint4 rq[2], rk[2], ra[2], rb[2];
       ok = mbar_wait(&sm.bar_in, par, status, 207) && ok;
+      ok = mbar_wait(&sm.bar_ia, par, status, 208) && ok;
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
         const int e = tid + 256 * n;
@@ -252,27 +275,26 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
         *reinterpret_cast<uint4*>(sm.bt + off) = make_uint4(ob[0], ob[1], ob[2], ob[3]);
       }
     }
-    if (st_thread) bulk_wait_read();      // the previous results have left their tiles, which the epilogue below rewrites
     fence_async_smem();
-    tc_fence_before();
-    ok = __syncthreads_and(ok);
+    __syncthreads();
 
     R7C_STAMP(2);
     // ---- MMA 1: [q~; a~] [k~; b~]^T  ->  TMEM columns 0..127, row r on lane r
-    if (tid == 0 && ok) {
+    if (tid == 0) {
+      bulk_wait_read();      // the previous W, U copies are done: the epilogue below rewrites their tiles
       tc_fence_after();
       umma_tile<128, 128, 0, 0>(tm, smem_u32(sm.qt), smem_u32(sm.kt), false);
       umma_commit(&sm.bar_m1);
     }
-    if (st_thread && ok && keep_for_bwd) {
-      bulk_store(out_tiles + S_QT * TILE_BYTES, sm.qt, TILE_BYTES);
-      bulk_store(out_tiles + S_KT * TILE_BYTES, sm.kt, 2 * TILE_BYTES);      // k~, b~
-      bulk_store(out_tiles + S_AT * TILE_BYTES, sm.at, TILE_BYTES);
-      bulk_commit();
-    }
-    ok = ok && mbar_wait(&sm.bar_m1, par, status, 201);
+    ok = mbar_wait(&sm.bar_m1, par, status, 201) && ok;
     tc_fence_after();
     R7C_STAMP(3);
+    if (tid == 0 && ok) {      // MMA 1 was the last reader of q~, k~, b~ in shared memory: copy them out now
+      bulk_store(out_tiles + S_QT * TILE_BYTES, sm.qt, TILE_BYTES);
+      bulk_store(out_tiles + S_KT * TILE_BYTES, sm.kt, TILE_BYTES);
+      bulk_store(out_tiles + S_BT * TILE_BYTES, sm.bt, TILE_BYTES);
+      bulk_commit();
+    }
     if (ok) {
       const int r = 32 * wq + lane, i = r & 63;
       const bool lower = r >= 64;       // rows of a~: strictly lower triangle; rows of q~: lower incl. diagonal
@@ -323,20 +345,21 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
     ok = __syncthreads_and(ok);
 
     R7C_STAMP(4);
-    // ---- MMA 2: Y = A_ak v (columns 128..191), and the first terms of N = k~^T v | O' = A_qk v (columns 64..127)
-    if (tid == 0 && ok) {
-      ok = mbar_wait(&sm.bar_v, par, status, 202);
+    // ---- MMA 2: [A_qk; A_ak] v  ->  TMEM columns 128..191 (rows 0..63 = O1, 64..127 = Y)
+    if (tid == 0) {
+      ok = mbar_wait(&sm.bar_v, par, status, 202) && ok;
       tc_fence_after();
-      umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 128), smem_u32(sm.aak), smem_u32(sm.v), false);
-      umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 64), smem_u32(sm.kt), smem_u32(sm.v), false);
-      umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 64), smem_u32(sm.aqk), smem_u32(sm.v), false);
+      umma_tile<128, 64, 0, 1>(tmem_addr(tm, 0, 128), smem_u32(sm.aqk), smem_u32(sm.v), false);
       umma_commit(&sm.bar_m2);
+      if (keep_for_bwd) {   // A_qk, A_ak, a~ are operands of the backward: copy them out before they are overwritten
+        bulk_store(out_tiles + S_AQK * TILE_BYTES, sm.aqk, TILE_BYTES);
+        bulk_store(out_tiles + S_AAK * TILE_BYTES, sm.aak, TILE_BYTES);
+        bulk_store(out_tiles + S_AT * TILE_BYTES, sm.at, TILE_BYTES);
+        bulk_commit();
+      }
     }
-    if (st_thread && ok && keep_for_bwd) {
-      bulk_store(out_tiles + S_AQK * TILE_BYTES, sm.aqk, 2 * TILE_BYTES);      // A_qk, A_ak
-      bulk_commit();
-    }
-    // ---- Ainv = X = (I - N)^-1, N = stril(A_ab), by two levels of block inversion:
+    // ---- rows of MMA 2 (warps 2-7), then Ainv = X = (I - N)^-1, N = stril(A_ab), by two levels of block
+    // inversion:
     //   D. the four 16 x 16 diagonal blocks D_I = (I - N_II)^-1 in fp32, one column per thread, row by row --
     //      the only substitutions, all four side by side (in place in nmat);
     //   1. the two 32 x 32 diagonal blocks in fp32: X_10 = D_1 (N_10 D_0) and X_32 = D_3 (N_32 D_2), 64 threads
@@ -367,25 +390,39 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
 #pragma unroll
         for (int rr = 0; rr < 16; ++rr) sm.nmat[(16 * I + rr) * NROW + c] = xb[rr];
       }
-      ok = ok && mbar_wait(&sm.bar_m2, par, status, 203);
-      tc_fence_after();
-      if (ok) {      // Y rows (lower lane halves)
-        uint32_t rr[32];
-        tmem_ld32(tmem_addr(tm, 32 * wq, 128 + 32 * hsel), rr);
-        tmem_ld_wait();
-        if (lane < 16) {
+      if (warp >= 2) {
+        // warps 4-5 take O1 (both column halves), warps 2-3 and 6-7 take Y (one column half each)
+        ok = mbar_wait(&sm.bar_m2, par, status, 203) && ok;
+        tc_fence_after();
+        const int i = (32 * wq + lane) & 63;
+        if (wq < 2) {        // warps 4, 5
+#pragma unroll
+          for (int part = 0; part < 2; ++part) {
+            uint32_t rr[32];
+            tmem_ld32(tmem_addr(tm, 32 * wq, 128 + 32 * part), rr);
+            tmem_ld_wait();
+            float x[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
+            tile_store_row32(sm.o1, i, 32 * part, x);
+          }
+        } else {             // warps 2, 3, 6, 7
+          uint32_t rr[32];
+          tmem_ld32(tmem_addr(tm, 32 * wq, 128 + 32 * hsel), rr);
+          tmem_ld_wait();
           float x[32];
 #pragma unroll
           for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
-          tile_store_row32(sm.y, 16 * wq + lane, 32 * hsel, x);
+          tile_store_row32(sm.y, i, 32 * hsel, x);
         }
       }
-      // the scratch area: MMA 2 is done with it, the copies kept for the backward have to be
-      if (st_thread && ok) {
-        bulk_wait_read();                          // (q~, k~, b~, a~ have left shared memory as well)
-        if (more) { load_v(nxt); load_k(nxt); }    // MMA 2 was the last to read v and k~
+      // the scratch area: MMA 2 (and the copies of A_qk / A_ak kept for the backward) must be done with it
+      ok = mbar_wait(&sm.bar_m2, par, status, 205) && ok;
+      if (tid == 0) {
+        bulk_wait_read();                  // q~, k~, b~ (and the tiles kept for the backward) have left shared memory
+        if (next < n_ch) { load_v(nxt); load_qkb(nxt); }      // MMA 2 has read the v tile; nothing reads q~, k~, b~ any more
       }
-      ok = __syncthreads_and(ok);
+      __syncthreads();
       R7C_STAMP(10);
       if (I & 1) {               // step 1: row block I, column block I - 1
         const int cl = tid & 15, r0 = ((tid & 63) >> 4) * 4;
@@ -407,7 +444,8 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) P[(r0 + q) * 16 + cl] = acc[q];
-        if (I == 1) bar_sync(1, 64); else bar_sync(2, 64);
+        if (I == 1) asm volatile("bar.sync 1, 64;" ::: "memory");
+        else        asm volatile("bar.sync 2, 64;" ::: "memory");
 #pragma unroll
         for (int kk = 0; kk < 16; ++kk) col[kk] = P[kk * 16 + cl];
 #pragma unroll
@@ -448,7 +486,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
       R7C_STAMP(12);
       if (tid == 0) {
         tc_fence_after();
-        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 128), smem_u32(sm.aqk), smem_u32(sm.ainv), false);     // T = Q P
+        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 128), smem_u32(sm.aqk), smem_u32(sm.ainv), false);     // T = Q P
         umma_commit(&sm.bar_m4);
       }
       ok = mbar_wait(&sm.bar_m4, par, status, 209) && ok;
@@ -457,11 +495,11 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
         uint32_t rr[32];
         tmem_ld32(tmem_addr(tm, 32 * wq, 128 + 32 * hsel), rr);
         tmem_ld_wait();
-        if (lane >= 16) {
+        if (lane < 16) {        // an M = 64 accumulator lives on the lower 16 lanes of every warp's window
           float x[32];
 #pragma unroll
           for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
-          tile_store_row32(sm.aak, 16 * wq + (lane & 15), 32 * hsel, x);
+          tile_store_row32(sm.aak, 16 * wq + lane, 32 * hsel, x);
         }
       }
       fence_async_smem();
@@ -469,20 +507,20 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
       ok = __syncthreads_and(ok);
       if (tid == 0 && ok) {
         tc_fence_after();
-        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 128), smem_u32(sm.ainv), smem_u32(sm.aak), false);     // P T
+        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 128), smem_u32(sm.ainv), smem_u32(sm.aak), false);     // P T
         umma_commit(&sm.bar_m5);
       }
-      ok = ok && mbar_wait(&sm.bar_m5, par, status, 210);
+      ok = mbar_wait(&sm.bar_m5, par, status, 210) && ok;
       tc_fence_after();
       if (ok && hsel == 0) {      // rows 32..63, columns 0..31: the BA quadrant of Ainv
         uint32_t rr[32];
         tmem_ld32(tmem_addr(tm, 32 * wq, 128), rr);
         tmem_ld_wait();
-        if (lane >= 16 && wq >= 2) {
+        if (lane < 16 && wq >= 2) {
           float x[32];
 #pragma unroll
           for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
-          tile_store_row32(sm.ainv, 16 * wq + (lane & 15), 0, x);
+          tile_store_row32(sm.ainv, 16 * wq + lane, 0, x);
         }
       }
       R7C_STAMP(13);
@@ -493,135 +531,48 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
     ok = __syncthreads_and(ok);
 
     R7C_STAMP(6);
-    // ---- MMA 3: W = Ainv a~ | U = Ainv Y (columns 192..255); for the backward G = A_qb Ainv | B2 = Ainv^T b~ (0..63)
-    if (tid == 0 && ok) {
+    // ---- MMA 3: W = Ainv a~ (lower lane halves), U = Ainv Y (upper lane halves) -> TMEM columns 0..63
+    if (tid == 0) {
+      if (ok && next < n_ch) load_w(nxt);      // the scratch area in the A_qk tile is free again
       tc_fence_after();
-      umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 192), smem_u32(sm.ainv), smem_u32(sm.at), false);
-      umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 192), smem_u32(sm.ainv), smem_u32(sm.y), false);
+      umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 0), smem_u32(sm.ainv), smem_u32(sm.at), false);
+      umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 0), smem_u32(sm.ainv), smem_u32(sm.y), false);
       umma_commit(&sm.bar_m3);
+      bulk_store(out_tiles + S_AQB * TILE_BYTES, sm.aqb, TILE_BYTES);
+      bulk_store(out_tiles + S_O1 * TILE_BYTES, sm.o1, TILE_BYTES);
+      if (keep_for_bwd) bulk_store(out_tiles + S_AINV * TILE_BYTES, sm.ainv, TILE_BYTES);
+      bulk_commit();
     }
-    if (tid == 32 && ok) {
-      tc_fence_after();
-      if (keep_for_bwd) {
-        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 0), smem_u32(sm.aqb), smem_u32(sm.ainv), false);
-        umma_tile<64, 64, 1, 1>(tmem_addr(tm, 16, 0), smem_u32(sm.ainv), smem_u32(sm.bt), false);
-      }
-      umma_commit(&sm.bar_m3);
-    }
-    ok = ok && mbar_wait(&sm.bar_m3, par, status, 204);
+    ok = mbar_wait(&sm.bar_m3, par, status, 204) && ok;
     tc_fence_after();
     R7C_STAMP(7);
-    if (st_thread && ok && more) load_a(nxt);      // MMA 3 was the last to read a~
-    const int i = 16 * wq + (lane & 15), c0 = 32 * hsel;
-    const bool lo = lane < 16;
-    if (ok) {
+
+    {
+      // W -> the A_ak tile (free since MMA 2), U -> the Y tile (free: MMA 3 has completed)
+      const int i = 16 * wq + (lane & 15);
+      unsigned char* dst = lane < 16 ? sm.aak : sm.y;
       uint32_t rr[32];
-      float x[32];
-      tmem_ld32(tmem_addr(tm, 32 * wq, 192 + c0), rr);
+      tmem_ld32(tmem_addr(tm, 32 * wq, 32 * hsel), rr);
       tmem_ld_wait();
+      float x[32];
 #pragma unroll
       for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
-      if (!lo) {
-        tile_store_row32(sm.aak, i, c0, x);                         // U
-      } else {
-        if (keep_for_bwd) tile_store_row32(sm.y, i, c0, x);         // W
-#pragma unroll
-        for (int j = 0; j < 32; j += 4) {                           // W^
-          const float4 e = *reinterpret_cast<const float4*>(&sm.vec[0][c0 + j]);
-          x[j] *= e.x; x[j + 1] *= e.y; x[j + 2] *= e.z; x[j + 3] *= e.w;
-        }
-        tile_store_row32(sm.aqk, i, c0, x);
-      }
-      if (keep_for_bwd) {
-        tmem_ld32(tmem_addr(tm, 32 * wq, c0), rr);
-        tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
-        tile_store_row32(lo ? sm.ainv : sm.x1, i, c0, x);           // G | B2
-      }
+      tile_store_row32(dst, i, 32 * hsel, x);
     }
     fence_async_smem();
     tc_fence_before();
     ok = __syncthreads_and(ok);
-
     R7C_STAMP(8);
-    // ---- MMA 4: P = b~^T W^ | Q = A_qb W^ (columns 0..63); N += b~^T U | O' += A_qb U (columns 64..127)
     if (tid == 0 && ok) {
-      tc_fence_after();
-      umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 0), smem_u32(sm.bt), smem_u32(sm.aqk), false);
-      umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 64), smem_u32(sm.bt), smem_u32(sm.aak), true);
-      umma_commit(&sm.bar_m6);
-    }
-    if (tid == 32 && ok) {
-      tc_fence_after();
-      umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 0), smem_u32(sm.aqb), smem_u32(sm.aqk), false);
-      umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 64), smem_u32(sm.aqb), smem_u32(sm.aak), true);
-      umma_commit(&sm.bar_m6);
-    }
-    if (st_thread && ok) {
-      if (keep_for_bwd) {
-        bulk_store(out_tiles + S_G * TILE_BYTES, sm.ainv, TILE_BYTES);
-        bulk_store(out_tiles + S_B2 * TILE_BYTES, sm.x1, TILE_BYTES);
-        bulk_store(out_tiles + S_W * TILE_BYTES, sm.y, TILE_BYTES);
-        bulk_store(out_tiles + S_U * TILE_BYTES, sm.aak, TILE_BYTES);
-        bulk_commit();
-        bulk_wait_read();
-      }
-      mbar_arrive(&sm.bar_dr);      // the copies have left the tiles that the epilogue rewrites
-    }
-    ok = ok && mbar_wait(&sm.bar_m6, par, status, 205);
-    ok = ok && mbar_wait(&sm.bar_dr, par, status, 208);
-    tc_fence_after();
-    if (st_thread && ok && more) { load_w(nxt); load_b(nxt); }
-    if (ok) {
-      uint32_t rr[32];
-      float x[32];
-      tmem_ld32(tmem_addr(tm, 32 * wq, c0), rr);
-      tmem_ld_wait();
-      const float dl = sm.vec[1][i];
-      if (lo) {      // P, row i = key channel
-#pragma unroll
-        for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]) * dl;
-      } else {       // Q = q~ e^{gref} + A_qb W^, row i = token
-        tile_load_row32(sm.qt, i, c0, x);
-#pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-          const float4 e = *reinterpret_cast<const float4*>(&sm.vec[0][c0 + j]);
-          x[j] = x[j] * e.x + __uint_as_float(rr[j]);
-          x[j + 1] = x[j + 1] * e.y + __uint_as_float(rr[j + 1]);
-          x[j + 2] = x[j + 2] * e.z + __uint_as_float(rr[j + 2]);
-          x[j + 3] = x[j + 3] * e.w + __uint_as_float(rr[j + 3]);
-        }
-      }
-      tile_store_row32(lo ? sm.aqb : sm.ainv, i, c0, x);
-      tmem_ld32(tmem_addr(tm, 32 * wq, 64 + c0), rr);
-      tmem_ld_wait();
-      if (lo) {      // N, float32
-#pragma unroll
-        for (int j = 0; j < 32; j += 4)
-          *reinterpret_cast<float4*>(sm.aqk + n_piece_off(i, (c0 + j) >> 2)) =
-              make_float4(__uint_as_float(rr[j]) * dl, __uint_as_float(rr[j + 1]) * dl, __uint_as_float(rr[j + 2]) * dl,
-                          __uint_as_float(rr[j + 3]) * dl);
-      } else {       // O'
-#pragma unroll
-        for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
-        tile_store_row32(sm.x1, i, c0, x);
-      }
-    }
-    fence_async_smem();
-    tc_fence_before();
-    ok = __syncthreads_and(ok);
-    R7C_STAMP(9);
-    if (st_thread && ok) {
-      bulk_store(out_tiles + S_P * TILE_BYTES, sm.aqb, TILE_BYTES);
-      bulk_store(out_tiles + S_Q * TILE_BYTES, sm.ainv, TILE_BYTES);
-      bulk_store(out_tiles + S_N * TILE_BYTES, sm.aqk, 2 * TILE_BYTES);
-      bulk_store(out_tiles + S_O * TILE_BYTES, sm.x1, TILE_BYTES);
+      bulk_store(out_tiles + S_W * TILE_BYTES, sm.aak, TILE_BYTES);
+      bulk_store(out_tiles + S_U * TILE_BYTES, sm.y, TILE_BYTES);
       bulk_commit();
-      if (more) load_q(nxt);      // q~ was last read by the epilogue
+      // MMA 3 has read a~ (and its copy for the backward left shared memory long ago): the next raw a may land
+      if (next < n_ch) load_a(nxt);
     }
+    R7C_STAMP(9);
   }
-  if (st_thread) bulk_wait_all();
+  if (tid == 0) bulk_wait_all();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tm, 256);
@@ -629,56 +580,78 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
 }
 
 // ---------------------------------------------------------------------------------------------
-// scan kernel: grid = B*H, 256 threads, chunks in order: h <- e^{glast} h + P h + N,  o = Q h + O'
+// scan kernel: grid = B*H, 256 threads, chunks in order, fp32 state in TMEM.  Warp w reads TMEM lanes
+// 32*(w&3)..; the two warps that share a lane window take 32 of the 64 columns each (hsel = w>>2).
 // ---------------------------------------------------------------------------------------------
-// One 128x64x64 product per chunk, [P; Q] h, row r on TMEM lane r: warps 0, 1 (and 4, 5 for the upper 32 columns) own
-// the state rows, warps 2, 3 (6, 7) the token rows.  The two groups meet through mbarriers only.  The chain from
-// chunk to chunk runs through the state warps: h (fp32, registers) -> bf16 tile -> product -> read-out -> h; the token
-// warps write the output a chunk behind, from the other one of two accumulators.
-// STAGES = 2: two CTAs (two sequences) share an SM, the choice when there are more sequences than SMs; bound by the
-// 40 KB of tiles per chunk there.  STAGES = 4: one CTA per SM with loads three chunks ahead, for few sequences; the
-// latency of the chain bounds it.
-struct ScanStage {
-  unsigned char p[TILE_BYTES], q[TILE_BYTES];      // [P; Q]  (128-row A operand)
-  unsigned char n[2 * TILE_BYTES];                 // N, fp32
-  unsigned char o[TILE_BYTES];                     // O'
+// Operand tiles come in two groups, each requested again the moment the MMAs that read it have completed.
+// STAGES = 1 (single-buffered, 11 tiles = 88 KB): two CTAs (two sequences) share an SM, the choice when
+// there are more sequences than SMs; U and O1, which are only added row by row, do not enter shared
+// memory: every thread fetches its row into registers at the top of a chunk.  STAGES = 2 (21 tiles): one
+// CTA per SM with the groups of chunk c + 2 requested during chunk c and U, O1 staged with group 1, for
+// the case of few sequences, where nothing else on the SM covers a load latency.
+template <int STAGES> struct ScanGroup1 {
+  unsigned char qt[TILE_BYTES], kt[TILE_BYTES];   // read by step a: q~, k~ (adjacent slots)
+  unsigned char w[TILE_BYTES], v[TILE_BYTES];     //                 W, v (TMA)
+};
+template <> struct ScanGroup1<2> {
+  unsigned char qt[TILE_BYTES], kt[TILE_BYTES];
+  unsigned char o1[TILE_BYTES], w[TILE_BYTES], u[TILE_BYTES];   // adjacent slots O1, W, U: one copy
+  unsigned char v[TILE_BYTES];
+};
+struct ScanGroup2 {
+  unsigned char bt[TILE_BYTES], aqb[TILE_BYTES];  // read by step c: b~, A_qb (adjacent slots)
 };
 template <int STAGES>
 struct ScanSmem {
-  ScanStage st[STAGES];
-  unsigned char ht[TILE_BYTES];             // h as bf16, [k][v]
-  unsigned char hs[2][TILE_BYTES];          // h~0 = e^{gref} h as bf16 (kept for the backward)
-  unsigned char ot[TILE_BYTES];             // output rows of a chunk, staged for a TMA store
-  uint64_t bar_ld[STAGES], bar_free[STAGES], bar_m[2], bar_o[2];
+  ScanGroup1<STAGES> g1[STAGES];
+  ScanGroup2 g2[STAGES];
+  unsigned char ht[TILE_BYTES];             // h~0 as bf16, [k][v]
+  unsigned char sa[TILE_BYTES];             // sa as bf16, [token][v]
+  unsigned char xt[TILE_BYTES];             // X = h~0 + k~^T v + b~^T sa as bf16 (kept for the backward)
+  unsigned char ot[2][TILE_BYTES];          // output rows of a chunk, staged for a TMA store
+  uint64_t bar_g1[STAGES], bar_g2[STAGES], bar_a, bar_c;
   uint32_t tmem_base;
 };
-static_assert(sizeof(ScanSmem<2>) <= 115712, "two CTAs per SM");
 
 template <int STAGES, bool PACKED>
-__global__ void __launch_bounds__(256, STAGES == 2 ? 2 : 1)
-r7c_scan_fwd_kernel(const unsigned char* __restrict__ ws_tiles, const float* __restrict__ ws_aux, int tiles_per_chunk,
-                    unsigned char* __restrict__ bwd_tiles, unsigned char* __restrict__ fin_tiles,
+__global__ void __launch_bounds__(256, 3 - STAGES)
+r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned char* __restrict__ ws_tiles,
+                    const float* __restrict__ ws_aux, int tiles_per_chunk, unsigned char* __restrict__ bwd_tiles,
                     const float* __restrict__ h0, int n_state, const __grid_constant__ CUtensorMap tmap_o,
                     int write_o, float* __restrict__ ht, bf16* __restrict__ o_rows, SeqView sv, int H, int NT_slots,
-                    TokLayout lay, int* status) {
-  extern __shared__ __align__(1024) unsigned char smem_al[];
-  ScanSmem<STAGES>& sm = *reinterpret_cast<ScanSmem<STAGES>*>(smem_al);
+                    TokLayout lay, int* status, long long* dbg) {
+#ifdef RWKVB200_DEVTOOLS
+#define R7C_STAMP(n) do { if (dbg && tid == 0 && blockIdx.x == gridDim.x / 2 && c == 2) dbg[n] = clock64(); } while (0)
+#else
+#define R7C_STAMP(n) do {} while (0)
+#endif
+  extern __shared__ unsigned char smem_raw[];
+  ScanSmem<STAGES>& sm =
+      *reinterpret_cast<ScanSmem<STAGES>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int wq = warp & 3, hsel = warp >> 2, c0 = 32 * hsel;
-  if (smem_u32(smem_al) & 1023u) {      // the swizzled tiles need this alignment; there is no room to align by hand
-    if (tid == 0) atomicCAS(status, 0, 216);
-    return;
-  }
   const int unit = blockIdx.x, bi = unit / H, hi = unit % H;
   const size_t ch0 = (size_t)unit * NT_slots;
   const int Tn = sv.length<PACKED>(bi), tb = sv.first<PACKED>(bi), brow = sv.row<PACKED>(bi);
   const int NT = (Tn + L - 1) / L;           // chunks of this sequence (at least one)
-  const bool state_warp = wq < 2;
-  const int row = 32 * (wq & 1) + lane;      // state row k or token row i
+  const int row = 16 * wq + (lane & 15);     // state row k (lanes 0-15) or token row i (lanes 16-31)
+  const bool state_lane = lane < 16;
+  // With one CTA per SM the single-thread jobs of a chunk lie on the chain from chunk to chunk, and each
+  // bulk copy costs its issuing thread about a hundred cycles: they go to the first threads of four warps and
+  // run side by side (-12 % per chunk).  Thread 0 issues the MMAs (with the first threads of warps 1 and 2, one
+  // accumulator each), ld_thread requests operand tiles,
+  // st_thread copies sa and h~0 out for the backward, out_thread copies X and the output rows out.  Bulk-copy
+  // groups belong to the thread that committed them, so each storing thread waits for its own copies.  With
+  // two CTAs per SM the other CTA fills such gaps and thread 0 keeps all four jobs.
+  constexpr bool SPREAD = STAGES == 2;
+  const bool ld_thread = tid == (SPREAD ? 32 : 0), st_thread = tid == (SPREAD ? 64 : 0),
+             out_thread = tid == (SPREAD ? 96 : 0);
 
   if (tid == 0) {
-    for (int s = 0; s < STAGES; ++s) { mbar_init(&sm.bar_ld[s], 1); mbar_init(&sm.bar_free[s], 8); }
-    for (int t = 0; t < 2; ++t) { mbar_init(&sm.bar_m[t], 1); mbar_init(&sm.bar_o[t], 4); }
+    for (int i = 0; i < STAGES; ++i) { mbar_init(&sm.bar_g1[i], 1); mbar_init(&sm.bar_g2[i], 1); }
+    // with one CTA per SM each accumulator of an MMA group has its own issuing thread (one thread issues an
+    // MMA about every 80 cycles, the tensor pipe takes them faster), and a group completes with all arrivals
+    mbar_init(&sm.bar_a, SPREAD ? 3 : 1); mbar_init(&sm.bar_c, SPREAD ? 2 : 1);
     fence_mbar_init();
   }
   if (warp == 0) tmem_alloc(&sm.tmem_base, 128);
@@ -686,144 +659,196 @@ r7c_scan_fwd_kernel(const unsigned char* __restrict__ ws_tiles, const float* __r
   __syncthreads();
   tc_fence_after();
   const uint32_t tm = sm.tmem_base;
+  const uint32_t tm_p1 = tmem_addr(tm, 32 * wq, c0), tm_p2 = tmem_addr(tm, 32 * wq, 64 + c0);
 
-  auto issue_load = [&](int c) {
-    ScanStage& g = sm.st[c % STAGES];
-    mbar_expect_tx(&sm.bar_ld[c % STAGES], sizeof(ScanStage));
-    bulk_load(g.p, ws_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES, sizeof(ScanStage), &sm.bar_ld[c % STAGES]);
+  auto issue_g1 = [&](int c) {      // ld_thread (thread 0 for the first chunks)
+    const unsigned char* tiles = ws_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES;
+    ScanGroup1<STAGES>& g = sm.g1[c % STAGES];
+    uint64_t* bar = &sm.bar_g1[c % STAGES];
+    mbar_expect_tx(bar, (STAGES == 2 ? 6 : 4) * TILE_BYTES);
+    bulk_load(g.qt, tiles + S_QT * TILE_BYTES, 2 * TILE_BYTES, bar);
+    if constexpr (STAGES == 2) bulk_load(g.o1, tiles + S_O1 * TILE_BYTES, 3 * TILE_BYTES, bar);
+    else                       bulk_load(g.w, tiles + S_W * TILE_BYTES, TILE_BYTES, bar);
+    tma_load_4d(g.v, &tmap_v, bar, 0, tb + c * L, hi, brow);
   };
-  bool ok = true;
-  if (state_warp) {
-    float x[32];      // h[k = row][c0 .. c0 + 31]
-    if (n_state > 0) {
-      const float* S = h0 + (size_t)(n_state == 1 ? hi : unit) * 4096;   // S[v][k], h[k][v] = S[v][k]
+  auto issue_g2 = [&](int c) {      // ld_thread (thread 0 for the first chunks)
+    const unsigned char* tiles = ws_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES;
+    uint64_t* bar = &sm.bar_g2[c % STAGES];
+    mbar_expect_tx(bar, 2 * TILE_BYTES);
+    bulk_load(sm.g2[c % STAGES].bt, tiles + S_BT * TILE_BYTES, 2 * TILE_BYTES, bar);
+  };
+  if (tid == 0) {
+    for (int c = 0; c < STAGES && c < NT; ++c) { issue_g1(c); issue_g2(c); }
+  }
+
+  // ---- initial state: h~0 = e^{gref(chunk 0)} h0, fp32 into TMEM (lower lane halves of P2), bf16 into ht
+  {
+    float x[32];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) x[j] = S[(c0 + j) * 64 + row];
-    } else {
+    for (int vv = 0; vv < 32; ++vv) x[vv] = 0.f;
+    if (state_lane) {
+      const float e0 = ws_aux[ch0 * AUX_FLOATS + row];
+      if (n_state > 0) {
+        const float* S = h0 + (size_t)(n_state == 1 ? hi : unit) * 4096;   // S[v][k], h[k][v] = S[v][k]
 #pragma unroll
-      for (int j = 0; j < 32; ++j) x[j] = 0.f;
-    }
-    float eg_next = ws_aux[ch0 * AUX_FLOATS + row], dl_next = ws_aux[ch0 * AUX_FLOATS + 64 + row];
-    for (int c = 0; c < NT; ++c) {
-      const int s = c % STAGES, t = c & 1;
-      const uint32_t sp = (c / STAGES) & 1, tp = (c >> 1) & 1;
-      const float eg = eg_next, dl = dl_next;
-      if (c + 1 < NT) {      // fetched a chunk ahead
-        eg_next = ws_aux[(ch0 + c + 1) * AUX_FLOATS + row];
-        dl_next = ws_aux[(ch0 + c + 1) * AUX_FLOATS + 64 + row];
+        for (int vv = 0; vv < 32; ++vv) x[vv] = e0 * S[(c0 + vv) * 64 + row];
       }
       tile_store_row32(sm.ht, row, c0, x);
-      if (tid == 32 && bwd_tiles) bulk_wait_read();      // the h~0 tile about to be rewritten has left shared memory
-      fence_async_smem();
-      tc_fence_before();
-      ok = bar_sync_and(1, 128, ok);      // the one place where the group may leave the loop: all of it or none
-      if (!ok) break;
-      if (tid == 0) {
-        ok = mbar_wait(&sm.bar_ld[s], sp, status, 211);
-        if (c >= 2) ok = mbar_wait(&sm.bar_o[t], ((c >> 1) - 1) & 1, status, 212) && ok;      // this accumulator has been read
-        if (ok) {
-          tc_fence_after();
-          umma_tile<128, 64, 0, 1>(tmem_addr(tm, 0, 64 * t), smem_u32(sm.st[s].p), smem_u32(sm.ht), false);
-          umma_commit(&sm.bar_m[t]);
-        }
-      }
-      if (bwd_tiles) {      // h~0 for the backward, under the product; its tile of the chunk before goes out now
-        if (tid == 32 && c > 0) {
-          bulk_store(bwd_tiles + ((ch0 + c - 1) * (size_t)tiles_per_chunk + S_H0) * TILE_BYTES, sm.hs[t ^ 1], TILE_BYTES);
-          bulk_commit();
-        }
-        float y[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) y[j] = x[j] * eg;
-        tile_store_row32(sm.hs[t], row, c0, y);
-      }
-      ok = ok && mbar_wait(&sm.bar_ld[s], sp, status, 213);
-      ok = ok && mbar_wait(&sm.bar_m[t], tp, status, 214);
-      tc_fence_after();
-      if (ok) {
-        uint32_t r[32];
-        tmem_ld32(tmem_addr(tm, 32 * wq, 64 * t + c0), r);
-        tmem_ld_wait();
-        const float et = eg * dl;
-#pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-          const float4 n4 = *reinterpret_cast<const float4*>(sm.st[s].n + n_piece_off(row, (c0 + j) >> 2));
-          x[j] = et * x[j] + (__uint_as_float(r[j]) + n4.x);
-          x[j + 1] = et * x[j + 1] + (__uint_as_float(r[j + 1]) + n4.y);
-          x[j + 2] = et * x[j + 2] + (__uint_as_float(r[j + 2]) + n4.z);
-          x[j + 3] = et * x[j + 3] + (__uint_as_float(r[j + 3]) + n4.w);
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sm.bar_free[s]);
-      }
     }
-    // ---- the final state: fp32 for the caller, a bf16 tile for the backward
-    if (ok && ht) {
-      float* S = ht + (size_t)unit * 4096;
+    uint32_t r[32];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) S[(c0 + j) * 64 + row] = x[j];
-    }
-    if (bwd_tiles) {
-      if (ok) tile_store_row32(sm.ht, row, c0, x);
-      fence_async_smem();
-      ok = bar_sync_and(1, 128, ok);
-      if (tid == 32) {
-        if (ok) {
-          bulk_store(bwd_tiles + ((ch0 + NT - 1) * (size_t)tiles_per_chunk + S_H0) * TILE_BYTES, sm.hs[(NT - 1) & 1], TILE_BYTES);
-          bulk_store(fin_tiles + (size_t)unit * TILE_BYTES, sm.ht, TILE_BYTES);
-          bulk_commit();
-        }
-        bulk_wait_all();
-      }
-    }
-  } else {
-    const bool ld_thread = tid == 64;
-    bool ld_ok = true;
-    if (ld_thread)
-      for (int c = 0; c < STAGES && c < NT; ++c) issue_load(c);
-    for (int c = 0; c < NT; ++c) {
-      const int s = c % STAGES, t = c & 1, t0 = c * L;
-      const uint32_t sp = (c / STAGES) & 1, tp = (c >> 1) & 1;
-      ok = mbar_wait(&sm.bar_ld[s], sp, status, 215);
-      ok = ok && mbar_wait(&sm.bar_m[t], tp, status, 217);
-      tc_fence_after();
-      if (ok) {
-        uint32_t r[32];
-        float x[32];
-        tmem_ld32(tmem_addr(tm, 32 * wq, 64 * t + c0), r);
-        tmem_ld_wait();
-        tc_fence_before();
-        tile_load_row32(sm.st[s].o, row, c0, x);
-        __syncwarp();
-        if (lane == 0) { mbar_arrive(&sm.bar_o[t]); mbar_arrive(&sm.bar_free[s]); }
-#pragma unroll
-        for (int j = 0; j < 32; ++j) x[j] += __uint_as_float(r[j]);
-        if (ld_thread) bulk_wait_read();      // the output tile of the chunk before has left shared memory
-        bar_sync(2, 128);
-        tile_store_row32(sm.ot, row, c0, x);
-        fence_async_smem();
-      } else {
-        bar_sync(2, 128);
-      }
-      ok = bar_sync_and(2, 128, ok && ld_ok);      // the one place where the group may leave the loop
-      if (!ok) break;
-      if (write_o) {
-        if (PACKED && t0 + L > Tn) {  // the last rows of the box belong to the next sequence: row by row
-          store_tile_rows<128>(o_rows + brow * lay.sb + hi * lay.sh + (long long)(tb + t0) * lay.st, lay.st,
-                               sm.ot, Tn - t0, 32 * ((warp & 1) + 2 * hsel) + lane);
-        } else if (ld_thread) {           // rows past the end of the tensor are clipped by the TMA store
-          tma_store_4d(&tmap_o, sm.ot, 0, tb + t0, hi, brow);
-          bulk_commit();
-        }
-      }
-      if (ld_thread && c + STAGES < NT) {
-        ld_ok = mbar_wait(&sm.bar_free[s], sp, status, 218);
-        if (ld_ok) issue_load(c + STAGES);
-      }
-    }
-    if (ld_thread) bulk_wait_all();
+    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(x[j]);
+    tmem_st32(tm_p2, r);
+    tmem_st_wait();
   }
+  fence_async_smem();
   tc_fence_before();
+  __syncthreads();
+
+  bool ok = true;
+  for (int c = 0; c < NT && ok; ++c) {
+    const int t0 = c * L;
+    R7C_STAMP(48);
+    // this thread's row of U (state lanes) or O1 (token lanes), straight from the workspace
+    uint4 addrow[4];
+    if constexpr (STAGES == 1) {
+      const unsigned char* tile = ws_tiles + ((ch0 + c) * (size_t)tiles_per_chunk + (state_lane ? S_U : S_O1)) * TILE_BYTES;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) addrow[q] = __ldg(reinterpret_cast<const uint4*>(tile + tile_chunk_off(row, 4 * hsel + q)));
+      if (c + 1 < NT && hsel == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(tile + (size_t)tiles_per_chunk * TILE_BYTES + row * 128));
+    }
+    // decay factors needed at the end of this chunk, fetched early
+    // (applied one after the other: their product can underflow float32 where neither factor does)
+    float scale = 1.f, scale_next = 1.f;
+    if (state_lane) {
+      scale = ws_aux[(ch0 + c) * AUX_FLOATS + 64 + row];                       // e^{glast-gref} of this chunk
+      if (c + 1 < NT) scale_next = ws_aux[(ch0 + c + 1) * AUX_FLOATS + row];    // e^{gref} of the next chunk
+    }
+    // (a) SA = W h~0, QH = q~ h~0 (P1);  H += k~^T v (P2 lower)
+    if (lane == 0 && warp < (SPREAD ? 3 : 1)) {
+      ScanGroup1<STAGES>& g = sm.g1[c % STAGES];
+      ok = mbar_wait(&sm.bar_g1[c % STAGES], (c / STAGES) & 1, status, 211);
+      R7C_STAMP(49);
+      if (ok) {
+        tc_fence_after();
+        if (!SPREAD || warp == 0) umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 0), smem_u32(g.w), smem_u32(sm.ht), false);
+        if (!SPREAD || warp == 1) umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 0), smem_u32(g.qt), smem_u32(sm.ht), false);
+        if (!SPREAD || warp == 2) umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 64), smem_u32(g.kt), smem_u32(g.v), true);
+        umma_commit(&sm.bar_a);
+      }
+    }
+    ok = ok && mbar_wait(&sm.bar_a, c & 1, status, 212);
+    tc_fence_after();
+    R7C_STAMP(50);
+    // group 1 has been read by the MMAs: request the next (the staged O1 / U rows are still to be read)
+    if (STAGES == 1 && ld_thread && ok && c + STAGES < NT) issue_g1(c + STAGES);
+    float keep[32];     // token lanes: q~ h~0 + O1
+    if constexpr (STAGES == 2) {      // the staged O1 / U rows: observe the arrival of group 1 before reading them
+      ok = ok && mbar_wait(&sm.bar_g1[c % STAGES], (c / STAGES) & 1, status, 215);
+      const unsigned char* tile = state_lane ? sm.g1[c % STAGES].u : sm.g1[c % STAGES].o1;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) addrow[q] = *reinterpret_cast<const uint4*>(tile + tile_chunk_off(row, 4 * hsel + q));
+    }
+    if (ok) {
+      uint32_t r[32];
+      tmem_ld32(tm_p1, r);
+      tmem_ld_wait();
+      float add[32];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint4 u = addrow[q];
+        add[8 * q + 0] = bf16_lo(u.x); add[8 * q + 1] = bf16_hi(u.x);
+        add[8 * q + 2] = bf16_lo(u.y); add[8 * q + 3] = bf16_hi(u.y);
+        add[8 * q + 4] = bf16_lo(u.z); add[8 * q + 5] = bf16_hi(u.z);
+        add[8 * q + 6] = bf16_lo(u.w); add[8 * q + 7] = bf16_hi(u.w);
+      }
+#pragma unroll
+      for (int j = 0; j < 32; ++j) keep[j] = __uint_as_float(r[j]) + add[j];
+      if (state_lane) tile_store_row32(sm.sa, row, c0, keep);   // sa = W h~0 + U
+    }
+    fence_async_smem();
+    tc_fence_before();
+    ok = __syncthreads_and(ok);
+    if (STAGES == 2 && ld_thread && ok && c + STAGES < NT) issue_g1(c + STAGES);
+    if (bwd_tiles && st_thread && ok) {   // the backward needs sa and h~0 of every chunk
+      unsigned char* dst = bwd_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES;
+      bulk_store(dst + S_SA * TILE_BYTES, sm.sa, TILE_BYTES);
+      bulk_store(dst + S_H0 * TILE_BYTES, sm.ht, TILE_BYTES);
+      bulk_commit();
+    }
+    // (c) H += b~^T sa (P2 lower);  OQ = A_qb sa (P2 upper)
+    R7C_STAMP(51);
+    if (lane == 0 && warp < (SPREAD ? 2 : 1) && ok) {
+      ScanGroup2& g = sm.g2[c % STAGES];
+      ok = mbar_wait(&sm.bar_g2[c % STAGES], (c / STAGES) & 1, status, 214);
+      R7C_STAMP(52);
+      if (ok) {
+        tc_fence_after();
+        if (!SPREAD || warp == 0) umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 64), smem_u32(g.bt), smem_u32(sm.sa), true);
+        if (!SPREAD || warp == 1) umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 64), smem_u32(g.aqb), smem_u32(sm.sa), false);
+        umma_commit(&sm.bar_c);
+      }
+    }
+    ok = ok && mbar_wait(&sm.bar_c, c & 1, status, 213);
+    tc_fence_after();
+    R7C_STAMP(53);
+    if (ld_thread && ok && c + STAGES < NT) issue_g2(c + STAGES);     // group 2 has been read
+    if (bwd_tiles) {                                  // ht / sa are rewritten below and in the next chunk
+      if (st_thread) bulk_wait_read();
+      __syncthreads();
+    }
+    R7C_STAMP(54);
+    if (ok) {
+      const bool last = c + 1 == NT;
+      uint32_t r[32];
+      tmem_ld32(tm_p2, r);
+      tmem_ld_wait();
+      float x[32];
+      if (state_lane) {
+        if (bwd_tiles) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(r[j]);
+          tile_store_row32(sm.xt, row, c0, x);
+        }
+#pragma unroll
+        for (int j = 0; j < 32; ++j) { x[j] = (__uint_as_float(r[j]) * scale) * scale_next; r[j] = __float_as_uint(x[j]); }
+        if (!last) {
+          tile_store_row32(sm.ht, row, c0, x);
+        } else if (ht) {
+          float* S = ht + (size_t)unit * 4096;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) S[(c0 + j) * 64 + row] = x[j];
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(r[j]) + keep[j];
+        if (write_o) tile_store_row32(sm.ot[c & 1], row, c0, x);
+      }
+      tmem_st32(tm_p2, r);   // state lanes: rescaled state; token lanes: unchanged
+      tmem_st_wait();
+    }
+    fence_async_smem();
+    tc_fence_before();
+    ok = __syncthreads_and(ok);
+    R7C_STAMP(55);
+    if (bwd_tiles && out_thread && ok) {
+      bulk_store(bwd_tiles + ((ch0 + c) * (size_t)tiles_per_chunk + S_X) * TILE_BYTES, sm.xt, TILE_BYTES);
+      bulk_commit();
+    }
+    if (write_o && ok) {
+      if (PACKED && t0 + L > Tn) {  // the last rows of the box belong to the next sequence: row by row
+        store_tile_rows<256>(o_rows + brow * lay.sb + hi * lay.sh + (long long)(tb + t0) * lay.st, lay.st,
+                             sm.ot[c & 1], Tn - t0, tid);
+      } else if (out_thread) {           // rows past the end of the tensor are clipped by the TMA store
+        tma_store_4d(&tmap_o, sm.ot[c & 1], 0, tb + t0, hi, brow);
+        bulk_commit();
+        bulk_wait_read_1();              // the buffer of the previous chunk is free again
+      }
+    }
+    R7C_STAMP(56);
+  }
+#undef R7C_STAMP
+  if (st_thread || out_thread) bulk_wait_all();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tm, 128);
 }
@@ -886,17 +911,18 @@ int launch_rwkv7_chunked_fwd(const void* r, const void* w, const void* k, const 
     if (cuda_ok(cudaGetDevice(&dev)) || cuda_ok(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)))
       return RWKVB200_E_CUDA;
     ProfScope prof("r7c_scan_fwd_kernel", st);
-    // more sequences than SMs: two CTAs per SM with two stages each; else one CTA per SM with loads further ahead
+    // more sequences than SMs: two single-buffered CTAs per SM; else one double-buffered CTA per SM
 #define R7C_LAUNCH_SCAN(S, P)                                                                                      \
     do {                                                                                                           \
-      const int smem = (int)sizeof(ScanSmem<S>);                                                                   \
+      const int smem = (int)sizeof(ScanSmem<S>) + 1024;                                                            \
       if (cuda_ok(cudaFuncSetAttribute(r7c_scan_fwd_kernel<S, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem))) \
         return RWKVB200_E_CUDA;                                                                                    \
-      r7c_scan_fwd_kernel<S, P><<<B * H, 256, smem, st>>>(ws.tiles, ws.aux, tpc, keep_for_bwd ? ws.tiles : nullptr, \
-          ws.fin, h0, n_state, tmap_o, o ? 1 : 0, ht, (bf16*)o, sv, H, NT, lay, status);                           \
+      r7c_scan_fwd_kernel<S, P><<<B * H, 256, smem, st>>>(tmap_v, ws.tiles, ws.aux, tpc,                           \
+          keep_for_bwd ? ws.tiles : nullptr, h0, n_state, tmap_o, o ? 1 : 0, ht, (bf16*)o, sv, H, NT, lay, status, \
+          debug_stamp_buffer());                                                                                   \
     } while (0)
-    if (B * H > sms) { if (seq_start) R7C_LAUNCH_SCAN(2, true); else R7C_LAUNCH_SCAN(2, false); }
-    else             { if (seq_start) R7C_LAUNCH_SCAN(4, true); else R7C_LAUNCH_SCAN(4, false); }
+    if (B * H > sms) { if (seq_start) R7C_LAUNCH_SCAN(1, true); else R7C_LAUNCH_SCAN(1, false); }
+    else             { if (seq_start) R7C_LAUNCH_SCAN(2, true); else R7C_LAUNCH_SCAN(2, false); }
 #undef R7C_LAUNCH_SCAN
   }
   e = check_launch();

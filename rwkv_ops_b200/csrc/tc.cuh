@@ -76,24 +76,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
   return __all_sync(__activemask(), done) != 0;
 }
 
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-// Named barriers (id 1..15) over `n` threads of the CTA, a multiple of 32; the second form also combines a predicate,
-// so that every thread of a group takes the same decision after a bounded wait ran out in one of them.
-__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
-__device__ __forceinline__ bool bar_sync_and(int id, int n, bool ok) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.u32 p, %1, 0;\n\t"
-      "bar.red.and.pred q, %2, %3, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}"
-      : "=r"(r) : "r"((uint32_t)ok), "r"(id), "r"(n) : "memory");
-  return r != 0;
-}
-
 // ---------------------------------------------------------------------------------------------
 // proxies and fences
 // ---------------------------------------------------------------------------------------------
