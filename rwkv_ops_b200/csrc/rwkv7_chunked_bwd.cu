@@ -71,7 +71,7 @@ r7c_bwd_pre_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* _
   };
   ChunkPos cur = chunk_pos(blockIdx.x, NT, H);
   if (cur.ch < n_ch && empty(cur)) cur = advance(cur);
-  if (cur.ch < n_ch && tid == 0) issue_loads(cur, 0);
+  if (cur.ch < n_ch && warp == 0 && elect_one()) issue_loads(cur, 0);
 
   bool ok = true;
   int it = 0;
@@ -82,9 +82,9 @@ r7c_bwd_pre_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* _
     unsigned char* tiles = ws_tiles + (size_t)cur.ch * tiles_per_chunk * TILE_BYTES;
     nxt = advance(cur);
     // the other stage was last read by the MMAs of the previous chunk-head, which have completed
-    if (tid == 0 && nxt.ch < n_ch) issue_loads(nxt, s ^ 1);
+    if (warp == 0 && elect_one() && nxt.ch < n_ch) issue_loads(nxt, s ^ 1);
     ok = mbar_wait(&sm.bar_ld[s], (it >> 1) & 1, status, 301);
-    if (tid == 0 && ok) {
+    if (warp == 0 && elect_one() && ok) {
       bulk_wait_read();      // the copies of the previous B2 / P2 have left their tiles, which are rewritten below
       tc_fence_after();
       umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 0), smem_u32(g.aqb), smem_u32(g.dout), false);   // A_qb^T do
@@ -108,7 +108,7 @@ r7c_bwd_pre_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* _
     fence_async_smem();
     tc_fence_before();
     ok = __syncthreads_and(ok);
-    if (tid == 0 && ok) {
+    if (warp == 0 && elect_one() && ok) {
       tc_fence_after();
       umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 64), smem_u32(g.ainv), smem_u32(sm.p1), false);   // Ainv^T P1
       umma_commit(&sm.bar_m2);
@@ -134,12 +134,12 @@ r7c_bwd_pre_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* _
     fence_async_smem();
     tc_fence_before();
     ok = __syncthreads_and(ok);
-    if (tid == 0 && ok) {
+    if (warp == 0 && elect_one() && ok) {
       bulk_store(tiles + S_P2 * TILE_BYTES, sm.p2, TILE_BYTES);
       bulk_commit();
     }
   }
-  if (tid == 0) bulk_wait_all();
+  if (warp == 0 && elect_one()) bulk_wait_all();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tm, 128);
@@ -175,11 +175,11 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
   const int wq = warp & 3, hsel = warp >> 2, c0 = 32 * hsel;
   const int row = 16 * wq + (lane & 15);
   const bool state_lane = lane < 16;
-  // single-thread jobs side by side: thread 0 issues the MMAs (thread 96 one product of the first group, when
-  // the CTA has the SM to itself), st_thread copies dh^ and dz out (and waits for
-  // its own bulk-copy groups), ld_thread requests the operand tiles of the chunk after the next
-  // (they share the SM with a second CTA when there are more sequences than SMs, and then stay with thread 0)
-  const bool st_thread = tid == (spread ? 32 : 0), ld_thread = tid == (spread ? 64 : 0);
+  // single-thread jobs side by side: warp 0 issues the MMAs (warp 3 one product of the first group, when
+  // the CTA has the SM to itself), st_warp copies dh^ and dz out (and waits for
+  // its own bulk-copy groups), ld_warp requests the operand tiles of the chunk after the next
+  // (they share the SM with a second CTA when there are more sequences than SMs, and then stay with warp 0)
+  const int st_warp = spread ? 1 : 0, ld_warp = spread ? 2 : 0;
 
   if (tid == 0) {
     mbar_init(&sm.bar_full[0], 1); mbar_init(&sm.bar_full[1], 1);
@@ -204,7 +204,7 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
     bulk_load(s.qt, tiles + S_QT * TILE_BYTES, TILE_BYTES, &sm.bar_full[n & 1]);
     tma_load_4d(s.dout, &tmap_do, &sm.bar_full[n & 1], 0, tb + c * L, hi, brow);
   };
-  if (tid == 0) {
+  if (warp == 0 && elect_one()) {
     issue_loads(0);
     if (NT > 1) issue_loads(1);
   }
@@ -243,22 +243,22 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
       }
     }
     ok = tail_ok && mbar_wait(&sm.bar_full[n & 1], (n >> 1) & 1, status, 311);
-    if (st_thread) bulk_wait_read();    // the copy of the previous chunk's dz has left its tile, rewritten below
+    if (warp == st_warp && elect_one()) bulk_wait_read();    // the copy of the previous chunk's dz has left its tile, rewritten below
     fence_async_smem();
     tc_fence_before();
     ok = __syncthreads_and(ok);
-    if (tid == 0 && ok) {
+    if (warp == 0 && elect_one() && ok) {
       tc_fence_after();
       umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 0), smem_u32(s.b2), smem_u32(sm.dhh), false);   // B2 dh^
       if (!spread) umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 0), smem_u32(s.qt), smem_u32(s.dout), false);    // q~^T do
       umma_commit(&sm.bar_m1);
     }
-    if (spread && tid == 96 && ok) {
+    if (spread && warp == 3 && elect_one() && ok) {
       tc_fence_after();
       umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 0), smem_u32(s.qt), smem_u32(s.dout), false);    // q~^T do
       umma_commit(&sm.bar_m1);
     }
-    if (st_thread && ok) {
+    if (warp == st_warp && elect_one() && ok) {
       bulk_store(tiles + S_DHH * TILE_BYTES, sm.dhh, TILE_BYTES);
       bulk_commit();
     }
@@ -276,23 +276,23 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
         tile_store_row32(sm.dz, row, c0, x);
       }
     }
-    if (st_thread) bulk_wait_read();    // the copy of dh^ has left its tile, rewritten at the top of the next chunk
+    if (warp == st_warp && elect_one()) bulk_wait_read();    // the copy of dh^ has left its tile, rewritten at the top of the next chunk
     fence_async_smem();
     tc_fence_before();
     ok = __syncthreads_and(ok);
-    if (tid == 0 && ok) {
+    if (warp == 0 && elect_one() && ok) {
       tc_fence_after();
       umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 0), smem_u32(s.at), smem_u32(sm.dz), true);      // += a~^T dz
       umma_commit(&sm.bar_m2);
     }
-    if (st_thread && ok) {
+    if (warp == st_warp && elect_one() && ok) {
       bulk_store(tiles + S_DZ * TILE_BYTES, sm.dz, TILE_BYTES);
       bulk_commit();
     }
     tail_ok = ok && mbar_wait(&sm.bar_m2, n & 1, status, 313);
     tc_fence_after();
     // this stage has been read: p2 by every thread before the last barrier, the rest by the two MMA groups
-    if (ld_thread && tail_ok && n + 2 < NT) issue_loads(n + 2);
+    if (warp == ld_warp && elect_one() && tail_ok && n + 2 < NT) issue_loads(n + 2);
     if (tail_ok) {
       uint32_t r[32];
       tmem_ld32(tm_w, r);
@@ -310,7 +310,7 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
 #pragma unroll
     for (int vv = 0; vv < 32; ++vv) S[(c0 + vv) * 64 + row] = dh[vv];
   }
-  if (st_thread) bulk_wait_all();
+  if (warp == st_warp && elect_one()) bulk_wait_all();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tm, 64);
 }
@@ -373,8 +373,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
   }
 
   if (tid == 0) {
-    // an MMA group is issued by several threads, one accumulator each, and completes with the arrival of all: one
-    // thread issues an MMA about every 80 cycles, the tensor pipe takes them faster
+    // an MMA group is issued by several threads, one accumulator each, and completes with the arrival of all
     mbar_init(&sm.bar_l0, 1); mbar_init(&sm.bar_l1, 1); mbar_init(&sm.bar_l2, 1);
     mbar_init(&sm.bar_m1, 3); mbar_init(&sm.bar_m2, 2);
     fence_mbar_init();
@@ -384,7 +383,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
   __syncthreads();
   tc_fence_after();
   const uint32_t tm = sm.tmem_base;
-  const bool st_thread = tid == 96;      // requests the tiles, stores the results
+  constexpr int st_warp = 3;      // requests the tiles, stores the results
 
   // the tiles of a chunk-head in the order in which their space becomes free
   auto load_0 = [&](const ChunkPos& p) {      // dh^, v
@@ -418,7 +417,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
   auto prefetch_l2 = [&](const ChunkPos& p) {      // one warp
     const int t0 = p.c * L;
     const unsigned char* tiles = ws_tiles + (size_t)p.ch * tiles_per_chunk * TILE_BYTES;
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_4d(&tmap_do, 0, sv.first<PACKED>(p.bi) + t0, p.hi, sv.row<PACKED>(p.bi));
       tma_prefetch_4d(&tmap_v, 0, sv.first<PACKED>(p.bi) + t0, p.hi, sv.row<PACKED>(p.bi));
       bulk_prefetch_l2(tiles + S_QT * TILE_BYTES, 3 * TILE_BYTES);     // q~, k~, b~
@@ -452,7 +451,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
 
   uint4 rw[2];
   if (cur.ch < n_ch) {
-    if (st_thread) { load_0(cur); load_1a(cur); load_2(cur); load_1b(cur); }
+    if (warp == st_warp && elect_one()) { load_0(cur); load_1a(cur); load_2(cur); load_1b(cur); }
     load_w(cur, rw);
   }
 
@@ -494,7 +493,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     }
     R7C_STAMP(17);
     // ---- MMA group 1: all four dA products; dv; the state part of [dq~; da~]
-    if (lane == 0 && warp < 3) {
+    if (warp < 3 && elect_one()) {
       ok = mbar_wait(&sm.bar_l0, par, status, 321) && ok;
       ok = mbar_wait(&sm.bar_l1, par, status, 324) && ok;
       if (ok) {
@@ -601,7 +600,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     R7C_STAMP(20);
 
     // ---- MMA group 2: [dq~; da~] completed (columns 128..191), and [dk~; db~] (columns 0..63)
-    if (lane == 0 && warp < 2 && ok) {
+    if (warp < 2 && elect_one() && ok) {
       ok = mbar_wait(&sm.bar_l2, par, status, 326);
       if (ok) {
         tc_fence_after();
@@ -616,7 +615,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
         umma_commit(&sm.bar_m2);
       }
     }
-    if (st_thread && ok && !row_stores) {
+    if (warp == st_warp && elect_one() && ok && !row_stores) {
       tma_store_4d(&tmap_dv, sm.h0, 0, tt, hi, br);
       bulk_commit();
     }
@@ -627,7 +626,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     ok = mbar_wait(&sm.bar_l1, par, status, 328) && ok;
     tc_fence_after();
     R7C_STAMP(21);
-    if (st_thread && ok) {
+    if (warp == st_warp && elect_one() && ok) {
       if (more) load_0(nxt);      // dh^ and v have been read for the last time
       bulk_wait_read();           // the copy of dv has left its tile, which will hold dw
     }
@@ -693,7 +692,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
       store_tile_rows<256>(da_rows + out_base, lay.st, sm.at, Tn - t0, tid);
       store_tile_rows<256>(db_rows + out_base, lay.st, sm.bt, Tn - t0, tid);
     }
-    if (st_thread && ok && !row_stores) {
+    if (warp == st_warp && elect_one() && ok && !row_stores) {
       tma_store_4d(&tmap_dq, sm.qt, 0, tt, hi, br);
       tma_store_4d(&tmap_dk, sm.kt, 0, tt, hi, br);
       tma_store_4d(&tmap_da, sm.at, 0, tt, hi, br);
@@ -735,7 +734,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
       fence_async_smem();
       __syncthreads();      // the rows are read before their space is loaded again
     }
-    if (st_thread && ok) {
+    if (warp == st_warp && elect_one() && ok) {
       if (!row_stores) {
         tma_store_4d(&tmap_dw, sm.h0, 0, tt, hi, br);
         bulk_commit();
@@ -750,7 +749,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     }
     R7C_STAMP(23);
   }
-  if (st_thread) bulk_wait_all();
+  if (warp == st_warp && elect_one()) bulk_wait_all();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tm, 256);

@@ -130,7 +130,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
   };
   ChunkPos cur = chunk_pos(blockIdx.x, NT, H);
   if (cur.ch < n_ch && empty(cur)) cur = advance(cur);
-  if (cur.ch < n_ch && tid == 0) { load_w(cur); load_qkb(cur); load_a(cur); load_v(cur); }
+  if (cur.ch < n_ch && warp == 0 && elect_one()) { load_w(cur); load_qkb(cur); load_a(cur); load_v(cur); }
   // The two CTAs that share an SM would otherwise run their phases in lockstep and compete for the
   // same unit (shared-memory pipe during the triangular solve); start every other CTA half a
   // chunk-head late.
@@ -280,7 +280,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
 
     R7C_STAMP(2);
     // ---- MMA 1: [q~; a~] [k~; b~]^T  ->  TMEM columns 0..127, row r on lane r
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
       bulk_wait_read();      // the previous W, U copies are done: the epilogue below rewrites their tiles
       tc_fence_after();
       umma_tile<128, 128, 0, 0>(tm, smem_u32(sm.qt), smem_u32(sm.kt), false);
@@ -289,7 +289,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
     ok = mbar_wait(&sm.bar_m1, par, status, 201) && ok;
     tc_fence_after();
     R7C_STAMP(3);
-    if (tid == 0 && ok) {      // MMA 1 was the last reader of q~, k~, b~ in shared memory: copy them out now
+    if (warp == 0 && elect_one() && ok) {      // MMA 1 was the last reader of q~, k~, b~ in shared memory: copy them out now
       bulk_store(out_tiles + S_QT * TILE_BYTES, sm.qt, TILE_BYTES);
       bulk_store(out_tiles + S_KT * TILE_BYTES, sm.kt, TILE_BYTES);
       bulk_store(out_tiles + S_BT * TILE_BYTES, sm.bt, TILE_BYTES);
@@ -346,7 +346,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
 
     R7C_STAMP(4);
     // ---- MMA 2: [A_qk; A_ak] v  ->  TMEM columns 128..191 (rows 0..63 = O1, 64..127 = Y)
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
       ok = mbar_wait(&sm.bar_v, par, status, 202) && ok;
       tc_fence_after();
       umma_tile<128, 64, 0, 1>(tmem_addr(tm, 0, 128), smem_u32(sm.aqk), smem_u32(sm.v), false);
@@ -418,7 +418,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
       }
       // the scratch area: MMA 2 (and the copies of A_qk / A_ak kept for the backward) must be done with it
       ok = mbar_wait(&sm.bar_m2, par, status, 205) && ok;
-      if (tid == 0) {
+      if (warp == 0 && elect_one()) {
         bulk_wait_read();                  // q~, k~, b~ (and the tiles kept for the backward) have left shared memory
         if (next < n_ch) { load_v(nxt); load_qkb(nxt); }      // MMA 2 has read the v tile; nothing reads q~, k~, b~ any more
       }
@@ -484,7 +484,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
       tc_fence_before();
       __syncthreads();
       R7C_STAMP(12);
-      if (tid == 0) {
+      if (warp == 0 && elect_one()) {
         tc_fence_after();
         umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 128), smem_u32(sm.aqk), smem_u32(sm.ainv), false);     // T = Q P
         umma_commit(&sm.bar_m4);
@@ -505,7 +505,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
       fence_async_smem();
       tc_fence_before();
       ok = __syncthreads_and(ok);
-      if (tid == 0 && ok) {
+      if (warp == 0 && elect_one() && ok) {
         tc_fence_after();
         umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 128), smem_u32(sm.ainv), smem_u32(sm.aak), false);     // P T
         umma_commit(&sm.bar_m5);
@@ -532,7 +532,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
 
     R7C_STAMP(6);
     // ---- MMA 3: W = Ainv a~ (lower lane halves), U = Ainv Y (upper lane halves) -> TMEM columns 0..63
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
       if (ok && next < n_ch) load_w(nxt);      // the scratch area in the A_qk tile is free again
       tc_fence_after();
       umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 0), smem_u32(sm.ainv), smem_u32(sm.at), false);
@@ -563,7 +563,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
     tc_fence_before();
     ok = __syncthreads_and(ok);
     R7C_STAMP(8);
-    if (tid == 0 && ok) {
+    if (warp == 0 && elect_one() && ok) {
       bulk_store(out_tiles + S_W * TILE_BYTES, sm.aak, TILE_BYTES);
       bulk_store(out_tiles + S_U * TILE_BYTES, sm.y, TILE_BYTES);
       bulk_commit();
@@ -572,7 +572,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
     }
     R7C_STAMP(9);
   }
-  if (tid == 0) bulk_wait_all();
+  if (warp == 0 && elect_one()) bulk_wait_all();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tm, 256);
@@ -636,21 +636,18 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
   const int NT = (Tn + L - 1) / L;           // chunks of this sequence (at least one)
   const int row = 16 * wq + (lane & 15);     // state row k (lanes 0-15) or token row i (lanes 16-31)
   const bool state_lane = lane < 16;
-  // With one CTA per SM the single-thread jobs of a chunk lie on the chain from chunk to chunk, and each
-  // bulk copy costs its issuing thread about a hundred cycles: they go to the first threads of four warps and
-  // run side by side (-12 % per chunk).  Thread 0 issues the MMAs (with the first threads of warps 1 and 2, one
-  // accumulator each), ld_thread requests operand tiles,
-  // st_thread copies sa and h~0 out for the backward, out_thread copies X and the output rows out.  Bulk-copy
+  // With one CTA per SM the single-thread jobs of a chunk lie on the chain from chunk to chunk: they go to one thread of
+  // each of four warps and run side by side.  Warps 0, 1 and 2 issue the MMAs, one accumulator each, ld_warp requests
+  // operand tiles, st_warp copies sa and h~0 out for the backward, out_warp copies X and the output rows out.  Bulk-copy
   // groups belong to the thread that committed them, so each storing thread waits for its own copies.  With
-  // two CTAs per SM the other CTA fills such gaps and thread 0 keeps all four jobs.
+  // two CTAs per SM the other CTA fills such gaps and warp 0 keeps all four jobs.
   constexpr bool SPREAD = STAGES == 2;
-  const bool ld_thread = tid == (SPREAD ? 32 : 0), st_thread = tid == (SPREAD ? 64 : 0),
-             out_thread = tid == (SPREAD ? 96 : 0);
+  constexpr int ld_warp = SPREAD ? 1 : 0, st_warp = SPREAD ? 2 : 0, out_warp = SPREAD ? 3 : 0;
 
   if (tid == 0) {
     for (int i = 0; i < STAGES; ++i) { mbar_init(&sm.bar_g1[i], 1); mbar_init(&sm.bar_g2[i], 1); }
-    // with one CTA per SM each accumulator of an MMA group has its own issuing thread (one thread issues an
-    // MMA about every 80 cycles, the tensor pipe takes them faster), and a group completes with all arrivals
+    // with one CTA per SM each accumulator of an MMA group has its own issuing thread, and a group completes with all
+    // arrivals
     mbar_init(&sm.bar_a, SPREAD ? 3 : 1); mbar_init(&sm.bar_c, SPREAD ? 2 : 1);
     fence_mbar_init();
   }
@@ -661,7 +658,7 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
   const uint32_t tm = sm.tmem_base;
   const uint32_t tm_p1 = tmem_addr(tm, 32 * wq, c0), tm_p2 = tmem_addr(tm, 32 * wq, 64 + c0);
 
-  auto issue_g1 = [&](int c) {      // ld_thread (thread 0 for the first chunks)
+  auto issue_g1 = [&](int c) {      // ld_warp (warp 0 for the first chunks)
     const unsigned char* tiles = ws_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES;
     ScanGroup1<STAGES>& g = sm.g1[c % STAGES];
     uint64_t* bar = &sm.bar_g1[c % STAGES];
@@ -671,13 +668,13 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
     else                       bulk_load(g.w, tiles + S_W * TILE_BYTES, TILE_BYTES, bar);
     tma_load_4d(g.v, &tmap_v, bar, 0, tb + c * L, hi, brow);
   };
-  auto issue_g2 = [&](int c) {      // ld_thread (thread 0 for the first chunks)
+  auto issue_g2 = [&](int c) {      // ld_warp (warp 0 for the first chunks)
     const unsigned char* tiles = ws_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES;
     uint64_t* bar = &sm.bar_g2[c % STAGES];
     mbar_expect_tx(bar, 2 * TILE_BYTES);
     bulk_load(sm.g2[c % STAGES].bt, tiles + S_BT * TILE_BYTES, 2 * TILE_BYTES, bar);
   };
-  if (tid == 0) {
+  if (warp == 0 && elect_one()) {
     for (int c = 0; c < STAGES && c < NT; ++c) { issue_g1(c); issue_g2(c); }
   }
 
@@ -725,7 +722,7 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
       if (c + 1 < NT) scale_next = ws_aux[(ch0 + c + 1) * AUX_FLOATS + row];    // e^{gref} of the next chunk
     }
     // (a) SA = W h~0, QH = q~ h~0 (P1);  H += k~^T v (P2 lower)
-    if (lane == 0 && warp < (SPREAD ? 3 : 1)) {
+    if (warp < (SPREAD ? 3 : 1) && elect_one()) {
       ScanGroup1<STAGES>& g = sm.g1[c % STAGES];
       ok = mbar_wait(&sm.bar_g1[c % STAGES], (c / STAGES) & 1, status, 211);
       R7C_STAMP(49);
@@ -741,7 +738,7 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
     tc_fence_after();
     R7C_STAMP(50);
     // group 1 has been read by the MMAs: request the next (the staged O1 / U rows are still to be read)
-    if (STAGES == 1 && ld_thread && ok && c + STAGES < NT) issue_g1(c + STAGES);
+    if (STAGES == 1 && warp == ld_warp && elect_one() && ok && c + STAGES < NT) issue_g1(c + STAGES);
     float keep[32];     // token lanes: q~ h~0 + O1
     if constexpr (STAGES == 2) {      // the staged O1 / U rows: observe the arrival of group 1 before reading them
       ok = ok && mbar_wait(&sm.bar_g1[c % STAGES], (c / STAGES) & 1, status, 215);
@@ -769,8 +766,8 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
     fence_async_smem();
     tc_fence_before();
     ok = __syncthreads_and(ok);
-    if (STAGES == 2 && ld_thread && ok && c + STAGES < NT) issue_g1(c + STAGES);
-    if (bwd_tiles && st_thread && ok) {   // the backward needs sa and h~0 of every chunk
+    if (STAGES == 2 && warp == ld_warp && elect_one() && ok && c + STAGES < NT) issue_g1(c + STAGES);
+    if (bwd_tiles && warp == st_warp && elect_one() && ok) {   // the backward needs sa and h~0 of every chunk
       unsigned char* dst = bwd_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES;
       bulk_store(dst + S_SA * TILE_BYTES, sm.sa, TILE_BYTES);
       bulk_store(dst + S_H0 * TILE_BYTES, sm.ht, TILE_BYTES);
@@ -778,7 +775,7 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
     }
     // (c) H += b~^T sa (P2 lower);  OQ = A_qb sa (P2 upper)
     R7C_STAMP(51);
-    if (lane == 0 && warp < (SPREAD ? 2 : 1) && ok) {
+    if (warp < (SPREAD ? 2 : 1) && elect_one() && ok) {
       ScanGroup2& g = sm.g2[c % STAGES];
       ok = mbar_wait(&sm.bar_g2[c % STAGES], (c / STAGES) & 1, status, 214);
       R7C_STAMP(52);
@@ -792,9 +789,9 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
     ok = ok && mbar_wait(&sm.bar_c, c & 1, status, 213);
     tc_fence_after();
     R7C_STAMP(53);
-    if (ld_thread && ok && c + STAGES < NT) issue_g2(c + STAGES);     // group 2 has been read
+    if (warp == ld_warp && elect_one() && ok && c + STAGES < NT) issue_g2(c + STAGES);     // group 2 has been read
     if (bwd_tiles) {                                  // ht / sa are rewritten below and in the next chunk
-      if (st_thread) bulk_wait_read();
+      if (warp == st_warp && elect_one()) bulk_wait_read();
       __syncthreads();
     }
     R7C_STAMP(54);
@@ -831,7 +828,7 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
     tc_fence_before();
     ok = __syncthreads_and(ok);
     R7C_STAMP(55);
-    if (bwd_tiles && out_thread && ok) {
+    if (bwd_tiles && warp == out_warp && elect_one() && ok) {
       bulk_store(bwd_tiles + ((ch0 + c) * (size_t)tiles_per_chunk + S_X) * TILE_BYTES, sm.xt, TILE_BYTES);
       bulk_commit();
     }
@@ -839,7 +836,7 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
       if (PACKED && t0 + L > Tn) {  // the last rows of the box belong to the next sequence: row by row
         store_tile_rows<256>(o_rows + brow * lay.sb + hi * lay.sh + (long long)(tb + t0) * lay.st, lay.st,
                              sm.ot[c & 1], Tn - t0, tid);
-      } else if (out_thread) {           // rows past the end of the tensor are clipped by the TMA store
+      } else if (warp == out_warp && elect_one()) {           // rows past the end of the tensor are clipped by the TMA store
         tma_store_4d(&tmap_o, sm.ot[c & 1], 0, tb + t0, hi, brow);
         bulk_commit();
         bulk_wait_read_1();              // the buffer of the previous chunk is free again
@@ -848,7 +845,7 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
     R7C_STAMP(56);
   }
 #undef R7C_STAMP
-  if (st_thread || out_thread) bulk_wait_all();
+  if ((warp == st_warp || warp == out_warp) && elect_one()) bulk_wait_all();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tm, 128);
 }

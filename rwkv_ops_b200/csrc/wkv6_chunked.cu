@@ -282,7 +282,7 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     tma_load_4d(sm.rt[0], &tmap_r, &sm.bar_in, 0, tok0 + c * L, hi, brow);
     tma_load_4d(sm.kt[0], &tmap_k, &sm.bar_in, 0, tok0 + c * L, hi, brow);
   };
-  if (tid == 0 && ok && c_lo < c_hi) load_in(c_lo);
+  if (warp == 0 && elect_one() && ok && c_lo < c_hi) load_in(c_lo);
 
   for (int c = c_lo; c < c_hi && ok; ++c, ++n_done) {
     const int t0 = c * L;
@@ -379,7 +379,7 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
       if (c4 == 0) sm.dgs[row] = dg;
     }
     // ask for the next chunk's rows to be brought into L2 while this chunk is in its MMA phases
-    if (tid == 0 && c + 1 < c_hi) {
+    if (warp == 0 && elect_one() && c + 1 < c_hi) {
       tma_prefetch_4d(&tmap_w, 0, tok0 + t0 + L, hi, brow);
       tma_prefetch_4d(&tmap_v, 0, tok0 + t0 + L, hi, brow);
       tma_prefetch_4d(&tmap_r, 0, tok0 + t0 + L, hi, brow);
@@ -391,7 +391,7 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
 
     W6C_STAMP(4);
     // ---- batch 1: r~ k~^T (columns 0..63), y = r~ S~0 (columns 64.., lower), k~^T v (upper)
-    if (lane == 0 && warp < 3) {
+    if (warp < 3 && elect_one()) {
       tc_fence_after();
       if (warp == 0)      umma_split<64, 64, 0, 0>(tmem_addr(tm, 0, 0), smem_u32(sm.rt[0]), smem_u32(sm.kt[0]), false);
       else if (warp == 1) umma_split<64, 64, 0, 1>(tmem_addr(tm, 0, 64), smem_u32(sm.rt[0]), smem_u32(sm.st[0]), false);
@@ -419,7 +419,7 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
 
     W6C_STAMP(6);
     // ---- batch 2: y += A v
-    if (tid == 0 && ok) {
+    if (warp == 0 && elect_one() && ok) {
       tc_fence_after();
       umma_split<64, 64, 0, 1>(tmem_addr(tm, 0, 64), smem_u32(sm.at[0]), smem_u32(sm.vt[0]), true);
       umma_commit(&sm.bar_2);
@@ -427,7 +427,7 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     ok = mbar_wait(&sm.bar_2, par, status, 402) && ok;
     tc_fence_after();
     W6C_STAMP(7);
-    if (tid == 0 && ok && c + 1 < c_hi) load_in(c + 1);      // the tiles of this chunk have been read for the last time
+    if (warp == 0 && elect_one() && ok && c + 1 < c_hi) load_in(c + 1);      // the tiles of this chunk have been read for the last time
     if (ok) {
       uint32_t rr[32];
       tmem_ld32(tm_ys, rr);
@@ -481,7 +481,7 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   if (!last_part) {
     __threadfence();
     __syncthreads();
-    if (tid == 0 && ok)
+    if (warp == 0 && elect_one() && ok)
       asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(handoff_flags + unit), "r"(part + 1) : "memory");
   }
   __syncthreads();      // the tiles and next_item are the next item's
@@ -559,7 +559,7 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
 
   if (tid == 0) {
     // every MMA batch is issued by two threads (threads 0 and 32, each with accumulators of its own) and completes
-    // with the arrival of both: one thread issues an MMA about every 55 cycles, the tensor pipe takes them faster
+    // with the arrival of both
     mbar_init(&sm.bar_1, 2); mbar_init(&sm.bar_2, 2); mbar_init(&sm.bar_2a, 2);
     mbar_init(&sm.bar_in_a, 1); mbar_init(&sm.bar_in_b, 1); mbar_init(&sm.bar_in_c, 1);
     fence_mbar_init();
@@ -670,7 +670,7 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     mbar_expect_tx(&sm.bar_in_c, RAW_BYTES);
     tma_load_4d(sm.red_e, &tmap_v, &sm.bar_in_c, 0, tok0 + c * L, hi, brow);
   };
-  if (tid == 0 && ok) { load_in_a(c_hi); load_in_c(c_hi); load_in_b(c_hi); }
+  if (warp == 0 && elect_one() && ok) { load_in_a(c_hi); load_in_c(c_hi); load_in_b(c_hi); }
 
   for (int c = c_hi; c >= c_lo && ok; --c, ++n_done) {
     const int t0 = c * L;
@@ -738,7 +738,7 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
       if (c4 == 0) sm.dds[row] = dd;
     }
     __syncthreads();
-    if (tid == 0 && ok && c > c_lo) load_in_a(c - 1);      // every thread has taken its w and dy elements
+    if (warp == 0 && elect_one() && ok && c > c_lo) load_in_a(c - 1);      // every thread has taken its w and dy elements
 #pragma unroll
     for (int n = 0; n < 4; ++n) {
       const int e = tid + 256 * n, row = e >> 4;
@@ -763,7 +763,7 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
 #pragma unroll
       for (int j = 0; j < 8; ++j) srow4[j] = *reinterpret_cast<const float4*>(Srow + 4 * j);
     }
-    if (tid == 0 && c > c_lo) {   // bring the previous chunk's rows into L2 while this chunk is in its MMA phases
+    if (warp == 0 && elect_one() && c > c_lo) {   // bring the previous chunk's rows into L2 while this chunk is in its MMA phases
       tma_prefetch_4d(&tmap_w, 0, tok0 + t0 - L, hi, brow);
       tma_prefetch_4d(&tmap_dy, 0, tok0 + t0 - L, hi, brow);
       tma_prefetch_4d(&tmap_v, 0, tok0 + t0 - L, hi, brow);
@@ -778,12 +778,12 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
 
     W6C_STAMP(36);
     // ---- batch 1: r~ k~^T (lower halves) and dy v^T (upper halves), columns 0..63
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
       tc_fence_after();
       umma_split<64, 64, 0, 0>(tmem_addr(tm, 0, 0), smem_u32(sm.rt[0]), smem_u32(sm.kt[0]), false);
       umma_commit(&sm.bar_1);
     }
-    if (tid == 32) {
+    if (warp == 1 && elect_one()) {
       tc_fence_after();
       umma_split<64, 64, 0, 0>(tmem_addr(tm, 16, 0), smem_u32(sm.dyt[0]), smem_u32(sm.vt[0]), false);
       umma_commit(&sm.bar_1);
@@ -833,7 +833,7 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     // ---- batch 2, committed in two parts: the products the heavier part of the read-out needs first, so that its
     // arithmetic runs while the tensor pipe works on the rest (its results stay in registers until then: the
     // staging arrays lie over operand tiles of the products still running)
-    if (tid == 0 && ok) {
+    if (warp == 0 && elect_one() && ok) {
       tc_fence_after();
       // dr~ = dy S~0^T + stril(dA) k~               (upper halves, columns 64..127)
       umma_split<64, 64, 0, 0>(tmem_addr(tm, 16, 64), smem_u32(sm.dyt[0]), smem_u32(sm.st[0]), false);
@@ -844,7 +844,7 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
       umma_split<64, 64, 0, 1>(tmem_addr(tm, 0, 128), smem_u32(sm.kt[0]), smem_u32(sm.dst[0]), true);
       umma_commit(&sm.bar_2);
     }
-    if (tid == 32 && ok) {
+    if (warp == 1 && elect_one() && ok) {
       tc_fence_after();
       // the part of dk~ from inside the chunk, stril(dA)^T r~   (lower halves, columns 64..127: beside dr~, so
       // that one piece of code scales both in the epilogue)
@@ -921,7 +921,7 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     }
     tc_fence_before();
     ok = __syncthreads_and(ok);
-    if (tid == 0 && ok && c > c_lo) load_in_b(c - 1);      // the epilogue above was the last reader of rt / kt
+    if (warp == 0 && elect_one() && ok && c > c_lo) load_in_b(c - 1);      // the epilogue above was the last reader of rt / kt
     W6C_STAMP(40);
     // ---- decay gradient, with I_i = -(stril(dA)^T r~)_i k~_i and X_i k~_i the two parts of dgi_i = -dk~_i k~_i:
     // dg_j = sum_{i>j} (dge_i + I_i) + I_j + sum_v dS^ S~0 + sum_{i<j} X_i k~_i;   dw = dg g.
@@ -955,7 +955,7 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
       }
     }
     __syncthreads();
-    if (tid == 0 && ok && c > c_lo) load_in_c(c - 1);      // red_e has been read for the last time
+    if (warp == 0 && elect_one() && ok && c > c_lo) load_in_c(c - 1);      // red_e has been read for the last time
     W6C_STAMP(41);
     // ---- outputs, coalesced, plus the u-term parts of dr, dk and du
 #pragma unroll
@@ -998,7 +998,7 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   if (hand_on) {
     __threadfence();
     __syncthreads();
-    if (tid == 0 && ok) asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(handoff_flags + unit), "r"(1) : "memory");
+    if (warp == 0 && elect_one() && ok) asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(handoff_flags + unit), "r"(1) : "memory");
   }
   __syncthreads();      // du_s and the tiles are the next item's
   }   // items
