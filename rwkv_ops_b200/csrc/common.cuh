@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/rwkv_ops_b200.h"
 
 namespace rwkvb200 {
@@ -107,6 +109,22 @@ inline int cuda_ok(cudaError_t e) {
 }
 
 inline int check_launch() { return cuda_ok(cudaGetLastError()); }
+
+// What a launch needs to know about the current device, asked once per device (tc_host.cu): a call launches up to nine
+// kernels, and the attribute queries and settings between them were a third of its host time.
+struct DeviceFacts { int dev, sms; int* status; };      // status: the device status word of the kernels' bounded waits
+int device_facts(DeviceFacts* out);
+
+// Allow `Kernel` its dynamic shared memory, once per device.
+template <auto Kernel>
+int allow_smem(const DeviceFacts& f, int bytes) {
+  static std::atomic<uint64_t> done{0};
+  const uint64_t bit = uint64_t(1) << f.dev;
+  if (done.load(std::memory_order_acquire) & bit) return RWKVB200_OK;
+  if (cuda_ok(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes))) return RWKVB200_E_CUDA;
+  done.fetch_or(bit, std::memory_order_release);
+  return RWKVB200_OK;
+}
 
 // Brackets one kernel launch with timing events when profiling is on (see profile.cu).
 struct ProfScope {

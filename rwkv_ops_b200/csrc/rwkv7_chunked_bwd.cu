@@ -232,7 +232,7 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
     const int c = NT - 1 - n;
     BScanStage& s = sm.st[n & 1];
     unsigned char* tiles = ws_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES;
-    const float dc = dc_next, e0 = e0_next;
+    const float dc = fabsf(dc_next), e0 = e0_next;
     if (state_lane) {
 #pragma unroll
       for (int vv = 0; vv < 32; ++vv) dh[vv] *= dc;      // dh^ = e^{glast-gref} dh_L
@@ -832,8 +832,10 @@ int launch_rwkv7_chunked_bwd(const void* r, const void* w, const void* k, const 
                                  true, st, seq_start, seq_len, T_total, fused);
     if (e) return e;
   }
-  int* status = device_status_ptr();
-  if (!status) { last_cuda_error_slot() = 99999; return RWKVB200_E_CUDA; }
+  DeviceFacts dev;
+  e = device_facts(&dev);
+  if (e) return e;
+  int* status = dev.status;
   CUtensorMap tmap_do, tmap_v, tmap_out[6];
   const SeqView sv{seq_start, seq_len, Tn};
   const int mapB = seq_start ? 1 : B, mapT = seq_start ? T_total : Tn;   // shape of the token tensors
@@ -853,27 +855,21 @@ int launch_rwkv7_chunked_bwd(const void* r, const void* w, const void* k, const 
 #define R7C_DISPATCH_PACKED(...) do { if (seq_start) { constexpr bool P = true; __VA_ARGS__; } else { constexpr bool P = false; __VA_ARGS__; } } while (0)
   if (phases & PHASE_PREPARE) {
     const int smem = (int)sizeof(PreSmem) + 1024;
-    int dev = 0, sms = 0;
-    if (cuda_ok(cudaGetDevice(&dev)) || cuda_ok(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)))
-      return RWKVB200_E_CUDA;
+    const int sms = dev.sms;
     const int pre_grid = B * H * NT < 2 * sms ? B * H * NT : 2 * sms;     // persistent: two CTAs per SM
     ProfScope prof("r7c_bwd_pre_kernel", st);
     R7C_DISPATCH_PACKED(
-      if (cuda_ok(cudaFuncSetAttribute(r7c_bwd_pre_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)))
-        return RWKVB200_E_CUDA;
+      if (allow_smem<r7c_bwd_pre_kernel<P>>(dev, smem)) return RWKVB200_E_CUDA;
       r7c_bwd_pre_kernel<P><<<pre_grid, 128, smem, st>>>(tmap_do, ws.tiles, ALL_TILES, sv, H, NT, B * H * NT, status));
   }
   e = check_launch();
   if (e) return e;
   if (phases & PHASE_SCAN) {
     const int smem = (int)sizeof(BScanSmem) + 1024;
-    int dev = 0, sms = 0;
-    if (cuda_ok(cudaGetDevice(&dev)) || cuda_ok(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)))
-      return RWKVB200_E_CUDA;
+    const int sms = dev.sms;
     ProfScope prof("r7c_bwd_scan_kernel", st);
     R7C_DISPATCH_PACKED(
-      if (cuda_ok(cudaFuncSetAttribute(r7c_bwd_scan_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)))
-        return RWKVB200_E_CUDA;
+      if (allow_smem<r7c_bwd_scan_kernel<P>>(dev, smem)) return RWKVB200_E_CUDA;
       r7c_bwd_scan_kernel<P><<<B * H, 256, smem, st>>>(tmap_do, ws.tiles, ws.aux, ALL_TILES, d_ht, d_h0, sv, H, NT,
                                                        B * H <= sms ? 1 : 0, status));
   }
@@ -904,13 +900,11 @@ int launch_rwkv7_chunked_bwd(const void* r, const void* w, const void* k, const 
     const int smem = (int)sizeof(FinalSmem);
     ProfScope prof("r7c_bwd_final_kernel", st);
     const int n_ch = B * H * NT;
-    int dev = 0, sms = 0;
-    if (cuda_ok(cudaGetDevice(&dev)) || cuda_ok(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)))
-      return RWKVB200_E_CUDA;
+    const int sms = dev.sms;
     const int grid = n_ch < 2 * sms ? n_ch : 2 * sms;     // persistent: two CTAs per SM
 #define R7C_LAUNCH_FINAL(P, F)                                                                                    \
     do {                                                                                                          \
-      if (cuda_ok(cudaFuncSetAttribute(r7c_bwd_final_kernel<P, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem))) \
+      if (allow_smem<r7c_bwd_final_kernel<P, F>>(dev, smem)) \
         return RWKVB200_E_CUDA;                                                                                   \
       r7c_bwd_final_kernel<P, F><<<grid, 256, smem, st>>>((const bf16*)w, tmap_do, tmap_v, ws.tiles, ALL_TILES,   \
           tmap_out[0], tmap_out[1], tmap_out[2], tmap_out[3], tmap_out[4], tmap_out[5], (bf16*)dr, (bf16*)dw,     \

@@ -47,7 +47,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
                      const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_a,
                      const __grid_constant__ CUtensorMap tmap_b,
                      const __grid_constant__ CUtensorMap tmap_v, unsigned char* __restrict__ ws_tiles,
-                     float* __restrict__ ws_aux, int* __restrict__ ws_flags, int tiles_per_chunk,
+                     float* __restrict__ ws_aux, int tiles_per_chunk,
                      int keep_for_bwd, SeqView sv, int H, int NT, int n_ch, TokLayout lay, int* status, long long* dbg) {
 #ifdef RWKVB200_DEVTOOLS
 #define R7C_STAMP(n) do { if (dbg && tid == 0 && blockIdx.x == gridDim.x / 2 && it == 30) dbg[n] = clock64(); } while (0)
@@ -133,8 +133,8 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
   if (cur.ch < n_ch && warp == 0 && elect_one()) { load_w(cur); load_qkb(cur); load_a(cur); load_v(cur); }
   // The two CTAs that share an SM would otherwise run their phases in lockstep and compete for the
   // same unit (shared-memory pipe during the triangular solve); start every other CTA half a
-  // chunk-head late.
-  if (blockIdx.x & 1) __nanosleep(6000);
+  // chunk-head late (unless it has a single one to do, or none: then the delay would be all it adds).
+  if ((blockIdx.x & 1) && n_ch > 2 * (int)gridDim.x) __nanosleep(6000);
 
   bool ok = true;
   int it = 0;
@@ -201,9 +201,10 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
       if (tid < 64) {
         const float tot0 = sm.qtot[0][tid] + sm.qtot[1][tid], tot1 = sm.qtot[2][tid] + sm.qtot[3][tid];
         ws_aux[(size_t)ch * AUX_FLOATS + tid] = ex2(fmaxf(tot0, EXP2_FLOOR));        // e^{gref}
-        ws_aux[(size_t)ch * AUX_FLOATS + 64 + tid] = ex2(fmaxf(tot1, EXP2_FLOOR));   // e^{glast-gref}
-        // a half-chunk decay sum beyond the limit: the unit is recomputed by the float32 recurrence
-        if (fminf(tot0, tot1) < -DECAY_LIMIT * LOG2E || Tn < SHORT_SEQ) ws_flags[bi * H + hi] = 1;
+        // a half-chunk decay sum beyond the limit: the unit is recomputed by the float32 recurrence.  The mark is the
+        // factor's sign; the scan, which reads every factor of its unit anyway, gathers it into Workspace::flags.
+        const bool mark = fminf(tot0, tot1) < -DECAY_LIMIT * LOG2E || Tn < SHORT_SEQ;
+        ws_aux[(size_t)ch * AUX_FLOATS + 64 + tid] = copysignf(ex2(fmaxf(tot1, EXP2_FLOOR)), mark ? -1.f : 1.f);   // e^{glast-gref}
       }
       // the raw q, k, a, b: each thread scales its own 2 x 16 bytes in place (the previous chunk-head's W, U,
       // A_qb, O1 copies may still be reading their tiles: those are rewritten only after MMA 1)
@@ -616,7 +617,8 @@ struct ScanSmem {
 template <int STAGES, bool PACKED>
 __global__ void __launch_bounds__(256, 3 - STAGES)
 r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned char* __restrict__ ws_tiles,
-                    const float* __restrict__ ws_aux, int tiles_per_chunk, unsigned char* __restrict__ bwd_tiles,
+                    const float* __restrict__ ws_aux, int* __restrict__ ws_flags, int tiles_per_chunk,
+                    unsigned char* __restrict__ bwd_tiles,
                     const float* __restrict__ h0, int n_state, const __grid_constant__ CUtensorMap tmap_o,
                     int write_o, float* __restrict__ ht, bf16* __restrict__ o_rows, SeqView sv, int H, int NT_slots,
                     TokLayout lay, int* status, long long* dbg) {
@@ -703,6 +705,7 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
   __syncthreads();
 
   bool ok = true;
+  int marked = 0;       // a chunk's decay left the range of the scaled operands (the sign of its factors)
   for (int c = 0; c < NT && ok; ++c) {
     const int t0 = c * L;
     R7C_STAMP(48);
@@ -807,8 +810,10 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
           for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(r[j]);
           tile_store_row32(sm.xt, row, c0, x);
         }
+        marked |= scale < 0.f;
+        const float sc = fabsf(scale);
 #pragma unroll
-        for (int j = 0; j < 32; ++j) { x[j] = (__uint_as_float(r[j]) * scale) * scale_next; r[j] = __float_as_uint(x[j]); }
+        for (int j = 0; j < 32; ++j) { x[j] = (__uint_as_float(r[j]) * sc) * scale_next; r[j] = __float_as_uint(x[j]); }
         if (!last) {
           tile_store_row32(sm.ht, row, c0, x);
         } else if (ht) {
@@ -846,7 +851,8 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
   }
 #undef R7C_STAMP
   if ((warp == st_warp || warp == out_warp) && elect_one()) bulk_wait_all();
-  __syncthreads();
+  marked = __syncthreads_or(marked);
+  if (tid == 0) ws_flags[unit] = marked;
   if (warp == 0) tmem_dealloc(tm, 128);
 }
 
@@ -861,10 +867,12 @@ int launch_rwkv7_chunked_fwd(const void* r, const void* w, const void* k, const 
   if (fused && seq_start) return RWKVB200_E_UNSUPPORTED;
   const SeqView sv{seq_start, seq_len, Tn};
   const int mapB = seq_start ? 1 : B, mapT = seq_start ? T_total : Tn;   // shape of the token tensors
-  int* status = device_status_ptr();
-  if (!status) { last_cuda_error_slot() = 99999; return RWKVB200_E_CUDA; }
+  DeviceFacts dev;
+  int e = device_facts(&dev);
+  if (e) return e;
+  int* status = dev.status;
   CUtensorMap tmap_v, tmap_o;
-  int e = make_token_tensor_map(&tmap_v, v, mapB, mapT, H, head_first);
+  e = make_token_tensor_map(&tmap_v, v, mapB, mapT, H, head_first);
   if (e) return e;
   e = make_token_tensor_map(&tmap_o, o ? o : v, mapB, mapT, H, head_first);   // unused when o is NULL
   if (e) return e;
@@ -879,21 +887,18 @@ int launch_rwkv7_chunked_fwd(const void* r, const void* w, const void* k, const 
   Workspace ws = carve(workspace, B, Tn, H, tpc);
   TokLayout lay(mapT, H, head_first);
   if (phases & PHASE_PREPARE) {
-    if (cuda_ok(cudaMemsetAsync(ws.flags, 0, (size_t)B * H * sizeof(int), st))) return RWKVB200_E_CUDA;
     const int smem = (int)sizeof(IntraSmem) + 1024;
     ProfScope prof("r7c_intra_fwd_kernel", st);
     const int n_ch = B * H * NT;
-    int dev = 0, sms = 0;
-    if (cuda_ok(cudaGetDevice(&dev)) || cuda_ok(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)))
-      return RWKVB200_E_CUDA;
+    const int sms = dev.sms;
     const int grid = n_ch < 2 * sms ? n_ch : 2 * sms;     // persistent: two CTAs per SM
 #define R7C_LAUNCH_INTRA(P, F)                                                                                     \
     do {                                                                                                           \
-      if (cuda_ok(cudaFuncSetAttribute(r7c_intra_fwd_kernel<P, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem))) \
+      if (allow_smem<r7c_intra_fwd_kernel<P, F>>(dev, smem)) \
         return RWKVB200_E_CUDA;                                                                                    \
       r7c_intra_fwd_kernel<P, F><<<grid, 256, smem, st>>>((const bf16*)r, (const bf16*)w, (const bf16*)k,         \
           (const bf16*)a, (const bf16*)b, tmap_in[0], tmap_in[1], tmap_in[2], tmap_in[3], tmap_in[4], tmap_v,      \
-          ws.tiles, ws.aux, ws.flags, tpc, keep_for_bwd ? 1 : 0, sv, H, NT, n_ch, lay, status,                    \
+          ws.tiles, ws.aux, tpc, keep_for_bwd ? 1 : 0, sv, H, NT, n_ch, lay, status,                              \
           debug_stamp_buffer());                                                                                   \
     } while (0)
     if (seq_start) R7C_LAUNCH_INTRA(true, false);
@@ -904,17 +909,15 @@ int launch_rwkv7_chunked_fwd(const void* r, const void* w, const void* k, const 
   e = check_launch();
   if (e || !(phases & PHASE_SCAN)) return e;
   {
-    int dev = 0, sms = 0;
-    if (cuda_ok(cudaGetDevice(&dev)) || cuda_ok(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)))
-      return RWKVB200_E_CUDA;
+    const int sms = dev.sms;
     ProfScope prof("r7c_scan_fwd_kernel", st);
     // more sequences than SMs: two single-buffered CTAs per SM; else one double-buffered CTA per SM
 #define R7C_LAUNCH_SCAN(S, P)                                                                                      \
     do {                                                                                                           \
       const int smem = (int)sizeof(ScanSmem<S>) + 1024;                                                            \
-      if (cuda_ok(cudaFuncSetAttribute(r7c_scan_fwd_kernel<S, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem))) \
+      if (allow_smem<r7c_scan_fwd_kernel<S, P>>(dev, smem)) \
         return RWKVB200_E_CUDA;                                                                                    \
-      r7c_scan_fwd_kernel<S, P><<<B * H, 256, smem, st>>>(tmap_v, ws.tiles, ws.aux, tpc,                           \
+      r7c_scan_fwd_kernel<S, P><<<B * H, 256, smem, st>>>(tmap_v, ws.tiles, ws.aux, ws.flags, tpc,                 \
           keep_for_bwd ? ws.tiles : nullptr, h0, n_state, tmap_o, o ? 1 : 0, ht, (bf16*)o, sv, H, NT, lay, status, \
           debug_stamp_buffer());                                                                                   \
     } while (0)

@@ -423,6 +423,8 @@ int launch_rwkv7_rec_bwd(const void* r, const void* w, const void* k, const void
   ProfScope prof("rwkv7_rec_bwd_kernel", st);
   RWKVB200_DISPATCH_HEAD(head_size,
     const int smem = (int)sizeof(BwdSmem<N>);
+    DeviceFacts dev;
+    if (int e = device_facts(&dev)) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(B * H, N / VS);
     cfg.blockDim = dim3(N);
@@ -434,7 +436,7 @@ int launch_rwkv7_rec_bwd(const void* r, const void* w, const void* k, const void
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     RWKVB200_DISPATCH_DTYPE(dtype,
-      if (cuda_ok(cudaFuncSetAttribute(rwkv7_rec_bwd_kernel<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)))
+      if (allow_smem<rwkv7_rec_bwd_kernel<T, N>>(dev, smem))
         return RWKVB200_E_CUDA;
       if (cuda_ok(cudaLaunchKernelEx(&cfg, rwkv7_rec_bwd_kernel<T, N>, (const T*)r, (const T*)w, (const T*)k,
                                      (const T*)v, (const T*)a, (const T*)b, (const T*)d_o, d_ht, ckpt, (T*)dr, (T*)dw,

@@ -30,9 +30,19 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
+// The driver entry point needs the device's primary context current on THIS host thread; a thread that has only been
+// handed the device by its framework (e.g. an autograd worker) may not have it yet.  Once per thread and device.
+int bind_context() {
+  static thread_local int bound = -1;
+  int dev = 0;
+  if (cuda_ok(cudaGetDevice(&dev))) return RWKVB200_E_CUDA;
+  if (dev == bound) return RWKVB200_OK;
+  if (cuda_ok(cudaSetDevice(dev))) return RWKVB200_E_CUDA;
+  bound = dev;
+  return RWKVB200_OK;
+}
+
 static __device__ int g_status_word;
-std::mutex g_mu;
-int* g_status_ptr[64] = {};
 
 }  // namespace
 
@@ -48,10 +58,7 @@ int make_token_tensor_map(CUtensorMap* out, const void* base, int B, int T, int 
   strides[2] = row * (cuuint64_t)T * H;
   cuuint32_t box[4] = {(cuuint32_t)HS, 64, 1, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
-  // The driver entry point needs the device's primary context current on THIS host thread; a thread
-  // that has only been handed the device by its framework (e.g. an autograd worker) may not have it yet.
-  int dev = 0;
-  if (cuda_ok(cudaGetDevice(&dev)) || cuda_ok(cudaSetDevice(dev))) return RWKVB200_E_CUDA;
+  if (bind_context()) return RWKVB200_E_CUDA;
   CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -70,8 +77,7 @@ int make_row_tensor_map(CUtensorMap* out, const void* base, int B, int T, int H,
   cuuint64_t strides[3] = {row * H, row, row * (cuuint64_t)T * H};
   cuuint32_t box[4] = {(cuuint32_t)HS, 64, 1, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
-  int dev = 0;
-  if (cuda_ok(cudaGetDevice(&dev)) || cuda_ok(cudaSetDevice(dev))) return RWKVB200_E_CUDA;
+  if (bind_context()) return RWKVB200_E_CUDA;
   CUresult r = fn(out, elem_bytes == 4 ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 4,
                   const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -87,16 +93,33 @@ long long* debug_stamp_buffer() { return g_stamp_buffer; }
 long long* debug_stamp_buffer() { return nullptr; }
 #endif
 
-int* device_status_ptr() {
+int device_facts(DeviceFacts* out) {
+  static std::atomic<int> sms[64];
+  static std::atomic<int*> status[64];
   int dev = -1;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  std::lock_guard<std::mutex> lk(g_mu);
-  if (!g_status_ptr[dev]) {
-    void* p = nullptr;
-    if (cudaGetSymbolAddress(&p, g_status_word) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-    g_status_ptr[dev] = reinterpret_cast<int*>(p);
+  if (cuda_ok(cudaGetDevice(&dev))) return RWKVB200_E_CUDA;
+  if (dev < 0 || dev >= 64) { last_cuda_error_slot() = (int)cudaErrorInvalidDevice; return RWKVB200_E_CUDA; }
+  int n = sms[dev].load(std::memory_order_relaxed);
+  if (!n) {
+    if (cuda_ok(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev))) return RWKVB200_E_CUDA;
+    sms[dev].store(n, std::memory_order_relaxed);
   }
-  return g_status_ptr[dev];
+  int* word = status[dev].load(std::memory_order_acquire);
+  if (!word) {
+    void* p = nullptr;
+    if (cuda_ok(cudaGetSymbolAddress(&p, g_status_word))) { cudaGetLastError(); return RWKVB200_E_CUDA; }
+    word = reinterpret_cast<int*>(p);
+    status[dev].store(word, std::memory_order_release);
+  }
+  out->dev = dev;
+  out->sms = n;
+  out->status = word;
+  return RWKVB200_OK;
+}
+
+int* device_status_ptr() {
+  DeviceFacts f;
+  return device_facts(&f) ? nullptr : f.status;
 }
 
 #ifdef RWKVB200_DEVTOOLS

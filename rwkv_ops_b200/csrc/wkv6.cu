@@ -492,7 +492,9 @@ int launch_bwd_cluster(const void* r, const void* k, const void* v, const void* 
                        float* du_partial, float* d_s0, int B, int Tn, int H, cudaStream_t st, const UnitSel& sel) {
   typedef typename std::conditional<COARSE, BwdSmemCoarse<N>, BwdSmem<N>>::type Smem;
   const int smem = (int)sizeof(Smem);
-  if (cuda_ok(cudaFuncSetAttribute(wkv6_bwd_kernel<T, N, COARSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)))
+  DeviceFacts dev;
+  if (int e = device_facts(&dev)) return e;
+  if (allow_smem<wkv6_bwd_kernel<T, N, COARSE>>(dev, smem))
     return RWKVB200_E_CUDA;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(B * H, N / VS);

@@ -1020,12 +1020,14 @@ int launch_wkv6_chunked_fwd(const void* r, const void* k, const void* v, const v
   const int mapB = packed ? 1 : B, mapT = packed ? T_total : Tn;
   const Seqs seqs{seq_start, seq_len, (Tn + L - 1) / L + 1};
   if (cuda_ok(cudaMemsetAsync(flags, 0, (size_t)B * H * sizeof(int), st))) return RWKVB200_E_CUDA;
-  int* status = device_status_ptr();
-  if (!status) { last_cuda_error_slot() = 99999; return RWKVB200_E_CUDA; }
+  DeviceFacts dev;
+  int e = device_facts(&dev);
+  if (e) return e;
+  int* status = dev.status;
   const int smem = (int)sizeof(FwdSmem) + 1024;
   const int esz = dtype == RWKVB200_F32 ? 4 : 2;
   CUtensorMap tm_r, tm_k, tm_v, tm_w;
-  int e = make_row_tensor_map(&tm_r, r, mapB, mapT, H, esz);
+  e = make_row_tensor_map(&tm_r, r, mapB, mapT, H, esz);
   if (!e) e = make_row_tensor_map(&tm_k, k, mapB, mapT, H, esz);
   if (!e) e = make_row_tensor_map(&tm_v, v, mapB, mapT, H, esz);
   if (!e) e = make_row_tensor_map(&tm_w, w, mapB, mapT, H, esz);
@@ -1034,9 +1036,7 @@ int launch_wkv6_chunked_fwd(const void* r, const void* k, const void* v, const v
   {
     // more units than the two CTAs per SM hold at once: every unit as 2 or 4 stretches of its chunks on a
     // persistent grid, whichever evens out the last round best (see the kernel); else one CTA per unit
-    int dev = 0, sms = 0;
-    if (cuda_ok(cudaGetDevice(&dev)) || cuda_ok(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)))
-      return RWKVB200_E_CUDA;
+    const int sms = dev.sms;
     const int n_units = B * H, slots = 2 * sms, NTmax = (Tn + L - 1) / L;
     int parts = 1;
     if (n_units > slots) {
@@ -1050,8 +1050,7 @@ int launch_wkv6_chunked_fwd(const void* r, const void* k, const void* v, const v
     if (parts > 1 && cuda_ok(cudaMemsetAsync(hflags, 0, ((size_t)n_units + 1) * sizeof(int), st))) return RWKVB200_E_CUDA;
     ProfScope prof("wkv6c_fwd_kernel", st);
     RWKVB200_DISPATCH_DTYPE(dtype, W6C_DISPATCH_PACKED(
-      if (cuda_ok(cudaFuncSetAttribute(wkv6c_fwd_kernel<T, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)))
-        return RWKVB200_E_CUDA;
+      if (allow_smem<wkv6c_fwd_kernel<T, P>>(dev, smem)) return RWKVB200_E_CUDA;
       wkv6c_fwd_kernel<T, P><<<grid, 256, smem, st>>>((const T*)r, (const T*)k, (const T*)v, (const T*)w, u, s0,
                                                        n_state, smap, (T*)y, sT, states, flags, tm_r, tm_k, tm_v, tm_w,
                                                        mapT, H, seqs, n_units, parts, handoff, hflags, status,
@@ -1143,8 +1142,10 @@ int launch_wkv6_chunked_bwd(const void* r, const void* k, const void* v, const v
                                 ws.hflags, B, Tn, H, dtype, st, seq_start, seq_len, T_total);
     if (e) return e;
   }
-  int* status = device_status_ptr();
-  if (!status) { last_cuda_error_slot() = 99999; return RWKVB200_E_CUDA; }
+  DeviceFacts dev;
+  e = device_facts(&dev);
+  if (e) return e;
+  int* status = dev.status;
   const int smem = (int)sizeof(BwdSmem) + 1024;
   bool split = false;
   {
@@ -1158,17 +1159,14 @@ int launch_wkv6_chunked_bwd(const void* r, const void* k, const void* v, const v
     if (e) return e;
     // more units than SMs: every unit as two half-length items on one persistent CTA per SM, which evens out
     // the last round (see the kernel); else one CTA per unit
-    int dev = 0, sms = 0;
-    if (cuda_ok(cudaGetDevice(&dev)) || cuda_ok(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)))
-      return RWKVB200_E_CUDA;
+    const int sms = dev.sms;
     const int n_units = B * H;
     split = n_units > sms && (Tn + L - 1) / L >= 4;
     const int grid = split ? sms : n_units;
     if (split && cuda_ok(cudaMemsetAsync(ws.hflags, 0, ((size_t)n_units + 1) * sizeof(int), st))) return RWKVB200_E_CUDA;
     ProfScope prof("wkv6c_bwd_kernel", st);
     RWKVB200_DISPATCH_DTYPE(dtype, W6C_DISPATCH_PACKED(
-      if (cuda_ok(cudaFuncSetAttribute(wkv6c_bwd_kernel<T, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)))
-        return RWKVB200_E_CUDA;
+      if (allow_smem<wkv6c_bwd_kernel<T, P>>(dev, smem)) return RWKVB200_E_CUDA;
       wkv6c_bwd_kernel<T, P><<<grid, 256, smem, st>>>((const T*)r, (const T*)k, (const T*)v, (const T*)w, u,
                                                        (const T*)d_y, d_sT, states, (T*)dr, (T*)dk, (T*)dv, (T*)dw,
                                                        du_partial, d_s0, tm_r, tm_k, tm_v, tm_w, tm_dy, mapT, H, seqs,
