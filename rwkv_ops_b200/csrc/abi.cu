@@ -95,8 +95,8 @@ int rwkvb200_rwkv7_step(const void* r, const void* w, const void* k, const void*
   const void* ps[] = {r, w, k, v, a, b, state_in, state_out, o};
   for (const void* p : ps) if (p && !aligned16(p)) return RWKVB200_E_ALIGN;
   if (head_size != HS)      // one token of the float32 recurrence
-    return launch_rwkv7_rec_fwd(r, w, k, v, a, b, n_state ? state_in : nullptr, n_state, o, state_out, nullptr,
-                                R7_CKPT, B, 1, H, dtype, 0, (cudaStream_t)stream, nullptr, 0, head_size);
+    return launch_rwkv7_rec_step(r, w, k, v, a, b, n_state ? state_in : nullptr, n_state, o, state_out, B, H, dtype,
+                                 (cudaStream_t)stream);
   return launch_rwkv7_step(r, w, k, v, a, b, n_state ? state_in : nullptr, n_state, state_out, o, B, H, dtype,
                            (cudaStream_t)stream);
 }
@@ -142,8 +142,8 @@ int rwkvb200_rwkv7_fwd(const void* r, const void* w, const void* k, const void* 
     return RWKVB200_E_UNSUPPORTED;
   switch (resolve_r7_algo(algo, dtype, head_size)) {
     case RWKVB200_ALGO_RECURRENT:
-      return launch_rwkv7_rec_fwd(r, w, k, v, a, b, n_state ? h0 : nullptr, n_state, o, ht, nullptr, R7_CKPT,
-                                  B, T, H, dtype, head_first, (cudaStream_t)stream, nullptr, 0, head_size);
+      return launch_rwkv7_block_fwd(r, w, k, v, a, b, n_state ? h0 : nullptr, n_state, o, ht, B, T, H, dtype,
+                                    head_first, (cudaStream_t)stream, head_size);
     case RWKVB200_ALGO_CHUNKED:
       if (dtype != RWKVB200_BF16) return RWKVB200_E_UNSUPPORTED;
       return launch_rwkv7_chunked_fwd(r, w, k, v, a, b, n_state ? h0 : nullptr, n_state, o, ht, workspace,
@@ -186,14 +186,10 @@ int rwkvb200_rwkv7_bwd(const void* r, const void* w, const void* k, const void* 
   if (phases_of(algo) != PHASE_ALL && resolve_r7_algo(algo, dtype, head_size) != RWKVB200_ALGO_CHUNKED)
     return RWKVB200_E_UNSUPPORTED;
   switch (resolve_r7_algo(algo, dtype, head_size)) {
-    case RWKVB200_ALGO_RECURRENT: {
-      float* ckpt = reinterpret_cast<float*>(workspace);
-      e = launch_rwkv7_rec_fwd(r, w, k, v, a, b, n_state ? h0 : nullptr, n_state, nullptr, nullptr, ckpt, R7_CKPT,
-                               B, T, H, dtype, head_first, st, nullptr, 0, head_size);
-      if (e) return e;
-      return launch_rwkv7_rec_bwd(r, w, k, v, a, b, d_o, d_ht, ckpt, dr, dw, dk, dv, da, db, d_h0,
-                                  B, T, H, dtype, head_first, st, nullptr, 0, head_size);
-    }
+    case RWKVB200_ALGO_RECURRENT:
+      return launch_rwkv7_block_bwd(r, w, k, v, a, b, n_state ? h0 : nullptr, n_state, d_o, d_ht,
+                                    reinterpret_cast<float*>(workspace), dr, dw, dk, dv, da, db, d_h0, B, T, H, dtype,
+                                    head_first, st, head_size);
     case RWKVB200_ALGO_CHUNKED:
       if (dtype != RWKVB200_BF16) return RWKVB200_E_UNSUPPORTED;
       return launch_rwkv7_chunked_bwd(r, w, k, v, a, b, n_state ? h0 : nullptr, n_state, d_o, d_ht,

@@ -161,17 +161,27 @@ int launch_rwkv7_step(const void* r, const void* w, const void* k, const void* v
                       const float* s_in, int n_state, float* s_out, void* o, int B, int H, int dtype,
                       cudaStream_t st);
 
-// Recurrent (token-by-token) RWKV7 forward.  ckpt (may be NULL) receives the state before every
-// ckpt_every-th token as [B,H,ceil(T/ckpt_every),64,64]; o and ht may be NULL.
+// One token of the float32 recurrence at head size 128.
+int launch_rwkv7_rec_step(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
+                          const float* h0, int n_state, void* o, float* ht, int B, int H, int dtype, cudaStream_t st);
+// The token-by-token recurrence, bfloat16 at head size 64.  Backward: over the units marked in sel.flags, or all of a dense
+// batch; ckpt: sel.ckpt_unit_stride floats of scratch per unit (0: dense), 4096 for every R7_CKPT tokens.
 int launch_rwkv7_rec_fwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
-                         const float* h0, int n_state, void* o, float* ht, float* ckpt, int ckpt_every,
-                         int B, int Tn, int H, int dtype, int head_first, cudaStream_t st,
-                         const UnitSel* sel = nullptr, int T_total = 0, int head_size = HS);
+                         const float* h0, int n_state, void* o, float* ht, int B, int Tn, int H, int head_first,
+                         cudaStream_t st);
 int launch_rwkv7_rec_bwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
-                         const void* d_o, const float* d_ht, const float* ckpt,
+                         const float* h0, int n_state, const void* d_o, const float* d_ht, float* ckpt,
                          void* dr, void* dw, void* dk, void* dv, void* da, void* db, float* d_h0,
-                         int B, int Tn, int H, int dtype, int head_first, cudaStream_t st,
-                         const UnitSel* sel = nullptr, int T_total = 0, int head_size = HS);
+                         int B, int Tn, int H, int head_first, cudaStream_t st, const UnitSel& sel, int T_total);
+// Float32 recurrence over blocks of tokens (rwkv7_block.cu), head size 64 or 128; o and ht may be NULL.  ckpt: room for
+// a state every R7_CKPT tokens of each unit.
+int launch_rwkv7_block_fwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
+                           const float* h0, int n_state, void* o, float* ht, int B, int Tn, int H, int dtype,
+                           int head_first, cudaStream_t st, int head_size = HS);
+int launch_rwkv7_block_bwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
+                           const float* h0, int n_state, const void* d_o, const float* d_ht, float* ckpt,
+                           void* dr, void* dw, void* dk, void* dv, void* da, void* db, float* d_h0, int B, int Tn, int H,
+                           int dtype, int head_first, cudaStream_t st, int head_size = HS);
 constexpr int R7_CKPT = 8;   // tokens between state checkpoints of the recurrent backward
 
 int launch_wkv6_fwd(const void* r, const void* k, const void* v, const void* w, const float* u,

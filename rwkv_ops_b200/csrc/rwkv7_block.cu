@@ -1,0 +1,806 @@
+// RWKV7 generalized delta rule in float32 on the CUDA cores, eight tokens at a time (forward and backward).
+//
+// The exact path of the reference's native operator (rwkv_ops/rwkv7_kernel/native_keras_op.py:80-91),
+//
+//   d_t = exp(-exp(w_t));  sa_t = S_{t-1} a_t;  S_t = S_{t-1} diag(d_t) + sa_t b_t^T + v_t k_t^T;  o_t = S_t r_t,
+//
+// for float32 and float16 tokens and for head size 128.  Token by token its time is a serial chain: two
+// reductions over the key channels per token, 930 cycles forward and 2300 backward, whatever the size.  Written out
+// over a block of W tokens that chain shrinks to one reduction per block.  With S the state before the block, D_j the
+// product of the decays of tokens 0..j of the block and x_j^(i) = x_j times the decays in between,
+//
+//   sa_j = S (D_{j-1} a_j) + sum_{i<j} sa_i A_ab(j,i) + v_i A_ak(j,i)      A_ab(j,i) = b_i^(j-1) . a_j, ...
+//   o_j  = S (D_j r_j)     + sum_{i<=j} sa_i A_qb(j,i) + v_i A_qk(j,i)     A_qb(j,i) = b_i^(j) . r_j, ...
+//   S'   = S D_{W-1}       + sum_i sa_i b_i^(W-1) + v_i k_i^(W-1)
+//
+// and the scalars A do not depend on the state.  Substituting the first line into itself and into the second gives
+// sa_j = S x_j + sum_l xv(j,l) v_l and o_j = S y_j + sum_l yv(j,l) v_l, with vectors x, y and scalars xv, yv that are
+// prepared ahead of the state.  Every decay factor is a product of factors <= 1, so nothing over- or underflows that
+// the token-by-token form would keep, and all arithmetic is float32.
+//
+// The gradient G of the state runs backward in time through the same equations with the roles exchanged
+// (sa -> dsa, o -> dv, v -> do; a <-> b, r <-> k, every A transposed): one kernel serves both directions.  The other
+// five gradients do not feed the chain.  A third kernel computes them for every 16 tokens at once, from the states
+// and state gradients that the two sweeps leave at those boundaries (as much memory as a state every 8 tokens).
+//
+// B 2, T 1024, 16 heads, float32: forward 500 -> @FWD@ us, backward (all kernels) 1750 -> @BWD@ us.
+#include <type_traits>
+
+#include "common.cuh"
+
+namespace rwkvb200 {
+
+namespace {
+
+constexpr int W = 8;          // tokens per block
+constexpr int RV = 16;        // value rows per CTA
+constexpr int GT = 2 * W;     // tokens per work item of the gradient kernel, and between two checkpoints
+
+// packed pairs of float32
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+struct Quad { f32x2 lo, hi; };      // four consecutive floats
+__device__ __forceinline__ Quad quad_of(float4 f) { return Quad{pack2(f.x, f.y), pack2(f.z, f.w)}; }
+__device__ __forceinline__ Quad lds4(const float* p) { return quad_of(*reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ float sum2(f32x2 v) { const float2 f = unpack2(v); return f.x + f.y; }
+
+// Sum CNT values over the lanes that differ in the bits of MASK, MASK/2, .., LAST; the values are shared out on the
+// way: a lane whose bit is set goes on with the upper half.
+template <int CNT, int MASK, int LAST, int M>
+__device__ __forceinline__ void reduce_scatter(float (&v)[M], int lane) {
+  const bool up = lane & MASK;
+#pragma unroll
+  for (int k = 0; k < CNT / 2; ++k) {
+    const float send = up ? v[k] : v[k + CNT / 2], keep = up ? v[k + CNT / 2] : v[k];
+    v[k] = keep + __shfl_xor_sync(0xffffffffu, send, MASK);
+  }
+  if constexpr (MASK > LAST) reduce_scatter<CNT / 2, MASK / 2, LAST>(v, lane);
+}
+
+__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+// 16 bytes into shared memory, zeros when !live (the address must be valid all the same)
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool live) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
+template <typename T> struct Vecs { const T* p[5]; };      // r, w, k, a, b
+enum { VR = 0, VW = 1, VK = 2, VA = 3, VB = 4 };
+
+// ---------------------------------------------------------------------------------------------
+// the sweep over the blocks: forward (S, sa, o) or backward (G, dsa, dv)
+// ---------------------------------------------------------------------------------------------
+// A CTA owns 16 value rows of one (batch, head) unit.  Its state warps hold them in registers, N/8 lanes to a row and
+// 8 columns to a lane; its N x GROUPS other threads prepare blocks ahead of them, a group of N threads per block in
+// turn.  Preparing takes about twice as long as consuming and more instructions, so what bounds the kernel is the issue rate
+// of its one SM.  In processing order p (time forward, or reversed), the stage a group hands over:
+template <int N>
+struct Stage {
+  float x[W][N], y[W][N];       // sa_p = S x_p + xv[p][.] v ;  o_p = S y_p + yv[p][.] v
+  float u1[W][N], u2[W][N];     // S' = S diag(d) + sum_p sa_p u1_p + v_p u2_p
+  float d[N];
+  float xv[W][W], yv[W][W];
+  float vt[RV][W];
+};
+template <typename T, int N>
+struct Prep {
+  T raw[2][5][W][N];            // the block at work and the next one (requested while the first is worked on)
+  T rawv[2][W][RV];
+  float d[W][N];
+  float sx[W][W], sxv[W][W], sy[W][W], syv[W][W];     // the scalars A, processing order; never-written entries stay 0
+};
+template <typename T, int N>
+struct SweepSmem {
+  static constexpr int GROUPS = N == 64 ? 4 : 3;
+  Stage<N> stage[GROUPS];
+  Prep<T, N> prep[GROUPS];
+};
+template <typename T, int N> constexpr int sweep_threads() { return RV * N / 8 + N * SweepSmem<T, N>::GROUPS; }
+
+template <typename T, int N, bool BWD>
+__global__ void __launch_bounds__((sweep_threads<T, N>()))
+r7_sweep_kernel(Vecs<T> in, const T* __restrict__ v, const float* __restrict__ s_in, int n_state,
+                T* __restrict__ out, float* __restrict__ s_out, float* __restrict__ ckpt, int Tn, int H, TokLayout lay) {
+  typedef SweepSmem<T, N> Smem;
+  constexpr int GROUPS = Smem::GROUPS, NCONS = RV * N / 8;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
+  const int unit = blockIdx.x, ys = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
+  const int bi = unit / H, hi = unit % H;
+  const long long base = bi * lay.sb + hi * lay.sh;
+  const int NB = (Tn + W - 1) / W;
+  const int FULL = 1 + GROUPS, EMPTY = 1 + 2 * GROUPS;      // named barriers: 1.. within a group, then these
+
+  if (tid < NCONS) {
+    // ---- state warps
+    constexpr int CL = N / 8;                    // lanes per row
+    const int row = tid / CL, kq = tid % CL, jl = kq & 7;
+    const int c0 = 4 * kq, c1 = N / 2 + 4 * kq;  // this thread's columns: two quads
+    const int NG = (Tn + GT - 1) / GT;
+    const long long srow = (long long)(ys * RV + row) * N;
+    Quad S0 = Quad{0ull, 0ull}, S1 = S0;
+    if (s_in && n_state > 0) {
+      const float* p = s_in + (long long)(n_state == 1 ? hi : unit) * N * N + srow;
+      S0 = quad_of(*reinterpret_cast<const float4*>(p + c0));
+      S1 = quad_of(*reinterpret_cast<const float4*>(p + c1));
+    }
+    auto put_state = [&](float* p) {
+      const float2 a = unpack2(S0.lo), b = unpack2(S0.hi), c = unpack2(S1.lo), d = unpack2(S1.hi);
+      *reinterpret_cast<float4*>(p + srow + c0) = make_float4(a.x, a.y, b.x, b.y);
+      *reinterpret_cast<float4*>(p + srow + c1) = make_float4(c.x, c.y, d.x, d.y);
+    };
+    for (int idx = 0, g = 0; idx < NB; ++idx, g = g + 1 == GROUPS ? 0 : g + 1) {
+      const int n = BWD ? NB - 1 - idx : idx;
+      const Stage<N>& st = sm.stage[g];
+      if (ckpt) {      // forward: the state before every GT tokens but the first; backward: the gradient after them, but the last
+        const int m = n >> 1;
+        if (!BWD && (n & 1) == 0 && m > 0) put_state(ckpt + ((long long)unit * 2 * (NG - 1) + m - 1) * N * N);
+        if (BWD && (n & 1) == 1 && m < NG - 1) put_state(ckpt + ((long long)unit * 2 * (NG - 1) + (NG - 1) + m) * N * N);
+      }
+      bar_sync(FULL + g, NCONS + N);
+      const float4 va = *reinterpret_cast<const float4*>(&st.vt[row][0]), vb = *reinterpret_cast<const float4*>(&st.vt[row][4]);
+      const float vv[W] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
+      float ax[N == 64 ? W : 2 * W], ay[W];
+#pragma unroll
+      for (int p = 0; p < W; ++p) {
+        const Quad xa = lds4(&st.x[p][c0]), xb = lds4(&st.x[p][c1]);
+        ax[p] = sum2(fma2(S1.hi, xb.hi, fma2(S1.lo, xb.lo, fma2(S0.hi, xa.hi, mul2(S0.lo, xa.lo)))));
+      }
+#pragma unroll
+      for (int p = 0; p < W; ++p) {
+        const Quad ya = lds4(&st.y[p][c0]), yb = lds4(&st.y[p][c1]);
+        ay[p] = sum2(fma2(S1.hi, yb.hi, fma2(S1.lo, yb.lo, fma2(S0.hi, ya.hi, mul2(S0.lo, ya.lo)))));
+      }
+      float sa, oo;
+      const float* xv = &st.xv[jl][0];
+      const float* yv = &st.yv[jl][0];
+      if constexpr (N == 64) {      // lane jl of a row ends with token jl of both
+        reduce_scatter<W, 4, 1>(ax, lane);
+        reduce_scatter<W, 4, 1>(ay, lane);
+        sa = ax[0]; oo = ay[0];
+      } else {                      // lanes 0-7 of a row take sa, lanes 8-15 the outputs
+#pragma unroll
+        for (int p = 0; p < W; ++p) ax[W + p] = ay[p];
+        reduce_scatter<2 * W, 8, 1>(ax, lane);
+        sa = oo = ax[0];
+      }
+#pragma unroll
+      for (int l = 0; l < W; l += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(xv + l), y = *reinterpret_cast<const float4*>(yv + l);
+        sa += x.x * vv[l] + x.y * vv[l + 1] + (x.z * vv[l + 2] + x.w * vv[l + 3]);
+        oo += y.x * vv[l] + y.y * vv[l + 1] + (y.z * vv[l + 2] + y.w * vv[l + 3]);
+      }
+      {
+        const Quad da = lds4(&st.d[c0]), db = lds4(&st.d[c1]);
+        S0.lo = mul2(S0.lo, da.lo); S0.hi = mul2(S0.hi, da.hi);
+        S1.lo = mul2(S1.lo, db.lo); S1.hi = mul2(S1.hi, db.hi);
+      }
+#pragma unroll
+      for (int p = 0; p < W; ++p) {
+        const Quad ua = lds4(&st.u2[p][c0]), ub = lds4(&st.u2[p][c1]);
+        const f32x2 s = pack2(vv[p], vv[p]);
+        S0.lo = fma2(s, ua.lo, S0.lo); S0.hi = fma2(s, ua.hi, S0.hi);
+        S1.lo = fma2(s, ub.lo, S1.lo); S1.hi = fma2(s, ub.hi, S1.hi);
+      }
+#pragma unroll
+      for (int p = 0; p < W; ++p) {
+        const Quad ua = lds4(&st.u1[p][c0]), ub = lds4(&st.u1[p][c1]);
+        const float sp = __shfl_sync(0xffffffffu, sa, (lane & ~(CL - 1)) | p);
+        const f32x2 s = pack2(sp, sp);
+        S0.lo = fma2(s, ua.lo, S0.lo); S0.hi = fma2(s, ua.hi, S0.hi);
+        S1.lo = fma2(s, ub.lo, S1.lo); S1.hi = fma2(s, ub.hi, S1.hi);
+      }
+      if (idx + GROUPS < NB) bar_arrive(EMPTY + g, NCONS + N);
+      const int t = n * W + (BWD ? W - 1 - jl : jl);
+      if (out && t < Tn && (N == 64 || kq >= 8)) out[base + (long long)t * lay.st + ys * RV + row] = from_f32<T>(oo);
+    }
+    if (s_out) put_state(s_out + (long long)unit * N * N);
+    return;
+  }
+
+  // ---- preparing groups
+  const int g = (tid - NCONS) / N, q = (tid - NCONS) % N;
+  Prep<T, N>& pr = sm.prep[g];
+  Stage<N>& st = sm.stage[g];
+  constexpr int NL = N / 4;                     // lanes per pair of source tokens below
+  constexpr int EPC = 16 / sizeof(T), CPR = N / EPC, VPR = RV / EPC;     // elements per 16 bytes; copies per token row
+
+  auto request = [&](int idx) {
+    if (idx < NB) {
+      const int t0 = (BWD ? NB - 1 - idx : idx) * W, buf = (idx / GROUPS) & 1;
+#pragma unroll
+      for (int m = 0; m < W * CPR / N; ++m) {
+        const int e = q + N * m, row = e / CPR, ch = e % CPR;
+        const bool live = t0 + row < Tn;
+        const long long off = base + (live ? (long long)(t0 + row) * lay.st : 0) + ch * EPC;
+#pragma unroll
+        for (int i = 0; i < 5; ++i) cp_async16(&pr.raw[buf][i][row][ch * EPC], in.p[i] + off, live);
+      }
+      if (q < W * VPR) {
+        const int row = q / VPR, ch = q % VPR;
+        const bool live = t0 + row < Tn;
+        cp_async16(&pr.rawv[buf][row][ch * EPC], v + base + (live ? (long long)(t0 + row) * lay.st : 0) + ys * RV + ch * EPC, live);
+      }
+    }
+    cp_async_commit();
+  };
+  request(g);
+
+  // The scalars: a thread takes four channels of the source tokens pi and 7 - pi (nine (source, later token) pairs
+  // whatever pi, so all warps have the same work), 32 sums that N/4 lanes then reduce and share out.
+  const int pi = q / NL, gq = q % NL;
+  for (int e = q; e < 4 * W * W; e += N) (&pr.sx[0][0])[e] = 0.f;
+  constexpr int HELD = 32 / NL;
+  float* dst[HELD];
+#pragma unroll
+  for (int h = 0; h < HELD; ++h) {
+    const int e = gq * HELD + h;
+    const int kind = e < 9 ? 0 : e < 18 ? 1 : e < 25 ? 2 : 3;           // A_qb, A_qk, A_ab, A_ak
+    const int x = e - (kind == 0 ? 0 : kind == 1 ? 9 : kind == 2 ? 17 : 24);
+    const int i = x <= 7 - pi ? pi : 7 - pi, j = x <= 7 - pi ? pi + x : 7 - pi + (8 - x);
+    float (*m)[W] = BWD ? (kind == 0 ? pr.sxv : kind == 1 ? pr.syv : kind == 2 ? pr.sx : pr.sy)
+                        : (kind == 0 ? pr.sy : kind == 1 ? pr.syv : kind == 2 ? pr.sx : pr.sxv);
+    dst[h] = BWD ? &m[W - 1 - i][W - 1 - j] : &m[j][i];
+  }
+
+  for (int idx = g; idx < NB; idx += GROUPS) {
+    const int n = BWD ? NB - 1 - idx : idx, t0 = n * W, buf = (idx / GROUPS) & 1;
+    cp_async_wait();
+    bar_sync(1 + g, N);             // the block's tokens are here, and the last block's scalars and decays have been read
+    request(idx + GROUPS);
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const int t = 4 * m + q / NL, c = 4 * (q % NL);
+      const float4 f = load4_shared(&pr.raw[buf][VW][t][c]);
+      *reinterpret_cast<float4*>(&pr.d[t][c]) = t0 + t < Tn ? make_float4(decay_of(f.x), decay_of(f.y), decay_of(f.z), decay_of(f.w))
+                                                            : make_float4(1.f, 1.f, 1.f, 1.f);
+    }
+    bar_sync(1 + g, N);
+    {
+      float s[32];
+#pragma unroll
+      for (int e = 0; e < 32; ++e) s[e] = 0.f;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int i = half ? 7 - pi : pi, last = half ? pi : 7 - pi;      // later tokens i .. i + last
+        Quad pb = quad_of(load4_shared(&pr.raw[buf][VB][i][4 * gq])), pk = quad_of(load4_shared(&pr.raw[buf][VK][i][4 * gq]));
+#pragma unroll
+        for (int x = 0; x < (half ? 4 : 8); ++x) {
+          if (x > last) break;
+          const int j = i + x, at = half ? 8 - x : x;
+          if (x > 0) {
+            const Quad aj = quad_of(load4_shared(&pr.raw[buf][VA][j][4 * gq])), dj = lds4(&pr.d[j][4 * gq]);
+            s[17 + at] = sum2(fma2(pb.hi, aj.hi, mul2(pb.lo, aj.lo)));
+            s[24 + at] = sum2(fma2(pk.hi, aj.hi, mul2(pk.lo, aj.lo)));
+            pb.lo = mul2(pb.lo, dj.lo); pb.hi = mul2(pb.hi, dj.hi);
+            pk.lo = mul2(pk.lo, dj.lo); pk.hi = mul2(pk.hi, dj.hi);
+          }
+          const Quad rj = quad_of(load4_shared(&pr.raw[buf][VR][j][4 * gq]));
+          s[at] = sum2(fma2(pb.hi, rj.hi, mul2(pb.lo, rj.lo)));
+          s[9 + at] = sum2(fma2(pk.hi, rj.hi, mul2(pk.lo, rj.lo)));
+        }
+      }
+      __syncwarp();
+      reduce_scatter<32, NL / 2, 1>(s, lane);
+#pragma unroll
+      for (int h = 0; h < HELD; ++h) *dst[h] = s[h];
+    }
+    if (idx >= GROUPS) bar_sync(EMPTY + g, NCONS + N);      // the stage has been read (and the group's scalars are written)
+    else               bar_sync(1 + g, N);
+    // one channel per thread: x and y by substitution, in processing order
+    auto solve = [&](float (&xs)[W], float (&ys_)[W]) {
+#pragma unroll
+      for (int p = 0; p < W; ++p) {
+        float m[W];
+#pragma unroll
+        for (int i = 0; i < p; i += 4) *reinterpret_cast<float4*>(&m[i]) = *reinterpret_cast<const float4*>(&pr.sx[p][i]);
+#pragma unroll
+        for (int i = 0; i < p; ++i) xs[p] += m[i] * xs[i];
+      }
+#pragma unroll
+      for (int p = 0; p < W; ++p) {
+        float m[W];
+#pragma unroll
+        for (int i = 0; i <= p; i += 4) *reinterpret_cast<float4*>(&m[i]) = *reinterpret_cast<const float4*>(&pr.sy[p][i]);
+#pragma unroll
+        for (int i = 0; i <= p; ++i) ys_[p] += m[i] * xs[i];
+      }
+    };
+    {
+      float xs[W], ys_[W], dd[W];
+      float run = 1.f;
+#pragma unroll
+      for (int p = 0; p < W; ++p) {
+        const int t = BWD ? W - 1 - p : p;
+        dd[p] = pr.d[t][q];
+        xs[p] = run * to_f32(pr.raw[buf][BWD ? VB : VA][t][q]);
+        if (!BWD) run *= dd[p];
+        ys_[p] = run * to_f32(pr.raw[buf][BWD ? VK : VR][t][q]);
+        if (BWD) run *= dd[p];
+      }
+      st.d[q] = run;
+      run = 1.f;
+#pragma unroll
+      for (int p = W - 1; p >= 0; --p) {
+        const int t = BWD ? W - 1 - p : p;
+        st.u1[p][q] = run * to_f32(pr.raw[buf][BWD ? VA : VB][t][q]);
+        if (BWD) run *= dd[p];
+        st.u2[p][q] = run * to_f32(pr.raw[buf][BWD ? VR : VK][t][q]);
+        if (!BWD) run *= dd[p];
+      }
+      solve(xs, ys_);
+#pragma unroll
+      for (int p = 0; p < W; ++p) { st.x[p][q] = xs[p]; st.y[p][q] = ys_[p]; }
+    }
+    if (q < W) {      // the columns of A_ak and A_qk go through the same substitution
+      float xs[W], ys_[W];
+#pragma unroll
+      for (int p = 0; p < W; ++p) { xs[p] = pr.sxv[p][q]; ys_[p] = pr.syv[p][q]; }
+      solve(xs, ys_);
+#pragma unroll
+      for (int p = 0; p < W; ++p) { st.xv[p][q] = xs[p]; st.yv[p][q] = ys_[p]; }
+    }
+    for (int e = q; e < RV * W; e += N) {
+      const int p = e % W, row = e / W;
+      st.vt[row][p] = to_f32(pr.rawv[buf][BWD ? W - 1 - p : p][row]);
+    }
+    bar_arrive(FULL + g, NCONS + N);
+  }
+  cp_async_wait();
+}
+
+// ---------------------------------------------------------------------------------------------
+// the other gradients, 16 tokens of one unit per CTA
+// ---------------------------------------------------------------------------------------------
+// S = state before the tokens, G = gradient of the state after them.  With S_j, G_j the state after token j and its
+// whole gradient, dr_j = S_j^T do_j, da_j = S_{j-1}^T dsa_j, dk_j = G_j^T v_j, db_j = G_j^T sa_j and
+// dd_j = sum_v G_j S_{j-1}.  Three 64 x 64 states are multiplied with the block's vectors (rows: S a~ -> sa, G b^ ->
+// dsa; columns: S^T [do dsa], G^T [sa v]), after which every channel is on its own: it steps S_j^T do_i, S_j^T dsa_i,
+// G_j^T v_i and G_j^T sa_i through the 16 tokens with the scalars sa.do, v.do, sa.dsa, v.dsa (four threads to a
+// channel).  dd_j is summed from the same quantities, positive decay factors throughout, so no term cancels that does not in
+// the token-by-token form.  Bound by shared-memory reads (two 16-byte reads per 16 products).
+template <int N>
+struct GradSmem {
+  float st[N][N + 4];                 // S, then G, then S again
+  float raw[5][GT][N];                // r, d, k, a, b
+  float xs[GT][N + 4];                // a~, then b^
+  float cat1[N][36], cat2[N][36];     // [sa v], [do dsa], one row per value channel
+  float outG[N][36], outS[N][36];     // G^T cat1, S^T cat2, one row per key channel
+  float sc[4][GT][GT];                // A_qb, A_qk, A_ab, A_ak (row = later token)
+  float sv[2 * GT][36], svT[2 * GT][36];      // cat1^T cat2 and its transpose
+};
+
+template <typename T, int N>
+__global__ void __launch_bounds__(4 * N, N == 64 ? 2 : 1)
+r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, const float* __restrict__ h0, int n_state,
+               const float* __restrict__ d_ht, const float* __restrict__ ckpt, T* __restrict__ dr, T* __restrict__ dw,
+               T* __restrict__ dk, T* __restrict__ da, T* __restrict__ db, int Tn, int H, TokLayout lay) {
+  constexpr int NTHR = 4 * N;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  GradSmem<N>& sm = *reinterpret_cast<GradSmem<N>*>(smem_raw);
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int NG = (Tn + GT - 1) / GT;
+  const int unit = blockIdx.x / NG, m = blockIdx.x % NG, bi = unit / H, hi = unit % H;
+  const int t0 = m * GT;
+  const long long base = bi * lay.sb + hi * lay.sh + (long long)t0 * lay.st;
+  const int nt = min(GT, Tn - t0);
+  const float* cu = ckpt + (long long)unit * 2 * (NG - 1) * N * N;
+  const float* Sg = m > 0 ? cu + (long long)(m - 1) * N * N : n_state > 0 ? h0 + (long long)(n_state == 1 ? hi : unit) * N * N : nullptr;
+  const float* Gg = m < NG - 1 ? cu + (long long)(NG - 1 + m) * N * N : d_ht ? d_ht + (long long)unit * N * N : nullptr;
+
+  // ---- tokens and S
+  const int kq = tid % (N / 4), row0 = tid / (N / 4);      // quad of channels, token / state row (16 at a time)
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  {
+    const bool live = row0 < nt;
+    const long long off = base + (live ? (long long)row0 * lay.st : 0) + 4 * kq;
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      float4 f = live ? load4(in.p[i] + off) : zero;
+      if (i == VW) f = live ? make_float4(decay_of(f.x), decay_of(f.y), decay_of(f.z), decay_of(f.w)) : make_float4(1.f, 1.f, 1.f, 1.f);
+      *reinterpret_cast<float4*>(&sm.raw[i][row0][4 * kq]) = f;
+    }
+    const float4 fv = live ? load4(v + off) : zero, fo = live ? load4(d_o + off) : zero;
+    const float ev[4] = {fv.x, fv.y, fv.z, fv.w}, eo[4] = {fo.x, fo.y, fo.z, fo.w};
+#pragma unroll
+    for (int x = 0; x < 4; ++x) { sm.cat1[4 * kq + x][GT + row0] = ev[x]; sm.cat2[4 * kq + x][row0] = eo[x]; }
+  }
+  auto get_state = [&](const float* g) {
+#pragma unroll
+    for (int x = 0; x < N / 16; ++x) {
+      const int rr = row0 + 16 * x;
+      *reinterpret_cast<float4*>(&sm.st[rr][4 * kq]) = g ? __ldg(reinterpret_cast<const float4*>(g + (long long)rr * N + 4 * kq)) : zero;
+    }
+  };
+  get_state(Sg);
+  for (int e = tid; e < 4 * GT * GT; e += NTHR) (&sm.sc[0][0][0])[e] = 0.f;
+  __syncthreads();
+
+  // ---- scalars A: sources i and 15 - i per group of N/2 threads (17 pairs whatever i), two channels per thread
+  {
+    constexpr int NL = N / 2;
+    const int pi = tid / NL, gq = tid % NL;
+    float s[64];
+#pragma unroll
+    for (int e = 0; e < 64; ++e) s[e] = 0.f;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int i = half ? 15 - pi : pi, last = half ? pi : 15 - pi;
+      f32x2 pb = *reinterpret_cast<const f32x2*>(&sm.raw[VB][i][2 * gq]), pk = *reinterpret_cast<const f32x2*>(&sm.raw[VK][i][2 * gq]);
+#pragma unroll
+      for (int x = 0; x < (half ? 8 : 16); ++x) {
+        if (x > last) break;
+        const int j = i + x, at = half ? 16 - x : x;
+        if (x > 0) {
+          const f32x2 aj = *reinterpret_cast<const f32x2*>(&sm.raw[VA][j][2 * gq]), dj = *reinterpret_cast<const f32x2*>(&sm.raw[VW][j][2 * gq]);
+          s[33 + at] = sum2(mul2(pb, aj));
+          s[48 + at] = sum2(mul2(pk, aj));
+          pb = mul2(pb, dj); pk = mul2(pk, dj);
+        }
+        const f32x2 rj = *reinterpret_cast<const f32x2*>(&sm.raw[VR][j][2 * gq]);
+        s[at] = sum2(mul2(pb, rj));
+        s[17 + at] = sum2(mul2(pk, rj));
+      }
+    }
+    __syncwarp();
+    reduce_scatter<64, 16, 1>(s, lane);      // two sums per lane
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int e = 2 * lane + h;
+      const int kind = e < 17 ? 0 : e < 34 ? 1 : e < 49 ? 2 : 3;
+      const int x = e - (kind == 0 ? 0 : kind == 1 ? 17 : kind == 2 ? 33 : 48);
+      const int i = x <= 15 - pi ? pi : 15 - pi, j = x <= 15 - pi ? pi + x : 15 - pi + (16 - x);
+      if constexpr (N == 64) sm.sc[kind][j][i] = s[h];
+      else                   atomicAdd(&sm.sc[kind][j][i], s[h]);      // two warps' halves: one addition to 0, one to the other
+    }
+  }
+  // ---- a~_j = a_j times the decays before it in the block
+  auto scaled = [&](bool back) {
+    if (tid < N) {
+      float run = 1.f;
+#pragma unroll
+      for (int p = 0; p < GT; ++p) {
+        const int j = back ? GT - 1 - p : p;
+        sm.xs[j][tid] = run * sm.raw[back ? VB : VA][j][tid];
+        run *= sm.raw[VW][j][tid];
+      }
+    }
+  };
+  scaled(false);
+  __syncthreads();
+
+  // rows: dst[v][j] = sum_k st[v][k] xs[j][k]; a 4 x 4 tile per thread and a quarter of the channels
+  auto row_product = [&](float (*dst)[36], int j0) {
+    const int s = tid & 3, tj = (tid >> 2) & 3, tv = tid >> 4;
+    f32x2 acc[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) acc[e] = 0ull;
+#pragma unroll
+    for (int x = 0; x < N / 16; ++x) {
+      const int c = 4 * (s + 4 * x);
+      Quad A[4], B[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) { A[e] = lds4(&sm.st[4 * tv + e][c]); B[e] = lds4(&sm.xs[4 * tj + e][c]); }
+#pragma unroll
+      for (int e = 0; e < 16; ++e) acc[e] = fma2(A[e >> 2].hi, B[e & 3].hi, fma2(A[e >> 2].lo, B[e & 3].lo, acc[e]));
+    }
+    float r[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) r[e] = sum2(acc[e]);
+    reduce_scatter<16, 2, 1>(r, lane);      // lane s keeps row s of the tile
+    *reinterpret_cast<float4*>(&dst[4 * tv + s][j0 + 4 * tj]) = make_float4(r[0], r[1], r[2], r[3]);
+  };
+  // columns: acc(k, j) = sum_v A[v][k] B[v][j] over 4 x 4 tiles, NS lanes share the rows of a tile
+  auto col_product = [&](const float* A, int lda, const float (*B)[36], int tk, int tj, int s, int NS, float (&r)[16]) {
+    f32x2 acc[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[e] = 0ull;
+#pragma unroll 4
+    for (int x = s; x < N; x += NS) {
+      const Quad a = lds4(A + x * lda + 4 * tk);
+      const float4 b = *reinterpret_cast<const float4*>(&B[x][4 * tj]);
+      const f32x2 bb[4] = {pack2(b.x, b.x), pack2(b.y, b.y), pack2(b.z, b.z), pack2(b.w, b.w)};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) { acc[j] = fma2(a.lo, bb[j], acc[j]); acc[4 + j] = fma2(a.hi, bb[j], acc[4 + j]); }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 lo = unpack2(acc[j]), hi = unpack2(acc[4 + j]);
+      r[j] = lo.x; r[4 + j] = lo.y; r[8 + j] = hi.x; r[12 + j] = hi.y;      // r[4 k + j]
+    }
+  };
+  auto state_cols = [&](float (*dst)[36], const float (*B)[36]) {
+    const int s = tid & 1, tj = (tid >> 1) & 7, tk = tid >> 4;
+    float r[16];
+    col_product(&sm.st[0][0], N + 4, B, tk, tj, s, 2, r);
+    reduce_scatter<16, 1, 1>(r, lane);      // lane s keeps channels 2 s, 2 s + 1
+    *reinterpret_cast<float4*>(&dst[4 * tk + 2 * s][4 * tj]) = make_float4(r[0], r[1], r[2], r[3]);
+    *reinterpret_cast<float4*>(&dst[4 * tk + 2 * s + 1][4 * tj]) = make_float4(r[4], r[5], r[6], r[7]);
+  };
+
+  row_product(sm.cat1, 0);
+  __syncthreads();
+  if (tid < N) {      // sa_j, one value row per thread
+    float sa[GT], vv[GT];
+#pragma unroll
+    for (int j = 0; j < GT; j += 4) {
+      const float4 y = *reinterpret_cast<const float4*>(&sm.cat1[tid][j]), f = *reinterpret_cast<const float4*>(&sm.cat1[tid][GT + j]);
+      sa[j] = y.x; sa[j + 1] = y.y; sa[j + 2] = y.z; sa[j + 3] = y.w;
+      vv[j] = f.x; vv[j + 1] = f.y; vv[j + 2] = f.z; vv[j + 3] = f.w;
+    }
+#pragma unroll
+    for (int j = 1; j < GT; ++j) {
+      float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+      for (int i = 0; i < j; i += 4) {      // entries on and right of the diagonal are 0
+        const float4 ab = *reinterpret_cast<const float4*>(&sm.sc[2][j][i]), ak = *reinterpret_cast<const float4*>(&sm.sc[3][j][i]);
+        s1 += ak.x * vv[i]; s1 += ak.y * vv[i + 1]; s1 += ak.z * vv[i + 2]; s1 += ak.w * vv[i + 3];
+        s2 += ab.x * sa[i];
+        if (i + 1 < j) s2 += ab.y * sa[i + 1];
+        if (i + 2 < j) s2 += ab.z * sa[i + 2];
+        if (i + 3 < j) s2 += ab.w * sa[i + 3];
+      }
+      sa[j] += s1 + s2;
+    }
+#pragma unroll
+    for (int j = 0; j < GT; j += 4) *reinterpret_cast<float4*>(&sm.cat1[tid][j]) = make_float4(sa[j], sa[j + 1], sa[j + 2], sa[j + 3]);
+  }
+  // ---- G replaces S; sum_v G S on the way (16 partial rows in outS)
+  {
+    float4 z = zero;
+#pragma unroll
+    for (int x = 0; x < N / 16; ++x) {
+      const int rr = row0 + 16 * x;
+      float4* p = reinterpret_cast<float4*>(&sm.st[rr][4 * kq]);
+      const float4 G = Gg ? __ldg(reinterpret_cast<const float4*>(Gg + (long long)rr * N + 4 * kq)) : zero, S = *p;
+      z.x += G.x * S.x; z.y += G.y * S.y; z.z += G.z * S.z; z.w += G.w * S.w;
+      *p = G;
+    }
+    const float ez[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+    for (int x = 0; x < 4; ++x) sm.outS[4 * kq + x][row0] = ez[x];
+  }
+  scaled(true);
+  __syncthreads();
+  float zsum = 0.f;      // role 2 below: this channel's sum_v G S
+  if (tid / N == 2) {
+#pragma unroll
+    for (int x = 0; x < 16; x += 4) {
+      const float4 f = *reinterpret_cast<const float4*>(&sm.outS[tid % N][x]);
+      zsum += (f.x + f.y) + (f.z + f.w);
+    }
+  }
+  row_product(sm.cat2, GT);
+  state_cols(sm.outG, sm.cat1);
+  __syncthreads();
+  get_state(Sg);
+  if (tid < N) {      // dsa_j, from the last token to the first
+    float ds[GT], dov[GT];
+#pragma unroll
+    for (int j = 0; j < GT; j += 4) {
+      const float4 e = *reinterpret_cast<const float4*>(&sm.cat2[tid][GT + j]), f = *reinterpret_cast<const float4*>(&sm.cat2[tid][j]);
+      ds[j] = e.x; ds[j + 1] = e.y; ds[j + 2] = e.z; ds[j + 3] = e.w;
+      dov[j] = f.x; dov[j + 1] = f.y; dov[j + 2] = f.z; dov[j + 3] = f.w;
+    }
+#pragma unroll
+    for (int i = GT - 1; i >= 0; --i) {
+      ds[i] += sm.sc[0][i][i] * dov[i];      // now final
+#pragma unroll
+      for (int j = 0; j < i; j += 4) {
+        const float4 qb = *reinterpret_cast<const float4*>(&sm.sc[0][i][j]), ab = *reinterpret_cast<const float4*>(&sm.sc[2][i][j]);
+        const float q_[4] = {qb.x, qb.y, qb.z, qb.w}, a_[4] = {ab.x, ab.y, ab.z, ab.w};
+#pragma unroll
+        for (int x = 0; x < 4; ++x) if (j + x < i) ds[j + x] += q_[x] * dov[i];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) if (j + x < i) ds[j + x] += a_[x] * ds[i];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < GT; j += 4) *reinterpret_cast<float4*>(&sm.cat2[tid][GT + j]) = make_float4(ds[j], ds[j + 1], ds[j + 2], ds[j + 3]);
+  }
+  __syncthreads();
+  state_cols(sm.outS, sm.cat2);
+  {
+    constexpr int NS = NTHR / 64;      // 4 or 8 lanes per tile
+    const int s = tid % NS, ti = tid / NS % 8, tj = tid / (NS * 8);
+    float r[16];
+    col_product(&sm.cat1[0][0], 36, sm.cat2, ti, tj, s, NS, r);
+    reduce_scatter<16, NS / 2, 1>(r, lane);
+    constexpr int KEEP = 16 / NS;
+#pragma unroll
+    for (int x = 0; x < KEEP; ++x) {
+      const int e = s * KEEP + x, i = 4 * ti + (e >> 2), j = 4 * tj + (e & 3);
+      sm.sv[i][j] = r[x];
+      sm.svT[j][i] = r[x];
+    }
+  }
+  __syncthreads();
+
+  // ---- one channel per thread and role
+  const int role = tid / N, c = tid % N;
+  float d[GT];
+#pragma unroll
+  for (int j = 0; j < GT; ++j) d[j] = sm.raw[VW][j][c];
+  float dd[GT];      // role 0: the parts of dd that come from the outputs; role 1: from dsa; role 2: from G
+  if (role < 2) {
+    float x[GT], p[GT];      // S_{j-1}^T do_i or dsa_i, and the vector of token i that meets it in G_j
+#pragma unroll
+    for (int j = 0; j < GT; j += 4) {
+      const float4 f = *reinterpret_cast<const float4*>(&sm.outS[c][GT * role + j]);
+      x[j] = f.x; x[j + 1] = f.y; x[j + 2] = f.z; x[j + 3] = f.w;
+    }
+#pragma unroll
+    for (int j = 0; j < GT; ++j) p[j] = sm.raw[role == 0 ? VR : VA][j][c];
+    T* const dst = role == 0 ? dr : da;
+#pragma unroll
+    for (int j = 0; j < GT; ++j) {
+      const float bj = sm.raw[VB][j][c], kj = sm.raw[VK][j][c];
+      float run = 1.f, s = 0.f;
+      if (role == 0) {
+        s = x[j] * p[j];
+#pragma unroll
+        for (int i = j + 1; i < GT; ++i) { run *= d[i]; s += x[i] * (run * p[i]); }
+      } else {
+        if (j < nt) dst[base + (long long)j * lay.st + c] = from_f32<T>(x[j]);
+#pragma unroll
+        for (int i = j + 1; i < GT; ++i) { s += x[i] * (run * p[i]); run *= d[i]; }
+      }
+      dd[j] = s;
+#pragma unroll
+      for (int i4 = j & ~3; i4 < GT; i4 += 4) {
+        const float4 fs = *reinterpret_cast<const float4*>(&sm.sv[j][GT * role + i4]);
+        const float4 fv = *reinterpret_cast<const float4*>(&sm.sv[GT + j][GT * role + i4]);
+        const float es[4] = {fs.x, fs.y, fs.z, fs.w}, ev[4] = {fv.x, fv.y, fv.z, fv.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) if (i4 + e >= j) x[i4 + e] = x[i4 + e] * d[j] + (es[e] * bj + ev[e] * kj);
+      }
+      if (role == 0 && j < nt) dst[base + (long long)j * lay.st + c] = from_f32<T>(x[j]);
+    }
+    if (role == 1) {
+#pragma unroll
+      for (int j = 0; j < GT; j += 4) *reinterpret_cast<float4*>(&sm.outS[c][GT + j]) = make_float4(dd[j], dd[j + 1], dd[j + 2], dd[j + 3]);
+    }
+  } else {
+    float x[GT];      // G_j^T v_i (role 2) or G_j^T sa_i (role 3)
+    const int o = role == 2 ? GT : 0;
+#pragma unroll
+    for (int j = 0; j < GT; j += 4) {
+      const float4 f = *reinterpret_cast<const float4*>(&sm.outG[c][o + j]);
+      x[j] = f.x; x[j + 1] = f.y; x[j + 2] = f.z; x[j + 3] = f.w;
+    }
+    if (role == 2) {      // sum_v G S_{j-1}, times the decays after token j
+      float q[GT], z = zsum, after = 1.f;
+#pragma unroll
+      for (int j = 0; j < GT; j += 4) {
+        const float4 f = *reinterpret_cast<const float4*>(&sm.outG[c][j]);
+        q[j] = f.x; q[j + 1] = f.y; q[j + 2] = f.z; q[j + 3] = f.w;
+      }
+#pragma unroll
+      for (int j = 0; j < GT; ++j) { dd[j] = z; z = z * d[j] + (q[j] * sm.raw[VB][j][c] + x[j] * sm.raw[VK][j][c]); }
+#pragma unroll
+      for (int j = GT - 1; j >= 0; --j) { dd[j] *= after; after *= d[j]; }
+#pragma unroll
+      for (int j = 0; j < GT; j += 4) *reinterpret_cast<float4*>(&sm.outG[c][GT + j]) = make_float4(dd[j], dd[j + 1], dd[j + 2], dd[j + 3]);
+    }
+    T* const dst = role == 2 ? dk : db;
+#pragma unroll
+    for (int j = GT - 1; j >= 0; --j) {
+      const float rj = sm.raw[VR][j][c], aj = sm.raw[VA][j][c];
+#pragma unroll
+      for (int i4 = 0; i4 <= j; i4 += 4) {
+        const float4 fo = *reinterpret_cast<const float4*>(&sm.svT[j][o + i4]);
+        const float4 fs = *reinterpret_cast<const float4*>(&sm.svT[GT + j][o + i4]);
+        const float eo[4] = {fo.x, fo.y, fo.z, fo.w}, es[4] = {fs.x, fs.y, fs.z, fs.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if (i4 + e == j) x[j] += eo[e] * rj;
+          if (i4 + e < j) x[i4 + e] = (x[i4 + e] + eo[e] * rj) * d[j] + es[e] * aj;
+        }
+      }
+      if (j < nt) dst[base + (long long)j * lay.st + c] = from_f32<T>(x[j]);
+    }
+  }
+  __syncthreads();
+  if (role == 0) {
+#pragma unroll
+    for (int j = 0; j < GT; ++j) {
+      if (j < nt) {
+        const long long off = base + (long long)j * lay.st + c;
+        const float s = dd[j] + sm.outS[c][GT + j] + sm.outG[c][GT + j];
+        dw[off] = from_f32<T>(s * d[j] * -expf(to_f32(in.p[VW][off])));
+      }
+    }
+  }
+}
+
+template <typename T, int N, bool BWD>
+int sweep(const Vecs<T>& in, const void* v, const float* s_in, int n_state, void* out, float* s_out, float* ckpt, int B,
+          int Tn, int H, const TokLayout& lay, cudaStream_t st) {
+  DeviceFacts dev;
+  if (int e = device_facts(&dev)) return e;
+  const int smem = (int)sizeof(SweepSmem<T, N>);
+  if (allow_smem<r7_sweep_kernel<T, N, BWD>>(dev, smem)) return RWKVB200_E_CUDA;
+  ProfScope prof(BWD ? "r7_sweep_bwd_kernel" : "r7_sweep_fwd_kernel", st);
+  r7_sweep_kernel<T, N, BWD><<<dim3(B * H, N / RV), sweep_threads<T, N>(), smem, st>>>(in, (const T*)v, s_in, n_state, (T*)out, s_out,
+                                                                                  ckpt, Tn, H, lay);
+  return check_launch();
+}
+
+template <typename T, int N>
+int fwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b, const float* h0, int n_state,
+        void* o, float* ht, int B, int Tn, int H, int head_first, cudaStream_t st) {
+  const Vecs<T> in{{(const T*)r, (const T*)w, (const T*)k, (const T*)a, (const T*)b}};
+  return sweep<T, N, false>(in, v, h0, n_state, o, ht, nullptr, B, Tn, H, TokLayout(Tn, H, head_first, N), st);
+}
+
+template <typename T, int N>
+int bwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b, const float* h0, int n_state,
+        const void* d_o, const float* d_ht, float* ckpt, void* dr, void* dw, void* dk, void* dv, void* da, void* db, float* d_h0,
+        int B, int Tn, int H, int head_first, cudaStream_t st) {
+  const Vecs<T> in{{(const T*)r, (const T*)w, (const T*)k, (const T*)a, (const T*)b}};
+  const TokLayout lay(Tn, H, head_first, N);
+  int e = RWKVB200_OK;
+  if (Tn > GT) e = sweep<T, N, false>(in, v, h0, n_state, nullptr, nullptr, ckpt, B, Tn, H, lay, st);
+  if (!e) e = sweep<T, N, true>(in, d_o, d_ht, d_ht ? B * H : 0, dv, d_h0, ckpt, B, Tn, H, lay, st);
+  if (e) return e;
+  DeviceFacts dev;
+  if ((e = device_facts(&dev))) return e;
+  const int smem = (int)sizeof(GradSmem<N>);
+  if (allow_smem<r7_grad_kernel<T, N>>(dev, smem)) return RWKVB200_E_CUDA;
+  ProfScope prof("r7_grad_kernel", st);
+  r7_grad_kernel<T, N><<<B * H * ((Tn + GT - 1) / GT), 4 * N, smem, st>>>(in, (const T*)v, (const T*)d_o, h0, h0 ? n_state : 0, d_ht,
+                                                                         ckpt, (T*)dr, (T*)dw, (T*)dk, (T*)da, (T*)db, Tn, H, lay);
+  return check_launch();
+}
+
+}  // namespace
+
+// bfloat16 at head size 64 stays token by token: what is asked for there is the chunked path's fallback, bit for bit
+#define R7_BLOCK_DISPATCH(CALL)                                                                                        \
+  if (head_size == 64 && dtype == RWKVB200_F32) { constexpr int N = 64; using T = float; return CALL; }                \
+  if (head_size == 64 && dtype == RWKVB200_F16) { constexpr int N = 64; using T = __half; return CALL; }               \
+  if (head_size == 128) { constexpr int N = 128; RWKVB200_DISPATCH_DTYPE(dtype, return CALL); }   \
+  return RWKVB200_E_UNSUPPORTED;
+
+int launch_rwkv7_block_fwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
+                           const float* h0, int n_state, void* o, float* ht, int B, int Tn, int H, int dtype,
+                           int head_first, cudaStream_t st, int head_size) {
+  if (head_size == 64 && dtype == RWKVB200_BF16)
+    return launch_rwkv7_rec_fwd(r, w, k, v, a, b, h0, n_state, o, ht, B, Tn, H, head_first, st);
+  R7_BLOCK_DISPATCH((fwd<T, N>(r, w, k, v, a, b, h0, n_state, o, ht, B, Tn, H, head_first, st)))
+}
+
+int launch_rwkv7_block_bwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
+                           const float* h0, int n_state, const void* d_o, const float* d_ht, float* ckpt,
+                           void* dr, void* dw, void* dk, void* dv, void* da, void* db, float* d_h0, int B, int Tn, int H,
+                           int dtype, int head_first, cudaStream_t st, int head_size) {
+  if (head_size == 64 && dtype == RWKVB200_BF16)
+    return launch_rwkv7_rec_bwd(r, w, k, v, a, b, h0, n_state, d_o, d_ht, ckpt, dr, dw, dk, dv, da, db, d_h0, B, Tn, H,
+                                head_first, st, UnitSel{}, 0);
+  R7_BLOCK_DISPATCH((bwd<T, N>(r, w, k, v, a, b, h0, n_state, d_o, d_ht, ckpt, dr, dw, dk, dv, da, db, d_h0, B, Tn, H,
+                               head_first, st)))
+}
+
+}  // namespace rwkvb200

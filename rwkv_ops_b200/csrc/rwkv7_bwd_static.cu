@@ -73,12 +73,8 @@ int rwkvb200_rwkv7_bwd_static(const void* r, const void* w, const void* k, const
   float* ckpt = nullptr;
   int e = static_scratch(&ckpt);
   if (e) return e;
-  cudaStream_t st = (cudaStream_t)stream;
-  e = launch_rwkv7_rec_fwd(r, w, k, v, a, b, n_state ? h0 : nullptr, n_state, nullptr, nullptr, ckpt, R7_CKPT,
-                           B, T, H, dtype, head_first, st);
-  if (e) return e;
-  return launch_rwkv7_rec_bwd(r, w, k, v, a, b, d_o, d_ht, ckpt, dr, dw, dk, dv, da, db, d_h0,
-                              B, T, H, dtype, head_first, st);
+  return launch_rwkv7_block_bwd(r, w, k, v, a, b, n_state ? h0 : nullptr, n_state, d_o, d_ht, ckpt, dr, dw, dk, dv, da, db,
+                                d_h0, B, T, H, dtype, head_first, (cudaStream_t)stream);
 }
 
 }  // extern "C"

@@ -883,12 +883,8 @@ int launch_rwkv7_chunked_bwd(const void* r, const void* w, const void* k, const 
     const long long unit_floats = (long long)NT * ALL_TILES * TILE_BYTES / (long long)sizeof(float);
     float* ckpt = reinterpret_cast<float*>(ws.tiles);
     const UnitSel sel{ws.flags, seq_start, seq_len, unit_floats};
-    const int tt = seq_start ? T_total : 0;
-    int e2 = launch_rwkv7_rec_fwd(r, w, k, v, a, b, h0, n_state, nullptr, nullptr, ckpt, R7_CKPT, B, Tn, H,
-                                  RWKVB200_BF16, head_first, st, &sel, tt);
-    if (e2) return e2;
-    return launch_rwkv7_rec_bwd(r, w, k, v, a, b, d_o, d_ht, ckpt, dr, dw, dk, dv, da, db, d_h0, B, Tn, H,
-                                RWKVB200_BF16, head_first, st, &sel, tt);
+    return launch_rwkv7_rec_bwd(r, w, k, v, a, b, h0, n_state, d_o, d_ht, ckpt, dr, dw, dk, dv, da, db, d_h0, B, Tn, H,
+                                head_first, st, sel, seq_start ? T_total : 0);
   };
   if (!(phases & PHASE_FINISH)) {
     // a scan-only call hands the gradient of the initial state to its caller (who passes it to the rank on the

@@ -1,6 +1,7 @@
 // Chunked RWKV7 forward on tcgen05 (bf16 token tensors, fp32 state).  Equations and the
 // two-kernel structure are described in rwkv7_chunked.cuh.
 #include "rwkv7_chunked.cuh"
+#include "rwkv7_recurrent.cuh"
 
 namespace rwkvb200 {
 namespace r7c {
@@ -621,7 +622,7 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
                     unsigned char* __restrict__ bwd_tiles,
                     const float* __restrict__ h0, int n_state, const __grid_constant__ CUtensorMap tmap_o,
                     int write_o, float* __restrict__ ht, bf16* __restrict__ o_rows, SeqView sv, int H, int NT_slots,
-                    TokLayout lay, int* status, long long* dbg) {
+                    TokLayout lay, r7rec::FwdArgs<bf16> exact, int* status, long long* dbg) {
 #ifdef RWKVB200_DEVTOOLS
 #define R7C_STAMP(n) do { if (dbg && tid == 0 && blockIdx.x == gridDim.x / 2 && c == 2) dbg[n] = clock64(); } while (0)
 #else
@@ -854,6 +855,17 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
   marked = __syncthreads_or(marked);
   if (tid == 0) ws_flags[unit] = marked;
   if (warp == 0) tmem_dealloc(tm, 128);
+  // A marked unit again, by the exact recurrence: 64 threads per 16 rows, in place of what the chunks gave (inside this
+  // kernel, because a launch of its own over all units costs every call 2 us of device time and as much on the host).
+  if (marked && exact.r && ok) {
+    r7rec::FwdArgs<bf16> args = exact;
+    args.base = brow * lay.sb + hi * lay.sh + tb * lay.st;
+    args.Tn = Tn;
+    args.S0 = n_state > 0 ? h0 + (size_t)(n_state == 1 ? hi : unit) * 4096 : nullptr;
+    args.ht = ht ? ht + (size_t)unit * 4096 : nullptr;
+    static_assert(4 * sizeof(r7rec::FwdSmem<64>) <= sizeof(ScanSmem<STAGES>), "the recurrence runs in the scan's shared memory");
+    r7rec::fwd_rows<bf16, 64>(args, reinterpret_cast<r7rec::FwdSmem<64>*>(smem_raw)[tid >> 6], tid >> 6, tid & 63);
+  }
 }
 
 }  // namespace r7c
@@ -911,6 +923,11 @@ int launch_rwkv7_chunked_fwd(const void* r, const void* w, const void* k, const 
   {
     const int sms = dev.sms;
     ProfScope prof("r7c_scan_fwd_kernel", st);
+    // what a unit needs whose decay left the range of the scaled operands (fused producers bound |g| by e^{-1/2}: none)
+    r7rec::FwdArgs<bf16> exact{};
+    if (!fused && (o || ht))
+      exact = r7rec::FwdArgs<bf16>{(const bf16*)r, (const bf16*)w, (const bf16*)k, (const bf16*)v, (const bf16*)a, (const bf16*)b,
+                                   0, lay.st, 0, nullptr, (bf16*)o, nullptr, nullptr, 1};
     // more sequences than SMs: two single-buffered CTAs per SM; else one double-buffered CTA per SM
 #define R7C_LAUNCH_SCAN(S, P)                                                                                      \
     do {                                                                                                           \
@@ -918,23 +935,14 @@ int launch_rwkv7_chunked_fwd(const void* r, const void* w, const void* k, const 
       if (allow_smem<r7c_scan_fwd_kernel<S, P>>(dev, smem)) \
         return RWKVB200_E_CUDA;                                                                                    \
       r7c_scan_fwd_kernel<S, P><<<B * H, 256, smem, st>>>(tmap_v, ws.tiles, ws.aux, ws.flags, tpc,                 \
-          keep_for_bwd ? ws.tiles : nullptr, h0, n_state, tmap_o, o ? 1 : 0, ht, (bf16*)o, sv, H, NT, lay, status, \
+          keep_for_bwd ? ws.tiles : nullptr, h0, n_state, tmap_o, o ? 1 : 0, ht, (bf16*)o, sv, H, NT, lay, exact, status, \
           debug_stamp_buffer());                                                                                   \
     } while (0)
     if (B * H > sms) { if (seq_start) R7C_LAUNCH_SCAN(1, true); else R7C_LAUNCH_SCAN(1, false); }
     else             { if (seq_start) R7C_LAUNCH_SCAN(2, true); else R7C_LAUNCH_SCAN(2, false); }
 #undef R7C_LAUNCH_SCAN
   }
-  e = check_launch();
-  if (e || fused) return e;      // fused producers bound |g| by e^{-1/2}: no unit can be marked
-  // units whose decay left the range of the scaled operands: exact float32 recurrence over them (the
-  // kernel's other CTAs leave at once)
-  if (o || ht) {
-    const UnitSel sel{ws.flags, seq_start, seq_len, 0};
-    e = launch_rwkv7_rec_fwd(r, w, k, v, a, b, h0, n_state, o, ht, nullptr, R7_CKPT, B, Tn, H, RWKVB200_BF16,
-                             head_first, st, &sel, seq_start ? T_total : 0);
-  }
-  return e;
+  return check_launch();
 }
 
 }  // namespace rwkvb200
