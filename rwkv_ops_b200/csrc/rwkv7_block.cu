@@ -23,7 +23,8 @@
 // five gradients do not feed the chain.  A third kernel computes them for every 16 tokens at once, from the states
 // and state gradients that the two sweeps leave at those boundaries (as much memory as a state every 8 tokens).
 //
-// B 2, T 1024, 16 heads, float32: forward 500 -> @FWD@ us, backward (all kernels) 1750 -> @BWD@ us.
+// B 2, T 1024, 16 heads, float32, against the token-by-token kernels: forward 500 -> 124 us, backward with its forward sweep
+// 1740 -> 415 us.  Head size 128 at T 512: 2800 -> 912 us for both.
 #include <type_traits>
 
 #include "common.cuh"
@@ -34,6 +35,7 @@ namespace {
 
 constexpr int W = 8;          // tokens per block
 constexpr int RV = 16;        // value rows per CTA
+template <int N> constexpr int rows_per_thread() { return N / 32; }      // value rows per thread of the state warps: two warps of them
 constexpr int GT = 2 * W;     // tokens per work item of the gradient kernel, and between two checkpoints
 
 // packed pairs of float32
@@ -92,10 +94,12 @@ enum { VR = 0, VW = 1, VK = 2, VA = 3, VB = 4 };
 // ---------------------------------------------------------------------------------------------
 // the sweep over the blocks: forward (S, sa, o) or backward (G, dsa, dv)
 // ---------------------------------------------------------------------------------------------
-// A CTA owns 16 value rows of one (batch, head) unit.  Its state warps hold them in registers, N/8 lanes to a row and
-// 8 columns to a lane; its N x GROUPS other threads prepare blocks ahead of them, a group of N threads per block in
-// turn.  Preparing takes about twice as long as consuming and more instructions, so what bounds the kernel is the issue rate
-// of its one SM.  In processing order p (time forward, or reversed), the stage a group hands over:
+// A CTA owns 16 value rows of one (batch, head) unit.  Its two state warps hold them in registers (N/32 rows and 8 columns
+// to a lane, N/8 lanes to a row); its other threads prepare blocks ahead of them, a group of N threads per block in turn.
+// A vector of the stage is read from shared memory once per lane and serves N/32 rows: with one row per lane the reads
+// alone took 82 % of the shared-memory cycles (138 us per sweep at B 2, T 1024, 16 heads; 124 now), with four rows per
+// lane at N = 64 there is a single state warp and its own latency is the bound (190 us).
+// In processing order p (time forward, or reversed), the stage a group hands over:
 template <int N>
 struct Stage {
   float x[W][N], y[W][N];       // sa_p = S x_p + xv[p][.] v ;  o_p = S y_p + yv[p][.] v
@@ -117,14 +121,14 @@ struct SweepSmem {
   Stage<N> stage[GROUPS];
   Prep<T, N> prep[GROUPS];
 };
-template <typename T, int N> constexpr int sweep_threads() { return RV * N / 8 + N * SweepSmem<T, N>::GROUPS; }
+template <typename T, int N> constexpr int sweep_threads() { return RV / rows_per_thread<N>() * N / 8 + N * SweepSmem<T, N>::GROUPS; }
 
 template <typename T, int N, bool BWD>
 __global__ void __launch_bounds__((sweep_threads<T, N>()))
 r7_sweep_kernel(Vecs<T> in, const T* __restrict__ v, const float* __restrict__ s_in, int n_state,
                 T* __restrict__ out, float* __restrict__ s_out, float* __restrict__ ckpt, int Tn, int H, TokLayout lay) {
   typedef SweepSmem<T, N> Smem;
-  constexpr int GROUPS = Smem::GROUPS, NCONS = RV * N / 8;
+  constexpr int GROUPS = Smem::GROUPS, ROWS = rows_per_thread<N>(), NCONS = RV / ROWS * N / 8;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   const int unit = blockIdx.x, ys = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
@@ -136,20 +140,38 @@ r7_sweep_kernel(Vecs<T> in, const T* __restrict__ v, const float* __restrict__ s
   if (tid < NCONS) {
     // ---- state warps
     constexpr int CL = N / 8;                    // lanes per row
-    const int row = tid / CL, kq = tid % CL, jl = kq & 7;
-    const int c0 = 4 * kq, c1 = N / 2 + 4 * kq;  // this thread's columns: two quads
+    const int r0 = ROWS * (tid / CL), kq = tid % CL, jl = kq & 7;
+    const int c0 = 4 * kq, c1 = N / 2 + 4 * kq;  // this thread's columns: two quads of ROWS rows
     const int NG = (Tn + GT - 1) / GT;
-    const long long srow = (long long)(ys * RV + row) * N;
-    Quad S0 = Quad{0ull, 0ull}, S1 = S0;
-    if (s_in && n_state > 0) {
-      const float* p = s_in + (long long)(n_state == 1 ? hi : unit) * N * N + srow;
-      S0 = quad_of(*reinterpret_cast<const float4*>(p + c0));
-      S1 = quad_of(*reinterpret_cast<const float4*>(p + c1));
+    Quad S[ROWS][2];
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+      S[i][0] = S[i][1] = Quad{0ull, 0ull};
+      if (s_in && n_state > 0) {
+        const float* p = s_in + (long long)(n_state == 1 ? hi : unit) * N * N + (long long)(ys * RV + r0 + i) * N;
+        S[i][0] = quad_of(*reinterpret_cast<const float4*>(p + c0));
+        S[i][1] = quad_of(*reinterpret_cast<const float4*>(p + c1));
+      }
     }
     auto put_state = [&](float* p) {
-      const float2 a = unpack2(S0.lo), b = unpack2(S0.hi), c = unpack2(S1.lo), d = unpack2(S1.hi);
-      *reinterpret_cast<float4*>(p + srow + c0) = make_float4(a.x, a.y, b.x, b.y);
-      *reinterpret_cast<float4*>(p + srow + c1) = make_float4(c.x, c.y, d.x, d.y);
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const float2 a = unpack2(S[i][h].lo), b = unpack2(S[i][h].hi);
+          *reinterpret_cast<float4*>(p + (long long)(ys * RV + r0 + i) * N + (h ? c1 : c0)) = make_float4(a.x, a.y, b.x, b.y);
+        }
+      }
+    };
+    // S row . vector, for all rows and tokens: dots[4 p + i]
+    auto dots = [&](const float (*vec)[N], float* out4) {
+#pragma unroll
+      for (int p = 0; p < W; ++p) {
+        const Quad xa = lds4(&vec[p][c0]), xb = lds4(&vec[p][c1]);
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i)
+          out4[ROWS * p + i] = sum2(fma2(S[i][1].hi, xb.hi, fma2(S[i][1].lo, xb.lo, fma2(S[i][0].hi, xa.hi, mul2(S[i][0].lo, xa.lo)))));
+      }
     };
     for (int idx = 0, g = 0; idx < NB; ++idx, g = g + 1 == GROUPS ? 0 : g + 1) {
       const int n = BWD ? NB - 1 - idx : idx;
@@ -160,61 +182,71 @@ r7_sweep_kernel(Vecs<T> in, const T* __restrict__ v, const float* __restrict__ s
         if (BWD && (n & 1) == 1 && m < NG - 1) put_state(ckpt + ((long long)unit * 2 * (NG - 1) + (NG - 1) + m) * N * N);
       }
       bar_sync(FULL + g, NCONS + N);
-      const float4 va = *reinterpret_cast<const float4*>(&st.vt[row][0]), vb = *reinterpret_cast<const float4*>(&st.vt[row][4]);
-      const float vv[W] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
-      float ax[N == 64 ? W : 2 * W], ay[W];
+      // the reduction leaves token jl of the thread's rows: in every lane both sa and o (N = 64: 8 lanes to a row), or sa
+      // in lanes 0-7 and o in lanes 8-15 of a row
+      float ax[(N == 64 ? 1 : 2) * W * ROWS], ay[W * ROWS];
+      dots(st.x, ax);
+      float sa[ROWS], oo[ROWS];
+      if constexpr (N == 64) {
+        reduce_scatter<W * ROWS, 4, 1>(ax, lane);
+        dots(st.y, ay);
+        reduce_scatter<W * ROWS, 4, 1>(ay, lane);
 #pragma unroll
-      for (int p = 0; p < W; ++p) {
-        const Quad xa = lds4(&st.x[p][c0]), xb = lds4(&st.x[p][c1]);
-        ax[p] = sum2(fma2(S1.hi, xb.hi, fma2(S1.lo, xb.lo, fma2(S0.hi, xa.hi, mul2(S0.lo, xa.lo)))));
-      }
+        for (int i = 0; i < ROWS; ++i) { sa[i] = ax[i]; oo[i] = ay[i]; }
+      } else {
+        dots(st.y, ax + W * ROWS);
+        reduce_scatter<2 * W * ROWS, 8, 1>(ax, lane);
 #pragma unroll
-      for (int p = 0; p < W; ++p) {
-        const Quad ya = lds4(&st.y[p][c0]), yb = lds4(&st.y[p][c1]);
-        ay[p] = sum2(fma2(S1.hi, yb.hi, fma2(S1.lo, yb.lo, fma2(S0.hi, ya.hi, mul2(S0.lo, ya.lo)))));
-      }
-      float sa, oo;
-      const float* xv = &st.xv[jl][0];
-      const float* yv = &st.yv[jl][0];
-      if constexpr (N == 64) {      // lane jl of a row ends with token jl of both
-        reduce_scatter<W, 4, 1>(ax, lane);
-        reduce_scatter<W, 4, 1>(ay, lane);
-        sa = ax[0]; oo = ay[0];
-      } else {                      // lanes 0-7 of a row take sa, lanes 8-15 the outputs
-#pragma unroll
-        for (int p = 0; p < W; ++p) ax[W + p] = ay[p];
-        reduce_scatter<2 * W, 8, 1>(ax, lane);
-        sa = oo = ax[0];
-      }
-#pragma unroll
-      for (int l = 0; l < W; l += 4) {
-        const float4 x = *reinterpret_cast<const float4*>(xv + l), y = *reinterpret_cast<const float4*>(yv + l);
-        sa += x.x * vv[l] + x.y * vv[l + 1] + (x.z * vv[l + 2] + x.w * vv[l + 3]);
-        oo += y.x * vv[l] + y.y * vv[l + 1] + (y.z * vv[l + 2] + y.w * vv[l + 3]);
+        for (int i = 0; i < ROWS; ++i) sa[i] = oo[i] = ax[i];
       }
       {
         const Quad da = lds4(&st.d[c0]), db = lds4(&st.d[c1]);
-        S0.lo = mul2(S0.lo, da.lo); S0.hi = mul2(S0.hi, da.hi);
-        S1.lo = mul2(S1.lo, db.lo); S1.hi = mul2(S1.hi, db.hi);
-      }
 #pragma unroll
-      for (int p = 0; p < W; ++p) {
-        const Quad ua = lds4(&st.u2[p][c0]), ub = lds4(&st.u2[p][c1]);
-        const f32x2 s = pack2(vv[p], vv[p]);
-        S0.lo = fma2(s, ua.lo, S0.lo); S0.hi = fma2(s, ua.hi, S0.hi);
-        S1.lo = fma2(s, ub.lo, S1.lo); S1.hi = fma2(s, ub.hi, S1.hi);
+        for (int i = 0; i < ROWS; ++i) {
+          S[i][0].lo = mul2(S[i][0].lo, da.lo); S[i][0].hi = mul2(S[i][0].hi, da.hi);
+          S[i][1].lo = mul2(S[i][1].lo, db.lo); S[i][1].hi = mul2(S[i][1].hi, db.hi);
+        }
+      }
+      auto add_outer = [&](const Quad& ua, const Quad& ub, int i, float f) {
+        const f32x2 s = pack2(f, f);
+        S[i][0].lo = fma2(s, ua.lo, S[i][0].lo); S[i][0].hi = fma2(s, ua.hi, S[i][0].hi);
+        S[i][1].lo = fma2(s, ub.lo, S[i][1].lo); S[i][1].hi = fma2(s, ub.hi, S[i][1].hi);
+      };
+#pragma unroll
+      for (int l = 0; l < W; l += 4) {
+        const float4 x = *reinterpret_cast<const float4*>(&st.xv[jl][l]), y = *reinterpret_cast<const float4*>(&st.yv[jl][l]);
+        float vv[ROWS][4];
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) {
+          const float4 f = *reinterpret_cast<const float4*>(&st.vt[r0 + i][l]);
+          vv[i][0] = f.x; vv[i][1] = f.y; vv[i][2] = f.z; vv[i][3] = f.w;
+          sa[i] += x.x * f.x + x.y * f.y + (x.z * f.z + x.w * f.w);
+          oo[i] += y.x * f.x + y.y * f.y + (y.z * f.z + y.w * f.w);
+        }
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+          const Quad ua = lds4(&st.u2[l + p][c0]), ub = lds4(&st.u2[l + p][c1]);
+#pragma unroll
+          for (int i = 0; i < ROWS; ++i) add_outer(ua, ub, i, vv[i][p]);
+        }
       }
 #pragma unroll
       for (int p = 0; p < W; ++p) {
         const Quad ua = lds4(&st.u1[p][c0]), ub = lds4(&st.u1[p][c1]);
-        const float sp = __shfl_sync(0xffffffffu, sa, (lane & ~(CL - 1)) | p);
-        const f32x2 s = pack2(sp, sp);
-        S0.lo = fma2(s, ua.lo, S0.lo); S0.hi = fma2(s, ua.hi, S0.hi);
-        S1.lo = fma2(s, ub.lo, S1.lo); S1.hi = fma2(s, ub.hi, S1.hi);
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) add_outer(ua, ub, i, __shfl_sync(0xffffffffu, sa[i], (lane & ~(CL - 1)) | p));
       }
       if (idx + GROUPS < NB) bar_arrive(EMPTY + g, NCONS + N);
       const int t = n * W + (BWD ? W - 1 - jl : jl);
-      if (out && t < Tn && (N == 64 || kq >= 8)) out[base + (long long)t * lay.st + ys * RV + row] = from_f32<T>(oo);
+      if (out && t < Tn && (N == 64 || kq >= 8)) {
+        T* p = out + base + (long long)t * lay.st + ys * RV + r0;
+        if constexpr (ROWS == 4) {
+          store4(p, make_float4(oo[0], oo[1], oo[2], oo[3]));
+        } else {
+          p[0] = from_f32<T>(oo[0]);
+          p[1] = from_f32<T>(oo[1]);
+        }
+      }
     }
     if (s_out) put_state(s_out + (long long)unit * N * N);
     return;
