@@ -6,15 +6,16 @@
 //   glast = gi at token 63.
 //   q~ = q e^{gi-gref}   k~ = k e^{gref-gi}   a~ = a e^{ge-gref}   b~ = b e^{gref-gi}
 //   A_qk = tril(q~ k~^T)  A_qb = tril(q~ b~^T)  A_ak = stril(a~ k~^T)  A_ab = stril(a~ b~^T)
-//   Ainv = (I - A_ab)^-1,  W = Ainv a~,  U = Ainv A_ak v,  O1 = A_qk v
+//   Ainv = (I - A_ab)^-1,  W = Ainv a~,  U = Ainv A_ak v
 //   with h~0 = diag(e^{gref}) h0:
 //     sa  = W h~0 + U                       (rows a_i^T h_{i-1})
-//     o   = q~ h~0 + O1 + A_qb sa
+//     o   = q~ h~0 + A_qk v + A_qb sa
 //     h_L = diag(e^{glast-gref}) (h~0 + k~^T v + b~^T sa)
 // Backward (do = grad of o, dh_L = grad of the state after the chunk, gref held constant: the result
 // does not depend on it):
 //     dh^  = diag(e^{glast-gref}) dh_L
-//     dz   = Ainv^T (A_qb^T do + b~ dh^)  = P2 + B2 dh^          (z = a~ h~0 + A_ak v,  sa = Ainv z)
+//     dz   = Ainv^T (A_qb^T do + b~ dh^)  = C^T do + B2 dh^      (z = a~ h~0 + A_ak v,  sa = Ainv z)
+//     with C = A_qb Ainv and B2 = Ainv^T b~
 //     dh~0 = q~^T do + a~^T dz + dh^,   dh0 = diag(e^{gref}) dh~0
 //     dv   = A_qk^T do + A_ak^T dz + k~ dh^
 //     dA_qk = tril(do v^T)  dA_qb = tril(do sa^T)  dA_ak = stril(dz v^T)  dA_ab = stril(dz sa^T)
@@ -43,13 +44,12 @@ namespace r7c {
 
 constexpr int L = 64;                 // chunk length
 // tiles of one chunk in the workspace, in this order (the first FWD_TILES feed the forward scan)
-enum Slot { S_QT = 0, S_KT, S_BT, S_AQB, S_O1, S_W, S_U, FWD_TILES,
-            // kept for the backward: a~, A_qk, A_ak, Ainv (intra kernel); sa, h~0 and
-            // X = h~0 + k~^T v + b~^T sa (forward scan)
-            S_AT = FWD_TILES, S_AQK, S_AAK, S_AINV, S_SA, S_H0, S_X,
-            // backward intermediates: B2 = Ainv^T b~, P2 = Ainv^T A_qb^T do (adjacent), then
-            // dz = Ainv^T dsa and dh^ = e^{glast-gref} dh_L written by the reverse scan
-            S_B2, S_P2, S_DZ, S_DHH, ALL_TILES };
+enum Slot { S_KT = 0, S_AQK, S_W, S_U, S_QT, S_BT, S_AQB, FWD_TILES,
+            // kept for the backward: a~, A_ak (intra kernel); sa, h~0 and X = h~0 + k~^T v + b~^T sa (forward scan);
+            // C = A_qb Ainv and B2 = Ainv^T b~ (intra kernel)
+            S_AT = FWD_TILES, S_AAK, S_SA, S_H0, S_X, S_C, S_B2,
+            // written by the reverse scan: dz = Ainv^T dsa and dh^ = e^{glast-gref} dh_L
+            S_DZ, S_DHH, ALL_TILES };
 constexpr int AUX_FLOATS = 128;       // per chunk: e^{gref}[64], e^{glast-gref}[64]
 
 inline int num_chunks(int T) { return (T + L - 1) / L; }

@@ -1,11 +1,11 @@
 // Chunked RWKV7 backward on tcgen05 (bf16 token tensors).  Equations in rwkv7_chunked.cuh.
 //
 // Launch sequence (all on the caller's stream, tiles exchanged through the workspace):
-//   1. forward intra kernel with keep_for_bwd (q~, k~, b~, a~, A_qk, A_ak, A_qb, Ainv, W, U, decay factors)
+//   1. forward intra kernel with keep_for_bwd (q~, k~, b~, a~, A_qk, A_ak, A_qb, W, U, C, B2, decay factors)
 //   2. forward scan without output, keeping sa, h~0 and X of every chunk
-//   3. r7c_bwd_pre_kernel    (parallel over chunks)   B2 = Ainv^T b~,  P2 = Ainv^T A_qb^T do
-//   4. r7c_bwd_scan_kernel   (one CTA per (b,h), chunks in reverse)  dz, dh^ per chunk, d initial state
-//   5. r7c_bwd_final_kernel  (parallel over chunks)   dq, dk, dv, da, db, dw
+//      (1 and 2 only if the forward pass did not keep its workspace)
+//   3. r7c_bwd_scan_kernel   (one CTA per (b,h), chunks in reverse)  dz, dh^ per chunk, d initial state
+//   4. r7c_bwd_final_kernel  (parallel over chunks)   dq, dk, dv, da, db, dw
 #include "rwkv7_chunked.cuh"
 
 namespace rwkvb200 {
@@ -17,139 +17,13 @@ typedef __nv_bfloat16 bf16;
 // decay sums are kept in units of log 2 (tc::ex2), as in the forward kernels; nothing is clamped
 
 // ---------------------------------------------------------------------------------------------
-// 3. B2 = Ainv^T b~ and P2 = Ainv^T (A_qb^T do): persistent CTAs of 128 threads over the chunk-heads
+// 3. reverse scan: grid = B*H, 256 threads (the two warps of a TMEM lane window take 32 columns each)
 // ---------------------------------------------------------------------------------------------
-struct PreStage {
-  unsigned char ainv[TILE_BYTES], bt[TILE_BYTES], aqb[TILE_BYTES], dout[TILE_BYTES];
-};
-struct PreSmem {
-  PreStage st[2];             // the operand tiles of this chunk-head and of the next one
-  unsigned char p1[TILE_BYTES], b2[TILE_BYTES], p2[TILE_BYTES];
-  uint64_t bar_ld[2], bar_m1, bar_m2;
-  uint32_t tmem_base;
-};
-
-// Two CTAs per SM walk over chunk-heads ch = blockIdx.x, blockIdx.x + gridDim.x, ...; the four operand tiles
-// of the next chunk-head are requested before the current one is worked on, so that loads, the two dependent
-// MMAs and the copies of the results overlap.
-template <bool PACKED>
-__global__ void __launch_bounds__(128)
-r7c_bwd_pre_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* __restrict__ ws_tiles,
-                   int tiles_per_chunk, SeqView sv, int H, int NT, int n_ch, int* status) {
-  extern __shared__ unsigned char smem_raw[];
-  PreSmem& sm = *reinterpret_cast<PreSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int row = 16 * warp + (lane & 15);
-  const bool lo = lane < 16;
-
-  if (tid == 0) {
-    mbar_init(&sm.bar_ld[0], 1); mbar_init(&sm.bar_ld[1], 1); mbar_init(&sm.bar_m1, 1); mbar_init(&sm.bar_m2, 1);
-    fence_mbar_init();
-  }
-  if (warp == 0) tmem_alloc(&sm.tmem_base, 128);
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tm = sm.tmem_base;
-
-  auto empty = [&](const ChunkPos& p) {
-    if constexpr (!PACKED) return false;
-    return p.c * L >= sv.length<PACKED>(p.bi);      // a chunk slot past the end of a packed sequence
-  };
-  auto advance = [&](ChunkPos p) {
-    do { chunk_step(p, gridDim.x, NT, H); } while (p.ch < n_ch && empty(p));
-    return p;
-  };
-  auto issue_loads = [&](const ChunkPos& p, int s) {      // tid 0
-    const unsigned char* tiles = ws_tiles + (size_t)p.ch * tiles_per_chunk * TILE_BYTES;
-    PreStage& g = sm.st[s];
-    mbar_expect_tx(&sm.bar_ld[s], 4 * TILE_BYTES);
-    bulk_load(g.ainv, tiles + S_AINV * TILE_BYTES, TILE_BYTES, &sm.bar_ld[s]);
-    bulk_load(g.bt, tiles + S_BT * TILE_BYTES, TILE_BYTES, &sm.bar_ld[s]);
-    bulk_load(g.aqb, tiles + S_AQB * TILE_BYTES, TILE_BYTES, &sm.bar_ld[s]);
-    tma_load_4d(g.dout, &tmap_do, &sm.bar_ld[s], 0, sv.first<PACKED>(p.bi) + p.c * L, p.hi, sv.row<PACKED>(p.bi));
-  };
-  ChunkPos cur = chunk_pos(blockIdx.x, NT, H);
-  if (cur.ch < n_ch && empty(cur)) cur = advance(cur);
-  if (cur.ch < n_ch && warp == 0 && elect_one()) issue_loads(cur, 0);
-
-  bool ok = true;
-  int it = 0;
-  for (ChunkPos nxt; cur.ch < n_ch && ok; cur = nxt, ++it) {
-    const int s = it & 1;
-    const uint32_t par = it & 1;
-    PreStage& g = sm.st[s];
-    unsigned char* tiles = ws_tiles + (size_t)cur.ch * tiles_per_chunk * TILE_BYTES;
-    nxt = advance(cur);
-    // the other stage was last read by the MMAs of the previous chunk-head, which have completed
-    if (warp == 0 && elect_one() && nxt.ch < n_ch) issue_loads(nxt, s ^ 1);
-    ok = mbar_wait(&sm.bar_ld[s], (it >> 1) & 1, status, 301);
-    if (warp == 0 && elect_one() && ok) {
-      bulk_wait_read();      // the copies of the previous B2 / P2 have left their tiles, which are rewritten below
-      tc_fence_after();
-      umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 0), smem_u32(g.aqb), smem_u32(g.dout), false);   // A_qb^T do
-      umma_tile<64, 64, 1, 1>(tmem_addr(tm, 16, 0), smem_u32(g.ainv), smem_u32(g.bt), false);   // Ainv^T b~
-      umma_commit(&sm.bar_m1);
-    }
-    ok = mbar_wait(&sm.bar_m1, par, status, 302) && ok;
-    tc_fence_after();
-    if (ok) {
-#pragma unroll
-      for (int part = 0; part < 2; ++part) {
-        uint32_t r[32];
-        tmem_ld32(tmem_addr(tm, 32 * warp, 32 * part), r);
-        tmem_ld_wait();
-        float x[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(r[j]);
-        tile_store_row32(lo ? sm.p1 : sm.b2, row, 32 * part, x);
-      }
-    }
-    fence_async_smem();
-    tc_fence_before();
-    ok = __syncthreads_and(ok);
-    if (warp == 0 && elect_one() && ok) {
-      tc_fence_after();
-      umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 64), smem_u32(g.ainv), smem_u32(sm.p1), false);   // Ainv^T P1
-      umma_commit(&sm.bar_m2);
-      bulk_store(tiles + S_B2 * TILE_BYTES, sm.b2, TILE_BYTES);
-      bulk_commit();
-    }
-    ok = mbar_wait(&sm.bar_m2, par, status, 303) && ok;
-    tc_fence_after();
-    if (ok) {
-#pragma unroll
-      for (int part = 0; part < 2; ++part) {
-        uint32_t r[32];
-        tmem_ld32(tmem_addr(tm, 32 * warp, 64 + 32 * part), r);
-        tmem_ld_wait();
-        if (lo) {
-          float x[32];
-#pragma unroll
-          for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(r[j]);
-          tile_store_row32(sm.p2, row, 32 * part, x);
-        }
-      }
-    }
-    fence_async_smem();
-    tc_fence_before();
-    ok = __syncthreads_and(ok);
-    if (warp == 0 && elect_one() && ok) {
-      bulk_store(tiles + S_P2 * TILE_BYTES, sm.p2, TILE_BYTES);
-      bulk_commit();
-    }
-  }
-  if (warp == 0 && elect_one()) bulk_wait_all();
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tm, 128);
-}
-
-// ---------------------------------------------------------------------------------------------
-// 4. reverse scan: grid = B*H, 256 threads (the two warps of a TMEM lane window take 32 columns each)
-// ---------------------------------------------------------------------------------------------
+// With more sequences than SMs, two CTAs share an SM and memory bounds it (five tiles in, two out per chunk); with
+// fewer, the chain dh^ -> B2 dh^ -> dz -> a~^T dz -> dh.  The two products of a chunk that do not need dh, C^T do and
+// q~^T do, are issued while the chunk before is read out, into accumulators of their own (by parity of the chunk).
 struct BScanStage {
-  unsigned char b2[TILE_BYTES], p2[TILE_BYTES];   // adjacent workspace slots: one bulk copy
+  unsigned char cm[TILE_BYTES], b2[TILE_BYTES];   // adjacent workspace slots: one bulk copy
   unsigned char at[TILE_BYTES], qt[TILE_BYTES], dout[TILE_BYTES];
 };
 struct BScanSmem {
@@ -164,7 +38,7 @@ template <bool PACKED>
 __global__ void __launch_bounds__(256, 2)
 r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* __restrict__ ws_tiles,
                     const float* __restrict__ ws_aux, int tiles_per_chunk, const float* __restrict__ d_ht,
-                    float* __restrict__ d_h0, SeqView sv, int H, int NT_slots, int spread, int* status) {
+                    float* __restrict__ d_h0, SeqView sv, int H, int NT_slots, int* status) {
   extern __shared__ unsigned char smem_raw[];
   BScanSmem& sm = *reinterpret_cast<BScanSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -175,38 +49,44 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
   const int wq = warp & 3, hsel = warp >> 2, c0 = 32 * hsel;
   const int row = 16 * wq + (lane & 15);
   const bool state_lane = lane < 16;
-  // single-thread jobs side by side: warp 0 issues the MMAs (warp 3 one product of the first group, when
-  // the CTA has the SM to itself), st_warp copies dh^ and dz out (and waits for
-  // its own bulk-copy groups), ld_warp requests the operand tiles of the chunk after the next
-  // (they share the SM with a second CTA when there are more sequences than SMs, and then stay with warp 0)
-  const int st_warp = spread ? 1 : 0, ld_warp = spread ? 2 : 0;
+  // single-thread jobs side by side: warp 0 issues the MMAs, st_warp copies dh^ and dz out (and waits for its own
+  // bulk-copy groups), ld_warp requests the operand tiles of the chunk after the next
+  constexpr int st_warp = 1, ld_warp = 2;
 
   if (tid == 0) {
     mbar_init(&sm.bar_full[0], 1); mbar_init(&sm.bar_full[1], 1);
-    // with one CTA per SM the two products of the first MMA group have an issuing thread each
-    mbar_init(&sm.bar_m1, spread ? 2 : 1); mbar_init(&sm.bar_m2, 1);
+    mbar_init(&sm.bar_m1, 1); mbar_init(&sm.bar_m2, 1);
     fence_mbar_init();
   }
-  if (warp == 0) tmem_alloc(&sm.tmem_base, 64);
+  if (warp == 0) tmem_alloc(&sm.tmem_base, 128);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tm = sm.tmem_base;
-  const uint32_t tm_w = tmem_addr(tm, 32 * wq, c0);
+  // TMEM: columns 64 p .., p = parity of the chunk's place: lower lane halves q~^T do + a~^T dz, upper halves dz
 
   auto issue_loads = [&](int n) {     // n-th chunk in reverse order
     const int c = NT - 1 - n;
     BScanStage& s = sm.st[n & 1];
     unsigned char* tiles = ws_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES;
     mbar_expect_tx(&sm.bar_full[n & 1], 5 * TILE_BYTES);
-    bulk_load(s.b2, tiles + S_B2 * TILE_BYTES, 2 * TILE_BYTES, &sm.bar_full[n & 1]);
+    bulk_load(s.cm, tiles + S_C * TILE_BYTES, 2 * TILE_BYTES, &sm.bar_full[n & 1]);
     bulk_load(s.at, tiles + S_AT * TILE_BYTES, TILE_BYTES, &sm.bar_full[n & 1]);
     bulk_load(s.qt, tiles + S_QT * TILE_BYTES, TILE_BYTES, &sm.bar_full[n & 1]);
     tma_load_4d(s.dout, &tmap_do, &sm.bar_full[n & 1], 0, tb + c * L, hi, brow);
   };
+  auto mma_ahead = [&](int n) {       // warp 0's thread: what the n-th chunk does not need dh for
+    BScanStage& s = sm.st[n & 1];
+    if (!mbar_wait(&sm.bar_full[n & 1], (n >> 1) & 1, status, 311)) return false;
+    umma_tile<64, 64, 1, 1>(tmem_addr(tm, 16, 64 * (n & 1)), smem_u32(s.cm), smem_u32(s.dout), false);    // C^T do
+    umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 64 * (n & 1)), smem_u32(s.qt), smem_u32(s.dout), false);     // q~^T do
+    return true;
+  };
+  bool ok = true;          // the same in every thread at the loop's head: the result of the last barrier
   if (warp == 0 && elect_one()) {
     issue_loads(0);
     if (NT > 1) issue_loads(1);
+    ok = mma_ahead(0);
   }
 
   // gradient of the state after the current chunk, row k of dh[k][v] = d_ht[v][k]
@@ -226,11 +106,12 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
     dc_next = ws_aux[(ch0 + NT - 1) * AUX_FLOATS + 64 + row];
     e0_next = ws_aux[(ch0 + NT - 1) * AUX_FLOATS + row];
   }
-  bool ok = true;          // the same in every thread at the loop's head: the result of the last barrier
-  bool tail_ok = true;     // this thread's wait at the end of the previous chunk
+  bool tail_ok = ok;       // this thread's wait at the end of the previous chunk
+  ok = true;
   for (int n = 0; n < NT && ok; ++n) {
     const int c = NT - 1 - n;
     BScanStage& s = sm.st[n & 1];
+    const uint32_t tm_w = tmem_addr(tm, 32 * wq, 64 * (n & 1) + c0);
     unsigned char* tiles = ws_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES;
     const float dc = fabsf(dc_next), e0 = e0_next;
     if (state_lane) {
@@ -242,20 +123,13 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
         e0_next = ws_aux[(ch0 + c - 1) * AUX_FLOATS + row];
       }
     }
-    ok = tail_ok && mbar_wait(&sm.bar_full[n & 1], (n >> 1) & 1, status, 311);
     if (warp == st_warp && elect_one()) bulk_wait_read();    // the copy of the previous chunk's dz has left its tile, rewritten below
     fence_async_smem();
     tc_fence_before();
-    ok = __syncthreads_and(ok);
+    ok = __syncthreads_and(tail_ok);
     if (warp == 0 && elect_one() && ok) {
       tc_fence_after();
-      umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 0), smem_u32(s.b2), smem_u32(sm.dhh), false);   // B2 dh^
-      if (!spread) umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 0), smem_u32(s.qt), smem_u32(s.dout), false);    // q~^T do
-      umma_commit(&sm.bar_m1);
-    }
-    if (spread && warp == 3 && elect_one() && ok) {
-      tc_fence_after();
-      umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 0), smem_u32(s.qt), smem_u32(s.dout), false);    // q~^T do
+      umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 64 * (n & 1)), smem_u32(s.b2), smem_u32(sm.dhh), true);   // += B2 dh^
       umma_commit(&sm.bar_m1);
     }
     if (warp == st_warp && elect_one() && ok) {
@@ -268,11 +142,10 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
       uint32_t r[32];
       tmem_ld32(tm_w, r);
       tmem_ld_wait();
-      if (!state_lane) {      // dz = P2 + B2 dh^
-        float x[32], p[32];
-        tile_load_row32(s.p2, row, c0, p);
+      if (!state_lane) {      // dz = C^T do + B2 dh^
+        float x[32];
 #pragma unroll
-        for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(r[j]) + p[j];
+        for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(r[j]);
         tile_store_row32(sm.dz, row, c0, x);
       }
     }
@@ -282,8 +155,10 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
     ok = __syncthreads_and(ok);
     if (warp == 0 && elect_one() && ok) {
       tc_fence_after();
-      umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 0), smem_u32(s.at), smem_u32(sm.dz), true);      // += a~^T dz
+      umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 64 * (n & 1)), smem_u32(s.at), smem_u32(sm.dz), true);      // += a~^T dz
       umma_commit(&sm.bar_m2);
+      // the next chunk's accumulators were read out before the barrier at the head of this one
+      if (n + 1 < NT) ok = mma_ahead(n + 1);
     }
     if (warp == st_warp && elect_one() && ok) {
       bulk_store(tiles + S_DZ * TILE_BYTES, sm.dz, TILE_BYTES);
@@ -291,7 +166,7 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
     }
     tail_ok = ok && mbar_wait(&sm.bar_m2, n & 1, status, 313);
     tc_fence_after();
-    // this stage has been read: p2 by every thread before the last barrier, the rest by the two MMA groups
+    // this stage has been read by the two MMA groups
     if (warp == ld_warp && elect_one() && tail_ok && n + 2 < NT) issue_loads(n + 2);
     if (tail_ok) {
       uint32_t r[32];
@@ -312,11 +187,11 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
   }
   if (warp == st_warp && elect_one()) bulk_wait_all();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tm, 64);
+  if (warp == 0) tmem_dealloc(tm, 128);
 }
 
 // ---------------------------------------------------------------------------------------------
-// 5. all token gradients of one chunk: persistent CTAs of 256 threads over the B*H*NT chunk-heads
+// 4. all token gradients of one chunk: persistent CTAs of 256 threads over the B*H*NT chunk-heads
 // ---------------------------------------------------------------------------------------------
 // What bounds it: per chunk-head about 14 k warp instructions in phases that wait for one another (tiles ->
 // products -> read-out -> products -> read-out -> prefix sums).  With one CTA per SM (213 KB of shared memory) the
@@ -398,7 +273,8 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     tma_load_4d(sm.dout, &tmap_do, &sm.bar_l1, 0, sv.first<PACKED>(p.bi) + p.c * L, p.hi, sv.row<PACKED>(p.bi));
     bulk_load(sm.dz, tiles + S_DZ * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
     bulk_load(sm.sa, tiles + S_SA * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
-    bulk_load(sm.aqk, tiles + S_AQK * TILE_BYTES, 2 * TILE_BYTES, &sm.bar_l1);
+    bulk_load(sm.aqk, tiles + S_AQK * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
+    bulk_load(sm.aak, tiles + S_AAK * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
   };
   auto load_2 = [&](const ChunkPos& p) {      // k~; q~, a~, b~ (MMA group 2 and the epilogue)
     const unsigned char* tiles = ws_tiles + (size_t)p.ch * tiles_per_chunk * TILE_BYTES;
@@ -420,9 +296,9 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     if (elect_one()) {
       tma_prefetch_4d(&tmap_do, 0, sv.first<PACKED>(p.bi) + t0, p.hi, sv.row<PACKED>(p.bi));
       tma_prefetch_4d(&tmap_v, 0, sv.first<PACKED>(p.bi) + t0, p.hi, sv.row<PACKED>(p.bi));
-      bulk_prefetch_l2(tiles + S_QT * TILE_BYTES, 3 * TILE_BYTES);     // q~, k~, b~
-      bulk_prefetch_l2(tiles + S_AT * TILE_BYTES, 3 * TILE_BYTES);     // a~, A_qk, A_ak
-      bulk_prefetch_l2(tiles + S_SA * TILE_BYTES, 3 * TILE_BYTES);     // sa, h~0, X
+      bulk_prefetch_l2(tiles + S_KT * TILE_BYTES, 2 * TILE_BYTES);     // k~, A_qk
+      bulk_prefetch_l2(tiles + S_QT * TILE_BYTES, 2 * TILE_BYTES);     // q~, b~
+      bulk_prefetch_l2(tiles + S_AT * TILE_BYTES, 5 * TILE_BYTES);     // a~, A_ak, sa, h~0, X
       bulk_prefetch_l2(tiles + S_DZ * TILE_BYTES, 2 * TILE_BYTES);     // dz, dh^
     }
   };
@@ -853,32 +729,21 @@ int launch_rwkv7_chunked_bwd(const void* r, const void* w, const void* k, const 
   TokLayout lay(mapT, H, head_first);
   // every kernel exists for dense batches and for packed variable-length ones
 #define R7C_DISPATCH_PACKED(...) do { if (seq_start) { constexpr bool P = true; __VA_ARGS__; } else { constexpr bool P = false; __VA_ARGS__; } } while (0)
-  if (phases & PHASE_PREPARE) {
-    const int smem = (int)sizeof(PreSmem) + 1024;
-    const int sms = dev.sms;
-    const int pre_grid = B * H * NT < 2 * sms ? B * H * NT : 2 * sms;     // persistent: two CTAs per SM
-    ProfScope prof("r7c_bwd_pre_kernel", st);
-    R7C_DISPATCH_PACKED(
-      if (allow_smem<r7c_bwd_pre_kernel<P>>(dev, smem)) return RWKVB200_E_CUDA;
-      r7c_bwd_pre_kernel<P><<<pre_grid, 128, smem, st>>>(tmap_do, ws.tiles, ALL_TILES, sv, H, NT, B * H * NT, status));
-  }
-  e = check_launch();
-  if (e) return e;
   if (phases & PHASE_SCAN) {
     const int smem = (int)sizeof(BScanSmem) + 1024;
-    const int sms = dev.sms;
     ProfScope prof("r7c_bwd_scan_kernel", st);
     R7C_DISPATCH_PACKED(
       if (allow_smem<r7c_bwd_scan_kernel<P>>(dev, smem)) return RWKVB200_E_CUDA;
       r7c_bwd_scan_kernel<P><<<B * H, 256, smem, st>>>(tmap_do, ws.tiles, ws.aux, ALL_TILES, d_ht, d_h0, sv, H, NT,
-                                                       B * H <= sms ? 1 : 0, status));
+                                                       status));
   }
   e = check_launch();
   if (e) return e;
   // Units the forward marked (decay beyond the range of the scaled operands, or a very short sequence): their
   // gradients come from the float32 recurrence instead.  Its state checkpoints (16 KB per 8 tokens = 128 KB per
-  // chunk) go into the unit's own tile region of the workspace (144 KB per chunk), whose contents are void for
+  // chunk) go into the unit's own tile region of the workspace (as much per chunk), whose contents are void for
   // such a unit.
+  static_assert(ALL_TILES * TILE_BYTES >= L / R7_CKPT * HS * HS * (int)sizeof(float), "checkpoints fit a unit's tiles");
   auto exact_units = [&]() -> int {
     const long long unit_floats = (long long)NT * ALL_TILES * TILE_BYTES / (long long)sizeof(float);
     float* ckpt = reinterpret_cast<float*>(ws.tiles);

@@ -23,10 +23,10 @@ struct IntraSmem {
   unsigned char qt[TILE_BYTES], at[TILE_BYTES];     // [q~; a~]  (128-row A operand)
   unsigned char kt[TILE_BYTES], bt[TILE_BYTES];     // [k~; b~]  (128-row B operand)
   unsigned char aqk[TILE_BYTES], aak[TILE_BYTES];   // [A_qk; A_ak] (128-row A operand); aak later holds W
-  unsigned char o1[TILE_BYTES];                     // A_qk v
+  unsigned char cm[TILE_BYTES];                     // C = A_qb Ainv
   unsigned char aqb[TILE_BYTES];
   unsigned char v[TILE_BYTES];                      // TMA; later U
-  unsigned char ainv[TILE_BYTES];
+  unsigned char ainv[TILE_BYTES];                   // later holds B2
   unsigned char y[TILE_BYTES];                      // A_ak v
   float nmat[L * NROW];                             // stril(A_ab) in fp32
   float qtot[4][64];                                // sums of g over the four quarters of the chunk
@@ -36,7 +36,7 @@ struct IntraSmem {
 
 // Persistent: CTAs (two per SM) walk over chunk-heads ch = blockIdx.x, blockIdx.x + gridDim.x, ...  The
 // raw q, k, a, b, w tiles of the next chunk-head are requested by TMA as soon as the tiles they land in
-// (q~, k~, a~, b~, which are then scaled in place, and O1) have been copied out, its v tile as soon as
+// (q~, k~, a~, b~, which are then scaled in place, and A_qk) have been copied out, its v tile as soon as
 // MMA 2 has read the current one, and the rows of the one after that are asked into L2.
 // 256 threads: warp w reads TMEM lanes 32*(w&3).. and the two warps that share a lane window split
 // the columns (hsel = w>>2); the triangular solve runs on warps 0-1 while the other warps drain MMA 2.
@@ -81,21 +81,22 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
     mbar_expect_tx(&sm.bar_w, TILE_BYTES);
     tma_load_4d(sm.aqk, &tmap_w, &sm.bar_w, 0, sv.first<PACKED>(bi) + t0, hi, sv.row<PACKED>(bi));
   };
-  // q, k, b land in tiles that only MMA 1 reads and are requested as soon as MMA 2 has completed (their
-  // copies to the workspace have left shared memory by then); a lands in the tile MMA 3 reads and is requested
-  // after it: both are on their way most of a chunk-head before the next one needs them.
-  auto load_qkb = [&](const ChunkPos& p) {     // tid 0
+  // q, k land in tiles that only MMA 1 reads and are requested as soon as MMA 2 has completed (their
+  // copies to the workspace have left shared memory by then); a, b land in tiles that MMA 3 reads and are requested
+  // after it (the rows have been asked into L2 by then).
+  auto load_qk = [&](const ChunkPos& p) {     // tid 0
     int bi, hi, t0; coords(p, bi, hi, t0);
     const int tt = sv.first<PACKED>(bi) + t0, br = sv.row<PACKED>(bi);
-    mbar_expect_tx(&sm.bar_in, 3 * TILE_BYTES);
+    mbar_expect_tx(&sm.bar_in, 2 * TILE_BYTES);
     tma_load_4d(sm.qt, &tmap_q, &sm.bar_in, 0, tt, hi, br);
     tma_load_4d(sm.kt, &tmap_k, &sm.bar_in, 0, tt, hi, br);
-    tma_load_4d(sm.bt, &tmap_b, &sm.bar_in, 0, tt, hi, br);
   };
-  auto load_a = [&](const ChunkPos& p) {       // tid 0
+  auto load_ab = [&](const ChunkPos& p) {      // tid 0
     int bi, hi, t0; coords(p, bi, hi, t0);
-    mbar_expect_tx(&sm.bar_ia, TILE_BYTES);
-    tma_load_4d(sm.at, &tmap_a, &sm.bar_ia, 0, sv.first<PACKED>(bi) + t0, hi, sv.row<PACKED>(bi));
+    const int tt = sv.first<PACKED>(bi) + t0, br = sv.row<PACKED>(bi);
+    mbar_expect_tx(&sm.bar_ia, 2 * TILE_BYTES);
+    tma_load_4d(sm.at, &tmap_a, &sm.bar_ia, 0, tt, hi, br);
+    tma_load_4d(sm.bt, &tmap_b, &sm.bar_ia, 0, tt, hi, br);
   };
   // chunk slots past the end of a (packed) sequence are skipped
   auto empty = [&](const ChunkPos& p) {
@@ -131,7 +132,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
   };
   ChunkPos cur = chunk_pos(blockIdx.x, NT, H);
   if (cur.ch < n_ch && empty(cur)) cur = advance(cur);
-  if (cur.ch < n_ch && warp == 0 && elect_one()) { load_w(cur); load_qkb(cur); load_a(cur); load_v(cur); }
+  if (cur.ch < n_ch && warp == 0 && elect_one()) { load_w(cur); load_qk(cur); load_ab(cur); load_v(cur); }
   // The two CTAs that share an SM would otherwise run their phases in lockstep and compete for the
   // same unit (shared-memory pipe during the triangular solve); start every other CTA half a
   // chunk-head late (unless it has a single one to do, or none: then the delay would be all it adds).
@@ -208,7 +209,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
         ws_aux[(size_t)ch * AUX_FLOATS + 64 + tid] = copysignf(ex2(fmaxf(tot1, EXP2_FLOOR)), mark ? -1.f : 1.f);   // e^{glast-gref}
       }
       // the raw q, k, a, b: each thread scales its own 2 x 16 bytes in place (the previous chunk-head's W, U,
-      // A_qb, O1 copies may still be reading their tiles: those are rewritten only after MMA 1)
+      // A_qb copies may still be reading their tiles: those are rewritten only after MMA 1)
       uint4 rq[2], rk[2], ra[2], rb[2];
       ok = mbar_wait(&sm.bar_in, par, status, 207) && ok;
       ok = mbar_wait(&sm.bar_ia, par, status, 208) && ok;
@@ -347,20 +348,21 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
     ok = __syncthreads_and(ok);
 
     R7C_STAMP(4);
-    // ---- MMA 2: [A_qk; A_ak] v  ->  TMEM columns 128..191 (rows 0..63 = O1, 64..127 = Y)
+    // ---- MMA 2: [A_qk; A_ak] v  ->  TMEM columns 128..191 (rows 64..127 = Y; the scan computes A_qk v itself, and a
+    // 64-row product of A_ak alone takes the tensor pipe as long)
     if (warp == 0 && elect_one()) {
       ok = mbar_wait(&sm.bar_v, par, status, 202) && ok;
       tc_fence_after();
       umma_tile<128, 64, 0, 1>(tmem_addr(tm, 0, 128), smem_u32(sm.aqk), smem_u32(sm.v), false);
       umma_commit(&sm.bar_m2);
-      if (keep_for_bwd) {   // A_qk, A_ak, a~ are operands of the backward: copy them out before they are overwritten
-        bulk_store(out_tiles + S_AQK * TILE_BYTES, sm.aqk, TILE_BYTES);
+      bulk_store(out_tiles + S_AQK * TILE_BYTES, sm.aqk, TILE_BYTES);
+      if (keep_for_bwd) {   // A_ak, a~ are operands of the backward: copy them out before they are overwritten
         bulk_store(out_tiles + S_AAK * TILE_BYTES, sm.aak, TILE_BYTES);
         bulk_store(out_tiles + S_AT * TILE_BYTES, sm.at, TILE_BYTES);
-        bulk_commit();
       }
+      bulk_commit();
     }
-    // ---- rows of MMA 2 (warps 2-7), then Ainv = X = (I - N)^-1, N = stril(A_ab), by two levels of block
+    // ---- rows of MMA 2 (warps 2, 3, 6, 7), then Ainv = X = (I - N)^-1, N = stril(A_ab), by two levels of block
     // inversion:
     //   D. the four 16 x 16 diagonal blocks D_I = (I - N_II)^-1 in fp32, one column per thread, row by row --
     //      the only substitutions, all four side by side (in place in nmat);
@@ -392,37 +394,23 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
 #pragma unroll
         for (int rr = 0; rr < 16; ++rr) sm.nmat[(16 * I + rr) * NROW + c] = xb[rr];
       }
-      if (warp >= 2) {
-        // warps 4-5 take O1 (both column halves), warps 2-3 and 6-7 take Y (one column half each)
+      if (wq >= 2) {      // Y, one column half per warp
         ok = mbar_wait(&sm.bar_m2, par, status, 203) && ok;
         tc_fence_after();
         const int i = (32 * wq + lane) & 63;
-        if (wq < 2) {        // warps 4, 5
+        uint32_t rr[32];
+        tmem_ld32(tmem_addr(tm, 32 * wq, 128 + 32 * hsel), rr);
+        tmem_ld_wait();
+        float x[32];
 #pragma unroll
-          for (int part = 0; part < 2; ++part) {
-            uint32_t rr[32];
-            tmem_ld32(tmem_addr(tm, 32 * wq, 128 + 32 * part), rr);
-            tmem_ld_wait();
-            float x[32];
-#pragma unroll
-            for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
-            tile_store_row32(sm.o1, i, 32 * part, x);
-          }
-        } else {             // warps 2, 3, 6, 7
-          uint32_t rr[32];
-          tmem_ld32(tmem_addr(tm, 32 * wq, 128 + 32 * hsel), rr);
-          tmem_ld_wait();
-          float x[32];
-#pragma unroll
-          for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
-          tile_store_row32(sm.y, i, 32 * hsel, x);
-        }
+        for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
+        tile_store_row32(sm.y, i, 32 * hsel, x);
       }
       // the scratch area: MMA 2 (and the copies of A_qk / A_ak kept for the backward) must be done with it
       ok = mbar_wait(&sm.bar_m2, par, status, 205) && ok;
       if (warp == 0 && elect_one()) {
         bulk_wait_read();                  // q~, k~, b~ (and the tiles kept for the backward) have left shared memory
-        if (next < n_ch) { load_v(nxt); load_qkb(nxt); }      // MMA 2 has read the v tile; nothing reads q~, k~, b~ any more
+        if (next < n_ch) { load_v(nxt); load_qk(nxt); }       // MMA 2 has read the v tile; nothing reads q~, k~ any more
       }
       __syncthreads();
       R7C_STAMP(10);
@@ -533,16 +521,19 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
     ok = __syncthreads_and(ok);
 
     R7C_STAMP(6);
-    // ---- MMA 3: W = Ainv a~ (lower lane halves), U = Ainv Y (upper lane halves) -> TMEM columns 0..63
+    // ---- MMA 3: W = Ainv a~ (lower lane halves), U = Ainv Y (upper lane halves) -> TMEM columns 0..63; for the
+    // backward B2 = Ainv^T b~ and C = A_qb Ainv -> columns 64..127
     if (warp == 0 && elect_one()) {
       if (ok && next < n_ch) load_w(nxt);      // the scratch area in the A_qk tile is free again
       tc_fence_after();
       umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 0), smem_u32(sm.ainv), smem_u32(sm.at), false);
       umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 0), smem_u32(sm.ainv), smem_u32(sm.y), false);
+      if (keep_for_bwd) {
+        umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 64), smem_u32(sm.ainv), smem_u32(sm.bt), false);
+        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 64), smem_u32(sm.aqb), smem_u32(sm.ainv), false);
+      }
       umma_commit(&sm.bar_m3);
       bulk_store(out_tiles + S_AQB * TILE_BYTES, sm.aqb, TILE_BYTES);
-      bulk_store(out_tiles + S_O1 * TILE_BYTES, sm.o1, TILE_BYTES);
-      if (keep_for_bwd) bulk_store(out_tiles + S_AINV * TILE_BYTES, sm.ainv, TILE_BYTES);
       bulk_commit();
     }
     ok = mbar_wait(&sm.bar_m3, par, status, 204) && ok;
@@ -550,16 +541,20 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
     R7C_STAMP(7);
 
     {
-      // W -> the A_ak tile (free since MMA 2), U -> the Y tile (free: MMA 3 has completed)
+      // W -> the A_ak tile (free since MMA 2), U -> the Y tile, B2 -> the Ainv tile (free: MMA 3 has completed)
       const int i = 16 * wq + (lane & 15);
-      unsigned char* dst = lane < 16 ? sm.aak : sm.y;
-      uint32_t rr[32];
-      tmem_ld32(tmem_addr(tm, 32 * wq, 32 * hsel), rr);
-      tmem_ld_wait();
-      float x[32];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
-      tile_store_row32(dst, i, 32 * hsel, x);
+      for (int part = 0; part < 2; ++part) {
+        if (part && !keep_for_bwd) break;
+        unsigned char* dst = part ? (lane < 16 ? sm.ainv : sm.cm) : (lane < 16 ? sm.aak : sm.y);
+        uint32_t rr[32];
+        tmem_ld32(tmem_addr(tm, 32 * wq, 64 * part + 32 * hsel), rr);
+        tmem_ld_wait();
+        float x[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
+        tile_store_row32(dst, i, 32 * hsel, x);
+      }
     }
     fence_async_smem();
     tc_fence_before();
@@ -568,9 +563,13 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
     if (warp == 0 && elect_one() && ok) {
       bulk_store(out_tiles + S_W * TILE_BYTES, sm.aak, TILE_BYTES);
       bulk_store(out_tiles + S_U * TILE_BYTES, sm.y, TILE_BYTES);
+      if (keep_for_bwd) {
+        bulk_store(out_tiles + S_C * TILE_BYTES, sm.cm, TILE_BYTES);
+        bulk_store(out_tiles + S_B2 * TILE_BYTES, sm.ainv, TILE_BYTES);
+      }
       bulk_commit();
-      // MMA 3 has read a~ (and its copy for the backward left shared memory long ago): the next raw a may land
-      if (next < n_ch) load_a(nxt);
+      // MMA 3 has read a~ and b~ (their copies left shared memory long ago): the next raw a, b may land
+      if (next < n_ch) load_ab(nxt);
     }
     R7C_STAMP(9);
   }
@@ -582,36 +581,43 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
 }
 
 // ---------------------------------------------------------------------------------------------
-// scan kernel: grid = B*H, 256 threads, chunks in order, fp32 state in TMEM.  Warp w reads TMEM lanes
-// 32*(w&3)..; the two warps that share a lane window take 32 of the 64 columns each (hsel = w>>2).
+// scan kernel: grid = B*H, 256 threads, chunks in order.  Warp w reads TMEM lanes 32*(w&3)..; the two warps that share a
+// lane window take 32 of the 64 columns each (hsel = w>>2).  Lanes 0-15 of a warp own state rows, lanes 16-31 token rows.
 // ---------------------------------------------------------------------------------------------
-// Operand tiles come in two groups, each requested again the moment the MMAs that read it have completed.
-// STAGES = 1 (single-buffered, 11 tiles = 88 KB): two CTAs (two sequences) share an SM, the choice when
-// there are more sequences than SMs; U and O1, which are only added row by row, do not enter shared
+// What bounds it: with more sequences than SMs, memory (eight tiles in, four out per chunk); with fewer, the chain
+// from chunk to chunk, W h~0 -> sa -> b~^T sa -> h.  Everything else is kept off that chain: the state stays in registers
+// (fp32) and takes its update from an accumulator that starts at zero, so k~^T v, A_qk v and q~ h~0 run beside the
+// read-outs; the output rows of a chunk are read out with sa of the next one; copies are waited for a phase after they
+// were issued; and one elected thread issues all MMAs in the order of that chain.
+// Operand tiles come in two groups, each requested again once the MMAs that read it have completed.
+// STAGES = 1 (single-buffered, 12 tiles = 96 KB): two CTAs (two sequences) share an SM, the choice when
+// there are more sequences than SMs; U, which is only added row by row, does not enter shared
 // memory: every thread fetches its row into registers at the top of a chunk.  STAGES = 2 (21 tiles): one
-// CTA per SM with the groups of chunk c + 2 requested during chunk c and U, O1 staged with group 1, for
+// CTA per SM with two chunks of operands in shared memory and U staged with group 1, for
 // the case of few sequences, where nothing else on the SM covers a load latency.
-template <int STAGES> struct ScanGroup1 {
-  unsigned char qt[TILE_BYTES], kt[TILE_BYTES];   // read by step a: q~, k~ (adjacent slots)
-  unsigned char w[TILE_BYTES], v[TILE_BYTES];     //                 W, v (TMA)
+template <int STAGES> struct ScanGroup1 {         // free once W h~0 and q~ h~0 have been computed
+  unsigned char kt[TILE_BYTES], aqk[TILE_BYTES], w[TILE_BYTES];   // adjacent slots
+  unsigned char v[TILE_BYTES], qt[TILE_BYTES];
+};
+template <int STAGES> struct ScanGroup2 {         // free at the end of the chunk
+  unsigned char bt[TILE_BYTES], aqb[TILE_BYTES];  // adjacent slots
 };
 template <> struct ScanGroup1<2> {
-  unsigned char qt[TILE_BYTES], kt[TILE_BYTES];
-  unsigned char o1[TILE_BYTES], w[TILE_BYTES], u[TILE_BYTES];   // adjacent slots O1, W, U: one copy
+  unsigned char kt[TILE_BYTES], aqk[TILE_BYTES], w[TILE_BYTES], u[TILE_BYTES];
   unsigned char v[TILE_BYTES];
 };
-struct ScanGroup2 {
-  unsigned char bt[TILE_BYTES], aqb[TILE_BYTES];  // read by step c: b~, A_qb (adjacent slots)
+template <> struct ScanGroup2<2> {                // here q~ h~0 runs beside the read-out of sa: q~ is free later
+  unsigned char qt[TILE_BYTES], bt[TILE_BYTES], aqb[TILE_BYTES];
 };
 template <int STAGES>
 struct ScanSmem {
   ScanGroup1<STAGES> g1[STAGES];
-  ScanGroup2 g2[STAGES];
-  unsigned char ht[TILE_BYTES];             // h~0 as bf16, [k][v]
+  ScanGroup2<STAGES> g2[STAGES];
+  unsigned char ht[2][TILE_BYTES];          // h~0 as bf16, [k][v]
   unsigned char sa[TILE_BYTES];             // sa as bf16, [token][v]
   unsigned char xt[TILE_BYTES];             // X = h~0 + k~^T v + b~^T sa as bf16 (kept for the backward)
-  unsigned char ot[2][TILE_BYTES];          // output rows of a chunk, staged for a TMA store
-  uint64_t bar_g1[STAGES], bar_g2[STAGES], bar_a, bar_c;
+  unsigned char ot[TILE_BYTES];             // output rows of a chunk, staged for a TMA store
+  uint64_t bar_g1[STAGES], bar_g2[STAGES], bar_a, bar_c, bar_o;
   uint32_t tmem_base;
 };
 
@@ -639,222 +645,277 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
   const int NT = (Tn + L - 1) / L;           // chunks of this sequence (at least one)
   const int row = 16 * wq + (lane & 15);     // state row k (lanes 0-15) or token row i (lanes 16-31)
   const bool state_lane = lane < 16;
-  // With one CTA per SM the single-thread jobs of a chunk lie on the chain from chunk to chunk: they go to one thread of
-  // each of four warps and run side by side.  Warps 0, 1 and 2 issue the MMAs, one accumulator each, ld_warp requests
-  // operand tiles, st_warp copies sa and h~0 out for the backward, out_warp copies X and the output rows out.  Bulk-copy
-  // groups belong to the thread that committed them, so each storing thread waits for its own copies.  With
-  // two CTAs per SM the other CTA fills such gaps and warp 0 keeps all four jobs.
-  constexpr bool SPREAD = STAGES == 2;
-  constexpr int ld_warp = SPREAD ? 1 : 0, st_warp = SPREAD ? 2 : 0, out_warp = SPREAD ? 3 : 0;
+  // Single-thread jobs: warp 0 issues the MMAs, ld_warp requests operand tiles, st_warp copies sa, h~0 and X out for the
+  // backward, out_warp the output rows.  Bulk-copy groups belong to the thread that committed them, so each storing
+  // thread waits for its own copies.
+  constexpr int ld_warp = 1, st_warp = 2, out_warp = 3;
+  constexpr bool AHEAD = STAGES == 2;      // k~^T v and A_qk v of the next chunk are issued at the end of this one
 
   if (tid == 0) {
     for (int i = 0; i < STAGES; ++i) { mbar_init(&sm.bar_g1[i], 1); mbar_init(&sm.bar_g2[i], 1); }
-    // with one CTA per SM each accumulator of an MMA group has its own issuing thread, and a group completes with all
-    // arrivals
-    mbar_init(&sm.bar_a, SPREAD ? 3 : 1); mbar_init(&sm.bar_c, SPREAD ? 2 : 1);
+    mbar_init(&sm.bar_a, 1); mbar_init(&sm.bar_c, 1); mbar_init(&sm.bar_o, 1);
     fence_mbar_init();
   }
-  if (warp == 0) tmem_alloc(&sm.tmem_base, 128);
+  if (warp == 0) tmem_alloc(&sm.tmem_base, 256);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tm = sm.tmem_base;
-  const uint32_t tm_p1 = tmem_addr(tm, 32 * wq, c0), tm_p2 = tmem_addr(tm, 32 * wq, 64 + c0);
+  // TMEM: columns 0..63 lower lane halves = W h~0; columns 64 + 64 p .., p = parity of the chunk: lower halves
+  // k~^T v + b~^T sa, upper halves the output rows
+  const uint32_t tm_sa = tmem_addr(tm, 32 * wq, c0);
 
-  auto issue_g1 = [&](int c) {      // ld_warp (warp 0 for the first chunks)
+  auto issue_g1 = [&](int c) {      // one thread
     const unsigned char* tiles = ws_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES;
     ScanGroup1<STAGES>& g = sm.g1[c % STAGES];
     uint64_t* bar = &sm.bar_g1[c % STAGES];
-    mbar_expect_tx(bar, (STAGES == 2 ? 6 : 4) * TILE_BYTES);
-    bulk_load(g.qt, tiles + S_QT * TILE_BYTES, 2 * TILE_BYTES, bar);
-    if constexpr (STAGES == 2) bulk_load(g.o1, tiles + S_O1 * TILE_BYTES, 3 * TILE_BYTES, bar);
-    else                       bulk_load(g.w, tiles + S_W * TILE_BYTES, TILE_BYTES, bar);
+    mbar_expect_tx(bar, 5 * TILE_BYTES);
+    bulk_load(g.kt, tiles + S_KT * TILE_BYTES, (STAGES == 2 ? 4 : 3) * TILE_BYTES, bar);
+    if constexpr (STAGES == 1) bulk_load(g.qt, tiles + S_QT * TILE_BYTES, TILE_BYTES, bar);
     tma_load_4d(g.v, &tmap_v, bar, 0, tb + c * L, hi, brow);
   };
-  auto issue_g2 = [&](int c) {      // ld_warp (warp 0 for the first chunks)
+  auto issue_g2 = [&](int c) {      // one thread
     const unsigned char* tiles = ws_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES;
     uint64_t* bar = &sm.bar_g2[c % STAGES];
-    mbar_expect_tx(bar, 2 * TILE_BYTES);
-    bulk_load(sm.g2[c % STAGES].bt, tiles + S_BT * TILE_BYTES, 2 * TILE_BYTES, bar);
+    mbar_expect_tx(bar, (STAGES == 2 ? 3 : 2) * TILE_BYTES);
+    if constexpr (STAGES == 2) bulk_load(sm.g2[c % STAGES].qt, tiles + S_QT * TILE_BYTES, 3 * TILE_BYTES, bar);
+    else                       bulk_load(sm.g2[c % STAGES].bt, tiles + S_BT * TILE_BYTES, 2 * TILE_BYTES, bar);
   };
-  if (warp == 0 && elect_one()) {
+  auto wait_g1 = [&](int c) { return mbar_wait(&sm.bar_g1[c % STAGES], (c / STAGES) & 1, status, 211); };
+  auto wait_g2 = [&](int c) { return mbar_wait(&sm.bar_g2[c % STAGES], (c / STAGES) & 1, status, 214); };
+  auto mma_kv = [&](int c) {        // the two products of a chunk that do not need the state
+    ScanGroup1<STAGES>& g = sm.g1[c % STAGES];
+    const uint32_t acc = 64 + 64 * (c & 1);
+    umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, acc), smem_u32(g.kt), smem_u32(g.v), false);
+    umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, acc), smem_u32(g.aqk), smem_u32(g.v), false);
+  };
+  if (warp == ld_warp && elect_one()) {
     for (int c = 0; c < STAGES && c < NT; ++c) { issue_g1(c); issue_g2(c); }
   }
 
-  // ---- initial state: h~0 = e^{gref(chunk 0)} h0, fp32 into TMEM (lower lane halves of P2), bf16 into ht
-  {
-    float x[32];
+  // ---- initial state: h~0 = e^{gref(chunk 0)} h0, fp32 in the registers of the state lanes, bf16 in the tile
+  float h[32];
 #pragma unroll
-    for (int vv = 0; vv < 32; ++vv) x[vv] = 0.f;
-    if (state_lane) {
-      const float e0 = ws_aux[ch0 * AUX_FLOATS + row];
-      if (n_state > 0) {
-        const float* S = h0 + (size_t)(n_state == 1 ? hi : unit) * 4096;   // S[v][k], h[k][v] = S[v][k]
+  for (int vv = 0; vv < 32; ++vv) h[vv] = 0.f;
+  if (state_lane) {
+    const float e0 = ws_aux[ch0 * AUX_FLOATS + row];
+    if (n_state > 0) {
+      const float* S = h0 + (size_t)(n_state == 1 ? hi : unit) * 4096;   // S[v][k], h[k][v] = S[v][k]
 #pragma unroll
-        for (int vv = 0; vv < 32; ++vv) x[vv] = e0 * S[(c0 + vv) * 64 + row];
-      }
-      tile_store_row32(sm.ht, row, c0, x);
+      for (int vv = 0; vv < 32; ++vv) h[vv] = e0 * S[(c0 + vv) * 64 + row];
     }
-    uint32_t r[32];
-#pragma unroll
-    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(x[j]);
-    tmem_st32(tm_p2, r);
-    tmem_st_wait();
+    tile_store_row32(sm.ht[0], row, c0, h);
+  }
+  bool ok = true;
+  if (AHEAD && warp == 0 && elect_one()) {
+    ok = wait_g1(0);
+    if (ok) mma_kv(0);
   }
   fence_async_smem();
   tc_fence_before();
-  __syncthreads();
+  ok = __syncthreads_and(ok);
 
-  bool ok = true;
   int marked = 0;       // a chunk's decay left the range of the scaled operands (the sign of its factors)
-  for (int c = 0; c < NT && ok; ++c) {
-    const int t0 = c * L;
-    R7C_STAMP(48);
-    // this thread's row of U (state lanes) or O1 (token lanes), straight from the workspace
-    uint4 addrow[4];
-    if constexpr (STAGES == 1) {
-      const unsigned char* tile = ws_tiles + ((ch0 + c) * (size_t)tiles_per_chunk + (state_lane ? S_U : S_O1)) * TILE_BYTES;
+  uint4 xp[4];          // X of the previous chunk, packed (state lanes)
+  auto store_x = [&]() {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) addrow[q] = __ldg(reinterpret_cast<const uint4*>(tile + tile_chunk_off(row, 4 * hsel + q)));
-      if (c + 1 < NT && hsel == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(tile + (size_t)tiles_per_chunk * TILE_BYTES + row * 128));
-    }
-    // decay factors needed at the end of this chunk, fetched early
-    // (applied one after the other: their product can underflow float32 where neither factor does)
-    float scale = 1.f, scale_next = 1.f;
-    if (state_lane) {
-      scale = ws_aux[(ch0 + c) * AUX_FLOATS + 64 + row];                       // e^{glast-gref} of this chunk
-      if (c + 1 < NT) scale_next = ws_aux[(ch0 + c + 1) * AUX_FLOATS + row];    // e^{gref} of the next chunk
-    }
-    // (a) SA = W h~0, QH = q~ h~0 (P1);  H += k~^T v (P2 lower)
-    if (warp < (SPREAD ? 3 : 1) && elect_one()) {
+    for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(sm.xt + tile_chunk_off(row, 4 * hsel + q)) = xp[q];
+  };
+  for (int c = 0; c < NT && ok; ++c) {
+    const int p = c & 1;
+    R7C_STAMP(48);
+    // (a) SA = W h~0, then q~ h~0
+    if (warp == 0 && elect_one()) {
       ScanGroup1<STAGES>& g = sm.g1[c % STAGES];
-      ok = mbar_wait(&sm.bar_g1[c % STAGES], (c / STAGES) & 1, status, 211);
-      R7C_STAMP(49);
+      if constexpr (!AHEAD) ok = wait_g1(c);
       if (ok) {
         tc_fence_after();
-        if (!SPREAD || warp == 0) umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 0), smem_u32(g.w), smem_u32(sm.ht), false);
-        if (!SPREAD || warp == 1) umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 0), smem_u32(g.qt), smem_u32(sm.ht), false);
-        if (!SPREAD || warp == 2) umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 64), smem_u32(g.kt), smem_u32(g.v), true);
-        umma_commit(&sm.bar_a);
+        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 0), smem_u32(g.w), smem_u32(sm.ht[p]), false);
+        if constexpr (AHEAD) {
+          umma_commit(&sm.bar_a);
+          ok = wait_g2(c);
+          if (ok) umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 64 + 64 * p), smem_u32(sm.g2[c % STAGES].qt), smem_u32(sm.ht[p]), true);
+        } else {
+          mma_kv(c);
+          umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 64 + 64 * p), smem_u32(g.qt), smem_u32(sm.ht[p]), true);
+          umma_commit(&sm.bar_a);
+        }
+      }
+    }
+    if (bwd_tiles && warp == st_warp && elect_one()) {
+      bulk_store(bwd_tiles + ((ch0 + c) * (size_t)tiles_per_chunk + S_H0) * TILE_BYTES, sm.ht[p], TILE_BYTES);
+      bulk_commit();
+    }
+    // this thread's row of U (state lanes), and the decay factors needed at the end of this chunk
+    // (applied one after the other: their product can underflow float32 where neither factor does)
+    uint4 addrow[4];
+    float scale = 1.f, scale_next = 1.f;
+    if (state_lane) {
+      if constexpr (STAGES == 1) {
+        const unsigned char* tile = ws_tiles + ((ch0 + c) * (size_t)tiles_per_chunk + S_U) * TILE_BYTES;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) addrow[q] = __ldg(reinterpret_cast<const uint4*>(tile + tile_chunk_off(row, 4 * hsel + q)));
+        if (c + 1 < NT && hsel == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(tile + (size_t)tiles_per_chunk * TILE_BYTES + row * 128));
+      }
+      scale = ws_aux[(ch0 + c) * AUX_FLOATS + 64 + row];                       // e^{glast-gref} of this chunk
+      if (c + 1 < NT) scale_next = ws_aux[(ch0 + c + 1) * AUX_FLOATS + row];    // e^{gref} of the next chunk
+      if (bwd_tiles && c > 0) store_x();
+    }
+    if constexpr (STAGES == 2) {
+      ok = ok && wait_g1(c);
+      if (state_lane) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) addrow[q] = *reinterpret_cast<const uint4*>(sm.g1[c % STAGES].u + tile_chunk_off(row, 4 * hsel + q));
       }
     }
     ok = ok && mbar_wait(&sm.bar_a, c & 1, status, 212);
     tc_fence_after();
     R7C_STAMP(50);
-    // group 1 has been read by the MMAs: request the next (the staged O1 / U rows are still to be read)
-    if (STAGES == 1 && warp == ld_warp && elect_one() && ok && c + STAGES < NT) issue_g1(c + STAGES);
-    float keep[32];     // token lanes: q~ h~0 + O1
-    if constexpr (STAGES == 2) {      // the staged O1 / U rows: observe the arrival of group 1 before reading them
-      ok = ok && mbar_wait(&sm.bar_g1[c % STAGES], (c / STAGES) & 1, status, 215);
-      const unsigned char* tile = state_lane ? sm.g1[c % STAGES].u : sm.g1[c % STAGES].o1;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) addrow[q] = *reinterpret_cast<const uint4*>(tile + tile_chunk_off(row, 4 * hsel + q));
-    }
+    // (b) sa = W h~0 + U (state lanes); the output rows of the previous chunk (token lanes)
     if (ok) {
-      uint32_t r[32];
-      tmem_ld32(tm_p1, r);
-      tmem_ld_wait();
-      float add[32];
+      unsigned char* dst = state_lane ? sm.sa : sm.ot;
+      const bool act = state_lane || (c > 0 && write_o);
+      const uint32_t tm_o = tmem_addr(tm, 32 * wq, 64 + 64 * (p ^ 1) + c0);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const uint4 u = addrow[q];
-        add[8 * q + 0] = bf16_lo(u.x); add[8 * q + 1] = bf16_hi(u.x);
-        add[8 * q + 2] = bf16_lo(u.y); add[8 * q + 3] = bf16_hi(u.y);
-        add[8 * q + 4] = bf16_lo(u.z); add[8 * q + 5] = bf16_hi(u.z);
-        add[8 * q + 6] = bf16_lo(u.w); add[8 * q + 7] = bf16_hi(u.w);
+      for (int half = 0; half < 2; ++half) {
+        uint32_t r[16], ro[16];
+        tmem_ld16(tm_sa + 16 * half, r);
+        tmem_ld16(tm_o + 16 * half, ro);
+        tmem_ld_wait();
+        float x[16];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const uint4 u = addrow[2 * half + q];
+          const uint32_t uu[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+          for (int m = 0; m < 4; ++m) {
+            const int j = 8 * q + 2 * m;
+            x[j] = state_lane ? __uint_as_float(r[j]) + bf16_lo(uu[m]) : __uint_as_float(ro[j]);
+            x[j + 1] = state_lane ? __uint_as_float(r[j + 1]) + bf16_hi(uu[m]) : __uint_as_float(ro[j + 1]);
+          }
+        }
+        if (act) {
+#pragma unroll
+          for (int q = 0; q < 2; ++q)
+            *reinterpret_cast<uint4*>(dst + tile_chunk_off(row, 4 * hsel + 2 * half + q)) =
+                make_uint4(pack_bf16(x[8 * q], x[8 * q + 1]), pack_bf16(x[8 * q + 2], x[8 * q + 3]),
+                           pack_bf16(x[8 * q + 4], x[8 * q + 5]), pack_bf16(x[8 * q + 6], x[8 * q + 7]));
+        }
       }
-#pragma unroll
-      for (int j = 0; j < 32; ++j) keep[j] = __uint_as_float(r[j]) + add[j];
-      if (state_lane) tile_store_row32(sm.sa, row, c0, keep);   // sa = W h~0 + U
     }
     fence_async_smem();
     tc_fence_before();
     ok = __syncthreads_and(ok);
-    if (STAGES == 2 && warp == ld_warp && elect_one() && ok && c + STAGES < NT) issue_g1(c + STAGES);
-    if (bwd_tiles && warp == st_warp && elect_one() && ok) {   // the backward needs sa and h~0 of every chunk
-      unsigned char* dst = bwd_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES;
-      bulk_store(dst + S_SA * TILE_BYTES, sm.sa, TILE_BYTES);
-      bulk_store(dst + S_H0 * TILE_BYTES, sm.ht, TILE_BYTES);
-      bulk_commit();
-    }
-    // (c) H += b~^T sa (P2 lower);  OQ = A_qb sa (P2 upper)
     R7C_STAMP(51);
-    if (warp < (SPREAD ? 2 : 1) && elect_one() && ok) {
-      ScanGroup2& g = sm.g2[c % STAGES];
-      ok = mbar_wait(&sm.bar_g2[c % STAGES], (c / STAGES) & 1, status, 214);
-      R7C_STAMP(52);
+    // (c) H += b~^T sa, then the rest of the output rows, A_qb sa
+    if (warp == 0 && elect_one() && ok) {
+      ScanGroup2<STAGES>& g = sm.g2[c % STAGES];
+      if constexpr (!AHEAD) ok = wait_g2(c);
       if (ok) {
         tc_fence_after();
-        if (!SPREAD || warp == 0) umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 64), smem_u32(g.bt), smem_u32(sm.sa), true);
-        if (!SPREAD || warp == 1) umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 64), smem_u32(g.aqb), smem_u32(sm.sa), false);
+        umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 64 + 64 * p), smem_u32(g.bt), smem_u32(sm.sa), true);
         umma_commit(&sm.bar_c);
+        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 64 + 64 * p), smem_u32(g.aqb), smem_u32(sm.sa), true);
+        umma_commit(&sm.bar_o);
+        if (AHEAD && c + 1 < NT) {
+          ok = wait_g1(c + 1);
+          if (ok) mma_kv(c + 1);
+        }
       }
     }
+    if (warp == ld_warp && elect_one() && ok && c + STAGES < NT) issue_g1(c + STAGES);
+    if (bwd_tiles && warp == st_warp && elect_one() && ok) {   // the backward needs sa, h~0 and X of every chunk
+      unsigned char* tiles = bwd_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES;
+      bulk_store(tiles + S_SA * TILE_BYTES, sm.sa, TILE_BYTES);
+      if (c > 0) bulk_store(tiles - ((size_t)tiles_per_chunk - S_X) * TILE_BYTES, sm.xt, TILE_BYTES);
+      bulk_commit();
+    }
+    if (write_o && c > 0 && warp == out_warp && elect_one() && ok) {      // a chunk that is not the last one is whole
+      tma_store_4d(&tmap_o, sm.ot, 0, tb + (c - 1) * L, hi, brow);
+      bulk_commit();
+    }
+    R7C_STAMP(52);
     ok = ok && mbar_wait(&sm.bar_c, c & 1, status, 213);
     tc_fence_after();
     R7C_STAMP(53);
-    if (warp == ld_warp && elect_one() && ok && c + STAGES < NT) issue_g2(c + STAGES);     // group 2 has been read
-    if (bwd_tiles) {                                  // ht / sa are rewritten below and in the next chunk
-      if (warp == st_warp && elect_one()) bulk_wait_read();
-      __syncthreads();
-    }
-    R7C_STAMP(54);
+    // (d) X and the next h~0
     if (ok) {
       const bool last = c + 1 == NT;
       uint32_t r[32];
-      tmem_ld32(tm_p2, r);
+      tmem_ld32(tmem_addr(tm, 32 * wq, 64 + 64 * p + c0), r);
       tmem_ld_wait();
-      float x[32];
       if (state_lane) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) h[j] += __uint_as_float(r[j]);
         if (bwd_tiles) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(r[j]);
-          tile_store_row32(sm.xt, row, c0, x);
+          for (int q = 0; q < 4; ++q)
+            xp[q] = make_uint4(pack_bf16(h[8 * q], h[8 * q + 1]), pack_bf16(h[8 * q + 2], h[8 * q + 3]),
+                               pack_bf16(h[8 * q + 4], h[8 * q + 5]), pack_bf16(h[8 * q + 6], h[8 * q + 7]));
         }
         marked |= scale < 0.f;
         const float sc = fabsf(scale);
 #pragma unroll
-        for (int j = 0; j < 32; ++j) { x[j] = (__uint_as_float(r[j]) * sc) * scale_next; r[j] = __float_as_uint(x[j]); }
-        if (!last) {
-          tile_store_row32(sm.ht, row, c0, x);
-        } else if (ht) {
-          float* S = ht + (size_t)unit * 4096;
-#pragma unroll
-          for (int j = 0; j < 32; ++j) S[(c0 + j) * 64 + row] = x[j];
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(r[j]) + keep[j];
-        if (write_o) tile_store_row32(sm.ot[c & 1], row, c0, x);
+        for (int j = 0; j < 32; ++j) h[j] = (h[j] * sc) * scale_next;
+        if (!last) tile_store_row32(sm.ht[p ^ 1], row, c0, h);
       }
-      tmem_st32(tm_p2, r);   // state lanes: rescaled state; token lanes: unchanged
-      tmem_st_wait();
     }
+    // the copies out of sa, h~0, X and of the output rows have left their tiles: the next chunk rewrites them
+    if ((warp == st_warp || warp == out_warp) && elect_one()) bulk_wait_read();
+    if (warp == ld_warp && elect_one() && ok && c + STAGES < NT) {      // group 2 has been read
+      ok = mbar_wait(&sm.bar_o, c & 1, status, 216);
+      if (ok) issue_g2(c + STAGES);
+    }
+    R7C_STAMP(54);
     fence_async_smem();
     tc_fence_before();
     ok = __syncthreads_and(ok);
     R7C_STAMP(55);
-    if (bwd_tiles && warp == out_warp && elect_one() && ok) {
-      bulk_store(bwd_tiles + ((ch0 + c) * (size_t)tiles_per_chunk + S_X) * TILE_BYTES, sm.xt, TILE_BYTES);
-      bulk_commit();
-    }
-    if (write_o && ok) {
-      if (PACKED && t0 + L > Tn) {  // the last rows of the box belong to the next sequence: row by row
-        store_tile_rows<256>(o_rows + brow * lay.sb + hi * lay.sh + (long long)(tb + t0) * lay.st, lay.st,
-                             sm.ot[c & 1], Tn - t0, tid);
-      } else if (warp == out_warp && elect_one()) {           // rows past the end of the tensor are clipped by the TMA store
-        tma_store_4d(&tmap_o, sm.ot[c & 1], 0, tb + t0, hi, brow);
-        bulk_commit();
-        bulk_wait_read_1();              // the buffer of the previous chunk is free again
-      }
-    }
-    R7C_STAMP(56);
   }
 #undef R7C_STAMP
+  // ---- what the last chunk still holds: its output rows and X, and the final state
+  ok = ok && mbar_wait(&sm.bar_o, (NT - 1) & 1, status, 217);
+  tc_fence_after();
+  if (ok) {
+    uint32_t r[32];
+    tmem_ld32(tmem_addr(tm, 32 * wq, 64 + 64 * ((NT - 1) & 1) + c0), r);
+    tmem_ld_wait();
+    if (state_lane) {
+      if (bwd_tiles) store_x();
+      if (ht) {
+        float* S = ht + (size_t)unit * 4096;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) S[(c0 + j) * 64 + row] = h[j];
+      }
+    } else if (write_o) {
+      float x[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(r[j]);
+      tile_store_row32(sm.ot, row, c0, x);
+    }
+  }
+  fence_async_smem();
+  tc_fence_before();
+  ok = __syncthreads_and(ok);
+  if (ok) {
+    const int t0 = (NT - 1) * L;
+    if (bwd_tiles && warp == st_warp && elect_one()) {
+      bulk_store(bwd_tiles + ((ch0 + NT - 1) * (size_t)tiles_per_chunk + S_X) * TILE_BYTES, sm.xt, TILE_BYTES);
+      bulk_commit();
+    }
+    if (write_o) {
+      if (PACKED && t0 + L > Tn) {  // the last rows of the box belong to the next sequence: row by row
+        store_tile_rows<256>(o_rows + brow * lay.sb + hi * lay.sh + (long long)(tb + t0) * lay.st, lay.st, sm.ot, Tn - t0, tid);
+      } else if (warp == out_warp && elect_one()) {           // rows past the end of the tensor are clipped by the TMA store
+        tma_store_4d(&tmap_o, sm.ot, 0, tb + t0, hi, brow);
+        bulk_commit();
+      }
+    }
+  }
   if ((warp == st_warp || warp == out_warp) && elect_one()) bulk_wait_all();
   marked = __syncthreads_or(marked);
   if (tid == 0) ws_flags[unit] = marked;
-  if (warp == 0) tmem_dealloc(tm, 128);
+  if (warp == 0) tmem_dealloc(tm, 256);
   // A marked unit again, by the exact recurrence: 64 threads per 16 rows, in place of what the chunks gave (inside this
   // kernel, because a launch of its own over all units costs every call 2 us of device time and as much on the host).
   if (marked && exact.r && ok) {
