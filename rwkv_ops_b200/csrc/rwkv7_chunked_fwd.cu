@@ -584,45 +584,44 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
 // scan kernel: grid = B*H, 256 threads, chunks in order.  Warp w reads TMEM lanes 32*(w&3)..; the two warps that share a
 // lane window take 32 of the 64 columns each (hsel = w>>2).  Lanes 0-15 of a warp own state rows, lanes 16-31 token rows.
 // ---------------------------------------------------------------------------------------------
-// What bounds it: with more sequences than SMs, memory (eight tiles in, four out per chunk); with fewer, the chain
-// from chunk to chunk, W h~0 -> sa -> b~^T sa -> h.  Everything else is kept off that chain: the state stays in registers
-// (fp32) and takes its update from an accumulator that starts at zero, so k~^T v, A_qk v and q~ h~0 run beside the
-// read-outs; the output rows of a chunk are read out with sa of the next one; copies are waited for a phase after they
-// were issued; and one elected thread issues all MMAs in the order of that chain.
-// Operand tiles come in two groups, each requested again once the MMAs that read it have completed.
-// STAGES = 1 (single-buffered, 12 tiles = 96 KB): two CTAs (two sequences) share an SM, the choice when
-// there are more sequences than SMs; U, which is only added row by row, does not enter shared
-// memory: every thread fetches its row into registers at the top of a chunk.  STAGES = 2 (21 tiles): one
-// CTA per SM with two chunks of operands in shared memory and U staged with group 1, for
-// the case of few sequences, where nothing else on the SM covers a load latency.
-template <int STAGES> struct ScanGroup1 {         // free once W h~0 and q~ h~0 have been computed
+// For more sequences than SMs: two CTAs (two sequences) share an SM, and memory bounds it (eight tiles in, four out per
+// chunk).  The state stays in registers (fp32) and takes its update from an accumulator that starts at zero, so k~^T v and
+// A_qk v need no state; the output rows of a chunk are read out with sa of the next one; copies are waited for a phase
+// after they were issued.
+// Operand tiles come in two groups, each requested again once the MMAs that read it have completed.  U, which is only
+// added row by row, does not enter shared memory: every thread fetches its row into registers at the top of a chunk.
+struct ScanGroup1 {         // free once W h~0 and q~ h~0 have been computed
   unsigned char kt[TILE_BYTES], aqk[TILE_BYTES], w[TILE_BYTES];   // adjacent slots
   unsigned char v[TILE_BYTES], qt[TILE_BYTES];
 };
-template <int STAGES> struct ScanGroup2 {         // free at the end of the chunk
+struct ScanGroup2 {         // free at the end of the chunk
   unsigned char bt[TILE_BYTES], aqb[TILE_BYTES];  // adjacent slots
 };
-template <> struct ScanGroup1<2> {
-  unsigned char kt[TILE_BYTES], aqk[TILE_BYTES], w[TILE_BYTES], u[TILE_BYTES];
-  unsigned char v[TILE_BYTES];
-};
-template <> struct ScanGroup2<2> {                // here q~ h~0 runs beside the read-out of sa: q~ is free later
-  unsigned char qt[TILE_BYTES], bt[TILE_BYTES], aqb[TILE_BYTES];
-};
-template <int STAGES>
 struct ScanSmem {
-  ScanGroup1<STAGES> g1[STAGES];
-  ScanGroup2<STAGES> g2[STAGES];
+  ScanGroup1 g1;
+  ScanGroup2 g2;
   unsigned char ht[2][TILE_BYTES];          // h~0 as bf16, [k][v]
   unsigned char sa[TILE_BYTES];             // sa as bf16, [token][v]
   unsigned char xt[TILE_BYTES];             // X = h~0 + k~^T v + b~^T sa as bf16 (kept for the backward)
   unsigned char ot[TILE_BYTES];             // output rows of a chunk, staged for a TMA store
-  uint64_t bar_g1[STAGES], bar_g2[STAGES], bar_a, bar_c, bar_o;
+  uint64_t bar_g1, bar_g2, bar_a, bar_c, bar_o;
   uint32_t tmem_base;
 };
 
-template <int STAGES, bool PACKED>
-__global__ void __launch_bounds__(256, 3 - STAGES)
+// A marked unit again, by the exact recurrence: 64 threads per 16 rows, in place of what the chunks gave (inside the scan
+// kernels, because a launch of its own over all units costs every call 2 us of device time and as much on the host).
+__device__ __forceinline__ void exact_unit(r7rec::FwdArgs<bf16> args, unsigned char* smem, int tid, int unit, int hi, int brow,
+                                           int tb, int Tn, const float* h0, int n_state, float* ht, const TokLayout& lay) {
+  args.base = brow * lay.sb + hi * lay.sh + tb * lay.st;
+  args.Tn = Tn;
+  args.S0 = n_state > 0 ? h0 + (size_t)(n_state == 1 ? hi : unit) * 4096 : nullptr;
+  args.ht = ht ? ht + (size_t)unit * 4096 : nullptr;
+  static_assert(4 * sizeof(r7rec::FwdSmem<64>) <= sizeof(ScanSmem), "the recurrence runs in the scan's shared memory");
+  r7rec::fwd_rows<bf16, 64, 256>(args, reinterpret_cast<r7rec::FwdSmem<64>*>(smem)[tid >> 6], tid >> 6, tid & 63);
+}
+
+template <bool PACKED>
+__global__ void __launch_bounds__(256, 2)
 r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned char* __restrict__ ws_tiles,
                     const float* __restrict__ ws_aux, int* __restrict__ ws_flags, int tiles_per_chunk,
                     unsigned char* __restrict__ bwd_tiles,
@@ -635,8 +634,7 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
 #define R7C_STAMP(n) do {} while (0)
 #endif
   extern __shared__ unsigned char smem_raw[];
-  ScanSmem<STAGES>& sm =
-      *reinterpret_cast<ScanSmem<STAGES>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  ScanSmem& sm = *reinterpret_cast<ScanSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int wq = warp & 3, hsel = warp >> 2, c0 = 32 * hsel;
   const int unit = blockIdx.x, bi = unit / H, hi = unit % H;
@@ -649,10 +647,9 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
   // backward, out_warp the output rows.  Bulk-copy groups belong to the thread that committed them, so each storing
   // thread waits for its own copies.
   constexpr int ld_warp = 1, st_warp = 2, out_warp = 3;
-  constexpr bool AHEAD = STAGES == 2;      // k~^T v and A_qk v of the next chunk are issued at the end of this one
 
   if (tid == 0) {
-    for (int i = 0; i < STAGES; ++i) { mbar_init(&sm.bar_g1[i], 1); mbar_init(&sm.bar_g2[i], 1); }
+    mbar_init(&sm.bar_g1, 1); mbar_init(&sm.bar_g2, 1);
     mbar_init(&sm.bar_a, 1); mbar_init(&sm.bar_c, 1); mbar_init(&sm.bar_o, 1);
     fence_mbar_init();
   }
@@ -667,31 +664,17 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
 
   auto issue_g1 = [&](int c) {      // one thread
     const unsigned char* tiles = ws_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES;
-    ScanGroup1<STAGES>& g = sm.g1[c % STAGES];
-    uint64_t* bar = &sm.bar_g1[c % STAGES];
-    mbar_expect_tx(bar, 5 * TILE_BYTES);
-    bulk_load(g.kt, tiles + S_KT * TILE_BYTES, (STAGES == 2 ? 4 : 3) * TILE_BYTES, bar);
-    if constexpr (STAGES == 1) bulk_load(g.qt, tiles + S_QT * TILE_BYTES, TILE_BYTES, bar);
-    tma_load_4d(g.v, &tmap_v, bar, 0, tb + c * L, hi, brow);
+    mbar_expect_tx(&sm.bar_g1, 5 * TILE_BYTES);
+    bulk_load(sm.g1.kt, tiles + S_KT * TILE_BYTES, 3 * TILE_BYTES, &sm.bar_g1);
+    bulk_load(sm.g1.qt, tiles + S_QT * TILE_BYTES, TILE_BYTES, &sm.bar_g1);
+    tma_load_4d(sm.g1.v, &tmap_v, &sm.bar_g1, 0, tb + c * L, hi, brow);
   };
   auto issue_g2 = [&](int c) {      // one thread
     const unsigned char* tiles = ws_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES;
-    uint64_t* bar = &sm.bar_g2[c % STAGES];
-    mbar_expect_tx(bar, (STAGES == 2 ? 3 : 2) * TILE_BYTES);
-    if constexpr (STAGES == 2) bulk_load(sm.g2[c % STAGES].qt, tiles + S_QT * TILE_BYTES, 3 * TILE_BYTES, bar);
-    else                       bulk_load(sm.g2[c % STAGES].bt, tiles + S_BT * TILE_BYTES, 2 * TILE_BYTES, bar);
+    mbar_expect_tx(&sm.bar_g2, 2 * TILE_BYTES);
+    bulk_load(sm.g2.bt, tiles + S_BT * TILE_BYTES, 2 * TILE_BYTES, &sm.bar_g2);
   };
-  auto wait_g1 = [&](int c) { return mbar_wait(&sm.bar_g1[c % STAGES], (c / STAGES) & 1, status, 211); };
-  auto wait_g2 = [&](int c) { return mbar_wait(&sm.bar_g2[c % STAGES], (c / STAGES) & 1, status, 214); };
-  auto mma_kv = [&](int c) {        // the two products of a chunk that do not need the state
-    ScanGroup1<STAGES>& g = sm.g1[c % STAGES];
-    const uint32_t acc = 64 + 64 * (c & 1);
-    umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, acc), smem_u32(g.kt), smem_u32(g.v), false);
-    umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, acc), smem_u32(g.aqk), smem_u32(g.v), false);
-  };
-  if (warp == ld_warp && elect_one()) {
-    for (int c = 0; c < STAGES && c < NT; ++c) { issue_g1(c); issue_g2(c); }
-  }
+  if (warp == ld_warp && elect_one()) { issue_g1(0); issue_g2(0); }
 
   // ---- initial state: h~0 = e^{gref(chunk 0)} h0, fp32 in the registers of the state lanes, bf16 in the tile
   float h[32];
@@ -707,10 +690,6 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
     tile_store_row32(sm.ht[0], row, c0, h);
   }
   bool ok = true;
-  if (AHEAD && warp == 0 && elect_one()) {
-    ok = wait_g1(0);
-    if (ok) mma_kv(0);
-  }
   fence_async_smem();
   tc_fence_before();
   ok = __syncthreads_and(ok);
@@ -724,22 +703,17 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
   for (int c = 0; c < NT && ok; ++c) {
     const int p = c & 1;
     R7C_STAMP(48);
-    // (a) SA = W h~0, then q~ h~0
+    // (a) SA = W h~0, and the products that do not need sa: k~^T v (lower lane halves), A_qk v + q~ h~0 (upper)
+    const uint32_t acc = 64 + 64 * p;
     if (warp == 0 && elect_one()) {
-      ScanGroup1<STAGES>& g = sm.g1[c % STAGES];
-      if constexpr (!AHEAD) ok = wait_g1(c);
+      ok = mbar_wait(&sm.bar_g1, c & 1, status, 211);
       if (ok) {
         tc_fence_after();
-        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 0), smem_u32(g.w), smem_u32(sm.ht[p]), false);
-        if constexpr (AHEAD) {
-          umma_commit(&sm.bar_a);
-          ok = wait_g2(c);
-          if (ok) umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 64 + 64 * p), smem_u32(sm.g2[c % STAGES].qt), smem_u32(sm.ht[p]), true);
-        } else {
-          mma_kv(c);
-          umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 64 + 64 * p), smem_u32(g.qt), smem_u32(sm.ht[p]), true);
-          umma_commit(&sm.bar_a);
-        }
+        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 0), smem_u32(sm.g1.w), smem_u32(sm.ht[p]), false);
+        umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, acc), smem_u32(sm.g1.kt), smem_u32(sm.g1.v), false);
+        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, acc), smem_u32(sm.g1.aqk), smem_u32(sm.g1.v), false);
+        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, acc), smem_u32(sm.g1.qt), smem_u32(sm.ht[p]), true);
+        umma_commit(&sm.bar_a);
       }
     }
     if (bwd_tiles && warp == st_warp && elect_one()) {
@@ -751,22 +725,13 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
     uint4 addrow[4];
     float scale = 1.f, scale_next = 1.f;
     if (state_lane) {
-      if constexpr (STAGES == 1) {
-        const unsigned char* tile = ws_tiles + ((ch0 + c) * (size_t)tiles_per_chunk + S_U) * TILE_BYTES;
+      const unsigned char* tile = ws_tiles + ((ch0 + c) * (size_t)tiles_per_chunk + S_U) * TILE_BYTES;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) addrow[q] = __ldg(reinterpret_cast<const uint4*>(tile + tile_chunk_off(row, 4 * hsel + q)));
-        if (c + 1 < NT && hsel == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(tile + (size_t)tiles_per_chunk * TILE_BYTES + row * 128));
-      }
+      for (int q = 0; q < 4; ++q) addrow[q] = __ldg(reinterpret_cast<const uint4*>(tile + tile_chunk_off(row, 4 * hsel + q)));
+      if (c + 1 < NT && hsel == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(tile + (size_t)tiles_per_chunk * TILE_BYTES + row * 128));
       scale = ws_aux[(ch0 + c) * AUX_FLOATS + 64 + row];                       // e^{glast-gref} of this chunk
       if (c + 1 < NT) scale_next = ws_aux[(ch0 + c + 1) * AUX_FLOATS + row];    // e^{gref} of the next chunk
       if (bwd_tiles && c > 0) store_x();
-    }
-    if constexpr (STAGES == 2) {
-      ok = ok && wait_g1(c);
-      if (state_lane) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) addrow[q] = *reinterpret_cast<const uint4*>(sm.g1[c % STAGES].u + tile_chunk_off(row, 4 * hsel + q));
-      }
     }
     ok = ok && mbar_wait(&sm.bar_a, c & 1, status, 212);
     tc_fence_after();
@@ -809,21 +774,16 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
     R7C_STAMP(51);
     // (c) H += b~^T sa, then the rest of the output rows, A_qb sa
     if (warp == 0 && elect_one() && ok) {
-      ScanGroup2<STAGES>& g = sm.g2[c % STAGES];
-      if constexpr (!AHEAD) ok = wait_g2(c);
+      ok = mbar_wait(&sm.bar_g2, c & 1, status, 214);
       if (ok) {
         tc_fence_after();
-        umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 64 + 64 * p), smem_u32(g.bt), smem_u32(sm.sa), true);
+        umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, acc), smem_u32(sm.g2.bt), smem_u32(sm.sa), true);
         umma_commit(&sm.bar_c);
-        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 64 + 64 * p), smem_u32(g.aqb), smem_u32(sm.sa), true);
+        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, acc), smem_u32(sm.g2.aqb), smem_u32(sm.sa), true);
         umma_commit(&sm.bar_o);
-        if (AHEAD && c + 1 < NT) {
-          ok = wait_g1(c + 1);
-          if (ok) mma_kv(c + 1);
-        }
       }
     }
-    if (warp == ld_warp && elect_one() && ok && c + STAGES < NT) issue_g1(c + STAGES);
+    if (warp == ld_warp && elect_one() && ok && c + 1 < NT) issue_g1(c + 1);
     if (bwd_tiles && warp == st_warp && elect_one() && ok) {   // the backward needs sa, h~0 and X of every chunk
       unsigned char* tiles = bwd_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES;
       bulk_store(tiles + S_SA * TILE_BYTES, sm.sa, TILE_BYTES);
@@ -862,9 +822,9 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
     }
     // the copies out of sa, h~0, X and of the output rows have left their tiles: the next chunk rewrites them
     if ((warp == st_warp || warp == out_warp) && elect_one()) bulk_wait_read();
-    if (warp == ld_warp && elect_one() && ok && c + STAGES < NT) {      // group 2 has been read
+    if (warp == ld_warp && elect_one() && ok && c + 1 < NT) {      // group 2 has been read
       ok = mbar_wait(&sm.bar_o, c & 1, status, 216);
-      if (ok) issue_g2(c + STAGES);
+      if (ok) issue_g2(c + 1);
     }
     R7C_STAMP(54);
     fence_async_smem();
@@ -916,17 +876,290 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
   marked = __syncthreads_or(marked);
   if (tid == 0) ws_flags[unit] = marked;
   if (warp == 0) tmem_dealloc(tm, 256);
-  // A marked unit again, by the exact recurrence: 64 threads per 16 rows, in place of what the chunks gave (inside this
-  // kernel, because a launch of its own over all units costs every call 2 us of device time and as much on the host).
-  if (marked && exact.r && ok) {
-    r7rec::FwdArgs<bf16> args = exact;
-    args.base = brow * lay.sb + hi * lay.sh + tb * lay.st;
-    args.Tn = Tn;
-    args.S0 = n_state > 0 ? h0 + (size_t)(n_state == 1 ? hi : unit) * 4096 : nullptr;
-    args.ht = ht ? ht + (size_t)unit * 4096 : nullptr;
-    static_assert(4 * sizeof(r7rec::FwdSmem<64>) <= sizeof(ScanSmem<STAGES>), "the recurrence runs in the scan's shared memory");
-    r7rec::fwd_rows<bf16, 64>(args, reinterpret_cast<r7rec::FwdSmem<64>*>(smem_raw)[tid >> 6], tid >> 6, tid & 63);
+  if (marked && exact.r && ok) exact_unit(exact, smem_raw, tid, unit, hi, brow, tb, Tn, h0, n_state, ht, lay);
+}
+
+// The same scan for fewer sequences than SMs: one CTA per SM, nothing else there to cover a wait, and the chain from
+// chunk to chunk bounds it.  So every kind of work has warps of its own and they meet at mbarriers only: warps 0-7 read
+// accumulators out (as above), one thread each of warps 8, 9, 10 issues the MMAs, fetches operand tiles and copies results
+// out.  (With everything between two block barriers the issue of 24 MMAs per chunk, which waits for the tensor pipe, the
+// requests for tiles and the waits for copies all held the read-outs up.)  The chain that is left: W h~0, its read-out
+// plus U -> sa, b~^T sa, its read-out -> h; the other products run beside the read-outs, and the output rows of a
+// chunk are read out while b~^T sa of the next one is computed.  The readers load nothing from global memory: a proxy fence
+// waits for such loads too (1200 cycles from W h~0 to sa instead of 320), so U and the decay factors come with the tiles.
+// B 2, T 4096, 32 heads, training: 123 -> 100 us (5.0 TB/s with twice the sequences).
+struct AloneSmem {
+  struct { unsigned char kt[TILE_BYTES], aqk[TILE_BYTES], w[TILE_BYTES], u[TILE_BYTES], v[TILE_BYTES]; } g1[2];
+  struct { unsigned char qt[TILE_BYTES], bt[TILE_BYTES], aqb[TILE_BYTES]; } g2[2];
+  unsigned char ht[2][TILE_BYTES], sa[2][TILE_BYTES], xt[2][TILE_BYTES], ot[2][TILE_BYTES];
+  float aux[2][AUX_FLOATS];         // the chunks' decay factors, with the first group
+  uint64_t bar_g1[2], bar_g2[2];
+  uint64_t bar_h, bar_s;            // h~0, sa of a chunk are in shared memory (one arrival per reading warp)
+  uint64_t bar_a, bar_c, bar_o;     // W h~0; b~^T sa; all products of a chunk have completed
+  uint64_t bar_free;                // the copies issued in the previous chunk have left shared memory
+  uint32_t tmem_base;
+};
+constexpr int ALONE_THREADS = 352;
+
+template <bool PACKED>
+__global__ void __launch_bounds__(ALONE_THREADS, 1)
+r7c_scan_fwd_alone_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned char* __restrict__ ws_tiles,
+                          const float* __restrict__ ws_aux, int* __restrict__ ws_flags, int tiles_per_chunk,
+                          unsigned char* __restrict__ bwd_tiles, const float* __restrict__ h0, int n_state,
+                          const __grid_constant__ CUtensorMap tmap_o, int write_o, float* __restrict__ ht,
+                          bf16* __restrict__ o_rows, SeqView sv, int H, int NT_slots, TokLayout lay,
+                          r7rec::FwdArgs<bf16> exact, int* status, long long* dbg) {
+#ifdef RWKVB200_DEVTOOLS
+#define R7C_STAMP(n) do { if (dbg && tid == 0 && blockIdx.x == gridDim.x / 2 && c == 2) dbg[n] = clock64(); } while (0)
+#else
+#define R7C_STAMP(n) do {} while (0)
+#endif
+  extern __shared__ unsigned char smem_raw[];
+  AloneSmem& sm = *reinterpret_cast<AloneSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int wq = warp & 3, c0 = 32 * (warp >> 2);
+  const int unit = blockIdx.x, bi = unit / H, hi = unit % H;
+  const size_t ch0 = (size_t)unit * NT_slots;
+  const int Tn = sv.length<PACKED>(bi), tb = sv.first<PACKED>(bi), brow = sv.row<PACKED>(bi);
+  const int NT = (Tn + L - 1) / L;           // chunks of this sequence (at least one)
+  const int row = 16 * wq + (lane & 15);     // state row k (lanes 0-15) or token row i (lanes 16-31)
+  const bool state_lane = lane < 16;
+  auto chunk_tiles = [&](int c) { return ws_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES; };
+
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i) { mbar_init(&sm.bar_g1[i], 1); mbar_init(&sm.bar_g2[i], 1); }
+    mbar_init(&sm.bar_h, 8); mbar_init(&sm.bar_s, 8);
+    mbar_init(&sm.bar_a, 1); mbar_init(&sm.bar_c, 1); mbar_init(&sm.bar_o, 1); mbar_init(&sm.bar_free, 1);
+    fence_mbar_init();
   }
+  if (warp == 0) tmem_alloc(&sm.tmem_base, 256);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  // TMEM: columns 0..63 lower lane halves = W h~0; three accumulators in turn: lower halves k~^T v + b~^T sa, upper halves
+  // the output rows, which are read out while the next chunk's is in use and the one after it is being started
+  const uint32_t tm = sm.tmem_base;
+  auto acc_col = [](int c) { return 64u + 64u * (uint32_t)(c % 3); };
+  bool ok = true;
+  int marked = 0;       // a chunk's decay left the range of the scaled operands (the sign of its factors)
+  float h[32];          // state lanes: row of the state, columns c0 .. c0 + 31
+
+  if (warp < 8) {       // ---- readers
+    const uint32_t tm_w = tmem_addr(tm, 32 * wq, c0);
+    auto store_row = [&](unsigned char* tile, const float* x) { tile_store_row32(tile, row, c0, x); };
+    // this warp's writes and TMEM reads so far are done, for the async proxy and the tensor pipe too
+    auto arrive = [&](uint64_t* bar) {
+      fence_async_smem();
+      tc_fence_before();
+      __syncwarp();
+      if (elect_one()) mbar_arrive(bar);
+    };
+    auto wait = [&](uint64_t* bar, int phase, int code) {
+      ok = __all_sync(0xffffffffu, mbar_wait(bar, phase & 1, status, code));
+      tc_fence_after();
+      return ok;
+    };
+    auto read_o = [&](int c) {      // the output rows of chunk c into their tile
+      uint32_t r[32];
+      tmem_ld32(tm_w + acc_col(c), r);
+      tmem_ld_wait();
+      float x[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(r[j]);
+      if (!state_lane) store_row(sm.ot[c & 1], x);
+    };
+#pragma unroll
+    for (int vv = 0; vv < 32; ++vv) h[vv] = 0.f;
+    if (state_lane) {      // initial state: h~0 = e^{gref(chunk 0)} h0
+      const float e0 = ws_aux[ch0 * AUX_FLOATS + row];
+      if (n_state > 0) {
+        const float* S = h0 + (size_t)(n_state == 1 ? hi : unit) * 4096;   // S[v][k], h[k][v] = S[v][k]
+#pragma unroll
+        for (int vv = 0; vv < 32; ++vv) h[vv] = e0 * S[(c0 + vv) * 64 + row];
+      }
+      store_row(sm.ht[0], h);
+    }
+    arrive(&sm.bar_h);
+    for (int c = 0; c < NT; ++c) {
+      const int p = c & 1;
+      R7C_STAMP(48);
+      // sa = W h~0 + U
+      if (!wait(&sm.bar_g1[p], c >> 1, 211)) break;
+      uint4 u[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) u[q] = *reinterpret_cast<const uint4*>(sm.g1[p].u + tile_chunk_off(row, c0 / 8 + q));
+      const float scale = sm.aux[p][64 + row];      // e^{glast-gref} of this chunk
+      if (!wait(&sm.bar_a, c, 212)) break;
+      R7C_STAMP(49);
+      {
+        uint32_t r[32];
+        tmem_ld32(tm_w, r);
+        tmem_ld_wait();
+        float x[32];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const uint32_t uu[4] = {u[q].x, u[q].y, u[q].z, u[q].w};
+#pragma unroll
+          for (int m = 0; m < 4; ++m) {
+            x[8 * q + 2 * m] = __uint_as_float(r[8 * q + 2 * m]) + bf16_lo(uu[m]);
+            x[8 * q + 2 * m + 1] = __uint_as_float(r[8 * q + 2 * m + 1]) + bf16_hi(uu[m]);
+          }
+        }
+        if (state_lane) store_row(sm.sa[p], x);
+      }
+      arrive(&sm.bar_s);
+      R7C_STAMP(50);
+      if (!wait(&sm.bar_free, c, 218)) break;
+      if (write_o && c > 0) read_o(c - 1);
+      R7C_STAMP(51);
+      // X and the next h~0, scaled by e^{glast-gref} of this chunk and e^{gref} of the next
+      // (one after the other: their product can underflow float32 where neither factor does)
+      if (c + 1 < NT && !wait(&sm.bar_g1[p ^ 1], (c + 1) >> 1, 211)) break;
+      const float scale_next = c + 1 < NT ? sm.aux[p ^ 1][row] : 1.f;
+      if (!wait(&sm.bar_c, c, 213)) break;
+      R7C_STAMP(52);
+      {
+        uint32_t r[32];
+        tmem_ld32(tm_w + acc_col(c), r);
+        tmem_ld_wait();
+        uint4 xp[4];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) h[j] += __uint_as_float(r[j]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          xp[q] = make_uint4(pack_bf16(h[8 * q], h[8 * q + 1]), pack_bf16(h[8 * q + 2], h[8 * q + 3]),
+                             pack_bf16(h[8 * q + 4], h[8 * q + 5]), pack_bf16(h[8 * q + 6], h[8 * q + 7]));
+        if (state_lane) marked |= scale < 0.f;
+        const float sc = fabsf(scale);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) h[j] = (h[j] * sc) * scale_next;
+        if (state_lane) store_row(sm.ht[p ^ 1], h);
+        arrive(&sm.bar_h);
+        if (state_lane && bwd_tiles) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) *reinterpret_cast<uint4*>(sm.xt[p] + tile_chunk_off(row, c0 / 8 + q)) = xp[q];
+        }
+      }
+      R7C_STAMP(53);
+    }
+    ok = ok && wait(&sm.bar_o, NT - 1, 217);
+  } else if (warp == 8) {      // ---- MMAs
+    if (elect_one()) {
+      auto ahead = [&](int c) {      // the two products of a chunk that need neither the state nor sa
+        auto& g = sm.g1[c & 1];
+        if (!mbar_wait(&sm.bar_g1[c & 1], (c >> 1) & 1, status, 211)) return false;
+        umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, acc_col(c)), smem_u32(g.kt), smem_u32(g.v), false);      // k~^T v
+        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, acc_col(c)), smem_u32(g.aqk), smem_u32(g.v), false);    // A_qk v
+        return true;
+      };
+      ok = ahead(0);
+      for (int c = 0; c < NT && ok; ++c) {
+        const uint32_t acc = acc_col(c);
+        auto& g1 = sm.g1[c & 1];
+        auto& g2 = sm.g2[c & 1];
+        ok = mbar_wait(&sm.bar_h, c & 1, status, 219);
+        if (!ok) break;
+        tc_fence_after();
+        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 0), smem_u32(g1.w), smem_u32(sm.ht[c & 1]), false);        // W h~0
+        umma_commit(&sm.bar_a);
+        ok = mbar_wait(&sm.bar_g2[c & 1], (c >> 1) & 1, status, 214) && mbar_wait(&sm.bar_s, c & 1, status, 220);
+        if (!ok) break;
+        tc_fence_after();
+        umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, acc), smem_u32(g2.bt), smem_u32(sm.sa[c & 1]), true);      // += b~^T sa
+        umma_commit(&sm.bar_c);
+        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, acc), smem_u32(g2.qt), smem_u32(sm.ht[c & 1]), true);     // += q~ h~0
+        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, acc), smem_u32(g2.aqb), smem_u32(sm.sa[c & 1]), true);    // += A_qb sa
+        umma_commit(&sm.bar_o);
+        if (c + 1 < NT) ok = ahead(c + 1);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 9) {      // ---- operand tiles
+    if (elect_one()) {
+      auto load_1 = [&](int c) {
+        auto& g = sm.g1[c & 1];
+        uint64_t* bar = &sm.bar_g1[c & 1];
+        mbar_expect_tx(bar, 5 * TILE_BYTES + AUX_FLOATS * (uint32_t)sizeof(float));
+        bulk_load(g.kt, chunk_tiles(c) + S_KT * TILE_BYTES, 4 * TILE_BYTES, bar);      // k~, A_qk, W, U: adjacent slots
+        tma_load_4d(g.v, &tmap_v, bar, 0, tb + c * L, hi, brow);
+        bulk_load(sm.aux[c & 1], ws_aux + (ch0 + c) * AUX_FLOATS, AUX_FLOATS * (uint32_t)sizeof(float), bar);
+      };
+      auto load_2 = [&](int c) {
+        mbar_expect_tx(&sm.bar_g2[c & 1], 3 * TILE_BYTES);
+        bulk_load(sm.g2[c & 1].qt, chunk_tiles(c) + S_QT * TILE_BYTES, 3 * TILE_BYTES, &sm.bar_g2[c & 1]);     // q~, b~, A_qb
+      };
+      for (int c = 0; c < 2 && c < NT; ++c) { load_1(c); load_2(c); }
+      for (int c = 0; c + 2 < NT && ok; ++c) {
+        if (c + 4 < NT) {      // further ahead into L2
+          bulk_prefetch_l2(chunk_tiles(c + 4), FWD_TILES * TILE_BYTES);
+          tma_prefetch_4d(&tmap_v, 0, tb + (c + 4) * L, hi, brow);
+        }
+        ok = mbar_wait(&sm.bar_o, c & 1, status, 216);      // the tiles of chunk c have been read
+        if (ok) { load_1(c + 2); load_2(c + 2); }
+      }
+    }
+    __syncwarp();
+  } else {                     // ---- results
+    if (elect_one()) {
+      for (int c = 0; c < NT && ok; ++c) {
+        ok = mbar_wait(&sm.bar_s, c & 1, status, 221);
+        bulk_wait_read();      // what was issued a chunk ago
+        if (!ok) break;
+        mbar_arrive(&sm.bar_free);
+        if (bwd_tiles) {       // the backward needs sa, h~0 and X of every chunk
+          unsigned char* tiles = bwd_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES;
+          bulk_store(tiles + S_H0 * TILE_BYTES, sm.ht[c & 1], TILE_BYTES);
+          bulk_store(tiles + S_SA * TILE_BYTES, sm.sa[c & 1], TILE_BYTES);
+          if (c > 0) bulk_store(tiles - ((size_t)tiles_per_chunk - S_X) * TILE_BYTES, sm.xt[(c + 1) & 1], TILE_BYTES);
+        }
+        if (write_o && c > 1) tma_store_4d(&tmap_o, sm.ot[c & 1], 0, tb + (c - 2) * L, hi, brow);     // staged in chunk c - 1
+        bulk_commit();
+      }
+      bulk_wait_read();
+    }
+    __syncwarp();
+  }
+#undef R7C_STAMP
+  // ---- what the last chunk still holds: its output rows, X, the final state, and the output rows of the chunk before
+  ok = __syncthreads_and(ok);
+  tc_fence_after();
+  if (ok && warp < 8) {
+    uint32_t r[32];
+    tmem_ld32(tmem_addr(tm, 32 * wq, acc_col(NT - 1) + c0), r);
+    tmem_ld_wait();
+    float x[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(r[j]);
+    if (!state_lane) {
+      if (write_o) tile_store_row32(sm.ot[(NT - 1) & 1], row, c0, x);
+    } else if (ht) {
+      float* S = ht + (size_t)unit * 4096;
+#pragma unroll
+      for (int j = 0; j < 32; ++j) S[(c0 + j) * 64 + row] = h[j];
+    }
+  }
+  fence_async_smem();
+  tc_fence_before();
+  __syncthreads();
+  if (ok) {
+    const int t0 = (NT - 1) * L;
+    const bool part = PACKED && t0 + L > Tn;      // the last rows of the box belong to the next sequence: row by row
+    if (warp == 10 && elect_one()) {
+      if (bwd_tiles)
+        bulk_store(bwd_tiles + ((ch0 + NT - 1) * (size_t)tiles_per_chunk + S_X) * TILE_BYTES, sm.xt[(NT - 1) & 1], TILE_BYTES);
+      if (write_o && NT > 1) tma_store_4d(&tmap_o, sm.ot[NT & 1], 0, tb + t0 - L, hi, brow);
+      if (write_o && !part) tma_store_4d(&tmap_o, sm.ot[(NT - 1) & 1], 0, tb + t0, hi, brow);     // rows past the tensor's end are clipped
+      bulk_commit();
+    }
+    if (write_o && part && warp < 8)
+      store_tile_rows<256>(o_rows + brow * lay.sb + hi * lay.sh + (long long)(tb + t0) * lay.st, lay.st, sm.ot[(NT - 1) & 1],
+                           Tn - t0, tid);
+  }
+  if (warp == 10 && elect_one()) bulk_wait_all();
+  marked = __syncthreads_or(marked);
+  if (tid == 0) ws_flags[unit] = marked;
+  if (warp == 0) tmem_dealloc(tm, 256);
+  if (warp < 8 && marked && exact.r && ok) exact_unit(exact, smem_raw, tid, unit, hi, brow, tb, Tn, h0, n_state, ht, lay);
 }
 
 }  // namespace r7c
@@ -982,25 +1215,29 @@ int launch_rwkv7_chunked_fwd(const void* r, const void* w, const void* k, const 
   e = check_launch();
   if (e || !(phases & PHASE_SCAN)) return e;
   {
-    const int sms = dev.sms;
     ProfScope prof("r7c_scan_fwd_kernel", st);
     // what a unit needs whose decay left the range of the scaled operands (fused producers bound |g| by e^{-1/2}: none)
     r7rec::FwdArgs<bf16> exact{};
     if (!fused && (o || ht))
       exact = r7rec::FwdArgs<bf16>{(const bf16*)r, (const bf16*)w, (const bf16*)k, (const bf16*)v, (const bf16*)a, (const bf16*)b,
                                    0, lay.st, 0, nullptr, (bf16*)o, nullptr, nullptr, 1};
-    // more sequences than SMs: two single-buffered CTAs per SM; else one double-buffered CTA per SM
-#define R7C_LAUNCH_SCAN(S, P)                                                                                      \
+    // more sequences than SMs: two CTAs per SM
+#define R7C_LAUNCH_SCAN(KERNEL, P, THREADS, SMEM)                                                                  \
     do {                                                                                                           \
-      const int smem = (int)sizeof(ScanSmem<S>) + 1024;                                                            \
-      if (allow_smem<r7c_scan_fwd_kernel<S, P>>(dev, smem)) \
+      const int smem = (int)sizeof(SMEM) + 1024;                                                                   \
+      if (allow_smem<KERNEL<P>>(dev, smem))                                                                        \
         return RWKVB200_E_CUDA;                                                                                    \
-      r7c_scan_fwd_kernel<S, P><<<B * H, 256, smem, st>>>(tmap_v, ws.tiles, ws.aux, ws.flags, tpc,                 \
-          keep_for_bwd ? ws.tiles : nullptr, h0, n_state, tmap_o, o ? 1 : 0, ht, (bf16*)o, sv, H, NT, lay, exact, status, \
-          debug_stamp_buffer());                                                                                   \
+      KERNEL<P><<<B * H, THREADS, smem, st>>>(tmap_v, ws.tiles, ws.aux, ws.flags, tpc,                             \
+          keep_for_bwd ? ws.tiles : nullptr, h0, n_state, tmap_o, o ? 1 : 0, ht, (bf16*)o, sv, H, NT, lay, exact,  \
+          status, debug_stamp_buffer());                                                                           \
     } while (0)
-    if (B * H > sms) { if (seq_start) R7C_LAUNCH_SCAN(1, true); else R7C_LAUNCH_SCAN(1, false); }
-    else             { if (seq_start) R7C_LAUNCH_SCAN(2, true); else R7C_LAUNCH_SCAN(2, false); }
+    if (B * H > dev.sms) {
+      if (seq_start) R7C_LAUNCH_SCAN(r7c_scan_fwd_kernel, true, 256, ScanSmem);
+      else           R7C_LAUNCH_SCAN(r7c_scan_fwd_kernel, false, 256, ScanSmem);
+    } else {
+      if (seq_start) R7C_LAUNCH_SCAN(r7c_scan_fwd_alone_kernel, true, ALONE_THREADS, AloneSmem);
+      else           R7C_LAUNCH_SCAN(r7c_scan_fwd_alone_kernel, false, ALONE_THREADS, AloneSmem);
+    }
 #undef R7C_LAUNCH_SCAN
   }
   return check_launch();

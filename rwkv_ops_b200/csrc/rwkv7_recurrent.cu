@@ -43,7 +43,7 @@ rwkv7_rec_fwd_kernel(FwdArgs<T> args, const float* __restrict__ h0, int n_state,
   args.base = bi * lay.sb + hi * lay.sh;
   args.S0 = h0 && n_state > 0 ? h0 + (long long)(n_state == 1 ? hi : unit) * N * N : nullptr;
   args.ht = ht ? ht + (long long)unit * N * N : nullptr;
-  fwd_rows<T, N>(args, sm, blockIdx.y, threadIdx.x);
+  fwd_rows<T, N, N>(args, sm, blockIdx.y, threadIdx.x);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -89,7 +89,7 @@ rwkv7_rec_bwd_kernel(const T* __restrict__ r, const T* __restrict__ w, const T* 
     static_assert(sizeof(FwdSmem<N>) <= sizeof(BwdSmem<N>), "the forward's tiles live in the backward's shared memory");
     const FwdArgs<T> args{r, w, k, v, a, b, base, lay.st, Tn,
                           n_state > 0 ? h0 + (long long)(n_state == 1 ? hi : unit) * N * N : nullptr, nullptr, nullptr, ckpt, CK};
-    fwd_rows<T, N>(args, *reinterpret_cast<FwdSmem<N>*>(smem_raw), y, tid);
+    fwd_rows<T, N, N>(args, *reinterpret_cast<FwdSmem<N>*>(smem_raw), y, tid);
     __syncthreads();
   }
 

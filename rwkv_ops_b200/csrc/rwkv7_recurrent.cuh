@@ -36,8 +36,8 @@ struct FwdArgs {
   int ckpt_every;
 };
 
-// Called by N threads per slice `y` of 16 rows (tid < N), by all threads of the block at once (it has block barriers).
-template <typename T, int N>
+// Called by N threads per slice `y` of 16 rows (tid < N), by NTHREADS threads of the block at once (which meet at barrier 1).
+template <typename T, int N, int NTHREADS>
 __device__ __noinline__ void fwd_rows(const FwdArgs<T>& A, FwdSmem<N>& sm, int y, int tid) {
   constexpr int TL = FwdSmem<N>::TL;
   constexpr int KSEG = N / 16;      // lanes per state row
@@ -87,7 +87,7 @@ __device__ __noinline__ void fwd_rows(const FwdArgs<T>& A, FwdSmem<N>& sm, int y
   for (int t0 = 0; t0 < Tn; t0 += TL) {
     const int nt = min(TL, Tn - t0);
     stash();
-    __syncthreads();
+    asm volatile("bar.sync 1, %0;" ::"n"(NTHREADS) : "memory");
     if (t0 + TL < Tn) fetch(t0 + TL);
 
     for (int tl = 0; tl < nt; ++tl) {
@@ -126,7 +126,7 @@ __device__ __noinline__ void fwd_rows(const FwdArgs<T>& A, FwdSmem<N>& sm, int y
       for (int m = 1; m < KSEG; m <<= 1) oo += __shfl_xor_sync(0xffffffffu, oo, m);
       if (kq == 0) sm.ot[tl][vl] = oo;
     }
-    __syncthreads();
+    asm volatile("bar.sync 1, %0;" ::"n"(NTHREADS) : "memory");
     if (A.o && tid < nt * 4) {
       const int tl = tid >> 2, quad = tid & 3;
       store4(A.o + A.base + (long long)(t0 + tl) * A.st + y * VS + 4 * quad,
