@@ -17,7 +17,7 @@ constexpr float EXP2_FLOOR = -126.f;      // 2^x below this is flushed to zero a
 // ---------------------------------------------------------------------------------------------
 // intra-chunk kernel: persistent CTAs of 256 threads over the B*H*NT chunk-heads
 // ---------------------------------------------------------------------------------------------
-constexpr int NROW = 68;   // padded row of the fp32 copy of A_ab (keeps float4 alignment)
+constexpr int NROW = 68;   // padded row of a 64 x 64 fp32 array (keeps float4 alignment)
 
 struct IntraSmem {
   unsigned char qt[TILE_BYTES], at[TILE_BYTES];     // [q~; a~]  (128-row A operand)
@@ -25,21 +25,22 @@ struct IntraSmem {
   unsigned char aqk[TILE_BYTES], aak[TILE_BYTES];   // [A_qk; A_ak] (128-row A operand); aak later holds W
   unsigned char cm[TILE_BYTES];                     // C = A_qb Ainv
   unsigned char aqb[TILE_BYTES];
-  unsigned char v[TILE_BYTES];                      // TMA; later U
+  unsigned char v[TILE_BYTES];                      // raw a, then v
   unsigned char ainv[TILE_BYTES];                   // later holds B2
   unsigned char y[TILE_BYTES];                      // A_ak v
-  float nmat[L * NROW];                             // stril(A_ab) in fp32
+  float gs[L * NROW];                               // e^{gi-gref}; later the diagonal blocks of A_ab
   float qtot[4][64];                                // sums of g over the four quarters of the chunk
-  uint64_t bar_v, bar_w, bar_in, bar_ia, bar_m1, bar_m2, bar_m3, bar_m4, bar_m5;
+  float efirst[64];                                 // e^{-gref}
+  uint64_t bar_v, bar_w, bar_in, bar_b, bar_m1, bar_m2, bar_m3, bar_m4, bar_m5;
   uint32_t tmem_base;
 };
 
-// Persistent: CTAs (two per SM) walk over chunk-heads ch = blockIdx.x, blockIdx.x + gridDim.x, ...  The
-// raw q, k, a, b, w tiles of the next chunk-head are requested by TMA as soon as the tiles they land in
-// (q~, k~, a~, b~, which are then scaled in place, and A_qk) have been copied out, its v tile as soon as
-// MMA 2 has read the current one, and the rows of the one after that are asked into L2.
+// Persistent: CTAs (two per SM) walk over chunk-heads ch = blockIdx.x, blockIdx.x + gridDim.x, ...
 // 256 threads: warp w reads TMEM lanes 32*(w&3).. and the two warps that share a lane window split
-// the columns (hsel = w>>2); the triangular solve runs on warps 0-1 while the other warps drain MMA 2.
+// the columns (hsel = w>>2); warps 6 and 7 invert the diagonal blocks of A_ab while the other warps mask the rest of
+// MMA 1, issue MMA 2 and drain it.
+// What bounds it: 17 tiles per chunk-head through memory (348 us at B 8, T 4096, 32 heads) if two CTAs per SM can
+// overlap their chains of phases well enough (503 us with 15.3 k cycles per chunk-head; 414 us with 13.3 k now).
 template <bool PACKED, bool FUSED>
 __global__ void __launch_bounds__(256, 2)
 r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, const bf16* __restrict__ k,
@@ -61,7 +62,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
   const int wq = warp & 3, hsel = warp >> 2;
 
   if (tid == 0) {
-    mbar_init(&sm.bar_v, 1); mbar_init(&sm.bar_w, 1); mbar_init(&sm.bar_in, 1); mbar_init(&sm.bar_ia, 1); mbar_init(&sm.bar_m1, 1); mbar_init(&sm.bar_m2, 1); mbar_init(&sm.bar_m3, 1);
+    mbar_init(&sm.bar_v, 1); mbar_init(&sm.bar_w, 1); mbar_init(&sm.bar_in, 1); mbar_init(&sm.bar_b, 1); mbar_init(&sm.bar_m1, 1); mbar_init(&sm.bar_m2, 1); mbar_init(&sm.bar_m3, 1);
     mbar_init(&sm.bar_m4, 1); mbar_init(&sm.bar_m5, 1);
     fence_mbar_init();
   }
@@ -72,32 +73,22 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
   const uint32_t tm = sm.tmem_base;
 
   auto coords = [&](const ChunkPos& p, int& bi, int& hi, int& t0) { bi = p.bi; hi = p.hi; t0 = p.c * L; };
-  // The raw tiles of a chunk-head (rows past the end of the sequence arrive as zeros).  w, needed first,
-  // lands in the A_qk tile, free from the end of the triangular inverse to the first epilogue of the next
-  // chunk-head; q, k, a, b, needed only after the prefix sums, land in the tiles that will hold their
-  // scaled versions once those have been copied out.
-  auto load_w = [&](const ChunkPos& p) {       // tid 0
-    int bi, hi, t0; coords(p, bi, hi, t0);
-    mbar_expect_tx(&sm.bar_w, TILE_BYTES);
-    tma_load_4d(sm.aqk, &tmap_w, &sm.bar_w, 0, sv.first<PACKED>(bi) + t0, hi, sv.row<PACKED>(bi));
+  // The raw tiles of a chunk-head (rows past the end of the sequence arrive as zeros), requested most of a chunk-head
+  // before they are needed: w, q, k land in the A_qk, q~, k~ tiles and a in the v tile as soon as MMA 2 has completed (the
+  // copies to the workspace have left shared memory by then), b in the space of the decay factors once the diagonal
+  // blocks have been inverted there.  Only v, needed last, is requested in its own chunk-head, when a has been scaled.
+  auto load = [&](unsigned char* dst, const CUtensorMap* map, uint64_t* bar, const ChunkPos& p) {      // one thread
+    tma_load_4d(dst, map, bar, 0, sv.first<PACKED>(p.bi) + p.c * L, p.hi, sv.row<PACKED>(p.bi));
   };
-  // q, k land in tiles that only MMA 1 reads and are requested as soon as MMA 2 has completed (their
-  // copies to the workspace have left shared memory by then); a, b land in tiles that MMA 3 reads and are requested
-  // after it (the rows have been asked into L2 by then).
-  auto load_qk = [&](const ChunkPos& p) {     // tid 0
-    int bi, hi, t0; coords(p, bi, hi, t0);
-    const int tt = sv.first<PACKED>(bi) + t0, br = sv.row<PACKED>(bi);
-    mbar_expect_tx(&sm.bar_in, 2 * TILE_BYTES);
-    tma_load_4d(sm.qt, &tmap_q, &sm.bar_in, 0, tt, hi, br);
-    tma_load_4d(sm.kt, &tmap_k, &sm.bar_in, 0, tt, hi, br);
+  auto load_w = [&](const ChunkPos& p) { mbar_expect_tx(&sm.bar_w, TILE_BYTES); load(sm.aqk, &tmap_w, &sm.bar_w, p); };
+  auto load_qka = [&](const ChunkPos& p) {
+    mbar_expect_tx(&sm.bar_in, 3 * TILE_BYTES);
+    load(sm.qt, &tmap_q, &sm.bar_in, p);
+    load(sm.kt, &tmap_k, &sm.bar_in, p);
+    load(sm.v, &tmap_a, &sm.bar_in, p);
   };
-  auto load_ab = [&](const ChunkPos& p) {      // tid 0
-    int bi, hi, t0; coords(p, bi, hi, t0);
-    const int tt = sv.first<PACKED>(bi) + t0, br = sv.row<PACKED>(bi);
-    mbar_expect_tx(&sm.bar_ia, 2 * TILE_BYTES);
-    tma_load_4d(sm.at, &tmap_a, &sm.bar_ia, 0, tt, hi, br);
-    tma_load_4d(sm.bt, &tmap_b, &sm.bar_ia, 0, tt, hi, br);
-  };
+  auto load_b = [&](const ChunkPos& p) { mbar_expect_tx(&sm.bar_b, TILE_BYTES); load(reinterpret_cast<unsigned char*>(sm.gs), &tmap_b, &sm.bar_b, p); };
+  auto load_v = [&](const ChunkPos& p) { mbar_expect_tx(&sm.bar_v, TILE_BYTES); load(sm.v, &tmap_v, &sm.bar_v, p); };
   // chunk slots past the end of a (packed) sequence are skipped
   auto empty = [&](const ChunkPos& p) {
     if constexpr (!PACKED) return false;      // a dense batch has no empty slots
@@ -108,31 +99,18 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
     return p;
   };
   // Ask for a chunk-head's token rows to be brought into L2, ahead of the TMA loads above.
-  auto prefetch_rows = [&](const ChunkPos& p) {
-    int bi, hi, t0; coords(p, bi, hi, t0);
-    const int Tn = sv.length<PACKED>(bi);
-    const long long base = sv.row<PACKED>(bi) * lay.sb + hi * lay.sh + sv.first<PACKED>(bi) * lay.st;
-#pragma unroll
-    for (int n = 0; n < 2; ++n) {
-      const int e = tid + 256 * n, row = e >> 3, cc = e & 7, tok = t0 + row;
-      if (tok < Tn && cc == 0) {      // one 128-byte row per request
-        const long long off = base + (long long)tok * lay.st;
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(w + off));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(q + off));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(k + off));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(a + off));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(b + off));
-      }
-    }
-  };
-  auto load_v = [&](const ChunkPos& p) {   // tid 0
-    int bi, hi, t0; coords(p, bi, hi, t0);
-    mbar_expect_tx(&sm.bar_v, TILE_BYTES);
-    tma_load_4d(sm.v, &tmap_v, &sm.bar_v, 0, sv.first<PACKED>(bi) + t0, hi, sv.row<PACKED>(bi));
+  auto prefetch_rows = [&](const ChunkPos& p) {      // one thread
+    const int tt = sv.first<PACKED>(p.bi) + p.c * L, br = sv.row<PACKED>(p.bi);
+    tma_prefetch_4d(&tmap_w, 0, tt, p.hi, br);
+    tma_prefetch_4d(&tmap_q, 0, tt, p.hi, br);
+    tma_prefetch_4d(&tmap_k, 0, tt, p.hi, br);
+    tma_prefetch_4d(&tmap_a, 0, tt, p.hi, br);
+    tma_prefetch_4d(&tmap_b, 0, tt, p.hi, br);
+    tma_prefetch_4d(&tmap_v, 0, tt, p.hi, br);
   };
   ChunkPos cur = chunk_pos(blockIdx.x, NT, H);
   if (cur.ch < n_ch && empty(cur)) cur = advance(cur);
-  if (cur.ch < n_ch && warp == 0 && elect_one()) { load_w(cur); load_qk(cur); load_ab(cur); load_v(cur); }
+  if (cur.ch < n_ch && warp == 0 && elect_one()) { load_w(cur); load_qka(cur); load_b(cur); }
   // The two CTAs that share an SM would otherwise run their phases in lockstep and compete for the
   // same unit (shared-memory pipe during the triangular solve); start every other CTA half a
   // chunk-head late (unless it has a single one to do, or none: then the delay would be all it adds).
@@ -150,77 +128,61 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
     const int next = nxt.ch;
 
     R7C_STAMP(0);
-    if (next < n_ch) prefetch_rows(nxt);
-    // this thread's 2 x 16 bytes (8 channels of one token) of the raw w tile
-    uint4 rw[2];
-    ok = mbar_wait(&sm.bar_w, par, status, 206) && ok;
+    if (next < n_ch && warp == 1 && elect_one()) prefetch_rows(nxt);
+    // ---- phase A: decay prefix sums (in units of log 2), thread = (channel, quarter of the chunk), straight from the
+    // raw w tile.  What everybody needs of them is e^{gi-gref}: its reciprocal is the factor of k~ and b~, and the row
+    // before gives the factor of a~.
+    ok = mbar_wait(&sm.bar_b, par, status, 208) && ok;
+    uint4 rb[2];      // this thread's 2 x 16 bytes (8 channels of one token) of the raw b tile, which lies where the factors will
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
       const int e = tid + 256 * n;
-      rw[n] = *reinterpret_cast<const uint4*>(sm.aqk + tile_chunk_off(e >> 3, e & 7));
+      rb[n] = *reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned char*>(sm.gs) + tile_chunk_off(e >> 3, e & 7));
     }
-    // ---- phase A: decay prefix sums (in units of log 2) and the four scaled operands; the prefix sum over tokens goes
-    // through shared memory (the fp32 area that later holds A_ab).
+    ok = mbar_wait(&sm.bar_w, par, status, 206) && ok;
     {
-      float* gs = sm.nmat;
-      float gown[2][8];     // g of this thread's 2 x 8 (token, channel) entries
+      const int c = tid & 63, quarter = tid >> 6;
+      float gi[16];
+      float run = 0.f;
+      const int n_rows = Tn - t0 - 16 * quarter;      // rows of this quarter inside the sequence
 #pragma unroll
-      for (int n = 0; n < 2; ++n) {
-        const int e = tid + 256 * n, row = e >> 3, cc = e & 7;
-        const bool valid = t0 + row < Tn;
-        const uint32_t u[4] = {rw[n].x, rw[n].y, rw[n].z, rw[n].w};
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          float w0 = bf16_lo(u[m]), w1 = bf16_hi(u[m]);
-          if constexpr (FUSED) {      // the tile holds p: w = -e^{-1/2} sigmoid(p), as a bfloat16 value
-            w0 = round_bf16(W_SCALE * sigmoidf_(w0));
-            w1 = round_bf16(W_SCALE * sigmoidf_(w1));
-          }
-          gown[n][2 * m] = valid ? -LOG2E * ex2(LOG2E * w0) : 0.f;
-          gown[n][2 * m + 1] = valid ? -LOG2E * ex2(LOG2E * w1) : 0.f;
-        }
-        *reinterpret_cast<float4*>(&gs[row * NROW + 8 * cc]) = make_float4(gown[n][0], gown[n][1], gown[n][2], gown[n][3]);
-        *reinterpret_cast<float4*>(&gs[row * NROW + 8 * cc + 4]) = make_float4(gown[n][4], gown[n][5], gown[n][6], gown[n][7]);
+      for (int j = 0; j < 16; ++j) {
+        float w = __uint_as_float((uint32_t)*reinterpret_cast<const unsigned short*>(sm.aqk + tile_off(16 * quarter + j, c)) << 16);
+        if constexpr (FUSED) w = round_bf16(W_SCALE * sigmoidf_(w));      // the tile holds p: w = -e^{-1/2} sigmoid(p), as bfloat16
+        const float e = ex2(LOG2E * w);
+        if (j < n_rows) run -= LOG2E * e;
+        gi[j] = run;
       }
+      sm.qtot[quarter][c] = run;
       __syncthreads();
       R7C_STAMP(1);
-      {
-        const int c = tid & 63, quarter = tid >> 6;
-        float gv[16];
+      // gi - gref: the prefix inside the half; the reference point is the end of the first half
+      const float add = quarter == 0 ? -(run + sm.qtot[1][c]) : quarter == 1 ? -run : quarter == 3 ? sm.qtot[2][c] : 0.f;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) gv[j] = gs[(16 * quarter + j) * NROW + c];
-        float run = 0.f;
-#pragma unroll
-        for (int j = 0; j < 16; ++j) { run += gv[j]; gv[j] = run; }
-        sm.qtot[quarter][c] = run;
-        __syncthreads();
-        // gi - gref: the prefix inside the half; the reference point is the end of the first half
-        const float add = quarter == 0 ? -(run + sm.qtot[1][c]) : quarter == 1 ? -run : quarter == 3 ? sm.qtot[2][c] : 0.f;
-#pragma unroll
-        for (int j = 0; j < 16; ++j) gs[(16 * quarter + j) * NROW + c] = gv[j] + add;
-      }
-      __syncthreads();
-      if (tid < 64) {
-        const float tot0 = sm.qtot[0][tid] + sm.qtot[1][tid], tot1 = sm.qtot[2][tid] + sm.qtot[3][tid];
-        ws_aux[(size_t)ch * AUX_FLOATS + tid] = ex2(fmaxf(tot0, EXP2_FLOOR));        // e^{gref}
+      for (int j = 0; j < 16; ++j) sm.gs[(16 * quarter + j) * NROW + c] = ex2(gi[j] + add);
+      if (quarter == 0) {
+        const float tot0 = -add, tot1 = sm.qtot[2][c] + sm.qtot[3][c];
+        sm.efirst[c] = ex2(add);                                                     // for the exclusive prefix of the first token
+        ws_aux[(size_t)ch * AUX_FLOATS + c] = ex2(fmaxf(tot0, EXP2_FLOOR));          // e^{gref}
         // a half-chunk decay sum beyond the limit: the unit is recomputed by the float32 recurrence.  The mark is the
         // factor's sign; the scan, which reads every factor of its unit anyway, gathers it into Workspace::flags.
         const bool mark = fminf(tot0, tot1) < -DECAY_LIMIT * LOG2E || Tn < SHORT_SEQ;
-        ws_aux[(size_t)ch * AUX_FLOATS + 64 + tid] = copysignf(ex2(fmaxf(tot1, EXP2_FLOOR)), mark ? -1.f : 1.f);   // e^{glast-gref}
+        ws_aux[(size_t)ch * AUX_FLOATS + 64 + c] = copysignf(ex2(fmaxf(tot1, EXP2_FLOOR)), mark ? -1.f : 1.f);   // e^{glast-gref}
       }
-      // the raw q, k, a, b: each thread scales its own 2 x 16 bytes in place (the previous chunk-head's W, U,
+    }
+    __syncthreads();
+    {
+      // the raw q, k, a, b: each thread scales its own 2 x 16 bytes (the previous chunk-head's W, U,
       // A_qb copies may still be reading their tiles: those are rewritten only after MMA 1)
-      uint4 rq[2], rk[2], ra[2], rb[2];
+      uint4 rq[2], rk[2], ra[2];
       ok = mbar_wait(&sm.bar_in, par, status, 207) && ok;
-      ok = mbar_wait(&sm.bar_ia, par, status, 208) && ok;
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
         const int e = tid + 256 * n;
         const uint32_t off = tile_chunk_off(e >> 3, e & 7);
         rq[n] = *reinterpret_cast<const uint4*>(sm.qt + off);
         rk[n] = *reinterpret_cast<const uint4*>(sm.kt + off);
-        ra[n] = *reinterpret_cast<const uint4*>(sm.at + off);
-        rb[n] = *reinterpret_cast<const uint4*>(sm.bt + off);
+        ra[n] = *reinterpret_cast<const uint4*>(sm.v + off);
         if (PACKED && t0 + (e >> 3) >= Tn) {      // in a packed batch these rows belong to the next sequence
           rq[n] = make_uint4(0u, 0u, 0u, 0u); rk[n] = rq[n]; ra[n] = rq[n]; rb[n] = rq[n];
         }
@@ -249,9 +211,12 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
         const int e = tid + 256 * n, row = e >> 3, cc = e & 7;
-        float gl[8];
-        *reinterpret_cast<float4*>(gl) = *reinterpret_cast<const float4*>(&gs[row * NROW + 8 * cc]);
-        *reinterpret_cast<float4*>(gl + 4) = *reinterpret_cast<const float4*>(&gs[row * NROW + 8 * cc + 4]);
+        float eq[8], ea[8];      // e^{gi-gref} of the row; e^{ge-gref}: of the row before it
+        const float* before = row ? &sm.gs[(row - 1) * NROW + 8 * cc] : &sm.efirst[8 * cc];
+        *reinterpret_cast<float4*>(eq) = *reinterpret_cast<const float4*>(&sm.gs[row * NROW + 8 * cc]);
+        *reinterpret_cast<float4*>(eq + 4) = *reinterpret_cast<const float4*>(&sm.gs[row * NROW + 8 * cc + 4]);
+        *reinterpret_cast<float4*>(ea) = *reinterpret_cast<const float4*>(before);
+        *reinterpret_cast<float4*>(ea + 4) = *reinterpret_cast<const float4*>(before + 4);
         const uint32_t uq[4] = {rq[n].x, rq[n].y, rq[n].z, rq[n].w};
         const uint32_t uk[4] = {rk[n].x, rk[n].y, rk[n].z, rk[n].w};
         const uint32_t ua[4] = {ra[n].x, ra[n].y, ra[n].z, ra[n].w};
@@ -259,17 +224,11 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
         uint32_t oq[4], ok_[4], oa[4], ob[4];
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
-          float eq[2], ek[2], ea[2];
-#pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {
-            const int x = 2 * m + hh;
-            const float d1 = gl[x];                                         // gi - gref
-            eq[hh] = ex2(d1); ek[hh] = ex2(-d1); ea[hh] = ex2(d1 - gown[n][x]);
-          }
-          oq[m] = pack_bf16(bf16_lo(uq[m]) * eq[0], bf16_hi(uq[m]) * eq[1]);
-          ok_[m] = pack_bf16(bf16_lo(uk[m]) * ek[0], bf16_hi(uk[m]) * ek[1]);
-          oa[m] = pack_bf16(bf16_lo(ua[m]) * ea[0], bf16_hi(ua[m]) * ea[1]);
-          ob[m] = pack_bf16(bf16_lo(ub[m]) * ek[0], bf16_hi(ub[m]) * ek[1]);
+          const float ek0 = rcp(eq[2 * m]), ek1 = rcp(eq[2 * m + 1]);
+          oq[m] = pack_bf16(bf16_lo(uq[m]) * eq[2 * m], bf16_hi(uq[m]) * eq[2 * m + 1]);
+          ok_[m] = pack_bf16(bf16_lo(uk[m]) * ek0, bf16_hi(uk[m]) * ek1);
+          oa[m] = pack_bf16(bf16_lo(ua[m]) * ea[2 * m], bf16_hi(ua[m]) * ea[2 * m + 1]);
+          ob[m] = pack_bf16(bf16_lo(ub[m]) * ek0, bf16_hi(ub[m]) * ek1);
         }
         const uint32_t off = tile_chunk_off(row, cc);
         *reinterpret_cast<uint4*>(sm.qt + off) = make_uint4(oq[0], oq[1], oq[2], oq[3]);
@@ -288,6 +247,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
       tc_fence_after();
       umma_tile<128, 128, 0, 0>(tm, smem_u32(sm.qt), smem_u32(sm.kt), false);
       umma_commit(&sm.bar_m1);
+      load_v(cur);           // the raw a has been scaled
     }
     ok = mbar_wait(&sm.bar_m1, par, status, 201) && ok;
     tc_fence_after();
@@ -298,224 +258,174 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
       bulk_store(out_tiles + S_BT * TILE_BYTES, sm.bt, TILE_BYTES);
       bulk_commit();
     }
-    if (ok) {
-      const int r = 32 * wq + lane, i = r & 63;
-      const bool lower = r >= 64;       // rows of a~: strictly lower triangle; rows of q~: lower incl. diagonal
-      // The warp's 32 rows are i = 32*ihalf + lane, so which side of the diagonal a block of 32 columns lies on is
-      // the same for the whole warp: left of the diagonal block every element is kept, right of it every element
-      // is zero (TMEM is not read), and only the diagonal block takes a per-element choice.
-      const int ihalf = wq & 1;
-      auto emit = [&](const float (&x)[32], int j0) {
-        if (!lower) {
-          tile_store_row32(hsel ? sm.aqb : sm.aqk, i, j0, x);
-        } else if (!hsel) {
-          tile_store_row32(sm.aak, i, j0, x);
-        } else {
+    // Rows r < 64 are q~'s, the others a~'s; the warp's 32 rows are i = 32*ihalf + lane, so which side of the diagonal
+    // a block of 32 columns lies on is the same for the whole warp: left of the diagonal block every element is kept,
+    // right of it every element is zero (TMEM is not read), and only the diagonal block takes a per-element choice.
+    const int ihalf = wq & 1;
+    if (warp < 6) {      // A_qk (warps 0, 1), A_ak (2, 3), A_qb (4, 5)
+      if (ok) {
+        const bool strict = wq >= 2;
+        unsigned char* dst = hsel ? sm.aqb : strict ? sm.aak : sm.aqk;
 #pragma unroll
-          for (int j = 0; j < 32; j += 4)
-            *reinterpret_cast<float4*>(&sm.nmat[i * NROW + j0 + j]) = make_float4(x[j], x[j + 1], x[j + 2], x[j + 3]);
-        }
-      };
+        for (int pp = 0; pp < 2; ++pp) {
+          float x[32];
+          uint32_t rr[32];
+          if (pp > ihalf) {
 #pragma unroll
-      for (int pp = 0; pp < 2; ++pp) {
-        const int j0 = 32 * pp;
-        float x[32];
-        if (pp > ihalf) {
+            for (int j = 0; j < 32; ++j) x[j] = 0.f;
+          } else {
+            tmem_ld32(tmem_addr(tm, 32 * wq, 64 * hsel + 32 * pp), rr);   // hsel 0: products with k~, 1: with b~
+            tmem_ld_wait();
+            if (pp < ihalf) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) x[j] = 0.f;
-          emit(x, j0);
-          continue;
-        }
-        uint32_t rr[32];
-        tmem_ld32(tmem_addr(tm, 32 * wq, 64 * hsel + 32 * pp), rr);   // hsel 0: products with k~, 1: with b~
-        tmem_ld_wait();
-        if (pp < ihalf) {
+              for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
+            } else {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
-          emit(x, j0);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const bool keep = lower ? (j < lane) : (j <= lane);
-            x[j] = keep ? __uint_as_float(rr[j]) : 0.f;
+              for (int j = 0; j < 32; ++j) x[j] = (strict ? j < lane : j <= lane) ? __uint_as_float(rr[j]) : 0.f;
+            }
           }
-          emit(x, j0);
+          tile_store_row32(dst, 32 * ihalf + lane, 32 * pp, x);
         }
+      }
+      fence_async_smem();
+      tc_fence_before();
+      asm volatile("bar.sync 1, 192;" ::: "memory");
+
+      R7C_STAMP(4);
+      // ---- MMA 2: Y = A_ak v  ->  TMEM columns 128..191 (lower lane halves)
+      if (warp == 0 && elect_one()) {
+        ok = mbar_wait(&sm.bar_v, par, status, 202) && ok;
+        tc_fence_after();
+        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 128), smem_u32(sm.aak), smem_u32(sm.v), false);
+        umma_commit(&sm.bar_m2);
+        bulk_store(out_tiles + S_AQK * TILE_BYTES, sm.aqk, TILE_BYTES);
+        if (keep_for_bwd) {   // A_ak, a~ are operands of the backward
+          bulk_store(out_tiles + S_AAK * TILE_BYTES, sm.aak, TILE_BYTES);
+          bulk_store(out_tiles + S_AT * TILE_BYTES, sm.at, TILE_BYTES);
+        }
+        bulk_commit();
+      }
+      ok = mbar_wait(&sm.bar_m2, par, status, 203) && ok;
+      tc_fence_after();
+      if (ok) {      // Y rows; warps 2, 3 take both column halves of theirs
+#pragma unroll
+        for (int pp = 0; pp < 2; ++pp) {
+          if (pp != hsel && wq < 2) continue;
+          uint32_t rr[32];
+          tmem_ld32(tmem_addr(tm, 32 * wq, 128 + 32 * pp), rr);
+          tmem_ld_wait();
+          if (lane < 16) {        // an M = 64 accumulator lives on the lower 16 lanes of every warp's window
+            float x[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
+            tile_store_row32(sm.y, 16 * wq + lane, 32 * pp, x);
+          }
+        }
+      }
+      if (warp == 0 && elect_one()) {
+        bulk_wait_read();                  // q~, k~, b~, A_qk (and the tiles kept for the backward) have left shared memory
+        if (next < n_ch) { load_w(nxt); load_qka(nxt); }      // nothing reads A_qk, q~, k~, v any more
+      }
+    } else if (ok) {     // warps 6, 7: the diagonal 32 x 32 blocks of A_ab, inverted at once (fp32); warp 7 also N_BA
+      // Ainv = X = (I - N)^-1, N = stril(A_ab); with A = rows 0..31, B = rows 32..63 its blocks are X_A = (I - N_AA)^-1,
+      // X_B = (I - N_BB)^-1 and X_BA = X_B N_BA X_A.
+      float* nd = sm.gs + 1024 * ihalf;       // this warp's 32 x 32 block transposed: nd[32 r + i] = N[i][r]
+      uint32_t rr[32];
+      float x[32];
+      tmem_ld32(tmem_addr(tm, 32 * wq, 64 + 32 * ihalf), rr);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 32; ++j) nd[32 * j + lane] = __uint_as_float(rr[j]);      // (at or above the diagonal: never used)
+      if (ihalf) {
+        tmem_ld32(tmem_addr(tm, 32 * wq, 64), rr);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
+        tile_store_row32(sm.cm, 32 + lane, 0, x);         // Q: N_BA in rows 32..63 (its other rows and columns are not used)
+      } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) x[j] = 0.f;
+        tile_store_row32(sm.ainv, lane, 32, x);           // the upper right block of X
+      }
+      __syncwarp();
+      // Column `lane` of (I - N)^-1.  Once x[r] is known its products with column r of N go into all later rows, two per
+      // instruction and independent of one another, so that the chain from row to row is one multiply-add (summing up
+      // a row at a time instead, 85 cycles per row).  The next column is on its way from shared memory.
+      float4 nc[2][8];
+#pragma unroll
+      for (int m = 0; m < 8; ++m) nc[0][m] = *reinterpret_cast<const float4*>(&nd[4 * m]);
+#pragma unroll
+      for (int r = 0; r < 32; ++r) x[r] = r == lane ? 1.f : 0.f;
+#pragma unroll
+      for (int r = 0; r < 31; ++r) {
+        if (r < 30) {
+#pragma unroll
+          for (int m = (r + 2) / 4; m < 8; ++m) nc[(r + 1) & 1][m] = *reinterpret_cast<const float4*>(&nd[32 * (r + 1) + 4 * m]);
+        }
+        const float* n = reinterpret_cast<const float*>(nc[r & 1]);
+        if ((r & 1) == 0) x[r + 1] += n[r + 1] * x[r];
+#pragma unroll
+        for (int i = (r + 2) & ~1; i < 32; i += 2) fma2(x[i], x[i + 1], n[i], n[i + 1], x[r], x[r], x[i], x[i + 1]);
+      }
+#pragma unroll
+      for (int r = 0; r < 32; r += 2) {
+        const uint32_t u = pack_bf16(x[r], x[r + 1]);
+        *reinterpret_cast<unsigned short*>(sm.ainv + tile_off(32 * ihalf + r, 32 * ihalf + lane)) = (unsigned short)u;
+        *reinterpret_cast<unsigned short*>(sm.ainv + tile_off(32 * ihalf + r + 1, 32 * ihalf + lane)) = (unsigned short)(u >> 16);
       }
     }
     fence_async_smem();
     tc_fence_before();
     ok = __syncthreads_and(ok);
 
-    R7C_STAMP(4);
-    // ---- MMA 2: [A_qk; A_ak] v  ->  TMEM columns 128..191 (rows 64..127 = Y; the scan computes A_qk v itself, and a
-    // 64-row product of A_ak alone takes the tensor pipe as long)
-    if (warp == 0 && elect_one()) {
-      ok = mbar_wait(&sm.bar_v, par, status, 202) && ok;
+    R7C_STAMP(10);
+    // ---- X_BA on the tensor cores: T = N_BA X_A, then X_B T, with bf16 operands (N_BA is a small correction: rounding
+    // it, X_A, X_B and T to bf16 changes the rounded inverse by less than the rounding of the inverse itself).  Only rows
+    // 32..63 of both products are used, and only half of the 64 contraction elements are not zero.
+    if (warp == 0 && elect_one() && ok) {
       tc_fence_after();
-      umma_tile<128, 64, 0, 1>(tmem_addr(tm, 0, 128), smem_u32(sm.aqk), smem_u32(sm.v), false);
-      umma_commit(&sm.bar_m2);
-      bulk_store(out_tiles + S_AQK * TILE_BYTES, sm.aqk, TILE_BYTES);
-      if (keep_for_bwd) {   // A_ak, a~ are operands of the backward: copy them out before they are overwritten
-        bulk_store(out_tiles + S_AAK * TILE_BYTES, sm.aak, TILE_BYTES);
-        bulk_store(out_tiles + S_AT * TILE_BYTES, sm.at, TILE_BYTES);
-      }
-      bulk_commit();
+      umma_tile<64, 64, 0, 1, 2>(tmem_addr(tm, 0, 128), smem_u32(sm.cm), smem_u32(sm.ainv), false);
+      umma_commit(&sm.bar_m4);
+      if (next < n_ch) load_b(nxt);      // the diagonal blocks have been read
     }
-    // ---- rows of MMA 2 (warps 2, 3, 6, 7), then Ainv = X = (I - N)^-1, N = stril(A_ab), by two levels of block
-    // inversion:
-    //   D. the four 16 x 16 diagonal blocks D_I = (I - N_II)^-1 in fp32, one column per thread, row by row --
-    //      the only substitutions, all four side by side (in place in nmat);
-    //   1. the two 32 x 32 diagonal blocks in fp32: X_10 = D_1 (N_10 D_0) and X_32 = D_3 (N_32 D_2), 64 threads
-    //      each (in place; P = N_IJ D_J passes through the A_qk tile, free once MMA 2 has read it);
-    //   2., 3. the last block X_BA = X_B N_BA X_A (A = rows 0..31, B = rows 32..63) as two tensor-core products.
-    {
-      const int c = tid & 63, I = tid >> 6;
-      float* scratch = reinterpret_cast<float*>(sm.aqk);
-      if ((c >> 4) == I) {       // step D (while MMA 2 runs)
-        float xb[16];
-#pragma unroll
-        for (int rr = 0; rr < 16; ++rr) xb[rr] = (rr == (c & 15)) ? 1.f : 0.f;
-#pragma unroll
-        for (int rr = 1; rr < 16; ++rr) {
-          const float* nrow = &sm.nmat[(16 * I + rr) * NROW + 16 * I];
-          float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f;   // entries at or right of the diagonal are 0
-#pragma unroll
-          for (int jj = 0; jj < (rr + 3) / 4; ++jj) {
-            const float4 n = *reinterpret_cast<const float4*>(nrow + 4 * jj);
-            p0 += n.x * xb[4 * jj];
-            if (4 * jj + 1 < rr) p1 += n.y * xb[4 * jj + 1];
-            if (4 * jj + 2 < rr) p2 += n.z * xb[4 * jj + 2];
-            if (4 * jj + 3 < rr) p3 += n.w * xb[4 * jj + 3];
-          }
-          xb[rr] += (p0 + p1) + (p2 + p3);
-        }
-        __syncwarp((c & 16) ? 0xffff0000u : 0x0000ffffu);   // the 16 columns of a block share a half-warp
-#pragma unroll
-        for (int rr = 0; rr < 16; ++rr) sm.nmat[(16 * I + rr) * NROW + c] = xb[rr];
-      }
-      if (wq >= 2) {      // Y, one column half per warp
-        ok = mbar_wait(&sm.bar_m2, par, status, 203) && ok;
-        tc_fence_after();
-        const int i = (32 * wq + lane) & 63;
-        uint32_t rr[32];
-        tmem_ld32(tmem_addr(tm, 32 * wq, 128 + 32 * hsel), rr);
-        tmem_ld_wait();
+    ok = ok && mbar_wait(&sm.bar_m4, par, status, 209);
+    tc_fence_after();
+    R7C_STAMP(11);
+    if (ok && wq >= 2) {      // T's rows 32..63 (the A_ak tile is free: its copy has left it, MMA 2 has read it)
+      uint32_t rr[32];
+      tmem_ld32(tmem_addr(tm, 32 * wq, 128 + 32 * hsel), rr);
+      tmem_ld_wait();
+      if (lane < 16) {
         float x[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
-        tile_store_row32(sm.y, i, 32 * hsel, x);
+        tile_store_row32(sm.aak, 16 * wq + lane, 32 * hsel, x);
       }
-      // the scratch area: MMA 2 (and the copies of A_qk / A_ak kept for the backward) must be done with it
-      ok = mbar_wait(&sm.bar_m2, par, status, 205) && ok;
-      if (warp == 0 && elect_one()) {
-        bulk_wait_read();                  // q~, k~, b~ (and the tiles kept for the backward) have left shared memory
-        if (next < n_ch) { load_v(nxt); load_qk(nxt); }       // MMA 2 has read the v tile; nothing reads q~, k~ any more
-      }
-      __syncthreads();
-      R7C_STAMP(10);
-      if (I & 1) {               // step 1: row block I, column block I - 1
-        const int cl = tid & 15, r0 = ((tid & 63) >> 4) * 4;
-        const int rb = 16 * I, cbk = 16 * (I - 1);
-        float* P = scratch + (I >> 1) * 256;
-        float col[16], acc[4];
-#pragma unroll
-        for (int kk = 0; kk < 16; ++kk) col[kk] = sm.nmat[(cbk + kk) * NROW + cbk + cl];     // D_J[:, cl]
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float* nrow = &sm.nmat[(rb + r0 + q) * NROW + cbk];
-          float s_ = 0.f;
-#pragma unroll
-          for (int jj = 0; jj < 4; ++jj) {
-            const float4 n = *reinterpret_cast<const float4*>(nrow + 4 * jj);
-            s_ += n.x * col[4 * jj] + n.y * col[4 * jj + 1] + n.z * col[4 * jj + 2] + n.w * col[4 * jj + 3];
-          }
-          acc[q] = s_;
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) P[(r0 + q) * 16 + cl] = acc[q];
-        if (I == 1) asm volatile("bar.sync 1, 64;" ::: "memory");
-        else        asm volatile("bar.sync 2, 64;" ::: "memory");
-#pragma unroll
-        for (int kk = 0; kk < 16; ++kk) col[kk] = P[kk * 16 + cl];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float* drow = &sm.nmat[(rb + r0 + q) * NROW + rb];       // D_I is stored in full (zeros above)
-          float s_ = 0.f;
-#pragma unroll
-          for (int jj = 0; jj < 4; ++jj) {
-            const float4 n = *reinterpret_cast<const float4*>(drow + 4 * jj);
-            s_ += n.x * col[4 * jj] + n.y * col[4 * jj + 1] + n.z * col[4 * jj + 2] + n.w * col[4 * jj + 3];
-          }
-          acc[q] = s_;
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) sm.nmat[(rb + r0 + q) * NROW + cbk + cl] = acc[q];
-      }
-      __syncthreads();
-      R7C_STAMP(11);
-      // steps 2 and 3 on the tensor cores.  With P = diag(X_A, X_B) (the two finished 32 x 32 blocks) and
-      // Q = [0 0; N_BA 0], the missing block is X_BA = (P Q P)_BA: T = Q P, then P T, two 64x64x64 products
-      // of bf16 operands (N_BA is a small correction: rounding it, X_A, X_B and T to bf16 changes the rounded
-      // inverse by less than the rounding of the inverse itself).  P is the Ainv tile with a zero BA
-      // quadrant; Q and T pass through the A_qk / A_ak tiles, free since MMA 2.
-#pragma unroll
-      for (int n = 0; n < 2; ++n) {
-        const int e = tid + 256 * n, row = e >> 3, cc = e & 7;
-        const float4 f0 = *reinterpret_cast<const float4*>(&sm.nmat[row * NROW + 8 * cc]);
-        const float4 f1 = *reinterpret_cast<const float4*>(&sm.nmat[row * NROW + 8 * cc + 4]);
-        const uint4 val = make_uint4(pack_bf16(f0.x, f0.y), pack_bf16(f0.z, f0.w), pack_bf16(f1.x, f1.y), pack_bf16(f1.z, f1.w));
-        const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-        const bool ba = row >= 32 && cc < 4;
-        *reinterpret_cast<uint4*>(sm.ainv + tile_chunk_off(row, cc)) = ba ? zero : val;
-        *reinterpret_cast<uint4*>(sm.aqk + tile_chunk_off(row, cc)) = ba ? val : zero;
-      }
-      fence_async_smem();
-      tc_fence_before();
-      __syncthreads();
-      R7C_STAMP(12);
-      if (warp == 0 && elect_one()) {
-        tc_fence_after();
-        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 128), smem_u32(sm.aqk), smem_u32(sm.ainv), false);     // T = Q P
-        umma_commit(&sm.bar_m4);
-      }
-      ok = mbar_wait(&sm.bar_m4, par, status, 209) && ok;
-      tc_fence_after();
-      if (ok) {
-        uint32_t rr[32];
-        tmem_ld32(tmem_addr(tm, 32 * wq, 128 + 32 * hsel), rr);
-        tmem_ld_wait();
-        if (lane < 16) {        // an M = 64 accumulator lives on the lower 16 lanes of every warp's window
-          float x[32];
-#pragma unroll
-          for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
-          tile_store_row32(sm.aak, 16 * wq + lane, 32 * hsel, x);
-        }
-      }
-      fence_async_smem();
-      tc_fence_before();
-      ok = __syncthreads_and(ok);
-      if (warp == 0 && elect_one() && ok) {
-        tc_fence_after();
-        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 128), smem_u32(sm.ainv), smem_u32(sm.aak), false);     // P T
-        umma_commit(&sm.bar_m5);
-      }
-      ok = mbar_wait(&sm.bar_m5, par, status, 210) && ok;
-      tc_fence_after();
-      if (ok && hsel == 0) {      // rows 32..63, columns 0..31: the BA quadrant of Ainv
-        uint32_t rr[32];
-        tmem_ld32(tmem_addr(tm, 32 * wq, 128), rr);
-        tmem_ld_wait();
-        if (lane < 16 && wq >= 2) {
-          float x[32];
-#pragma unroll
-          for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
-          tile_store_row32(sm.ainv, 16 * wq + lane, 0, x);
-        }
-      }
-      R7C_STAMP(13);
     }
-    R7C_STAMP(5);
+    fence_async_smem();
+    tc_fence_before();
+    ok = __syncthreads_and(ok);
+    R7C_STAMP(12);
+    if (warp == 0 && elect_one() && ok) {
+      tc_fence_after();
+      // contraction elements 32..63: 64 bytes into the rows of A, 32 rows into B
+      umma_tile<64, 64, 0, 1, 2>(tmem_addr(tm, 0, 128), smem_u32(sm.ainv) + 64, smem_u32(sm.aak) + 32 * 128, false);
+      umma_commit(&sm.bar_m5);
+    }
+    ok = ok && mbar_wait(&sm.bar_m5, par, status, 210);
+    tc_fence_after();
+    if (ok && hsel == 0 && wq >= 2) {      // rows 32..63, columns 0..31: the BA quadrant of Ainv
+      uint32_t rr[32];
+      tmem_ld32(tmem_addr(tm, 32 * wq, 128), rr);
+      tmem_ld_wait();
+      if (lane < 16) {
+        float x[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
+        tile_store_row32(sm.ainv, 16 * wq + lane, 0, x);
+      }
+    }
+    R7C_STAMP(13);
     fence_async_smem();
     tc_fence_before();
     ok = __syncthreads_and(ok);
@@ -524,7 +434,6 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
     // ---- MMA 3: W = Ainv a~ (lower lane halves), U = Ainv Y (upper lane halves) -> TMEM columns 0..63; for the
     // backward B2 = Ainv^T b~ and C = A_qb Ainv -> columns 64..127
     if (warp == 0 && elect_one()) {
-      if (ok && next < n_ch) load_w(nxt);      // the scratch area in the A_qk tile is free again
       tc_fence_after();
       umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 0), smem_u32(sm.ainv), smem_u32(sm.at), false);
       umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, 0), smem_u32(sm.ainv), smem_u32(sm.y), false);
@@ -568,8 +477,6 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
         bulk_store(out_tiles + S_B2 * TILE_BYTES, sm.ainv, TILE_BYTES);
       }
       bulk_commit();
-      // MMA 3 has read a~ and b~ (their copies left shared memory long ago): the next raw a, b may land
-      if (next < n_ch) load_ab(nxt);
     }
     R7C_STAMP(9);
   }

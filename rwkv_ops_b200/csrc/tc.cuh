@@ -215,7 +215,7 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
 template <int M, int N, int A_MN, int B_MN, int KSTEPS = 4>
 __device__ __forceinline__ void umma_tile(uint32_t tmem_d, uint32_t a_addr, uint32_t b_addr, bool accumulate,
                                           uint32_t a_lbo = TILE_BYTES, uint32_t b_lbo = TILE_BYTES) {
-  static_assert(KSTEPS == 4 || (A_MN && B_MN), "a K-major operand holds 64 contraction elements");
+  static_assert(KSTEPS <= 4 || (A_MN && B_MN), "a K-major operand holds 64 contraction elements");
   constexpr uint32_t id = idesc_bf16(M, N, A_MN, B_MN);
   // lower descriptor words of step 0; a K=16 step advances the start address by 32 B (K-major) or 2048 B
   // (MN-major), i.e. the word by 2 or 128 (no carry out of the 14-bit field: shared addresses stay below 256 KB)
@@ -287,6 +287,17 @@ __device__ __forceinline__ float ex2(float x) {
 // ---------------------------------------------------------------------------------------------
 // small helpers for moving rows between registers and swizzled tiles
 // ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ float rcp(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// two multiply-adds as one packed instruction
+__device__ __forceinline__ void fma2(float& o0, float& o1, float a0, float a1, float b0, float b1, float c0, float c1) {
+  asm("{\n\t.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+      "mov.b64 c, {%6, %7};\n\tfma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
+      : "=f"(o0), "=f"(o1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1), "f"(c0), "f"(c1));
+}
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
