@@ -438,14 +438,16 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     bulk_load(sm.dhh, tiles + S_DHH * TILE_BYTES, TILE_BYTES, &sm.bar_l0);
     tma_load_4d(sm.v, &tmap_v, &sm.bar_l0, 0, sv.first<PACKED>(p.bi) + p.c * L, p.hi, sv.row<PACKED>(p.bi));
   };
-  auto load_1a = [&](const ChunkPos& p) {     // the other operands of MMA group 1, but for k~ and h~0
+  auto load_1a = [&](const ChunkPos& p) {     // the other operands of MMA group 1, but for sa, k~ and h~0
     const unsigned char* tiles = ws_tiles + (size_t)p.ch * tiles_per_chunk * TILE_BYTES;
     mbar_expect_tx(&sm.bar_l1, 7 * TILE_BYTES);
     tma_load_4d(sm.dout, &tmap_do, &sm.bar_l1, 0, sv.first<PACKED>(p.bi) + p.c * L, p.hi, sv.row<PACKED>(p.bi));
     bulk_load(sm.dz, tiles + S_DZ * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
-    bulk_load(sm.sa, tiles + S_SA * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
     bulk_load(sm.aqk, tiles + S_AQK * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
     bulk_load(sm.aak, tiles + S_AAK * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
+  };
+  auto load_sa = [&](const ChunkPos& p) {
+    bulk_load(sm.sa, ws_tiles + ((size_t)p.ch * tiles_per_chunk + S_SA) * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
   };
   auto load_2 = [&](const ChunkPos& p) {      // k~; q~, a~, b~ (MMA group 2 and the epilogue)
     const unsigned char* tiles = ws_tiles + (size_t)p.ch * tiles_per_chunk * TILE_BYTES;
@@ -498,7 +500,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
 
   uint4 rw[2];
   if (cur.ch < n_ch) {
-    if (warp == st_warp && elect_one()) { load_0(cur); load_1a(cur); load_2(cur); load_1b(cur); }
+    if (warp == st_warp && elect_one()) { load_0(cur); load_1a(cur); load_sa(cur); load_2(cur); load_1b(cur); }
     load_w(cur, rw);
   }
 
@@ -518,6 +520,13 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     const bool more = nxt.ch < n_ch;
     R7C_STAMP(16);
 
+    // X, straight from the workspace: the threads of the last quarter hold a row each until they have dh^
+    uint4 xa[8];
+    if (tid >= 192) {
+      const uint4* xr = reinterpret_cast<const uint4*>(tiles + S_X * TILE_BYTES);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) xa[q] = __ldg(xr + (tile_chunk_off(tid & 63, q) >> 4));
+    }
     // ---- g of every (token, channel), from the w rows already in registers
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
@@ -576,17 +585,15 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
       if (quarter == 0) sm.quart[2][c] = add;      // -gref: the exclusive prefix of the first token
 #pragma unroll
       for (int j = 0; j < 16; ++j) sm.gs[sw64(16 * quarter + j, c)] = gv[j] + add;
-      if (quarter == 3 && ok) {      // X straight from the workspace
+      if (quarter == 3 && ok) {
         ok = mbar_wait(&sm.bar_l0, par, status, 325) && ok;
-        const uint4* xr = reinterpret_cast<const uint4*>(tiles + S_X * TILE_BYTES);
 #pragma unroll
-        for (int cchunk = 0; cchunk < 8; ++cchunk) {
-          const uint4 xa = __ldg(xr + (tile_chunk_off(c, cchunk) >> 4));
-          const uint4 da_ = *reinterpret_cast<const uint4*>(sm.dhh + tile_chunk_off(c, cchunk));
-          dglast += bf16_lo(xa.x) * bf16_lo(da_.x) + bf16_hi(xa.x) * bf16_hi(da_.x);
-          dglast += bf16_lo(xa.y) * bf16_lo(da_.y) + bf16_hi(xa.y) * bf16_hi(da_.y);
-          dglast += bf16_lo(xa.z) * bf16_lo(da_.z) + bf16_hi(xa.z) * bf16_hi(da_.z);
-          dglast += bf16_lo(xa.w) * bf16_lo(da_.w) + bf16_hi(xa.w) * bf16_hi(da_.w);
+        for (int q = 0; q < 8; ++q) {
+          const uint4 da_ = *reinterpret_cast<const uint4*>(sm.dhh + tile_chunk_off(c, q));
+          dglast += bf16_lo(xa[q].x) * bf16_lo(da_.x) + bf16_hi(xa[q].x) * bf16_hi(da_.x);
+          dglast += bf16_lo(xa[q].y) * bf16_lo(da_.y) + bf16_hi(xa[q].y) * bf16_hi(da_.y);
+          dglast += bf16_lo(xa[q].z) * bf16_lo(da_.z) + bf16_hi(xa[q].z) * bf16_hi(da_.z);
+          dglast += bf16_lo(xa[q].w) * bf16_lo(da_.w) + bf16_hi(xa[q].w) * bf16_hi(da_.w);
         }
       }
     }
@@ -756,7 +763,9 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
 #pragma unroll
       for (int j = 15; j >= 0; --j) { run += rv[j]; rv[j] = run; }
       const float gfirst = quarter ? sm.gs[sw64(16 * quarter - 1, c)] : sm.quart[2][c];
-      __syncthreads();      // -gref has been read
+      fence_async_smem();
+      __syncthreads();      // -gref has been read, and red1, red2
+      if (warp == st_warp && elect_one() && ok && more) load_1a(nxt);
       if (quarter) sm.quart[quarter - 1][c] = run;      // the last quarter's sum carries dglast
       __syncthreads();
       float add = 0.f;
@@ -787,7 +796,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
         bulk_commit();
       }
       if (more) {
-        load_1a(nxt);
+        load_sa(nxt);
         bulk_wait_read_1();       // dq, dk, da, db have left their tiles
         load_2(nxt);
         bulk_wait_read();         // and dw
