@@ -365,6 +365,7 @@ int make_token_tensor_map(CUtensorMap* out, const void* base, int B, int T, int 
 int* device_status_ptr();
 
 int make_row_tensor_map(CUtensorMap* out, const void* base, int B, int T, int H, int elem_bytes);
+int make_state_tensor_map(CUtensorMap* out, const void* base, long long rows);
 
 // Device buffer (>= 64 long long) that kernels fill with clock64() stamps at their phase boundaries (one
 // designated CTA).  Only the developer build (-DRWKVB200_DEVTOOLS) can install one and only its kernels

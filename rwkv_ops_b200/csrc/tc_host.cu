@@ -86,6 +86,24 @@ int make_row_tensor_map(CUtensorMap* out, const void* base, int B, int T, int H,
   return RWKVB200_E_CUDA;
 }
 
+// [rows][64] float32, box = 64 rows x 32 elements, 128-byte swizzle: the box lands like a bf16 tile, with 16-byte pieces of
+// four floats
+int make_state_tensor_map(CUtensorMap* out, const void* base, long long rows) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) { last_cuda_error_slot() = 100000; return RWKVB200_E_CUDA; }
+  cuuint64_t dims[4] = {(cuuint64_t)HS, (cuuint64_t)rows, 1, 1};
+  cuuint64_t strides[3] = {HS * 4, (cuuint64_t)rows * HS * 4, (cuuint64_t)rows * HS * 4};
+  cuuint32_t box[4] = {32, 64, 1, 1};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  if (bind_context()) return RWKVB200_E_CUDA;
+  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r == CUDA_SUCCESS) return RWKVB200_OK;
+  last_cuda_error_slot() = 100000 + (int)r;
+  return RWKVB200_E_CUDA;
+}
+
 #ifdef RWKVB200_DEVTOOLS
 static long long* g_stamp_buffer = nullptr;
 long long* debug_stamp_buffer() { return g_stamp_buffer; }

@@ -67,11 +67,11 @@ __device__ __forceinline__ void store_split4(unsigned char* hi_t, unsigned char*
   *reinterpret_cast<uint2*>(hi_t + off) = h;
   *reinterpret_cast<uint2*>(lo_t + off) = l;
 }
-// write 32 consecutive fp32 values of `row` (columns col0 .., col0 a multiple of 8) into a hi and a lo tile
-__device__ __forceinline__ void store_split_row32(unsigned char* hi_t, unsigned char* lo_t, int row, int col0,
-                                                  const float* x) {
+// write CW consecutive fp32 values of `row` (columns col0 .., col0 a multiple of 8) into a hi and a lo tile
+template <int CW>
+__device__ __forceinline__ void store_split_row(unsigned char* hi_t, unsigned char* lo_t, int row, int col0, const float* x) {
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
+  for (int c = 0; c < CW / 8; ++c) {
     uint4 h, l;
     split_pair(x[8 * c + 0], x[8 * c + 1], h.x, l.x);
     split_pair(x[8 * c + 2], x[8 * c + 3], h.y, l.y);
@@ -83,6 +83,36 @@ __device__ __forceinline__ void store_split_row32(unsigned char* hi_t, unsigned 
   }
 }
 
+// How a CTA of NTHR threads (256 or 512) splits a chunk of 64 tokens x 64 channels: a token row is 16 threads wide (four
+// channels each); a (channel, part) thread owns PL consecutive tokens; a thread that reads an accumulator takes CW
+// columns of its lane.
+template <int NTHR>
+struct Split {
+  static constexpr int NE = 1024 / NTHR;        // token rows per thread
+  static constexpr int PARTS = NTHR / 64, PL = 64 / PARTS;
+  static constexpr int CW = 8192 / NTHR;
+};
+// sums over the parts of the first / second half of the chunk, from the sums over the parts
+template <int PARTS>
+__device__ __forceinline__ float half_sum(const float (*tot)[64], int half, int ch) {
+  float x = tot[half * (PARTS / 2)][ch];
+#pragma unroll
+  for (int q = 1; q < PARTS / 2; ++q) x += tot[half * (PARTS / 2) + q][ch];
+  return x;
+}
+// What to add to the prefix sums of a part (its own sum is `run`) so that they count from the end of the first half.
+template <int PARTS>
+__device__ __forceinline__ float from_middle(const float (*tot)[64], int part, int ch, float run) {
+  constexpr int HALF = PARTS / 2;
+  float add = part < HALF ? -run : 0.f;
+#pragma unroll
+  for (int q = 0; q < HALF; ++q) {
+    if (part < HALF && q > part) add -= tot[q][ch];
+    if (part >= HALF && HALF + q < part) add += tot[HALF + q][ch];
+  }
+  return add;
+}
+
 // D (+)= X Y with X = xh + xl, Y = yh + yl (lo tile = hi tile + TILE_BYTES): hi*hi + hi*lo + lo*hi
 template <int M, int N, int A_MN, int B_MN>
 __device__ __forceinline__ void umma_split(uint32_t tmem_d, uint32_t a_hi, uint32_t b_hi, bool accumulate) {
@@ -91,38 +121,39 @@ __device__ __forceinline__ void umma_split(uint32_t tmem_d, uint32_t a_hi, uint3
   umma_tile<M, N, A_MN, B_MN>(tmem_d, a_hi + TILE_BYTES, b_hi, true);
 }
 
-// Row `lr` (0..15) of a warp's 16 x 32 block of a 64 x 64 product that is kept strictly below the diagonal, the
+// Row `lr` (0..15) of a warp's 16 x CW block of a 64 x 64 product that is kept strictly below the diagonal, the
 // diagonal itself set to `diag`, split and stored.  Where the diagonal crosses the block depends on the warp alone:
-// left of column JLO (of the block's 32) every element is kept, from JLO + 16 on every element is zero, and only
-// the 16 columns between take a per-element choice.  JLO = 32: the whole block is kept; JLO = -16: all zero
+// left of column JLO (of the block's CW) every element is kept, from JLO + 16 on every element is zero, and only
+// the 16 columns between take a per-element choice.  JLO = CW: the whole block is kept; JLO = -16: all zero
 // (`rr` is not read).
-template <int JLO>
-__device__ __forceinline__ void store_masked_row(const uint32_t (&rr)[32], int lr, float diag, unsigned char* hi_t,
+template <int CW, int JLO>
+__device__ __forceinline__ void store_masked_row(const uint32_t (&rr)[CW], int lr, float diag, unsigned char* hi_t,
                                                  int row, int col0) {
-  float x[32];
+  float x[CW];
 #pragma unroll
-  for (int j = 0; j < 32; ++j) {
+  for (int j = 0; j < CW; ++j) {
     if (j < JLO) x[j] = __uint_as_float(rr[j]);
     else if (j >= JLO + 16) x[j] = 0.f;
     else x[j] = (j - JLO) < lr ? __uint_as_float(rr[j]) : ((j - JLO) == lr ? diag : 0.f);
   }
-  store_split_row32(hi_t, hi_t + TILE_BYTES, row, col0, x);
+  store_split_row<CW>(hi_t, hi_t + TILE_BYTES, row, col0, x);
 }
-// the same for a warp whose rows are 16*wq .. and whose columns are 32*hsel ..; all lanes of the warp call it
+// the same for a warp whose rows are 16*wq .. and whose columns are CW*hsel ..; all lanes of the warp call it
+template <int CW>
 __device__ __forceinline__ void load_store_masked_row(uint32_t taddr, int wq, int hsel, int lr, float diag,
                                                       unsigned char* hi_t, int row, bool active) {
-  const int jlo = 16 * wq - 32 * hsel;
-  uint32_t rr[32];
+  const int jlo = 16 * wq - CW * hsel;
+  uint32_t rr[CW];
   if (jlo < 0) {
-    if (active) store_masked_row<-16>(rr, lr, diag, hi_t, row, 32 * hsel);
+    if (active) store_masked_row<CW, -16>(rr, lr, diag, hi_t, row, CW * hsel);
     return;
   }
-  tmem_ld32(taddr, rr);
+  tmem_ld<CW>(taddr, rr);
   tmem_ld_wait();
   if (!active) return;
-  if (jlo >= 32) store_masked_row<32>(rr, lr, diag, hi_t, row, 32 * hsel);
-  else if (jlo == 16) store_masked_row<16>(rr, lr, diag, hi_t, row, 32 * hsel);
-  else store_masked_row<0>(rr, lr, diag, hi_t, row, 32 * hsel);
+  if (jlo >= CW) store_masked_row<CW, CW>(rr, lr, diag, hi_t, row, CW * hsel);
+  else if (CW == 32 && jlo == 16) store_masked_row<CW, 16>(rr, lr, diag, hi_t, row, CW * hsel);
+  else store_masked_row<CW, 0>(rr, lr, diag, hi_t, row, CW * hsel);
 }
 
 __device__ __forceinline__ long long state_row(const int32_t* smap, int n_state, int bi) {
@@ -152,7 +183,7 @@ struct FwdSmem {
   unsigned char at[2][TILE_BYTES];    // A hi, lo       [token i][token j]
   unsigned char st[2][TILE_BYTES];    // S~0 hi, lo     [k][v]
   float gs[L * NROW];                 // gi - gref (prefix of g relative to the reference point); later the staged y rows
-  float qtot[4][64];
+  float qtot[8][64];
   float dgs[64];                      // sum_k r u k per token
   uint64_t bar_1, bar_2, bar_in;
   uint32_t tmem_base;
@@ -164,8 +195,8 @@ struct FwdSmem {
 // the last MMA of the current one has read those tiles; a thread reads its elements, all threads meet at a
 // barrier, and then the split tiles are written over the raw rows.
 // S0 of every chunk (and the final state) goes to `states` [B*H][NT+1][64][64] when it is not NULL.
-template <typename T, bool PACKED>
-__global__ void __launch_bounds__(256, 2)
+template <typename T, bool PACKED, int NTHR>
+__global__ void __launch_bounds__(NTHR, 512 / NTHR)
 wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ w,
                  const float* __restrict__ u, const float* __restrict__ s0, int n_state,
                  const int32_t* __restrict__ smap, T* __restrict__ y, float* __restrict__ sT,
@@ -182,6 +213,7 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   FwdSmem& sm = *reinterpret_cast<FwdSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int wq = warp & 3, hsel = warp >> 2;
+  constexpr int NE = Split<NTHR>::NE, PARTS = Split<NTHR>::PARTS, PL = Split<NTHR>::PL, CW = Split<NTHR>::CW;
   const long long tstride = (long long)H * HS;
   const int srow = 16 * wq + (lane & 15);     // state row k (upper lane halves) / token row (lower lane halves)
   const bool tok_lane = lane < 16;            // lower lane halves hold token rows, upper halves state rows
@@ -197,8 +229,8 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   tc_fence_after();
   const uint32_t tm = sm.tmem_base;
   // TMEM: columns 0..63 lower halves = r~ k~^T; columns 64..127 lower halves = y, upper halves = k~^T v
-  const uint32_t tm_a = tmem_addr(tm, 32 * wq, 32 * hsel);
-  const uint32_t tm_ys = tmem_addr(tm, 32 * wq, 64 + 32 * hsel);
+  const uint32_t tm_a = tmem_addr(tm, 32 * wq, CW * hsel);
+  const uint32_t tm_ys = tmem_addr(tm, 32 * wq, 64 + CW * hsel);
 
   const int c4 = tid & 15;
   const T* raw_r = reinterpret_cast<const T*>(sm.rt[0]);
@@ -241,9 +273,9 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   const float4 u4 = *reinterpret_cast<const float4*>(u + hi * HS + 4 * c4);
 
   // ---- state at the item's first chunk: rows k on the upper lane halves, this warp's 32 columns
-  float sreg[32];
+  float sreg[CW];
 #pragma unroll
-  for (int j = 0; j < 32; ++j) sreg[j] = 0.f;
+  for (int j = 0; j < CW; ++j) sreg[j] = 0.f;
   if (part > 0) {
     // wait for the stretch before this one (taken before this item, by a CTA that is running): bounded
     if (tid == 0) {
@@ -259,21 +291,29 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     __syncthreads();
     ok = sm.handoff_ok != 0;
     if (!tok_lane && ok) {
-      const float* S = handoff + (((size_t)unit * HS) + srow) * HS + 32 * hsel;
+      const float* S = handoff + (((size_t)unit * HS) + srow) * HS + CW * hsel;
 #pragma unroll
-      for (int j = 0; j < 32; j += 4) {
+      for (int j = 0; j < CW; j += 4) {
         const float4 fv = __ldcg(reinterpret_cast<const float4*>(S + j));
         sreg[j] = fv.x; sreg[j + 1] = fv.y; sreg[j + 2] = fv.z; sreg[j + 3] = fv.w;
       }
     }
   } else if (!tok_lane && s0 && n_state > 0) {
-    const float* S = s0 + ((state_row(smap, n_state, bi) * H + hi) * HS + srow) * HS + 32 * hsel;
+    const float* S = s0 + ((state_row(smap, n_state, bi) * H + hi) * HS + srow) * HS + CW * hsel;
 #pragma unroll
-    for (int j = 0; j < 32; j += 4) {
+    for (int j = 0; j < CW; j += 4) {
       const float4 fv = *reinterpret_cast<const float4*>(S + j);
       sreg[j] = fv.x; sreg[j + 1] = fv.y; sreg[j + 2] = fv.z; sreg[j + 3] = fv.w;
     }
   }
+
+  auto keep_state = [&](int c) {      // the state before chunk c
+    float* dst = states + (((size_t)unit * nts + c) * HS + srow) * HS + CW * hsel;
+#pragma unroll
+    for (int j = 0; j < CW; j += 4)
+      *reinterpret_cast<float4*>(dst + j) = make_float4(sreg[j], sreg[j + 1], sreg[j + 2], sreg[j + 3]);
+  };
+  if (states && !tok_lane && part == 0) keep_state(0);
 
   auto load_in = [&](int c) {      // tid 0; rows past the end of the sequence arrive as zeros
     mbar_expect_tx(&sm.bar_in, 4 * 64 * 64 * (uint32_t)sizeof(T));
@@ -290,10 +330,10 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     W6C_STAMP(0);
     // ---- the raw rows of the chunk have landed: this thread's w and v elements
     ok = mbar_wait(&sm.bar_in, par, status, 403) && ok;
-    float4 gw[4], vv4[4];
+    float4 gw[NE], vv4[NE];
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      const int e = tid + 256 * n, row = e >> 4;
+    for (int n = 0; n < NE; ++n) {
+      const int e = tid + NTHR * n, row = e >> 4;
       gw[n] = load4_shared(raw_w + row * 64 + 4 * c4);
       vv4[n] = load4_shared(raw_v + row * 64 + 4 * c4);
       if (PACKED && t0 + row >= Tn) vv4[n] = make_float4(0.f, 0.f, 0.f, 0.f);      // the next sequence's row
@@ -301,8 +341,8 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     __syncthreads();      // every raw v element is in registers: the split v tiles may overwrite the rows
     // ---- pass W: g and its prefix sums; pass V
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      const int e = tid + 256 * n, row = e >> 4, tok = t0 + row;
+    for (int n = 0; n < NE; ++n) {
+      const int e = tid + NTHR * n, row = e >> 4, tok = t0 + row;
       float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
       if (tok < Tn)
         f = make_float4(-LOG2E * ex2(LOG2E * gw[n].x), -LOG2E * ex2(LOG2E * gw[n].y), -LOG2E * ex2(LOG2E * gw[n].z),
@@ -314,26 +354,25 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     __syncthreads();
     W6C_STAMP(1);
     {
-      const int ch = tid & 63, quarter = tid >> 6;
-      float gv[16];
+      const int ch = tid & 63, part = tid >> 6;
+      float gv[PL];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) gv[j] = sm.gs[(16 * quarter + j) * NROW + ch];
+      for (int j = 0; j < PL; ++j) gv[j] = sm.gs[(PL * part + j) * NROW + ch];
       float run = 0.f;
 #pragma unroll
-      for (int j = 0; j < 16; ++j) { run += gv[j]; gv[j] = run; }
-      sm.qtot[quarter][ch] = run;
+      for (int j = 0; j < PL; ++j) { run += gv[j]; gv[j] = run; }
+      sm.qtot[part][ch] = run;
       __syncthreads();
-      // gi - gref: the prefix inside the half; the reference point is the end of the first half
-      const float add = quarter == 0 ? -(run + sm.qtot[1][ch]) : quarter == 1 ? -run : quarter == 3 ? sm.qtot[2][ch] : 0.f;
+      const float add = from_middle<PARTS>(sm.qtot, part, ch, run);
 #pragma unroll
-      for (int j = 0; j < 16; ++j) sm.gs[(16 * quarter + j) * NROW + ch] = gv[j] + add;
+      for (int j = 0; j < PL; ++j) sm.gs[(PL * part + j) * NROW + ch] = gv[j] + add;
     }
     __syncthreads();
     W6C_STAMP(2);
     // decay factors of the state rows: e^{gref} of this chunk scales the incoming state, e^{glast-gref} the outgoing
     float e0 = 1.f, dlast = 1.f;
     if (!tok_lane) {
-      const float tot0 = sm.qtot[0][srow] + sm.qtot[1][srow], tot1 = sm.qtot[2][srow] + sm.qtot[3][srow];
+      const float tot0 = half_sum<PARTS>(sm.qtot, 0, srow), tot1 = half_sum<PARTS>(sm.qtot, 1, srow);
       e0 = ex2(fmaxf(tot0, EXP2_FLOOR));
       dlast = ex2(fmaxf(tot1, EXP2_FLOOR));
       // a half-chunk decay sum beyond the limit: the unit is recomputed by the float32 recurrence
@@ -341,30 +380,24 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     }
     // ---- S~0 = e^{gref} S0 stays in registers (fp32); hi/lo bf16 tiles for the r~ S~0 product
     if (!tok_lane) {
-      if (states) {
-        float* dst = states + (((size_t)unit * nts + c) * HS + srow) * HS + 32 * hsel;
 #pragma unroll
-        for (int j = 0; j < 32; j += 4)
-          *reinterpret_cast<float4*>(dst + j) = make_float4(sreg[j], sreg[j + 1], sreg[j + 2], sreg[j + 3]);
-      }
-#pragma unroll
-      for (int j = 0; j < 32; ++j) sreg[j] *= e0;
-      store_split_row32(sm.st[0], sm.st[1], srow, 32 * hsel, sreg);
+      for (int j = 0; j < CW; ++j) sreg[j] *= e0;
+      store_split_row<CW>(sm.st[0], sm.st[1], srow, CW * hsel, sreg);
     }
     W6C_STAMP(3);
     // ---- pass RK: scaled r, k (split hi/lo) and the diagonal term
-    float4 rr4[4], kk4[4];
+    float4 rr4[NE], kk4[NE];
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      const int row = (tid + 256 * n) >> 4;
+    for (int n = 0; n < NE; ++n) {
+      const int row = (tid + NTHR * n) >> 4;
       rr4[n] = load4_shared(raw_r + row * 64 + 4 * c4);
       kk4[n] = load4_shared(raw_k + row * 64 + 4 * c4);
       if (PACKED && t0 + row >= Tn) { rr4[n] = make_float4(0.f, 0.f, 0.f, 0.f); kk4[n] = rr4[n]; }
     }
     __syncthreads();      // every raw r, k element is in registers
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      const int e = tid + 256 * n, row = e >> 4;
+    for (int n = 0; n < NE; ++n) {
+      const int e = tid + NTHR * n, row = e >> 4;
       const float4 r4 = rr4[n], k4 = kk4[n];
       const float4 gp = *reinterpret_cast<const float4*>(&sm.gs[row * NROW + 4 * c4]);
       const float d1x = gp.x, d1y = gp.y, d1z = gp.z, d1w = gp.w;   // gi - gref
@@ -403,14 +436,14 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     W6C_STAMP(5);
     if (ok) {
       // A rows (lower halves of columns 0..63): strictly lower part plus the diagonal term, split hi/lo
-      uint32_t rr[32];
-      load_store_masked_row(tm_a, wq, hsel, lane & 15, tok_lane ? sm.dgs[srow] : 0.f, sm.at[0], srow, tok_lane);
+      uint32_t rr[CW];
+      load_store_masked_row<CW>(tm_a, wq, hsel, lane & 15, tok_lane ? sm.dgs[srow] : 0.f, sm.at[0], srow, tok_lane);
       // state rows (k~^T v on the upper halves of columns 64..127): S_L = e^{glast-gref} (S~0 + k~^T v)
-      tmem_ld32(tm_ys, rr);
+      tmem_ld<CW>(tm_ys, rr);
       tmem_ld_wait();
       if (!tok_lane) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) sreg[j] = (sreg[j] + __uint_as_float(rr[j])) * dlast;
+        for (int j = 0; j < CW; ++j) sreg[j] = (sreg[j] + __uint_as_float(rr[j])) * dlast;
       }
     }
     fence_async_smem();
@@ -424,18 +457,21 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
       umma_split<64, 64, 0, 1>(tmem_addr(tm, 0, 64), smem_u32(sm.at[0]), smem_u32(sm.vt[0]), true);
       umma_commit(&sm.bar_2);
     }
+    // the state of the next chunk's start, stored here because the next proxy fence, which waits for global stores too, is
+    // most of a chunk away
+    if (states && !tok_lane && ok) keep_state(c + 1);
     ok = mbar_wait(&sm.bar_2, par, status, 402) && ok;
     tc_fence_after();
     W6C_STAMP(7);
     if (warp == 0 && elect_one() && ok && c + 1 < c_hi) load_in(c + 1);      // the tiles of this chunk have been read for the last time
     if (ok) {
-      uint32_t rr[32];
-      tmem_ld32(tm_ys, rr);
+      uint32_t rr[CW];
+      tmem_ld<CW>(tm_ys, rr);
       tmem_ld_wait();
       if (tok_lane) {     // stage the y rows (fp32) in the prefix-sum area, then store them coalesced
 #pragma unroll
-        for (int j = 0; j < 32; j += 4)
-          *reinterpret_cast<float4*>(&sm.gs[srow * NROW + 32 * hsel + j]) =
+        for (int j = 0; j < CW; j += 4)
+          *reinterpret_cast<float4*>(&sm.gs[srow * NROW + CW * hsel + j]) =
               make_float4(__uint_as_float(rr[j]), __uint_as_float(rr[j + 1]), __uint_as_float(rr[j + 2]),
                           __uint_as_float(rr[j + 3]));
       }
@@ -445,8 +481,8 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     W6C_STAMP(8);
     if (y && ok) {
 #pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        const int e = tid + 256 * n, row = e >> 4, tok = t0 + row;
+      for (int n = 0; n < NE; ++n) {
+        const int e = tid + NTHR * n, row = e >> 4, tok = t0 + row;
         if (tok < Tn)
           store4(y + base + (long long)tok * tstride + 4 * c4,
                  *reinterpret_cast<const float4*>(&sm.gs[row * NROW + 4 * c4]));
@@ -460,21 +496,15 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   if (!tok_lane && ok) {
     if (last_part) {
       if (sT) {
-        float* dst = sT + (((size_t)unit * HS) + srow) * HS + 32 * hsel;
+        float* dst = sT + (((size_t)unit * HS) + srow) * HS + CW * hsel;
 #pragma unroll
-        for (int j = 0; j < 32; j += 4)
-          *reinterpret_cast<float4*>(dst + j) = make_float4(sreg[j], sreg[j + 1], sreg[j + 2], sreg[j + 3]);
-      }
-      if (states) {
-        float* dst = states + (((size_t)unit * nts + NT) * HS + srow) * HS + 32 * hsel;
-#pragma unroll
-        for (int j = 0; j < 32; j += 4)
+        for (int j = 0; j < CW; j += 4)
           *reinterpret_cast<float4*>(dst + j) = make_float4(sreg[j], sreg[j + 1], sreg[j + 2], sreg[j + 3]);
       }
     } else {
-      float* dst = handoff + (((size_t)unit * HS) + srow) * HS + 32 * hsel;
+      float* dst = handoff + (((size_t)unit * HS) + srow) * HS + CW * hsel;
 #pragma unroll
-      for (int j = 0; j < 32; j += 4)
+      for (int j = 0; j < CW; j += 4)
         *reinterpret_cast<float4*>(dst + j) = make_float4(sreg[j], sreg[j + 1], sreg[j + 2], sreg[j + 3]);
     }
   }
@@ -508,32 +538,34 @@ struct BwdSmem {
   float gs[L * NROW];                 // gi - gref (prefix of g relative to the reference point)
   float gg[L * NROW];                 // g log2(e)
   float red_e[L * NROW];              // dr~ r~
-  float qtot[4][64];
-  float rqtot[4][64];
-  float pqtot[4][64];
+  float qtot[8][64];
+  float rqtot[8][64];
+  float pqtot[8][64];
   float dgs[64];                      // sum_k r u k per token
   float dds[64];                      // dy_i . v_i per token
-  float dgl[2][64];                   // sum_v dS^ S~0, one partial per column half
+  float dgl[4][64];                   // sum_v dS^ S~0, one partial per group of columns
   float du_s[64];
   // raw rows of the next chunk, requested by TMA a chunk ahead: w and dy (needed first) here; r and k land
   // in the space of rt / kt once the last epilogue has read those, v in red_e once the decay gradient has
   alignas(128) unsigned char raw_w[L * 64 * 4];
   alignas(128) unsigned char raw_dy[L * 64 * 4];
-  uint64_t bar_1, bar_2, bar_2a, bar_in_a, bar_in_b, bar_in_c;
+  uint64_t bar_1, bar_2, bar_2a, bar_in_a, bar_in_b, bar_in_c, bar_s;
   uint32_t tmem_base;
   int handoff_ok, next_item;
 };
 static_assert(sizeof(BwdSmem) + 1024 <= 227 * 1024, "backward shared memory");
 
+constexpr int BWD_THREADS = 256;
+
 template <typename T, bool PACKED>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(BWD_THREADS)
 wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ w,
                  const float* __restrict__ u, const T* __restrict__ d_y, const float* __restrict__ d_sT,
                  const float* __restrict__ states, T* __restrict__ dr, T* __restrict__ dk, T* __restrict__ dv,
                  T* __restrict__ dw, float* __restrict__ du_partial, float* __restrict__ d_s0,
                  const __grid_constant__ CUtensorMap tmap_r, const __grid_constant__ CUtensorMap tmap_k,
                  const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_w,
-                 const __grid_constant__ CUtensorMap tmap_dy, int Tn_dense, int H, Seqs seqs, int n_units,
+                 const __grid_constant__ CUtensorMap tmap_dy, const __grid_constant__ CUtensorMap tmap_s, int Tn_dense, int H, Seqs seqs, int n_units,
                  int split, float* __restrict__ handoff, int* __restrict__ handoff_flags, int* status,
                  long long* dbg) {
 #ifdef RWKVB200_DEVTOOLS
@@ -545,6 +577,8 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   BwdSmem& sm = *reinterpret_cast<BwdSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int wq = warp & 3, hsel = warp >> 2;
+  constexpr int NTHR = BWD_THREADS;
+  constexpr int NE = Split<NTHR>::NE, PARTS = Split<NTHR>::PARTS, PL = Split<NTHR>::PL, CW = Split<NTHR>::CW;
   const long long tstride = (long long)H * HS;
   const int srow = 16 * wq + (lane & 15);
   const bool lower = lane < 16;
@@ -561,7 +595,7 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     // every MMA batch is issued by two threads (threads 0 and 32, each with accumulators of its own) and completes
     // with the arrival of both
     mbar_init(&sm.bar_1, 2); mbar_init(&sm.bar_2, 2); mbar_init(&sm.bar_2a, 2);
-    mbar_init(&sm.bar_in_a, 1); mbar_init(&sm.bar_in_b, 1); mbar_init(&sm.bar_in_c, 1);
+    mbar_init(&sm.bar_in_a, 1); mbar_init(&sm.bar_in_b, 1); mbar_init(&sm.bar_in_c, 1); mbar_init(&sm.bar_s, 1);
     fence_mbar_init();
   }
   if (warp == 0) tmem_alloc(&sm.tmem_base, 256);
@@ -569,10 +603,10 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   __syncthreads();
   tc_fence_after();
   const uint32_t tm = sm.tmem_base;
-  const uint32_t tm_c0 = tmem_addr(tm, 32 * wq, 32 * hsel);          // A (lower), dA (upper)
-  const uint32_t tm_c1 = tmem_addr(tm, 32 * wq, 64 + 32 * hsel);     // dk~ (lower), dr~ (upper)
-  const uint32_t tm_c2 = tmem_addr(tm, 32 * wq, 128 + 32 * hsel);    // dv (lower), dS~0 (upper)
-  const uint32_t tm_c3 = tmem_addr(tm, 32 * wq, 192 + 32 * hsel);    // X = v dS^^T (lower): the state part of dk~
+  const uint32_t tm_c0 = tmem_addr(tm, 32 * wq, CW * hsel);          // A (lower), dA (upper)
+  const uint32_t tm_c1 = tmem_addr(tm, 32 * wq, 64 + CW * hsel);     // dk~ (lower), dr~ (upper)
+  const uint32_t tm_c2 = tmem_addr(tm, 32 * wq, 128 + CW * hsel);    // dv (lower), dS~0 (upper)
+  const uint32_t tm_c3 = tmem_addr(tm, 32 * wq, 192 + CW * hsel);    // X = v dS^^T (lower): the state part of dk~
 
   constexpr uint32_t RAW_BYTES = 64 * 64 * (uint32_t)sizeof(T);
   const T* raw_w = reinterpret_cast<const T*>(sm.raw_w);
@@ -621,9 +655,9 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   if (tid < 64) sm.du_s[tid] = 0.f;
 
   // gradient of the state after the current chunk: row k = srow (upper lane halves), 32 columns
-  float dsreg[32];
+  float dsreg[CW];
 #pragma unroll
-  for (int j = 0; j < 32; ++j) dsreg[j] = 0.f;
+  for (int j = 0; j < CW; ++j) dsreg[j] = 0.f;
   if (early_half) {
     // wait for the later half of this unit (taken before this item, by a CTA that is running): bounded
     if (tid == 0) {
@@ -639,17 +673,17 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     __syncthreads();
     ok = sm.handoff_ok != 0;
     if (!lower && ok) {
-      const float* S = handoff + (((size_t)unit * HS) + srow) * HS + 32 * hsel;
+      const float* S = handoff + (((size_t)unit * HS) + srow) * HS + CW * hsel;
 #pragma unroll
-      for (int j = 0; j < 32; j += 4) {
+      for (int j = 0; j < CW; j += 4) {
         const float4 f = __ldcg(reinterpret_cast<const float4*>(S + j));
         dsreg[j] = f.x; dsreg[j + 1] = f.y; dsreg[j + 2] = f.z; dsreg[j + 3] = f.w;
       }
     }
   } else if (!lower && d_sT) {
-    const float* S = d_sT + (((size_t)unit * HS) + srow) * HS + 32 * hsel;
+    const float* S = d_sT + (((size_t)unit * HS) + srow) * HS + CW * hsel;
 #pragma unroll
-    for (int j = 0; j < 32; j += 4) {
+    for (int j = 0; j < CW; j += 4) {
       const float4 f = *reinterpret_cast<const float4*>(S + j);
       dsreg[j] = f.x; dsreg[j + 1] = f.y; dsreg[j + 2] = f.z; dsreg[j + 3] = f.w;
     }
@@ -677,13 +711,13 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     const uint32_t par = n_done & 1;
     W6C_STAMP(32);
     // ---- r and k are read at pass RK and stay in registers until the u-term gradients at the end of the chunk
-    float4 gw[4], rr4[4], kk4[4];
+    float4 gw[NE], rr4[NE], kk4[NE];
     {
       ok = mbar_wait(&sm.bar_in_a, par, status, 413) && ok;
       // ---- pass W: g; pass DY: split tiles
 #pragma unroll
-      for (int n = 0; n < 4; ++n) {
-        const int e = tid + 256 * n, row = e >> 4, tok = t0 + row;
+      for (int n = 0; n < NE; ++n) {
+        const int e = tid + NTHR * n, row = e >> 4, tok = t0 + row;
         const float4 w4 = load4_shared(raw_w + row * 64 + 4 * c4);
         float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
         if (tok < Tn)
@@ -698,21 +732,30 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     }
     __syncthreads();
     W6C_STAMP(33);
+    // S0 of this chunk (fp32, two 64 x 32 halves swizzled like the tiles) into the space of A, which nothing else uses until
+    // MMA batch 1 is read out.  By TMA, because loads to registers are uncoalesced here and the proxy fence before batch
+    // 1 waits for them.
+    if (warp == 1 && elect_one() && ok) {
+      fence_async_smem();
+      const int srow0 = (int)(((size_t)unit * nts + c) * HS);
+      mbar_expect_tx(&sm.bar_s, 2 * TILE_BYTES);
+      tma_load_4d(sm.at[0], &tmap_s, &sm.bar_s, 0, srow0, 0, 0);
+      tma_load_4d(sm.at[1], &tmap_s, &sm.bar_s, 32, srow0, 0, 0);
+    }
 
     {
-      const int ch = tid & 63, quarter = tid >> 6;
-      float gv[16];
+      const int ch = tid & 63, part = tid >> 6;
+      float gv[PL];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) gv[j] = sm.gg[(16 * quarter + j) * NROW + ch];
+      for (int j = 0; j < PL; ++j) gv[j] = sm.gg[(PL * part + j) * NROW + ch];
       float run = 0.f;
 #pragma unroll
-      for (int j = 0; j < 16; ++j) { run += gv[j]; gv[j] = run; }
-      sm.qtot[quarter][ch] = run;
+      for (int j = 0; j < PL; ++j) { run += gv[j]; gv[j] = run; }
+      sm.qtot[part][ch] = run;
       __syncthreads();
-      // gi - gref: the prefix inside the half; the reference point is the end of the first half
-      const float add = quarter == 0 ? -(run + sm.qtot[1][ch]) : quarter == 1 ? -run : quarter == 3 ? sm.qtot[2][ch] : 0.f;
+      const float add = from_middle<PARTS>(sm.qtot, part, ch, run);
 #pragma unroll
-      for (int j = 0; j < 16; ++j) sm.gs[(16 * quarter + j) * NROW + ch] = gv[j] + add;
+      for (int j = 0; j < PL; ++j) sm.gs[(PL * part + j) * NROW + ch] = gv[j] + add;
     }
     __syncthreads();
     W6C_STAMP(34);
@@ -722,8 +765,8 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     ok = mbar_wait(&sm.bar_in_b, par, status, 415) && ok;
     ok = mbar_wait(&sm.bar_in_c, par, status, 414) && ok;
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      const int row = (tid + 256 * n) >> 4;
+    for (int n = 0; n < NE; ++n) {
+      const int row = (tid + NTHR * n) >> 4;
       rr4[n] = load4_shared(raw_r + row * 64 + 4 * c4);
       kk4[n] = load4_shared(raw_k + row * 64 + 4 * c4);
       // pass V: split tiles and dd_i = dy_i . v_i
@@ -740,8 +783,8 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     __syncthreads();
     if (warp == 0 && elect_one() && ok && c > c_lo) load_in_a(c - 1);      // every thread has taken its w and dy elements
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      const int e = tid + 256 * n, row = e >> 4;
+    for (int n = 0; n < NE; ++n) {
+      const int e = tid + NTHR * n, row = e >> 4;
       const float4 r4 = rr4[n], k4 = kk4[n];
       const float4 gp = *reinterpret_cast<const float4*>(&sm.gs[row * NROW + 4 * c4]);
       const float d1x = gp.x, d1y = gp.y, d1z = gp.z, d1w = gp.w;   // gi - gref
@@ -754,14 +797,6 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
 #pragma unroll
       for (int m = 8; m >= 1; m >>= 1) dg += __shfl_xor_sync(0xffffffffu, dg, m);
       if (c4 == 0) sm.dgs[row] = dg;
-    }
-    // the row of S0 (both lanes of a pair: the lower one for S~0, the upper one for sum_v dS^ S~0) is requested
-    // here and used under MMA batch 1 (requested a phase earlier, the loads held the pass above up instead)
-    float4 srow4[8];
-    {
-      const float* Srow = states + (((size_t)unit * nts + c) * HS + srow) * HS + 32 * hsel;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) srow4[j] = *reinterpret_cast<const float4*>(Srow + 4 * j);
     }
     if (warp == 0 && elect_one() && c > c_lo) {   // bring the previous chunk's rows into L2 while this chunk is in its MMA phases
       tma_prefetch_4d(&tmap_w, 0, tok0 + t0 - L, hi, brow);
@@ -789,41 +824,49 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
       umma_commit(&sm.bar_1);
     }
     // decay factors of state row k = srow (both lanes of a pair work on that row below)
-    const float e0 = ex2(fmaxf(sm.qtot[0][srow] + sm.qtot[1][srow], EXP2_FLOOR));
-    const float dlast = ex2(fmaxf(sm.qtot[2][srow] + sm.qtot[3][srow], EXP2_FLOOR));
+    const float e0 = ex2(fmaxf(half_sum<PARTS>(sm.qtot, 0, srow), EXP2_FLOOR));
+    const float dlast = ex2(fmaxf(half_sum<PARTS>(sm.qtot, 1, srow), EXP2_FLOOR));
     // ---- state rows, while MMA batch 1 runs (it reads neither of the two tiles written here): the upper lane of a
     // pair holds dS and takes sum_v dS^ S~0 (the part of dglast that nothing
     // cancels) and dS^ = e^{glast-gref} dS_L, the lower lane takes S~0 = e^{gref} S0; one split-and-store call
     // serves both
+    ok = mbar_wait(&sm.bar_s, par, status, 418) && ok;
+    float4 srow4[CW / 4];      // the row of S0 (both lanes of a pair: the lower one for S~0, the upper one for sum_v dS^ S~0)
+#pragma unroll
+    for (int j = 0; j < CW / 4; ++j) {
+      const int q = CW / 4 * hsel + j;      // 16-byte piece of the row
+      srow4[j] = *reinterpret_cast<const float4*>(sm.at[q >> 3] + tile_chunk_off(srow, q & 7));
+    }
     {
-      float x[32];
+      float x[CW];
       if (!lower) {
         float acc = 0.f;
 #pragma unroll
-        for (int j = 0; j < 32; j += 4) {
+        for (int j = 0; j < CW; j += 4) {
           const float4 f = srow4[j >> 2];
           acc += dsreg[j] * f.x + dsreg[j + 1] * f.y + dsreg[j + 2] * f.z + dsreg[j + 3] * f.w;
         }
         sm.dgl[hsel][srow] = acc * (e0 * dlast);      // sum_v dS^ S~0 = e^{gref} e^{glast-gref} sum_v dS_L S0
 #pragma unroll
-        for (int j = 0; j < 32; ++j) { dsreg[j] *= dlast; x[j] = dsreg[j]; }     // dsreg now holds dS^
+        for (int j = 0; j < CW; ++j) { dsreg[j] *= dlast; x[j] = dsreg[j]; }     // dsreg now holds dS^
       } else {
 #pragma unroll
-        for (int j = 0; j < 32; j += 4) {
+        for (int j = 0; j < CW; j += 4) {
           const float4 f = srow4[j >> 2];
           x[j] = f.x * e0; x[j + 1] = f.y * e0; x[j + 2] = f.z * e0; x[j + 3] = f.w * e0;
         }
       }
       unsigned char* hi_t = lower ? sm.st[0] : sm.dst[0];
-      store_split_row32(hi_t, hi_t + TILE_BYTES, srow, 32 * hsel, x);
+      store_split_row<CW>(hi_t, hi_t + TILE_BYTES, srow, CW * hsel, x);
     }
     ok = mbar_wait(&sm.bar_1, par, status, 411) && ok;
     tc_fence_after();
+    ok = __syncthreads_and(ok);      // S0 has been read by every thread: A goes over it
     W6C_STAMP(37);
     if (ok) {
       const float dgi = lower ? sm.dgs[srow] : 0.f;     // the diagonal of A carries the u term; dA's does not
       // one call: both lane halves run the same code
-      load_store_masked_row(tm_c0, wq, hsel, lane & 15, dgi, lower ? sm.at[0] : sm.dat[0], srow, true);
+      load_store_masked_row<CW>(tm_c0, wq, hsel, lane & 15, dgi, lower ? sm.at[0] : sm.dat[0], srow, true);
     }
     fence_async_smem();
     tc_fence_before();
@@ -859,20 +902,20 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     }
     ok = mbar_wait(&sm.bar_2a, par, status, 416) && ok;
     tc_fence_after();
-    const int c0 = 32 * hsel;
-    float o[32], rd[32], rs[32];
+    const int c0 = CW * hsel;
+    float o[CW], rd[CW], rs[CW];
     if (ok) {
       // r1: the part of dk~ from inside the chunk (lower halves) / dr~ (upper halves), row of token srow; rx: the
       // state part of dk~ (lower halves only)
-      uint32_t r1[32], rx[32];
-      tmem_ld32(tm_c1, r1);
-      tmem_ld32(tm_c3, rx);
+      uint32_t r1[CW], rx[CW];
+      tmem_ld<CW>(tm_c1, r1);
+      tmem_ld<CW>(tm_c3, rx);
       tmem_ld_wait();
-      float th[32], tl[32];
-      tile_load_row32(lower ? sm.kt[0] : sm.rt[0], srow, c0, th);
-      tile_load_row32(lower ? sm.kt[1] : sm.rt[1], srow, c0, tl);
+      float th[CW], tl[CW];
+      tile_load_row<CW>(lower ? sm.kt[0] : sm.rt[0], srow, c0, th);
+      tile_load_row<CW>(lower ? sm.kt[1] : sm.rt[1], srow, c0, tl);
 #pragma unroll
-      for (int j4 = 0; j4 < 32; j4 += 4) {
+      for (int j4 = 0; j4 < CW; j4 += 4) {
         const int cc = c0 + j4;
         const float4 gs4 = *reinterpret_cast<const float4*>(&sm.gs[srow * NROW + cc]);
         const float4 gg4 = *reinterpret_cast<const float4*>(&sm.gg[srow * NROW + cc]);
@@ -897,7 +940,7 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
       float* so = lower ? stage_dk : stage_dr;
       float* sd = lower ? red_i : sm.red_e;
 #pragma unroll
-      for (int j4 = 0; j4 < 32; j4 += 4) {
+      for (int j4 = 0; j4 < CW; j4 += 4) {
         const int cc = c0 + j4;
         *reinterpret_cast<float4*>(&so[srow * NROW + cc]) = make_float4(o[j4], o[j4 + 1], o[j4 + 2], o[j4 + 3]);
         *reinterpret_cast<float4*>(&sd[srow * NROW + cc]) = make_float4(rd[j4], rd[j4 + 1], rd[j4 + 2], rd[j4 + 3]);
@@ -905,15 +948,15 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
           *reinterpret_cast<float4*>(&red_x[srow * NROW + cc]) = make_float4(rs[j4], rs[j4 + 1], rs[j4 + 2], rs[j4 + 3]);
       }
       // dv row of token srow (lower halves) / dS~0 row k = srow (upper halves)
-      uint32_t r2[32];
-      tmem_ld32(tm_c2, r2);
+      uint32_t r2[CW];
+      tmem_ld<CW>(tm_c2, r2);
       tmem_ld_wait();
       if (!lower) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) dsreg[j] = e0 * (__uint_as_float(r2[j]) + dsreg[j]);   // dS0 = e^{gref}(r~^T dy + dS^)
+        for (int j = 0; j < CW; ++j) dsreg[j] = e0 * (__uint_as_float(r2[j]) + dsreg[j]);   // dS0 = e^{gref}(r~^T dy + dS^)
       } else {
 #pragma unroll
-        for (int j4 = 0; j4 < 32; j4 += 4)
+        for (int j4 = 0; j4 < CW; j4 += 4)
           *reinterpret_cast<float4*>(&stage_dv[srow * NROW + c0 + j4]) =
               make_float4(__uint_as_float(r2[j4]), __uint_as_float(r2[j4 + 1]), __uint_as_float(r2[j4 + 2]),
                           __uint_as_float(r2[j4 + 3]));
@@ -928,29 +971,33 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     // (dglast = sum_v dS_L S_L contains sum_i X_i k~_i; taking the sum over i < j instead of dglast minus the
     // sum over i >= j keeps the two large, nearly equal terms from cancelling.)
     {
-      const int ch = tid & 63, quarter = tid >> 6;
-      float rv[16], px[16];
+      const int ch = tid & 63, part = tid >> 6;
+      float rv[PL], px[PL];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        rv[j] = red_i[(16 * quarter + j) * NROW + ch] + sm.red_e[(16 * quarter + j) * NROW + ch];
-        px[j] = red_x[(16 * quarter + j) * NROW + ch];
+      for (int j = 0; j < PL; ++j) {
+        rv[j] = red_i[(PL * part + j) * NROW + ch] + sm.red_e[(PL * part + j) * NROW + ch];
+        px[j] = red_x[(PL * part + j) * NROW + ch];
       }
       float run = 0.f, prun = 0.f;
 #pragma unroll
-      for (int j = 15; j >= 0; --j) { const float t = rv[j]; rv[j] = run; run += t; }      // sums over i > j
+      for (int j = PL - 1; j >= 0; --j) { const float t = rv[j]; rv[j] = run; run += t; }      // sums over i > j
 #pragma unroll
-      for (int j = 0; j < 16; ++j) { const float t = px[j]; px[j] = prun; prun += t; }      // sums over i < j
-      sm.rqtot[quarter][ch] = run;
-      sm.pqtot[quarter][ch] = prun;
+      for (int j = 0; j < PL; ++j) { const float t = px[j]; px[j] = prun; prun += t; }          // sums over i < j
+      sm.rqtot[part][ch] = run;
+      sm.pqtot[part][ch] = prun;
       __syncthreads();
-      float add = sm.dgl[0][ch] + sm.dgl[1][ch];
-      for (int q2 = quarter + 1; q2 < 4; ++q2) add += sm.rqtot[q2][ch];
-      for (int q2 = 0; q2 < quarter; ++q2) add += sm.pqtot[q2][ch];
+      float add = 0.f;
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const int ii = 16 * quarter + j;
+      for (int q2 = 0; q2 < 64 / CW; ++q2) add += sm.dgl[q2][ch];
+#pragma unroll
+      for (int q2 = 1; q2 < PARTS; ++q2) if (q2 > part) add += sm.rqtot[q2][ch];
+#pragma unroll
+      for (int q2 = 0; q2 < PARTS - 1; ++q2) if (q2 < part) add += sm.pqtot[q2][ch];
+#pragma unroll
+      for (int j = 0; j < PL; ++j) {
+        const int ii = PL * part + j;
         const float dg = (rv[j] + px[j]) + add + red_i[ii * NROW + ch];
-        // stage_dw lies over red_x: this thread has read its 16 entries above and writes the same 16
+        // stage_dw lies over red_x: this thread has read its entries above and writes the same ones
         stage_dw[ii * NROW + ch] = dg * (LN2 * sm.gg[ii * NROW + ch]);      // dw = dg g, g = gg ln 2
       }
     }
@@ -959,8 +1006,8 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     W6C_STAMP(41);
     // ---- outputs, coalesced, plus the u-term parts of dr, dk and du
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      const int e = tid + 256 * n, row = e >> 4, tok = t0 + row;
+    for (int n = 0; n < NE; ++n) {
+      const int e = tid + NTHR * n, row = e >> 4, tok = t0 + row;
       if (tok < Tn) {
         const long long off = base + (long long)tok * tstride + 4 * c4;
         const float4 r4 = rr4[n], k4 = kk4[n];
@@ -990,9 +1037,9 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   const bool hand_on = split && !early_half && mid > 0;
   float* dS_out = hand_on ? handoff : d_s0;
   if (!lower && dS_out && ok) {
-    float* dst = dS_out + (((size_t)unit * HS) + srow) * HS + 32 * hsel;
+    float* dst = dS_out + (((size_t)unit * HS) + srow) * HS + CW * hsel;
 #pragma unroll
-    for (int j = 0; j < 32; j += 4)
+    for (int j = 0; j < CW; j += 4)
       *reinterpret_cast<float4*>(dst + j) = make_float4(dsreg[j], dsreg[j + 1], dsreg[j + 2], dsreg[j + 3]);
   }
   if (hand_on) {
@@ -1049,12 +1096,15 @@ int launch_wkv6_chunked_fwd(const void* r, const void* k, const void* v, const v
     const int grid = parts > 1 ? slots : n_units;
     if (parts > 1 && cuda_ok(cudaMemsetAsync(hflags, 0, ((size_t)n_units + 1) * sizeof(int), st))) return RWKVB200_E_CUDA;
     ProfScope prof("wkv6c_fwd_kernel", st);
-    RWKVB200_DISPATCH_DTYPE(dtype, W6C_DISPATCH_PACKED(
-      if (allow_smem<wkv6c_fwd_kernel<T, P>>(dev, smem)) return RWKVB200_E_CUDA;
-      wkv6c_fwd_kernel<T, P><<<grid, 256, smem, st>>>((const T*)r, (const T*)k, (const T*)v, (const T*)w, u, s0,
-                                                       n_state, smap, (T*)y, sT, states, flags, tm_r, tm_k, tm_v, tm_w,
-                                                       mapT, H, seqs, n_units, parts, handoff, hflags, status,
-                                                       debug_stamp_buffer())));
+    // a unit per SM at most: 512 threads, since nothing else on the SM fills the waits of 256
+#define W6C_LAUNCH_FWD(NTHR)                                                                                          \
+    RWKVB200_DISPATCH_DTYPE(dtype, W6C_DISPATCH_PACKED(                                                               \
+      if (allow_smem<wkv6c_fwd_kernel<T, P, NTHR>>(dev, smem)) return RWKVB200_E_CUDA;                                \
+      wkv6c_fwd_kernel<T, P, NTHR><<<grid, NTHR, smem, st>>>(                                                         \
+          (const T*)r, (const T*)k, (const T*)v, (const T*)w, u, s0, n_state, smap, (T*)y, sT, states, flags, tm_r,   \
+          tm_k, tm_v, tm_w, mapT, H, seqs, n_units, parts, handoff, hflags, status, debug_stamp_buffer())))
+    if (n_units <= sms) W6C_LAUNCH_FWD(512) else W6C_LAUNCH_FWD(256)
+#undef W6C_LAUNCH_FWD
   }
   e = check_launch();
   if (e) return e;
@@ -1150,12 +1200,13 @@ int launch_wkv6_chunked_bwd(const void* r, const void* k, const void* v, const v
   bool split = false;
   {
     const int esz = dtype == RWKVB200_F32 ? 4 : 2;
-    CUtensorMap tm_r, tm_k, tm_v, tm_w, tm_dy;
+    CUtensorMap tm_r, tm_k, tm_v, tm_w, tm_dy, tm_s;
     e = make_row_tensor_map(&tm_r, r, mapB, mapT, H, esz);
     if (!e) e = make_row_tensor_map(&tm_k, k, mapB, mapT, H, esz);
     if (!e) e = make_row_tensor_map(&tm_v, v, mapB, mapT, H, esz);
     if (!e) e = make_row_tensor_map(&tm_w, w, mapB, mapT, H, esz);
     if (!e) e = make_row_tensor_map(&tm_dy, d_y, mapB, mapT, H, esz);
+    if (!e) e = make_state_tensor_map(&tm_s, states, (long long)B * H * seqs.nts * HS);
     if (e) return e;
     // more units than SMs: every unit as two half-length items on one persistent CTA per SM, which evens out
     // the last round (see the kernel); else one CTA per unit
@@ -1167,9 +1218,9 @@ int launch_wkv6_chunked_bwd(const void* r, const void* k, const void* v, const v
     ProfScope prof("wkv6c_bwd_kernel", st);
     RWKVB200_DISPATCH_DTYPE(dtype, W6C_DISPATCH_PACKED(
       if (allow_smem<wkv6c_bwd_kernel<T, P>>(dev, smem)) return RWKVB200_E_CUDA;
-      wkv6c_bwd_kernel<T, P><<<grid, 256, smem, st>>>((const T*)r, (const T*)k, (const T*)v, (const T*)w, u,
+      wkv6c_bwd_kernel<T, P><<<grid, BWD_THREADS, smem, st>>>((const T*)r, (const T*)k, (const T*)v, (const T*)w, u,
                                                        (const T*)d_y, d_sT, states, (T*)dr, (T*)dk, (T*)dv, (T*)dw,
-                                                       du_partial, d_s0, tm_r, tm_k, tm_v, tm_w, tm_dy, mapT, H, seqs,
+                                                       du_partial, d_s0, tm_r, tm_k, tm_v, tm_w, tm_dy, tm_s, mapT, H, seqs,
                                                        n_units, split ? 1 : 0, ws.handoff, ws.hflags, status,
                                                        debug_stamp_buffer())));
   }
