@@ -24,6 +24,8 @@
 // the inputs and outputs touches HBM in the forward pass (plus, for the backward, the fp32 state at every
 // chunk boundary).  The raw rows of the next chunk arrive by TMA while the current chunk is worked on.
 // Tile and TMEM conventions are those of tc.cuh.
+#include <type_traits>
+
 #include "common.cuh"
 #include "tc.cuh"
 
@@ -59,13 +61,14 @@ __device__ __forceinline__ void split_pair(float x0, float x1, uint32_t& hi, uin
   lo = pack_bf16(x0 - bf16_lo(hi), x1 - bf16_hi(hi));
 }
 // write 4 consecutive values (columns col .. col+3, col a multiple of 4) of `row` into a hi and a lo tile
+template <bool LO = true>
 __device__ __forceinline__ void store_split4(unsigned char* hi_t, unsigned char* lo_t, int row, int col, float4 x) {
   uint2 h, l;
   split_pair(x.x, x.y, h.x, l.x);
   split_pair(x.z, x.w, h.y, l.y);
   const uint32_t off = tile_off(row, col);
   *reinterpret_cast<uint2*>(hi_t + off) = h;
-  *reinterpret_cast<uint2*>(lo_t + off) = l;
+  if constexpr (LO) *reinterpret_cast<uint2*>(lo_t + off) = l;
 }
 // write CW consecutive fp32 values of `row` (columns col0 .., col0 a multiple of 8) into a hi and a lo tile
 template <int CW>
@@ -113,13 +116,16 @@ __device__ __forceinline__ float from_middle(const float (*tot)[64], int part, i
   return add;
 }
 
-// D (+)= X Y with X = xh + xl, Y = yh + yl (lo tile = hi tile + TILE_BYTES): hi*hi + hi*lo + lo*hi
-template <int M, int N, int A_MN, int B_MN>
+// D (+)= X Y with X = xh + xl, Y = yh + yl (lo tile = hi tile + TILE_BYTES): hi*hi + hi*lo + lo*hi.  A_LO / B_LO = false: that
+// operand's lo tile would be zero (v and dy of bfloat16 tokens) and is neither written nor multiplied.
+template <int M, int N, int A_MN, int B_MN, bool A_LO = true, bool B_LO = true>
 __device__ __forceinline__ void umma_split(uint32_t tmem_d, uint32_t a_hi, uint32_t b_hi, bool accumulate) {
   umma_tile<M, N, A_MN, B_MN>(tmem_d, a_hi, b_hi, accumulate);
-  umma_tile<M, N, A_MN, B_MN>(tmem_d, a_hi, b_hi + TILE_BYTES, true);
-  umma_tile<M, N, A_MN, B_MN>(tmem_d, a_hi + TILE_BYTES, b_hi, true);
+  if constexpr (B_LO) umma_tile<M, N, A_MN, B_MN>(tmem_d, a_hi, b_hi + TILE_BYTES, true);
+  if constexpr (A_LO) umma_tile<M, N, A_MN, B_MN>(tmem_d, a_hi + TILE_BYTES, b_hi, true);
 }
+// whether token values have a lo part
+template <typename T> constexpr bool has_lo() { return !std::is_same<T, __nv_bfloat16>::value; }
 
 // Row `lr` (0..15) of a warp's 16 x CW block of a 64 x 64 product that is kept strictly below the diagonal, the
 // diagonal itself set to `diag`, split and stored.  Where the diagonal crosses the block depends on the warp alone:
@@ -349,7 +355,7 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
                         -LOG2E * ex2(LOG2E * gw[n].w));
       gw[n] = f;
       *reinterpret_cast<float4*>(&sm.gs[row * NROW + 4 * c4]) = f;
-      store_split4(sm.vt[0], sm.vt[1], row, 4 * c4, vv4[n]);
+      store_split4<has_lo<T>()>(sm.vt[0], sm.vt[1], row, 4 * c4, vv4[n]);
     }
     __syncthreads();
     W6C_STAMP(1);
@@ -428,7 +434,7 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
       tc_fence_after();
       if (warp == 0)      umma_split<64, 64, 0, 0>(tmem_addr(tm, 0, 0), smem_u32(sm.rt[0]), smem_u32(sm.kt[0]), false);
       else if (warp == 1) umma_split<64, 64, 0, 1>(tmem_addr(tm, 0, 64), smem_u32(sm.rt[0]), smem_u32(sm.st[0]), false);
-      else                umma_split<64, 64, 1, 1>(tmem_addr(tm, 16, 64), smem_u32(sm.kt[0]), smem_u32(sm.vt[0]), false);
+      else                umma_split<64, 64, 1, 1, true, has_lo<T>()>(tmem_addr(tm, 16, 64), smem_u32(sm.kt[0]), smem_u32(sm.vt[0]), false);
       umma_commit(&sm.bar_1);
     }
     ok = mbar_wait(&sm.bar_1, par, status, 401) && ok;
@@ -454,7 +460,7 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     // ---- batch 2: y += A v
     if (warp == 0 && elect_one() && ok) {
       tc_fence_after();
-      umma_split<64, 64, 0, 1>(tmem_addr(tm, 0, 64), smem_u32(sm.at[0]), smem_u32(sm.vt[0]), true);
+      umma_split<64, 64, 0, 1, true, has_lo<T>()>(tmem_addr(tm, 0, 64), smem_u32(sm.at[0]), smem_u32(sm.vt[0]), true);
       umma_commit(&sm.bar_2);
     }
     // the state of the next chunk's start, stored here because the next proxy fence, which waits for global stores too, is
@@ -727,7 +733,7 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
         *reinterpret_cast<float4*>(&sm.gg[row * NROW + 4 * c4]) = f;
         float4 y4 = load4_shared(raw_dy + row * 64 + 4 * c4);
         if (PACKED && tok >= Tn) y4 = make_float4(0.f, 0.f, 0.f, 0.f);      // the next sequence's row
-        store_split4(sm.dyt[0], sm.dyt[1], row, 4 * c4, y4);
+        store_split4<has_lo<T>()>(sm.dyt[0], sm.dyt[1], row, 4 * c4, y4);
       }
     }
     __syncthreads();
@@ -774,7 +780,7 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
       if (PACKED && t0 + row >= Tn) {
         v4 = make_float4(0.f, 0.f, 0.f, 0.f); y4 = v4; rr4[n] = v4; kk4[n] = v4;
       }
-      store_split4(sm.vt[0], sm.vt[1], row, 4 * c4, v4);
+      store_split4<has_lo<T>()>(sm.vt[0], sm.vt[1], row, 4 * c4, v4);
       float dd = v4.x * y4.x + v4.y * y4.y + v4.z * y4.z + v4.w * y4.w;
 #pragma unroll
       for (int m = 8; m >= 1; m >>= 1) dd += __shfl_xor_sync(0xffffffffu, dd, m);
@@ -820,7 +826,7 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     }
     if (warp == 1 && elect_one()) {
       tc_fence_after();
-      umma_split<64, 64, 0, 0>(tmem_addr(tm, 16, 0), smem_u32(sm.dyt[0]), smem_u32(sm.vt[0]), false);
+      umma_split<64, 64, 0, 0, has_lo<T>(), has_lo<T>()>(tmem_addr(tm, 16, 0), smem_u32(sm.dyt[0]), smem_u32(sm.vt[0]), false);
       umma_commit(&sm.bar_1);
     }
     // decay factors of state row k = srow (both lanes of a pair work on that row below)
@@ -879,11 +885,11 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     if (warp == 0 && elect_one() && ok) {
       tc_fence_after();
       // dr~ = dy S~0^T + stril(dA) k~               (upper halves, columns 64..127)
-      umma_split<64, 64, 0, 0>(tmem_addr(tm, 16, 64), smem_u32(sm.dyt[0]), smem_u32(sm.st[0]), false);
+      umma_split<64, 64, 0, 0, has_lo<T>(), true>(tmem_addr(tm, 16, 64), smem_u32(sm.dyt[0]), smem_u32(sm.st[0]), false);
       umma_split<64, 64, 0, 1>(tmem_addr(tm, 16, 64), smem_u32(sm.dat[0]), smem_u32(sm.kt[0]), true);
       umma_commit(&sm.bar_2a);
       // dv = A^T dy + k~ dS^                        (lower halves, columns 128..191)
-      umma_split<64, 64, 1, 1>(tmem_addr(tm, 0, 128), smem_u32(sm.at[0]), smem_u32(sm.dyt[0]), false);
+      umma_split<64, 64, 1, 1, true, has_lo<T>()>(tmem_addr(tm, 0, 128), smem_u32(sm.at[0]), smem_u32(sm.dyt[0]), false);
       umma_split<64, 64, 0, 1>(tmem_addr(tm, 0, 128), smem_u32(sm.kt[0]), smem_u32(sm.dst[0]), true);
       umma_commit(&sm.bar_2);
     }
@@ -894,10 +900,10 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
       umma_split<64, 64, 1, 1>(tmem_addr(tm, 0, 64), smem_u32(sm.dat[0]), smem_u32(sm.rt[0]), false);
       // its state part X = v dS^^T apart (lower halves, columns 192..255): the decay gradient takes the two
       // parts of dk~ k~ in different sums
-      umma_split<64, 64, 0, 0>(tmem_addr(tm, 0, 192), smem_u32(sm.vt[0]), smem_u32(sm.dst[0]), false);
+      umma_split<64, 64, 0, 0, has_lo<T>(), true>(tmem_addr(tm, 0, 192), smem_u32(sm.vt[0]), smem_u32(sm.dst[0]), false);
       umma_commit(&sm.bar_2a);
       // dS~0 = r~^T dy                              (upper halves, columns 128..191)
-      umma_split<64, 64, 1, 1>(tmem_addr(tm, 16, 128), smem_u32(sm.rt[0]), smem_u32(sm.dyt[0]), false);
+      umma_split<64, 64, 1, 1, true, has_lo<T>()>(tmem_addr(tm, 16, 128), smem_u32(sm.rt[0]), smem_u32(sm.dyt[0]), false);
       umma_commit(&sm.bar_2);
     }
     ok = mbar_wait(&sm.bar_2a, par, status, 416) && ok;
