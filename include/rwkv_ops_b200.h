@@ -67,6 +67,9 @@ enum {
    * forward call left there, so skip the recomputation.  Without the flag the backward recomputes the
    * forward from the inputs, as the reference does (rwkv_ops/rwkv7_kernel/torch_op.py:163-183). */
   RWKVB200_ALGO_KEEP = 0x100,
+  /* Flag, OR-ed into the algo of rwkvb200_wkv6_fwd (not with KEEP): u, s0 and sT hold the token dtype instead of
+   * float32 (the arithmetic is float32 either way), which saves a caller with such states their conversions. */
+  RWKVB200_ALGO_TOKEN_STATES = 0x200,
   /* Flags, OR-ed into algo (chunked path of rwkvb200_rwkv7_fwd / _bwd only): run part of the call.  None set
    * = the whole call.  The parts of one call must run in order on the same workspace with the same
    * arguments.  Forward: PREPARE does everything that does not depend on the initial state (h0, o and ht

@@ -94,7 +94,9 @@ def _register_fakes():
     def _(r, k, v, w, u, s0, state_map, algo, keep):
         B, T, C = r.shape
         H, N = u.shape
-        return torch.empty_like(r), state(r, B, H, N), kept(r, _lib.wkv6_kept_bytes(B, T, H) if keep else 0)
+        sT = state(r, B, H, N)
+        return (torch.empty_like(r), sT.to(r.dtype) if algo & _lib.ALGO_TOKEN_STATES else sT,
+                kept(r, _lib.wkv6_kept_bytes(B, T, H) if keep else 0))
 
     @fake("rwkv_ops_b200::wkv6_bwd")
     def _(r, k, v, w, u, s0, state_map, d_y, d_sT, k_, algo):

@@ -312,6 +312,8 @@ int rwkvb200_wkv6_fwd(const void* r, const void* k, const void* v, const void* w
   if (n_state > 1 && !state_map && n_state != B) return RWKVB200_E_STATE_MAP;
   const void* ps[] = {r, k, v, w, u, s0, y, sT};
   for (const void* p : ps) if (p && !aligned16(p)) return RWKVB200_E_ALIGN;
+  const bool typed = (algo & RWKVB200_ALGO_TOKEN_STATES) != 0;
+  if (typed && (algo & RWKVB200_ALGO_KEEP)) return RWKVB200_E_UNSUPPORTED;
   if (resolve_w6_algo(algo, head_size) == RWKVB200_ALGO_CHUNKED) {
     if (!workspace || !aligned16(workspace) ||
         workspace_bytes < rwkvb200_wkv6_fwd_workspace_bytes(B, T, H, head_size, dtype, algo))
@@ -327,10 +329,10 @@ int rwkvb200_wkv6_fwd(const void* r, const void* k, const void* v, const void* w
       wkv6_chunked_fwd_scratch(workspace, B, H, &flags, &handoff, &hflags);
     }
     return launch_wkv6_chunked_fwd(r, k, v, w, u, n_state ? s0 : nullptr, n_state, state_map, y, sT, states, flags,
-                                   handoff, hflags, B, T, H, dtype, (cudaStream_t)stream);
+                                   handoff, hflags, B, T, H, dtype, (cudaStream_t)stream, nullptr, nullptr, 0, typed);
   }
   return launch_wkv6_fwd(r, k, v, w, u, n_state ? s0 : nullptr, n_state, state_map, y, sT, nullptr,
-                         B, T, H, dtype, (cudaStream_t)stream, nullptr, 0, head_size);
+                         B, T, H, dtype, (cudaStream_t)stream, nullptr, 0, head_size, typed);
 }
 
 size_t rwkvb200_wkv6_bwd_workspace_bytes(int B, int T, int H, int head_size, int dtype, int algo) {

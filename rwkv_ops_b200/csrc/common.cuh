@@ -84,6 +84,14 @@ template <> __device__ __forceinline__ void store4<__half>(__half* p, float4 f) 
   *reinterpret_cast<uint2*>(p) = u;
 }
 
+// Four consecutive elements of an array that holds T (`typed`) or float32.
+template <typename T> __device__ __forceinline__ float4 load4_as(const void* p, long long i, bool typed) {
+  return typed ? load4(static_cast<const T*>(p) + i) : load4(static_cast<const float*>(p) + i);
+}
+template <typename T> __device__ __forceinline__ void store4_as(void* p, long long i, bool typed, float4 f) {
+  if (typed) store4(static_cast<T*>(p) + i, f); else store4(static_cast<float*>(p) + i, f);
+}
+
 // The decay every operator applies to its w input.
 __device__ __forceinline__ float decay_of(float w) { return expf(-expf(w)); }
 
@@ -187,7 +195,7 @@ constexpr int R7_CKPT = 8;   // tokens between state checkpoints of the recurren
 int launch_wkv6_fwd(const void* r, const void* k, const void* v, const void* w, const float* u,
                     const float* s0, int n_state, const int32_t* smap, void* y, float* sT,
                     float* ckpt, int B, int Tn, int H, int dtype, cudaStream_t st, const UnitSel* sel = nullptr,
-                    int ckpt_every = 0, int head_size = HS);
+                    int ckpt_every = 0, int head_size = HS, bool typed = false);
 int launch_wkv6_bwd_coarse(const void* r, const void* k, const void* v, const void* w, const float* u,
                            const void* d_y, const float* d_sT, const float* ckpt,
                            void* dr, void* dk, void* dv, void* dw, float* du_partial, float* d_s0,
@@ -200,13 +208,14 @@ int launch_wkv6_bwd(const void* r, const void* k, const void* v, const void* w, 
                     int B, int Tn, int H, int dtype, cudaStream_t st, int head_size = HS);
 constexpr int W6_CKPT = 8;
 
+// `typed`: u, s0 and sT hold the token dtype instead of float32.
 // Chunked tcgen05 wkv6 (wkv6_chunked.cu).  `states` (may be NULL) receives the fp32 state at every chunk
 // boundary, [B*H][ceil(T/64)+1][64][64].
 int launch_wkv6_chunked_fwd(const void* r, const void* k, const void* v, const void* w, const float* u,
                             const float* s0, int n_state, const int32_t* smap, void* y, float* sT,
                             float* states, int* flags, float* handoff, int* hflags, int B, int Tn, int H, int dtype,
                             cudaStream_t st, const int32_t* seq_start = nullptr, const int32_t* seq_len = nullptr,
-                            int T_total = 0);
+                            int T_total = 0, bool typed = false);
 size_t wkv6_chunked_fwd_scratch_bytes(int B, int H);
 void wkv6_chunked_fwd_scratch(void* workspace, int B, int H, int** flags, float** handoff, int** hflags);
 void wkv6_chunked_workspace_parts(void* workspace, int B, int Tn, int H, int** flags, float** handoff, int** hflags);

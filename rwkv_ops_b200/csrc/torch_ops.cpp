@@ -465,7 +465,7 @@ Three wkv6_fwd(const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& 
   const c10::cuda::CUDAGuard guard(r.device());
   const int B = (int)r.size(0), T = (int)r.size(1), H = (int)u.size(0), N = (int)u.size(1);
   const int code = dtype_code(r.scalar_type()), flags = (int)algo | (keep ? RWKVB200_ALGO_KEEP : 0);
-  Tensor y = fresh_like(r), sT = fresh({B, H, N, N}, at::kFloat, r);
+  Tensor y = fresh_like(r), sT = fresh({B, H, N, N}, algo & RWKVB200_ALGO_TOKEN_STATES ? r.scalar_type() : at::kFloat, r);
   // a training forward of the chunked path leaves the chunk-boundary states for the backward
   const size_t nws = rwkvb200_wkv6_fwd_workspace_bytes(B, T, H, N, code, flags);
   Tensor ws = bytes(nws, r);
@@ -535,7 +535,7 @@ struct Wkv6Args {
   OptTensor s0, map;
 };
 Wkv6Args wkv6_args(const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& u, int64_t N,
-                   int64_t rows, const OptTensor& init_state, const OptTensor& state_map) {
+                   int64_t rows, const OptTensor& init_state, const OptTensor& state_map, bool typed = false) {
   check_tokens(r, {&k, &v, &w}, 3);
   const int64_t C = r.size(2), H = C / N;
   const at::ScalarType dt = r.scalar_type(), t = compute_dtype(dt);
@@ -555,12 +555,13 @@ Wkv6Args wkv6_args(const Tensor& r, const Tensor& k, const Tensor& v, const Tens
       TORCH_CHECK_VALUE(s.size(0) == 1 || s.size(0) == rows,
                         "state_map cannot be inferred from init_state; pass it explicitly");
     }
-    x.s0 = s.to(at::kFloat).contiguous();
+    x.s0 = typed ? s.contiguous() : s.to(at::kFloat).contiguous();
   } else {
     TORCH_CHECK_VALUE(!has(state_map), "state_map needs init_state");
   }
   x.r = dense(r, t); x.k = dense(k, t); x.v = dense(v, t); x.w = dense(w, t);
-  x.u = u.reshape({H, N}).to(at::kFloat).contiguous();
+  x.u = u.reshape({H, N});
+  x.u = typed ? x.u.contiguous() : x.u.to(at::kFloat).contiguous();
   return x;
 }
 // the dtype of the states an operator hands to its caller
@@ -570,7 +571,11 @@ std::tuple<Tensor, Tensor> wkv6(const Tensor& r, const Tensor& k, const Tensor& 
                                 int64_t head_size, const OptTensor& init_state, const OptTensor& state_map,
                                 bool with_state) {
   TORCH_CHECK_VALUE(r.dim() == 3, "expected [B, T, C] tensors, got ", r.sizes());
-  const Wkv6Args x = wkv6_args(r, k, v, w, u, head_size, r.size(0), init_state, state_map);
+  // bfloat16 states outside training are read and written as they are: each conversion would be a launch of its own
+  const bool typed = r.scalar_type() == at::kBFloat16 && u.scalar_type() == at::kBFloat16 &&
+                     (!has(init_state) || init_state->scalar_type() == at::kBFloat16) &&
+                     !any_requires_grad({&r, &k, &v, &w, &u}, init_state);
+  const Wkv6Args x = wkv6_args(r, k, v, w, u, head_size, r.size(0), init_state, state_map, typed);
   int algo = algo_from_env("RWKV_OPS_B200_WKV6_ALGO");
   if (head_size != HEAD) {
     TORCH_CHECK_VALUE(algo != RWKVB200_ALGO_CHUNKED, "the chunked wkv6 path is built for head size 64");
@@ -578,6 +583,7 @@ std::tuple<Tensor, Tensor> wkv6(const Tensor& r, const Tensor& k, const Tensor& 
   }
   const bool keep = algo != RWKVB200_ALGO_RECURRENT && r.size(1) > 1 &&
                     any_requires_grad({&x.r, &x.k, &x.v, &x.w, &x.u}, x.s0);
+  if (typed) algo |= RWKVB200_ALGO_TOKEN_STATES;
   auto [y, sT, kept] = RWKV_OP(wkv6_fwd, "wkv6_fwd", x.r, x.k, x.v, x.w, x.u, x.s0, x.map, algo, keep);
   return {y.to(r.scalar_type()), with_state ? sT.to(state_dtype(r.scalar_type())) : sT};
 }

@@ -57,10 +57,10 @@ __device__ __forceinline__ float sum_kq(float x) {
 template <typename T, int N>
 __global__ void __launch_bounds__(N)
 wkv6_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __restrict__ v,
-                const T* __restrict__ w, const float* __restrict__ u,
-                const float* __restrict__ s0, int n_state, const int32_t* __restrict__ smap,
-                T* __restrict__ yout, float* __restrict__ sT, float* __restrict__ ckpt, int ckpt_every,
-                int Tn_dense, int H, UnitSel sel) {
+                const T* __restrict__ w, const void* __restrict__ u,
+                const void* __restrict__ s0, int n_state, const int32_t* __restrict__ smap,
+                T* __restrict__ yout, void* __restrict__ sT, float* __restrict__ ckpt, int ckpt_every,
+                int Tn_dense, int H, UnitSel sel, int typed) {
   constexpr int NKQ = N / VS, QUADS = N / 4;
   __shared__ __align__(16) float tile[TL][4][NP<N>()];   // r, d, k, r*u*k
   __shared__ __align__(16) float vt[TL][VS];
@@ -77,13 +77,14 @@ wkv6_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __res
   const long long tstride = (long long)H * N;
   const long long ckpt_unit = sel.ckpt_unit_stride ? sel.ckpt_unit_stride
                                                    : (long long)((Tn_dense + ckpt_every - 1) / ckpt_every) * N * N;
-  const float4 u4 = *reinterpret_cast<const float4*>(u + hi * N + 4 * (tid % QUADS));
+  const float4 u4 = load4_as<T>(u, hi * N + 4 * (tid % QUADS), typed);
 
   float S[16];
   if (s0 && n_state > 0) {
-    const float* p = s0 + ((state_row(smap, n_state, bi) * H + hi) * N + 16 * kq) * N + y * VS + vl;
+    const long long p = ((state_row(smap, n_state, bi) * H + hi) * N + 16 * kq) * N + y * VS + vl;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) S[j] = p[j * N];
+    for (int j = 0; j < 16; ++j)
+      S[j] = typed ? to_f32(static_cast<const T*>(s0)[p + j * N]) : static_cast<const float*>(s0)[p + j * N];
   } else {
 #pragma unroll
     for (int j = 0; j < 16; ++j) S[j] = 0.f;
@@ -171,9 +172,12 @@ wkv6_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __res
     }
   }
   if (sT) {
-    float* p = sT + (((long long)unit * N) + 16 * kq) * N + y * VS + vl;
+    const long long p = (((long long)unit * N) + 16 * kq) * N + y * VS + vl;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) p[j * N] = S[j];
+    for (int j = 0; j < 16; ++j) {
+      if (typed) static_cast<T*>(sT)[p + j * N] = from_f32<T>(S[j]);
+      else       static_cast<float*>(sT)[p + j * N] = S[j];
+    }
   }
 }
 
@@ -473,14 +477,15 @@ wkv6_du_reduce_mixed_kernel(const float* __restrict__ part_chunked, const float*
 int launch_wkv6_fwd(const void* r, const void* k, const void* v, const void* w, const float* u,
                     const float* s0, int n_state, const int32_t* smap, void* y, float* sT,
                     float* ckpt, int B, int Tn, int H, int dtype, cudaStream_t st, const UnitSel* sel_,
-                    int ckpt_every, int head_size) {
+                    int ckpt_every, int head_size, bool typed) {
   const UnitSel sel = sel_ ? *sel_ : UnitSel{nullptr, nullptr, nullptr, 0};
   ProfScope prof("wkv6_fwd_kernel", st);
   RWKVB200_DISPATCH_HEAD6(head_size,
     dim3 grid(B * H, N / VS);
     RWKVB200_DISPATCH_DTYPE(dtype,
       wkv6_fwd_kernel<T, N><<<grid, N, 0, st>>>((const T*)r, (const T*)k, (const T*)v, (const T*)w, u, s0, n_state,
-                                                smap, (T*)y, sT, ckpt, ckpt_every ? ckpt_every : CK, Tn, H, sel)));
+                                                smap, (T*)y, sT, ckpt, ckpt_every ? ckpt_every : CK, Tn, H, sel,
+                                                typed)));
   return check_launch();
 }
 

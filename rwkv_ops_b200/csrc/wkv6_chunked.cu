@@ -204,8 +204,8 @@ struct FwdSmem {
 template <typename T, bool PACKED, int NTHR>
 __global__ void __launch_bounds__(NTHR, 512 / NTHR)
 wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ w,
-                 const float* __restrict__ u, const float* __restrict__ s0, int n_state,
-                 const int32_t* __restrict__ smap, T* __restrict__ y, float* __restrict__ sT,
+                 const void* __restrict__ u, const void* __restrict__ s0, int n_state,
+                 const int32_t* __restrict__ smap, T* __restrict__ y, void* __restrict__ sT, int typed,
                  float* __restrict__ states, int* __restrict__ flags, const __grid_constant__ CUtensorMap tmap_r,
                  const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                  const __grid_constant__ CUtensorMap tmap_w, int Tn_dense, int H, Seqs seqs, int n_units, int parts,
@@ -276,7 +276,7 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   const bool last_part = part == parts - 1;
   // (a stretch without a chunk, in a sequence shorter than `parts` chunks, just passes the state on)
   // per-thread slice of u (4 channels) for the diagonal term
-  const float4 u4 = *reinterpret_cast<const float4*>(u + hi * HS + 4 * c4);
+  const float4 u4 = load4_as<T>(u, hi * HS + 4 * c4, typed);
 
   // ---- state at the item's first chunk: rows k on the upper lane halves, this warp's 32 columns
   float sreg[CW];
@@ -305,10 +305,10 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
       }
     }
   } else if (!tok_lane && s0 && n_state > 0) {
-    const float* S = s0 + ((state_row(smap, n_state, bi) * H + hi) * HS + srow) * HS + CW * hsel;
+    const long long S = ((state_row(smap, n_state, bi) * H + hi) * HS + srow) * HS + CW * hsel;
 #pragma unroll
     for (int j = 0; j < CW; j += 4) {
-      const float4 fv = *reinterpret_cast<const float4*>(S + j);
+      const float4 fv = load4_as<T>(s0, S + j, typed);
       sreg[j] = fv.x; sreg[j + 1] = fv.y; sreg[j + 2] = fv.z; sreg[j + 3] = fv.w;
     }
   }
@@ -502,10 +502,10 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   if (!tok_lane && ok) {
     if (last_part) {
       if (sT) {
-        float* dst = sT + (((size_t)unit * HS) + srow) * HS + CW * hsel;
+        const long long dst = (((long long)unit * HS) + srow) * HS + CW * hsel;
 #pragma unroll
         for (int j = 0; j < CW; j += 4)
-          *reinterpret_cast<float4*>(dst + j) = make_float4(sreg[j], sreg[j + 1], sreg[j + 2], sreg[j + 3]);
+          store4_as<T>(sT, dst + j, typed, make_float4(sreg[j], sreg[j + 1], sreg[j + 2], sreg[j + 3]));
       }
     } else {
       float* dst = handoff + (((size_t)unit * HS) + srow) * HS + CW * hsel;
@@ -1066,7 +1066,7 @@ int launch_wkv6_chunked_fwd(const void* r, const void* k, const void* v, const v
                             const float* s0, int n_state, const int32_t* smap, void* y, float* sT,
                             float* states, int* flags, float* handoff, int* hflags, int B, int Tn, int H,
                             int dtype, cudaStream_t st, const int32_t* seq_start, const int32_t* seq_len,
-                            int T_total) {
+                            int T_total, bool typed) {
   using namespace w6c;
   // a packed batch: B sequences (the longest of Tn tokens) end to end in one row of T_total tokens
   const bool packed = seq_start != nullptr;
@@ -1107,8 +1107,8 @@ int launch_wkv6_chunked_fwd(const void* r, const void* k, const void* v, const v
     RWKVB200_DISPATCH_DTYPE(dtype, W6C_DISPATCH_PACKED(                                                               \
       if (allow_smem<wkv6c_fwd_kernel<T, P, NTHR>>(dev, smem)) return RWKVB200_E_CUDA;                                \
       wkv6c_fwd_kernel<T, P, NTHR><<<grid, NTHR, smem, st>>>(                                                         \
-          (const T*)r, (const T*)k, (const T*)v, (const T*)w, u, s0, n_state, smap, (T*)y, sT, states, flags, tm_r,   \
-          tm_k, tm_v, tm_w, mapT, H, seqs, n_units, parts, handoff, hflags, status, debug_stamp_buffer())))
+          (const T*)r, (const T*)k, (const T*)v, (const T*)w, u, s0, n_state, smap, (T*)y, sT, typed, states, flags,   \
+          tm_r, tm_k, tm_v, tm_w, mapT, H, seqs, n_units, parts, handoff, hflags, status, debug_stamp_buffer())))
     if (n_units <= sms) W6C_LAUNCH_FWD(512) else W6C_LAUNCH_FWD(256)
 #undef W6C_LAUNCH_FWD
   }
@@ -1117,7 +1117,7 @@ int launch_wkv6_chunked_fwd(const void* r, const void* k, const void* v, const v
   // the marked units again, exactly: outputs, final state and (for the backward) the chunk-boundary states
   const long long unit_floats = (long long)seqs.nts * HS * HS;
   const UnitSel sel{flags, seq_start, seq_len, states ? unit_floats : 0};
-  return launch_wkv6_fwd(r, k, v, w, u, s0, n_state, smap, y, sT, states, B, Tn, H, dtype, st, &sel, L);
+  return launch_wkv6_fwd(r, k, v, w, u, s0, n_state, smap, y, sT, states, B, Tn, H, dtype, st, &sel, L, HS, typed);
 }
 
 }  // namespace rwkvb200
