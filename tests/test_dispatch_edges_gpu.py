@@ -1,0 +1,63 @@
+"""The kernels a call is dispatched to by its size and types, at the edges of their blocks: the scans for few and for
+many sequences, the float32 recurrence over blocks of tokens, and wkv6 with few units or bfloat16 states."""
+import pytest
+import torch
+
+import rwkv_ops_b200 as ro
+from oracle import generalized_delta_rule as oracle_gdr
+from rwkv_ops_b200.workloads import rwkv7_inputs, wkv6_inputs, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+def _train(d, grads, fn=ro.generalized_delta_rule):
+    g = {n: d[n].clone().requires_grad_(True) for n in "rwkvab"}
+    h0 = d["initial_state"].clone().requires_grad_(True)
+    o, s = fn(*[g[n] for n in "rwkvab"], initial_state=h0)
+    torch.autograd.backward([o, s], grads)
+    return {"o": o.detach(), "s": s.detach(), "dh0": h0.grad, **{f"d{n}": g[n].grad for n in "rwkvab"}}
+
+
+# one to six chunks: the chunk counts at which the accumulators and the operand buffers of the scans wrap around
+@pytest.mark.parametrize("T", [8, 64, 65, 129, 200, 257, 384])
+def test_scans_for_few_and_many_sequences(T):
+    """Two units on their own (one CTA per SM) and among more units than there are SMs (two CTAs per SM)."""
+    d = {n: t.cuda() for n, t in rwkv7_inputs(1, T, 2, dtype=torch.bfloat16, seed=70 + T, with_state=True, with_grads=True).items()}
+    few = _train(d, [d["d_out"], d["d_state"]])
+    ref = _train({n: t.float().cpu() for n, t in d.items()}, [d["d_out"].float().cpu(), d["d_state"].float().cpu()], oracle_gdr)
+    for n in ref:
+        assert rel_l2(few[n], ref[n]) < 2e-2, n
+    B = torch.cuda.get_device_properties(0).multi_processor_count // 2 + 4
+    big = {n: t.expand(B, *t.shape[1:]).contiguous() for n, t in d.items()}
+    many = _train(big, [big["d_out"], big["d_state"]])
+    for n in few:
+        for row in (0, B - 1):
+            assert rel_l2(many[n][row], few[n][0]) < 2e-3, n
+
+
+@pytest.mark.parametrize("T", [1, 2, 7, 8, 9, 15, 16, 17, 33, 48])
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.float16, 2e-3)])
+def test_token_blocks(T, dtype, tol):
+    """Blocks of 8 tokens in the sweeps, items of 16 in the gradient kernel."""
+    d = rwkv7_inputs(2, T, 3, dtype=dtype, seed=40 + T, with_state=True, with_grads=True)
+    ref = _train({n: t.double() for n, t in d.items()}, [d["d_out"].double(), d["d_state"].double()], oracle_gdr)
+    out = _train({n: t.cuda() for n, t in d.items()}, [d["d_out"].cuda(), d["d_state"].cuda()])
+    for n in ref:
+        assert rel_l2(out[n], ref[n]) < tol, n
+
+
+@pytest.mark.parametrize("T", [1, 9, 64, 65, 200])
+@pytest.mark.parametrize("many", [False, True])
+def test_wkv6_states_in_the_token_dtype(T, many):
+    """bfloat16 u, state table and final state, read and written as they are, against the call that converts them."""
+    H = 2
+    B = torch.cuda.get_device_properties(0).multi_processor_count // H + 4 if many else 2
+    d = {n: t.cuda() for n, t in wkv6_inputs(B, T, H, dtype=torch.bfloat16, seed=20 + T, n_state=3).items()}
+    s0, u = d["init_state"].bfloat16(), d["u"].bfloat16()
+    smap = torch.arange(B, device="cuda", dtype=torch.int32) % 3
+    op = ro.RWKV6_OP(64, T)
+    with torch.no_grad():
+        y, s = op(d["r"], d["k"], d["v"], d["w"], u, with_state=True, init_state=s0, state_map=smap)
+        y32, s32 = op(d["r"], d["k"], d["v"], d["w"], u.float(), with_state=True, init_state=s0.float(), state_map=smap)
+    assert y.dtype == s.dtype == torch.bfloat16
+    assert torch.equal(y, y32) and torch.equal(s, s32.to(torch.bfloat16))
