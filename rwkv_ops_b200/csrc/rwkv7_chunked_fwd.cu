@@ -28,9 +28,8 @@ struct IntraSmem {
   unsigned char v[TILE_BYTES];                      // raw a, then v
   unsigned char ainv[TILE_BYTES];                   // later holds B2
   unsigned char y[TILE_BYTES];                      // A_ak v
-  float gs[L * NROW];                               // e^{gi-gref}; later the diagonal blocks of A_ab
+  float gs[L * NROW];                               // gi - gref; before that the raw b tile, later the inverse's blocks
   float qtot[4][64];                                // sums of g over the four quarters of the chunk
-  float efirst[64];                                 // e^{-gref}
   uint64_t bar_v, bar_w, bar_in, bar_b, bar_m1, bar_m2, bar_m3, bar_m4, bar_m5;
   uint32_t tmem_base;
 };
@@ -130,8 +129,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
     R7C_STAMP(0);
     if (next < n_ch && warp == 1 && elect_one()) prefetch_rows(nxt);
     // ---- phase A: decay prefix sums (in units of log 2), thread = (channel, quarter of the chunk), straight from the
-    // raw w tile.  What everybody needs of them is e^{gi-gref}: its reciprocal is the factor of k~ and b~, and the row
-    // before gives the factor of a~.
+    // raw w tile.
     ok = mbar_wait(&sm.bar_b, par, status, 208) && ok;
     uint4 rb[2];      // this thread's 2 x 16 bytes (8 channels of one token) of the raw b tile, which lies where the factors will
 #pragma unroll
@@ -149,8 +147,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
       for (int j = 0; j < 16; ++j) {
         float w = __uint_as_float((uint32_t)*reinterpret_cast<const unsigned short*>(sm.aqk + tile_off(16 * quarter + j, c)) << 16);
         if constexpr (FUSED) w = round_bf16(W_SCALE * sigmoidf_(w));      // the tile holds p: w = -e^{-1/2} sigmoid(p), as bfloat16
-        const float e = ex2(LOG2E * w);
-        if (j < n_rows) run -= LOG2E * e;
+        run += j < n_rows ? __fmul_rn(-LOG2E, ex2(LOG2E * w)) : 0.f;      // (rounded as in the scaling below)
         gi[j] = run;
       }
       sm.qtot[quarter][c] = run;
@@ -159,10 +156,9 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
       // gi - gref: the prefix inside the half; the reference point is the end of the first half
       const float add = quarter == 0 ? -(run + sm.qtot[1][c]) : quarter == 1 ? -run : quarter == 3 ? sm.qtot[2][c] : 0.f;
 #pragma unroll
-      for (int j = 0; j < 16; ++j) sm.gs[(16 * quarter + j) * NROW + c] = ex2(gi[j] + add);
+      for (int j = 0; j < 16; ++j) sm.gs[(16 * quarter + j) * NROW + c] = gi[j] + add;
       if (quarter == 0) {
         const float tot0 = -add, tot1 = sm.qtot[2][c] + sm.qtot[3][c];
-        sm.efirst[c] = ex2(add);                                                     // for the exclusive prefix of the first token
         ws_aux[(size_t)ch * AUX_FLOATS + c] = ex2(fmaxf(tot0, EXP2_FLOOR));          // e^{gref}
         // a half-chunk decay sum beyond the limit: the unit is recomputed by the float32 recurrence.  The mark is the
         // factor's sign; the scan, which reads every factor of its unit anyway, gathers it into Workspace::flags.
@@ -211,12 +207,11 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
         const int e = tid + 256 * n, row = e >> 3, cc = e & 7;
-        float eq[8], ea[8];      // e^{gi-gref} of the row; e^{ge-gref}: of the row before it
-        const float* before = row ? &sm.gs[(row - 1) * NROW + 8 * cc] : &sm.efirst[8 * cc];
-        *reinterpret_cast<float4*>(eq) = *reinterpret_cast<const float4*>(&sm.gs[row * NROW + 8 * cc]);
-        *reinterpret_cast<float4*>(eq + 4) = *reinterpret_cast<const float4*>(&sm.gs[row * NROW + 8 * cc + 4]);
-        *reinterpret_cast<float4*>(ea) = *reinterpret_cast<const float4*>(before);
-        *reinterpret_cast<float4*>(ea + 4) = *reinterpret_cast<const float4*>(before + 4);
+        float gl[8];      // gi - gref
+        *reinterpret_cast<float4*>(gl) = *reinterpret_cast<const float4*>(&sm.gs[row * NROW + 8 * cc]);
+        *reinterpret_cast<float4*>(gl + 4) = *reinterpret_cast<const float4*>(&sm.gs[row * NROW + 8 * cc + 4]);
+        const uint4 rw = *reinterpret_cast<const uint4*>(sm.aqk + tile_chunk_off(row, cc));
+        const uint32_t uw[4] = {rw.x, rw.y, rw.z, rw.w};
         const uint32_t uq[4] = {rq[n].x, rq[n].y, rq[n].z, rq[n].w};
         const uint32_t uk[4] = {rk[n].x, rk[n].y, rk[n].z, rk[n].w};
         const uint32_t ua[4] = {ra[n].x, ra[n].y, ra[n].z, ra[n].w};
@@ -224,11 +219,19 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
         uint32_t oq[4], ok_[4], oa[4], ob[4];
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
-          const float ek0 = rcp(eq[2 * m]), ek1 = rcp(eq[2 * m + 1]);
-          oq[m] = pack_bf16(bf16_lo(uq[m]) * eq[2 * m], bf16_hi(uq[m]) * eq[2 * m + 1]);
-          ok_[m] = pack_bf16(bf16_lo(uk[m]) * ek0, bf16_hi(uk[m]) * ek1);
-          oa[m] = pack_bf16(bf16_lo(ua[m]) * ea[2 * m], bf16_hi(ua[m]) * ea[2 * m + 1]);
-          ob[m] = pack_bf16(bf16_lo(ub[m]) * ek0, bf16_hi(ub[m]) * ek1);
+          float eq[2], ek[2], ea[2];
+#pragma unroll
+          for (int hh = 0; hh < 2; ++hh) {
+            const float d1 = gl[2 * m + hh];
+            float w = hh ? bf16_hi(uw[m]) : bf16_lo(uw[m]);
+            if constexpr (FUSED) w = round_bf16(W_SCALE * sigmoidf_(w));
+            const float g = t0 + row < Tn ? __fmul_rn(-LOG2E, ex2(LOG2E * w)) : 0.f;
+            eq[hh] = ex2(d1); ek[hh] = ex2(-d1); ea[hh] = ex2(d1 - g);
+          }
+          oq[m] = pack_bf16(bf16_lo(uq[m]) * eq[0], bf16_hi(uq[m]) * eq[1]);
+          ok_[m] = pack_bf16(bf16_lo(uk[m]) * ek[0], bf16_hi(uk[m]) * ek[1]);
+          oa[m] = pack_bf16(bf16_lo(ua[m]) * ea[0], bf16_hi(ua[m]) * ea[1]);
+          ob[m] = pack_bf16(bf16_lo(ub[m]) * ek[0], bf16_hi(ub[m]) * ek[1]);
         }
         const uint32_t off = tile_chunk_off(row, cc);
         *reinterpret_cast<uint4*>(sm.qt + off) = make_uint4(oq[0], oq[1], oq[2], oq[3]);
@@ -326,16 +329,20 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
         bulk_wait_read();                  // q~, k~, b~, A_qk (and the tiles kept for the backward) have left shared memory
         if (next < n_ch) { load_w(nxt); load_qka(nxt); }      // nothing reads A_qk, q~, k~, v any more
       }
-    } else if (ok) {     // warps 6, 7: the diagonal 32 x 32 blocks of A_ab, inverted at once (fp32); warp 7 also N_BA
+    } else if (ok) {     // warps 6, 7: the diagonal 32 x 32 blocks of A_ab, inverted (fp32); warp 7 also N_BA
       // Ainv = X = (I - N)^-1, N = stril(A_ab); with A = rows 0..31, B = rows 32..63 its blocks are X_A = (I - N_AA)^-1,
-      // X_B = (I - N_BB)^-1 and X_BA = X_B N_BA X_A.
-      float* nd = sm.gs + 1024 * ihalf;       // this warp's 32 x 32 block transposed: nd[32 r + i] = N[i][r]
+      // X_B = (I - N_BB)^-1 and X_BA = X_B N_BA X_A.  A 32 x 32 block is inverted by its 16 x 16 blocks: D_0, D_1 by
+      // substitution, one column per lane, side by side, then X_10 = D_1 (N_10 D_0), half a column per lane.
+      constexpr int ND = 36;                            // padded row
+      float* nd = sm.gs + 1408 * ihalf;                 // this warp's block, one row per lane
+      float* P = nd + 32 * ND;
       uint32_t rr[32];
       float x[32];
       tmem_ld32(tmem_addr(tm, 32 * wq, 64 + 32 * ihalf), rr);
       tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 32; ++j) nd[32 * j + lane] = __uint_as_float(rr[j]);      // (at or above the diagonal: never used)
+      for (int j = 0; j < 32; j += 4)      // (entries at or right of the diagonal are never used)
+        *reinterpret_cast<uint4*>(&nd[ND * lane + j]) = make_uint4(rr[j], rr[j + 1], rr[j + 2], rr[j + 3]);
       if (ihalf) {
         tmem_ld32(tmem_addr(tm, 32 * wq, 64), rr);
         tmem_ld_wait();
@@ -348,30 +355,67 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
         tile_store_row32(sm.ainv, lane, 32, x);           // the upper right block of X
       }
       __syncwarp();
-      // Column `lane` of (I - N)^-1.  Once x[r] is known its products with column r of N go into all later rows, two per
-      // instruction and independent of one another, so that the chain from row to row is one multiply-add (summing up
-      // a row at a time instead, 85 cycles per row).  The next column is on its way from shared memory.
-      float4 nc[2][8];
+      const int bl = lane >> 4, cl = lane & 15;
+      float xb[16];
 #pragma unroll
-      for (int m = 0; m < 8; ++m) nc[0][m] = *reinterpret_cast<const float4*>(&nd[4 * m]);
+      for (int i = 0; i < 16; ++i) xb[i] = (i == cl) ? 1.f : 0.f;
 #pragma unroll
-      for (int r = 0; r < 32; ++r) x[r] = r == lane ? 1.f : 0.f;
+      for (int i = 1; i < 16; ++i) {
+        const float* nrow = &nd[(16 * bl + i) * ND + 16 * bl];
+        float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f;
 #pragma unroll
-      for (int r = 0; r < 31; ++r) {
-        if (r < 30) {
-#pragma unroll
-          for (int m = (r + 2) / 4; m < 8; ++m) nc[(r + 1) & 1][m] = *reinterpret_cast<const float4*>(&nd[32 * (r + 1) + 4 * m]);
+        for (int jj = 0; jj < (i + 3) / 4; ++jj) {
+          const float4 n = *reinterpret_cast<const float4*>(nrow + 4 * jj);
+          p0 += n.x * xb[4 * jj];
+          if (4 * jj + 1 < i) p1 += n.y * xb[4 * jj + 1];
+          if (4 * jj + 2 < i) p2 += n.z * xb[4 * jj + 2];
+          if (4 * jj + 3 < i) p3 += n.w * xb[4 * jj + 3];
         }
-        const float* n = reinterpret_cast<const float*>(nc[r & 1]);
-        if ((r & 1) == 0) x[r + 1] += n[r + 1] * x[r];
+        xb[i] += (p0 + p1) + (p2 + p3);
+      }
+      __syncwarp();
+      auto put = [&](int row, int col, float f) {
+        *reinterpret_cast<bf16*>(sm.ainv + tile_off(32 * ihalf + row, 32 * ihalf + col)) = __float2bfloat16_rn(f);
+      };
 #pragma unroll
-        for (int i = (r + 2) & ~1; i < 32; i += 2) fma2(x[i], x[i + 1], n[i], n[i + 1], x[r], x[r], x[i], x[i + 1]);
+      for (int i = 0; i < 16; ++i) {
+        nd[(16 * bl + i) * ND + 16 * bl + cl] = xb[i];
+        put(16 * bl + i, 16 * bl + cl, xb[i]);
+      }
+      if (lane < 16) {      // the upper right 16 x 16 block
+        *reinterpret_cast<uint4*>(sm.ainv + tile_chunk_off(32 * ihalf + lane, 4 * ihalf + 2)) = make_uint4(0u, 0u, 0u, 0u);
+        *reinterpret_cast<uint4*>(sm.ainv + tile_chunk_off(32 * ihalf + lane, 4 * ihalf + 3)) = make_uint4(0u, 0u, 0u, 0u);
+      }
+      __syncwarp();
+      float col[16], acc[8];
+#pragma unroll
+      for (int kk = 0; kk < 16; ++kk) col[kk] = nd[kk * ND + cl];      // D_0[:, cl]
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const float* nrow = &nd[(16 + 8 * bl + q) * ND];               // N_10
+        float s_ = 0.f;
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) {
+          const float4 n = *reinterpret_cast<const float4*>(nrow + 4 * jj);
+          s_ += n.x * col[4 * jj] + n.y * col[4 * jj + 1] + n.z * col[4 * jj + 2] + n.w * col[4 * jj + 3];
+        }
+        acc[q] = s_;
       }
 #pragma unroll
-      for (int r = 0; r < 32; r += 2) {
-        const uint32_t u = pack_bf16(x[r], x[r + 1]);
-        *reinterpret_cast<unsigned short*>(sm.ainv + tile_off(32 * ihalf + r, 32 * ihalf + lane)) = (unsigned short)u;
-        *reinterpret_cast<unsigned short*>(sm.ainv + tile_off(32 * ihalf + r + 1, 32 * ihalf + lane)) = (unsigned short)(u >> 16);
+      for (int q = 0; q < 8; ++q) P[(8 * bl + q) * 16 + cl] = acc[q];
+      __syncwarp();
+#pragma unroll
+      for (int kk = 0; kk < 16; ++kk) col[kk] = P[kk * 16 + cl];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const float* drow = &nd[(16 + 8 * bl + q) * ND + 16];          // D_1 in full (zeros above its diagonal)
+        float s_ = 0.f;
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) {
+          const float4 n = *reinterpret_cast<const float4*>(drow + 4 * jj);
+          s_ += n.x * col[4 * jj] + n.y * col[4 * jj + 1] + n.z * col[4 * jj + 2] + n.w * col[4 * jj + 3];
+        }
+        put(16 + 8 * bl + q, cl, s_);
       }
     }
     fence_async_smem();
@@ -492,9 +536,8 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
 // lane window take 32 of the 64 columns each (hsel = w>>2).  Lanes 0-15 of a warp own state rows, lanes 16-31 token rows.
 // ---------------------------------------------------------------------------------------------
 // For more sequences than SMs: two CTAs (two sequences) share an SM, and memory bounds it (eight tiles in, four out per
-// chunk).  The state stays in registers (fp32) and takes its update from an accumulator that starts at zero, so k~^T v and
-// A_qk v need no state; the output rows of a chunk are read out with sa of the next one; copies are waited for a phase
-// after they were issued.
+// chunk).  The products of a chunk accumulate onto its state (fp32, in TMEM); the output rows of a chunk are read out with
+// sa of the next one; copies are waited for a phase after they were issued.
 // Operand tiles come in two groups, each requested again once the MMAs that read it have completed.  U, which is only
 // added row by row, does not enter shared memory: every thread fetches its row into registers at the top of a chunk.
 struct ScanGroup1 {         // free once W h~0 and q~ h~0 have been computed
@@ -597,6 +640,13 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
     tile_store_row32(sm.ht[0], row, c0, h);
   }
   bool ok = true;
+  {
+    uint32_t rh[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) rh[j] = __float_as_uint(h[j]);
+    tmem_st32(tmem_addr(tm, 32 * wq, 64 + c0), rh);
+    tmem_st_wait();
+  }
   fence_async_smem();
   tc_fence_before();
   ok = __syncthreads_and(ok);
@@ -617,7 +667,7 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
       if (ok) {
         tc_fence_after();
         umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 0), smem_u32(sm.g1.w), smem_u32(sm.ht[p]), false);
-        umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, acc), smem_u32(sm.g1.kt), smem_u32(sm.g1.v), false);
+        umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, acc), smem_u32(sm.g1.kt), smem_u32(sm.g1.v), true);      // onto h~0
         umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, acc), smem_u32(sm.g1.aqk), smem_u32(sm.g1.v), false);
         umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, acc), smem_u32(sm.g1.qt), smem_u32(sm.ht[p]), true);
         umma_commit(&sm.bar_a);
@@ -713,7 +763,7 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
       tmem_ld_wait();
       if (state_lane) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) h[j] += __uint_as_float(r[j]);
+        for (int j = 0; j < 32; ++j) h[j] = __uint_as_float(r[j]);
         if (bwd_tiles) {
 #pragma unroll
           for (int q = 0; q < 4; ++q)
@@ -723,9 +773,11 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
         marked |= scale < 0.f;
         const float sc = fabsf(scale);
 #pragma unroll
-        for (int j = 0; j < 32; ++j) h[j] = (h[j] * sc) * scale_next;
+        for (int j = 0; j < 32; ++j) { h[j] = (h[j] * sc) * scale_next; r[j] = __float_as_uint(h[j]); }
         if (!last) tile_store_row32(sm.ht[p ^ 1], row, c0, h);
       }
+      tmem_st32(tmem_addr(tm, 32 * wq, 64 + 64 * (p ^ 1) + c0), r);      // (the upper lane halves there have been read)
+      tmem_st_wait();
     }
     // the copies out of sa, h~0, X and of the output rows have left their tiles: the next chunk rewrites them
     if ((warp == st_warp || warp == out_warp) && elect_one()) bulk_wait_read();
@@ -844,7 +896,7 @@ r7c_scan_fwd_alone_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsi
   __syncthreads();
   tc_fence_after();
   // TMEM: columns 0..63 lower lane halves = W h~0; three accumulators in turn: lower halves k~^T v + b~^T sa, upper halves
-  // the output rows, which are read out while the next chunk's is in use and the one after it is being started
+  // the output rows, which are read out while the next chunk is worked on and the state of the one after it is stored
   const uint32_t tm = sm.tmem_base;
   auto acc_col = [](int c) { return 64u + 64u * (uint32_t)(c % 3); };
   bool ok = true;
@@ -886,6 +938,14 @@ r7c_scan_fwd_alone_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsi
       }
       store_row(sm.ht[0], h);
     }
+    auto put_h = [&](int c) {      // the state at the start of chunk c into its accumulator, whose upper lane halves are free
+      uint32_t rh[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) rh[j] = __float_as_uint(h[j]);
+      tmem_st32(tm_w + acc_col(c), rh);
+      tmem_st_wait();
+    };
+    put_h(0);
     arrive(&sm.bar_h);
     for (int c = 0; c < NT; ++c) {
       const int p = c & 1;
@@ -931,7 +991,7 @@ r7c_scan_fwd_alone_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsi
         tmem_ld_wait();
         uint4 xp[4];
 #pragma unroll
-        for (int j = 0; j < 32; ++j) h[j] += __uint_as_float(r[j]);
+        for (int j = 0; j < 32; ++j) h[j] = __uint_as_float(r[j]);
 #pragma unroll
         for (int q = 0; q < 4; ++q)
           xp[q] = make_uint4(pack_bf16(h[8 * q], h[8 * q + 1]), pack_bf16(h[8 * q + 2], h[8 * q + 3]),
@@ -941,6 +1001,7 @@ r7c_scan_fwd_alone_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsi
 #pragma unroll
         for (int j = 0; j < 32; ++j) h[j] = (h[j] * sc) * scale_next;
         if (state_lane) store_row(sm.ht[p ^ 1], h);
+        put_h(c + 1);
         arrive(&sm.bar_h);
         if (state_lane && bwd_tiles) {
 #pragma unroll
@@ -952,23 +1013,17 @@ r7c_scan_fwd_alone_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsi
     ok = ok && wait(&sm.bar_o, NT - 1, 217);
   } else if (warp == 8) {      // ---- MMAs
     if (elect_one()) {
-      auto ahead = [&](int c) {      // the two products of a chunk that need neither the state nor sa
-        auto& g = sm.g1[c & 1];
-        if (!mbar_wait(&sm.bar_g1[c & 1], (c >> 1) & 1, status, 211)) return false;
-        umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, acc_col(c)), smem_u32(g.kt), smem_u32(g.v), false);      // k~^T v
-        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, acc_col(c)), smem_u32(g.aqk), smem_u32(g.v), false);    // A_qk v
-        return true;
-      };
-      ok = ahead(0);
       for (int c = 0; c < NT && ok; ++c) {
         const uint32_t acc = acc_col(c);
         auto& g1 = sm.g1[c & 1];
         auto& g2 = sm.g2[c & 1];
-        ok = mbar_wait(&sm.bar_h, c & 1, status, 219);
+        ok = mbar_wait(&sm.bar_g1[c & 1], (c >> 1) & 1, status, 211) && mbar_wait(&sm.bar_h, c & 1, status, 219);
         if (!ok) break;
         tc_fence_after();
         umma_tile<64, 64, 0, 1>(tmem_addr(tm, 0, 0), smem_u32(g1.w), smem_u32(sm.ht[c & 1]), false);        // W h~0
         umma_commit(&sm.bar_a);
+        umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, acc), smem_u32(g1.kt), smem_u32(g1.v), true);              // h~0 + k~^T v
+        umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, acc), smem_u32(g1.aqk), smem_u32(g1.v), false);           // A_qk v
         ok = mbar_wait(&sm.bar_g2[c & 1], (c >> 1) & 1, status, 214) && mbar_wait(&sm.bar_s, c & 1, status, 220);
         if (!ok) break;
         tc_fence_after();
@@ -977,7 +1032,6 @@ r7c_scan_fwd_alone_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsi
         umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, acc), smem_u32(g2.qt), smem_u32(sm.ht[c & 1]), true);     // += q~ h~0
         umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, acc), smem_u32(g2.aqb), smem_u32(sm.sa[c & 1]), true);    // += A_qb sa
         umma_commit(&sm.bar_o);
-        if (c + 1 < NT) ok = ahead(c + 1);
       }
     }
     __syncwarp();
