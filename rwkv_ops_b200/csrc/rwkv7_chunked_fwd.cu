@@ -145,8 +145,12 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
       const int n_rows = Tn - t0 - 16 * quarter;      // rows of this quarter inside the sequence
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
-        float w = __uint_as_float((uint32_t)*reinterpret_cast<const unsigned short*>(sm.aqk + tile_off(16 * quarter + j, c)) << 16);
-        if constexpr (FUSED) w = round_bf16(W_SCALE * sigmoidf_(w));      // the tile holds p: w = -e^{-1/2} sigmoid(p), as bfloat16
+        unsigned short* raw = reinterpret_cast<unsigned short*>(sm.aqk + tile_off(16 * quarter + j, c));
+        float w = __uint_as_float((uint32_t)*raw << 16);
+        if constexpr (FUSED) {      // the tile holds p: w = -e^{-1/2} sigmoid(p), as bfloat16, goes back for the scaling
+          w = round_bf16(W_SCALE * sigmoidf_(w));
+          *raw = (unsigned short)(__float_as_uint(w) >> 16);
+        }
         run += j < n_rows ? __fmul_rn(-LOG2E, ex2(LOG2E * w)) : 0.f;      // (rounded as in the scaling below)
         gi[j] = run;
       }
@@ -223,8 +227,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {
             const float d1 = gl[2 * m + hh];
-            float w = hh ? bf16_hi(uw[m]) : bf16_lo(uw[m]);
-            if constexpr (FUSED) w = round_bf16(W_SCALE * sigmoidf_(w));
+            const float w = hh ? bf16_hi(uw[m]) : bf16_lo(uw[m]);
             const float g = t0 + row < Tn ? __fmul_rn(-LOG2E, ex2(LOG2E * w)) : 0.f;
             eq[hh] = ex2(d1); ek[hh] = ex2(-d1); ea[hh] = ex2(d1 - g);
           }
@@ -308,6 +311,19 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
         }
         bulk_commit();
       }
+      if (warp == 3 && ok) {      // Q: N_BA in rows 32..63 (its other rows and columns are not used)
+        uint32_t rr[32];
+        tmem_ld32(tmem_addr(tm, 32 * wq, 64), rr);
+        tmem_ld_wait();
+        float x[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
+        tile_store_row32(sm.cm, 32 + lane, 0, x);
+      }
+      if (warp == 1) {            // the upper right block of X
+        const float x[32] = {};
+        tile_store_row32(sm.ainv, lane, 32, x);
+      }
       ok = mbar_wait(&sm.bar_m2, par, status, 203) && ok;
       tc_fence_after();
       if (ok) {      // Y rows; warps 2, 3 take both column halves of theirs
@@ -333,89 +349,85 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
       // Ainv = X = (I - N)^-1, N = stril(A_ab); with A = rows 0..31, B = rows 32..63 its blocks are X_A = (I - N_AA)^-1,
       // X_B = (I - N_BB)^-1 and X_BA = X_B N_BA X_A.  A 32 x 32 block is inverted by its 16 x 16 blocks: D_0, D_1 by
       // substitution, one column per lane, side by side, then X_10 = D_1 (N_10 D_0), half a column per lane.
-      constexpr int ND = 36;                            // padded row
-      float* nd = sm.gs + 1408 * ihalf;                 // this warp's block, one row per lane
-      float* P = nd + 32 * ND;
+      float* nd = sm.gs + 1024 * ihalf;                 // this warp's block transposed: nd[32 j + i] = N[i][j]; later D_1
       uint32_t rr[32];
-      float x[32];
       tmem_ld32(tmem_addr(tm, 32 * wq, 64 + 32 * ihalf), rr);
       tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 32; j += 4)      // (entries at or right of the diagonal are never used)
-        *reinterpret_cast<uint4*>(&nd[ND * lane + j]) = make_uint4(rr[j], rr[j + 1], rr[j + 2], rr[j + 3]);
-      if (ihalf) {
-        tmem_ld32(tmem_addr(tm, 32 * wq, 64), rr);
-        tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < 32; ++j) x[j] = __uint_as_float(rr[j]);
-        tile_store_row32(sm.cm, 32 + lane, 0, x);         // Q: N_BA in rows 32..63 (its other rows and columns are not used)
-      } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) x[j] = 0.f;
-        tile_store_row32(sm.ainv, lane, 32, x);           // the upper right block of X
-      }
+      for (int j = 0; j < 32; ++j) nd[32 * j + lane] = __uint_as_float(rr[j]);      // (at or above the diagonal: never used)
       __syncwarp();
       const int bl = lane >> 4, cl = lane & 15;
-      float xb[16];
+      // Once x[j] is known its products with column j of N go into all later rows, two rows per instruction and
+      // independent of one another; a row collects them in four partial sums, by j mod 4.  The next column is on its way.
+      float xb[16], p[4][16];
+      {
+        const float* nb = nd + (32 + 1) * 16 * bl;      // column j of the block: nb + 32 j
+        float4 nc[2][4];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) xb[i] = (i == cl) ? 1.f : 0.f;
+        for (int m = 0; m < 4; ++m) nc[0][m] = *reinterpret_cast<const float4*>(nb + 4 * m);
 #pragma unroll
-      for (int i = 1; i < 16; ++i) {
-        const float* nrow = &nd[(16 * bl + i) * ND + 16 * bl];
-        float p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f;
-#pragma unroll
-        for (int jj = 0; jj < (i + 3) / 4; ++jj) {
-          const float4 n = *reinterpret_cast<const float4*>(nrow + 4 * jj);
-          p0 += n.x * xb[4 * jj];
-          if (4 * jj + 1 < i) p1 += n.y * xb[4 * jj + 1];
-          if (4 * jj + 2 < i) p2 += n.z * xb[4 * jj + 2];
-          if (4 * jj + 3 < i) p3 += n.w * xb[4 * jj + 3];
+        for (int i = 0; i < 16; ++i) {
+          p[0][i] = p[1][i] = p[2][i] = p[3][i] = 0.f;
+          xb[i] = i == cl ? 1.f : 0.f;
         }
-        xb[i] += (p0 + p1) + (p2 + p3);
+#pragma unroll
+        for (int j = 0; j < 15; ++j) {
+          if (j < 14) {
+#pragma unroll
+            for (int m = (j + 2) / 4; m < 4; ++m) nc[(j + 1) & 1][m] = *reinterpret_cast<const float4*>(nb + 32 * (j + 1) + 4 * m);
+          }
+          const float* n = reinterpret_cast<const float*>(nc[j & 1]);
+          float* q = p[j & 3];
+          if ((j & 1) == 0) q[j + 1] = __fmaf_rn(n[j + 1], xb[j], q[j + 1]);
+#pragma unroll
+          for (int i = (j + 2) & ~1; i < 16; i += 2) fma2(q[i], q[i + 1], n[i], n[i + 1], xb[j], xb[j], q[i], q[i + 1]);
+          xb[j + 1] += (p[0][j + 1] + p[1][j + 1]) + (p[2][j + 1] + p[3][j + 1]);
+        }
       }
-      __syncwarp();
-      auto put = [&](int row, int col, float f) {
-        *reinterpret_cast<bf16*>(sm.ainv + tile_off(32 * ihalf + row, 32 * ihalf + col)) = __float2bfloat16_rn(f);
+      // P = N_10 D_0 and X_10 = D_1 P, rows 8 bl .. 8 bl + 7 of column cl; in groups of four terms
+      float col[16], acc[8];
+      auto product = [&](const float* m, int ld) {      // acc[q] = sum_k m[ld k + q] col[k]
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) {
+          float t[8];
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk) {
+            float n[8];
+            *reinterpret_cast<float4*>(n) = *reinterpret_cast<const float4*>(m + ld * (4 * jj + kk));
+            *reinterpret_cast<float4*>(n + 4) = *reinterpret_cast<const float4*>(m + ld * (4 * jj + kk) + 4);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) t[q] = kk ? __fmaf_rn(n[q], col[4 * jj + kk], t[q]) : __fmul_rn(n[q], col[4 * jj]);
+          }
+#pragma unroll
+          for (int q = 0; q < 8; ++q) acc[q] = jj ? __fadd_rn(acc[q], t[q]) : t[q];
+        }
       };
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        nd[(16 * bl + i) * ND + 16 * bl + cl] = xb[i];
-        put(16 * bl + i, 16 * bl + cl, xb[i]);
+      for (int kk = 0; kk < 16; ++kk) col[kk] = __shfl_sync(0xffffffffu, xb[kk], cl);      // D_0[:, cl]
+      product(nd + 16 + 8 * bl, 32);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const float other = __shfl_xor_sync(0xffffffffu, acc[q], 16);
+        col[q] = bl ? other : acc[q];
+        col[8 + q] = bl ? acc[q] : other;
       }
+      __syncwarp();
+      if (bl) {
+#pragma unroll
+        for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4*>(&nd[16 * cl + i]) = make_float4(xb[i], xb[i + 1], xb[i + 2], xb[i + 3]);
+      }
+      __syncwarp();
+      product(nd + 8 * bl, 16);
+      auto put = [&](int row, int c, float f) {
+        *reinterpret_cast<bf16*>(sm.ainv + tile_off(32 * ihalf + row, 32 * ihalf + c)) = __float2bfloat16_rn(f);
+      };
+#pragma unroll
+      for (int i = 0; i < 16; ++i) put(16 * bl + i, 16 * bl + cl, xb[i]);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) put(16 + 8 * bl + q, cl, acc[q]);
       if (lane < 16) {      // the upper right 16 x 16 block
         *reinterpret_cast<uint4*>(sm.ainv + tile_chunk_off(32 * ihalf + lane, 4 * ihalf + 2)) = make_uint4(0u, 0u, 0u, 0u);
         *reinterpret_cast<uint4*>(sm.ainv + tile_chunk_off(32 * ihalf + lane, 4 * ihalf + 3)) = make_uint4(0u, 0u, 0u, 0u);
-      }
-      __syncwarp();
-      float col[16], acc[8];
-#pragma unroll
-      for (int kk = 0; kk < 16; ++kk) col[kk] = nd[kk * ND + cl];      // D_0[:, cl]
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const float* nrow = &nd[(16 + 8 * bl + q) * ND];               // N_10
-        float s_ = 0.f;
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-          const float4 n = *reinterpret_cast<const float4*>(nrow + 4 * jj);
-          s_ += n.x * col[4 * jj] + n.y * col[4 * jj + 1] + n.z * col[4 * jj + 2] + n.w * col[4 * jj + 3];
-        }
-        acc[q] = s_;
-      }
-#pragma unroll
-      for (int q = 0; q < 8; ++q) P[(8 * bl + q) * 16 + cl] = acc[q];
-      __syncwarp();
-#pragma unroll
-      for (int kk = 0; kk < 16; ++kk) col[kk] = P[kk * 16 + cl];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const float* drow = &nd[(16 + 8 * bl + q) * ND + 16];          // D_1 in full (zeros above its diagonal)
-        float s_ = 0.f;
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-          const float4 n = *reinterpret_cast<const float4*>(drow + 4 * jj);
-          s_ += n.x * col[4 * jj] + n.y * col[4 * jj + 1] + n.z * col[4 * jj + 2] + n.w * col[4 * jj + 3];
-        }
-        put(16 + 8 * bl + q, cl, s_);
       }
     }
     fence_async_smem();
