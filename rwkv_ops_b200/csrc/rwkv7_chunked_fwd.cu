@@ -357,31 +357,34 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
       for (int j = 0; j < 32; ++j) nd[32 * j + lane] = __uint_as_float(rr[j]);      // (at or above the diagonal: never used)
       __syncwarp();
       const int bl = lane >> 4, cl = lane & 15;
-      // Once x[j] is known its products with column j of N go into all later rows, two rows per instruction and
-      // independent of one another; a row collects them in four partial sums, by j mod 4.  The next column is on its way.
-      float xb[16], p[4][16];
-      {
-        const float* nb = nd + (32 + 1) * 16 * bl;      // column j of the block: nb + 32 j
-        float4 nc[2][4];
+      // Once x[j] is known its products with column j of N go into all later rows (of the first, then of the second eight:
+      // registers), two rows per instruction and independent of one another; a row collects them in four partial sums, by
+      // j mod 4.  The next column is on its way.
+      float xb[16];
 #pragma unroll
-        for (int m = 0; m < 4; ++m) nc[0][m] = *reinterpret_cast<const float4*>(nb + 4 * m);
+      for (int i = 0; i < 16; ++i) xb[i] = i == cl ? 1.f : 0.f;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          p[0][i] = p[1][i] = p[2][i] = p[3][i] = 0.f;
-          xb[i] = i == cl ? 1.f : 0.f;
-        }
+      for (int h8 = 0; h8 < 16; h8 += 8) {
+        const float* nb = nd + (32 + 1) * 16 * bl + h8;      // rows h8 .. h8 + 7 of column j of the block: nb + 32 j
+        float p[4][8];
+        float4 nc[2][2];
+        nc[0][0] = *reinterpret_cast<const float4*>(nb);
+        nc[0][1] = *reinterpret_cast<const float4*>(nb + 4);
 #pragma unroll
-        for (int j = 0; j < 15; ++j) {
-          if (j < 14) {
+        for (int i = 0; i < 8; ++i) p[0][i] = p[1][i] = p[2][i] = p[3][i] = 0.f;
 #pragma unroll
-            for (int m = (j + 2) / 4; m < 4; ++m) nc[(j + 1) & 1][m] = *reinterpret_cast<const float4*>(nb + 32 * (j + 1) + 4 * m);
+        for (int j = 0; j < h8 + 7; ++j) {
+          if (j + 1 < h8 + 7) {
+            nc[(j + 1) & 1][0] = *reinterpret_cast<const float4*>(nb + 32 * (j + 1));
+            nc[(j + 1) & 1][1] = *reinterpret_cast<const float4*>(nb + 32 * (j + 1) + 4);
           }
           const float* n = reinterpret_cast<const float*>(nc[j & 1]);
           float* q = p[j & 3];
-          if ((j & 1) == 0) q[j + 1] = __fmaf_rn(n[j + 1], xb[j], q[j + 1]);
+          const int first = j + 1 > h8 ? j + 1 - h8 : 0;      // rows after j
+          if (first & 1) q[first] = __fmaf_rn(n[first], xb[j], q[first]);
 #pragma unroll
-          for (int i = (j + 2) & ~1; i < 16; i += 2) fma2(q[i], q[i + 1], n[i], n[i + 1], xb[j], xb[j], q[i], q[i + 1]);
-          xb[j + 1] += (p[0][j + 1] + p[1][j + 1]) + (p[2][j + 1] + p[3][j + 1]);
+          for (int i = (first + 1) & ~1; i < 8; i += 2) fma2(q[i], q[i + 1], n[i], n[i + 1], xb[j], xb[j], q[i], q[i + 1]);
+          if (j + 1 >= h8) xb[j + 1] += (p[0][j + 1 - h8] + p[1][j + 1 - h8]) + (p[2][j + 1 - h8] + p[3][j + 1 - h8]);
         }
       }
       // P = N_10 D_0 and X_10 = D_1 P, rows 8 bl .. 8 bl + 7 of column cl; in groups of four terms
