@@ -39,7 +39,9 @@ struct IntraSmem {
 // the columns (hsel = w>>2); warps 6 and 7 invert the diagonal blocks of A_ab while the other warps mask the rest of
 // MMA 1, issue MMA 2 and drain it.
 // What bounds it: 17 tiles per chunk-head through memory (348 us at B 8, T 4096, 32 heads) if two CTAs per SM can
-// overlap their chains of phases well enough (503 us with 15.3 k cycles per chunk-head; 414 us with 13.3 k now).
+// overlap their chains of phases well enough: 503 us before the inverse went to two warps and the raw tiles were requested
+// early, 475 us now.  The backward takes the difference of large sums over the tiles made here: a change of their arithmetic in
+// the last bit shows in dw (a 32 x 32 substitution and reciprocals for e^{gref-gi} gave 412 us and were taken back).
 template <bool PACKED, bool FUSED>
 __global__ void __launch_bounds__(256, 2)
 r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, const bf16* __restrict__ k,

@@ -19,7 +19,8 @@
 // operand X is split as X = hi + lo (two bf16 tiles) and every product is the three tensor-core
 // products hi*hi + hi*lo + lo*hi accumulated in fp32 TMEM (relative error ~2^-16 per term).
 //
-// One CTA of 256 threads per (batch, head) walks the chunks in order; the fp32 state (its gradient in the
+// One CTA of 256 threads per (batch, head) (512 in the forward when there is at most one unit per SM: 64.5 -> 60 us for
+// 4 prompts of 777 tokens, 32 heads, bfloat16) walks the chunks in order; the fp32 state (its gradient in the
 // backward) lives in the registers of the threads that own its rows, the products in TMEM, and nothing but
 // the inputs and outputs touches HBM in the forward pass (plus, for the backward, the fp32 state at every
 // chunk boundary).  The raw rows of the next chunk arrive by TMA while the current chunk is worked on.
