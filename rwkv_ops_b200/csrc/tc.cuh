@@ -312,17 +312,6 @@ __device__ __forceinline__ void tile_store_row32(unsigned char* tile, int row, i
     *reinterpret_cast<uint4*>(tile + tile_chunk_off(row, (col0 >> 3) + c)) = u;
   }
 }
-// read 32 consecutive bf16 values of `row` as fp32
-__device__ __forceinline__ void tile_load_row32(const unsigned char* tile, int row, int col0, float* x) {
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const uint4 u = *reinterpret_cast<const uint4*>(tile + tile_chunk_off(row, (col0 >> 3) + c));
-    x[8 * c + 0] = bf16_lo(u.x); x[8 * c + 1] = bf16_hi(u.x);
-    x[8 * c + 2] = bf16_lo(u.y); x[8 * c + 3] = bf16_hi(u.y);
-    x[8 * c + 4] = bf16_lo(u.z); x[8 * c + 5] = bf16_hi(u.z);
-    x[8 * c + 6] = bf16_lo(u.w); x[8 * c + 7] = bf16_hi(u.w);
-  }
-}
 
 // the same for N = 16 or 32 consecutive values (col0 a multiple of 8)
 template <int N>
