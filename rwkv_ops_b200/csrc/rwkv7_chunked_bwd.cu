@@ -374,14 +374,14 @@ r7c_bwd_scan_alone_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned 
 struct FinalSmem {
   unsigned char dout[TILE_BYTES], dz[TILE_BYTES];       // [do; dz]   then dA_qk, dA_ak   then red1 (fp32)
   unsigned char aqk[TILE_BYTES], aak[TILE_BYTES];       // A_qk, A_ak then dA_qb, dA_ab   then red2 (fp32)
-  unsigned char h0[TILE_BYTES];                         // h~0        then dv rows        then dw rows
+  unsigned char h0[TILE_BYTES];                         // h~0        then dv rows        then w, dw rows
   unsigned char dhh[TILE_BYTES];                        // dh^
   unsigned char v[TILE_BYTES], sa[TILE_BYTES];          // [v; sa]    (sa) then da~ a~ as bf16
   unsigned char qt[TILE_BYTES], at[TILE_BYTES];         // q~, a~     then dq, da rows
   unsigned char kt[TILE_BYTES], bt[TILE_BYTES];         // k~, b~     then dk, db rows
   float gs[L * 64];         // g log2(e), then (gi - gref) log2(e): inclusive prefix inside the chunk (sw64)
   float quart[3][64];       // sums over quarters of the chunk; [2] between the prefix sum and the epilogue: -gref
-  uint64_t bar_l0, bar_l1, bar_l2, bar_m1, bar_m2;
+  uint64_t bar_l0, bar_l1, bar_l2, bar_w, bar_m1, bar_m2;
   uint32_t tmem_base;
 };
 // two CTAs per SM: 228 KB shared by both, 1 KB of each reserved by the system
@@ -395,7 +395,8 @@ __device__ __forceinline__ int sw64(int row, int c) { return row * 64 + ((((c >>
 // window split the columns (hsel = w>>2), so every elementwise phase is spread over 8 warps.
 template <bool PACKED, bool FUSED>
 __global__ void __launch_bounds__(256, 2)
-r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtensorMap tmap_do,
+r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtensorMap tmap_w,
+                     const __grid_constant__ CUtensorMap tmap_do,
                      const __grid_constant__ CUtensorMap tmap_v, const unsigned char* __restrict__ ws_tiles,
                      int tiles_per_chunk, const __grid_constant__ CUtensorMap tmap_dq,
                      const __grid_constant__ CUtensorMap tmap_dw, const __grid_constant__ CUtensorMap tmap_dk,
@@ -421,7 +422,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
   if (tid == 0) {
     // an MMA group is issued by several threads, one accumulator each, and completes with the arrival of all
     mbar_init(&sm.bar_l0, 1); mbar_init(&sm.bar_l1, 1); mbar_init(&sm.bar_l2, 1);
-    mbar_init(&sm.bar_m1, 3); mbar_init(&sm.bar_m2, 2);
+    mbar_init(&sm.bar_w, 1); mbar_init(&sm.bar_m1, 3); mbar_init(&sm.bar_m2, 2);
     fence_mbar_init();
   }
   if (warp == 0) tmem_alloc(&sm.tmem_base, 256);
@@ -460,6 +461,10 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
   auto load_1b = [&](const ChunkPos& p) {     // h~0
     const unsigned char* tiles = ws_tiles + (size_t)p.ch * tiles_per_chunk * TILE_BYTES;
     bulk_load(sm.h0, tiles + S_H0 * TILE_BYTES, TILE_BYTES, &sm.bar_l1);
+  };
+  auto load_w_tile = [&](const ChunkPos& p) { // the w rows once more (from L2), for the decay gradient
+    mbar_expect_tx(&sm.bar_w, TILE_BYTES);
+    tma_load_4d(sm.h0, &tmap_w, &sm.bar_w, 0, sv.first<PACKED>(p.bi) + p.c * L, p.hi, sv.row<PACKED>(p.bi));
   };
   // Ask for everything a chunk-head will load to be brought into L2 (issued most of a chunk-head ahead of the
   // loads themselves, which then take an L2 round trip instead of a DRAM one).
@@ -682,7 +687,8 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     R7C_STAMP(21);
     if (warp == st_warp && elect_one() && ok) {
       if (more) load_0(nxt);      // dh^ and v have been read for the last time
-      bulk_wait_read();           // the copy of dv has left its tile, which will hold dw
+      bulk_wait_read();           // the copy of dv has left its tile, which will hold w and then dw
+      if (!row_stores) load_w_tile(cur);
     }
 
     // ---- epilogue.  Row r < 64 holds dq~_i and dk~_i (token i = r), row r >= 64 holds da~_i, db~_i; the
@@ -741,6 +747,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     ok = __syncthreads_and(ok);
     R7C_STAMP(22);
     if (row_stores && ok) {
+      if (warp == st_warp && elect_one()) load_w_tile(cur);      // (every thread has copied its dv rows out)
       store_tile_rows<256>(dq_rows + out_base, lay.st, sm.qt, Tn - t0, tid);
       store_tile_rows<256>(dk_rows + out_base, lay.st, sm.kt, Tn - t0, tid);
       store_tile_rows<256>(da_rows + out_base, lay.st, sm.at, Tn - t0, tid);
@@ -762,24 +769,24 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
       float run = dglast;
 #pragma unroll
       for (int j = 15; j >= 0; --j) { run += rv[j]; rv[j] = run; }
-      const float gfirst = quarter ? sm.gs[sw64(16 * quarter - 1, c)] : sm.quart[2][c];
-      fence_async_smem();
-      __syncthreads();      // -gref has been read, and red1, red2
-      if (warp == st_warp && elect_one() && ok && more) load_1a(nxt);
       if (quarter) sm.quart[quarter - 1][c] = run;      // the last quarter's sum carries dglast
-      __syncthreads();
+      fence_async_smem();
+      __syncthreads();      // red1 and red2 have been read
+      if (warp == st_warp && elect_one() && ok && more) load_1a(nxt);
       float add = 0.f;
       for (int q2 = quarter; q2 < 3; ++q2) add += sm.quart[q2][c];
-      float gprev = gfirst;
+      ok = ok && mbar_wait(&sm.bar_w, par, status, 329);
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         const int ii = 16 * quarter + j;
         const float e_ = __bfloat162float(*reinterpret_cast<const bf16*>(sm.sa + tile_off(ii, c)));
         const float dg = rv[j] + add - e_;
-        // dw = dg g; g is the difference of neighbouring prefix sums (in units of log 2)
-        const float gi = sm.gs[sw64(ii, c)];
-        *reinterpret_cast<bf16*>(sm.h0 + tile_off(ii, c)) = __float2bfloat16_rn(dg * (LN2 * (gi - gprev)));
-        gprev = gi;
+        // dw = dg g, with g from w itself: as the difference of two prefix sums (up to 87) the g of a token that decays
+        // slowly among faster ones would lose its digits (15 % at g = e^-11), and that of a masked token would not be 0
+        unsigned short* wp = reinterpret_cast<unsigned short*>(sm.h0 + tile_off(ii, c));
+        float w = __uint_as_float((uint32_t)*wp << 16);
+        if constexpr (FUSED) w = round_bf16(W_SCALE * sigmoidf_(w));
+        *reinterpret_cast<bf16*>(wp) = __float2bfloat16_rn(dg * (LN2 * (-LOG2E * ex2(LOG2E * w))));
       }
     }
     fence_async_smem();
@@ -892,12 +899,14 @@ int launch_rwkv7_chunked_bwd(const void* r, const void* w, const void* k, const 
   e = device_facts(&dev);
   if (e) return e;
   int* status = dev.status;
-  CUtensorMap tmap_do, tmap_v, tmap_out[6];
+  CUtensorMap tmap_do, tmap_v, tmap_w, tmap_out[6];
   const SeqView sv{seq_start, seq_len, Tn};
   const int mapB = seq_start ? 1 : B, mapT = seq_start ? T_total : Tn;   // shape of the token tensors
   e = make_token_tensor_map(&tmap_do, d_o, mapB, mapT, H, head_first);
   if (e) return e;
   e = make_token_tensor_map(&tmap_v, v, mapB, mapT, H, head_first);
+  if (e) return e;
+  e = make_token_tensor_map(&tmap_w, w, mapB, mapT, H, head_first);
   if (e) return e;
   void* outs[6] = {dr, dw, dk, dv, da, db};
   for (int i = 0; i < 6; ++i) {
@@ -954,7 +963,7 @@ int launch_rwkv7_chunked_bwd(const void* r, const void* w, const void* k, const 
     do {                                                                                                          \
       if (allow_smem<r7c_bwd_final_kernel<P, F>>(dev, smem)) \
         return RWKVB200_E_CUDA;                                                                                   \
-      r7c_bwd_final_kernel<P, F><<<grid, 256, smem, st>>>((const bf16*)w, tmap_do, tmap_v, ws.tiles, ALL_TILES,   \
+      r7c_bwd_final_kernel<P, F><<<grid, 256, smem, st>>>((const bf16*)w, tmap_w, tmap_do, tmap_v, ws.tiles, ALL_TILES, \
           tmap_out[0], tmap_out[1], tmap_out[2], tmap_out[3], tmap_out[4], tmap_out[5], (bf16*)dr, (bf16*)dw,     \
           (bf16*)dk, (bf16*)dv, (bf16*)da, (bf16*)db, sv, H, NT, n_ch, lay, status, debug_stamp_buffer());        \
     } while (0)
