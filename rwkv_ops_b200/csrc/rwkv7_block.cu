@@ -215,13 +215,16 @@ r7_sweep_kernel(Vecs<T> in, const T* __restrict__ v, const float* __restrict__ s
 #pragma unroll
       for (int l = 0; l < W; l += 4) {
         const float4 x = *reinterpret_cast<const float4*>(&st.xv[jl][l]), y = *reinterpret_cast<const float4*>(&st.yv[jl][l]);
+        // the factors of tokens after jl are 0, but 0 times an infinity or NaN is not: their v counts as 0 as well
+        const bool u0 = l <= jl, u1 = l + 1 <= jl, u2 = l + 2 <= jl, u3 = l + 3 <= jl;
         float vv[ROWS][4];
 #pragma unroll
         for (int i = 0; i < ROWS; ++i) {
           const float4 f = *reinterpret_cast<const float4*>(&st.vt[r0 + i][l]);
           vv[i][0] = f.x; vv[i][1] = f.y; vv[i][2] = f.z; vv[i][3] = f.w;
-          sa[i] += x.x * f.x + x.y * f.y + (x.z * f.z + x.w * f.w);
-          oo[i] += y.x * f.x + y.y * f.y + (y.z * f.z + y.w * f.w);
+          const float4 m = make_float4(u0 ? f.x : 0.f, u1 ? f.y : 0.f, u2 ? f.z : 0.f, u3 ? f.w : 0.f);
+          sa[i] += x.x * m.x + x.y * m.y + (x.z * m.z + x.w * m.w);
+          oo[i] += y.x * m.x + y.y * m.y + (y.z * m.z + y.w * m.w);
         }
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
@@ -586,9 +589,12 @@ r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, c
     for (int j = 1; j < GT; ++j) {
       float s1 = 0.f, s2 = 0.f;
 #pragma unroll
-      for (int i = 0; i < j; i += 4) {      // entries on and right of the diagonal are 0
+      for (int i = 0; i < j; i += 4) {
         const float4 ab = *reinterpret_cast<const float4*>(&sm.sc[2][j][i]), ak = *reinterpret_cast<const float4*>(&sm.sc[3][j][i]);
-        s1 += ak.x * vv[i]; s1 += ak.y * vv[i + 1]; s1 += ak.z * vv[i + 2]; s1 += ak.w * vv[i + 3];
+        s1 += ak.x * vv[i];
+        if (i + 1 < j) s1 += ak.y * vv[i + 1];
+        if (i + 2 < j) s1 += ak.z * vv[i + 2];
+        if (i + 3 < j) s1 += ak.w * vv[i + 3];
         s2 += ab.x * sa[i];
         if (i + 1 < j) s2 += ab.y * sa[i + 1];
         if (i + 2 < j) s2 += ab.z * sa[i + 2];

@@ -267,3 +267,37 @@ def test_float32_tokens_on_the_tensor_core_path_by_request(monkeypatch):
     assert all(g[n].grad.dtype == torch.float32 for n in "rwkvab")
     assert all(e < 2e-2 for e in errs.values()), errs
     assert errs["o"] > 1e-5      # the bfloat16 path did run (the recurrence is float32-exact)
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("dtype,K", [(torch.float32, 64), (torch.float16, 64), (torch.float32, 128), (torch.bfloat16, 128)])
+def test_tokens_before_a_non_finite_one_are_untouched(dtype, K, value):
+    """Token by token nothing after a token reaches it, whatever it holds; neither does it in blocks of tokens: outputs
+    before a NaN or an infinity stay what they are, bit for bit, and so do the gradients that do not see it."""
+    T, t = 40, 21      # inside a block of 8 and an item of 16
+    d = rwkv7_inputs(1, T, 2, K, dtype=dtype, seed=61, device="cuda", with_grads=True)
+
+    def run(x, d_o):
+        x = [y.clone().requires_grad_(True) for y in x]
+        o = ro.generalized_delta_rule(*x, output_final_state=False)
+        return o.detach(), dict(zip("rwkvab", torch.autograd.grad(o, x, d_o)))
+
+    tokens = [d[n] for n in "rwkvab"]
+    o, g = run(tokens, d["d_out"])
+    for i, n in enumerate("rwkvab"):
+        x = [y.clone() for y in tokens]
+        x[i][:, t] = value
+        o2, g2 = run(x, d["d_out"])
+        assert torch.equal(o2[:, :t], o[:, :t]), n
+        if n == "v":      # the state gradients do not depend on v: dv is what it was, the others up to the token
+            assert torch.equal(g2["v"], g["v"])
+            for m in "rwkab":
+                assert torch.equal(g2[m][:, :t], g[m][:, :t]), m
+            for m in "wab":      # ... and at the token, which they meet with the state before it
+                assert torch.isfinite(g2[m][:, t]).all(), m
+    d_o = d["d_out"].clone()
+    d_o[:, t] = value
+    _, g2 = run(tokens, d_o)
+    for m in "wkvab":      # gradients run backward in time
+        assert torch.equal(g2[m][:, t + 1:], g[m][:, t + 1:]), m
+    assert torch.equal(torch.cat([g2["r"][:, :t], g2["r"][:, t + 1:]], 1), torch.cat([g["r"][:, :t], g["r"][:, t + 1:]], 1))
