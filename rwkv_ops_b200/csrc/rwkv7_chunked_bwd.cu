@@ -200,7 +200,10 @@ struct BAloneSmem {
   float aux[4][AUX_FLOATS];     // the chunks' decay factors, with their tiles
   uint64_t bar_full[4];
   uint64_t bar_h, bar_z;        // dh^, dz of a chunk are in shared memory (one arrival per reading warp)
-  uint64_t bar_m1, bar_m2;      // dz, dh are in their accumulators
+  uint64_t bar_m1;              // dz is in its accumulator
+  // dh is in its accumulator and the chunk's tiles have been read: one barrier per stage, so that it cannot get a phase
+  // ahead of the loading warp, which waits here before it fills the stage again
+  uint64_t bar_m2[4];
   uint64_t bar_free;            // the copies issued in the previous chunk have left shared memory
   uint32_t tmem_base;
 };
@@ -224,9 +227,9 @@ r7c_bwd_scan_alone_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned 
   auto chunk_tiles = [&](int n) { return ws_tiles + (ch0 + NT - 1 - n) * (size_t)tiles_per_chunk * TILE_BYTES; };
 
   if (tid == 0) {
-    for (int i = 0; i < 4; ++i) mbar_init(&sm.bar_full[i], 1);
+    for (int i = 0; i < 4; ++i) { mbar_init(&sm.bar_full[i], 1); mbar_init(&sm.bar_m2[i], 1); }
     mbar_init(&sm.bar_h, 8); mbar_init(&sm.bar_z, 8);
-    mbar_init(&sm.bar_m1, 1); mbar_init(&sm.bar_m2, 1); mbar_init(&sm.bar_free, 1);
+    mbar_init(&sm.bar_m1, 1); mbar_init(&sm.bar_free, 1);
     fence_mbar_init();
   }
   if (warp == 0) tmem_alloc(&sm.tmem_base, 128);
@@ -277,7 +280,7 @@ r7c_bwd_scan_alone_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned 
         if (!state_lane) tile_store_row32(sm.dz[n & 1], row, c0, x);      // dz = C^T do + B2 dh^
       }
       arrive(&sm.bar_z);
-      if (!wait(&sm.bar_m2, n, 313)) break;
+      if (!wait(&sm.bar_m2[n & 3], n >> 2, 313)) break;
       {
         uint32_t r[32];
         tmem_ld32(tm_w, r);
@@ -312,7 +315,7 @@ r7c_bwd_scan_alone_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned 
         if (!ok) break;
         tc_fence_after();
         umma_tile<64, 64, 1, 1>(tmem_addr(tm, 0, 64 * (n & 1)), smem_u32(s.at), smem_u32(sm.dz[n & 1]), true);     // += a~^T dz
-        umma_commit(&sm.bar_m2);
+        umma_commit(&sm.bar_m2[n & 3]);
         // the next chunk's accumulators were read out before this chunk's dh^ arrived
         if (n + 1 < NT) ok = ahead(n + 1);
       }
@@ -332,7 +335,7 @@ r7c_bwd_scan_alone_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned 
       };
       for (int n = 0; n < 4 && n < NT; ++n) load(n);
       for (int n = 0; n + 4 < NT && ok; ++n) {
-        ok = mbar_wait(&sm.bar_m2, n & 1, status, 316);      // the tiles of the n-th chunk have been read
+        ok = mbar_wait(&sm.bar_m2[n & 3], (n >> 2) & 1, status, 316);      // the tiles of the n-th chunk have been read
         if (ok) load(n + 4);
       }
     }

@@ -871,7 +871,10 @@ struct AloneSmem {
   float aux[2][AUX_FLOATS];         // the chunks' decay factors, with the first group
   uint64_t bar_g1[2], bar_g2[2];
   uint64_t bar_h, bar_s;            // h~0, sa of a chunk are in shared memory (one arrival per reading warp)
-  uint64_t bar_a, bar_c, bar_o;     // W h~0; b~^T sa; all products of a chunk have completed
+  uint64_t bar_a, bar_c;            // W h~0; b~^T sa
+  // All products of a chunk have completed, one barrier per stage: the loading warp, whom nothing else holds back, waits
+  // here before it fills the stage again, so this barrier cannot get a phase ahead of that wait.
+  uint64_t bar_o[2];
   uint64_t bar_free;                // the copies issued in the previous chunk have left shared memory
   uint32_t tmem_base;
 };
@@ -903,9 +906,9 @@ r7c_scan_fwd_alone_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsi
   auto chunk_tiles = [&](int c) { return ws_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES; };
 
   if (tid == 0) {
-    for (int i = 0; i < 2; ++i) { mbar_init(&sm.bar_g1[i], 1); mbar_init(&sm.bar_g2[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&sm.bar_g1[i], 1); mbar_init(&sm.bar_g2[i], 1); mbar_init(&sm.bar_o[i], 1); }
     mbar_init(&sm.bar_h, 8); mbar_init(&sm.bar_s, 8);
-    mbar_init(&sm.bar_a, 1); mbar_init(&sm.bar_c, 1); mbar_init(&sm.bar_o, 1); mbar_init(&sm.bar_free, 1);
+    mbar_init(&sm.bar_a, 1); mbar_init(&sm.bar_c, 1); mbar_init(&sm.bar_free, 1);
     fence_mbar_init();
   }
   if (warp == 0) tmem_alloc(&sm.tmem_base, 256);
@@ -1027,7 +1030,7 @@ r7c_scan_fwd_alone_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsi
       }
       R7C_STAMP(53);
     }
-    ok = ok && wait(&sm.bar_o, NT - 1, 217);
+    ok = ok && wait(&sm.bar_o[(NT - 1) & 1], (NT - 1) >> 1, 217);
   } else if (warp == 8) {      // ---- MMAs
     if (elect_one()) {
       for (int c = 0; c < NT && ok; ++c) {
@@ -1048,7 +1051,7 @@ r7c_scan_fwd_alone_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsi
         umma_commit(&sm.bar_c);
         umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, acc), smem_u32(g2.qt), smem_u32(sm.ht[c & 1]), true);     // += q~ h~0
         umma_tile<64, 64, 0, 1>(tmem_addr(tm, 16, acc), smem_u32(g2.aqb), smem_u32(sm.sa[c & 1]), true);    // += A_qb sa
-        umma_commit(&sm.bar_o);
+        umma_commit(&sm.bar_o[c & 1]);
       }
     }
     __syncwarp();
@@ -1072,7 +1075,7 @@ r7c_scan_fwd_alone_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsi
           bulk_prefetch_l2(chunk_tiles(c + 4), FWD_TILES * TILE_BYTES);
           tma_prefetch_4d(&tmap_v, 0, tb + (c + 4) * L, hi, brow);
         }
-        ok = mbar_wait(&sm.bar_o, c & 1, status, 216);      // the tiles of chunk c have been read
+        ok = mbar_wait(&sm.bar_o[c & 1], (c >> 1) & 1, status, 216);      // the tiles of chunk c have been read
         if (ok) { load_1(c + 2); load_2(c + 2); }
       }
     }

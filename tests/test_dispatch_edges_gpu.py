@@ -4,6 +4,7 @@ import pytest
 import torch
 
 import rwkv_ops_b200 as ro
+from rwkv_ops_b200 import _lib
 from oracle import generalized_delta_rule as oracle_gdr
 from rwkv_ops_b200.workloads import rwkv7_inputs, wkv6_inputs, rel_l2
 
@@ -61,3 +62,16 @@ def test_wkv6_states_in_the_token_dtype(T, many):
         y32, s32 = op(d["r"], d["k"], d["v"], d["w"], u.float(), with_state=True, init_state=s0.float(), state_map=smap)
     assert y.dtype == s.dtype == torch.bfloat16
     assert torch.equal(y, y32) and torch.equal(s, s32.to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("T", [64 * 9, 64 * 17 - 5, 64 * 40 + 1])
+def test_stages_of_the_scans_for_few_sequences_wrap_around(T):
+    """Chunks enough to fill every stage of operand tiles several times over, against the recurrence; no wait runs out."""
+    d = {n: t.cuda() for n, t in rwkv7_inputs(1, T, 2, dtype=torch.bfloat16, seed=90, with_state=True, with_grads=True).items()}
+    lib = _lib.load()
+    lib.rwkvb200_device_status(1)
+    out = _train(d, [d["d_out"], d["d_state"]])
+    assert lib.rwkvb200_device_status(1) == 0
+    ref = _train({n: t.float() for n, t in d.items()}, [d["d_out"].float(), d["d_state"]])
+    for n in ref:
+        assert rel_l2(out[n], ref[n]) < 2e-2, n
