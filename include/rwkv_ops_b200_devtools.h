@@ -15,6 +15,10 @@ extern "C" {
  * clock64() stamps at its phase boundaries into it; NULL switches it off. */
 void rwkvb200_debug_stamps(void* device_buffer);
 
+/* Whether a kernel whose dynamic shared memory has to start 1024-byte aligned may be launched where a block's shared memory
+ * begins with `reserved` bytes of the system's and `static_bytes` of the kernel's own. */
+int rwkvb200_smem_starts_aligned(int reserved, int static_bytes);
+
 /*
  * rwkvb200_tc_selftest: runs one building block on caller data so a test can compare with a plain
  *   matrix product.  mode 0: out[128][128] = [X;Y] [Z;W]^T (X..W are 64x64 bf16, row-major);

@@ -64,6 +64,7 @@ SIGNATURES = {
 # the developer build adds these (include/rwkv_ops_b200_devtools.h)
 DEV_SIGNATURES = {
     "rwkvb200_debug_stamps": (None, [_P]),
+    "rwkvb200_smem_starts_aligned": (c_int, [_I] * 2),
     "rwkvb200_tc_selftest": (c_int, [_I] + [_P] * 6 + [_I] * 6 + [_P, _P]),
 }
 

@@ -134,6 +134,27 @@ int allow_smem(const DeviceFacts& f, int bytes) {
   return RWKVB200_OK;
 }
 
+// Whether a block's dynamic shared memory starts 1024-byte aligned, as swizzled tiles need it: it follows what the system
+// reserves and the kernel's static arrays.
+inline bool smem_starts_aligned(int reserved, int static_bytes) { return (reserved + static_bytes) % 1024 == 0; }
+// The same for `Kernel` on the current device, asked once per device: RWKVB200_E_UNSUPPORTED where it does not.  For a kernel
+// that has no room to align by hand; without this its own check would leave the outputs unwritten.
+template <auto Kernel>
+int need_aligned_smem(const DeviceFacts& f) {
+  static std::atomic<int> known[64];      // 1: yes, 2: no
+  int n = known[f.dev].load(std::memory_order_acquire);
+  if (!n) {
+    int reserved = 0;
+    cudaFuncAttributes a;
+    if (cuda_ok(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, f.dev)) ||
+        cuda_ok(cudaFuncGetAttributes(&a, Kernel)))
+      return RWKVB200_E_CUDA;
+    n = smem_starts_aligned(reserved, (int)a.sharedSizeBytes) ? 1 : 2;
+    known[f.dev].store(n, std::memory_order_release);
+  }
+  return n == 1 ? RWKVB200_OK : RWKVB200_E_UNSUPPORTED;
+}
+
 // Brackets one kernel launch with timing events when profiling is on (see profile.cu).
 struct ProfScope {
   ProfScope(const char* name, cudaStream_t st);

@@ -262,6 +262,7 @@ using namespace rwkvb200;
 extern "C" {
 
 #ifdef RWKVB200_DEVTOOLS
+int rwkvb200_smem_starts_aligned(int reserved, int static_bytes) { return smem_starts_aligned(reserved, static_bytes); }
 void rwkvb200_debug_stamps(void* device_buffer) { g_stamp_buffer = reinterpret_cast<long long*>(device_buffer); }
 #endif
 

@@ -113,3 +113,15 @@ def test_python_mirrors_of_the_kept_sizes_match_the_library(lib):
         assert _lib.rwkv7_kept_bytes(B, T, H) == lib.rwkvb200_rwkv7_varlen_workspace_bytes(B, T, H, 64, 1)
         assert _lib.wkv6_kept_bytes(B, T, H) == lib.rwkvb200_wkv6_fwd_workspace_bytes(B, T, H, 64, _lib.F32, keep)
         assert _lib.wkv6_kept_bytes(B, T, H) == lib.rwkvb200_wkv6_bwd_workspace_bytes(B, T, H, 64, _lib.F32, 0)
+
+
+def test_shared_memory_that_has_to_start_aligned():
+    """A kernel without room to align its tiles by hand is refused by its launch, not skipped by its own check, where the
+    system's and the kernel's own shared memory do not leave the rest 1024-byte aligned."""
+    if not os.path.exists(_lib.DEV_LIB_PATH):
+        from rwkv_ops_b200.build import build
+        build(dev=True)
+    f = _lib.load_dev().rwkvb200_smem_starts_aligned
+    assert f(1024, 0) == 1 and f(0, 2048) == 1 and f(0, 0) == 1
+    for reserved, static in ((0, 16), (1024, 8), (1000, 0), (2048, 1023)):
+        assert f(reserved, static) == 0
