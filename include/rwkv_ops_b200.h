@@ -232,6 +232,7 @@ int rwkvb200_rwkv7_bwd_static(const void* r, const void* w, const void* k, const
  *                  state_map is the caller's to check on the host (the Python layer does, before the
  *                  launch); out-of-range entries are clamped on the device instead of trapping.
  *   sT             final state [B,H,64,64], may be NULL.
+ *                  u, s0 and sT are float32, or of the token dtype with RWKVB200_ALGO_TOKEN_STATES.
  *   algo           RWKVB200_ALGO_AUTO / _RECURRENT (token-by-token float32) / _CHUNKED (tcgen05 with
  *                  split-precision bf16 operands, float32-grade accuracy for every dtype); AUTO = chunked.
  *                  With RWKVB200_ALGO_KEEP (chunked only) the forward also writes the state at every chunk
@@ -253,9 +254,9 @@ int rwkvb200_rwkv7_bwd_static(const void* r, const void* w, const void* k, const
  * ---------------------------------------------------------------------------------------- */
 size_t rwkvb200_wkv6_fwd_workspace_bytes(int B, int T, int H, int head_size, int dtype, int algo);
 
-int rwkvb200_wkv6_fwd(const void* r, const void* k, const void* v, const void* w, const float* u,
-                      const float* s0, int n_state, const int32_t* state_map,
-                      void* y, float* sT, void* workspace, size_t workspace_bytes,
+int rwkvb200_wkv6_fwd(const void* r, const void* k, const void* v, const void* w, const void* u,
+                      const void* s0, int n_state, const int32_t* state_map,
+                      void* y, void* sT, void* workspace, size_t workspace_bytes,
                       int B, int T, int H, int head_size, int dtype, int algo, void* stream);
 
 size_t rwkvb200_wkv6_bwd_workspace_bytes(int B, int T, int H, int head_size, int dtype, int algo);

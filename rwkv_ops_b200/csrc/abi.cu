@@ -300,9 +300,9 @@ size_t rwkvb200_wkv6_fwd_workspace_bytes(int B, int T, int H, int head_size, int
   return (algo & RWKVB200_ALGO_KEEP) ? wkv6_chunked_bwd_workspace_bytes(B, T, H) : wkv6_chunked_fwd_scratch_bytes(B, H);
 }
 
-int rwkvb200_wkv6_fwd(const void* r, const void* k, const void* v, const void* w, const float* u,
-                      const float* s0, int n_state, const int32_t* state_map,
-                      void* y, float* sT, void* workspace, size_t workspace_bytes,
+int rwkvb200_wkv6_fwd(const void* r, const void* k, const void* v, const void* w, const void* u,
+                      const void* s0, int n_state, const int32_t* state_map,
+                      void* y, void* sT, void* workspace, size_t workspace_bytes,
                       int B, int T, int H, int head_size, int dtype, int algo, void* stream) {
   int e = check_w6(B, T, H, head_size, dtype, algo);
   if (e) return e;

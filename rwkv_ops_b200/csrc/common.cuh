@@ -213,8 +213,8 @@ int launch_rwkv7_block_bwd(const void* r, const void* w, const void* k, const vo
                            int dtype, int head_first, cudaStream_t st, int head_size = HS);
 constexpr int R7_CKPT = 8;   // tokens between state checkpoints of the recurrent backward
 
-int launch_wkv6_fwd(const void* r, const void* k, const void* v, const void* w, const float* u,
-                    const float* s0, int n_state, const int32_t* smap, void* y, float* sT,
+int launch_wkv6_fwd(const void* r, const void* k, const void* v, const void* w, const void* u,
+                    const void* s0, int n_state, const int32_t* smap, void* y, void* sT,
                     float* ckpt, int B, int Tn, int H, int dtype, cudaStream_t st, const UnitSel* sel = nullptr,
                     int ckpt_every = 0, int head_size = HS, bool typed = false);
 int launch_wkv6_bwd_coarse(const void* r, const void* k, const void* v, const void* w, const float* u,
@@ -232,8 +232,8 @@ constexpr int W6_CKPT = 8;
 // `typed`: u, s0 and sT hold the token dtype instead of float32.
 // Chunked tcgen05 wkv6 (wkv6_chunked.cu).  `states` (may be NULL) receives the fp32 state at every chunk
 // boundary, [B*H][ceil(T/64)+1][64][64].
-int launch_wkv6_chunked_fwd(const void* r, const void* k, const void* v, const void* w, const float* u,
-                            const float* s0, int n_state, const int32_t* smap, void* y, float* sT,
+int launch_wkv6_chunked_fwd(const void* r, const void* k, const void* v, const void* w, const void* u,
+                            const void* s0, int n_state, const int32_t* smap, void* y, void* sT,
                             float* states, int* flags, float* handoff, int* hflags, int B, int Tn, int H, int dtype,
                             cudaStream_t st, const int32_t* seq_start = nullptr, const int32_t* seq_len = nullptr,
                             int T_total = 0, bool typed = false);

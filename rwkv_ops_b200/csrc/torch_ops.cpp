@@ -98,6 +98,7 @@ OptTensor dense_state(const OptTensor& x) {
 }
 bool has(const OptTensor& x) { return x.has_value() && x->defined(); }
 void* ptr(const Tensor& x) { return x.defined() ? x.data_ptr() : nullptr; }
+void* ptr(const OptTensor& x) { return x.has_value() ? ptr(*x) : nullptr; }
 float* fptr(const OptTensor& x) { return has(x) ? static_cast<float*>(x->data_ptr()) : nullptr; }
 float* fptr(const Tensor& x) { return static_cast<float*>(ptr(x)); }
 const int32_t* iptr(const OptTensor& x) { return has(x) ? x->data_ptr<int32_t>() : nullptr; }
@@ -460,17 +461,24 @@ std::tuple<Tensor, Tensor> rwkv7_fused(const Tensor& r, const Tensor& w_pre, con
 // ---------------------------------------------------------------------------------------------
 // RWKV6 wkv, dense
 // ---------------------------------------------------------------------------------------------
+// x itself if its first element is 16-byte aligned (what the C ABI asks for), else a copy
+Tensor aligned(const Tensor& x) { return reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 ? x.clone() : x; }
+
 Three wkv6_fwd(const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& u, const OptTensor& s0,
                const OptTensor& state_map, int64_t algo, bool keep) {
   const c10::cuda::CUDAGuard guard(r.device());
   const int B = (int)r.size(0), T = (int)r.size(1), H = (int)u.size(0), N = (int)u.size(1);
   const int code = dtype_code(r.scalar_type()), flags = (int)algo | (keep ? RWKVB200_ALGO_KEEP : 0);
   Tensor y = fresh_like(r), sT = fresh({B, H, N, N}, algo & RWKVB200_ALGO_TOKEN_STATES ? r.scalar_type() : at::kFloat, r);
+  // states and u in the token dtype come as the caller holds them, e.g. as a view into a larger buffer
+  const bool typed = algo & RWKVB200_ALGO_TOKEN_STATES;
+  const Tensor u_ = typed ? aligned(u) : u;
+  const OptTensor s0_ = typed && has(s0) ? OptTensor(aligned(*s0)) : s0;
   // a training forward of the chunked path leaves the chunk-boundary states for the backward
   const size_t nws = rwkvb200_wkv6_fwd_workspace_bytes(B, T, H, N, code, flags);
   Tensor ws = bytes(nws, r);
-  check(rwkvb200_wkv6_fwd(ptr(r), ptr(k), ptr(v), ptr(w), fptr(u), fptr(s0), n_state_of(s0), iptr(state_map), ptr(y),
-                          fptr(sT), nws ? ptr(ws) : nullptr, nws, B, T, H, N, code, flags, stream_of(r)), "wkv6_fwd");
+  check(rwkvb200_wkv6_fwd(ptr(r), ptr(k), ptr(v), ptr(w), ptr(u_), ptr(s0_), n_state_of(s0), iptr(state_map), ptr(y),
+                          ptr(sT), nws ? ptr(ws) : nullptr, nws, B, T, H, N, code, flags, stream_of(r)), "wkv6_fwd");
   return {y, sT, keep ? ws : bytes(0, r)};
 }
 

@@ -474,8 +474,8 @@ wkv6_du_reduce_mixed_kernel(const float* __restrict__ part_chunked, const float*
     default: return RWKVB200_E_UNSUPPORTED;                       \
   }
 
-int launch_wkv6_fwd(const void* r, const void* k, const void* v, const void* w, const float* u,
-                    const float* s0, int n_state, const int32_t* smap, void* y, float* sT,
+int launch_wkv6_fwd(const void* r, const void* k, const void* v, const void* w, const void* u,
+                    const void* s0, int n_state, const int32_t* smap, void* y, void* sT,
                     float* ckpt, int B, int Tn, int H, int dtype, cudaStream_t st, const UnitSel* sel_,
                     int ckpt_every, int head_size, bool typed) {
   const UnitSel sel = sel_ ? *sel_ : UnitSel{nullptr, nullptr, nullptr, 0};

@@ -1063,8 +1063,8 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
 
 }  // namespace w6c
 
-int launch_wkv6_chunked_fwd(const void* r, const void* k, const void* v, const void* w, const float* u,
-                            const float* s0, int n_state, const int32_t* smap, void* y, float* sT,
+int launch_wkv6_chunked_fwd(const void* r, const void* k, const void* v, const void* w, const void* u,
+                            const void* s0, int n_state, const int32_t* smap, void* y, void* sT,
                             float* states, int* flags, float* handoff, int* hflags, int B, int Tn, int H,
                             int dtype, cudaStream_t st, const int32_t* seq_start, const int32_t* seq_len,
                             int T_total, bool typed) {

@@ -232,3 +232,24 @@ def test_more_units_than_sms_work_items(B, H, T, monkeypatch):
         res[algo] = {"y": y, "s": s, "ds0": s0.grad, **{n: g[n].grad for n in "rkvwu"}}
     errs = {k_: rel_l2(res["chunked"][k_], res["recurrent"][k_]) for k_ in res["chunked"]}
     assert max(errs.values()) < 1e-4, errs
+
+
+@pytest.mark.parametrize("which", ["u", "init_state"])
+def test_bfloat16_states_as_views_that_start_anywhere(which):
+    """u or the state table as a view two bytes into a larger buffer, with and without gradients."""
+    B, T, H = 3, 70, 2
+    d = wkv6_inputs(B, T, H, dtype=torch.bfloat16, seed=5, device="cuda", n_state=3)
+    op = ro.RWKV6_OP(64, T)
+
+    def call():
+        return op(d["r"], d["k"], d["v"], d["w"], d["u"], with_state=True, init_state=d["init_state"], state_map=d["state_map"])
+
+    y, s = call()
+    flat = torch.empty(d[which].numel() + 1, dtype=torch.bfloat16, device="cuda")
+    flat[1:] = d[which].flatten()
+    d[which] = flat[1:].view(d[which].shape)
+    assert d[which].data_ptr() % 16 == 2 and d[which].is_contiguous()
+    for grad in (False, True):
+        d["r"].requires_grad_(grad)
+        y2, s2 = call()
+        assert torch.equal(y2, y) and torch.equal(s2, s)
