@@ -128,14 +128,14 @@ def _check_wkv6_args(r, k, v, w, u, cu_seqlens, init_state, state_map, head_size
         raise ValueError(f"u must have {H * N} elements")
     if isinstance(cu_seqlens, PackedSequences) and (cu_seqlens.total_len != r.shape[1] or cu_seqlens.start.device != dev):
         raise ValueError("the PackedSequences object was made for another token count or device")
-    n_seq = cu_seqlens.start.numel() if isinstance(cu_seqlens, PackedSequences) else len(cu_seqlens) - 1
+    n_seq = cu_seqlens.start.numel() if isinstance(cu_seqlens, PackedSequences) else torch.as_tensor(cu_seqlens).numel() - 1
     if init_state is not None:
         if init_state.dim() not in (3, 4) or tuple(init_state.shape[-3:]) != (H, N, N):
             raise ValueError(f"init_state must be [n_state, {H}, {N}, {N}] or [{H}, {N}, {N}]")
         n_state = 1 if init_state.dim() == 3 else init_state.shape[0]
         if state_map is None and n_state not in (1, n_seq):
             raise ValueError("state_map cannot be inferred from init_state; pass it explicitly")
-        if state_map is not None and len(state_map) != n_seq:
+        if state_map is not None and torch.as_tensor(state_map).numel() != n_seq:
             raise ValueError("state_map must have one entry per sequence")
     elif state_map is not None:
         raise ValueError("state_map needs init_state")
@@ -164,15 +164,15 @@ def wkv6_varlen(r, k, v, w, u, cu_seqlens, init_state=None, state_map=None, head
         else:
             _check_wkv6_args(r, k, v, w, u, cu_seqlens, init_state, state_map, head_size)
             p = cu_seqlens if isinstance(cu_seqlens, PackedSequences) else _pack(cu_seqlens, r.shape[1], r.device)
-        if state_map is not None and not (isinstance(state_map, torch.Tensor) and state_map.is_cuda):
+        if state_map is not None:
             if isinstance(state_map, (list, tuple)):
                 host_map = state_map = torch.tensor(state_map, dtype=torch.int32)
             if init_state is None:
                 raise ValueError("state_map needs init_state")
             n_state = 1 if init_state.dim() == 3 else init_state.shape[0]
-            if not (bool((state_map >= 0).all()) and bool((state_map < n_state).all())):
+            if not state_map.is_cuda and not (bool((state_map >= 0).all()) and bool((state_map < n_state).all())):
                 raise ValueError(f"state_map values must lie in [0, {n_state})")
-            state_map = state_map.to(r.device)
+            state_map = state_map.to(r.device, torch.int32)      # (any dtype that holds whole numbers)
         y, sT = _ops.load().wkv6_varlen(r, k, v, w, u, p.start, p.lens, p.max_len, init_state, state_map)
     except Exception as e:
         _check_wkv6_args(r, k, v, w, u, cu_seqlens, init_state, host_map, head_size)

@@ -3,7 +3,7 @@ import pytest
 import torch
 
 import rwkv_ops_b200 as ro
-from rwkv_ops_b200.workloads import rel_l2, rwkv7_inputs
+from rwkv_ops_b200.workloads import rel_l2, rwkv7_inputs, wkv6_inputs
 
 pytestmark = pytest.mark.gpu
 
@@ -282,3 +282,26 @@ def test_wkv6_packed_with_more_sequences_than_cta_slots():
     errs = {"y": rel_l2(y, torch.cat(ys, 1)), "s": rel_l2(s, torch.cat(ss, 0))}
     errs.update({n: rel_l2(g[n].grad, g2[n].grad) for n in "rkvwu"})
     assert max(errs.values()) < 1e-4, errs
+
+
+def test_wkv6_state_map_and_offsets_in_every_accepted_form():
+    """A state map of any dtype and shape that holds one whole number per sequence, on either device; offsets of any shape."""
+    H, cu = 2, [0, 30, 70]
+    d = wkv6_inputs(1, 70, H, dtype=torch.bfloat16, seed=5, device="cuda", n_state=3)
+
+    def call(state_map, cu_seqlens=cu):
+        return ro.wkv6_varlen(d["r"], d["k"], d["v"], d["w"], d["u"], cu_seqlens, init_state=d["init_state"], state_map=state_map)
+
+    y, s = call([0, 2])
+    packed = ro.PackedSequences(cu)
+    for offsets in (cu, packed):
+        for dtype in (torch.uint8, torch.int16, torch.int32, torch.int64, torch.float32):
+            for shape in ((2,), (1, 2), (2, 1)):
+                for device in ("cpu", "cuda"):
+                    y2, s2 = call(torch.tensor([0, 2], dtype=dtype, device=device).view(shape), offsets)
+                    assert torch.equal(y2, y) and torch.equal(s2, s), (dtype, shape, device)
+        for wrong in ([0], [0, 1, 2], [0, 3], [-1, 0], torch.tensor([0, 3]), torch.zeros(3, dtype=torch.int32, device="cuda")):
+            with pytest.raises(ValueError):
+                call(wrong, offsets)
+    y2, s2 = call([0, 2], torch.tensor([cu]))
+    assert torch.equal(y2, y) and torch.equal(s2, s)
