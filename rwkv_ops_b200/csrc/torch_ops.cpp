@@ -14,6 +14,9 @@
 //
 // The library is linked against torch only.  The rwkvb200_* symbols come from the C-ABI library that the Python
 // layer has loaded before (RTLD_GLOBAL).
+//
+// The composite operators are traced with symbolic sizes, so they look at sizes as SymInt: comparing them leaves a guard,
+// where asking for them as integers would make every length a program of its own.
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContextLight.h>
 #include <ATen/cuda/EmptyTensor.h>
@@ -34,6 +37,7 @@
 namespace {
 
 using at::Tensor;
+using c10::SymInt;
 typedef std::optional<Tensor> OptTensor;
 typedef torch::autograd::variable_list Vars;
 typedef torch::autograd::AutogradContext Ctx;
@@ -120,7 +124,7 @@ bool any_requires_grad(at::ArrayRef<const Tensor*> xs, const OptTensor& s) {
 
 // gradient of the states a batch started from, summed where one state served every row
 Tensor state_grad(const Tensor& rows, const OptTensor& s0) {
-  if (s0->size(0) == 1 && rows.size(0) != 1) return rows.sum(at::IntArrayRef{0}, /*keepdim=*/true);
+  if (s0->sym_size(0) == 1 && rows.sym_size(0) != 1) return rows.sum(at::IntArrayRef{0}, /*keepdim=*/true);
   return rows;
 }
 // gradients as the backward kernels take them
@@ -147,14 +151,14 @@ typedef std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> Seven
 void check_tokens(const Tensor& r, at::ArrayRef<const Tensor*> rest, int dims) {
   TORCH_CHECK_VALUE(r.is_cuda() && r.dim() == dims, "expected CUDA token tensors with ", dims, " dimensions");
   for (const Tensor* x : rest)
-    TORCH_CHECK_VALUE(x->is_cuda() && x->device() == r.device() && x->sizes() == r.sizes(),
+    TORCH_CHECK_VALUE(x->is_cuda() && x->device() == r.device() && x->sym_sizes() == r.sym_sizes(),
                       "token tensors must agree in shape and device");
 }
-void check_state(const OptTensor& s, const Tensor& r, int64_t B, int64_t H, int64_t N) {
+void check_state(const OptTensor& s, const Tensor& r, const SymInt& B, const SymInt& H, const SymInt& N) {
   if (!has(s)) return;
-  TORCH_CHECK_VALUE(s->is_cuda() && s->device() == r.device() && s->dim() == 4 && s->size(1) == H && s->size(2) == N &&
-                        s->size(3) == N && (s->size(0) == 1 || s->size(0) == B),
-                    "initial_state must be [", B, " or 1, ", H, ", ", N, ", ", N, "], got ", s->sizes());
+  TORCH_CHECK_VALUE(s->is_cuda() && s->device() == r.device() && s->dim() == 4 && s->sym_size(1) == H && s->sym_size(2) == N &&
+                        s->sym_size(3) == N && (s->sym_size(0) == 1 || s->sym_size(0) == B),
+                    "initial_state must be [", B, " or 1, ", H, ", ", N, ", ", N, "], got ", s->sym_sizes());
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -164,6 +168,18 @@ struct Dims { int B, T, H, K; };
 Dims dims_of(const Tensor& r, bool head_first) {
   const int T = head_first ? 2 : 1, H = head_first ? 1 : 2;
   return {(int)r.size(0), (int)r.size(T), (int)r.size(H), (int)r.size(3)};
+}
+
+struct SymDims { SymInt B, T, H, K; };
+SymDims sym_dims_of(const Tensor& r, bool head_first) {
+  const int T = head_first ? 2 : 1, H = head_first ? 1 : 2;
+  return {r.sym_size(0), r.sym_size(T), r.sym_size(H), r.sym_size(3)};
+}
+// whether the tiles that a training forward would leave for its backward stay within the limit
+bool keep_fits(const SymDims& d, int algo, const Tensor& r) {
+  const auto n = [](const SymInt& x) { return (int)x.guard_int(__FILE__, __LINE__); };
+  return rwkvb200_rwkv7_fwd_workspace_bytes(n(d.B), n(d.T), n(d.H), n(d.K), RWKVB200_BF16, algo | RWKVB200_ALGO_KEEP) <=
+         keep_limit_bytes(r.device().index());
 }
 
 Three rwkv7_fwd(const Tensor& r, const Tensor& w, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& b,
@@ -241,7 +257,7 @@ std::tuple<Tensor, Tensor> generalized_delta_rule(const Tensor& r, const Tensor&
                                                   const Tensor& a, const Tensor& b, const OptTensor& initial_state,
                                                   bool head_first) {
   check_tokens(r, {&w, &k, &v, &a, &b}, 4);
-  const Dims d = dims_of(r, head_first);
+  const SymDims d = sym_dims_of(r, head_first);
   TORCH_CHECK_VALUE(d.K == 64 || d.K == 128, "head size must be 64 or 128, got ", d.K);
   check_state(initial_state, r, d.B, d.H, d.K);
   const int algo = algo_from_env("RWKV_OPS_B200_RWKV7_ALGO");
@@ -252,8 +268,7 @@ std::tuple<Tensor, Tensor> generalized_delta_rule(const Tensor& r, const Tensor&
   bool keep = false;
   if (d.T > 1 && t == at::kBFloat16 && d.K == HEAD && algo != RWKVB200_ALGO_RECURRENT &&
       any_requires_grad({&r_, &w_, &k_, &v_, &a_, &b_}, h0))
-    keep = rwkvb200_rwkv7_fwd_workspace_bytes(d.B, d.T, d.H, d.K, RWKVB200_BF16, algo | RWKVB200_ALGO_KEEP) <=
-           keep_limit_bytes(r.device().index());
+    keep = keep_fits(d, algo, r);
   auto [o, ht, kept] = RWKV_OP(rwkv7_fwd, "rwkv7_fwd", r_, w_, k_, v_, a_, b_, h0, head_first, algo, keep);
   return {o.to(r.scalar_type()), ht};
 }
@@ -364,9 +379,9 @@ std::tuple<Tensor, Tensor> rwkv7_varlen(const Tensor& r, const Tensor& w, const 
                                         const Tensor& a, const Tensor& b, const Tensor& seq_start, const Tensor& seq_len,
                                         int64_t max_len, const OptTensor& initial_state) {
   check_tokens(r, {&w, &k, &v, &a, &b}, 4);
-  TORCH_CHECK_VALUE(r.size(0) == 1 && r.size(3) == HEAD && r.scalar_type() == at::kBFloat16,
-                    "expected packed bfloat16 token tensors [1, total_len, H, 64], got ", r.sizes());
-  check_state(initial_state, r, seq_start.numel(), r.size(2), HEAD);
+  TORCH_CHECK_VALUE(r.sym_size(0) == 1 && r.sym_size(3) == HEAD && r.scalar_type() == at::kBFloat16,
+                    "expected packed bfloat16 token tensors [1, total_len, H, 64], got ", r.sym_sizes());
+  check_state(initial_state, r, seq_start.sym_numel(), r.sym_size(2), HEAD);
   const at::ScalarType t = at::kBFloat16;
   const Tensor r_ = dense(r, t), w_ = dense(w, t), k_ = dense(k, t), v_ = dense(v, t), a_ = dense(a, t), b_ = dense(b, t);
   const OptTensor h0 = dense_state(initial_state);
@@ -443,17 +458,13 @@ Three rwkv7_fused_fwd_autograd(const Tensor& r, const Tensor& w_pre, const Tenso
 std::tuple<Tensor, Tensor> rwkv7_fused(const Tensor& r, const Tensor& w_pre, const Tensor& k, const Tensor& v,
                                        const Tensor& kk_pre, const Tensor& a_pre, const OptTensor& initial_state) {
   check_tokens(r, {&w_pre, &k, &v, &kk_pre, &a_pre}, 4);
-  const Dims d = dims_of(r, false);
+  const SymDims d = sym_dims_of(r, false);
   TORCH_CHECK_VALUE(d.K == HEAD, "head size must be 64, got ", d.K);
   check_state(initial_state, r, d.B, d.H, d.K);
   const Tensor r_ = r.contiguous(), w_ = w_pre.contiguous(), k_ = k.contiguous(), v_ = v.contiguous(),
                u_ = kk_pre.contiguous(), q_ = a_pre.contiguous();
   const OptTensor h0 = dense_state(initial_state);
-  bool keep = false;
-  if (any_requires_grad({&r_, &w_, &k_, &v_, &u_, &q_}, h0))
-    keep = rwkvb200_rwkv7_fwd_workspace_bytes(d.B, d.T, d.H, d.K, RWKVB200_BF16,
-                                              RWKVB200_ALGO_CHUNKED | RWKVB200_ALGO_KEEP) <=
-           keep_limit_bytes(r.device().index());
+  const bool keep = any_requires_grad({&r_, &w_, &k_, &v_, &u_, &q_}, h0) && keep_fits(d, RWKVB200_ALGO_CHUNKED, r);
   auto [o, ht, kept] = RWKV_OP(rwkv7_fused_fwd, "rwkv7_fused_fwd", r_, w_, k_, v_, u_, q_, h0, keep);
   return {o, ht};
 }
@@ -543,24 +554,24 @@ struct Wkv6Args {
   OptTensor s0, map;
 };
 Wkv6Args wkv6_args(const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& u, int64_t N,
-                   int64_t rows, const OptTensor& init_state, const OptTensor& state_map, bool typed = false) {
+                   const SymInt& rows, const OptTensor& init_state, const OptTensor& state_map, bool typed = false) {
   check_tokens(r, {&k, &v, &w}, 3);
-  const int64_t C = r.size(2), H = C / N;
+  const SymInt C = r.sym_size(2), H = C / N;
   const at::ScalarType dt = r.scalar_type(), t = compute_dtype(dt);
-  TORCH_CHECK_VALUE(C % N == 0 && u.is_cuda() && u.device() == r.device() && u.numel() == C && k.scalar_type() == dt &&
+  TORCH_CHECK_VALUE(C % N == 0 && u.is_cuda() && u.device() == r.device() && u.sym_numel() == C && k.scalar_type() == dt &&
                         v.scalar_type() == dt && w.scalar_type() == dt, "r, k, v, w, u do not agree");
   Wkv6Args x;
   if (has(init_state)) {
     const Tensor s = init_state->dim() == 3 ? init_state->unsqueeze(0) : *init_state;
-    TORCH_CHECK_VALUE(s.is_cuda() && s.device() == r.device() && s.dim() == 4 && s.size(1) == H && s.size(2) == N &&
-                          s.size(3) == N, "init_state must be [n_state, ", H, ", ", N, ", ", N, "]");
+    TORCH_CHECK_VALUE(s.is_cuda() && s.device() == r.device() && s.dim() == 4 && s.sym_size(1) == H &&
+                          s.sym_size(2) == N && s.sym_size(3) == N, "init_state must be [n_state, ", H, ", ", N, ", ", N, "]");
     if (has(state_map)) {
-      TORCH_CHECK_VALUE(state_map->is_cuda() && state_map->numel() == rows &&
+      TORCH_CHECK_VALUE(state_map->is_cuda() && state_map->sym_numel() == rows &&
                             (state_map->scalar_type() == at::kInt || state_map->scalar_type() == at::kLong),
                         "state_map must hold one int32 or int64 entry per row");
-      x.map = state_map->to(r.device(), at::kInt).contiguous().view({rows});
+      x.map = state_map->to(r.device(), at::kInt).contiguous().view(-1);
     } else {
-      TORCH_CHECK_VALUE(s.size(0) == 1 || s.size(0) == rows,
+      TORCH_CHECK_VALUE(s.sym_size(0) == 1 || s.sym_size(0) == rows,
                         "state_map cannot be inferred from init_state; pass it explicitly");
     }
     x.s0 = typed ? s.contiguous() : s.to(at::kFloat).contiguous();
@@ -568,7 +579,7 @@ Wkv6Args wkv6_args(const Tensor& r, const Tensor& k, const Tensor& v, const Tens
     TORCH_CHECK_VALUE(!has(state_map), "state_map needs init_state");
   }
   x.r = dense(r, t); x.k = dense(k, t); x.v = dense(v, t); x.w = dense(w, t);
-  x.u = u.reshape({H, N});
+  x.u = u.reshape_symint({H, N});
   x.u = typed ? x.u.contiguous() : x.u.to(at::kFloat).contiguous();
   return x;
 }
@@ -578,18 +589,18 @@ at::ScalarType state_dtype(at::ScalarType t) { return t == at::kHalf ? at::kFloa
 std::tuple<Tensor, Tensor> wkv6(const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& u,
                                 int64_t head_size, const OptTensor& init_state, const OptTensor& state_map,
                                 bool with_state) {
-  TORCH_CHECK_VALUE(r.dim() == 3, "expected [B, T, C] tensors, got ", r.sizes());
+  TORCH_CHECK_VALUE(r.dim() == 3, "expected [B, T, C] tensors, got ", r.sym_sizes());
   // bfloat16 states outside training are read and written as they are: each conversion would be a launch of its own
   const bool typed = r.scalar_type() == at::kBFloat16 && u.scalar_type() == at::kBFloat16 &&
                      (!has(init_state) || init_state->scalar_type() == at::kBFloat16) &&
                      !any_requires_grad({&r, &k, &v, &w, &u}, init_state);
-  const Wkv6Args x = wkv6_args(r, k, v, w, u, head_size, r.size(0), init_state, state_map, typed);
+  const Wkv6Args x = wkv6_args(r, k, v, w, u, head_size, r.sym_size(0), init_state, state_map, typed);
   int algo = algo_from_env("RWKV_OPS_B200_WKV6_ALGO");
   if (head_size != HEAD) {
     TORCH_CHECK_VALUE(algo != RWKVB200_ALGO_CHUNKED, "the chunked wkv6 path is built for head size 64");
     algo = RWKVB200_ALGO_RECURRENT;
   }
-  const bool keep = algo != RWKVB200_ALGO_RECURRENT && r.size(1) > 1 &&
+  const bool keep = algo != RWKVB200_ALGO_RECURRENT && r.sym_size(1) > 1 &&
                     any_requires_grad({&x.r, &x.k, &x.v, &x.w, &x.u}, x.s0);
   if (typed) algo |= RWKVB200_ALGO_TOKEN_STATES;
   auto [y, sT, kept] = RWKV_OP(wkv6_fwd, "wkv6_fwd", x.r, x.k, x.v, x.w, x.u, x.s0, x.map, algo, keep);
@@ -673,8 +684,8 @@ Three wkv6_fwd_varlen_autograd(const Tensor& r, const Tensor& k, const Tensor& v
 std::tuple<Tensor, Tensor> wkv6_varlen(const Tensor& r, const Tensor& k, const Tensor& v, const Tensor& w,
                                        const Tensor& u, const Tensor& seq_start, const Tensor& seq_len, int64_t max_len,
                                        const OptTensor& init_state, const OptTensor& state_map) {
-  TORCH_CHECK_VALUE(r.dim() == 3 && r.size(0) == 1, "expected packed token tensors [1, total_len, H*64], got ", r.sizes());
-  const Wkv6Args x = wkv6_args(r, k, v, w, u, HEAD, seq_start.numel(), init_state, state_map);
+  TORCH_CHECK_VALUE(r.dim() == 3 && r.sym_size(0) == 1, "expected packed token tensors [1, total_len, H*64], got ", r.sym_sizes());
+  const Wkv6Args x = wkv6_args(r, k, v, w, u, HEAD, seq_start.sym_numel(), init_state, state_map);
   const bool keep = any_requires_grad({&x.r, &x.k, &x.v, &x.w, &x.u}, x.s0);
   auto [y, sT, kept] = RWKV_OP(wkv6_fwd_varlen, "wkv6_fwd_varlen", x.r, x.k, x.v, x.w, x.u, seq_start, seq_len, max_len,
                                x.s0, x.map, keep);
