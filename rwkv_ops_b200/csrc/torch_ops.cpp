@@ -23,6 +23,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
+#include <torch/csrc/autograd/autograd_not_implemented_fallback.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/library.h>
 
@@ -740,4 +741,7 @@ TORCH_LIBRARY_IMPL(rwkv_ops_b200, Autograd, m) {
   m.impl("rwkv7_fused_fwd", rwkv7_fused_fwd_autograd);
   m.impl("wkv6_fwd", wkv6_fwd_autograd);
   m.impl("wkv6_fwd_varlen", wkv6_fwd_varlen_autograd);
+  // a gradient can be asked for with create_graph, but differentiating it again is an error, not a silent zero
+  for (const char* name : {"rwkv7_bwd", "rwkv7_bwd_varlen", "rwkv7_fused_bwd", "wkv6_bwd", "wkv6_bwd_varlen"})
+    m.impl(name, torch::autograd::autogradNotImplementedFallback());
 }
