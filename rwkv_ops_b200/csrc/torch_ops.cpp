@@ -27,8 +27,11 @@
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/library.h>
 
+#include <algorithm>
+#include <cctype>
 #include <cstdlib>
 #include <cstring>
+#include <limits>
 #include <strings.h>
 #include <string>
 #include <tuple>
@@ -92,7 +95,14 @@ int algo_from_env(const char* name) {
 // Largest per-call tile store that a training forward may hand to its backward: RWKV_OPS_B200_KEEP_LIMIT_MB when
 // set, else a quarter of the device's memory.
 size_t keep_limit_bytes(int device) {
-  if (const char* env = std::getenv("RWKV_OPS_B200_KEEP_LIMIT_MB")) return (size_t)std::strtoull(env, nullptr, 10) << 20;
+  if (const char* env = std::getenv("RWKV_OPS_B200_KEEP_LIMIT_MB")) {
+    char* end = nullptr;
+    const long long mb = std::strtoll(env, &end, 10);
+    while (std::isspace((unsigned char)*end)) ++end;
+    TORCH_CHECK_VALUE(end != env && !*end, "RWKV_OPS_B200_KEEP_LIMIT_MB must be a whole number, got ", env);
+    constexpr long long most = std::numeric_limits<long long>::max() >> 20;      // 8 exabytes
+    return mb < 0 ? 0 : (size_t)std::min(mb, most) << 20;                        // (strtoll saturates)
+  }
   return (size_t)at::cuda::getDeviceProperties(device)->totalGlobalMem / 4;
 }
 

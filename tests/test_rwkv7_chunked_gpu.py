@@ -146,3 +146,20 @@ def test_cfg2_full_size_padded_with_state():
         errs = {n: rel_l2(g[n].grad[b:b + 1, :, h:h + 1], gr) for n, gr in zip("rwkvab", grads[:6])}
         errs["h0"] = rel_l2(h0.grad[b:b + 1, h:h + 1], grads[6])
         assert all(e < 2e-2 for e in errs.values()), errs
+
+
+@pytest.mark.parametrize("limit,kept", [("64", True), (" 64 ", True), ("0", False), ("-1", False), ("99999999999999999999", True)])
+def test_keep_limit_values(limit, kept, monkeypatch):
+    """The limit on what a training forward holds for its backward is a whole number of MiB of any size and sign."""
+    d = rwkv7_inputs(2, 130, 3, dtype=torch.bfloat16, seed=3, device="cuda")
+    x = [d[n].requires_grad_(True) for n in "rwkvab"]
+    monkeypatch.setenv("RWKV_OPS_B200_KEEP_LIMIT_MB", limit)
+    before = torch.cuda.memory_allocated()
+    o, s = ro.generalized_delta_rule(*x)
+    outputs = o.numel() * 2 + s.numel() * 4
+    held = torch.cuda.memory_allocated() - before - outputs
+    assert (held > 2 * 3 * 3 * 16 * 8192) == kept      # 16 tiles of 8 KB for each of the three chunks of six units
+    for wrong in ("abc", "", "1.5", "64k"):
+        monkeypatch.setenv("RWKV_OPS_B200_KEEP_LIMIT_MB", wrong)
+        with pytest.raises(ValueError):
+            ro.generalized_delta_rule(*x)
