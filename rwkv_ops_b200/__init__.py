@@ -17,8 +17,11 @@ from .fused import generalized_delta_rule_fused
 
 from . import _ops
 
-if _ops.built():      # register the operators now, so that tracing finds them; an unbuilt package raises at the first call
-    _ops.load()
+if _ops.built():      # register the operators now, so that tracing finds them
+    try:
+        _ops.load()
+    except _ops.RwkvB200Error:
+        pass          # a library that does not load here (built against another torch, say) raises at the first call
 
 __version__ = "0.1"
 

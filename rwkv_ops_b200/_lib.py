@@ -86,9 +86,14 @@ def load() -> ctypes.CDLL:
             f"{LIB_PATH} not found. Build it with `python -m rwkv_ops_b200.build` (needs nvcc); "
             "rwkv_ops_b200 has no CPU or eager fallback."
         )
-    lib = ctypes.CDLL(LIB_PATH, mode=ctypes.RTLD_GLOBAL)      # the torch operators' library resolves against it
+    try:
+        lib = ctypes.CDLL(LIB_PATH, mode=ctypes.RTLD_GLOBAL)      # the torch operators' library resolves against it
+    except OSError as e:
+        raise RwkvB200Error(f"{LIB_PATH} does not load: {e}") from e
     for name, (res, args) in SIGNATURES.items():
-        fn = getattr(lib, name)  # AttributeError if the library does not export a declared symbol
+        if not hasattr(lib, name):
+            raise RwkvB200Error(f"{LIB_PATH} does not export {name}; rebuild it with `python -m rwkv_ops_b200.build`")
+        fn = getattr(lib, name)
         fn.restype = res
         fn.argtypes = args
     got = lib.rwkvb200_abi_version()

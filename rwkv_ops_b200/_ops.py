@@ -10,6 +10,7 @@ import os
 import torch
 
 from . import _lib
+from ._lib import RwkvB200Error
 
 OPS_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "librwkv_ops_b200_torch.so")
 
@@ -21,9 +22,13 @@ def load():
     if _ops is None:
         _lib.load()      # the C ABI the operators call
         if not os.path.exists(OPS_PATH):
-            raise _lib.RwkvB200Error(f"{OPS_PATH} not found. Build it with `python -m rwkv_ops_b200.build`; "
+            raise RwkvB200Error(f"{OPS_PATH} not found. Build it with `python -m rwkv_ops_b200.build`; "
                                      "rwkv_ops_b200 has no eager fallback.")
-        torch.ops.load_library(OPS_PATH)
+        try:
+            torch.ops.load_library(OPS_PATH)
+        except OSError as e:
+            raise RwkvB200Error(f"{OPS_PATH} does not load with torch {torch.__version__}; rebuild it with "
+                                f"`python -m rwkv_ops_b200.build`: {e}") from e
         _register_fakes()
         _ops = torch.ops.rwkv_ops_b200
     return _ops
@@ -37,7 +42,7 @@ def failed(error: Exception) -> Exception:
     """What to raise for an operator call that failed on valid arguments."""
     text = str(error)
     if type(error) is RuntimeError and text.startswith("rwkv_ops_b200 "):
-        return _lib.RwkvB200Error(text.splitlines()[0])
+        return RwkvB200Error(text.splitlines()[0])
     return error
 
 

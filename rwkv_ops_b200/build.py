@@ -101,7 +101,11 @@ def build_torch(force: bool = False) -> str:
 
     src = os.path.join(CSRC, "torch_ops.cpp")
     newest = max(os.path.getmtime(src), *(os.path.getmtime(h) for h in glob.glob(os.path.join(INCLUDE, "*.h"))))
-    if not force and os.path.exists(TORCH_LIB) and os.path.getmtime(TORCH_LIB) >= newest:
+    # what it was built against, beside the objects: another torch needs another build, whatever the file times say
+    stamp = os.path.join(BUILD, "torch_ops.built_with")
+    built_with = f"{torch.__version__} {torch.__file__}\n"
+    if not force and os.path.exists(TORCH_LIB) and os.path.getmtime(TORCH_LIB) >= newest and os.path.exists(stamp) \
+            and open(stamp).read() == built_with:
         return TORCH_LIB
     cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))), "include")
     root = os.path.dirname(torch.__file__)
@@ -112,6 +116,9 @@ def build_torch(force: bool = False) -> str:
     p = subprocess.run(cmd, capture_output=True, text=True)
     if p.returncode != 0:
         raise RuntimeError("g++ failed on torch_ops.cpp:\n" + p.stdout + p.stderr)
+    os.makedirs(BUILD, exist_ok=True)
+    with open(stamp, "w") as f:
+        f.write(built_with)
     return TORCH_LIB
 
 
