@@ -575,16 +575,18 @@ struct ScanSmem {
   uint32_t tmem_base;
 };
 
-// A marked unit again, by the exact recurrence: 64 threads per 16 rows, in place of what the chunks gave (inside the scan
-// kernels, because a launch of its own over all units costs every call 2 us of device time and as much on the host).
-__device__ __forceinline__ void exact_unit(r7rec::FwdArgs<bf16> args, unsigned char* smem, int tid, int unit, int hi, int brow,
+// A marked unit again, by the exact recurrence: 256 threads, half of them holding two rows each, in place of what the chunks
+// gave (inside the scan kernels, because a launch of its own over all units costs every call 2 us of device time and as much
+// on the host).  Out of line: it would only take registers from the loop over the chunks.
+__device__ __noinline__ void exact_unit(r7rec::FwdArgs<bf16> args, unsigned char* smem, int tid, int unit, int hi, int brow,
                                            int tb, int Tn, const float* h0, int n_state, float* ht, const TokLayout& lay) {
   args.base = brow * lay.sb + hi * lay.sh + tb * lay.st;
   args.Tn = Tn;
   args.S0 = n_state > 0 ? h0 + (size_t)(n_state == 1 ? hi : unit) * 4096 : nullptr;
   args.ht = ht ? ht + (size_t)unit * 4096 : nullptr;
-  static_assert(4 * sizeof(r7rec::FwdSmem<64>) <= sizeof(ScanSmem), "the recurrence runs in the scan's shared memory");
-  r7rec::fwd_rows<bf16, 64, 256>(args, reinterpret_cast<r7rec::FwdSmem<64>*>(smem)[tid >> 6], tid >> 6, tid & 63);
+  typedef r7rec::FwdSmem<64, 64, 16> Smem;
+  static_assert(sizeof(Smem) <= sizeof(ScanSmem), "the recurrence runs in the scan's shared memory");
+  r7rec::fwd_rows<bf16, 64, 64, 2, 16, 256>(args, *reinterpret_cast<Smem*>(smem), 0, tid);
 }
 
 template <bool PACKED>
@@ -1201,7 +1203,7 @@ int launch_rwkv7_chunked_fwd(const void* r, const void* w, const void* k, const 
     r7rec::FwdArgs<bf16> exact{};
     if (!fused && (o || ht))
       exact = r7rec::FwdArgs<bf16>{(const bf16*)r, (const bf16*)w, (const bf16*)k, (const bf16*)v, (const bf16*)a, (const bf16*)b,
-                                   0, lay.st, 0, nullptr, (bf16*)o, nullptr, nullptr, 1};
+                                   0, lay.st, 0, nullptr, (bf16*)o, nullptr, nullptr};
     // more sequences than SMs: two CTAs per SM
 #define R7C_LAUNCH_SCAN(KERNEL, P, THREADS, SMEM)                                                                  \
     do {                                                                                                           \

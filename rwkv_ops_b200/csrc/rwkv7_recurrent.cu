@@ -35,15 +35,15 @@ constexpr int CK = R7_CKPT;   // chunk of the backward = checkpoint interval
 // ---------------------------------------------------------------------------------------------
 // forward
 // ---------------------------------------------------------------------------------------------
-template <typename T, int N>
+template <typename T, int N, int TL>
 __global__ void __launch_bounds__(N)
 rwkv7_rec_fwd_kernel(FwdArgs<T> args, const float* __restrict__ h0, int n_state, float* __restrict__ ht, int H, TokLayout lay) {
-  __shared__ __align__(16) FwdSmem<N> sm;
+  __shared__ __align__(16) FwdSmem<N, VS, TL> sm;
   const int unit = blockIdx.x, bi = unit / H, hi = unit % H;
   args.base = bi * lay.sb + hi * lay.sh;
   args.S0 = h0 && n_state > 0 ? h0 + (long long)(n_state == 1 ? hi : unit) * N * N : nullptr;
   args.ht = ht ? ht + (long long)unit * N * N : nullptr;
-  fwd_rows<T, N, N>(args, sm, blockIdx.y, threadIdx.x);
+  fwd_rows<T, N, VS, 1, TL, N>(args, sm, VS * blockIdx.y, threadIdx.x);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -86,10 +86,10 @@ rwkv7_rec_bwd_kernel(const T* __restrict__ r, const T* __restrict__ w, const T* 
   ckpt += unit * (sel.ckpt_unit_stride ? sel.ckpt_unit_stride : (long long)((Tn_dense + CK - 1) / CK) * N * N);
   // The forward over this CTA's rows, for its checkpoints: every thread stores the very values that it loads below.
   {
-    static_assert(sizeof(FwdSmem<N>) <= sizeof(BwdSmem<N>), "the forward's tiles live in the backward's shared memory");
+    static_assert(sizeof(FwdSmem<N, VS, 16>) <= sizeof(BwdSmem<N>), "the forward's tiles live in the backward's shared memory");
     const FwdArgs<T> args{r, w, k, v, a, b, base, lay.st, Tn,
-                          n_state > 0 ? h0 + (long long)(n_state == 1 ? hi : unit) * N * N : nullptr, nullptr, nullptr, ckpt, CK};
-    fwd_rows<T, N, N>(args, *reinterpret_cast<FwdSmem<N>*>(smem_raw), y, tid);
+                          n_state > 0 ? h0 + (long long)(n_state == 1 ? hi : unit) * N * N : nullptr, nullptr, nullptr, ckpt};
+    fwd_rows<T, N, VS, 1, 16, N>(args, *reinterpret_cast<FwdSmem<N, VS, 16>*>(smem_raw), VS * y, tid);
     __syncthreads();
   }
 
@@ -284,8 +284,8 @@ int launch_rwkv7_rec_step(const void* r, const void* w, const void* k, const voi
   ProfScope prof("rwkv7_rec_fwd_kernel", st);
   RWKVB200_DISPATCH_DTYPE(dtype,
     const FwdArgs<T> args{(const T*)r, (const T*)w, (const T*)k, (const T*)v, (const T*)a, (const T*)b, 0, lay.st, 1,
-                          nullptr, (T*)o, nullptr, nullptr, 1};
-    rwkv7_rec_fwd_kernel<T, N><<<dim3(B * H, N / VS), N, 0, st>>>(args, h0, n_state, ht, H, lay));
+                          nullptr, (T*)o, nullptr, nullptr};
+    rwkv7_rec_fwd_kernel<T, N, 1><<<dim3(B * H, N / VS), N, 0, st>>>(args, h0, n_state, ht, H, lay));
   return check_launch();
 }
 
@@ -296,8 +296,8 @@ int launch_rwkv7_rec_fwd(const void* r, const void* w, const void* k, const void
   const TokLayout lay(Tn, H, head_first);
   ProfScope prof("rwkv7_rec_fwd_kernel", st);
   const FwdArgs<T> args{(const T*)r, (const T*)w, (const T*)k, (const T*)v, (const T*)a, (const T*)b, 0, lay.st, Tn,
-                        nullptr, (T*)o, nullptr, nullptr, 1};
-  rwkv7_rec_fwd_kernel<T, HS><<<dim3(B * H, HS / VS), HS, 0, st>>>(args, h0, n_state, ht, H, lay);
+                        nullptr, (T*)o, nullptr, nullptr};
+  rwkv7_rec_fwd_kernel<T, HS, 8><<<dim3(B * H, HS / VS), HS, 0, st>>>(args, h0, n_state, ht, H, lay);
   return check_launch();
 }
 

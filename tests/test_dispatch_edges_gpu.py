@@ -75,3 +75,71 @@ def test_stages_of_the_scans_for_few_sequences_wrap_around(T):
     ref = _train({n: t.float() for n, t in d.items()}, [d["d_out"].float(), d["d_state"]])
     for n in ref:
         assert rel_l2(out[n], ref[n]) < 2e-2, n
+
+
+def _recurrence(d, monkeypatch, grads):
+    monkeypatch.setenv("RWKV_OPS_B200_RWKV7_ALGO", "recurrent")
+    ref = _train(d, grads)
+    monkeypatch.delenv("RWKV_OPS_B200_RWKV7_ALGO")
+    return ref
+
+
+@pytest.mark.parametrize("many", [False, True])
+@pytest.mark.parametrize("T", [3, 7, 8, 15, 17, 33, 130])
+def test_units_recomputed_inside_both_scans(T, many, monkeypatch):
+    """Every third unit out of the range of the chunked kernels (all of them below 8 tokens), with one CTA per SM and with more
+    units than SMs: those carry the bits of the recurrence, forward and backward, and the others stay the chunked kernels'."""
+    H = 2
+    B = torch.cuda.get_device_properties(0).multi_processor_count // H + 5 if many else 5
+    d = {n: t.cuda() for n, t in rwkv7_inputs(B, T, H, dtype=torch.bfloat16, seed=50 + T, with_state=True, with_grads=True).items()}
+    grads = [d["d_out"], d["d_state"]]
+    inside = _train(d, grads)
+    # 1.9 .. 2.9 per token leaves the range (60 per 32 tokens) only where half a chunk is that long
+    fast = torch.zeros(B * H, dtype=torch.bool, device="cuda")
+    fast[1::3] = T > 8
+    w = torch.where(fast.view(B, 1, H, 1), (3.0 if T < 64 else 1.0) + 0.1 * d["w"].float(), d["w"].float()).bfloat16()
+    if 8 <= T < 16:
+        w = torch.where(fast.view(B, 1, H, 1), 3.0 + 0 * w, w)      # 15 tokens of e^3
+    d["w"] = w
+    out, ref = _train(d, grads), _recurrence(d, monkeypatch, grads)
+    exact = torch.ones_like(fast) if T < 8 else fast
+    for n in ref:
+        a, b, c = (t.view(B, -1, H, 64, 64) if n in ("s", "dh0") else t for t in (out[n], ref[n], inside[n]))
+        if n in ("s", "dh0"):
+            a, b, c = (t.permute(0, 2, 1, 3, 4).reshape(B * H, -1) for t in (a, b, c))
+        else:
+            a, b, c = (t.permute(0, 2, 1, 3).reshape(B * H, -1) for t in (a, b, c))
+        assert torch.equal(a[exact], b[exact]), n
+        assert torch.equal(a[~exact], c[~exact]), n
+
+
+def test_short_sequences_in_a_packed_batch_with_more_units_than_SMs(monkeypatch):
+    """Sequences of 1 to 9 tokens between longer ones: those below 8 carry the bits of the recurrence over the sequence alone."""
+    H, lens = 4, [1, 70, 2, 7, 8, 9, 130, 3] * 6
+    assert len(lens) * H > torch.cuda.get_device_properties(0).multi_processor_count
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    d = rwkv7_inputs(1, cu[-1], H, dtype=torch.bfloat16, seed=77, device="cuda", with_grads=True)
+    h0 = 0.1 * torch.randn(len(lens), H, 64, 64, device="cuda")
+    d_s = 0.1 * torch.randn(len(lens), H, 64, 64, device="cuda")
+
+    def run(fn, x, state, d_o, d_state):
+        x = [t.clone().requires_grad_(True) for t in x]
+        state = state.clone().requires_grad_(True)
+        o, s = fn(*x, initial_state=state)
+        return [o.detach(), s.detach(), *torch.autograd.grad([o, s], x + [state], [d_o, d_state])]
+
+    tokens = [d[n] for n in "rwkvab"]
+    out = run(lambda *x, **kw: ro.generalized_delta_rule_varlen(*x, cu, **kw), tokens, h0, d["d_out"], d_s)
+    for i, n in enumerate(lens[:8]):
+        at = slice(cu[i], cu[i] + n)
+        monkeypatch.setenv("RWKV_OPS_B200_RWKV7_ALGO", "recurrent" if n < 8 else "auto")
+        ref = run(ro.generalized_delta_rule, [t[:, at].contiguous() for t in tokens], h0[i:i + 1], d["d_out"][:, at].contiguous(), d_s[i:i + 1])
+        monkeypatch.delenv("RWKV_OPS_B200_RWKV7_ALGO")
+        for m, (a, b) in enumerate(zip(out, ref)):
+            a = a[i:i + 1] if m in (1, 8) else a[:, at]
+            if 1 < n < 8:
+                assert torch.equal(a, b), (n, m)
+            else:      # (one token alone is the decode step's kernel: other sums in float32, then perhaps another rounding)
+                assert rel_l2(a, b) < 2e-3, (n, m)
