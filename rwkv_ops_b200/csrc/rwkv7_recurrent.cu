@@ -285,6 +285,7 @@ int launch_rwkv7_rec_step(const void* r, const void* w, const void* k, const voi
   RWKVB200_DISPATCH_DTYPE(dtype,
     const FwdArgs<T> args{(const T*)r, (const T*)w, (const T*)k, (const T*)v, (const T*)a, (const T*)b, 0, lay.st, 1,
                           nullptr, (T*)o, nullptr, nullptr};
+    // (a tile of one token: 256 sequences of 16 heads 317 -> 134 us against a tile of 8)
     rwkv7_rec_fwd_kernel<T, N, 1><<<dim3(B * H, N / VS), N, 0, st>>>(args, h0, n_state, ht, H, lay));
   return check_launch();
 }
@@ -297,6 +298,7 @@ int launch_rwkv7_rec_fwd(const void* r, const void* w, const void* k, const void
   ProfScope prof("rwkv7_rec_fwd_kernel", st);
   const FwdArgs<T> args{(const T*)r, (const T*)w, (const T*)k, (const T*)v, (const T*)a, (const T*)b, 0, lay.st, Tn,
                         nullptr, (T*)o, nullptr, nullptr};
+  // tiles of 8 tokens: with 16, half as many CTAs fit an SM (B 16, T 512, 32 heads: 2269 us against 1281; 16 units 320 and 324)
   rwkv7_rec_fwd_kernel<T, HS, 8><<<dim3(B * H, HS / VS), HS, 0, st>>>(args, h0, n_state, ht, H, lay);
   return check_launch();
 }
