@@ -116,26 +116,31 @@ struct Prep {
   float sx[W][W], sxv[W][W], sy[W][W], syv[W][W];     // the scalars A, processing order; never-written entries stay 0
 };
 template <typename T, int N>
-struct SweepSmem {
-  static constexpr int GROUPS = N == 64 ? 4 : 3;
-  Stage<N> stage[GROUPS];
-  Prep<T, N> prep[GROUPS];
+struct Group {
+  Stage<N> stage;
+  Prep<T, N> prep;
 };
-template <typename T, int N> constexpr int sweep_threads() { return RV / rows_per_thread<N>() * N / 8 + N * SweepSmem<T, N>::GROUPS; }
+// Groups that prepare blocks: as many as keep up with the state warps where a CTA has its SM to itself.  A group takes 34 KB of
+// shared memory (60 at N = 128), so where there are more CTAs than SMs fewer of them let two or three CTAs share an SM and fill
+// each other's waits: B 64, T 32, 32 heads, forward 329 us with four groups, 196 with two (B 16, T 1024, 64 heads: 3385 and 2765);
+// N = 128, B 16, T 512, 16 heads: 1519 us with three, 1176 with one.  At 148 CTAs two groups lose, 48 us against 42 (T 300),
+// and so they do in float16, where two CTAs of four groups fit an SM as it is (B 16, T 512, 16 heads: 339 us and 364).
+template <int N> constexpr int FEW_CTAS = N == 64 ? 4 : 3;
+template <typename T, int N> constexpr int MANY_CTAS = N == 128 ? 1 : sizeof(T) == 4 ? 2 : FEW_CTAS<N>;
+template <int N> constexpr int state_threads() { return RV / rows_per_thread<N>() * N / 8; }
 
-template <typename T, int N, bool BWD>
-__global__ void __launch_bounds__((sweep_threads<T, N>()))
+template <typename T, int N, bool BWD, int GROUPS>
+__global__ void __launch_bounds__(state_threads<N>() + N * GROUPS)
 r7_sweep_kernel(Vecs<T> in, const T* __restrict__ v, const float* __restrict__ s_in, int n_state,
                 T* __restrict__ out, float* __restrict__ s_out, float* __restrict__ ckpt, int Tn, int H, TokLayout lay) {
-  typedef SweepSmem<T, N> Smem;
-  constexpr int GROUPS = Smem::GROUPS, ROWS = rows_per_thread<N>(), NCONS = RV / ROWS * N / 8;
+  constexpr int ROWS = rows_per_thread<N>(), NCONS = state_threads<N>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
+  Group<T, N>* const group = reinterpret_cast<Group<T, N>*>(smem_raw);
   const int unit = blockIdx.x, ys = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
   const int bi = unit / H, hi = unit % H;
   const long long base = bi * lay.sb + hi * lay.sh;
   const int NB = (Tn + W - 1) / W;
-  const int FULL = 1 + GROUPS, EMPTY = 1 + 2 * GROUPS;      // named barriers: 1.. within a group, then these
+  constexpr int FULL = 1 + GROUPS, EMPTY = 1 + 2 * GROUPS;      // named barriers: 1.. within a group, then these
 
   if (tid < NCONS) {
     // ---- state warps
@@ -175,7 +180,7 @@ r7_sweep_kernel(Vecs<T> in, const T* __restrict__ v, const float* __restrict__ s
     };
     for (int idx = 0, g = 0; idx < NB; ++idx, g = g + 1 == GROUPS ? 0 : g + 1) {
       const int n = BWD ? NB - 1 - idx : idx;
-      const Stage<N>& st = sm.stage[g];
+      const Stage<N>& st = group[g].stage;
       if (ckpt) {      // forward: the state before every GT tokens but the first; backward: the gradient after them, but the last
         const int m = n >> 1;
         if (!BWD && (n & 1) == 0 && m > 0) put_state(ckpt + ((long long)unit * 2 * (NG - 1) + m - 1) * N * N);
@@ -257,8 +262,8 @@ r7_sweep_kernel(Vecs<T> in, const T* __restrict__ v, const float* __restrict__ s
 
   // ---- preparing groups
   const int g = (tid - NCONS) / N, q = (tid - NCONS) % N;
-  Prep<T, N>& pr = sm.prep[g];
-  Stage<N>& st = sm.stage[g];
+  Prep<T, N>& pr = group[g].prep;
+  Stage<N>& st = group[g].stage;
   constexpr int NL = N / 4;                     // lanes per pair of source tokens below
   constexpr int EPC = 16 / sizeof(T), CPR = N / EPC, VPR = RV / EPC;     // elements per 16 bytes; copies per token row
 
@@ -773,17 +778,26 @@ r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, c
   }
 }
 
+template <typename T, int N, bool BWD, int GROUPS>
+int launch_sweep(const DeviceFacts& dev, const Vecs<T>& in, const void* v, const float* s_in, int n_state, void* out, float* s_out,
+                 float* ckpt, int B, int Tn, int H, const TokLayout& lay, cudaStream_t st) {
+  constexpr int bytes = (int)sizeof(Group<T, N>);
+  if (allow_smem<r7_sweep_kernel<T, N, BWD, GROUPS>>(dev, GROUPS * bytes)) return RWKVB200_E_CUDA;
+  const int blocks = (Tn + W - 1) / W, groups = blocks < GROUPS ? blocks : GROUPS;      // a group without a block is left out
+  ProfScope prof(BWD ? "r7_sweep_bwd_kernel" : "r7_sweep_fwd_kernel", st);
+  r7_sweep_kernel<T, N, BWD, GROUPS><<<dim3(B * H, N / RV), state_threads<N>() + N * groups, groups * bytes, st>>>(
+      in, (const T*)v, s_in, n_state, (T*)out, s_out, ckpt, Tn, H, lay);
+  return check_launch();
+}
+
 template <typename T, int N, bool BWD>
 int sweep(const Vecs<T>& in, const void* v, const float* s_in, int n_state, void* out, float* s_out, float* ckpt, int B,
           int Tn, int H, const TokLayout& lay, cudaStream_t st) {
   DeviceFacts dev;
   if (int e = device_facts(&dev)) return e;
-  const int smem = (int)sizeof(SweepSmem<T, N>);
-  if (allow_smem<r7_sweep_kernel<T, N, BWD>>(dev, smem)) return RWKVB200_E_CUDA;
-  ProfScope prof(BWD ? "r7_sweep_bwd_kernel" : "r7_sweep_fwd_kernel", st);
-  r7_sweep_kernel<T, N, BWD><<<dim3(B * H, N / RV), sweep_threads<T, N>(), smem, st>>>(in, (const T*)v, s_in, n_state, (T*)out, s_out,
-                                                                                  ckpt, Tn, H, lay);
-  return check_launch();
+  return B * H * (N / RV) > dev.sms
+             ? launch_sweep<T, N, BWD, MANY_CTAS<T, N>>(dev, in, v, s_in, n_state, out, s_out, ckpt, B, Tn, H, lay, st)
+             : launch_sweep<T, N, BWD, FEW_CTAS<N>>(dev, in, v, s_in, n_state, out, s_out, ckpt, B, Tn, H, lay, st);
 }
 
 template <typename T, int N>

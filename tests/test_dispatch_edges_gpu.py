@@ -143,3 +143,16 @@ def test_short_sequences_in_a_packed_batch_with_more_units_than_SMs(monkeypatch)
                 assert torch.equal(a, b), (n, m)
             else:      # (one token alone is the decode step's kernel: other sums in float32, then perhaps another rounding)
                 assert rel_l2(a, b) < 2e-3, (n, m)
+
+
+@pytest.mark.parametrize("K", [64, 128])
+@pytest.mark.parametrize("T", [1, 8, 9, 16, 17, 24, 33, 75])
+def test_token_blocks_with_more_units_than_SMs(K, T):
+    """Fewer preparing groups per CTA, down to one, and as many as there are blocks: the same bits as with few units."""
+    d = rwkv7_inputs(1, T, 2, K, dtype=torch.float32, seed=40 + T, device="cuda", with_state=True, with_grads=True)
+    few = _train(d, [d["d_out"], d["d_state"]])
+    B = torch.cuda.get_device_properties(0).multi_processor_count // (K // 8) + 2
+    big = {n: t.expand(B, *t.shape[1:]).contiguous() for n, t in d.items()}
+    many = _train(big, [big["d_out"], big["d_state"]])
+    for n in few:
+        assert torch.equal(many[n], few[n].expand_as(many[n])), n
