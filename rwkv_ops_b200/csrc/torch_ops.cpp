@@ -23,8 +23,9 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
-#include <torch/csrc/autograd/autograd_not_implemented_fallback.h>
 #include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/functions/utils.h>
 #include <torch/library.h>
 
 #include <algorithm>
@@ -703,6 +704,38 @@ std::tuple<Tensor, Tensor> wkv6_varlen(const Tensor& r, const Tensor& k, const T
   return {y.to(r.scalar_type()), sT.to(state_dtype(r.scalar_type()))};
 }
 
+// ---------------------------------------------------------------------------------------------
+// the backward operators under autograd: a gradient can be asked for with create_graph, but differentiating it again is an
+// error, not a silent zero
+// ---------------------------------------------------------------------------------------------
+constexpr char RWKV7_BWD[] = "rwkv_ops_b200::rwkv7_bwd", RWKV7_BWD_VARLEN[] = "rwkv_ops_b200::rwkv7_bwd_varlen",
+               RWKV7_FUSED_BWD[] = "rwkv_ops_b200::rwkv7_fused_bwd", WKV6_BWD[] = "rwkv_ops_b200::wkv6_bwd",
+               WKV6_BWD_VARLEN[] = "rwkv_ops_b200::wkv6_bwd_varlen";
+
+void differentiable_inputs(Vars& to, const Tensor& x) { if (x.defined() && x.requires_grad()) to.push_back(x); }
+void differentiable_inputs(Vars& to, const OptTensor& x) { if (has(x)) differentiable_inputs(to, *x); }
+template <typename X> void differentiable_inputs(Vars&, const X&) {}
+
+template <const char* NAME, auto F> struct Gradient;
+template <const char* NAME, typename R, typename... A, R (*F)(A...)>
+struct Gradient<NAME, F> {
+  static R call(A... args) {
+    static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow(NAME, "").template typed<R(A...)>();
+    Vars from;
+    if (at::GradMode::is_enabled()) (differentiable_inputs(from, args), ...);
+    R out = [&] {
+      at::AutoDispatchBelowADInplaceOrView below;
+      return op.call(args...);
+    }();
+    if (!from.empty()) {
+      auto node = std::make_shared<torch::autograd::NotImplemented>(NAME);
+      node->set_next_edges(torch::autograd::collect_next_edges(from));
+      std::apply([&](auto&... x) { (torch::autograd::set_history(x, node), ...); }, out);
+    }
+    return out;
+  }
+};
+
 }  // namespace
 
 TORCH_LIBRARY(rwkv_ops_b200, m) {
@@ -751,7 +784,9 @@ TORCH_LIBRARY_IMPL(rwkv_ops_b200, Autograd, m) {
   m.impl("rwkv7_fused_fwd", rwkv7_fused_fwd_autograd);
   m.impl("wkv6_fwd", wkv6_fwd_autograd);
   m.impl("wkv6_fwd_varlen", wkv6_fwd_varlen_autograd);
-  // a gradient can be asked for with create_graph, but differentiating it again is an error, not a silent zero
-  for (const char* name : {"rwkv7_bwd", "rwkv7_bwd_varlen", "rwkv7_fused_bwd", "wkv6_bwd", "wkv6_bwd_varlen"})
-    m.impl(name, torch::autograd::autogradNotImplementedFallback());
+  m.impl("rwkv7_bwd", Gradient<RWKV7_BWD, rwkv7_bwd>::call);
+  m.impl("rwkv7_bwd_varlen", Gradient<RWKV7_BWD_VARLEN, rwkv7_bwd_varlen>::call);
+  m.impl("rwkv7_fused_bwd", Gradient<RWKV7_FUSED_BWD, rwkv7_fused_bwd>::call);
+  m.impl("wkv6_bwd", Gradient<WKV6_BWD, wkv6_bwd>::call);
+  m.impl("wkv6_bwd_varlen", Gradient<WKV6_BWD_VARLEN, wkv6_bwd_varlen>::call);
 }
