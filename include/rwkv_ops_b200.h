@@ -74,7 +74,7 @@ enum {
    * = the whole call.  The parts of one call must run in order on the same workspace with the same
    * arguments.  Forward: PREPARE does everything that does not depend on the initial state (h0, o and ht
    * are not touched and o may be NULL), SCAN walks the state through the chunks and writes o and ht.
-   * Backward: PREPARE does what does not depend on d_ht, SCAN carries the state gradient back through the
+   * Backward: PREPARE recomputes the forward's tiles (nothing is left to do there with RWKVB200_ALGO_KEEP), SCAN carries the state gradient back through the
    * chunks and writes d_h0, FINISH writes the six token gradients (pass the same gradient buffers to every
    * part: for units beyond the decay range SCAN already runs the recurrence, which writes into them, so that
    * their share of d_h0 is exact when SCAN returns).  A caller that splits one sequence over

@@ -121,17 +121,6 @@ def load_dev() -> ctypes.CDLL:
     return lib
 
 
-def check_status(what: str) -> None:
-    """With ``RWKV_OPS_B200_CHECK_STATUS=1``: synchronise and raise if a bounded wait inside a tensor-core
-    kernel ran out during ``what`` (the kernel then wound down and its results are not valid).  Off by
-    default, because it synchronises the device after every operator call."""
-    if os.environ.get("RWKV_OPS_B200_CHECK_STATUS", "0") not in ("", "0"):
-        code = load().rwkvb200_device_status(1)
-        if code != 0:
-            raise RwkvB200Error(f"{what}: a bounded wait inside a tensor-core kernel ran out (code {code}); "
-                                "the results of this call are not valid")
-
-
 def _a256(x: int) -> int:
     return (x + 255) & ~255
 

@@ -124,19 +124,21 @@ __device__ __noinline__ void store_tile_rows(__nv_bfloat16* dst, long long st, c
 struct Workspace {
   unsigned char* tiles;   // [n_chunks_total][tiles_per_chunk][8192]
   float* aux;             // [n_chunks_total][128]
-  int* flags;             // [B*H] nonzero: the unit's decay left the range of the scaled operands (DECAY_LIMIT)
+  int* flags;             // [B*H] nonzero: the unit's decay left the range of the scaled operands (DECAY_LIMIT); written by
+                          // the forward scan, from the signs of the e^{glast-gref} in aux
   int tiles_per_chunk;
 };
 
 // The scaled operands carry e^{+-(gi - gref)}: with the reference point in the middle of the chunk the
 // exponent of a channel reaches the sum of |g| over half a chunk.  Up to DECAY_LIMIT every factor and every
 // scaled state entry stays a normal bfloat16 / float32 number and the chunk equations are exact; a
-// (batch, head) unit with a larger half-chunk sum in any channel is marked in Workspace::flags by the intra
-// kernel and recomputed afterwards by the float32 recurrence (rwkv7_recurrent.cu), so the operator never
+// chunk with a larger half-chunk sum in a channel has that channel's e^{glast-gref} negated by the intra kernel, and a
+// (batch, head) unit with such a chunk is recomputed by the float32 recurrence (rwkv7_recurrent.cuh: its outputs by the
+// forward scan, which gathers the marks into Workspace::flags, its gradients by those flags), so the operator never
 // returns values computed from clamped exponents.  |g| <= 1.875 per token never reaches the limit; RWKV7's
 // own parametrisation keeps |g| below 0.61.
 constexpr float DECAY_LIMIT = 60.f;
-// Sequences shorter than this are recomputed by the recurrence as well (marked in the same flags): with one or
+// Sequences shorter than this are recomputed by the recurrence as well (marked the same way): with one or
 // two tokens the decay gradient is what is left of sums over the whole chunk that cancel almost completely
 // (exactly zero for one token and no initial state), so the bfloat16 roundings of the chunk products would be all
 // there is in dw; the recurrence costs nothing at that length.
@@ -167,7 +169,7 @@ inline Workspace carve(void* ws, int B, int T, int H, int tiles_per_chunk) {
 // a sequence over several GPUs runs the state-independent phase on every GPU at once and only the scans one GPU
 // after the other (the workspace carries everything from one phase to the next).
 //   forward:  PREPARE = intra-chunk kernel;            SCAN = state scan over the chunks (+ exact fallback)
-//   backward: PREPARE = (forward recomputation and) the state-independent products of the reverse scan;
+//   backward: PREPARE = forward recomputation (nothing, when the forward left its tiles);
 //             SCAN = reverse scan (gradient of the state);   FINISH = token gradients (+ exact fallback)
 enum Phase { PHASE_PREPARE = 1, PHASE_SCAN = 2, PHASE_FINISH = 4, PHASE_ALL = 7 };
 

@@ -226,7 +226,7 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   const bool tok_lane = lane < 16;            // lower lane halves hold token rows, upper halves state rows
 
   if (tid == 0) {
-    // MMA batch 1 has three accumulators and three issuing threads (0, 32, 64) and completes with all arrivals
+    // MMA batch 1 has three accumulators and three issuing threads (of warps 0, 1, 2) and completes with all arrivals
     mbar_init(&sm.bar_1, 3); mbar_init(&sm.bar_2, 1); mbar_init(&sm.bar_in, 1);
     fence_mbar_init();
   }
@@ -599,7 +599,7 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   float* red_x = stage_dw;                     // X k~ per (token, channel), read before dw is staged over it
 
   if (tid == 0) {
-    // every MMA batch is issued by two threads (threads 0 and 32, each with accumulators of its own) and completes
+    // every MMA batch is issued by two threads (of warps 0 and 1, each with accumulators of its own) and completes
     // with the arrival of both
     mbar_init(&sm.bar_1, 2); mbar_init(&sm.bar_2, 2); mbar_init(&sm.bar_2a, 2);
     mbar_init(&sm.bar_in_a, 1); mbar_init(&sm.bar_in_b, 1); mbar_init(&sm.bar_in_c, 1); mbar_init(&sm.bar_s, 1);
@@ -765,7 +765,6 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
       for (int j = 0; j < PL; ++j) sm.gs[(PL * part + j) * NROW + ch] = gv[j] + add;
     }
     __syncthreads();
-    W6C_STAMP(34);
     W6C_STAMP(35);
     // ---- pass RK: scaled r, k (split, written over the raw rows once every thread has its elements) and
     // the diagonal term
