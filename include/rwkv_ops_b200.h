@@ -195,6 +195,30 @@ int rwkvb200_rwkv7_bwd(const void* r, const void* w, const void* k, const void* 
                        int B, int T, int H, int head_size, int dtype, int head_first, int algo,
                        void* stream);
 
+/* The forward and backward of a training step through the float32 recurrence, where the backward starts from states that
+ * the forward has left instead of sweeping forward once more.  `states`: rwkvb200_rwkv7_states_bytes of device memory, the
+ * state after every 16th token; the backward reads it, and its workspace is of the same size.  That size is 0 where there
+ * is nothing to leave (up to 16 tokens, the chunked path, bfloat16 at head size 64): use the plain backward there, this
+ * one returns RWKVB200_E_UNSUPPORTED.  Same results as rwkvb200_rwkv7_fwd / _bwd. */
+size_t rwkvb200_rwkv7_states_bytes(int B, int T, int H, int head_size, int dtype, int algo);
+
+int rwkvb200_rwkv7_fwd_states(const void* r, const void* w, const void* k, const void* v,
+                              const void* a, const void* b,
+                              const float* h0, int n_state, void* o, float* ht,
+                              float* states, size_t states_bytes,
+                              int B, int T, int H, int head_size, int dtype, int head_first, int algo,
+                              void* stream);
+
+int rwkvb200_rwkv7_bwd_states(const void* r, const void* w, const void* k, const void* v,
+                              const void* a, const void* b,
+                              const float* h0, int n_state,
+                              const void* d_o, const float* d_ht,
+                              const float* states, size_t states_bytes,
+                              void* dr, void* dw, void* dk, void* dv, void* da, void* db, float* d_h0,
+                              void* workspace, size_t workspace_bytes,
+                              int B, int T, int H, int head_size, int dtype, int head_first, int algo,
+                              void* stream);
+
 /* Backward without a workspace argument, for callers that cannot allocate device memory.
  * No counterpart in the reference.  It is the float32 recurrent backward (RWKVB200_ALGO_RECURRENT)
  * with the same inputs, outputs and results as rwkvb200_rwkv7_bwd, but its state checkpoints live in

@@ -44,6 +44,9 @@ SIGNATURES = {
     "rwkvb200_rwkv7_fwd": (c_int, [_P] * 6 + [_P, _I, _P, _P, _P, _Z] + [_I] * 7 + [_P]),
     "rwkvb200_rwkv7_bwd_workspace_bytes": (c_size_t, [_I] * 6),
     "rwkvb200_rwkv7_bwd": (c_int, [_P] * 6 + [_P, _I, _P, _P] + [_P] * 7 + [_P, _Z] + [_I] * 7 + [_P]),
+    "rwkvb200_rwkv7_states_bytes": (c_size_t, [_I] * 6),
+    "rwkvb200_rwkv7_fwd_states": (c_int, [_P] * 6 + [_P, _I, _P, _P, _P, _Z] + [_I] * 7 + [_P]),
+    "rwkvb200_rwkv7_bwd_states": (c_int, [_P] * 6 + [_P, _I, _P, _P, _P, _Z] + [_P] * 7 + [_P, _Z] + [_I] * 7 + [_P]),
     "rwkvb200_rwkv7_bwd_static_capacity_bytes": (c_size_t, []),
     "rwkvb200_rwkv7_bwd_static": (c_int, [_P] * 6 + [_P, _I, _P, _P] + [_P] * 7 + [_I] * 6 + [_P]),
     "rwkvb200_wkv6_fwd_workspace_bytes": (c_size_t, [_I] * 6),
@@ -131,6 +134,11 @@ def rwkv7_kept_bytes(n_seq: int, max_len: int, H: int) -> int:
     functions of the custom ops must run without a device)."""
     n = n_seq * H * ((max_len + 63) // 64)
     return _a256(n * 16 * 8192) + _a256(n * 128 * 4) + _a256(n_seq * H * 4) + 1024
+
+
+def rwkv7_states_bytes(B: int, T: int, H: int, K: int) -> int:
+    """Likewise for ``rwkvb200_rwkv7_states_bytes``: the states of the float32 recurrence between every 16 tokens."""
+    return B * H * ((T + 15) // 16 - 1) * K * K * 4
 
 
 def wkv6_kept_bytes(B: int, T: int, H: int) -> int:

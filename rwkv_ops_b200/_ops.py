@@ -65,7 +65,9 @@ def _register_fakes():
     @fake("rwkv_ops_b200::rwkv7_fwd")
     def _(r, w, k, v, a, b, h0, head_first, algo, keep):
         B, T, H, K = dims(r, head_first)
-        return torch.empty_like(r), state(r, B, H, K), kept(r, _lib.rwkv7_kept_bytes(B, T, H) if keep else 0)
+        tiles = K == 64 and r.dtype == torch.bfloat16 and algo & 0xff != _lib.ALGO_RECURRENT
+        n = 0 if not keep else _lib.rwkv7_kept_bytes(B, T, H) if tiles else _lib.rwkv7_states_bytes(B, T, H, K)
+        return torch.empty_like(r), state(r, B, H, K), kept(r, n)
 
     @fake("rwkv_ops_b200::rwkv7_bwd")
     def _(r, w, k, v, a, b, h0, d_o, d_ht, k_, head_first, algo):

@@ -201,6 +201,57 @@ int rwkvb200_rwkv7_bwd(const void* r, const void* w, const void* k, const void* 
   }
 }
 
+// ---- a training step of the float32 recurrence whose backward starts from states the forward has left
+size_t rwkvb200_rwkv7_states_bytes(int B, int T, int H, int head_size, int dtype, int algo) {
+  if (check_common(B, T, H, head_size, dtype, true) || resolve_r7_algo(algo, dtype, head_size) != RWKVB200_ALGO_RECURRENT) return 0;
+  return rwkv7_block_states_bytes(B, T, H, dtype, head_size);
+}
+
+int rwkvb200_rwkv7_fwd_states(const void* r, const void* w, const void* k, const void* v,
+                              const void* a, const void* b,
+                              const float* h0, int n_state, void* o, float* ht,
+                              float* states, size_t states_bytes,
+                              int B, int T, int H, int head_size, int dtype, int head_first, int algo,
+                              void* stream) {
+  int e = check_common(B, T, H, head_size, dtype, true);
+  if (e) return e;
+  if (resolve_r7_algo(algo, dtype, head_size) != RWKVB200_ALGO_RECURRENT || phases_of(algo) != PHASE_ALL)
+    return RWKVB200_E_UNSUPPORTED;
+  if (!r || !w || !k || !v || !a || !b || !o) return RWKVB200_E_NULL;
+  if (n_state != 0 && n_state != 1 && n_state != B) return RWKVB200_E_SHAPE;
+  if (n_state != 0 && !h0) return RWKVB200_E_NULL;
+  const void* ps[] = {r, w, k, v, a, b, h0, o, ht, states};
+  for (const void* p : ps) if (p && !aligned16(p)) return RWKVB200_E_ALIGN;
+  const size_t need = rwkvb200_rwkv7_states_bytes(B, T, H, head_size, dtype, algo);
+  if (states_bytes < need || (need && !states)) return RWKVB200_E_WORKSPACE;
+  return launch_rwkv7_block_fwd(r, w, k, v, a, b, n_state ? h0 : nullptr, n_state, o, ht, B, T, H, dtype, head_first,
+                                (cudaStream_t)stream, head_size, need ? states : nullptr);
+}
+
+int rwkvb200_rwkv7_bwd_states(const void* r, const void* w, const void* k, const void* v,
+                              const void* a, const void* b,
+                              const float* h0, int n_state,
+                              const void* d_o, const float* d_ht,
+                              const float* states, size_t states_bytes,
+                              void* dr, void* dw, void* dk, void* dv, void* da, void* db, float* d_h0,
+                              void* workspace, size_t workspace_bytes,
+                              int B, int T, int H, int head_size, int dtype, int head_first, int algo,
+                              void* stream) {
+  int e = check_common(B, T, H, head_size, dtype, true);
+  if (e) return e;
+  const size_t need = rwkvb200_rwkv7_states_bytes(B, T, H, head_size, dtype, algo);
+  if (!need || phases_of(algo) != PHASE_ALL) return RWKVB200_E_UNSUPPORTED;      // nothing that a forward could have left
+  if (!r || !w || !k || !v || !a || !b || !d_o || !dr || !dw || !dk || !dv || !da || !db) return RWKVB200_E_NULL;
+  if (n_state != 0 && n_state != 1 && n_state != B) return RWKVB200_E_SHAPE;
+  if (n_state != 0 && !h0) return RWKVB200_E_NULL;
+  const void* ps[] = {r, w, k, v, a, b, h0, d_o, d_ht, states, dr, dw, dk, dv, da, db, d_h0, workspace};
+  for (const void* p : ps) if (p && !aligned16(p)) return RWKVB200_E_ALIGN;
+  if (states_bytes < need || !states || workspace_bytes < need || !workspace) return RWKVB200_E_WORKSPACE;
+  return launch_rwkv7_block_bwd(r, w, k, v, a, b, n_state ? h0 : nullptr, n_state, d_o, d_ht,
+                                reinterpret_cast<float*>(workspace), dr, dw, dk, dv, da, db, d_h0, B, T, H, dtype,
+                                head_first, (cudaStream_t)stream, head_size, states);
+}
+
 // ---- packed variable-length batches (chunked bf16 path only)
 size_t rwkvb200_rwkv7_varlen_workspace_bytes(int n_seq, int max_len, int H, int head_size, int keep) {
   if (check_common(n_seq, max_len, H, head_size, RWKVB200_BF16)) return 0;

@@ -203,14 +203,16 @@ int launch_rwkv7_rec_bwd(const void* r, const void* w, const void* k, const void
                          void* dr, void* dw, void* dk, void* dv, void* da, void* db, float* d_h0,
                          int B, int Tn, int H, int head_first, cudaStream_t st, const UnitSel& sel, int T_total);
 // Float32 recurrence over blocks of tokens (rwkv7_block.cu), head size 64 or 128; o and ht may be NULL.  ckpt: room for
-// a state every R7_CKPT tokens of each unit.
+// a state every R7_CKPT tokens of each unit.  states (may be NULL): rwkv7_block_states_bytes of memory in which the forward
+// leaves the states its backward starts from; a backward that is given them needs only as much for ckpt.
+size_t rwkv7_block_states_bytes(int B, int Tn, int H, int dtype, int head_size);
 int launch_rwkv7_block_fwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
                            const float* h0, int n_state, void* o, float* ht, int B, int Tn, int H, int dtype,
-                           int head_first, cudaStream_t st, int head_size = HS);
+                           int head_first, cudaStream_t st, int head_size = HS, float* states = nullptr);
 int launch_rwkv7_block_bwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
                            const float* h0, int n_state, const void* d_o, const float* d_ht, float* ckpt,
                            void* dr, void* dw, void* dk, void* dv, void* da, void* db, float* d_h0, int B, int Tn, int H,
-                           int dtype, int head_first, cudaStream_t st, int head_size = HS);
+                           int dtype, int head_first, cudaStream_t st, int head_size = HS, const float* states = nullptr);
 constexpr int R7_CKPT = 8;   // tokens between state checkpoints of the recurrent backward
 
 int launch_wkv6_fwd(const void* r, const void* k, const void* v, const void* w, const void* u,

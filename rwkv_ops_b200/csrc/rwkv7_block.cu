@@ -183,8 +183,8 @@ r7_sweep_kernel(Vecs<T> in, const T* __restrict__ v, const float* __restrict__ s
       const Stage<N>& st = group[g].stage;
       if (ckpt) {      // forward: the state before every GT tokens but the first; backward: the gradient after them, but the last
         const int m = n >> 1;
-        if (!BWD && (n & 1) == 0 && m > 0) put_state(ckpt + ((long long)unit * 2 * (NG - 1) + m - 1) * N * N);
-        if (BWD && (n & 1) == 1 && m < NG - 1) put_state(ckpt + ((long long)unit * 2 * (NG - 1) + (NG - 1) + m) * N * N);
+        if (!BWD && (n & 1) == 0 && m > 0) put_state(ckpt + ((long long)unit * (NG - 1) + m - 1) * N * N);
+        if (BWD && (n & 1) == 1 && m < NG - 1) put_state(ckpt + ((long long)unit * (NG - 1) + m) * N * N);
       }
       bar_sync(FULL + g, NCONS + N);
       // the reduction leaves token jl of the thread's rows: in every lane both sa and o (N = 64: 8 lanes to a row), or sa
@@ -435,8 +435,8 @@ struct GradSmem {
 template <typename T, int N>
 __global__ void __launch_bounds__(4 * N, N == 64 ? 2 : 1)
 r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, const float* __restrict__ h0, int n_state,
-               const float* __restrict__ d_ht, const float* __restrict__ ckpt, T* __restrict__ dr, T* __restrict__ dw,
-               T* __restrict__ dk, T* __restrict__ da, T* __restrict__ db, int Tn, int H, TokLayout lay) {
+               const float* __restrict__ d_ht, const float* __restrict__ states, const float* __restrict__ d_states,
+               T* __restrict__ dr, T* __restrict__ dw, T* __restrict__ dk, T* __restrict__ da, T* __restrict__ db, int Tn, int H, TokLayout lay) {
   constexpr int NTHR = 4 * N;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   GradSmem<N>& sm = *reinterpret_cast<GradSmem<N>*>(smem_raw);
@@ -446,9 +446,9 @@ r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, c
   const int t0 = m * GT;
   const long long base = bi * lay.sb + hi * lay.sh + (long long)t0 * lay.st;
   const int nt = min(GT, Tn - t0);
-  const float* cu = ckpt + (long long)unit * 2 * (NG - 1) * N * N;
-  const float* Sg = m > 0 ? cu + (long long)(m - 1) * N * N : n_state > 0 ? h0 + (long long)(n_state == 1 ? hi : unit) * N * N : nullptr;
-  const float* Gg = m < NG - 1 ? cu + (long long)(NG - 1 + m) * N * N : d_ht ? d_ht + (long long)unit * N * N : nullptr;
+  const long long cu = (long long)unit * (NG - 1) + m;      // this unit's boundaries lie between its groups of tokens
+  const float* Sg = m > 0 ? states + (cu - 1) * N * N : n_state > 0 ? h0 + (long long)(n_state == 1 ? hi : unit) * N * N : nullptr;
+  const float* Gg = m < NG - 1 ? d_states + cu * N * N : d_ht ? d_ht + (long long)unit * N * N : nullptr;
 
   // ---- tokens and S
   const int kq = tid % (N / 4), row0 = tid / (N / 4);      // quad of channels, token / state row (16 at a time)
@@ -802,20 +802,27 @@ int sweep(const Vecs<T>& in, const void* v, const float* s_in, int n_state, void
 
 template <typename T, int N>
 int fwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b, const float* h0, int n_state,
-        void* o, float* ht, int B, int Tn, int H, int head_first, cudaStream_t st) {
+        void* o, float* ht, float* states, int B, int Tn, int H, int head_first, cudaStream_t st) {
   const Vecs<T> in{{(const T*)r, (const T*)w, (const T*)k, (const T*)a, (const T*)b}};
-  return sweep<T, N, false>(in, v, h0, n_state, o, ht, nullptr, B, Tn, H, TokLayout(Tn, H, head_first, N), st);
+  return sweep<T, N, false>(in, v, h0, n_state, o, ht, Tn > GT ? states : nullptr, B, Tn, H, TokLayout(Tn, H, head_first, N), st);
 }
 
 template <typename T, int N>
 int bwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b, const float* h0, int n_state,
-        const void* d_o, const float* d_ht, float* ckpt, void* dr, void* dw, void* dk, void* dv, void* da, void* db, float* d_h0,
-        int B, int Tn, int H, int head_first, cudaStream_t st) {
+        const void* d_o, const float* d_ht, const float* kept, float* ckpt, void* dr, void* dw, void* dk, void* dv, void* da, void* db,
+        float* d_h0, int B, int Tn, int H, int head_first, cudaStream_t st) {
   const Vecs<T> in{{(const T*)r, (const T*)w, (const T*)k, (const T*)a, (const T*)b}};
   const TokLayout lay(Tn, H, head_first, N);
   int e = RWKVB200_OK;
-  if (Tn > GT) e = sweep<T, N, false>(in, v, h0, n_state, nullptr, nullptr, ckpt, B, Tn, H, lay, st);
-  if (!e) e = sweep<T, N, true>(in, d_o, d_ht, d_ht ? B * H : 0, dv, d_h0, ckpt, B, Tn, H, lay, st);
+  // the states between the groups of tokens: as the forward left them, or from another sweep; then their gradients
+  const float* states = kept;
+  float* d_states = ckpt;
+  if (Tn > GT && !kept) {
+    states = ckpt;
+    d_states = ckpt + (long long)B * H * ((Tn + GT - 1) / GT - 1) * N * N;
+    e = sweep<T, N, false>(in, v, h0, n_state, nullptr, nullptr, ckpt, B, Tn, H, lay, st);
+  }
+  if (!e) e = sweep<T, N, true>(in, d_o, d_ht, d_ht ? B * H : 0, dv, d_h0, Tn > GT ? d_states : nullptr, B, Tn, H, lay, st);
   if (e) return e;
   DeviceFacts dev;
   if ((e = device_facts(&dev))) return e;
@@ -823,7 +830,7 @@ int bwd(const void* r, const void* w, const void* k, const void* v, const void* 
   if (allow_smem<r7_grad_kernel<T, N>>(dev, smem)) return RWKVB200_E_CUDA;
   ProfScope prof("r7_grad_kernel", st);
   r7_grad_kernel<T, N><<<B * H * ((Tn + GT - 1) / GT), 4 * N, smem, st>>>(in, (const T*)v, (const T*)d_o, h0, h0 ? n_state : 0, d_ht,
-                                                                         ckpt, (T*)dr, (T*)dw, (T*)dk, (T*)da, (T*)db, Tn, H, lay);
+                                                                         states, d_states, (T*)dr, (T*)dw, (T*)dk, (T*)da, (T*)db, Tn, H, lay);
   return check_launch();
 }
 
@@ -836,22 +843,27 @@ int bwd(const void* r, const void* w, const void* k, const void* v, const void* 
   if (head_size == 128) { constexpr int N = 128; RWKVB200_DISPATCH_DTYPE(dtype, return CALL); }   \
   return RWKVB200_E_UNSUPPORTED;
 
+size_t rwkv7_block_states_bytes(int B, int Tn, int H, int dtype, int head_size) {
+  if (head_size == 64 && dtype == RWKVB200_BF16) return 0;      // token by token
+  return Tn > GT ? (size_t)B * H * ((Tn + GT - 1) / GT - 1) * head_size * head_size * sizeof(float) : 0;
+}
+
 int launch_rwkv7_block_fwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
                            const float* h0, int n_state, void* o, float* ht, int B, int Tn, int H, int dtype,
-                           int head_first, cudaStream_t st, int head_size) {
+                           int head_first, cudaStream_t st, int head_size, float* states) {
   if (head_size == 64 && dtype == RWKVB200_BF16)
     return launch_rwkv7_rec_fwd(r, w, k, v, a, b, h0, n_state, o, ht, B, Tn, H, head_first, st);
-  R7_BLOCK_DISPATCH((fwd<T, N>(r, w, k, v, a, b, h0, n_state, o, ht, B, Tn, H, head_first, st)))
+  R7_BLOCK_DISPATCH((fwd<T, N>(r, w, k, v, a, b, h0, n_state, o, ht, states, B, Tn, H, head_first, st)))
 }
 
 int launch_rwkv7_block_bwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
                            const float* h0, int n_state, const void* d_o, const float* d_ht, float* ckpt,
                            void* dr, void* dw, void* dk, void* dv, void* da, void* db, float* d_h0, int B, int Tn, int H,
-                           int dtype, int head_first, cudaStream_t st, int head_size) {
+                           int dtype, int head_first, cudaStream_t st, int head_size, const float* states) {
   if (head_size == 64 && dtype == RWKVB200_BF16)
     return launch_rwkv7_rec_bwd(r, w, k, v, a, b, h0, n_state, d_o, d_ht, ckpt, dr, dw, dk, dv, da, db, d_h0, B, Tn, H,
                                 head_first, st, UnitSel{}, 0);
-  R7_BLOCK_DISPATCH((bwd<T, N>(r, w, k, v, a, b, h0, n_state, d_o, d_ht, ckpt, dr, dw, dk, dv, da, db, d_h0, B, Tn, H,
+  R7_BLOCK_DISPATCH((bwd<T, N>(r, w, k, v, a, b, h0, n_state, d_o, d_ht, states, ckpt, dr, dw, dk, dv, da, db, d_h0, B, Tn, H,
                                head_first, st)))
 }
 

@@ -20,6 +20,7 @@
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContextLight.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
@@ -104,6 +105,7 @@ size_t keep_limit_bytes(int device) {
     constexpr long long most = std::numeric_limits<long long>::max() >> 20;      // 8 exabytes
     return mb < 0 ? 0 : (size_t)std::min(mb, most) << 20;                        // (strtoll saturates)
   }
+  if (c10::cuda::device_count() == 0) return std::numeric_limits<size_t>::max();      // traced where there is no device
   return (size_t)at::cuda::getDeviceProperties(device)->totalGlobalMem / 4;
 }
 
@@ -194,6 +196,16 @@ bool keep_fits(const SymDims& d, int algo, const Tensor& r) {
          keep_limit_bytes(r.device().index());
 }
 
+// The same for the states of the float32 recurrence over blocks (rwkvb200_rwkv7_states_bytes): a length stays a symbol.
+bool states_fit(const SymDims& d, const Tensor& r) {
+  return d.T > 16 && d.B * d.H * ((d.T + 15) / 16 - 1) * d.K * d.K * 4 <=
+                         (int64_t)std::min<size_t>(keep_limit_bytes(r.device().index()), std::numeric_limits<int64_t>::max());
+}
+// whether rwkv7_fwd / _bwd take the chunked path, whose kept tensor holds tiles; elsewhere it holds states
+bool chunked_rwkv7(const Dims& d, int code, int64_t algo) {
+  return d.K == HEAD && code == RWKVB200_BF16 && (algo & 0xff) != RWKVB200_ALGO_RECURRENT;
+}
+
 Three rwkv7_fwd(const Tensor& r, const Tensor& w, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& b,
                 const OptTensor& h0, bool head_first, int64_t algo, bool keep) {
   const c10::cuda::CUDAGuard guard(r.device());
@@ -203,6 +215,12 @@ Three rwkv7_fwd(const Tensor& r, const Tensor& w, const Tensor& k, const Tensor&
   if (d.T == 1 && !keep) {
     check(rwkvb200_rwkv7_step(ptr(r), ptr(w), ptr(k), ptr(v), ptr(a), ptr(b), fptr(h0), n_state_of(h0), fptr(ht), ptr(o),
                               d.B, d.H, d.K, code, stream_of(r)), "rwkv7_step");
+  } else if (keep && !chunked_rwkv7(d, code, algo)) {
+    const size_t n = rwkvb200_rwkv7_states_bytes(d.B, d.T, d.H, d.K, code, (int)algo);
+    ws = bytes(n, r);
+    check(rwkvb200_rwkv7_fwd_states(ptr(r), ptr(w), ptr(k), ptr(v), ptr(a), ptr(b), fptr(h0), n_state_of(h0), ptr(o),
+                                    fptr(ht), fptr(ws), n, d.B, d.T, d.H, d.K, code, head_first, (int)algo, stream_of(r)),
+          "rwkv7_fwd");
   } else {
     const size_t nws = rwkvb200_rwkv7_fwd_workspace_bytes(d.B, d.T, d.H, d.K, code, flags);
     if (nws) ws = bytes(nws, r);
@@ -212,8 +230,8 @@ Three rwkv7_fwd(const Tensor& r, const Tensor& w, const Tensor& k, const Tensor&
   return {o, ht, keep ? ws : bytes(0, r)};
 }
 
-// `kept` (may be empty): what a forward with keep left; it also serves as scratch, but what the forward left in it
-// is not changed, so a second backward through the same graph stays legal.
+// `kept` (may be empty): what a forward with keep left; the tiles of the chunked path also serve as scratch, but what the
+// forward left in it is not changed, so a second backward through the same graph stays legal.
 Seven rwkv7_bwd(const Tensor& r, const Tensor& w, const Tensor& k, const Tensor& v, const Tensor& a, const Tensor& b,
                 const OptTensor& h0, const Tensor& d_o, const OptTensor& d_ht, const Tensor& kept, bool head_first,
                 int64_t algo) {
@@ -223,6 +241,14 @@ Seven rwkv7_bwd(const Tensor& r, const Tensor& w, const Tensor& k, const Tensor&
   const bool have = kept.numel() > 0;
   Tensor dr = fresh_like(r), dw = fresh_like(r), dk = fresh_like(r), dv = fresh_like(r), da = fresh_like(r),
          db = fresh_like(r), dh0 = fresh({d.B, d.H, d.K, d.K}, at::kFloat, r);
+  if (have && !chunked_rwkv7(d, code, algo)) {
+    const Tensor ws = fresh_like(kept);
+    const size_t n = (size_t)kept.numel();
+    check(rwkvb200_rwkv7_bwd_states(ptr(r), ptr(w), ptr(k), ptr(v), ptr(a), ptr(b), fptr(h0), n_state_of(h0), ptr(d_o),
+                                    fptr(d_ht), fptr(kept), n, ptr(dr), ptr(dw), ptr(dk), ptr(dv), ptr(da), ptr(db), fptr(dh0),
+                                    ptr(ws), n, d.B, d.T, d.H, d.K, code, head_first, (int)algo, stream_of(r)), "rwkv7_bwd");
+    return {dr, dw, dk, dv, da, db, dh0};
+  }
   const size_t nws = have ? (size_t)kept.numel() : rwkvb200_rwkv7_bwd_workspace_bytes(d.B, d.T, d.H, d.K, code, (int)algo);
   const Tensor ws = have ? kept : nws ? bytes(nws, r) : Tensor();
   check(rwkvb200_rwkv7_bwd(ptr(r), ptr(w), ptr(k), ptr(v), ptr(a), ptr(b), fptr(h0), n_state_of(h0), ptr(d_o), fptr(d_ht),
@@ -278,9 +304,12 @@ std::tuple<Tensor, Tensor> generalized_delta_rule(const Tensor& r, const Tensor&
   const Tensor r_ = dense(r, t), w_ = dense(w, t), k_ = dense(k, t), v_ = dense(v, t), a_ = dense(a, t), b_ = dense(b, t);
   const OptTensor h0 = dense_state(initial_state);
   bool keep = false;
-  if (d.T > 1 && t == at::kBFloat16 && d.K == HEAD && algo != RWKVB200_ALGO_RECURRENT &&
-      any_requires_grad({&r_, &w_, &k_, &v_, &a_, &b_}, h0))
-    keep = keep_fits(d, algo, r);
+  if (any_requires_grad({&r_, &w_, &k_, &v_, &a_, &b_}, h0)) {
+    if (t == at::kBFloat16 && d.K == HEAD)
+      keep = d.T > 1 && algo != RWKVB200_ALGO_RECURRENT && keep_fits(d, algo, r);
+    else
+      keep = algo != RWKVB200_ALGO_CHUNKED && states_fit(d, r);
+  }
   auto [o, ht, kept] = RWKV_OP(rwkv7_fwd, "rwkv7_fwd", r_, w_, k_, v_, a_, b_, h0, head_first, algo, keep);
   return {o.to(r.scalar_type()), ht};
 }

@@ -156,3 +156,22 @@ def test_token_blocks_with_more_units_than_SMs(K, T):
     many = _train(big, [big["d_out"], big["d_state"]])
     for n in few:
         assert torch.equal(many[n], few[n].expand_as(many[n])), n
+
+
+@pytest.mark.parametrize("K,dtype", [(64, torch.float32), (64, torch.float16), (128, torch.float32), (128, torch.bfloat16)])
+@pytest.mark.parametrize("T", [16, 17, 32, 33, 70])
+def test_states_kept_for_the_backward(T, K, dtype, monkeypatch):
+    """The float32 recurrence's backward from the states its forward left (none up to 16 tokens), twice through the same graph,
+    and from a second sweep: the same bits."""
+    d = rwkv7_inputs(2, T, 3, K, dtype=dtype, seed=60 + T, device="cuda", with_state=True, with_grads=True)
+
+    def grads():
+        x = [d[n].clone().requires_grad_(True) for n in (*"rwkvab", "initial_state")]
+        out = ro.generalized_delta_rule(*x[:6], initial_state=x[6])
+        return [torch.autograd.grad(out, x, [d["d_out"], d["d_state"]], retain_graph=True) for _ in range(2)]
+
+    kept = grads()
+    monkeypatch.setenv("RWKV_OPS_B200_KEEP_LIMIT_MB", "0")
+    again = grads()
+    for a, b, c in zip(*kept, again[0]):
+        assert torch.equal(a, b) and torch.equal(a, c)

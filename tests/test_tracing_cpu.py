@@ -67,6 +67,14 @@ def test_wkv6_training_keeps_symbolic_sizes():
         assert y.requires_grad and all(_symbolic(y, (0, 1))) and all(_symbolic(s, (0,)))
 
 
+def test_float32_rwkv7_training_keeps_symbolic_sizes():
+    mode, sizes, x = _tokens(6, (2, 100, 3, 64), torch.float32)
+    with mode:
+        x[0].requires_grad_(True)
+        o, s = ro.generalized_delta_rule(*x)
+        assert o.requires_grad and all(_symbolic(o, (0, 1))) and all(_symbolic(s, (0,)))
+
+
 def test_export_with_a_dynamic_length():
     class Layer(torch.nn.Module):
         def forward(self, *x):
