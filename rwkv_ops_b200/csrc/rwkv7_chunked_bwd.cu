@@ -407,7 +407,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
                      const __grid_constant__ CUtensorMap tmap_db,
                      bf16* __restrict__ dq_rows, bf16* __restrict__ dw_rows, bf16* __restrict__ dk_rows,
                      bf16* __restrict__ dv_rows, bf16* __restrict__ da_rows, bf16* __restrict__ db_rows,
-                     SeqView sv, int H, int NT, int n_ch, TokLayout lay, int* status, long long* dbg) {
+                     SeqView sv, const __grid_constant__ WalkDims dims, TokLayout lay, int* status, long long* dbg) {
 #ifdef RWKVB200_DEVTOOLS
 #define R7C_STAMP(n) do { if (dbg && tid == 0 && blockIdx.x == gridDim.x / 2 && it == 15) dbg[n] = clock64(); } while (0)
 #else
@@ -496,27 +496,18 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     }
   };
 
-  // chunk slots past the end of a (packed) sequence are skipped
-  auto empty = [&](const ChunkPos& p) {
-    if constexpr (!PACKED) return false;      // a dense batch has no empty slots
-    return p.c * L >= sv.length<PACKED>(p.bi);
-  };
-  auto advance = [&](ChunkPos p) {
-    do { chunk_step(p, gridDim.x, NT, H); } while (p.ch < n_ch && empty(p));
-    return p;
-  };
-  ChunkPos cur = chunk_pos(blockIdx.x, NT, H);
-  if (cur.ch < n_ch && empty(cur)) cur = advance(cur);
+  const ChunkWalk<PACKED, false> walk{sv, dims};
+  ChunkPos cur = walk.first();
 
   uint4 rw[2];
-  if (cur.ch < n_ch) {
+  if (cur.ch < dims.n_ch) {
     if (warp == st_warp && elect_one()) { load_0(cur); load_1a(cur); load_sa(cur); load_2(cur); load_1b(cur); }
     load_w(cur, rw);
   }
 
   bool ok = true;
   int it = 0;
-  for (ChunkPos nxt; cur.ch < n_ch && ok; cur = nxt, ++it) {
+  for (ChunkPos nxt; cur.ch < dims.n_ch && ok; cur = nxt, ++it) {
     const int bi = cur.bi, hi = cur.hi, t0 = cur.c * L;
     const int Tn = sv.length<PACKED>(bi);
     // in a packed batch the last rows of a sequence's last chunk belong to the next sequence: such a chunk
@@ -526,8 +517,8 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     const int tt = sv.first<PACKED>(bi) + t0, br = sv.row<PACKED>(bi);
     const unsigned char* tiles = ws_tiles + (size_t)cur.ch * tiles_per_chunk * TILE_BYTES;
     const uint32_t par = it & 1;
-    nxt = advance(cur);
-    const bool more = nxt.ch < n_ch;
+    nxt = walk.after(cur);
+    const bool more = nxt.ch < dims.n_ch;
     R7C_STAMP(16);
 
     // X, straight from the workspace: the threads of the last quarter hold a row each until they have dh^
@@ -984,7 +975,7 @@ int launch_rwkv7_chunked_bwd(const void* r, const void* w, const void* k, const 
         return RWKVB200_E_CUDA;                                                                                   \
       r7c_bwd_final_kernel<P, F><<<grid, 256, smem, st>>>((const bf16*)w, tmap_w, tmap_do, tmap_v, ws.tiles, ALL_TILES, \
           tmap_out[0], tmap_out[1], tmap_out[2], tmap_out[3], tmap_out[4], tmap_out[5], (bf16*)dr, (bf16*)dw,     \
-          (bf16*)dk, (bf16*)dv, (bf16*)da, (bf16*)db, sv, H, NT, n_ch, lay, status, debug_stamp_buffer());        \
+          (bf16*)dk, (bf16*)dv, (bf16*)da, (bf16*)db, sv, WalkDims(H, NT, B, grid), lay, status, debug_stamp_buffer());        \
     } while (0)
     if (seq_start) R7C_LAUNCH_FINAL(true, false);
     else if (fused) R7C_LAUNCH_FINAL(false, true);

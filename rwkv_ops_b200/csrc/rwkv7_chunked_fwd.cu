@@ -34,7 +34,7 @@ struct IntraSmem {
   uint32_t tmem_base;
 };
 
-// Persistent: CTAs (two per SM) walk over chunk-heads ch = blockIdx.x, blockIdx.x + gridDim.x, ...
+// Persistent: CTAs (two per SM) walk over the chunk-heads, the last chunks first (ChunkWalk).
 // 256 threads: warp w reads TMEM lanes 32*(w&3).. and the two warps that share a lane window split
 // the columns (hsel = w>>2); warps 6 and 7 invert the diagonal blocks of A_ab while the other warps mask the rest of
 // MMA 1, issue MMA 2 and drain it.
@@ -51,7 +51,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
                      const __grid_constant__ CUtensorMap tmap_b,
                      const __grid_constant__ CUtensorMap tmap_v, unsigned char* __restrict__ ws_tiles,
                      float* __restrict__ ws_aux, int tiles_per_chunk,
-                     int keep_for_bwd, SeqView sv, int H, int NT, int n_ch, TokLayout lay, int* status, long long* dbg) {
+                     int keep_for_bwd, SeqView sv, const __grid_constant__ WalkDims dims, TokLayout lay, int* status, long long* dbg) {
 #ifdef RWKVB200_DEVTOOLS
 #define R7C_STAMP(n) do { if (dbg && tid == 0 && blockIdx.x == gridDim.x / 2 && it == 30) dbg[n] = clock64(); } while (0)
 #else
@@ -90,15 +90,6 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
   };
   auto load_b = [&](const ChunkPos& p) { mbar_expect_tx(&sm.bar_b, TILE_BYTES); load(reinterpret_cast<unsigned char*>(sm.gs), &tmap_b, &sm.bar_b, p); };
   auto load_v = [&](const ChunkPos& p) { mbar_expect_tx(&sm.bar_v, TILE_BYTES); load(sm.v, &tmap_v, &sm.bar_v, p); };
-  // chunk slots past the end of a (packed) sequence are skipped
-  auto empty = [&](const ChunkPos& p) {
-    if constexpr (!PACKED) return false;      // a dense batch has no empty slots
-    return p.c * L >= sv.length<PACKED>(p.bi);
-  };
-  auto advance = [&](ChunkPos p) {
-    do { chunk_step(p, gridDim.x, NT, H); } while (p.ch < n_ch && empty(p));
-    return p;
-  };
   // Ask for a chunk-head's token rows to be brought into L2, ahead of the TMA loads above.
   auto prefetch_rows = [&](const ChunkPos& p) {      // one thread
     const int tt = sv.first<PACKED>(p.bi) + p.c * L, br = sv.row<PACKED>(p.bi);
@@ -109,27 +100,27 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
     tma_prefetch_4d(&tmap_b, 0, tt, p.hi, br);
     tma_prefetch_4d(&tmap_v, 0, tt, p.hi, br);
   };
-  ChunkPos cur = chunk_pos(blockIdx.x, NT, H);
-  if (cur.ch < n_ch && empty(cur)) cur = advance(cur);
-  if (cur.ch < n_ch && warp == 0 && elect_one()) { load_w(cur); load_qka(cur); load_b(cur); }
+  const ChunkWalk<PACKED, true> walk{sv, dims};
+  ChunkPos cur = walk.first();
+  if (cur.ch < dims.n_ch && warp == 0 && elect_one()) { load_w(cur); load_qka(cur); load_b(cur); }
   // The two CTAs that share an SM would otherwise run their phases in lockstep and compete for the
   // same unit (shared-memory pipe during the triangular solve); start every other CTA half a
   // chunk-head late (unless it has a single one to do, or none: then the delay would be all it adds).
-  if ((blockIdx.x & 1) && n_ch > 2 * (int)gridDim.x) __nanosleep(6000);
+  if ((blockIdx.x & 1) && dims.n_ch > 2 * (int)gridDim.x) __nanosleep(6000);
 
   bool ok = true;
   int it = 0;
-  for (ChunkPos nxt; cur.ch < n_ch && ok; cur = nxt, ++it) {
+  for (ChunkPos nxt; cur.ch < dims.n_ch && ok; cur = nxt, ++it) {
     const int ch = cur.ch;
     int bi, hi, t0; coords(cur, bi, hi, t0);
     const int Tn = sv.length<PACKED>(bi);
     unsigned char* out_tiles = ws_tiles + (size_t)ch * tiles_per_chunk * TILE_BYTES;
     const uint32_t par = it & 1;
-    nxt = advance(cur);
+    nxt = walk.after(cur);
     const int next = nxt.ch;
 
     R7C_STAMP(0);
-    if (next < n_ch && warp == 1 && elect_one()) prefetch_rows(nxt);
+    if (next < dims.n_ch && warp == 1 && elect_one()) prefetch_rows(nxt);
     // ---- phase A: decay prefix sums (in units of log 2), thread = (channel, quarter of the chunk), straight from the
     // raw w tile.
     ok = mbar_wait(&sm.bar_b, par, status, 208) && ok;
@@ -345,7 +336,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
       }
       if (warp == 0 && elect_one()) {
         bulk_wait_read();                  // q~, k~, b~, A_qk (and the tiles kept for the backward) have left shared memory
-        if (next < n_ch) { load_w(nxt); load_qka(nxt); }      // nothing reads A_qk, q~, k~, v any more
+        if (next < dims.n_ch) { load_w(nxt); load_qka(nxt); }      // nothing reads A_qk, q~, k~, v any more
       }
     } else if (ok) {     // warps 6, 7: the diagonal 32 x 32 blocks of A_ab, inverted (fp32); warp 7 also N_BA
       // Ainv = X = (I - N)^-1, N = stril(A_ab); with A = rows 0..31, B = rows 32..63 its blocks are X_A = (I - N_AA)^-1,
@@ -447,7 +438,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
       tc_fence_after();
       umma_tile<64, 64, 0, 1, 2>(tmem_addr(tm, 0, 128), smem_u32(sm.cm), smem_u32(sm.ainv), false);
       umma_commit(&sm.bar_m4);
-      if (next < n_ch) load_b(nxt);      // the diagonal blocks have been read
+      if (next < dims.n_ch) load_b(nxt);      // the diagonal blocks have been read
     }
     ok = ok && mbar_wait(&sm.bar_m4, par, status, 209);
     tc_fence_after();
@@ -1187,7 +1178,7 @@ int launch_rwkv7_chunked_fwd(const void* r, const void* w, const void* k, const 
         return RWKVB200_E_CUDA;                                                                                    \
       r7c_intra_fwd_kernel<P, F><<<grid, 256, smem, st>>>((const bf16*)r, (const bf16*)w, (const bf16*)k,         \
           (const bf16*)a, (const bf16*)b, tmap_in[0], tmap_in[1], tmap_in[2], tmap_in[3], tmap_in[4], tmap_v,      \
-          ws.tiles, ws.aux, tpc, keep_for_bwd ? 1 : 0, sv, H, NT, n_ch, lay, status,                              \
+          ws.tiles, ws.aux, tpc, keep_for_bwd ? 1 : 0, sv, WalkDims(H, NT, B, grid), lay, status,                              \
           debug_stamp_buffer());                                                                                   \
     } while (0)
     if (seq_start) R7C_LAUNCH_INTRA(true, false);
