@@ -136,6 +136,8 @@ r7_sweep_kernel(Vecs<T> in, const T* __restrict__ v, const float* __restrict__ s
   constexpr int ROWS = rows_per_thread<N>(), NCONS = state_threads<N>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Group<T, N>* const group = reinterpret_cast<Group<T, N>*>(smem_raw);
+  earlier_kernels_done();
+  later_kernels_may_start();
   const int unit = blockIdx.x, ys = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
   const int bi = unit / H, hi = unit % H;
   const long long base = bi * lay.sb + hi * lay.sh;
@@ -440,6 +442,8 @@ r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, c
   constexpr int NTHR = 4 * N;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   GradSmem<N>& sm = *reinterpret_cast<GradSmem<N>*>(smem_raw);
+  earlier_kernels_done();
+  later_kernels_may_start();
   const int tid = threadIdx.x, lane = tid & 31;
   const int NG = (Tn + GT - 1) / GT;
   const int unit = blockIdx.x / NG, m = blockIdx.x % NG, bi = unit / H, hi = unit % H;
@@ -785,9 +789,8 @@ int launch_sweep(const DeviceFacts& dev, const Vecs<T>& in, const void* v, const
   if (allow_smem<r7_sweep_kernel<T, N, BWD, GROUPS>>(dev, GROUPS * bytes)) return RWKVB200_E_CUDA;
   const int blocks = (Tn + W - 1) / W, groups = blocks < GROUPS ? blocks : GROUPS;      // a group without a block is left out
   ProfScope prof(BWD ? "r7_sweep_bwd_kernel" : "r7_sweep_fwd_kernel", st);
-  r7_sweep_kernel<T, N, BWD, GROUPS><<<dim3(B * H, N / RV), state_threads<N>() + N * groups, groups * bytes, st>>>(
-      in, (const T*)v, s_in, n_state, (T*)out, s_out, ckpt, Tn, H, lay);
-  return check_launch();
+  return launch(r7_sweep_kernel<T, N, BWD, GROUPS>, dim3(B * H, N / RV), state_threads<N>() + N * groups, groups * bytes, st, 1,
+                in, (const T*)v, s_in, n_state, (T*)out, s_out, ckpt, Tn, H, lay);
 }
 
 template <typename T, int N, bool BWD>
@@ -829,9 +832,8 @@ int bwd(const void* r, const void* w, const void* k, const void* v, const void* 
   const int smem = (int)sizeof(GradSmem<N>);
   if (allow_smem<r7_grad_kernel<T, N>>(dev, smem)) return RWKVB200_E_CUDA;
   ProfScope prof("r7_grad_kernel", st);
-  r7_grad_kernel<T, N><<<B * H * ((Tn + GT - 1) / GT), 4 * N, smem, st>>>(in, (const T*)v, (const T*)d_o, h0, h0 ? n_state : 0, d_ht,
-                                                                         states, d_states, (T*)dr, (T*)dw, (T*)dk, (T*)da, (T*)db, Tn, H, lay);
-  return check_launch();
+  return launch(r7_grad_kernel<T, N>, B * H * ((Tn + GT - 1) / GT), 4 * N, smem, st, 1, in, (const T*)v, (const T*)d_o, h0,
+                h0 ? n_state : 0, d_ht, states, (const float*)d_states, (T*)dr, (T*)dw, (T*)dk, (T*)da, (T*)db, Tn, H, lay);
 }
 
 }  // namespace

@@ -44,8 +44,6 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int unit = blockIdx.x, bi = unit / H, hi = unit % H;
   const size_t ch0 = (size_t)unit * NT_slots;
-  const int NT = (sv.length<PACKED>(bi) + L - 1) / L;      // chunks of this sequence
-  const int tb = sv.first<PACKED>(bi), brow = sv.row<PACKED>(bi);
   const int wq = warp & 3, hsel = warp >> 2, c0 = 32 * hsel;
   const int row = 16 * wq + (lane & 15);
   const bool state_lane = lane < 16;
@@ -62,6 +60,10 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  earlier_kernels_done();
+  later_kernels_may_start();
+  const int NT = (sv.length<PACKED>(bi) + L - 1) / L;      // chunks of this sequence
+  const int tb = sv.first<PACKED>(bi), brow = sv.row<PACKED>(bi);
   const uint32_t tm = sm.tmem_base;
   // TMEM: columns 64 p .., p = parity of the chunk's place: lower lane halves q~^T do + a~^T dz, upper halves dz
 
@@ -219,12 +221,9 @@ r7c_bwd_scan_alone_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int unit = blockIdx.x, bi = unit / H, hi = unit % H;
   const size_t ch0 = (size_t)unit * NT_slots;
-  const int NT = (sv.length<PACKED>(bi) + L - 1) / L;      // chunks of this sequence
-  const int tb = sv.first<PACKED>(bi), brow = sv.row<PACKED>(bi);
   const int wq = warp & 3, c0 = 32 * (warp >> 2);
   const int row = 16 * wq + (lane & 15);
   const bool state_lane = lane < 16;
-  auto chunk_tiles = [&](int n) { return ws_tiles + (ch0 + NT - 1 - n) * (size_t)tiles_per_chunk * TILE_BYTES; };
 
   if (tid == 0) {
     for (int i = 0; i < 4; ++i) { mbar_init(&sm.bar_full[i], 1); mbar_init(&sm.bar_m2[i], 1); }
@@ -236,6 +235,11 @@ r7c_bwd_scan_alone_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  earlier_kernels_done();
+  later_kernels_may_start();
+  const int NT = (sv.length<PACKED>(bi) + L - 1) / L;      // chunks of this sequence
+  const int tb = sv.first<PACKED>(bi), brow = sv.row<PACKED>(bi);
+  auto chunk_tiles = [&](int n) { return ws_tiles + (ch0 + NT - 1 - n) * (size_t)tiles_per_chunk * TILE_BYTES; };
   // TMEM: columns 64 p .., p = parity of the chunk's place: lower lane halves q~^T do + a~^T dz, upper halves dz
   const uint32_t tm = sm.tmem_base;
   bool ok = true;
@@ -434,6 +438,8 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  earlier_kernels_done();
+  later_kernels_may_start();
   const uint32_t tm = sm.tmem_base;
   constexpr int st_warp = 3;      // requests the tiles, stores the results
 
@@ -837,6 +843,8 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
 __global__ void __launch_bounds__(256)
 r7c_producer_bwd_kernel(const bf16* __restrict__ p, const bf16* __restrict__ u, const bf16* __restrict__ q,
                         bf16* dw_dp, bf16* da_du, bf16* db_dq, long long n_rows) {
+  earlier_kernels_done();
+  later_kernels_may_start();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long row = t >> 3;
   const bool live = row < n_rows;
@@ -885,9 +893,8 @@ int launch_rwkv7_producer_bwd(const void* p, const void* u, const void* q, void*
   typedef __nv_bfloat16 bf16;
   ProfScope prof("r7c_producer_bwd_kernel", st);
   const long long threads = n_rows * 8;
-  r7c::r7c_producer_bwd_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(
-      (const bf16*)p, (const bf16*)u, (const bf16*)q, (bf16*)dw_dp, (bf16*)da_du, (bf16*)db_dq, n_rows);
-  return check_launch();
+  return launch(r7c::r7c_producer_bwd_kernel, (unsigned)((threads + 255) / 256), 256, 0, st, 1, (const bf16*)p, (const bf16*)u,
+                (const bf16*)q, (bf16*)dw_dp, (bf16*)da_du, (bf16*)db_dq, n_rows);
 }
 
 int launch_rwkv7_chunked_bwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
@@ -931,7 +938,8 @@ int launch_rwkv7_chunked_bwd(const void* r, const void* w, const void* k, const 
     do {                                                                                                          \
       const int smem = (int)sizeof(SMEM) + 1024;                                                                  \
       if (allow_smem<KERNEL<P>>(dev, smem)) return RWKVB200_E_CUDA;                                               \
-      KERNEL<P><<<B * H, THREADS, smem, st>>>(tmap_do, ws.tiles, ws.aux, ALL_TILES, d_ht, d_h0, sv, H, NT, status); \
+      if (int rc = launch(KERNEL<P>, B * H, THREADS, smem, st, 1, tmap_do, ws.tiles, ws.aux, (int)ALL_TILES, d_ht, d_h0, sv, H, \
+                          NT, status)) return rc;                                                                  \
     } while (0)
     if (B * H > dev.sms) {      // two CTAs per SM
       if (seq_start) R7C_LAUNCH_BSCAN(r7c_bwd_scan_kernel, true, 256, BScanSmem);
@@ -973,9 +981,9 @@ int launch_rwkv7_chunked_bwd(const void* r, const void* w, const void* k, const 
       if (int rc = need_aligned_smem<r7c_bwd_final_kernel<P, F>>(dev)) return rc;                                 \
       if (allow_smem<r7c_bwd_final_kernel<P, F>>(dev, smem)) \
         return RWKVB200_E_CUDA;                                                                                   \
-      r7c_bwd_final_kernel<P, F><<<grid, 256, smem, st>>>((const bf16*)w, tmap_w, tmap_do, tmap_v, ws.tiles, ALL_TILES, \
+      if (int rc = launch(r7c_bwd_final_kernel<P, F>, grid, 256, smem, st, 1, (const bf16*)w, tmap_w, tmap_do, tmap_v, ws.tiles, (int)ALL_TILES, \
           tmap_out[0], tmap_out[1], tmap_out[2], tmap_out[3], tmap_out[4], tmap_out[5], (bf16*)dr, (bf16*)dw,     \
-          (bf16*)dk, (bf16*)dv, (bf16*)da, (bf16*)db, sv, WalkDims(H, NT, B, grid), lay, status, debug_stamp_buffer());        \
+          (bf16*)dk, (bf16*)dv, (bf16*)da, (bf16*)db, sv, WalkDims(H, NT, B, grid), lay, status, debug_stamp_buffer())) return rc; \
     } while (0)
     if (seq_start) R7C_LAUNCH_FINAL(true, false);
     else if (fused) R7C_LAUNCH_FINAL(false, true);

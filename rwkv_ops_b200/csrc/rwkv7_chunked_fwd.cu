@@ -71,6 +71,8 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  earlier_kernels_done();
+  later_kernels_may_start();
   const uint32_t tm = sm.tmem_base;
 
   auto coords = [&](const ChunkPos& p, int& bi, int& hi, int& t0) { bi = p.bi; hi = p.hi; t0 = p.c * L; };
@@ -599,8 +601,6 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
   const int wq = warp & 3, hsel = warp >> 2, c0 = 32 * hsel;
   const int unit = blockIdx.x, bi = unit / H, hi = unit % H;
   const size_t ch0 = (size_t)unit * NT_slots;
-  const int Tn = sv.length<PACKED>(bi), tb = sv.first<PACKED>(bi), brow = sv.row<PACKED>(bi);
-  const int NT = (Tn + L - 1) / L;           // chunks of this sequence (at least one)
   const int row = 16 * wq + (lane & 15);     // state row k (lanes 0-15) or token row i (lanes 16-31)
   const bool state_lane = lane < 16;
   // Single-thread jobs: warp 0 issues the MMAs, ld_warp requests operand tiles, st_warp copies sa, h~0 and X out for the
@@ -617,6 +617,10 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  earlier_kernels_done();
+  later_kernels_may_start();
+  const int Tn = sv.length<PACKED>(bi), tb = sv.first<PACKED>(bi), brow = sv.row<PACKED>(bi);
+  const int NT = (Tn + L - 1) / L;           // chunks of this sequence (at least one)
   const uint32_t tm = sm.tmem_base;
   // TMEM: columns 0..63 lower lane halves = W h~0; columns 64 + 64 p .., p = parity of the chunk: lower halves
   // k~^T v + b~^T sa, upper halves the output rows
@@ -892,8 +896,6 @@ r7c_scan_fwd_alone_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsi
   const int wq = warp & 3, c0 = 32 * (warp >> 2);
   const int unit = blockIdx.x, bi = unit / H, hi = unit % H;
   const size_t ch0 = (size_t)unit * NT_slots;
-  const int Tn = sv.length<PACKED>(bi), tb = sv.first<PACKED>(bi), brow = sv.row<PACKED>(bi);
-  const int NT = (Tn + L - 1) / L;           // chunks of this sequence (at least one)
   const int row = 16 * wq + (lane & 15);     // state row k (lanes 0-15) or token row i (lanes 16-31)
   const bool state_lane = lane < 16;
   auto chunk_tiles = [&](int c) { return ws_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES; };
@@ -908,6 +910,10 @@ r7c_scan_fwd_alone_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsi
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  earlier_kernels_done();
+  later_kernels_may_start();
+  const int Tn = sv.length<PACKED>(bi), tb = sv.first<PACKED>(bi), brow = sv.row<PACKED>(bi);
+  const int NT = (Tn + L - 1) / L;           // chunks of this sequence (at least one)
   // TMEM: columns 0..63 lower lane halves = W h~0; three accumulators in turn: lower halves k~^T v + b~^T sa, upper halves
   // the output rows, which are read out while the next chunk is worked on and the state of the one after it is stored
   const uint32_t tm = sm.tmem_base;
@@ -1176,10 +1182,10 @@ int launch_rwkv7_chunked_fwd(const void* r, const void* w, const void* k, const 
     do {                                                                                                           \
       if (allow_smem<r7c_intra_fwd_kernel<P, F>>(dev, smem)) \
         return RWKVB200_E_CUDA;                                                                                    \
-      r7c_intra_fwd_kernel<P, F><<<grid, 256, smem, st>>>((const bf16*)r, (const bf16*)w, (const bf16*)k,         \
+      if (int rc = launch(r7c_intra_fwd_kernel<P, F>, grid, 256, smem, st, 1, (const bf16*)r, (const bf16*)w, (const bf16*)k,         \
           (const bf16*)a, (const bf16*)b, tmap_in[0], tmap_in[1], tmap_in[2], tmap_in[3], tmap_in[4], tmap_v,      \
           ws.tiles, ws.aux, tpc, keep_for_bwd ? 1 : 0, sv, WalkDims(H, NT, B, grid), lay, status,                              \
-          debug_stamp_buffer());                                                                                   \
+          debug_stamp_buffer())) return rc;                                                                        \
     } while (0)
     if (seq_start) R7C_LAUNCH_INTRA(true, false);
     else if (fused) R7C_LAUNCH_INTRA(false, true);
@@ -1201,9 +1207,9 @@ int launch_rwkv7_chunked_fwd(const void* r, const void* w, const void* k, const 
       const int smem = (int)sizeof(SMEM) + 1024;                                                                   \
       if (allow_smem<KERNEL<P>>(dev, smem))                                                                        \
         return RWKVB200_E_CUDA;                                                                                    \
-      KERNEL<P><<<B * H, THREADS, smem, st>>>(tmap_v, ws.tiles, ws.aux, ws.flags, tpc,                             \
+      if (int rc = launch(KERNEL<P>, B * H, THREADS, smem, st, 1, tmap_v, ws.tiles, ws.aux, ws.flags, tpc,         \
           keep_for_bwd ? ws.tiles : nullptr, h0, n_state, tmap_o, o ? 1 : 0, ht, (bf16*)o, sv, H, NT, lay, exact,  \
-          status, debug_stamp_buffer());                                                                           \
+          status, debug_stamp_buffer())) return rc;                                                                \
     } while (0)
     if (B * H > dev.sms) {
       if (seq_start) R7C_LAUNCH_SCAN(r7c_scan_fwd_kernel, true, 256, ScanSmem);

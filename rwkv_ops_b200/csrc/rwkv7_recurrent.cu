@@ -39,6 +39,8 @@ template <typename T, int N, int TL>
 __global__ void __launch_bounds__(N)
 rwkv7_rec_fwd_kernel(FwdArgs<T> args, const float* __restrict__ h0, int n_state, float* __restrict__ ht, int H, TokLayout lay) {
   __shared__ __align__(16) FwdSmem<N, VS, TL> sm;
+  earlier_kernels_done();
+  later_kernels_may_start();
   const int unit = blockIdx.x, bi = unit / H, hi = unit % H;
   args.base = bi * lay.sb + hi * lay.sh;
   args.S0 = h0 && n_state > 0 ? h0 + (long long)(n_state == 1 ? hi : unit) * N * N : nullptr;
@@ -75,6 +77,8 @@ rwkv7_rec_bwd_kernel(const T* __restrict__ r, const T* __restrict__ w, const T* 
   constexpr int KSEG = N / 16, NQ = N / VS;
   cg::cluster_group cluster = cg::this_cluster();
 
+  earlier_kernels_done();
+  later_kernels_may_start();
   const int unit = blockIdx.x, y = blockIdx.y, tid = threadIdx.x;
   if (sel.flags && sel.flags[unit] == 0) return;      // the four CTAs of a cluster share the unit: all leave
   const int bi = unit / H, hi = unit % H;
@@ -286,8 +290,8 @@ int launch_rwkv7_rec_step(const void* r, const void* w, const void* k, const voi
     const FwdArgs<T> args{(const T*)r, (const T*)w, (const T*)k, (const T*)v, (const T*)a, (const T*)b, 0, lay.st, 1,
                           nullptr, (T*)o, nullptr, nullptr};
     // (a tile of one token: 256 sequences of 16 heads 317 -> 134 us against a tile of 8)
-    rwkv7_rec_fwd_kernel<T, N, 1><<<dim3(B * H, N / VS), N, 0, st>>>(args, h0, n_state, ht, H, lay));
-  return check_launch();
+    return launch(rwkv7_rec_fwd_kernel<T, N, 1>, dim3(B * H, N / VS), N, 0, st, 1, args, h0, n_state, ht, H, lay));
+  return RWKVB200_OK;
 }
 
 int launch_rwkv7_rec_fwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
@@ -299,8 +303,7 @@ int launch_rwkv7_rec_fwd(const void* r, const void* w, const void* k, const void
   const FwdArgs<T> args{(const T*)r, (const T*)w, (const T*)k, (const T*)v, (const T*)a, (const T*)b, 0, lay.st, Tn,
                         nullptr, (T*)o, nullptr, nullptr};
   // tiles of 8 tokens: with 16, half as many CTAs fit an SM (B 16, T 512, 32 heads: 2269 us against 1281; 16 units 320 and 324)
-  rwkv7_rec_fwd_kernel<T, HS, 8><<<dim3(B * H, HS / VS), HS, 0, st>>>(args, h0, n_state, ht, H, lay);
-  return check_launch();
+  return launch(rwkv7_rec_fwd_kernel<T, HS, 8>, dim3(B * H, HS / VS), HS, 0, st, 1, args, h0, n_state, ht, H, lay);
 }
 
 int launch_rwkv7_rec_bwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
@@ -314,22 +317,11 @@ int launch_rwkv7_rec_bwd(const void* r, const void* w, const void* k, const void
   const int smem = (int)sizeof(BwdSmem<N>);
   DeviceFacts dev;
   if (int e = device_facts(&dev)) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(B * H, N / VS);
-  cfg.blockDim = dim3(N);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;      // the CTAs of a unit exchange partial sums
-  attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = N / VS; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   if (allow_smem<rwkv7_rec_bwd_kernel<T, N>>(dev, smem)) return RWKVB200_E_CUDA;
-  if (cuda_ok(cudaLaunchKernelEx(&cfg, rwkv7_rec_bwd_kernel<T, N>, (const T*)r, (const T*)w, (const T*)k, (const T*)v,
-                                 (const T*)a, (const T*)b, (const T*)d_o, d_ht, h0, n_state, ckpt, (T*)dr, (T*)dw, (T*)dk,
-                                 (T*)dv, (T*)da, (T*)db, d_h0, Tn, H, lay, sel)))
-    return RWKVB200_E_CUDA;
-  return check_launch();
+  // a cluster: the CTAs of a unit exchange partial sums
+  return launch(rwkv7_rec_bwd_kernel<T, N>, dim3(B * H, N / VS), N, smem, st, N / VS, (const T*)r, (const T*)w, (const T*)k,
+                (const T*)v, (const T*)a, (const T*)b, (const T*)d_o, d_ht, h0, n_state, ckpt, (T*)dr, (T*)dw, (T*)dk, (T*)dv,
+                (T*)da, (T*)db, d_h0, Tn, H, lay, sel);
 }
 
 }  // namespace rwkvb200

@@ -54,6 +54,8 @@ rwkv7_step_kernel(const T* __restrict__ r, const T* __restrict__ w, const T* __r
   const int q = tid % LR;                      // key group
   const int rg = tid / LR;                     // row group, 0..15
   __shared__ __align__(16) float vec[5][HS];
+  earlier_kernels_done();
+  later_kernels_may_start();
   auto load_unit = [&](int unit, float (&X)[4][KQ]) {
     const long long sbase = (n_state == 1 ? (long long)(unit % H) : (long long)unit) * (HS * HS);
 #pragma unroll
@@ -148,6 +150,8 @@ rwkv7_step_bf16state_kernel(const T* __restrict__ r, const T* __restrict__ w, co
   const int tid = threadIdx.x, usel = tid >> 6, tu = tid & 63;
   const int q = tu % LR, rg = tu / LR;                 // key group, row group 0..7
   __shared__ __align__(16) float vec[2][6][HS];   // r, decay, k, a, b, v
+  earlier_kernels_done();
+  later_kernels_may_start();
   const int unit = 2 * blockIdx.x + usel;
   const bool live = unit < n_units;
   __nv_bfloat16* S = state + (long long)(live ? unit : 0) * (HS * HS);
@@ -223,9 +227,9 @@ int launch_rwkv7_step(const void* r, const void* w, const void* k, const void* v
                       cudaStream_t st) {
   ProfScope prof("rwkv7_step_kernel", st);
   RWKVB200_DISPATCH_DTYPE(dtype,
-    rwkv7_step_kernel<T, float, 4><<<B * H, 256, 0, st>>>(
-        (const T*)r, (const T*)w, (const T*)k, (const T*)v, (const T*)a, (const T*)b, s_in, n_state, s_out, (T*)o, H));
-  return check_launch();
+    return launch(rwkv7_step_kernel<T, float, 4>, B * H, 256, 0, st, 1, (const T*)r, (const T*)w, (const T*)k, (const T*)v,
+                  (const T*)a, (const T*)b, s_in, n_state, s_out, (T*)o, H));
+  return RWKVB200_OK;
 }
 
 // in place on a state the caller keeps on the device: [B][H][64][64], float32 or bfloat16
@@ -234,16 +238,14 @@ int launch_rwkv7_decode_step(const void* r, const void* w, const void* k, const 
   ProfScope prof("rwkv7_step_kernel", st);
   if (state_dtype == RWKVB200_BF16) {
     RWKVB200_DISPATCH_DTYPE(dtype,
-      rwkv7_step_bf16state_kernel<T><<<(B * H + 1) / 2, 128, 0, st>>>(
-          (const T*)r, (const T*)w, (const T*)k, (const T*)v, (const T*)a, (const T*)b, (__nv_bfloat16*)state, (T*)o,
-          B * H));
+      return launch(rwkv7_step_bf16state_kernel<T>, (B * H + 1) / 2, 128, 0, st, 1, (const T*)r, (const T*)w, (const T*)k,
+                    (const T*)v, (const T*)a, (const T*)b, (__nv_bfloat16*)state, (T*)o, B * H));
   } else {
     RWKVB200_DISPATCH_DTYPE(dtype,
-      rwkv7_step_kernel<T, float, 4><<<B * H, 256, 0, st>>>(
-          (const T*)r, (const T*)w, (const T*)k, (const T*)v, (const T*)a, (const T*)b, (const float*)state, B,
-          (float*)state, (T*)o, H));
+      return launch(rwkv7_step_kernel<T, float, 4>, B * H, 256, 0, st, 1, (const T*)r, (const T*)w, (const T*)k, (const T*)v,
+                    (const T*)a, (const T*)b, (const float*)state, B, (float*)state, (T*)o, H));
   }
-  return check_launch();
+  return RWKVB200_OK;
 }
 
 }  // namespace rwkvb200

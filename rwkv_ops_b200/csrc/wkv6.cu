@@ -66,6 +66,8 @@ wkv6_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __res
   __shared__ __align__(16) float vt[TL][VS];
   __shared__ __align__(16) float yt[TL][VS];
 
+  earlier_kernels_done();
+  later_kernels_may_start();
   const int unit = blockIdx.x, y = blockIdx.y, tid = threadIdx.x;
   if (sel.flags && sel.flags[unit] == 0) return;      // only the selected units run
   const int bi = unit / H, hi = unit % H;
@@ -210,6 +212,8 @@ wkv6_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __res
   typedef typename std::conditional<COARSE, BwdSmemCoarse<N>, BwdSmem<N>>::type Smem;
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   cg::cluster_group cluster = cg::this_cluster();
+  earlier_kernels_done();
+  later_kernels_may_start();
 
   const int unit = blockIdx.x, y = blockIdx.y, tid = threadIdx.x;
   if (sel.flags && sel.flags[unit] == 0) return;      // the CTAs of a cluster share the unit: all leave
@@ -436,6 +440,8 @@ wkv6_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __res
 // du[h][k] = sum over batch rows and the CTAs of a unit, in a fixed order (one thread per key channel).
 __global__ void __launch_bounds__(128)
 wkv6_du_reduce_kernel(const float* __restrict__ du_partial, float* __restrict__ du, int B, int H) {
+  earlier_kernels_done();
+  later_kernels_may_start();
   const int hi = blockIdx.x, kc = threadIdx.x, n = blockDim.x, nq = n / VS;
   float s = 0.f;
   for (int bi = 0; bi < B; ++bi)
@@ -450,6 +456,8 @@ __global__ void __launch_bounds__(64)
 wkv6_du_reduce_mixed_kernel(const float* __restrict__ part_chunked, const float* __restrict__ part_rec,
                             const int* __restrict__ flags, float* __restrict__ du, int B, int H, int rows) {
   constexpr int NQ = HS / VS;
+  earlier_kernels_done();
+  later_kernels_may_start();
   const int hi = blockIdx.x, kc = threadIdx.x;
   float s = 0.f;
   for (int bi = 0; bi < B; ++bi) {
@@ -483,10 +491,9 @@ int launch_wkv6_fwd(const void* r, const void* k, const void* v, const void* w, 
   RWKVB200_DISPATCH_HEAD6(head_size,
     dim3 grid(B * H, N / VS);
     RWKVB200_DISPATCH_DTYPE(dtype,
-      wkv6_fwd_kernel<T, N><<<grid, N, 0, st>>>((const T*)r, (const T*)k, (const T*)v, (const T*)w, u, s0, n_state,
-                                                smap, (T*)y, sT, ckpt, ckpt_every ? ckpt_every : CK, Tn, H, sel,
-                                                typed)));
-  return check_launch();
+      return launch(wkv6_fwd_kernel<T, N>, grid, N, 0, st, 1, (const T*)r, (const T*)k, (const T*)v, (const T*)w, u, s0, n_state,
+                    smap, (T*)y, sT, ckpt, ckpt_every ? ckpt_every : CK, Tn, H, sel, (int)typed)));
+  return RWKVB200_OK;
 }
 
 namespace {
@@ -501,21 +508,9 @@ int launch_bwd_cluster(const void* r, const void* k, const void* v, const void* 
   if (int e = device_facts(&dev)) return e;
   if (allow_smem<wkv6_bwd_kernel<T, N, COARSE>>(dev, smem))
     return RWKVB200_E_CUDA;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(B * H, N / VS);
-  cfg.blockDim = dim3(N);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;      // the CTAs of a unit exchange partial sums
-  attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = N / VS; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (cuda_ok(cudaLaunchKernelEx(&cfg, wkv6_bwd_kernel<T, N, COARSE>, (const T*)r, (const T*)k, (const T*)v,
-                                 (const T*)w, u, (const T*)d_y, d_sT, ckpt, (T*)dr, (T*)dk, (T*)dv, (T*)dw,
-                                 du_partial, d_s0, Tn, H, sel)))
-    return RWKVB200_E_CUDA;
-  return RWKVB200_OK;
+  // a cluster: the CTAs of a unit exchange partial sums
+  return launch(wkv6_bwd_kernel<T, N, COARSE>, dim3(B * H, N / VS), N, smem, st, N / VS, (const T*)r, (const T*)k, (const T*)v,
+                (const T*)w, u, (const T*)d_y, d_sT, ckpt, (T*)dr, (T*)dk, (T*)dv, (T*)dw, du_partial, d_s0, Tn, H, sel);
 }
 }  // namespace
 
@@ -536,8 +531,7 @@ int launch_wkv6_bwd_coarse(const void* r, const void* k, const void* v, const vo
 int launch_wkv6_du_reduce_mixed(const float* part_chunked, const float* part_rec, const int* flags, float* du,
                                 int B, int H, cudaStream_t st, int rows) {
   ProfScope prof("wkv6_du_reduce_kernel", st);
-  wkv6_du_reduce_mixed_kernel<<<H, 64, 0, st>>>(part_chunked, part_rec, flags, du, B, H, rows);
-  return check_launch();
+  return launch(wkv6_du_reduce_mixed_kernel, H, 64, 0, st, 1, part_chunked, part_rec, flags, du, B, H, rows);
 }
 
 int launch_wkv6_bwd(const void* r, const void* k, const void* v, const void* w, const float* u,
@@ -556,8 +550,7 @@ int launch_wkv6_bwd(const void* r, const void* k, const void* v, const void* w, 
   int e = check_launch();
   if (e) return e;
   ProfScope prof("wkv6_du_reduce_kernel", st);
-  wkv6_du_reduce_kernel<<<H, head_size, 0, st>>>(du_partial, du, B, H);
-  return check_launch();
+  return launch(wkv6_du_reduce_kernel, H, head_size, 0, st, 1, (const float*)du_partial, du, B, H);
 }
 
 }  // namespace rwkvb200

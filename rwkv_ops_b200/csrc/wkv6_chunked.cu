@@ -234,6 +234,8 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  earlier_kernels_done();
+  later_kernels_may_start();
   const uint32_t tm = sm.tmem_base;
   // TMEM: columns 0..63 lower halves = r~ k~^T; columns 64..127 lower halves = y, upper halves = k~^T v
   const uint32_t tm_a = tmem_addr(tm, 32 * wq, CW * hsel);
@@ -609,6 +611,8 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  earlier_kernels_done();
+  later_kernels_may_start();
   const uint32_t tm = sm.tmem_base;
   const uint32_t tm_c0 = tmem_addr(tm, 32 * wq, CW * hsel);          // A (lower), dA (upper)
   const uint32_t tm_c1 = tmem_addr(tm, 32 * wq, 64 + CW * hsel);     // dk~ (lower), dr~ (upper)
@@ -1106,9 +1110,9 @@ int launch_wkv6_chunked_fwd(const void* r, const void* k, const void* v, const v
 #define W6C_LAUNCH_FWD(NTHR)                                                                                          \
     RWKVB200_DISPATCH_DTYPE(dtype, W6C_DISPATCH_PACKED(                                                               \
       if (allow_smem<wkv6c_fwd_kernel<T, P, NTHR>>(dev, smem)) return RWKVB200_E_CUDA;                                \
-      wkv6c_fwd_kernel<T, P, NTHR><<<grid, NTHR, smem, st>>>(                                                         \
-          (const T*)r, (const T*)k, (const T*)v, (const T*)w, u, s0, n_state, smap, (T*)y, sT, typed, states, flags,   \
-          tm_r, tm_k, tm_v, tm_w, mapT, H, seqs, n_units, parts, handoff, hflags, status, debug_stamp_buffer())))
+      if (int rc = launch(wkv6c_fwd_kernel<T, P, NTHR>, grid, NTHR, smem, st, 1,                                      \
+          (const T*)r, (const T*)k, (const T*)v, (const T*)w, u, s0, n_state, smap, (T*)y, sT, (int)typed, states, flags, \
+          tm_r, tm_k, tm_v, tm_w, mapT, H, seqs, n_units, parts, handoff, hflags, status, debug_stamp_buffer())) return rc))
     if (n_units <= sms) W6C_LAUNCH_FWD(512) else W6C_LAUNCH_FWD(256)
 #undef W6C_LAUNCH_FWD
   }
@@ -1224,11 +1228,11 @@ int launch_wkv6_chunked_bwd(const void* r, const void* k, const void* v, const v
     ProfScope prof("wkv6c_bwd_kernel", st);
     RWKVB200_DISPATCH_DTYPE(dtype, W6C_DISPATCH_PACKED(
       if (allow_smem<wkv6c_bwd_kernel<T, P>>(dev, smem)) return RWKVB200_E_CUDA;
-      wkv6c_bwd_kernel<T, P><<<grid, BWD_THREADS, smem, st>>>((const T*)r, (const T*)k, (const T*)v, (const T*)w, u,
-                                                       (const T*)d_y, d_sT, states, (T*)dr, (T*)dk, (T*)dv, (T*)dw,
-                                                       du_partial, d_s0, tm_r, tm_k, tm_v, tm_w, tm_dy, tm_s, mapT, H, seqs,
-                                                       n_units, split ? 1 : 0, ws.handoff, ws.hflags, status,
-                                                       debug_stamp_buffer())));
+      if (int rc = launch(wkv6c_bwd_kernel<T, P>, grid, BWD_THREADS, smem, st, 1, (const T*)r, (const T*)k, (const T*)v, (const T*)w, u,
+                          (const T*)d_y, d_sT, states, (T*)dr, (T*)dk, (T*)dv, (T*)dw,
+                          du_partial, d_s0, tm_r, tm_k, tm_v, tm_w, tm_dy, tm_s, mapT, H, seqs,
+                          n_units, split ? 1 : 0, ws.handoff, ws.hflags, status,
+                          debug_stamp_buffer())) return rc));
   }
   e = check_launch();
   if (e) return e;
