@@ -65,6 +65,10 @@ __device__ __forceinline__ Quad quad_of(float4 f) { return Quad{pack2(f.x, f.y),
 __device__ __forceinline__ Quad lds4(const float* p) { return quad_of(*reinterpret_cast<const float4*>(p)); }
 __device__ __forceinline__ float sum2(f32x2 v) { const float2 f = unpack2(v); return f.x + f.y; }
 
+// A warp's 16-byte reads of shared memory take four cycles, but two where lanes that differ in bit 0 or bit 1 read the same
+// address (measured: sharing along the higher bits saves nothing).  So in the kernels below the lanes that share an operand
+// differ in one of these two bits, and where two operands are shared, each has one of them.
+
 // Sum CNT values over the lanes that differ in the bits of MASK, MASK/2, .., LAST; the values are shared out on the
 // way: a lane whose bit is set goes on with the upper half.
 template <int CNT, int MASK, int LAST, int M>
@@ -146,8 +150,9 @@ r7_sweep_kernel(Vecs<T> in, const T* __restrict__ v, const float* __restrict__ s
 
   if (tid < NCONS) {
     // ---- state warps
-    constexpr int CL = N / 8;                    // lanes per row
-    const int r0 = ROWS * (tid / CL), kq = tid % CL, jl = kq & 7;
+    // N/8 lanes per row; the lanes that read the same part of a vector are neighbours (see the note on 16-byte reads above)
+    constexpr int RG = 256 / N;                  // groups of rows in a warp
+    const int r0 = ROWS * (tid / 32 * RG + lane % RG), kq = lane / RG, jl = kq & 7;
     const int c0 = 4 * kq, c1 = N / 2 + 4 * kq;  // this thread's columns: two quads of ROWS rows
     const int NG = (Tn + GT - 1) / GT;
     Quad S[ROWS][2];
@@ -195,14 +200,14 @@ r7_sweep_kernel(Vecs<T> in, const T* __restrict__ v, const float* __restrict__ s
       dots(st.x, ax);
       float sa[ROWS], oo[ROWS];
       if constexpr (N == 64) {
-        reduce_scatter<W * ROWS, 4, 1>(ax, lane);
+        reduce_scatter<W * ROWS, 4 * RG, RG>(ax, lane);
         dots(st.y, ay);
-        reduce_scatter<W * ROWS, 4, 1>(ay, lane);
+        reduce_scatter<W * ROWS, 4 * RG, RG>(ay, lane);
 #pragma unroll
         for (int i = 0; i < ROWS; ++i) { sa[i] = ax[i]; oo[i] = ay[i]; }
       } else {
         dots(st.y, ax + W * ROWS);
-        reduce_scatter<2 * W * ROWS, 8, 1>(ax, lane);
+        reduce_scatter<2 * W * ROWS, 8 * RG, RG>(ax, lane);
 #pragma unroll
         for (int i = 0; i < ROWS; ++i) sa[i] = oo[i] = ax[i];
       }
@@ -244,7 +249,7 @@ r7_sweep_kernel(Vecs<T> in, const T* __restrict__ v, const float* __restrict__ s
       for (int p = 0; p < W; ++p) {
         const Quad ua = lds4(&st.u1[p][c0]), ub = lds4(&st.u1[p][c1]);
 #pragma unroll
-        for (int i = 0; i < ROWS; ++i) add_outer(ua, ub, i, __shfl_sync(0xffffffffu, sa[i], (lane & ~(CL - 1)) | p));
+        for (int i = 0; i < ROWS; ++i) add_outer(ua, ub, i, __shfl_sync(0xffffffffu, sa[i], lane % RG + RG * p));
       }
       if (idx + GROUPS < NB) bar_arrive(EMPTY + g, NCONS + N);
       const int t = n * W + (BWD ? W - 1 - jl : jl);
@@ -457,6 +462,15 @@ r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, c
   // ---- tokens and S
   const int kq = tid % (N / 4), row0 = tid / (N / 4);      // quad of channels, token / state row (16 at a time)
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  // four values down a column of an array whose rows are 36 floats long: every second lane starts with another one of
+  // them, which leaves two of the eight lanes that would meet on a bank
+  auto put_column = [&](const float (&f)[4], auto at) {
+    const int by = kq >> 1;
+    const float a0 = by & 1 ? f[1] : f[0], a1 = by & 1 ? f[2] : f[1], a2 = by & 1 ? f[3] : f[2], a3 = by & 1 ? f[0] : f[3];
+    const float b[4] = {by & 2 ? a2 : a0, by & 2 ? a3 : a1, by & 2 ? a0 : a2, by & 2 ? a1 : a3};
+#pragma unroll
+    for (int x = 0; x < 4; ++x) *at((x + by) & 3) = b[x];
+  };
   {
     const bool live = row0 < nt;
     const long long off = base + (live ? (long long)row0 * lay.st : 0) + 4 * kq;
@@ -468,8 +482,8 @@ r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, c
     }
     const float4 fv = live ? load4(v + off) : zero, fo = live ? load4(d_o + off) : zero;
     const float ev[4] = {fv.x, fv.y, fv.z, fv.w}, eo[4] = {fo.x, fo.y, fo.z, fo.w};
-#pragma unroll
-    for (int x = 0; x < 4; ++x) { sm.cat1[4 * kq + x][GT + row0] = ev[x]; sm.cat2[4 * kq + x][row0] = eo[x]; }
+    put_column(ev, [&](int x) { return &sm.cat1[4 * kq + x][GT + row0]; });
+    put_column(eo, [&](int x) { return &sm.cat2[4 * kq + x][row0]; });
   }
   auto get_state = [&](const float* g) {
 #pragma unroll
@@ -537,7 +551,7 @@ r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, c
 
   // rows: dst[v][j] = sum_k st[v][k] xs[j][k]; a 4 x 4 tile per thread and a quarter of the channels
   auto row_product = [&](float (*dst)[36], int j0) {
-    const int s = tid & 3, tj = (tid >> 2) & 3, tv = tid >> 4;
+    const int s = (tid >> 2) & 3, tj = (tid & 1) | ((tid >> 3) & 2), tv = ((tid >> 1) & 1) | (tid >> 5 << 1);
     f32x2 acc[16];
 #pragma unroll
     for (int e = 0; e < 16; ++e) acc[e] = 0ull;
@@ -553,16 +567,18 @@ r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, c
     float r[16];
 #pragma unroll
     for (int e = 0; e < 16; ++e) r[e] = sum2(acc[e]);
-    reduce_scatter<16, 2, 1>(r, lane);      // lane s keeps row s of the tile
+    reduce_scatter<16, 8, 4>(r, lane);      // lane s keeps row s of the tile
     *reinterpret_cast<float4*>(&dst[4 * tv + s][j0 + 4 * tj]) = make_float4(r[0], r[1], r[2], r[3]);
   };
-  // columns: acc(k, j) = sum_v A[v][k] B[v][j] over 4 x 4 tiles, NS lanes share the rows of a tile
-  auto col_product = [&](const float* A, int lda, const float (*B)[36], int tk, int tj, int s, int NS, float (&r)[16]) {
+  // columns: acc(k, j) = sum_v A[v][k] B[v][j] over 4 x 4 tiles; NS lanes share the rows of a tile, RUN rows at a time each
+  // (as many as put these lanes' rows, 36 or 68 floats apart, on different banks)
+  auto col_product = [&](const float* A, int lda, const float (*B)[36], int tk, int tj, int s, int NS, int RUN, float (&r)[16]) {
     f32x2 acc[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) acc[e] = 0ull;
 #pragma unroll 4
-    for (int x = s; x < N; x += NS) {
+    for (int it = 0; it < N / NS; ++it) {
+      const int x = it % RUN + RUN * (s + NS * (it / RUN));
       const Quad a = lds4(A + x * lda + 4 * tk);
       const float4 b = *reinterpret_cast<const float4*>(&B[x][4 * tj]);
       const f32x2 bb[4] = {pack2(b.x, b.x), pack2(b.y, b.y), pack2(b.z, b.z), pack2(b.w, b.w)};
@@ -576,10 +592,10 @@ r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, c
     }
   };
   auto state_cols = [&](float (*dst)[36], const float (*B)[36]) {
-    const int s = tid & 1, tj = (tid >> 1) & 7, tk = tid >> 4;
+    const int s = (tid >> 2) & 1, tj = (tid & 1) | ((tid >> 2) & 6), tk = ((tid >> 1) & 1) | (tid >> 5 << 1);
     float r[16];
-    col_product(&sm.st[0][0], N + 4, B, tk, tj, s, 2, r);
-    reduce_scatter<16, 1, 1>(r, lane);      // lane s keeps channels 2 s, 2 s + 1
+    col_product(&sm.st[0][0], N + 4, B, tk, tj, s, 2, 4, r);
+    reduce_scatter<16, 4, 4>(r, lane);      // lane s keeps channels 2 s, 2 s + 1
     *reinterpret_cast<float4*>(&dst[4 * tk + 2 * s][4 * tj]) = make_float4(r[0], r[1], r[2], r[3]);
     *reinterpret_cast<float4*>(&dst[4 * tk + 2 * s + 1][4 * tj]) = make_float4(r[4], r[5], r[6], r[7]);
   };
@@ -626,8 +642,7 @@ r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, c
       *p = G;
     }
     const float ez[4] = {z.x, z.y, z.z, z.w};
-#pragma unroll
-    for (int x = 0; x < 4; ++x) sm.outS[4 * kq + x][row0] = ez[x];
+    put_column(ez, [&](int x) { return &sm.outS[4 * kq + x][row0]; });
   }
   scaled(true);
   __syncthreads();
@@ -671,10 +686,11 @@ r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, c
   state_cols(sm.outS, sm.cat2);
   {
     constexpr int NS = NTHR / 64;      // 4 or 8 lanes per tile
-    const int s = tid % NS, ti = tid / NS % 8, tj = tid / (NS * 8);
+    const int s = (tid >> 2) % NS, high = tid / (4 * NS);      // tj bit 0, ti bit 0, s, then the other two bits of ti and of tj
+    const int ti = ((tid >> 1) & 1) | ((high & 3) << 1), tj = (tid & 1) | (high >> 2 << 1);
     float r[16];
-    col_product(&sm.cat1[0][0], 36, sm.cat2, ti, tj, s, NS, r);
-    reduce_scatter<16, NS / 2, 1>(r, lane);
+    col_product(&sm.cat1[0][0], 36, sm.cat2, ti, tj, s, NS, 2, r);
+    reduce_scatter<16, 2 * NS, 4>(r, lane);
     constexpr int KEEP = 16 / NS;
 #pragma unroll
     for (int x = 0; x < KEEP; ++x) {
