@@ -35,7 +35,6 @@ namespace {
 
 constexpr int W = 8;          // tokens per block
 constexpr int RV = 16;        // value rows per CTA
-template <int N> constexpr int rows_per_thread() { return N / 32; }      // value rows per thread of the state warps: two warps of them
 constexpr int GT = 2 * W;     // tokens per work item of the gradient kernel, and between two checkpoints
 
 // packed pairs of float32
@@ -98,11 +97,11 @@ enum { VR = 0, VW = 1, VK = 2, VA = 3, VB = 4 };
 // ---------------------------------------------------------------------------------------------
 // the sweep over the blocks: forward (S, sa, o) or backward (G, dsa, dv)
 // ---------------------------------------------------------------------------------------------
-// A CTA owns 16 value rows of one (batch, head) unit.  Its two state warps hold them in registers (N/32 rows and 8 columns
-// to a lane, N/8 lanes to a row); its other threads prepare blocks ahead of them, a group of N threads per block in turn.
-// A vector of the stage is read from shared memory once per lane and serves N/32 rows: with one row per lane the reads
-// alone took 82 % of the shared-memory cycles (138 us per sweep at B 2, T 1024, 16 heads; 124 now), with four rows per
-// lane at N = 64 there is a single state warp and its own latency is the bound (190 us).
+// A CTA owns 16 value rows of one (batch, head) unit.  Its state warps hold them in registers (ROWS rows and 8 columns to a
+// lane, N/8 lanes to a row); its other threads prepare blocks ahead of them, a group of N threads per block in turn.
+// ROWS = 1 (2 at N = 128), four state warps, where a CTA has its SM to itself: the instructions of a warp are then what a
+// block takes, and a warp of twice the rows needs 131 us per sweep where this takes 108 (B 2, T 1024, 16 heads).  ROWS = 2
+// where CTAs share an SM, whose shared memory they fill: B 16, T 512, 16 heads, forward 332 us against 360.
 // In processing order p (time forward, or reversed), the stage a group hands over:
 template <int N>
 struct Stage {
@@ -131,13 +130,15 @@ struct Group {
 // and so they do in float16, where two CTAs of four groups fit an SM as it is (B 16, T 512, 16 heads: 339 us and 364).
 template <int N> constexpr int FEW_CTAS = N == 64 ? 4 : 3;
 template <typename T, int N> constexpr int MANY_CTAS = N == 128 ? 1 : sizeof(T) == 4 ? 2 : FEW_CTAS<N>;
-template <int N> constexpr int state_threads() { return RV / rows_per_thread<N>() * N / 8; }
+template <int N> constexpr int FEW_CTAS_ROWS = N / 64;
+constexpr int MANY_CTAS_ROWS = 2;
+template <int N, int ROWS> constexpr int state_threads() { return RV / ROWS * N / 8; }
 
-template <typename T, int N, bool BWD, int GROUPS>
-__global__ void __launch_bounds__(state_threads<N>() + N * GROUPS)
+template <typename T, int N, bool BWD, int GROUPS, int ROWS>
+__global__ void __launch_bounds__(state_threads<N, ROWS>() + N * GROUPS)
 r7_sweep_kernel(Vecs<T> in, const T* __restrict__ v, const float* __restrict__ s_in, int n_state,
                 T* __restrict__ out, float* __restrict__ s_out, float* __restrict__ ckpt, int Tn, int H, TokLayout lay) {
-  constexpr int ROWS = rows_per_thread<N>(), NCONS = state_threads<N>();
+  constexpr int NCONS = state_threads<N, ROWS>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Group<T, N>* const group = reinterpret_cast<Group<T, N>*>(smem_raw);
   earlier_kernels_done();
@@ -255,12 +256,8 @@ r7_sweep_kernel(Vecs<T> in, const T* __restrict__ v, const float* __restrict__ s
       const int t = n * W + (BWD ? W - 1 - jl : jl);
       if (out && t < Tn && (N == 64 || kq >= 8)) {
         T* p = out + base + (long long)t * lay.st + ys * RV + r0;
-        if constexpr (ROWS == 4) {
-          store4(p, make_float4(oo[0], oo[1], oo[2], oo[3]));
-        } else {
-          p[0] = from_f32<T>(oo[0]);
-          p[1] = from_f32<T>(oo[1]);
-        }
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) p[i] = from_f32<T>(oo[i]);
       }
     }
     if (s_out) put_state(s_out + (long long)unit * N * N);
@@ -798,14 +795,14 @@ r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, c
   }
 }
 
-template <typename T, int N, bool BWD, int GROUPS>
+template <typename T, int N, bool BWD, int GROUPS, int ROWS>
 int launch_sweep(const DeviceFacts& dev, const Vecs<T>& in, const void* v, const float* s_in, int n_state, void* out, float* s_out,
                  float* ckpt, int B, int Tn, int H, const TokLayout& lay, cudaStream_t st) {
   constexpr int bytes = (int)sizeof(Group<T, N>);
-  if (allow_smem<r7_sweep_kernel<T, N, BWD, GROUPS>>(dev, GROUPS * bytes)) return RWKVB200_E_CUDA;
+  if (allow_smem<r7_sweep_kernel<T, N, BWD, GROUPS, ROWS>>(dev, GROUPS * bytes)) return RWKVB200_E_CUDA;
   const int blocks = (Tn + W - 1) / W, groups = blocks < GROUPS ? blocks : GROUPS;      // a group without a block is left out
   ProfScope prof(BWD ? "r7_sweep_bwd_kernel" : "r7_sweep_fwd_kernel", st);
-  return launch(r7_sweep_kernel<T, N, BWD, GROUPS>, dim3(B * H, N / RV), state_threads<N>() + N * groups, groups * bytes, st, 1,
+  return launch(r7_sweep_kernel<T, N, BWD, GROUPS, ROWS>, dim3(B * H, N / RV), state_threads<N, ROWS>() + N * groups, groups * bytes, st, 1,
                 in, (const T*)v, s_in, n_state, (T*)out, s_out, ckpt, Tn, H, lay);
 }
 
@@ -815,8 +812,8 @@ int sweep(const Vecs<T>& in, const void* v, const float* s_in, int n_state, void
   DeviceFacts dev;
   if (int e = device_facts(&dev)) return e;
   return B * H * (N / RV) > dev.sms
-             ? launch_sweep<T, N, BWD, MANY_CTAS<T, N>>(dev, in, v, s_in, n_state, out, s_out, ckpt, B, Tn, H, lay, st)
-             : launch_sweep<T, N, BWD, FEW_CTAS<N>>(dev, in, v, s_in, n_state, out, s_out, ckpt, B, Tn, H, lay, st);
+             ? launch_sweep<T, N, BWD, MANY_CTAS<T, N>, MANY_CTAS_ROWS>(dev, in, v, s_in, n_state, out, s_out, ckpt, B, Tn, H, lay, st)
+             : launch_sweep<T, N, BWD, FEW_CTAS<N>, FEW_CTAS_ROWS<N>>(dev, in, v, s_in, n_state, out, s_out, ckpt, B, Tn, H, lay, st);
 }
 
 template <typename T, int N>
