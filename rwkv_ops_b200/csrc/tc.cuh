@@ -78,8 +78,46 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
   if (!done) atomicCAS(status, 0, code);
   return __all_sync(__activemask(), done) != 0;
 }
+// The same for a barrier at which threads of other CTAs of the cluster arrive or whose bytes come from there.
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, int* status, int code) {
+  bool done = false;
+  for (uint32_t i = 0; i < WAIT_LIMIT && !done; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    done = ok != 0;
+  }
+  if (!done) atomicCAS(status, 0, code);
+  return __all_sync(__activemask(), done) != 0;
+}
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// ---------------------------------------------------------------------------------------------
+// thread-block clusters: shared memory of another CTA
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t smem_addr, uint32_t rank) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// 16 bytes into another CTA's shared memory; its barrier counts them
+__device__ __forceinline__ void store_async_16(uint32_t addr, float4 f, uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
+               ::"r"(addr), "f"(f.x), "f"(f.y), "f"(f.z), "f"(f.w), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void store_cluster(uint32_t addr, int x) {
+  asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(addr), "r"(x) : "memory");
 }
 
 // True for one thread of a warp whose 32 threads all get here (always the same one).  Single-thread jobs (MMAs, bulk
@@ -348,7 +386,9 @@ int make_token_tensor_map(CUtensorMap* out, const void* base, int B, int T, int 
 // ran out; nullptr if the lookup failed.  Read and cleared by rwkvb200_device_status().
 int* device_status_ptr();
 
-int make_row_tensor_map(CUtensorMap* out, const void* base, int B, int T, int H, int elem_bytes);
+// Token tensors [B,T,H,64] of 2 or 4 byte elements, a box of 64 tokens: plain rows, or `swizzled`, tiles of 128-byte rows (for 4
+// byte elements half the channels each).
+int make_row_tensor_map(CUtensorMap* out, const void* base, int B, int T, int H, int elem_bytes, bool swizzled = false);
 int make_state_tensor_map(CUtensorMap* out, const void* base, long long rows);
 
 // Device buffer (>= 64 long long) that kernels fill with clock64() stamps at their phase boundaries (one

@@ -19,8 +19,8 @@
 // operand X is split as X = hi + lo (two bf16 tiles) and every product is the three tensor-core
 // products hi*hi + hi*lo + lo*hi accumulated in fp32 TMEM (relative error ~2^-16 per term).
 //
-// One CTA of 256 threads per (batch, head) (512 in the forward when there is at most one unit per SM: 64.5 -> 60 us for
-// 4 prompts of 777 tokens, 32 heads, bfloat16) walks the chunks in order; the fp32 state (its gradient in the
+// A CTA of 256 threads per (batch, head) walks the chunks in order; in the forward, where that would leave SMs idle, a cluster
+// of CTAs takes the chunks of a unit in turn (a single chunk: 512 threads).  The fp32 state (its gradient in the
 // backward) lives in the registers of the threads that own its rows, the products in TMEM, and nothing but
 // the inputs and outputs touches HBM in the forward pass (plus, for the backward, the fp32 state at every
 // chunk boundary).  The raw rows of the next chunk arrive by TMA while the current chunk is worked on.
@@ -55,11 +55,14 @@ constexpr float DECAY_LIMIT = 45.f;
 // products), and the 2^-17 roundings of the split operands reached 5e-4 of dw there; the recurrence costs nothing
 // at that length.
 constexpr int SHORT_SEQ = 8;
+constexpr int MARKED = 1 << 30;      // in the forward's count of stretches done: one of them has to be recomputed
 
 // two values as packed bf16 pairs hi and lo with x = hi + lo (+ an error of about 2^-17 |x|)
 __device__ __forceinline__ void split_pair(float x0, float x1, uint32_t& hi, uint32_t& lo) {
   hi = pack_bf16(x0, x1);
-  lo = pack_bf16(x0 - bf16_lo(hi), x1 - bf16_hi(hi));
+  float l0, l1;
+  fma2(l0, l1, bf16_lo(hi), bf16_hi(hi), -1.f, -1.f, x0, x1);      // x - hi, both in one instruction
+  lo = pack_bf16(l0, l1);
 }
 // write 4 consecutive values (columns col .. col+3, col a multiple of 4) of `row` into a hi and a lo tile
 template <bool LO = true>
@@ -145,6 +148,31 @@ __device__ __forceinline__ void store_masked_row(const uint32_t (&rr)[CW], int l
   }
   store_split_row<CW>(hi_t, hi_t + TILE_BYTES, row, col0, x);
 }
+// Row `lr` of the same block as values, `other` in the lanes that do not hold a row of it.  All lanes of the warp call it.
+template <int CW>
+__device__ __forceinline__ void load_masked_row(uint32_t taddr, int wq, int hsel, int lr, float diag, bool active,
+                                                const float (&other)[CW], float (&x)[CW]) {
+  const int jlo = 16 * wq - CW * hsel;
+  if (jlo < 0) {
+#pragma unroll
+    for (int j = 0; j < CW; ++j) x[j] = active ? 0.f : other[j];
+    return;
+  }
+  uint32_t rr[CW];
+  tmem_ld<CW>(taddr, rr);
+  tmem_ld_wait();
+  auto crossed_at = [&](int at) {      // left of column `at` everything is kept, from at + 16 on nothing
+#pragma unroll
+    for (int j = 0; j < CW; ++j) {
+      const float f = __uint_as_float(rr[j]);
+      const float m = j < at ? f : j >= at + 16 ? 0.f : (j - at) < lr ? f : (j - at) == lr ? diag : 0.f;
+      x[j] = active ? m : other[j];
+    }
+  };
+  if (jlo >= CW) crossed_at(CW);
+  else if (CW == 32 && jlo == 16) crossed_at(16);
+  else crossed_at(0);
+}
 // the same for a warp whose rows are 16*wq .. and whose columns are CW*hsel ..; all lanes of the warp call it
 template <int CW>
 __device__ __forceinline__ void load_store_masked_row(uint32_t taddr, int wq, int hsel, int lr, float diag,
@@ -180,6 +208,13 @@ struct Seqs {
   int nts;      // chunk-boundary state slots per unit in `states` (chunks of the longest sequence + 1)
 };
 
+// The counters of the stretches, as a kernel: a memset would hold the next kernel's launch up.
+__global__ void w6c_clear_kernel(int* p, int n) {
+  earlier_kernels_done();
+  later_kernels_may_start();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) p[i] = 0;
+}
+
 // ---------------------------------------------------------------------------------------------
 // forward
 // ---------------------------------------------------------------------------------------------
@@ -193,8 +228,10 @@ struct FwdSmem {
   float qtot[8][64];
   float dgs[64];                      // sum_k r u k per token
   uint64_t bar_1, bar_2, bar_in;
+  uint64_t bar_state, bar_free;       // RELAY: the state is here (16 KB); the next CTA can take another one
   uint32_t tmem_base;
-  int handoff_ok, next_item;
+  int next_item, state_seen;
+  int marks[8];                       // RELAY: what each CTA of the cluster has marked (in the first one)
 };
 
 // The raw r, k, v, w rows of a chunk (64 rows of 64 elements each) arrive by TMA in the space of the tile
@@ -202,14 +239,15 @@ struct FwdSmem {
 // the last MMA of the current one has read those tiles; a thread reads its elements, all threads meet at a
 // barrier, and then the split tiles are written over the raw rows.
 // S0 of every chunk (and the final state) goes to `states` [B*H][NT+1][64][64] when it is not NULL.
-template <typename T, bool PACKED, int NTHR>
+template <typename T, bool PACKED, int NTHR, bool RELAY>
 __global__ void __launch_bounds__(NTHR, 512 / NTHR)
 wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ w,
                  const void* __restrict__ u, const void* __restrict__ s0, int n_state,
                  const int32_t* __restrict__ smap, T* __restrict__ y, void* __restrict__ sT, int typed,
                  float* __restrict__ states, int* __restrict__ flags, const __grid_constant__ CUtensorMap tmap_r,
                  const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
-                 const __grid_constant__ CUtensorMap tmap_w, int Tn_dense, int H, Seqs seqs, int n_units, int parts,
+                 const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_y, int Tn_dense, int H,
+                 Seqs seqs, int n_units, int per_item, int parts,
                  float* __restrict__ handoff, int* __restrict__ handoff_flags, int* status, long long* dbg) {
 #ifdef RWKVB200_DEVTOOLS
 #define W6C_STAMP(n) do { if (dbg && tid == 0 && item == gridDim.x / 2 && c == 2) dbg[n] = clock64(); } while (0)
@@ -226,8 +264,9 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   const bool tok_lane = lane < 16;            // lower lane halves hold token rows, upper halves state rows
 
   if (tid == 0) {
-    // MMA batch 1 has three accumulators and three issuing threads (of warps 0, 1, 2) and completes with all arrivals
-    mbar_init(&sm.bar_1, 3); mbar_init(&sm.bar_2, 1); mbar_init(&sm.bar_in, 1);
+    // MMA batch 1 has two accumulators and two issuing threads (of warps 0 and 1) and completes with both arrivals
+    mbar_init(&sm.bar_1, 2); mbar_init(&sm.bar_2, 1); mbar_init(&sm.bar_in, 1);
+    mbar_init(&sm.bar_state, 1); mbar_init(&sm.bar_free, 1);
     fence_mbar_init();
   }
   if (warp == 0) tmem_alloc(&sm.tmem_base, 128);
@@ -247,96 +286,150 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   const T* raw_v = reinterpret_cast<const T*>(sm.vt[0]);
   const T* raw_w = reinterpret_cast<const T*>(sm.at[0]);
 
-  // Work items.  parts == 1: an item is a (batch, head) unit and the grid has one CTA per unit.  parts > 1 (more
-  // units than the two CTAs per SM can hold at once): every unit is `parts` items, consecutive stretches of its
-  // chunks, on a persistent grid whose free CTAs take the next item from a counter (handoff_flags[n_units]); all
-  // first stretches come first in that order, so when a stretch is taken the one before it has been taken
-  // already, by a CTA that is running, and the state travels between them through `handoff` (handoff_flags[unit]
-  // counts the stretches of the unit that are done).  Shorter items even out the last round of CTAs (512 units
-  // on 296 slots: 1.75 unit times instead of 2).
+  // Work items.  parts == 1: an item is a (batch, head) unit and the grid has one CTA per unit.  parts > 1: every unit is
+  // `parts` items, stretches of `per_item` of its chunks, on a persistent grid whose CTAs take items from a counter
+  // (handoff_flags[n_units]), one ahead of the one they work on; all first stretches come first in that order.  The state
+  // travels from stretch to stretch through `states`, where a training forward leaves it anyway, or `handoff`;
+  // handoff_flags[unit] counts the stretches of the unit that have left theirs (MARKED: one of them left the decay range).
+  // The first item of those not done yet waits for none, and its CTA is at work on it: the wait needs no assumption
+  // about which CTAs are resident.  A chunk needs the state only for its second batch of products and has its own
+  // contribution to it by then, so one chunk waits for another only for a state to be fetched, scaled and left.
+  // RELAY (parts == 1): the CTAs of a cluster, at most eight, work on the chunks of one unit in turn, and the state goes from
+  // one's registers into the shared memory of the next.  A chunk then takes the unit a state's way from barrier to
+  // barrier (1.6 us) instead of its whole chain of phases (4.3): 1 sequence of 4096 tokens, 32 heads, bfloat16, 273 -> 101 us;
+  // 148 units of 777 tokens, where two CTAs to a unit fill the device, 66 -> 57.
   const int n_items = parts * n_units;
   bool ok = true;
   uint32_t n_done = 0;      // chunks this CTA has worked on: every barrier completes once per chunk
-  for (bool first = true; ok; first = false) {
+  uint32_t n_fetched = 0, n_sent = 0;      // RELAY: states received and sent
+  const int rank = RELAY ? (int)blockIdx.y : 0, n_cta = RELAY ? (int)gridDim.y : 1;
+  const uint32_t succ = RELAY ? (rank + 1 == n_cta ? 0 : rank + 1) : 0, pred = RELAY ? (rank ? rank - 1 : n_cta - 1) : 0;
+  if constexpr (RELAY) cluster_sync();      // the barriers of all CTAs are set up
+  int item = blockIdx.x;
   if (parts > 1) {
     if (tid == 0) sm.next_item = atomicAdd(handoff_flags + n_units, 1);
     __syncthreads();
-  } else if (!first) {
-    break;
+    item = sm.next_item;
   }
-  const int item = parts > 1 ? sm.next_item : (int)blockIdx.x;
-  if (item >= n_items) break;
-  const int unit = item % n_units, part = item / n_units;
-  const int bi = unit / H, hi = unit % H;
-  const int Tn = PACKED ? seqs.len[bi] : Tn_dense;
-  const int tok0 = PACKED ? seqs.start[bi] : 0;       // first token row of the sequence in its batch row
-  const int brow = PACKED ? 0 : bi;
-  const long long base = (((long long)brow * Tn_dense + tok0) * H + hi) * HS;   // Tn_dense: rows per batch row
-  const int NT = (Tn + L - 1) / L;
-  const size_t nts = PACKED ? (size_t)seqs.nts : (size_t)(NT + 1);
-  // this item's chunks: c_lo .. c_hi - 1; the unit's last item is the one that reaches NT
-  const int c_lo = (int)((long long)NT * part / parts), c_hi = (int)((long long)NT * (part + 1) / parts);
-  const bool last_part = part == parts - 1;
-  // (a stretch without a chunk, in a sequence shorter than `parts` chunks, just passes the state on)
+  struct Stretch {
+    int unit, part, bi, hi, Tn, tok0, brow, NT, c_lo, c_hi;
+  };
+  auto stretch = [&](int i) {
+    Stretch x;
+    x.unit = i % n_units; x.part = i / n_units;
+    x.bi = x.unit / H; x.hi = x.unit % H;
+    x.Tn = PACKED ? seqs.len[x.bi] : Tn_dense;
+    x.tok0 = PACKED ? seqs.start[x.bi] : 0;       // first token row of the sequence in its batch row
+    x.brow = PACKED ? 0 : x.bi;
+    x.NT = (x.Tn + L - 1) / L;
+    x.c_lo = x.part * per_item;      // the chunks c_lo .. c_hi - 1; none in a sequence that ends before them
+    x.c_hi = min(x.c_lo + per_item, x.NT);
+    return x;
+  };
+  auto load_in = [&](const Stretch& x, int c) {      // one thread; rows past the end of the sequence arrive as zeros
+    mbar_expect_tx(&sm.bar_in, 4 * 64 * 64 * (uint32_t)sizeof(T));
+    tma_load_4d(sm.at[0], &tmap_w, &sm.bar_in, 0, x.tok0 + c * L, x.hi, x.brow);
+    tma_load_4d(sm.vt[0], &tmap_v, &sm.bar_in, 0, x.tok0 + c * L, x.hi, x.brow);
+    tma_load_4d(sm.rt[0], &tmap_r, &sm.bar_in, 0, x.tok0 + c * L, x.hi, x.brow);
+    tma_load_4d(sm.kt[0], &tmap_k, &sm.bar_in, 0, x.tok0 + c * L, x.hi, x.brow);
+  };
+  if (item < n_items && warp == 0 && elect_one()) {
+    const Stretch x = stretch(item);
+    if (x.c_lo + rank < x.c_hi) load_in(x, x.c_lo + rank);
+  }
+  while (item < n_items && ok) {
+  const Stretch cur = stretch(item);
+  const int unit = cur.unit, part = cur.part, hi = cur.hi, Tn = cur.Tn, c_lo = cur.c_lo, c_hi = cur.c_hi;
+  const long long base = (((long long)cur.brow * Tn_dense + cur.tok0) * H + hi) * HS;   // Tn_dense: rows per batch row
+  const size_t nts = PACKED ? (size_t)seqs.nts : (size_t)(cur.NT + 1);
+  const bool last_part = c_hi == cur.NT;
+  if (c_lo < c_hi || c_hi == 0) {      // (c_hi == 0: an empty sequence, which just hands its state on)
   // per-thread slice of u (4 channels) for the diagonal term
   const float4 u4 = load4_as<T>(u, hi * HS + 4 * c4, typed);
+  int marked = Tn < SHORT_SEQ;      // thread-wise until the end of the item
 
   // ---- state at the item's first chunk: rows k on the upper lane halves, this warp's 32 columns
   float sreg[CW];
 #pragma unroll
   for (int j = 0; j < CW; ++j) sreg[j] = 0.f;
-  if (part > 0) {
-    // wait for the stretch before this one (taken before this item, by a CTA that is running): bounded
-    if (tid == 0) {
-      uint32_t polls = 0;
-      int seen = 0;
-      while (true) {
-        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(handoff_flags + unit) : "memory");
-        if (seen >= part || ++polls > (WAIT_LIMIT << 2)) break;
-        __nanosleep(200);
-      }
-      if (seen < part) { atomicExch(status, 405); sm.handoff_ok = 0; } else { sm.handoff_ok = 1; }
-    }
-    __syncthreads();
-    ok = sm.handoff_ok != 0;
-    if (!tok_lane && ok) {
-      const float* S = handoff + (((size_t)unit * HS) + srow) * HS + CW * hsel;
-#pragma unroll
-      for (int j = 0; j < CW; j += 4) {
-        const float4 fv = __ldcg(reinterpret_cast<const float4*>(S + j));
-        sreg[j] = fv.x; sreg[j + 1] = fv.y; sreg[j + 2] = fv.z; sreg[j + 3] = fv.w;
-      }
-    }
-  } else if (!tok_lane && s0 && n_state > 0) {
-    const long long S = ((state_row(smap, n_state, bi) * H + hi) * HS + srow) * HS + CW * hsel;
+  if (part == 0 && rank == 0 && !tok_lane && s0 && n_state > 0) {
+    const long long S = ((state_row(smap, n_state, cur.bi) * H + hi) * HS + srow) * HS + CW * hsel;
 #pragma unroll
     for (int j = 0; j < CW; j += 4) {
       const float4 fv = load4_as<T>(s0, S + j, typed);
       sreg[j] = fv.x; sreg[j + 1] = fv.y; sreg[j + 2] = fv.z; sreg[j + 3] = fv.w;
     }
   }
-
+  // where the state before chunk c travels
+  auto state_slot = [&](int c) {
+    return (states ? states + ((size_t)unit * nts + c) * (HS * HS) : handoff + (size_t)unit * (HS * HS)) + srow * HS + CW * hsel;
+  };
+  // The state the item's first chunk starts from: what the stretch before it has left (bounded wait; all threads).
+  auto fetch_state = [&]() {
+    if (tid == 0) {
+      int seen = 0;
+      uint32_t polls = 0;
+      while (true) {
+        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(seen) : "l"(handoff_flags + unit) : "memory");
+        if ((seen & ~MARKED) >= part || ++polls > (WAIT_LIMIT << 2)) break;
+        __nanosleep(100);
+      }
+      if ((seen & ~MARKED) < part) { atomicExch(status, 405); seen = -1; }
+      sm.state_seen = seen;
+    }
+    __syncthreads();
+    const int seen = sm.state_seen;
+    if (seen < 0) return false;
+    marked |= seen & MARKED;
+    if (!tok_lane) {
+      const float* S = state_slot(c_lo);
+#pragma unroll
+      for (int j = 0; j < CW; j += 4) {
+        const float4 fv = __ldcg(reinterpret_cast<const float4*>(S + j));
+        sreg[j] = fv.x; sreg[j + 1] = fv.y; sreg[j + 2] = fv.z; sreg[j + 3] = fv.w;
+      }
+    }
+    return true;
+  };
+  // RELAY: a row piece of the state travels through the 2 x 64 bytes that its S~0 takes up as hi and lo parts
+  auto piece = [&](int j) { return tile_chunk_off(srow, 4 * hsel + (j & 3)) + (j >> 2) * TILE_BYTES; };
+  auto receive_state = [&]() {
+    if (!mbar_wait_cluster(&sm.bar_state, n_fetched & 1, status, 406)) return false;
+    if (!tok_lane) {
+#pragma unroll
+      for (int j = 0; j < CW / 4; ++j) {
+        const float4 fv = *reinterpret_cast<const float4*>(sm.st[0] + piece(j));
+        sreg[4 * j] = fv.x; sreg[4 * j + 1] = fv.y; sreg[4 * j + 2] = fv.z; sreg[4 * j + 3] = fv.w;
+      }
+    }
+    return true;
+  };
+  auto send_state = [&](const float (&x)[CW]) {      // the CTA of the next chunk has no more use for its S~0
+    if (!tok_lane) {
+      const uint32_t to = cluster_addr(smem_u32(sm.st[0]), succ), bar = cluster_addr(smem_u32(&sm.bar_state), succ);
+#pragma unroll
+      for (int j = 0; j < CW / 4; ++j)
+        store_async_16(to + piece(j), make_float4(x[4 * j], x[4 * j + 1], x[4 * j + 2], x[4 * j + 3]), bar);
+    }
+  };
   auto keep_state = [&](int c) {      // the state before chunk c
-    float* dst = states + (((size_t)unit * nts + c) * HS + srow) * HS + CW * hsel;
+    float* dst = state_slot(c);
 #pragma unroll
     for (int j = 0; j < CW; j += 4)
       *reinterpret_cast<float4*>(dst + j) = make_float4(sreg[j], sreg[j + 1], sreg[j + 2], sreg[j + 3]);
   };
-  if (states && !tok_lane && part == 0) keep_state(0);
+  if (states && !tok_lane && part == 0 && rank == 0) keep_state(0);
+  if (RELAY && rank > 0 && rank < c_hi && warp == 1 && elect_one()) mbar_arrive_cluster(cluster_addr(smem_u32(&sm.bar_free), pred));
 
-  auto load_in = [&](int c) {      // tid 0; rows past the end of the sequence arrive as zeros
-    mbar_expect_tx(&sm.bar_in, 4 * 64 * 64 * (uint32_t)sizeof(T));
-    tma_load_4d(sm.at[0], &tmap_w, &sm.bar_in, 0, tok0 + c * L, hi, brow);
-    tma_load_4d(sm.vt[0], &tmap_v, &sm.bar_in, 0, tok0 + c * L, hi, brow);
-    tma_load_4d(sm.rt[0], &tmap_r, &sm.bar_in, 0, tok0 + c * L, hi, brow);
-    tma_load_4d(sm.kt[0], &tmap_k, &sm.bar_in, 0, tok0 + c * L, hi, brow);
-  };
-  if (warp == 0 && elect_one() && ok && c_lo < c_hi) load_in(c_lo);
-
-  for (int c = c_lo; c < c_hi && ok; ++c, ++n_done) {
+  for (int c = c_lo + rank; c < c_hi && ok; c += n_cta, ++n_done) {
     const int t0 = c * L;
     const uint32_t par = n_done & 1;
     W6C_STAMP(0);
+    // the next item is taken here and handed to the others once it has arrived
+    const bool take = !RELAY && parts > 1 && c + 1 == c_hi;
+    int ticket = 0;
+    if (take && tid == NTHR - 1) ticket = atomicAdd(handoff_flags + n_units, 1);
+    if (RELAY && c > 0 && warp == 0 && elect_one()) mbar_expect_tx(&sm.bar_state, HS * HS * (uint32_t)sizeof(float));
     // ---- the raw rows of the chunk have landed: this thread's w and v elements
     ok = mbar_wait(&sm.bar_in, par, status, 403) && ok;
     float4 gw[NE], vv4[NE];
@@ -344,9 +437,15 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     for (int n = 0; n < NE; ++n) {
       const int e = tid + NTHR * n, row = e >> 4;
       gw[n] = load4_shared(raw_w + row * 64 + 4 * c4);
-      vv4[n] = load4_shared(raw_v + row * 64 + 4 * c4);
-      if (PACKED && t0 + row >= Tn) vv4[n] = make_float4(0.f, 0.f, 0.f, 0.f);      // the next sequence's row
+      if constexpr (has_lo<T>()) {
+        vv4[n] = load4_shared(raw_v + row * 64 + 4 * c4);
+        if (PACKED && t0 + row >= Tn) vv4[n] = make_float4(0.f, 0.f, 0.f, 0.f);      // the next sequence's row
+      } else {
+        // bfloat16 rows have arrived as the tile that the products read
+        if (PACKED && t0 + row >= Tn) *reinterpret_cast<uint2*>(sm.vt[0] + tile_off(row, 4 * c4)) = make_uint2(0u, 0u);
+      }
     }
+    if (warp == 1 && elect_one()) bulk_wait_read();      // the last y rows have left the space of gs
     __syncthreads();      // every raw v element is in registers: the split v tiles may overwrite the rows
     // ---- pass W: g and its prefix sums; pass V
 #pragma unroll
@@ -358,7 +457,7 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
                         -LOG2E * ex2(LOG2E * gw[n].w));
       gw[n] = f;
       *reinterpret_cast<float4*>(&sm.gs[row * NROW + 4 * c4]) = f;
-      store_split4<has_lo<T>()>(sm.vt[0], sm.vt[1], row, 4 * c4, vv4[n]);
+      if constexpr (has_lo<T>()) store_split4(sm.vt[0], sm.vt[1], row, 4 * c4, vv4[n]);
     }
     __syncthreads();
     W6C_STAMP(1);
@@ -385,13 +484,7 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
       e0 = ex2(fmaxf(tot0, EXP2_FLOOR));
       dlast = ex2(fmaxf(tot1, EXP2_FLOOR));
       // a half-chunk decay sum beyond the limit: the unit is recomputed by the float32 recurrence
-      if (hsel == 0 && (fminf(tot0, tot1) < -DECAY_LIMIT * LOG2E || Tn < SHORT_SEQ)) flags[unit] = 1;
-    }
-    // ---- S~0 = e^{gref} S0 stays in registers (fp32); hi/lo bf16 tiles for the r~ S~0 product
-    if (!tok_lane) {
-#pragma unroll
-      for (int j = 0; j < CW; ++j) sreg[j] *= e0;
-      store_split_row<CW>(sm.st[0], sm.st[1], srow, CW * hsel, sreg);
+      marked |= fminf(tot0, tot1) < -DECAY_LIMIT * LOG2E;
     }
     W6C_STAMP(3);
     // ---- pass RK: scaled r, k (split hi/lo) and the diagonal term
@@ -420,111 +513,171 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
       for (int m = 8; m >= 1; m >>= 1) dg += __shfl_xor_sync(0xffffffffu, dg, m);
       if (c4 == 0) sm.dgs[row] = dg;
     }
-    // ask for the next chunk's rows to be brought into L2 while this chunk is in its MMA phases
-    if (warp == 0 && elect_one() && c + 1 < c_hi) {
-      tma_prefetch_4d(&tmap_w, 0, tok0 + t0 + L, hi, brow);
-      tma_prefetch_4d(&tmap_v, 0, tok0 + t0 + L, hi, brow);
-      tma_prefetch_4d(&tmap_r, 0, tok0 + t0 + L, hi, brow);
-      tma_prefetch_4d(&tmap_k, 0, tok0 + t0 + L, hi, brow);
-    }
+    if (take && tid == NTHR - 1) sm.next_item = ticket;
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
 
     W6C_STAMP(4);
-    // ---- batch 1: r~ k~^T (columns 0..63), y = r~ S~0 (columns 64.., lower), k~^T v (upper)
-    if (warp < 3 && elect_one()) {
+    // ---- batch 1: r~ k~^T (columns 0..63), k~^T v (columns 64.., upper halves)
+    if (warp < 2 && elect_one()) {
       tc_fence_after();
-      if (warp == 0)      umma_split<64, 64, 0, 0>(tmem_addr(tm, 0, 0), smem_u32(sm.rt[0]), smem_u32(sm.kt[0]), false);
-      else if (warp == 1) umma_split<64, 64, 0, 1>(tmem_addr(tm, 0, 64), smem_u32(sm.rt[0]), smem_u32(sm.st[0]), false);
-      else                umma_split<64, 64, 1, 1, true, has_lo<T>()>(tmem_addr(tm, 16, 64), smem_u32(sm.kt[0]), smem_u32(sm.vt[0]), false);
+      if (warp == 0) umma_split<64, 64, 0, 0>(tmem_addr(tm, 0, 0), smem_u32(sm.rt[0]), smem_u32(sm.kt[0]), false);
+      else           umma_split<64, 64, 1, 1, true, has_lo<T>()>(tmem_addr(tm, 16, 64), smem_u32(sm.kt[0]), smem_u32(sm.vt[0]), false);
       umma_commit(&sm.bar_1);
     }
+    // ask for the next chunk's rows to be brought into L2 while this chunk is in its MMA phases
+    if (warp == 2 && elect_one()) {
+      Stretch x = cur;
+      int cn = c + n_cta;
+      if (take && sm.next_item < n_items) { x = stretch(sm.next_item); cn = x.c_lo; }
+      if (cn < x.c_hi) {
+        tma_prefetch_4d(&tmap_w, 0, x.tok0 + cn * L, x.hi, x.brow);
+        tma_prefetch_4d(&tmap_v, 0, x.tok0 + cn * L, x.hi, x.brow);
+        tma_prefetch_4d(&tmap_r, 0, x.tok0 + cn * L, x.hi, x.brow);
+        tma_prefetch_4d(&tmap_k, 0, x.tok0 + cn * L, x.hi, x.brow);
+      }
+    }
+    const bool need_state = RELAY ? c > 0 : part > 0 && c == c_lo, hand_on = !RELAY && c + 1 == c_hi && !last_part;
+    if (!RELAY && need_state) ok = fetch_state() && ok;
     ok = mbar_wait(&sm.bar_1, par, status, 401) && ok;
     tc_fence_after();
     W6C_STAMP(5);
     if (ok) {
-      // A rows (lower halves of columns 0..63): strictly lower part plus the diagonal term, split hi/lo
+      // state rows: S~0 = e^{gref} S0, and (k~^T v on the upper halves of columns 64..127) S_L = e^{glast-gref} (S~0 + k~^T v)
+      float next_s[CW];
+      {
+        uint32_t rr[CW];
+        tmem_ld<CW>(tm_ys, rr);
+        tmem_ld_wait();
+        const bool send = RELAY && c + 1 < c_hi;      // (what can be waited for before the state arrives is)
+        if (send) ok = mbar_wait_cluster(&sm.bar_free, n_sent & 1, status, 407);
+        if (RELAY && need_state) ok = receive_state() && ok;
+#pragma unroll
+        for (int j = 0; j < CW; ++j) {
+          sreg[j] = __fmul_rn(sreg[j], e0);
+          next_s[j] = (sreg[j] + __uint_as_float(rr[j])) * dlast;
+        }
+        if (send && ok) send_state(next_s);
+      }
+      // A rows (lower halves of columns 0..63), strictly lower part plus the diagonal term, and S~0 rows: split, stored
+      float x[CW];
+      load_masked_row<CW>(tm_a, wq, hsel, lane & 15, tok_lane ? sm.dgs[srow] : 0.f, tok_lane, sreg, x);
+      unsigned char* hi_t = tok_lane ? sm.at[0] : sm.st[0];
+      store_split_row<CW>(hi_t, hi_t + TILE_BYTES, srow, CW * hsel, x);
+#pragma unroll
+      for (int j = 0; j < CW; ++j) sreg[j] = next_s[j];
+      if (hand_on && !tok_lane) { keep_state(c + 1); __threadfence(); }
+    }
+    fence_async_smem();
+    tc_fence_before();
+    if (need_state) ++n_fetched;
+    if (c + 1 < c_hi) ++n_sent;
+    if (hand_on) marked = __syncthreads_or(marked);
+    ok = __syncthreads_and(ok);
+
+    W6C_STAMP(6);
+    // ---- batch 2: y = r~ S~0 + A v
+    if (warp == 0 && elect_one() && ok) {
+      tc_fence_after();
+      umma_split<64, 64, 0, 1>(tmem_addr(tm, 0, 64), smem_u32(sm.rt[0]), smem_u32(sm.st[0]), false);
+      umma_split<64, 64, 0, 1, true, has_lo<T>()>(tmem_addr(tm, 0, 64), smem_u32(sm.at[0]), smem_u32(sm.vt[0]), true);
+      umma_commit(&sm.bar_2);
+    }
+    if (hand_on && warp == 1 && elect_one() && ok)
+      asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(handoff_flags + unit), "r"((part + 1) | (marked ? MARKED : 0)) : "memory");
+    // the state of the next chunk's start, stored here because the next proxy fence, which waits for global stores too, is
+    // most of a chunk away
+    if (states && !tok_lane && ok && !hand_on) keep_state(c + 1);
+    ok = mbar_wait(&sm.bar_2, par, status, 402) && ok;
+    tc_fence_after();
+    W6C_STAMP(7);
+    if (RELAY && c + n_cta < c_hi && warp == 1 && elect_one() && ok)      // and so has S~0
+      mbar_arrive_cluster(cluster_addr(smem_u32(&sm.bar_free), pred));
+    if (warp == 0 && elect_one() && ok) {      // the tiles of this chunk have been read for the last time
+      if (c + n_cta < c_hi) {
+        load_in(cur, c + n_cta);
+      } else if (take && sm.next_item < n_items) {
+        const Stretch x = stretch(sm.next_item);
+        if (x.c_lo < x.c_hi) load_in(x, x.c_lo);
+      }
+    }
+    // the y rows as swizzled tiles (of 32 channels each in float32) in the prefix-sum area
+    unsigned char* yt = reinterpret_cast<unsigned char*>(sm.gs);
+    if (ok && y) {
       uint32_t rr[CW];
-      load_store_masked_row<CW>(tm_a, wq, hsel, lane & 15, tok_lane ? sm.dgs[srow] : 0.f, sm.at[0], srow, tok_lane);
-      // state rows (k~^T v on the upper halves of columns 64..127): S_L = e^{glast-gref} (S~0 + k~^T v)
       tmem_ld<CW>(tm_ys, rr);
       tmem_ld_wait();
-      if (!tok_lane) {
+      if (tok_lane) {
 #pragma unroll
-        for (int j = 0; j < CW; ++j) sreg[j] = (sreg[j] + __uint_as_float(rr[j])) * dlast;
+        for (int j = 0; j < CW; j += 16 / sizeof(T)) {
+          uint4 u = make_uint4(rr[j], rr[j + 1], rr[j + 2], rr[j + 3]);
+          if constexpr (sizeof(T) == 2) {
+            auto pair = [&](int i) {
+              const float a = __uint_as_float(rr[j + i]), b = __uint_as_float(rr[j + i + 1]);
+              const T p[2] = {from_f32<T>(a), from_f32<T>(b)};
+              return *reinterpret_cast<const uint32_t*>(p);
+            };
+            u = make_uint4(pair(0), pair(2), pair(4), pair(6));
+          }
+          const int q = (CW * hsel + j) * (int)sizeof(T) / 16;      // 16-byte piece of the row
+          *reinterpret_cast<uint4*>(yt + (q >> 3) * TILE_BYTES + tile_chunk_off(srow, q & 7)) = u;
+        }
       }
     }
     fence_async_smem();
     tc_fence_before();
     ok = __syncthreads_and(ok);
-
-    W6C_STAMP(6);
-    // ---- batch 2: y += A v
-    if (warp == 0 && elect_one() && ok) {
-      tc_fence_after();
-      umma_split<64, 64, 0, 1, true, has_lo<T>()>(tmem_addr(tm, 0, 64), smem_u32(sm.at[0]), smem_u32(sm.vt[0]), true);
-      umma_commit(&sm.bar_2);
-    }
-    // the state of the next chunk's start, stored here because the next proxy fence, which waits for global stores too, is
-    // most of a chunk away
-    if (states && !tok_lane && ok) keep_state(c + 1);
-    ok = mbar_wait(&sm.bar_2, par, status, 402) && ok;
-    tc_fence_after();
-    W6C_STAMP(7);
-    if (warp == 0 && elect_one() && ok && c + 1 < c_hi) load_in(c + 1);      // the tiles of this chunk have been read for the last time
-    if (ok) {
-      uint32_t rr[CW];
-      tmem_ld<CW>(tm_ys, rr);
-      tmem_ld_wait();
-      if (tok_lane) {     // stage the y rows (fp32) in the prefix-sum area, then store them coalesced
-#pragma unroll
-        for (int j = 0; j < CW; j += 4)
-          *reinterpret_cast<float4*>(&sm.gs[srow * NROW + CW * hsel + j]) =
-              make_float4(__uint_as_float(rr[j]), __uint_as_float(rr[j + 1]), __uint_as_float(rr[j + 2]),
-                          __uint_as_float(rr[j + 3]));
-      }
-    }
-    tc_fence_before();
-    ok = __syncthreads_and(ok);
     W6C_STAMP(8);
     if (y && ok) {
-#pragma unroll
-      for (int n = 0; n < NE; ++n) {
-        const int e = tid + NTHR * n, row = e >> 4, tok = t0 + row;
-        if (tok < Tn)
-          store4(y + base + (long long)tok * tstride + 4 * c4,
-                 *reinterpret_cast<const float4*>(&sm.gs[row * NROW + 4 * c4]));
+      constexpr int ROW = HS * (int)sizeof(T) / 16;      // pieces per row
+      if (PACKED && t0 + L > Tn) {      // the last rows of a box belong to the next sequence: row by row
+        for (int e = tid; e < 64 * ROW; e += NTHR) {
+          const int row = e / ROW, q = e % ROW;
+          if (t0 + row < Tn)
+            *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(y + base + (long long)(t0 + row) * tstride) + 16 * q) =
+                *reinterpret_cast<const uint4*>(yt + (q >> 3) * TILE_BYTES + tile_chunk_off(row, q & 7));
+        }
+        __syncthreads();      // the rows have been read
+      } else if (warp == 1 && elect_one()) {      // rows past the end of the tensor are clipped
+        for (int h = 0; h < ROW / 8; ++h)
+          tma_store_4d(&tmap_y, yt + h * TILE_BYTES, h * (128 / (int)sizeof(T)), cur.tok0 + t0, hi, cur.brow);
+        bulk_commit();
       }
     }
-    __syncthreads();
     W6C_STAMP(9);
   }
 #undef W6C_STAMP
-  // ---- the state after the item's last chunk: the unit's final state, or what its next stretch starts from
-  if (!tok_lane && ok) {
-    if (last_part) {
-      if (sT) {
-        const long long dst = (((long long)unit * HS) + srow) * HS + CW * hsel;
-#pragma unroll
-        for (int j = 0; j < CW; j += 4)
-          store4_as<T>(sT, dst + j, typed, make_float4(sreg[j], sreg[j + 1], sreg[j + 2], sreg[j + 3]));
-      }
-    } else {
-      float* dst = handoff + (((size_t)unit * HS) + srow) * HS + CW * hsel;
+  // ---- the unit's final state
+  if (last_part) {
+    if (!tok_lane && ok && sT && (!RELAY || max(c_hi - 1, 0) % n_cta == rank)) {
+      const long long dst = (((long long)unit * HS) + srow) * HS + CW * hsel;
 #pragma unroll
       for (int j = 0; j < CW; j += 4)
-        *reinterpret_cast<float4*>(dst + j) = make_float4(sreg[j], sreg[j + 1], sreg[j + 2], sreg[j + 3]);
+        store4_as<T>(sT, dst + j, typed, make_float4(sreg[j], sreg[j + 1], sreg[j + 2], sreg[j + 3]));
+    }
+    marked = __syncthreads_or(marked);
+    if constexpr (RELAY) {
+      if (tid == 0) store_cluster(cluster_addr(smem_u32(&sm.marks[rank]), 0), marked);
+      __syncwarp();
+      cluster_sync();      // from here on no CTA of the cluster touches another one
+      for (int i = 0; i < n_cta; ++i) marked |= sm.marks[i];
+    }
+    if (tid == 0 && rank == 0) flags[unit] = marked != 0;
+  }
+  } else if (warp == 0 && elect_one()) {      // no chunk in this item in which to take the next one
+    sm.next_item = atomicAdd(handoff_flags + n_units, 1);
+    if (sm.next_item < n_items) {
+      const Stretch x = stretch(sm.next_item);
+      if (x.c_lo < x.c_hi) load_in(x, x.c_lo);
     }
   }
-  if (!last_part) {
-    __threadfence();
-    __syncthreads();
-    if (warp == 0 && elect_one() && ok)
-      asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(handoff_flags + unit), "r"(part + 1) : "memory");
-  }
+  if (parts == 1) break;
   __syncthreads();      // the tiles and next_item are the next item's
+  item = sm.next_item;
+  __syncthreads();
   }   // items
+  if (warp == 1 && elect_one()) bulk_wait_all();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tm, 128);
@@ -1064,6 +1217,34 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   if (warp == 0) tmem_dealloc(tm, 256);
 }
 
+// How many CTAs relay the chunks of a unit: a power of two, as many as there are chunks for and as can all be resident with
+// the other units' clusters.
+template <auto Kernel>
+int relay_ctas(const DeviceFacts& dev, int smem, int n_units, int chunks) {
+  static std::atomic<int> resident[64][3];      // clusters of 2, 4, 8 that fit the device, plus one
+  int best = 2;
+  for (int i = 0; i < 3 && (i == 0 || chunks > (1 << i)); ++i) {
+    int n = resident[dev.dev][i].load(std::memory_order_acquire);
+    if (!n) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(1, 2 << i);
+      cfg.blockDim = 256;
+      cfg.dynamicSmemBytes = smem;
+      cudaLaunchAttribute attr;
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim.x = 1; attr.val.clusterDim.y = 2 << i; attr.val.clusterDim.z = 1;
+      cfg.attrs = &attr;
+      cfg.numAttrs = 1;
+      int fit = 0;
+      if (cudaOccupancyMaxActiveClusters(&fit, Kernel, &cfg) != cudaSuccess) { (void)cudaGetLastError(); fit = 0; }
+      n = fit + 1;
+      resident[dev.dev][i].store(n, std::memory_order_release);
+    }
+    if (n_units < n) best = 2 << i;
+  }
+  return best;
+}
+
 }  // namespace w6c
 
 int launch_wkv6_chunked_fwd(const void* r, const void* k, const void* v, const void* w, const void* u,
@@ -1076,44 +1257,50 @@ int launch_wkv6_chunked_fwd(const void* r, const void* k, const void* v, const v
   const bool packed = seq_start != nullptr;
   const int mapB = packed ? 1 : B, mapT = packed ? T_total : Tn;
   const Seqs seqs{seq_start, seq_len, (Tn + L - 1) / L + 1};
-  if (cuda_ok(cudaMemsetAsync(flags, 0, (size_t)B * H * sizeof(int), st))) return RWKVB200_E_CUDA;
   DeviceFacts dev;
   int e = device_facts(&dev);
   if (e) return e;
   int* status = dev.status;
   const int smem = (int)sizeof(FwdSmem) + 1024;
   const int esz = dtype == RWKVB200_F32 ? 4 : 2;
-  CUtensorMap tm_r, tm_k, tm_v, tm_w;
+  CUtensorMap tm_r, tm_k, tm_v, tm_w, tm_y;
   e = make_row_tensor_map(&tm_r, r, mapB, mapT, H, esz);
   if (!e) e = make_row_tensor_map(&tm_k, k, mapB, mapT, H, esz);
-  if (!e) e = make_row_tensor_map(&tm_v, v, mapB, mapT, H, esz);
+  if (!e) e = make_row_tensor_map(&tm_v, v, mapB, mapT, H, esz, dtype == RWKVB200_BF16);      // as a tile, where that is all v needs
   if (!e) e = make_row_tensor_map(&tm_w, w, mapB, mapT, H, esz);
+  if (!e) e = make_row_tensor_map(&tm_y, y ? y : r, mapB, mapT, H, esz, true);      // (unused without y)
   if (e) return e;
 #define W6C_DISPATCH_PACKED(...) do { if (packed) { constexpr bool P = true; __VA_ARGS__; } else { constexpr bool P = false; __VA_ARGS__; } } while (0)
   {
-    // more units than the two CTAs per SM hold at once: every unit as 2 or 4 stretches of its chunks on a
-    // persistent grid, whichever evens out the last round best (see the kernel); else one CTA per unit
     const int sms = dev.sms;
     const int n_units = B * H, slots = 2 * sms, NTmax = (Tn + L - 1) / L;
-    int parts = 1;
+    int per_item = NTmax;
     if (n_units > slots) {
+      // more units than the two CTAs per SM hold at once: every unit as 2 or 4 stretches of its chunks, whichever evens out
+      // the last round best
       double best = (double)((n_units + slots - 1) / slots);      // rounds, in unit times
       for (int p2 = 2; p2 <= 4 && NTmax >= 4 * p2; p2 *= 2) {
         const double rounds = (double)(((long long)n_units * p2 + slots - 1) / slots) / p2;
-        if (rounds < best - 1e-9) { best = rounds; parts = p2; }
+        if (rounds < best - 1e-9) { best = rounds; per_item = (NTmax + p2 - 1) / p2; }
       }
     }
+    const int parts = (NTmax + per_item - 1) / per_item;
     const int grid = parts > 1 ? slots : n_units;
-    if (parts > 1 && cuda_ok(cudaMemsetAsync(hflags, 0, ((size_t)n_units + 1) * sizeof(int), st))) return RWKVB200_E_CUDA;
+    if (parts > 1)
+      if (int rc = launch(w6c_clear_kernel, 1, 256, 0, st, 1, hflags, n_units + 1)) return rc;
     ProfScope prof("wkv6c_fwd_kernel", st);
-    // a unit per SM at most: 512 threads, since nothing else on the SM fills the waits of 256
-#define W6C_LAUNCH_FWD(NTHR)                                                                                          \
+    // few units: clusters of up to eight CTAs relay the chunks of one (see the kernel); a single chunk per unit: 512 threads, since
+    // nothing else on the SM fills the waits of 256
+#define W6C_LAUNCH_FWD(NTHR, RELAY)                                                                                \
     RWKVB200_DISPATCH_DTYPE(dtype, W6C_DISPATCH_PACKED(                                                               \
-      if (allow_smem<wkv6c_fwd_kernel<T, P, NTHR>>(dev, smem)) return RWKVB200_E_CUDA;                                \
-      if (int rc = launch(wkv6c_fwd_kernel<T, P, NTHR>, grid, NTHR, smem, st, 1,                                      \
+      if (allow_smem<wkv6c_fwd_kernel<T, P, NTHR, RELAY>>(dev, smem)) return RWKVB200_E_CUDA;                         \
+      const int cluster = RELAY ? relay_ctas<wkv6c_fwd_kernel<T, P, NTHR, RELAY>>(dev, smem, n_units, NTmax) : 1;     \
+      if (int rc = launch(wkv6c_fwd_kernel<T, P, NTHR, RELAY>, dim3(grid, cluster), NTHR, smem, st, cluster,          \
           (const T*)r, (const T*)k, (const T*)v, (const T*)w, u, s0, n_state, smap, (T*)y, sT, (int)typed, states, flags, \
-          tm_r, tm_k, tm_v, tm_w, mapT, H, seqs, n_units, parts, handoff, hflags, status, debug_stamp_buffer())) return rc))
-    if (n_units <= sms) W6C_LAUNCH_FWD(512) else W6C_LAUNCH_FWD(256)
+          tm_r, tm_k, tm_v, tm_w, tm_y, mapT, H, seqs, n_units, per_item, parts, handoff, hflags, status, debug_stamp_buffer())) return rc))
+    if (NTmax == 1 && n_units <= sms) W6C_LAUNCH_FWD(512, false)
+    else if (2 * n_units <= slots)    W6C_LAUNCH_FWD(256, true)
+    else                              W6C_LAUNCH_FWD(256, false)
 #undef W6C_LAUNCH_FWD
   }
   e = check_launch();
