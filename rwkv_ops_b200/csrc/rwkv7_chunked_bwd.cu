@@ -56,6 +56,7 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
     mbar_init(&sm.bar_m1, 1); mbar_init(&sm.bar_m2, 1);
     fence_mbar_init();
   }
+  if (tid == 32) tma_prefetch_maps(tmap_do);
   if (warp == 0) tmem_alloc(&sm.tmem_base, 128);
   tc_fence_before();
   __syncthreads();
@@ -231,6 +232,7 @@ r7c_bwd_scan_alone_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned 
     mbar_init(&sm.bar_m1, 1); mbar_init(&sm.bar_free, 1);
     fence_mbar_init();
   }
+  if (tid == 32) tma_prefetch_maps(tmap_do);
   if (warp == 0) tmem_alloc(&sm.tmem_base, 128);
   tc_fence_before();
   __syncthreads();
@@ -434,6 +436,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     mbar_init(&sm.bar_w, 1); mbar_init(&sm.bar_m1, 3); mbar_init(&sm.bar_m2, 2);
     fence_mbar_init();
   }
+  if (tid == 32) tma_prefetch_maps(tmap_w, tmap_do, tmap_v, tmap_dq, tmap_dw, tmap_dk, tmap_dv, tmap_da, tmap_db);
   if (warp == 0) tmem_alloc(&sm.tmem_base, 256);
   tc_fence_before();
   __syncthreads();

@@ -67,6 +67,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
     mbar_init(&sm.bar_m4, 1); mbar_init(&sm.bar_m5, 1);
     fence_mbar_init();
   }
+  if (tid == 32) tma_prefetch_maps(tmap_q, tmap_w, tmap_k, tmap_a, tmap_b, tmap_v);
   if (warp == 0) tmem_alloc(&sm.tmem_base, 256);
   tc_fence_before();
   __syncthreads();
@@ -613,6 +614,7 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
     mbar_init(&sm.bar_a, 1); mbar_init(&sm.bar_c, 1); mbar_init(&sm.bar_o, 1);
     fence_mbar_init();
   }
+  if (tid == 32) tma_prefetch_maps(tmap_v, tmap_o);
   if (warp == 0) tmem_alloc(&sm.tmem_base, 256);
   tc_fence_before();
   __syncthreads();
@@ -906,6 +908,7 @@ r7c_scan_fwd_alone_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsi
     mbar_init(&sm.bar_a, 1); mbar_init(&sm.bar_c, 1); mbar_init(&sm.bar_free, 1);
     fence_mbar_init();
   }
+  if (tid == 32) tma_prefetch_maps(tmap_v, tmap_o);
   if (warp == 0) tmem_alloc(&sm.tmem_base, 256);
   tc_fence_before();
   __syncthreads();

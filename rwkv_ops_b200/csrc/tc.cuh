@@ -152,6 +152,11 @@ __device__ __forceinline__ void tma_load_4d(void* dst_smem, const CUtensorMap* m
       ::"r"(smem_u32(dst_smem)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)),
         "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
 }
+// fetch tensor maps (kernel parameters) ahead of their first use: possible before earlier_kernels_done()
+template <typename... M>
+__device__ __forceinline__ void tma_prefetch_maps(const M&... maps) {
+  (..., [&] { asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&maps)) : "memory"); }());
+}
 // Tiled store of one swizzled tile; rows past the end of the tensor are clipped by the hardware.
 __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, const void* src_smem,
                                              int c0, int c1, int c2, int c3) {

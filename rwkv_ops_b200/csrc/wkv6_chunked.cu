@@ -269,6 +269,7 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     mbar_init(&sm.bar_state, 1); mbar_init(&sm.bar_free, 1);
     fence_mbar_init();
   }
+  if (tid == 32) tma_prefetch_maps(tmap_r, tmap_k, tmap_v, tmap_w, tmap_y);
   if (warp == 0) tmem_alloc(&sm.tmem_base, 128);
   tc_fence_before();
   __syncthreads();
@@ -760,6 +761,7 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     mbar_init(&sm.bar_in_a, 1); mbar_init(&sm.bar_in_b, 1); mbar_init(&sm.bar_in_c, 1); mbar_init(&sm.bar_s, 1);
     fence_mbar_init();
   }
+  if (tid == 32) tma_prefetch_maps(tmap_r, tmap_k, tmap_v, tmap_w, tmap_dy, tmap_s);
   if (warp == 0) tmem_alloc(&sm.tmem_base, 256);
   tc_fence_before();
   __syncthreads();
