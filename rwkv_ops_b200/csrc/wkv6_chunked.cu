@@ -60,9 +60,7 @@ constexpr int MARKED = 1 << 30;      // in the forward's count of stretches done
 // two values as packed bf16 pairs hi and lo with x = hi + lo (+ an error of about 2^-17 |x|)
 __device__ __forceinline__ void split_pair(float x0, float x1, uint32_t& hi, uint32_t& lo) {
   hi = pack_bf16(x0, x1);
-  float l0, l1;
-  fma2(l0, l1, bf16_lo(hi), bf16_hi(hi), -1.f, -1.f, x0, x1);      // x - hi, both in one instruction
-  lo = pack_bf16(l0, l1);
+  lo = pack_bf16(x0 - bf16_lo(hi), x1 - bf16_hi(hi));
 }
 // write 4 consecutive values (columns col .. col+3, col a multiple of 4) of `row` into a hi and a lo tile
 template <bool LO = true>
@@ -688,10 +686,15 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
 // backward: one CTA per (batch, head), chunks in reverse; `states` holds the forward state at every
 // chunk boundary (written by the forward kernel)
 // ---------------------------------------------------------------------------------------------
+// index of (row, channel) in a 64 x 64 fp32 array whose 16-byte pieces are permuted by the row: threads that own a row and
+// threads that own a channel both access it without bank conflicts
+__device__ __forceinline__ int sw64(int row, int c) { return row * 64 + ((((c >> 2) ^ (row & 7)) << 2) | (c & 3)); }
+
 struct BwdSmem {
   unsigned char rt[2][TILE_BYTES];    // r~            [token][k]
   unsigned char kt[2][TILE_BYTES];    // k~            [token][k]
-  // the twelve tiles below are dead once MMA batch 2 has completed; the fp32 staging arrays overlay them
+  // most of the twelve tiles below are used again for the fp32 staging arrays: v, S~0 and stril(dA) once the first part of
+  // MMA batch 2 has completed, dy and A once all of it has
   unsigned char vt[2][TILE_BYTES];    // v             [token][v]
   unsigned char dyt[2][TILE_BYTES];   // dy            [token][v]
   unsigned char at[2][TILE_BYTES];    // A             [i][j]
@@ -700,7 +703,7 @@ struct BwdSmem {
   unsigned char dst[2][TILE_BYTES];   // dS^           [k][v]
   float gs[L * NROW];                 // gi - gref (prefix of g relative to the reference point)
   float gg[L * NROW];                 // g log2(e)
-  float red_e[L * NROW];              // dr~ r~
+  float red_e[L * 64];                // dr~ r~ (sw64)
   float qtot[8][64];
   float rqtot[8][64];
   float pqtot[8][64];
@@ -718,7 +721,11 @@ struct BwdSmem {
 };
 static_assert(sizeof(BwdSmem) + 1024 <= 227 * 1024, "backward shared memory");
 
-constexpr int BWD_THREADS = 256;
+// 512 threads: half the work of a phase per thread.  That pays only without spills (with shared memory taken to its limit there
+// is no L1 for them): so the read-out takes eight columns at a time and stages them at once, and r and k are fetched again
+// for the output rows.  B 16, T 4096, 32 heads, float32: 2237 us with 256 threads, 2032 with 512 (2750 with 280 bytes of
+// spills).
+constexpr int BWD_THREADS = 512;
 
 template <typename T, bool PACKED>
 __global__ void __launch_bounds__(BWD_THREADS)
@@ -746,12 +753,12 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   const int srow = 16 * wq + (lane & 15);
   const bool lower = lane < 16;
   const int c4 = tid & 15;
-  // fp32 arrays that overlay the dead tiles after MMA batch 2
-  float* stage_dr = reinterpret_cast<float*>(sm.vt[0]);
-  float* stage_dk = stage_dr + L * NROW;
-  float* stage_dv = stage_dk + L * NROW;
-  float* stage_dw = stage_dv + L * NROW;
-  float* red_i = stage_dw + L * NROW;          // 5 x 17408 B = 87040 B <= 12 tiles
+  // fp32 arrays (sw64) over tiles that the products are done with
+  float* stage_dr = reinterpret_cast<float*>(sm.vt[0]);       // these three once the first part of batch 2 has completed
+  float* stage_dk = reinterpret_cast<float*>(sm.st[0]);
+  float* red_i = reinterpret_cast<float*>(sm.dat[0]);
+  float* stage_dv = reinterpret_cast<float*>(sm.dyt[0]);
+  float* stage_dw = reinterpret_cast<float*>(sm.at[0]);
   float* red_x = stage_dw;                     // X k~ per (token, channel), read before dw is staged over it
 
   if (tid == 0) {
@@ -876,7 +883,6 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     const int t0 = c * L;
     const uint32_t par = n_done & 1;
     W6C_STAMP(32);
-    // ---- r and k are read at pass RK and stay in registers until the u-term gradients at the end of the chunk
     float4 gw[NE], rr4[NE], kk4[NE];
     {
       ok = mbar_wait(&sm.bar_in_a, par, status, 413) && ok;
@@ -1068,33 +1074,43 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     ok = mbar_wait(&sm.bar_2a, par, status, 416) && ok;
     tc_fence_after();
     const int c0 = CW * hsel;
-    float o[CW], rd[CW], rs[CW];
+    float rs[CW];
     if (ok) {
-      // r1: the part of dk~ from inside the chunk (lower halves) / dr~ (upper halves), row of token srow; rx: the
-      // state part of dk~ (lower halves only)
-      uint32_t r1[CW], rx[CW];
-      tmem_ld<CW>(tm_c1, r1);
-      tmem_ld<CW>(tm_c3, rx);
-      tmem_ld_wait();
-      float th[CW], tl[CW];
-      tile_load_row<CW>(lower ? sm.kt[0] : sm.rt[0], srow, c0, th);
-      tile_load_row<CW>(lower ? sm.kt[1] : sm.rt[1], srow, c0, tl);
+      float* so = lower ? stage_dk : stage_dr;
+      float* sd = lower ? red_i : sm.red_e;
+      // RB columns at a time (registers); what the remaining products still read is not written over yet
+      constexpr int RB = 8;
 #pragma unroll
-      for (int j4 = 0; j4 < CW; j4 += 4) {
-        const int cc = c0 + j4;
-        const float4 gs4 = *reinterpret_cast<const float4*>(&sm.gs[srow * NROW + cc]);
-        const float4 gg4 = *reinterpret_cast<const float4*>(&sm.gg[srow * NROW + cc]);
-        const float gsv[4] = {gs4.x, gs4.y, gs4.z, gs4.w}, ggv[4] = {gg4.x, gg4.y, gg4.z, gg4.w};
+      for (int jb = 0; jb < CW; jb += RB) {
+        // r1: the part of dk~ from inside the chunk (lower halves) / dr~ (upper halves), row of token srow; rx: the
+        // state part of dk~ (lower halves only)
+        uint32_t r1[RB], rx[RB];
+        tmem_ld<RB>(tm_c1 + jb, r1);
+        tmem_ld<RB>(tm_c3 + jb, rx);
+        float th[RB], tl[RB];
+        tile_load_row<RB>(lower ? sm.kt[0] : sm.rt[0], srow, c0 + jb, th);
+        tile_load_row<RB>(lower ? sm.kt[1] : sm.rt[1], srow, c0 + jb, tl);
+        tmem_ld_wait();
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-          const int j = j4 + m;
-          const float d1 = gsv[m];                                   // gi - gref
-          const float tt = th[j] + tl[j];                            // k~ (lower) / r~ (upper)
-          const float x = __uint_as_float(r1[j]);
-          const float xs = lower ? __uint_as_float(rx[j]) : 0.f;
-          o[j] = (x + xs) * ex2(lower ? -d1 : d1 - ggv[m]);          // dk = dk~ e^{gref-gi},  dr = dr~ e^{ge-gref}
-          rd[j] = lower ? -x * tt : x * tt;                          // -(stril(dA)^T r~) k~,  dge = dr~ r~
-          rs[j] = xs * tt;                                           // X k~
+        for (int j4 = 0; j4 < RB; j4 += 4) {
+          const int cc = c0 + jb + j4;
+          const float4 gs4 = *reinterpret_cast<const float4*>(&sm.gs[srow * NROW + cc]);
+          const float4 gg4 = *reinterpret_cast<const float4*>(&sm.gg[srow * NROW + cc]);
+          const float gsv[4] = {gs4.x, gs4.y, gs4.z, gs4.w}, ggv[4] = {gg4.x, gg4.y, gg4.z, gg4.w};
+          float o[4], rd[4];
+#pragma unroll
+          for (int m = 0; m < 4; ++m) {
+            const int j = j4 + m;
+            const float d1 = gsv[m];                                   // gi - gref
+            const float tt = th[j] + tl[j];                            // k~ (lower) / r~ (upper)
+            const float x = __uint_as_float(r1[j]);
+            const float xs = lower ? __uint_as_float(rx[j]) : 0.f;
+            o[m] = (x + xs) * ex2(lower ? -d1 : d1 - ggv[m]);          // dk = dk~ e^{gref-gi},  dr = dr~ e^{ge-gref}
+            rd[m] = lower ? -x * tt : x * tt;                          // -(stril(dA)^T r~) k~,  dge = dr~ r~
+            rs[jb + j] = xs * tt;                                      // X k~
+          }
+          *reinterpret_cast<float4*>(&so[sw64(srow, cc)]) = make_float4(o[0], o[1], o[2], o[3]);
+          *reinterpret_cast<float4*>(&sd[sw64(srow, cc)]) = make_float4(rd[0], rd[1], rd[2], rd[3]);
         }
       }
     }
@@ -1102,15 +1118,10 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     tc_fence_after();
     W6C_STAMP(39);
     if (ok) {
-      float* so = lower ? stage_dk : stage_dr;
-      float* sd = lower ? red_i : sm.red_e;
+      if (lower) {
 #pragma unroll
-      for (int j4 = 0; j4 < CW; j4 += 4) {
-        const int cc = c0 + j4;
-        *reinterpret_cast<float4*>(&so[srow * NROW + cc]) = make_float4(o[j4], o[j4 + 1], o[j4 + 2], o[j4 + 3]);
-        *reinterpret_cast<float4*>(&sd[srow * NROW + cc]) = make_float4(rd[j4], rd[j4 + 1], rd[j4 + 2], rd[j4 + 3]);
-        if (lower)
-          *reinterpret_cast<float4*>(&red_x[srow * NROW + cc]) = make_float4(rs[j4], rs[j4 + 1], rs[j4 + 2], rs[j4 + 3]);
+        for (int j4 = 0; j4 < CW; j4 += 4)
+          *reinterpret_cast<float4*>(&red_x[sw64(srow, c0 + j4)]) = make_float4(rs[j4], rs[j4 + 1], rs[j4 + 2], rs[j4 + 3]);
       }
       // dv row of token srow (lower halves) / dS~0 row k = srow (upper halves)
       uint32_t r2[CW];
@@ -1122,9 +1133,21 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
       } else {
 #pragma unroll
         for (int j4 = 0; j4 < CW; j4 += 4)
-          *reinterpret_cast<float4*>(&stage_dv[srow * NROW + c0 + j4]) =
+          *reinterpret_cast<float4*>(&stage_dv[sw64(srow, c0 + j4)]) =
               make_float4(__uint_as_float(r2[j4]), __uint_as_float(r2[j4 + 1]), __uint_as_float(r2[j4 + 2]),
                           __uint_as_float(r2[j4 + 3]));
+      }
+    }
+    // r and k once more, for the u terms of the output rows (they would take registers from here on back to where they were
+    // scaled; these rows are in L2)
+#pragma unroll
+    for (int n = 0; n < NE; ++n) {
+      const int row = (tid + NTHR * n) >> 4;
+      rr4[n] = kk4[n] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (t0 + row < Tn) {
+        const long long off = base + (long long)(t0 + row) * tstride + 4 * c4;
+        rr4[n] = load4(r + off);
+        kk4[n] = load4(k + off);
       }
     }
     tc_fence_before();
@@ -1140,8 +1163,9 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
       float rv[PL], px[PL];
 #pragma unroll
       for (int j = 0; j < PL; ++j) {
-        rv[j] = red_i[(PL * part + j) * NROW + ch] + sm.red_e[(PL * part + j) * NROW + ch];
-        px[j] = red_x[(PL * part + j) * NROW + ch];
+        const int at = sw64(PL * part + j, ch);
+        rv[j] = red_i[at] + sm.red_e[at];
+        px[j] = red_x[at];
       }
       float run = 0.f, prun = 0.f;
 #pragma unroll
@@ -1161,9 +1185,9 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
 #pragma unroll
       for (int j = 0; j < PL; ++j) {
         const int ii = PL * part + j;
-        const float dg = (rv[j] + px[j]) + add + red_i[ii * NROW + ch];
+        const float dg = (rv[j] + px[j]) + add + red_i[sw64(ii, ch)];
         // stage_dw lies over red_x: this thread has read its entries above and writes the same ones
-        stage_dw[ii * NROW + ch] = dg * (LN2 * sm.gg[ii * NROW + ch]);      // dw = dg g, g = gg ln 2
+        stage_dw[sw64(ii, ch)] = dg * (LN2 * sm.gg[ii * NROW + ch]);      // dw = dg g, g = gg ln 2
       }
     }
     __syncthreads();
@@ -1177,14 +1201,14 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
         const long long off = base + (long long)tok * tstride + 4 * c4;
         const float4 r4 = rr4[n], k4 = kk4[n];
         const float dd = sm.dds[row];
-        float4 a = *reinterpret_cast<const float4*>(&stage_dr[row * NROW + 4 * c4]);
+        float4 a = *reinterpret_cast<const float4*>(&stage_dr[sw64(row, 4 * c4)]);
         a.x += dd * u4.x * k4.x; a.y += dd * u4.y * k4.y; a.z += dd * u4.z * k4.z; a.w += dd * u4.w * k4.w;
         store4(dr + off, a);
-        float4 b = *reinterpret_cast<const float4*>(&stage_dk[row * NROW + 4 * c4]);
+        float4 b = *reinterpret_cast<const float4*>(&stage_dk[sw64(row, 4 * c4)]);
         b.x += dd * r4.x * u4.x; b.y += dd * r4.y * u4.y; b.z += dd * r4.z * u4.z; b.w += dd * r4.w * u4.w;
         store4(dk + off, b);
-        store4(dv + off, *reinterpret_cast<const float4*>(&stage_dv[row * NROW + 4 * c4]));
-        store4(dw + off, *reinterpret_cast<const float4*>(&stage_dw[row * NROW + 4 * c4]));
+        store4(dv + off, *reinterpret_cast<const float4*>(&stage_dv[sw64(row, 4 * c4)]));
+        store4(dw + off, *reinterpret_cast<const float4*>(&stage_dw[sw64(row, 4 * c4)]));
         du_acc.x += dd * r4.x * k4.x; du_acc.y += dd * r4.y * k4.y;
         du_acc.z += dd * r4.z * k4.z; du_acc.w += dd * r4.w * k4.w;
       }
