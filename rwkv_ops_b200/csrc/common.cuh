@@ -135,6 +135,31 @@ int allow_smem(const DeviceFacts& f, int bytes) {
   return RWKVB200_OK;
 }
 
+// How many clusters of `ctas` CTAs of `Kernel` (2, 4 or 8, along y) the device holds at once, asked once per device and size; a
+// cluster's CTAs share a group of SMs, so this can be less than the SMs alone would allow.
+template <auto Kernel>
+int resident_clusters(const DeviceFacts& f, int threads, int smem, int ctas) {
+  static std::atomic<int> known[64][3];      // plus one
+  std::atomic<int>& slot = known[f.dev][ctas == 2 ? 0 : ctas == 4 ? 1 : 2];
+  int n = slot.load(std::memory_order_acquire);
+  if (!n) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, ctas);
+    cfg.blockDim = threads;
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 1; attr.val.clusterDim.y = ctas; attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int fit = 0;
+    if (cudaOccupancyMaxActiveClusters(&fit, Kernel, &cfg) != cudaSuccess) { (void)cudaGetLastError(); fit = 0; }
+    n = fit + 1;
+    slot.store(n, std::memory_order_release);
+  }
+  return n - 1;
+}
+
 // Whether a block's dynamic shared memory starts 1024-byte aligned, as swizzled tiles need it: it follows what the system
 // reserves and the kernel's static arrays.
 inline bool smem_starts_aligned(int reserved, int static_bytes) { return (reserved + static_bytes) % 1024 == 0; }

@@ -78,21 +78,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
   if (!done) atomicCAS(status, 0, code);
   return __all_sync(__activemask(), done) != 0;
 }
-// The same for a barrier at which threads of other CTAs of the cluster arrive or whose bytes come from there.
-__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, int* status, int code) {
-  bool done = false;
-  for (uint32_t i = 0; i < WAIT_LIMIT && !done; ++i) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    done = ok != 0;
-  }
-  if (!done) atomicCAS(status, 0, code);
-  return __all_sync(__activemask(), done) != 0;
-}
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -113,8 +98,10 @@ __device__ __forceinline__ void store_async_16(uint32_t addr, float4 f, uint32_t
   asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
                ::"r"(addr), "f"(f.x), "f"(f.y), "f"(f.z), "f"(f.w), "r"(bar) : "memory");
 }
+// An arrival at another CTA's barrier.  (With the scope of the cluster spelled out it waits for the global stores the thread has in
+// flight, a microsecond: the arrivals here follow reads of shared memory only.)
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void store_cluster(uint32_t addr, int x) {
   asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(addr), "r"(x) : "memory");

@@ -393,7 +393,7 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   // RELAY: a row piece of the state travels through the 2 x 64 bytes that its S~0 takes up as hi and lo parts
   auto piece = [&](int j) { return tile_chunk_off(srow, 4 * hsel + (j & 3)) + (j >> 2) * TILE_BYTES; };
   auto receive_state = [&]() {
-    if (!mbar_wait_cluster(&sm.bar_state, n_fetched & 1, status, 406)) return false;
+    if (!mbar_wait(&sm.bar_state, n_fetched & 1, status, 406)) return false;
     if (!tok_lane) {
 #pragma unroll
       for (int j = 0; j < CW / 4; ++j) {
@@ -550,7 +550,7 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
         tmem_ld<CW>(tm_ys, rr);
         tmem_ld_wait();
         const bool send = RELAY && c + 1 < c_hi;      // (what can be waited for before the state arrives is)
-        if (send) ok = mbar_wait_cluster(&sm.bar_free, n_sent & 1, status, 407);
+        if (send) ok = mbar_wait(&sm.bar_free, n_sent & 1, status, 407);
         if (RELAY && need_state) ok = receive_state() && ok;
 #pragma unroll
         for (int j = 0; j < CW; ++j) {
@@ -1247,27 +1247,9 @@ wkv6c_bwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
 // the other units' clusters.
 template <auto Kernel>
 int relay_ctas(const DeviceFacts& dev, int smem, int n_units, int chunks) {
-  static std::atomic<int> resident[64][3];      // clusters of 2, 4, 8 that fit the device, plus one
   int best = 2;
-  for (int i = 0; i < 3 && (i == 0 || chunks > (1 << i)); ++i) {
-    int n = resident[dev.dev][i].load(std::memory_order_acquire);
-    if (!n) {
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(1, 2 << i);
-      cfg.blockDim = 256;
-      cfg.dynamicSmemBytes = smem;
-      cudaLaunchAttribute attr;
-      attr.id = cudaLaunchAttributeClusterDimension;
-      attr.val.clusterDim.x = 1; attr.val.clusterDim.y = 2 << i; attr.val.clusterDim.z = 1;
-      cfg.attrs = &attr;
-      cfg.numAttrs = 1;
-      int fit = 0;
-      if (cudaOccupancyMaxActiveClusters(&fit, Kernel, &cfg) != cudaSuccess) { (void)cudaGetLastError(); fit = 0; }
-      n = fit + 1;
-      resident[dev.dev][i].store(n, std::memory_order_release);
-    }
-    if (n_units < n) best = 2 << i;
-  }
+  for (int n = 2; n <= 8 && (n == 2 || 2 * chunks > n); n *= 2)
+    if (n_units <= resident_clusters<Kernel>(dev, 256, smem, n)) best = n;
   return best;
 }
 
