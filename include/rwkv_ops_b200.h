@@ -169,6 +169,8 @@ int rwkvb200_rwkv7_decode_step(const void* r, const void* w, const void* k, cons
                                const void* a, const void* b, void* state, int state_dtype, void* o,
                                int B, int H, int head_size, int dtype, void* stream);
 
+/* The workspace is needed on the chunked path.  The float32 recurrence takes what this asks for to run faster, and takes less,
+ * or NULL, too. */
 size_t rwkvb200_rwkv7_fwd_workspace_bytes(int B, int T, int H, int head_size, int dtype, int algo);
 
 int rwkvb200_rwkv7_fwd(const void* r, const void* w, const void* k, const void* v,
@@ -178,6 +180,7 @@ int rwkvb200_rwkv7_fwd(const void* r, const void* w, const void* k, const void* 
                        int B, int T, int H, int head_size, int dtype, int head_first, int algo,
                        void* stream);
 
+/* Of what this asks for on the float32 recurrence, all but B*H*ceil(T/8) states is for speed. */
 size_t rwkvb200_rwkv7_bwd_workspace_bytes(int B, int T, int H, int head_size, int dtype, int algo);
 
 /* Backward.  Recomputes the forward from the inputs (the reference's autograd node also saves
@@ -197,15 +200,18 @@ int rwkvb200_rwkv7_bwd(const void* r, const void* w, const void* k, const void* 
 
 /* The forward and backward of a training step through the float32 recurrence, where the backward starts from states that
  * the forward has left instead of sweeping forward once more.  `states`: rwkvb200_rwkv7_states_bytes of device memory, the
- * state after every 16th token; the backward reads it, and its workspace is of the same size.  That size is 0 where there
+ * state after every 16th token, which the backward reads.  That size is 0 where there
  * is nothing to leave (up to 16 tokens, the chunked path, bfloat16 at head size 64): use the plain backward there, this
- * one returns RWKVB200_E_UNSUPPORTED.  Same results as rwkvb200_rwkv7_fwd / _bwd. */
+ * one returns RWKVB200_E_UNSUPPORTED.  Workspace: rwkvb200_rwkv7_fwd_workspace_bytes for the forward (without KEEP; less, or
+ * NULL, is slower), rwkvb200_rwkv7_bwd_states_workspace_bytes for the backward (states_bytes of it are needed, the rest is for
+ * speed).  Same results as rwkvb200_rwkv7_fwd / _bwd. */
 size_t rwkvb200_rwkv7_states_bytes(int B, int T, int H, int head_size, int dtype, int algo);
+size_t rwkvb200_rwkv7_bwd_states_workspace_bytes(int B, int T, int H, int head_size, int dtype, int algo);
 
 int rwkvb200_rwkv7_fwd_states(const void* r, const void* w, const void* k, const void* v,
                               const void* a, const void* b,
                               const float* h0, int n_state, void* o, float* ht,
-                              float* states, size_t states_bytes,
+                              float* states, size_t states_bytes, void* workspace, size_t workspace_bytes,
                               int B, int T, int H, int head_size, int dtype, int head_first, int algo,
                               void* stream);
 

@@ -45,7 +45,8 @@ SIGNATURES = {
     "rwkvb200_rwkv7_bwd_workspace_bytes": (c_size_t, [_I] * 6),
     "rwkvb200_rwkv7_bwd": (c_int, [_P] * 6 + [_P, _I, _P, _P] + [_P] * 7 + [_P, _Z] + [_I] * 7 + [_P]),
     "rwkvb200_rwkv7_states_bytes": (c_size_t, [_I] * 6),
-    "rwkvb200_rwkv7_fwd_states": (c_int, [_P] * 6 + [_P, _I, _P, _P, _P, _Z] + [_I] * 7 + [_P]),
+    "rwkvb200_rwkv7_fwd_states": (c_int, [_P] * 6 + [_P, _I, _P, _P, _P, _Z, _P, _Z] + [_I] * 7 + [_P]),
+    "rwkvb200_rwkv7_bwd_states_workspace_bytes": (c_size_t, [_I] * 6),
     "rwkvb200_rwkv7_bwd_states": (c_int, [_P] * 6 + [_P, _I, _P, _P, _P, _Z] + [_P] * 7 + [_P, _Z] + [_I] * 7 + [_P]),
     "rwkvb200_rwkv7_bwd_static_capacity_bytes": (c_size_t, []),
     "rwkvb200_rwkv7_bwd_static": (c_int, [_P] * 6 + [_P, _I, _P, _P] + [_P] * 7 + [_I] * 6 + [_P]),

@@ -117,7 +117,7 @@ size_t rwkvb200_rwkv7_fwd_workspace_bytes(int B, int T, int H, int head_size, in
   if (check_common(B, T, H, head_size, dtype, true)) return 0;
   if (head_size == HS && resolve_r7_algo(algo, dtype, head_size) == RWKVB200_ALGO_CHUNKED)
     return r7c::fwd_workspace_bytes(B, T, H, (algo & RWKVB200_ALGO_KEEP) ? r7c::ALL_TILES : r7c::FWD_TILES);
-  return 0;
+  return resolve_r7_algo(algo, dtype, head_size) == RWKVB200_ALGO_RECURRENT ? rwkv7_block_scratch_bytes(B, T, H, dtype, head_size) : 0;
 }
 
 int rwkvb200_rwkv7_fwd(const void* r, const void* w, const void* k, const void* v,
@@ -136,14 +136,17 @@ int rwkvb200_rwkv7_fwd(const void* r, const void* w, const void* k, const void* 
   if (n_state != 0 && !h0) return RWKVB200_E_NULL;
   const void* ps[] = {r, w, k, v, a, b, h0, o, ht, workspace};
   for (const void* p : ps) if (p && !aligned16(p)) return RWKVB200_E_ALIGN;
-  const size_t need = rwkvb200_rwkv7_fwd_workspace_bytes(B, T, H, head_size, dtype, algo);
+  const size_t full = rwkvb200_rwkv7_fwd_workspace_bytes(B, T, H, head_size, dtype, algo);
+  const bool recurrent = resolve_r7_algo(algo, dtype, head_size) == RWKVB200_ALGO_RECURRENT;
+  const size_t need = recurrent ? 0 : full;      // the float32 recurrence runs without, slower
   if (workspace_bytes < need || (need && !workspace)) return RWKVB200_E_WORKSPACE;
   if (phases != PHASE_ALL && resolve_r7_algo(algo, dtype, head_size) != RWKVB200_ALGO_CHUNKED)
     return RWKVB200_E_UNSUPPORTED;
   switch (resolve_r7_algo(algo, dtype, head_size)) {
     case RWKVB200_ALGO_RECURRENT:
       return launch_rwkv7_block_fwd(r, w, k, v, a, b, n_state ? h0 : nullptr, n_state, o, ht, B, T, H, dtype,
-                                    head_first, (cudaStream_t)stream, head_size);
+                                    head_first, (cudaStream_t)stream, head_size, nullptr,
+                                    full && workspace_bytes >= full ? workspace : nullptr);
     case RWKVB200_ALGO_CHUNKED:
       if (dtype != RWKVB200_BF16) return RWKVB200_E_UNSUPPORTED;
       return launch_rwkv7_chunked_fwd(r, w, k, v, a, b, n_state ? h0 : nullptr, n_state, o, ht, workspace,
@@ -157,7 +160,7 @@ int rwkvb200_rwkv7_fwd(const void* r, const void* w, const void* k, const void* 
 size_t rwkvb200_rwkv7_bwd_workspace_bytes(int B, int T, int H, int head_size, int dtype, int algo) {
   if (check_common(B, T, H, head_size, dtype, true)) return 0;
   switch (resolve_r7_algo(algo, dtype, head_size)) {
-    case RWKVB200_ALGO_RECURRENT: return r7_ckpt_bytes(B, T, H, head_size);
+    case RWKVB200_ALGO_RECURRENT: return r7_ckpt_bytes(B, T, H, head_size) + rwkv7_block_scratch_bytes(B, T, H, dtype, head_size);
     case RWKVB200_ALGO_CHUNKED: return head_size == HS ? r7c::fwd_workspace_bytes(B, T, H, r7c::ALL_TILES) : 0;
     default: return 0;
   }
@@ -180,8 +183,10 @@ int rwkvb200_rwkv7_bwd(const void* r, const void* w, const void* k, const void* 
   if (n_state != 0 && !h0) return RWKVB200_E_NULL;
   const void* ps[] = {r, w, k, v, a, b, h0, d_o, d_ht, dr, dw, dk, dv, da, db, d_h0, workspace};
   for (const void* p : ps) if (p && !aligned16(p)) return RWKVB200_E_ALIGN;
-  const size_t need = rwkvb200_rwkv7_bwd_workspace_bytes(B, T, H, head_size, dtype, algo);
-  if (workspace_bytes < need || (need && !workspace)) return RWKVB200_E_WORKSPACE;
+  const size_t full = rwkvb200_rwkv7_bwd_workspace_bytes(B, T, H, head_size, dtype, algo);
+  const bool recurrent = resolve_r7_algo(algo, dtype, head_size) == RWKVB200_ALGO_RECURRENT;
+  const size_t ckpt = recurrent ? r7_ckpt_bytes(B, T, H, head_size) : full;      // the recurrence can do without the rest
+  if (workspace_bytes < ckpt || (ckpt && !workspace)) return RWKVB200_E_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
   if (phases_of(algo) != PHASE_ALL && resolve_r7_algo(algo, dtype, head_size) != RWKVB200_ALGO_CHUNKED)
     return RWKVB200_E_UNSUPPORTED;
@@ -189,7 +194,8 @@ int rwkvb200_rwkv7_bwd(const void* r, const void* w, const void* k, const void* 
     case RWKVB200_ALGO_RECURRENT:
       return launch_rwkv7_block_bwd(r, w, k, v, a, b, n_state ? h0 : nullptr, n_state, d_o, d_ht,
                                     reinterpret_cast<float*>(workspace), dr, dw, dk, dv, da, db, d_h0, B, T, H, dtype,
-                                    head_first, st, head_size);
+                                    head_first, st, head_size, nullptr,
+                                    full > ckpt && workspace_bytes >= full ? static_cast<char*>(workspace) + ckpt : nullptr);
     case RWKVB200_ALGO_CHUNKED:
       if (dtype != RWKVB200_BF16) return RWKVB200_E_UNSUPPORTED;
       return launch_rwkv7_chunked_bwd(r, w, k, v, a, b, n_state ? h0 : nullptr, n_state, d_o, d_ht,
@@ -210,7 +216,7 @@ size_t rwkvb200_rwkv7_states_bytes(int B, int T, int H, int head_size, int dtype
 int rwkvb200_rwkv7_fwd_states(const void* r, const void* w, const void* k, const void* v,
                               const void* a, const void* b,
                               const float* h0, int n_state, void* o, float* ht,
-                              float* states, size_t states_bytes,
+                              float* states, size_t states_bytes, void* workspace, size_t workspace_bytes,
                               int B, int T, int H, int head_size, int dtype, int head_first, int algo,
                               void* stream) {
   int e = check_common(B, T, H, head_size, dtype, true);
@@ -220,12 +226,19 @@ int rwkvb200_rwkv7_fwd_states(const void* r, const void* w, const void* k, const
   if (!r || !w || !k || !v || !a || !b || !o) return RWKVB200_E_NULL;
   if (n_state != 0 && n_state != 1 && n_state != B) return RWKVB200_E_SHAPE;
   if (n_state != 0 && !h0) return RWKVB200_E_NULL;
-  const void* ps[] = {r, w, k, v, a, b, h0, o, ht, states};
+  const void* ps[] = {r, w, k, v, a, b, h0, o, ht, states, workspace};
   for (const void* p : ps) if (p && !aligned16(p)) return RWKVB200_E_ALIGN;
   const size_t need = rwkvb200_rwkv7_states_bytes(B, T, H, head_size, dtype, algo);
+  const size_t scratch = rwkv7_block_scratch_bytes(B, T, H, dtype, head_size);
   if (states_bytes < need || (need && !states)) return RWKVB200_E_WORKSPACE;
   return launch_rwkv7_block_fwd(r, w, k, v, a, b, n_state ? h0 : nullptr, n_state, o, ht, B, T, H, dtype, head_first,
-                                (cudaStream_t)stream, head_size, need ? states : nullptr);
+                                (cudaStream_t)stream, head_size, need ? states : nullptr,
+                                scratch && workspace_bytes >= scratch ? workspace : nullptr);
+}
+
+size_t rwkvb200_rwkv7_bwd_states_workspace_bytes(int B, int T, int H, int head_size, int dtype, int algo) {
+  const size_t states = rwkvb200_rwkv7_states_bytes(B, T, H, head_size, dtype, algo);
+  return states ? align256(states) + rwkv7_block_scratch_bytes(B, T, H, dtype, head_size) : 0;
 }
 
 int rwkvb200_rwkv7_bwd_states(const void* r, const void* w, const void* k, const void* v,
@@ -246,10 +259,12 @@ int rwkvb200_rwkv7_bwd_states(const void* r, const void* w, const void* k, const
   if (n_state != 0 && !h0) return RWKVB200_E_NULL;
   const void* ps[] = {r, w, k, v, a, b, h0, d_o, d_ht, states, dr, dw, dk, dv, da, db, d_h0, workspace};
   for (const void* p : ps) if (p && !aligned16(p)) return RWKVB200_E_ALIGN;
+  const size_t full = rwkvb200_rwkv7_bwd_states_workspace_bytes(B, T, H, head_size, dtype, algo);
   if (states_bytes < need || !states || workspace_bytes < need || !workspace) return RWKVB200_E_WORKSPACE;
   return launch_rwkv7_block_bwd(r, w, k, v, a, b, n_state ? h0 : nullptr, n_state, d_o, d_ht,
                                 reinterpret_cast<float*>(workspace), dr, dw, dk, dv, da, db, d_h0, B, T, H, dtype,
-                                head_first, (cudaStream_t)stream, head_size, states);
+                                head_first, (cudaStream_t)stream, head_size, states,
+                                workspace_bytes >= full ? static_cast<char*>(workspace) + align256(need) : nullptr);
 }
 
 // ---- packed variable-length batches (chunked bf16 path only)

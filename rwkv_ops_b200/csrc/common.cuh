@@ -191,7 +191,8 @@ int need_aligned_smem(const DeviceFacts& f) {
 __device__ __forceinline__ void earlier_kernels_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void later_kernels_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// cluster_y: CTAs of a cluster along y
+// cluster_y: CTAs of a cluster along y; 0: none, and the kernel starts when all earlier ones have completed.  (Blocks that come
+// early take the SMs that are free first, as many of them as fit, and leave others without any.)
 template <typename... P, typename... A>
 int launch(void (*kernel)(P...), dim3 grid, dim3 block, int smem, cudaStream_t st, int cluster_y, A&&... args) {
   cudaLaunchConfig_t cfg = {};
@@ -205,7 +206,7 @@ int launch(void (*kernel)(P...), dim3 grid, dim3 block, int smem, cudaStream_t s
   attr[1].id = cudaLaunchAttributeClusterDimension;
   attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = cluster_y; attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = cluster_y > 1 ? 2 : 1;
+  cfg.numAttrs = cluster_y > 1 ? 2 : cluster_y;
   const int e = cuda_ok(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...));
   return e ? e : check_launch();
 }
@@ -261,13 +262,16 @@ int launch_rwkv7_rec_bwd(const void* r, const void* w, const void* k, const void
 // a state every R7_CKPT tokens of each unit.  states (may be NULL): rwkv7_block_states_bytes of memory in which the forward
 // leaves the states its backward starts from; a backward that is given them needs only as much for ckpt.
 size_t rwkv7_block_states_bytes(int B, int Tn, int H, int dtype, int head_size);
+// scratch (may be NULL: slower): this much memory for what a sweep over the blocks needs besides the state.
+size_t rwkv7_block_scratch_bytes(int B, int Tn, int H, int dtype, int head_size);
 int launch_rwkv7_block_fwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
                            const float* h0, int n_state, void* o, float* ht, int B, int Tn, int H, int dtype,
-                           int head_first, cudaStream_t st, int head_size = HS, float* states = nullptr);
+                           int head_first, cudaStream_t st, int head_size = HS, float* states = nullptr, void* scratch = nullptr);
 int launch_rwkv7_block_bwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
                            const float* h0, int n_state, const void* d_o, const float* d_ht, float* ckpt,
                            void* dr, void* dw, void* dk, void* dv, void* da, void* db, float* d_h0, int B, int Tn, int H,
-                           int dtype, int head_first, cudaStream_t st, int head_size = HS, const float* states = nullptr);
+                           int dtype, int head_first, cudaStream_t st, int head_size = HS, const float* states = nullptr,
+                           void* scratch = nullptr);
 constexpr int R7_CKPT = 8;   // tokens between state checkpoints of the recurrent backward
 
 int launch_wkv6_fwd(const void* r, const void* k, const void* v, const void* w, const void* u,

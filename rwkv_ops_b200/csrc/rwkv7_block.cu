@@ -28,6 +28,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "tc.cuh"
 
 namespace rwkvb200 {
 
@@ -98,30 +99,271 @@ enum { VR = 0, VW = 1, VK = 2, VA = 3, VB = 4 };
 // the sweep over the blocks: forward (S, sa, o) or backward (G, dsa, dv)
 // ---------------------------------------------------------------------------------------------
 // A CTA owns 16 value rows of one (batch, head) unit.  Its state warps hold them in registers (ROWS rows and 8 columns to a
-// lane, N/8 lanes to a row); its other threads prepare blocks ahead of them, a group of N threads per block in turn.
-// ROWS = 1 (2 at N = 128), four state warps, where a CTA has its SM to itself: the instructions of a warp are then what a
-// block takes, and a warp of twice the rows needs 131 us per sweep where this takes 108 (B 2, T 1024, 16 heads).  ROWS = 2
-// where CTAs share an SM, whose shared memory they fill: B 16, T 512, 16 heads, forward 332 us against 360.
-// In processing order p (time forward, or reversed), the stage a group hands over:
-template <int N>
+// lane, N/8 lanes to a row) and take them through the blocks; what a block needs besides the state, its stage, is prepared ahead
+// of them.  In processing order p (time forward, or reversed):
+template <int N, int VR_>
 struct Stage {
   float x[W][N], y[W][N];       // sa_p = S x_p + xv[p][.] v ;  o_p = S y_p + yv[p][.] v
   float u1[W][N], u2[W][N];     // S' = S diag(d) + sum_p sa_p u1_p + v_p u2_p
   float d[N];
   float xv[W][W], yv[W][W];
-  float vt[RV][W];
+  float vt[VR_][W];             // the tokens' v, for all N or for a CTA's RV rows
 };
-template <typename T, int N>
-struct Prep {
-  T raw[2][5][W][N];            // the block at work and the next one (requested while the first is worked on)
-  T rawv[2][W][RV];
-  float d[W][N];
+template <int N> constexpr uint32_t COMMON_BYTES = sizeof(Stage<N, RV>) - RV * W * sizeof(float);      // a stage without vt
+constexpr uint32_t SLICE_BYTES = RV * W * sizeof(float);                                               // a CTA's rows of vt
+
+template <int N>
+struct Scalars {
+  float d[W][N];                                      // decays
   float sx[W][W], sxv[W][W], sy[W][W], syv[W][W];     // the scalars A, processing order; never-written entries stay 0
 };
+// The preparation of one block by a group of N threads (thread q of them), in steps with a barrier of the group before each.
+template <typename T, int N, bool BWD>
+struct Preparer {
+  static constexpr int NL = N / 4, HELD = 32 / NL;      // lanes per pair of source tokens
+  Scalars<N>& sc;
+  const int q, pi, gq, lane;
+  float* dst[HELD];
+
+  // The scalars: a thread takes four channels of the source tokens pi and 7 - pi (nine (source, later token) pairs
+  // whatever pi, so all warps have the same work), 32 sums that N/4 lanes then reduce and share out.
+  __device__ __forceinline__ Preparer(Scalars<N>& sc_, int q_) : sc(sc_), q(q_), pi(q_ / NL), gq(q_ % NL), lane(q_ & 31) {
+    for (int e = q; e < 4 * W * W; e += N) (&sc.sx[0][0])[e] = 0.f;
+#pragma unroll
+    for (int h = 0; h < HELD; ++h) {
+      const int e = gq * HELD + h;
+      const int kind = e < 9 ? 0 : e < 18 ? 1 : e < 25 ? 2 : 3;           // A_qb, A_qk, A_ab, A_ak
+      const int x = e - (kind == 0 ? 0 : kind == 1 ? 9 : kind == 2 ? 17 : 24);
+      const int i = x <= 7 - pi ? pi : 7 - pi, j = x <= 7 - pi ? pi + x : 7 - pi + (8 - x);
+      float (*m)[W] = BWD ? (kind == 0 ? sc.sxv : kind == 1 ? sc.syv : kind == 2 ? sc.sx : sc.sy)
+                          : (kind == 0 ? sc.sy : kind == 1 ? sc.syv : kind == 2 ? sc.sx : sc.sxv);
+      dst[h] = BWD ? &m[W - 1 - i][W - 1 - j] : &m[j][i];
+    }
+  }
+  // the decays, 1 for tokens past the end
+  __device__ __forceinline__ void decays(const T (*raw)[W][N], int n_live) {
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const int t = 4 * m + q / NL, c = 4 * (q % NL);
+      const float4 f = load4_shared(&raw[VW][t][c]);
+      *reinterpret_cast<float4*>(&sc.d[t][c]) = t < n_live ? make_float4(decay_of(f.x), decay_of(f.y), decay_of(f.z), decay_of(f.w))
+                                                           : make_float4(1.f, 1.f, 1.f, 1.f);
+    }
+  }
+  __device__ __forceinline__ void scalars(const T (*raw)[W][N]) {
+    float s[32];
+#pragma unroll
+    for (int e = 0; e < 32; ++e) s[e] = 0.f;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int i = half ? 7 - pi : pi, last = half ? pi : 7 - pi;      // later tokens i .. i + last
+      Quad pb = quad_of(load4_shared(&raw[VB][i][4 * gq])), pk = quad_of(load4_shared(&raw[VK][i][4 * gq]));
+#pragma unroll
+      for (int x = 0; x < (half ? 4 : 8); ++x) {
+        if (x > last) break;
+        const int j = i + x, at = half ? 8 - x : x;
+        if (x > 0) {
+          const Quad aj = quad_of(load4_shared(&raw[VA][j][4 * gq])), dj = lds4(&sc.d[j][4 * gq]);
+          s[17 + at] = sum2(fma2(pb.hi, aj.hi, mul2(pb.lo, aj.lo)));
+          s[24 + at] = sum2(fma2(pk.hi, aj.hi, mul2(pk.lo, aj.lo)));
+          pb.lo = mul2(pb.lo, dj.lo); pb.hi = mul2(pb.hi, dj.hi);
+          pk.lo = mul2(pk.lo, dj.lo); pk.hi = mul2(pk.hi, dj.hi);
+        }
+        const Quad rj = quad_of(load4_shared(&raw[VR][j][4 * gq]));
+        s[at] = sum2(fma2(pb.hi, rj.hi, mul2(pb.lo, rj.lo)));
+        s[9 + at] = sum2(fma2(pk.hi, rj.hi, mul2(pk.lo, rj.lo)));
+      }
+    }
+    __syncwarp();
+    reduce_scatter<32, NL / 2, 1>(s, lane);
+#pragma unroll
+    for (int h = 0; h < HELD; ++h) *dst[h] = s[h];
+  }
+  // x and y by substitution, in processing order: of one channel, or of one column of A_ak and A_qk
+  __device__ __forceinline__ void solve(float (&xs)[W], float (&ys_)[W]) {
+#pragma unroll
+    for (int p = 0; p < W; ++p) {
+      float m[W];
+#pragma unroll
+      for (int i = 0; i < p; i += 4) *reinterpret_cast<float4*>(&m[i]) = *reinterpret_cast<const float4*>(&sc.sx[p][i]);
+#pragma unroll
+      for (int i = 0; i < p; ++i) xs[p] += m[i] * xs[i];
+    }
+#pragma unroll
+    for (int p = 0; p < W; ++p) {
+      float m[W];
+#pragma unroll
+      for (int i = 0; i <= p; i += 4) *reinterpret_cast<float4*>(&m[i]) = *reinterpret_cast<const float4*>(&sc.sy[p][i]);
+#pragma unroll
+      for (int i = 0; i <= p; ++i) ys_[p] += m[i] * xs[i];
+    }
+  }
+  template <int VROWS>
+  __device__ __forceinline__ void write(const T (*raw)[W][N], Stage<N, VROWS>& st) {      // all but vt; thread q: channel q
+    {
+      float xs[W], ys_[W], dd[W];
+      float run = 1.f;
+#pragma unroll
+      for (int p = 0; p < W; ++p) {
+        const int t = BWD ? W - 1 - p : p;
+        dd[p] = sc.d[t][q];
+        xs[p] = run * to_f32(raw[BWD ? VB : VA][t][q]);
+        if (!BWD) run *= dd[p];
+        ys_[p] = run * to_f32(raw[BWD ? VK : VR][t][q]);
+        if (BWD) run *= dd[p];
+      }
+      st.d[q] = run;
+      run = 1.f;
+#pragma unroll
+      for (int p = W - 1; p >= 0; --p) {
+        const int t = BWD ? W - 1 - p : p;
+        st.u1[p][q] = run * to_f32(raw[BWD ? VA : VB][t][q]);
+        if (BWD) run *= dd[p];
+        st.u2[p][q] = run * to_f32(raw[BWD ? VR : VK][t][q]);
+        if (!BWD) run *= dd[p];
+      }
+      solve(xs, ys_);
+#pragma unroll
+      for (int p = 0; p < W; ++p) { st.x[p][q] = xs[p]; st.y[p][q] = ys_[p]; }
+    }
+    if (q < W) {
+      float xs[W], ys_[W];
+#pragma unroll
+      for (int p = 0; p < W; ++p) { xs[p] = sc.sxv[p][q]; ys_[p] = sc.syv[p][q]; }
+      solve(xs, ys_);
+#pragma unroll
+      for (int p = 0; p < W; ++p) { st.xv[p][q] = xs[p]; st.yv[p][q] = ys_[p]; }
+    }
+  }
+};
+
+// The state warps' part of one block: the rows' S in registers through one stage.
+template <int N, int ROWS>
+struct StateRows {
+  // N/8 lanes per row; the lanes that read the same part of a vector are neighbours (see the note on 16-byte reads above)
+  static constexpr int RG = 256 / N;           // groups of rows in a warp
+  const int lane, r0, kq, jl, c0, c1;          // first row; this thread's columns: two quads of ROWS rows; its token
+  Quad S[ROWS][2];
+
+  __device__ __forceinline__ StateRows(int tid)
+      : lane(tid & 31), r0(ROWS * (tid / 32 * RG + tid % RG)), kq((tid & 31) / RG), jl(kq & 7), c0(4 * kq), c1(N / 2 + 4 * kq) {}
+  __device__ __forceinline__ void get(const float* p) {      // p: the CTA's first row, or nullptr
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+      S[i][0] = S[i][1] = Quad{0ull, 0ull};
+      if (p) {
+        S[i][0] = quad_of(*reinterpret_cast<const float4*>(p + (long long)(r0 + i) * N + c0));
+        S[i][1] = quad_of(*reinterpret_cast<const float4*>(p + (long long)(r0 + i) * N + c1));
+      }
+    }
+  }
+  __device__ __forceinline__ void put(float* p) const {
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float2 a = unpack2(S[i][h].lo), b = unpack2(S[i][h].hi);
+        *reinterpret_cast<float4*>(p + (long long)(r0 + i) * N + (h ? c1 : c0)) = make_float4(a.x, a.y, b.x, b.y);
+      }
+    }
+  }
+  // S row . vector, for all rows and tokens: dots[ROWS p + i]
+  __device__ __forceinline__ void dots(const float (*vec)[N], float* out) const {
+    Quad xa[W], xb[W];
+#pragma unroll
+    for (int p = 0; p < W; ++p) { xa[p] = lds4(&vec[p][c0]); xb[p] = lds4(&vec[p][c1]); }
+#pragma unroll
+    for (int p = 0; p < W; ++p)
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i)
+        out[ROWS * p + i] = sum2(fma2(S[i][1].hi, xb[p].hi, fma2(S[i][1].lo, xb[p].lo, fma2(S[i][0].hi, xa[p].hi, mul2(S[i][0].lo, xa[p].lo)))));
+  }
+  __device__ __forceinline__ void add_outer(const Quad& ua, const Quad& ub, int i, float f) {
+    const f32x2 s = pack2(f, f);
+    S[i][0].lo = fma2(s, ua.lo, S[i][0].lo); S[i][0].hi = fma2(s, ua.hi, S[i][0].hi);
+    S[i][1].lo = fma2(s, ub.lo, S[i][1].lo); S[i][1].hi = fma2(s, ub.hi, S[i][1].hi);
+  }
+  // Leaves token jl's output of the thread's rows in oo: in every lane (N = 64: 8 lanes to a row), or in lanes 8-15 of a row.
+  __device__ __forceinline__ void step(const Stage<N, RV>& st, float (&oo)[ROWS]) {
+    float ax[(N == 64 ? 1 : 2) * W * ROWS], ay[W * ROWS];
+    dots(st.x, ax);
+    float sa[ROWS];
+    if constexpr (N == 64) {
+      reduce_scatter<W * ROWS, 4 * RG, RG>(ax, lane);
+      dots(st.y, ay);
+      reduce_scatter<W * ROWS, 4 * RG, RG>(ay, lane);
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i) { sa[i] = ax[i]; oo[i] = ay[i]; }
+    } else {
+      dots(st.y, ax + W * ROWS);
+      reduce_scatter<2 * W * ROWS, 8 * RG, RG>(ax, lane);
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i) sa[i] = oo[i] = ax[i];
+    }
+    {
+      const Quad da = lds4(&st.d[c0]), db = lds4(&st.d[c1]);
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i) {
+        S[i][0].lo = mul2(S[i][0].lo, da.lo); S[i][0].hi = mul2(S[i][0].hi, da.hi);
+        S[i][1].lo = mul2(S[i][1].lo, db.lo); S[i][1].hi = mul2(S[i][1].hi, db.hi);
+      }
+    }
+#pragma unroll
+    for (int l = 0; l < W; l += 4) {
+      const float4 x = *reinterpret_cast<const float4*>(&st.xv[jl][l]), y = *reinterpret_cast<const float4*>(&st.yv[jl][l]);
+      // the factors of tokens after jl are 0, but 0 times an infinity or NaN is not: their v counts as 0 as well
+      const bool u0 = l <= jl, u1 = l + 1 <= jl, u2 = l + 2 <= jl, u3 = l + 3 <= jl;
+      float vv[ROWS][4];
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i) {
+        const float4 f = *reinterpret_cast<const float4*>(&st.vt[r0 + i][l]);
+        vv[i][0] = f.x; vv[i][1] = f.y; vv[i][2] = f.z; vv[i][3] = f.w;
+        const float4 m = make_float4(u0 ? f.x : 0.f, u1 ? f.y : 0.f, u2 ? f.z : 0.f, u3 ? f.w : 0.f);
+        sa[i] += x.x * m.x + x.y * m.y + (x.z * m.z + x.w * m.w);
+        oo[i] += y.x * m.x + y.y * m.y + (y.z * m.z + y.w * m.w);
+      }
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        const Quad ua = lds4(&st.u2[l + p][c0]), ub = lds4(&st.u2[l + p][c1]);
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) add_outer(ua, ub, i, vv[i][p]);
+      }
+    }
+#pragma unroll
+    for (int p = 0; p < W; ++p) {
+      const Quad ua = lds4(&st.u1[p][c0]), ub = lds4(&st.u1[p][c1]);
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i) add_outer(ua, ub, i, __shfl_sync(0xffffffffu, sa[i], lane % RG + RG * p));
+    }
+  }
+  template <typename T>
+  __device__ __forceinline__ void put_out(T* p, const float (&oo)[ROWS]) const {      // p: token jl's value channels of the CTA's rows
+    if (N == 64 || kq >= 8) {
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i) p[r0 + i] = from_f32<T>(oo[i]);
+    }
+  }
+};
+// where block n's state is kept: forward, the state before every GT tokens but the first; backward, the gradient after them, but
+// the last; nullptr: nowhere
+template <int N, bool BWD>
+__device__ __forceinline__ float* state_slot(float* ckpt, int unit, int NG, int n) {
+  const int m = n >> 1;
+  if (!BWD && (n & 1) == 0 && m > 0) return ckpt + ((long long)unit * (NG - 1) + m - 1) * N * N;
+  if (BWD && (n & 1) == 1 && m < NG - 1) return ckpt + ((long long)unit * (NG - 1) + m) * N * N;
+  return nullptr;
+}
+
+// ---- blocks prepared by the CTA itself, for calls of a few blocks, or without workspace
+// ROWS = 1 (2 at N = 128), four state warps, where a CTA has its SM to itself: the instructions of a warp are then what a
+// block takes, and a warp of twice the rows needs 131 us per sweep where this takes 108 (B 2, T 1024, 16 heads).  ROWS = 2
+// where CTAs share an SM, whose shared memory they fill: B 16, T 512, 16 heads, forward 332 us against 360.
 template <typename T, int N>
 struct Group {
-  Stage<N> stage;
-  Prep<T, N> prep;
+  Stage<N, RV> stage;
+  Scalars<N> scalars;
+  T raw[2][5][W][N];            // the block at work and the next one (requested while the first is worked on)
+  T rawv[2][W][RV];
 };
 // Groups that prepare blocks: as many as keep up with the state warps where a CTA has its SM to itself.  A group takes 34 KB of
 // shared memory (60 at N = 128), so where there are more CTAs than SMs fewer of them let two or three CTAs share an SM and fill
@@ -136,139 +378,43 @@ template <int N, int ROWS> constexpr int state_threads() { return RV / ROWS * N 
 
 template <typename T, int N, bool BWD, int GROUPS, int ROWS>
 __global__ void __launch_bounds__(state_threads<N, ROWS>() + N * GROUPS)
-r7_sweep_kernel(Vecs<T> in, const T* __restrict__ v, const float* __restrict__ s_in, int n_state,
-                T* __restrict__ out, float* __restrict__ s_out, float* __restrict__ ckpt, int Tn, int H, TokLayout lay) {
+r7_sweep_inline_kernel(Vecs<T> in, const T* __restrict__ v, const float* __restrict__ s_in, int n_state,
+                       T* __restrict__ out, float* __restrict__ s_out, float* __restrict__ ckpt, int Tn, int H, TokLayout lay) {
   constexpr int NCONS = state_threads<N, ROWS>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Group<T, N>* const group = reinterpret_cast<Group<T, N>*>(smem_raw);
   earlier_kernels_done();
   later_kernels_may_start();
-  const int unit = blockIdx.x, ys = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
+  const int unit = blockIdx.x, ys = blockIdx.y, tid = threadIdx.x;
   const int bi = unit / H, hi = unit % H;
   const long long base = bi * lay.sb + hi * lay.sh;
   const int NB = (Tn + W - 1) / W;
   constexpr int FULL = 1 + GROUPS, EMPTY = 1 + 2 * GROUPS;      // named barriers: 1.. within a group, then these
+  const long long rows = (long long)ys * RV * N;                // of the CTA's first row in a state
 
   if (tid < NCONS) {
     // ---- state warps
-    // N/8 lanes per row; the lanes that read the same part of a vector are neighbours (see the note on 16-byte reads above)
-    constexpr int RG = 256 / N;                  // groups of rows in a warp
-    const int r0 = ROWS * (tid / 32 * RG + lane % RG), kq = lane / RG, jl = kq & 7;
-    const int c0 = 4 * kq, c1 = N / 2 + 4 * kq;  // this thread's columns: two quads of ROWS rows
     const int NG = (Tn + GT - 1) / GT;
-    Quad S[ROWS][2];
-#pragma unroll
-    for (int i = 0; i < ROWS; ++i) {
-      S[i][0] = S[i][1] = Quad{0ull, 0ull};
-      if (s_in && n_state > 0) {
-        const float* p = s_in + (long long)(n_state == 1 ? hi : unit) * N * N + (long long)(ys * RV + r0 + i) * N;
-        S[i][0] = quad_of(*reinterpret_cast<const float4*>(p + c0));
-        S[i][1] = quad_of(*reinterpret_cast<const float4*>(p + c1));
-      }
-    }
-    auto put_state = [&](float* p) {
-#pragma unroll
-      for (int i = 0; i < ROWS; ++i) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const float2 a = unpack2(S[i][h].lo), b = unpack2(S[i][h].hi);
-          *reinterpret_cast<float4*>(p + (long long)(ys * RV + r0 + i) * N + (h ? c1 : c0)) = make_float4(a.x, a.y, b.x, b.y);
-        }
-      }
-    };
-    // S row . vector, for all rows and tokens: dots[4 p + i]
-    auto dots = [&](const float (*vec)[N], float* out4) {
-#pragma unroll
-      for (int p = 0; p < W; ++p) {
-        const Quad xa = lds4(&vec[p][c0]), xb = lds4(&vec[p][c1]);
-#pragma unroll
-        for (int i = 0; i < ROWS; ++i)
-          out4[ROWS * p + i] = sum2(fma2(S[i][1].hi, xb.hi, fma2(S[i][1].lo, xb.lo, fma2(S[i][0].hi, xa.hi, mul2(S[i][0].lo, xa.lo)))));
-      }
-    };
+    StateRows<N, ROWS> S(tid);
+    S.get(s_in && n_state > 0 ? s_in + (long long)(n_state == 1 ? hi : unit) * N * N + rows : nullptr);
     for (int idx = 0, g = 0; idx < NB; ++idx, g = g + 1 == GROUPS ? 0 : g + 1) {
       const int n = BWD ? NB - 1 - idx : idx;
-      const Stage<N>& st = group[g].stage;
-      if (ckpt) {      // forward: the state before every GT tokens but the first; backward: the gradient after them, but the last
-        const int m = n >> 1;
-        if (!BWD && (n & 1) == 0 && m > 0) put_state(ckpt + ((long long)unit * (NG - 1) + m - 1) * N * N);
-        if (BWD && (n & 1) == 1 && m < NG - 1) put_state(ckpt + ((long long)unit * (NG - 1) + m) * N * N);
-      }
+      if (ckpt)
+        if (float* p = state_slot<N, BWD>(ckpt, unit, NG, n)) S.put(p + rows);
       bar_sync(FULL + g, NCONS + N);
-      // the reduction leaves token jl of the thread's rows: in every lane both sa and o (N = 64: 8 lanes to a row), or sa
-      // in lanes 0-7 and o in lanes 8-15 of a row
-      float ax[(N == 64 ? 1 : 2) * W * ROWS], ay[W * ROWS];
-      dots(st.x, ax);
-      float sa[ROWS], oo[ROWS];
-      if constexpr (N == 64) {
-        reduce_scatter<W * ROWS, 4 * RG, RG>(ax, lane);
-        dots(st.y, ay);
-        reduce_scatter<W * ROWS, 4 * RG, RG>(ay, lane);
-#pragma unroll
-        for (int i = 0; i < ROWS; ++i) { sa[i] = ax[i]; oo[i] = ay[i]; }
-      } else {
-        dots(st.y, ax + W * ROWS);
-        reduce_scatter<2 * W * ROWS, 8 * RG, RG>(ax, lane);
-#pragma unroll
-        for (int i = 0; i < ROWS; ++i) sa[i] = oo[i] = ax[i];
-      }
-      {
-        const Quad da = lds4(&st.d[c0]), db = lds4(&st.d[c1]);
-#pragma unroll
-        for (int i = 0; i < ROWS; ++i) {
-          S[i][0].lo = mul2(S[i][0].lo, da.lo); S[i][0].hi = mul2(S[i][0].hi, da.hi);
-          S[i][1].lo = mul2(S[i][1].lo, db.lo); S[i][1].hi = mul2(S[i][1].hi, db.hi);
-        }
-      }
-      auto add_outer = [&](const Quad& ua, const Quad& ub, int i, float f) {
-        const f32x2 s = pack2(f, f);
-        S[i][0].lo = fma2(s, ua.lo, S[i][0].lo); S[i][0].hi = fma2(s, ua.hi, S[i][0].hi);
-        S[i][1].lo = fma2(s, ub.lo, S[i][1].lo); S[i][1].hi = fma2(s, ub.hi, S[i][1].hi);
-      };
-#pragma unroll
-      for (int l = 0; l < W; l += 4) {
-        const float4 x = *reinterpret_cast<const float4*>(&st.xv[jl][l]), y = *reinterpret_cast<const float4*>(&st.yv[jl][l]);
-        // the factors of tokens after jl are 0, but 0 times an infinity or NaN is not: their v counts as 0 as well
-        const bool u0 = l <= jl, u1 = l + 1 <= jl, u2 = l + 2 <= jl, u3 = l + 3 <= jl;
-        float vv[ROWS][4];
-#pragma unroll
-        for (int i = 0; i < ROWS; ++i) {
-          const float4 f = *reinterpret_cast<const float4*>(&st.vt[r0 + i][l]);
-          vv[i][0] = f.x; vv[i][1] = f.y; vv[i][2] = f.z; vv[i][3] = f.w;
-          const float4 m = make_float4(u0 ? f.x : 0.f, u1 ? f.y : 0.f, u2 ? f.z : 0.f, u3 ? f.w : 0.f);
-          sa[i] += x.x * m.x + x.y * m.y + (x.z * m.z + x.w * m.w);
-          oo[i] += y.x * m.x + y.y * m.y + (y.z * m.z + y.w * m.w);
-        }
-#pragma unroll
-        for (int p = 0; p < 4; ++p) {
-          const Quad ua = lds4(&st.u2[l + p][c0]), ub = lds4(&st.u2[l + p][c1]);
-#pragma unroll
-          for (int i = 0; i < ROWS; ++i) add_outer(ua, ub, i, vv[i][p]);
-        }
-      }
-#pragma unroll
-      for (int p = 0; p < W; ++p) {
-        const Quad ua = lds4(&st.u1[p][c0]), ub = lds4(&st.u1[p][c1]);
-#pragma unroll
-        for (int i = 0; i < ROWS; ++i) add_outer(ua, ub, i, __shfl_sync(0xffffffffu, sa[i], lane % RG + RG * p));
-      }
+      float oo[ROWS];
+      S.step(group[g].stage, oo);
       if (idx + GROUPS < NB) bar_arrive(EMPTY + g, NCONS + N);
-      const int t = n * W + (BWD ? W - 1 - jl : jl);
-      if (out && t < Tn && (N == 64 || kq >= 8)) {
-        T* p = out + base + (long long)t * lay.st + ys * RV + r0;
-#pragma unroll
-        for (int i = 0; i < ROWS; ++i) p[i] = from_f32<T>(oo[i]);
-      }
+      const int t = n * W + (BWD ? W - 1 - S.jl : S.jl);
+      if (out && t < Tn) S.put_out(out + base + (long long)t * lay.st + ys * RV, oo);
     }
-    if (s_out) put_state(s_out + (long long)unit * N * N);
+    if (s_out) S.put(s_out + (long long)unit * N * N + rows);
     return;
   }
 
   // ---- preparing groups
   const int g = (tid - NCONS) / N, q = (tid - NCONS) % N;
-  Prep<T, N>& pr = group[g].prep;
-  Stage<N>& st = group[g].stage;
-  constexpr int NL = N / 4;                     // lanes per pair of source tokens below
+  Group<T, N>& pr = group[g];
   constexpr int EPC = 16 / sizeof(T), CPR = N / EPC, VPR = RV / EPC;     // elements per 16 bytes; copies per token row
 
   auto request = [&](int idx) {
@@ -291,128 +437,138 @@ r7_sweep_kernel(Vecs<T> in, const T* __restrict__ v, const float* __restrict__ s
     cp_async_commit();
   };
   request(g);
-
-  // The scalars: a thread takes four channels of the source tokens pi and 7 - pi (nine (source, later token) pairs
-  // whatever pi, so all warps have the same work), 32 sums that N/4 lanes then reduce and share out.
-  const int pi = q / NL, gq = q % NL;
-  for (int e = q; e < 4 * W * W; e += N) (&pr.sx[0][0])[e] = 0.f;
-  constexpr int HELD = 32 / NL;
-  float* dst[HELD];
-#pragma unroll
-  for (int h = 0; h < HELD; ++h) {
-    const int e = gq * HELD + h;
-    const int kind = e < 9 ? 0 : e < 18 ? 1 : e < 25 ? 2 : 3;           // A_qb, A_qk, A_ab, A_ak
-    const int x = e - (kind == 0 ? 0 : kind == 1 ? 9 : kind == 2 ? 17 : 24);
-    const int i = x <= 7 - pi ? pi : 7 - pi, j = x <= 7 - pi ? pi + x : 7 - pi + (8 - x);
-    float (*m)[W] = BWD ? (kind == 0 ? pr.sxv : kind == 1 ? pr.syv : kind == 2 ? pr.sx : pr.sy)
-                        : (kind == 0 ? pr.sy : kind == 1 ? pr.syv : kind == 2 ? pr.sx : pr.sxv);
-    dst[h] = BWD ? &m[W - 1 - i][W - 1 - j] : &m[j][i];
-  }
-
+  Preparer<T, N, BWD> prep(pr.scalars, q);
   for (int idx = g; idx < NB; idx += GROUPS) {
-    const int n = BWD ? NB - 1 - idx : idx, t0 = n * W, buf = (idx / GROUPS) & 1;
+    const int t0 = (BWD ? NB - 1 - idx : idx) * W, buf = (idx / GROUPS) & 1;
     cp_async_wait();
     bar_sync(1 + g, N);             // the block's tokens are here, and the last block's scalars and decays have been read
     request(idx + GROUPS);
-#pragma unroll
-    for (int m = 0; m < 2; ++m) {
-      const int t = 4 * m + q / NL, c = 4 * (q % NL);
-      const float4 f = load4_shared(&pr.raw[buf][VW][t][c]);
-      *reinterpret_cast<float4*>(&pr.d[t][c]) = t0 + t < Tn ? make_float4(decay_of(f.x), decay_of(f.y), decay_of(f.z), decay_of(f.w))
-                                                            : make_float4(1.f, 1.f, 1.f, 1.f);
-    }
+    prep.decays(pr.raw[buf], Tn - t0);
     bar_sync(1 + g, N);
-    {
-      float s[32];
-#pragma unroll
-      for (int e = 0; e < 32; ++e) s[e] = 0.f;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int i = half ? 7 - pi : pi, last = half ? pi : 7 - pi;      // later tokens i .. i + last
-        Quad pb = quad_of(load4_shared(&pr.raw[buf][VB][i][4 * gq])), pk = quad_of(load4_shared(&pr.raw[buf][VK][i][4 * gq]));
-#pragma unroll
-        for (int x = 0; x < (half ? 4 : 8); ++x) {
-          if (x > last) break;
-          const int j = i + x, at = half ? 8 - x : x;
-          if (x > 0) {
-            const Quad aj = quad_of(load4_shared(&pr.raw[buf][VA][j][4 * gq])), dj = lds4(&pr.d[j][4 * gq]);
-            s[17 + at] = sum2(fma2(pb.hi, aj.hi, mul2(pb.lo, aj.lo)));
-            s[24 + at] = sum2(fma2(pk.hi, aj.hi, mul2(pk.lo, aj.lo)));
-            pb.lo = mul2(pb.lo, dj.lo); pb.hi = mul2(pb.hi, dj.hi);
-            pk.lo = mul2(pk.lo, dj.lo); pk.hi = mul2(pk.hi, dj.hi);
-          }
-          const Quad rj = quad_of(load4_shared(&pr.raw[buf][VR][j][4 * gq]));
-          s[at] = sum2(fma2(pb.hi, rj.hi, mul2(pb.lo, rj.lo)));
-          s[9 + at] = sum2(fma2(pk.hi, rj.hi, mul2(pk.lo, rj.lo)));
-        }
-      }
-      __syncwarp();
-      reduce_scatter<32, NL / 2, 1>(s, lane);
-#pragma unroll
-      for (int h = 0; h < HELD; ++h) *dst[h] = s[h];
-    }
+    prep.scalars(pr.raw[buf]);
     if (idx >= GROUPS) bar_sync(EMPTY + g, NCONS + N);      // the stage has been read (and the group's scalars are written)
     else               bar_sync(1 + g, N);
-    // one channel per thread: x and y by substitution, in processing order
-    auto solve = [&](float (&xs)[W], float (&ys_)[W]) {
-#pragma unroll
-      for (int p = 0; p < W; ++p) {
-        float m[W];
-#pragma unroll
-        for (int i = 0; i < p; i += 4) *reinterpret_cast<float4*>(&m[i]) = *reinterpret_cast<const float4*>(&pr.sx[p][i]);
-#pragma unroll
-        for (int i = 0; i < p; ++i) xs[p] += m[i] * xs[i];
-      }
-#pragma unroll
-      for (int p = 0; p < W; ++p) {
-        float m[W];
-#pragma unroll
-        for (int i = 0; i <= p; i += 4) *reinterpret_cast<float4*>(&m[i]) = *reinterpret_cast<const float4*>(&pr.sy[p][i]);
-#pragma unroll
-        for (int i = 0; i <= p; ++i) ys_[p] += m[i] * xs[i];
-      }
-    };
-    {
-      float xs[W], ys_[W], dd[W];
-      float run = 1.f;
-#pragma unroll
-      for (int p = 0; p < W; ++p) {
-        const int t = BWD ? W - 1 - p : p;
-        dd[p] = pr.d[t][q];
-        xs[p] = run * to_f32(pr.raw[buf][BWD ? VB : VA][t][q]);
-        if (!BWD) run *= dd[p];
-        ys_[p] = run * to_f32(pr.raw[buf][BWD ? VK : VR][t][q]);
-        if (BWD) run *= dd[p];
-      }
-      st.d[q] = run;
-      run = 1.f;
-#pragma unroll
-      for (int p = W - 1; p >= 0; --p) {
-        const int t = BWD ? W - 1 - p : p;
-        st.u1[p][q] = run * to_f32(pr.raw[buf][BWD ? VA : VB][t][q]);
-        if (BWD) run *= dd[p];
-        st.u2[p][q] = run * to_f32(pr.raw[buf][BWD ? VR : VK][t][q]);
-        if (!BWD) run *= dd[p];
-      }
-      solve(xs, ys_);
-#pragma unroll
-      for (int p = 0; p < W; ++p) { st.x[p][q] = xs[p]; st.y[p][q] = ys_[p]; }
-    }
-    if (q < W) {      // the columns of A_ak and A_qk go through the same substitution
-      float xs[W], ys_[W];
-#pragma unroll
-      for (int p = 0; p < W; ++p) { xs[p] = pr.sxv[p][q]; ys_[p] = pr.syv[p][q]; }
-      solve(xs, ys_);
-#pragma unroll
-      for (int p = 0; p < W; ++p) { st.xv[p][q] = xs[p]; st.yv[p][q] = ys_[p]; }
-    }
+    prep.write(pr.raw[buf], pr.stage);
     for (int e = q; e < RV * W; e += N) {
       const int p = e % W, row = e / W;
-      st.vt[row][p] = to_f32(pr.rawv[buf][BWD ? W - 1 - p : p][row]);
+      pr.stage.vt[row][p] = to_f32(pr.rawv[buf][BWD ? W - 1 - p : p][row]);
     }
     bar_arrive(FULL + g, NCONS + N);
   }
   cp_async_wait();
+}
+
+// ---- blocks prepared by a kernel of their own, once for all the CTAs of a unit
+// Prepared inside the sweep, a block is prepared N/16 times, and that is 60 % of the sweep's instructions and most of its
+// shared-memory traffic.  Here the stages go through memory, 11 KB per block and unit (L2, where they fit), and a sweep's CTAs
+// are state warps and one that fetches stages.  B 2, T 1024, 16 heads: 20 us and 80 per sweep against 105; B 16, T 512, 16 heads,
+// forward 332 -> 223 us; head size 128 1170 -> 660.  What bounds the sweep now with one CTA per SM: 414 instructions per block and
+// warp, one warp to a scheduler, and shared memory (682 of 1190 cycles).
+template <typename T, int N>
+struct PrepareSmem {
+  Scalars<N> scalars;
+  T raw[5][W][N];
+};
+constexpr int PREPARE_THREADS = 256;
+
+template <typename T, int N, bool BWD>
+__global__ void __launch_bounds__(PREPARE_THREADS)
+r7_prepare_kernel(Vecs<T> in, const T* __restrict__ v, Stage<N, N>* __restrict__ stages, int Tn, int H, int idx0, int nb, int n_items,
+                  TokLayout lay) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int g = threadIdx.x / N, q = threadIdx.x % N, item = blockIdx.x * (PREPARE_THREADS / N) + g;
+  PrepareSmem<T, N>& sm = reinterpret_cast<PrepareSmem<T, N>*>(smem_raw)[g];
+  earlier_kernels_done();
+  later_kernels_may_start();
+  if (item >= n_items) return;      // the whole group
+  const int unit = item / nb, idx = idx0 + item % nb, NB = (Tn + W - 1) / W;
+  const int t0 = (BWD ? NB - 1 - idx : idx) * W;
+  const long long base = unit / H * lay.sb + unit % H * lay.sh;
+  constexpr int EPC = 16 / sizeof(T), CPR = N / EPC;
+#pragma unroll
+  for (int m = 0; m < W * CPR / N; ++m) {
+    const int e = q + N * m, row = e / CPR, ch = e % CPR;
+    const bool live = t0 + row < Tn;
+    const long long off = base + (live ? (long long)(t0 + row) * lay.st : 0) + ch * EPC;
+#pragma unroll
+    for (int i = 0; i < 5; ++i) cp_async16(&sm.raw[i][row][ch * EPC], in.p[i] + off, live);
+  }
+  cp_async_commit();
+  Stage<N, N>& st = stages[item];
+  {
+    float f[W];
+#pragma unroll
+    for (int p = 0; p < W; ++p) {
+      const int t = t0 + (BWD ? W - 1 - p : p);
+      f[p] = t < Tn ? to_f32(v[base + (long long)t * lay.st + q]) : 0.f;
+    }
+#pragma unroll
+    for (int p = 0; p < W; p += 4) *reinterpret_cast<float4*>(&st.vt[q][p]) = make_float4(f[p], f[p + 1], f[p + 2], f[p + 3]);
+  }
+  Preparer<T, N, BWD> prep(sm.scalars, q);
+  cp_async_wait();
+  bar_sync(1 + g, N);
+  prep.decays(sm.raw, Tn - t0);
+  bar_sync(1 + g, N);
+  prep.scalars(sm.raw);
+  bar_sync(1 + g, N);
+  prep.write(sm.raw, st);
+}
+
+template <int N, int SLOTS>
+struct SweepSmem {
+  Stage<N, RV> stage[SLOTS];
+  uint64_t full[SLOTS], empty[SLOTS];
+};
+// With at most one CTA to an SM, slots enough that no two CTAs fit one: they may come while the preparing kernel runs out, and
+// would otherwise share the first SMs that are free (B 2, T 1024, 16 heads: 177 -> 230 us).
+template <int N> constexpr int FEW_CTAS_SLOTS = 116 * 1024 / sizeof(Stage<N, RV>) + 1;
+// Blocks idx0 .. idx0 + nb - 1 in processing order; a warp beside the state warps fetches their stages.
+template <typename T, int N, bool BWD, int SLOTS, int ROWS, int PER_SM>
+__global__ void __launch_bounds__(state_threads<N, ROWS>() + 32, PER_SM)
+r7_sweep_kernel(const Stage<N, N>* __restrict__ stages, const float* s_in, int n_state, T* __restrict__ out, float* s_out,
+                float* __restrict__ ckpt, int Tn, int H, int idx0, int nb, TokLayout lay, int* status) {
+  constexpr int NCONS = state_threads<N, ROWS>();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  auto& sm = *reinterpret_cast<SweepSmem<N, SLOTS>*>(smem_raw);
+  const int unit = blockIdx.x, ys = blockIdx.y, tid = threadIdx.x;
+  const int bi = unit / H, hi = unit % H;
+  if (tid == 0) {
+    for (int i = 0; i < SLOTS; ++i) { tc::mbar_init(&sm.full[i], 1); tc::mbar_init(&sm.empty[i], NCONS / 32); }
+    tc::fence_mbar_init();
+  }
+  __syncthreads();
+  earlier_kernels_done();
+  later_kernels_may_start();
+  if (tid < NCONS) {
+    const int NB = (Tn + W - 1) / W, NG = (Tn + GT - 1) / GT;
+    const long long base = bi * lay.sb + hi * lay.sh, rows = (long long)ys * RV * N;
+    StateRows<N, ROWS> S(tid);
+    S.get(s_in && n_state > 0 ? s_in + (long long)(n_state == 1 ? hi : unit) * N * N + rows : nullptr);
+    for (int i = 0, slot = 0, phase = 0; i < nb; ++i) {
+      const int n = BWD ? NB - 1 - idx0 - i : idx0 + i;
+      if (ckpt)
+        if (float* p = state_slot<N, BWD>(ckpt, unit, NG, n)) S.put(p + rows);
+      if (!tc::mbar_wait(&sm.full[slot], phase, status, 501)) break;
+      float oo[ROWS];
+      S.step(sm.stage[slot], oo);
+      __syncwarp();
+      if (S.lane == 0) tc::mbar_arrive(&sm.empty[slot]);
+      const int t = n * W + (BWD ? W - 1 - S.jl : S.jl);
+      if (out && t < Tn) S.put_out(out + base + (long long)t * lay.st + ys * RV, oo);
+      if (++slot == SLOTS) { slot = 0; phase ^= 1; }
+    }
+    if (s_out) S.put(s_out + (long long)unit * N * N + rows);
+  } else if (tc::elect_one()) {
+    const Stage<N, N>* src = stages + (long long)unit * nb;
+    for (int i = 0, slot = 0, phase = 1; i < nb; ++i, ++src) {
+      if (i >= SLOTS && !tc::mbar_wait(&sm.empty[slot], phase, status, 502)) break;
+      tc::mbar_expect_tx(&sm.full[slot], COMMON_BYTES<N> + SLICE_BYTES);
+      tc::bulk_load(&sm.stage[slot], src, COMMON_BYTES<N>, &sm.full[slot]);
+      tc::bulk_load(&sm.stage[slot].vt[0][0], &src->vt[ys * RV][0], SLICE_BYTES, &sm.full[slot]);
+      if (++slot == SLOTS) { slot = 0; phase ^= 1; }
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -796,37 +952,93 @@ r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, c
 }
 
 template <typename T, int N, bool BWD, int GROUPS, int ROWS>
-int launch_sweep(const DeviceFacts& dev, const Vecs<T>& in, const void* v, const float* s_in, int n_state, void* out, float* s_out,
-                 float* ckpt, int B, int Tn, int H, const TokLayout& lay, cudaStream_t st) {
+int launch_inline(const DeviceFacts& dev, const Vecs<T>& in, const void* v, const float* s_in, int n_state, void* out, float* s_out,
+                  float* ckpt, int B, int Tn, int H, const TokLayout& lay, cudaStream_t st) {
   constexpr int bytes = (int)sizeof(Group<T, N>);
-  if (allow_smem<r7_sweep_kernel<T, N, BWD, GROUPS, ROWS>>(dev, GROUPS * bytes)) return RWKVB200_E_CUDA;
+  if (allow_smem<r7_sweep_inline_kernel<T, N, BWD, GROUPS, ROWS>>(dev, GROUPS * bytes)) return RWKVB200_E_CUDA;
   const int blocks = (Tn + W - 1) / W, groups = blocks < GROUPS ? blocks : GROUPS;      // a group without a block is left out
   ProfScope prof(BWD ? "r7_sweep_bwd_kernel" : "r7_sweep_fwd_kernel", st);
-  return launch(r7_sweep_kernel<T, N, BWD, GROUPS, ROWS>, dim3(B * H, N / RV), state_threads<N, ROWS>() + N * groups, groups * bytes, st, 1,
-                in, (const T*)v, s_in, n_state, (T*)out, s_out, ckpt, Tn, H, lay);
+  return launch(r7_sweep_inline_kernel<T, N, BWD, GROUPS, ROWS>, dim3(B * H, N / RV), state_threads<N, ROWS>() + N * groups,
+                groups * bytes, st, 1, in, (const T*)v, s_in, n_state, (T*)out, s_out, ckpt, Tn, H, lay);
+}
+
+template <typename T, int N, bool BWD, int SLOTS, int ROWS, int PER_SM>
+int launch_sweep(const DeviceFacts& dev, const Stage<N, N>* stages, const float* s_in, int n_state, void* out, float* s_out, float* ckpt,
+                 int B, int Tn, int H, int idx0, int nb, const TokLayout& lay, cudaStream_t st) {
+  constexpr int bytes = (int)sizeof(SweepSmem<N, SLOTS>);
+  if (allow_smem<r7_sweep_kernel<T, N, BWD, SLOTS, ROWS, PER_SM>>(dev, bytes)) return RWKVB200_E_CUDA;
+  ProfScope prof(BWD ? "r7_sweep_bwd_kernel" : "r7_sweep_fwd_kernel", st);
+  return launch(r7_sweep_kernel<T, N, BWD, SLOTS, ROWS, PER_SM>, dim3(B * H, N / RV), state_threads<N, ROWS>() + 32, bytes, st, PER_SM == 1 ? 1 : 0, stages, s_in,
+                n_state, (T*)out, s_out, ckpt, Tn, H, idx0, nb, lay, dev.status);
+}
+
+// Scratch of a sweep: stages of as many blocks of every unit as fit STAGES_BYTES (at least 8), and the units' states between one
+// such stretch and the next.  (More than L2 holds costs little: 1.4 KB per token and head, where the inputs take 1.5.)
+constexpr size_t STAGES_BYTES = (size_t)256 << 20;
+// From how many blocks per unit on they are prepared by a kernel of their own (forward, us; inside the sweep against apart):
+// with at most one CTA per SM the sweep has to be long enough for the other kernel (12 units, T 128 15.8 and 15.0, T 300 32.7 and
+// 29.3, T 1024 101 and 83; 37 units 16.0 and 18.5, 33.0 and 31.6, 101 and 96); at head size 64 two CTAs per SM inside keep up
+// (60 units, T 300 57 and 60); beyond that it pays from the start (128 units, T 32 15.6 and 14.7, T 1024 364 and 227; head size
+// 128, 64 units, T 1024 711 and 375).
+constexpr int STAGED_BLOCKS = 4;
+template <int N> int staged_from(int ctas, int sms) {
+  if (ctas <= sms) return N == 64 ? 48 : 12;
+  return N == 64 && ctas <= 2 * sms ? 1 << 30 : STAGED_BLOCKS;
+}
+template <int N> int stretch_blocks(long long units, int NB) {
+  const long long fit = (long long)(STAGES_BYTES / sizeof(Stage<N, N>)) / units;
+  return (int)(fit < 8 ? (NB < 8 ? NB : 8) : fit < NB ? fit : NB);
+}
+template <int N> size_t scratch_bytes(long long units, int Tn) {
+  const int NB = (Tn + W - 1) / W;
+  if (NB < STAGED_BLOCKS) return 0;
+  return (size_t)units * (stretch_blocks<N>(units, NB) * sizeof(Stage<N, N>) + N * N * sizeof(float));
 }
 
 template <typename T, int N, bool BWD>
 int sweep(const Vecs<T>& in, const void* v, const float* s_in, int n_state, void* out, float* s_out, float* ckpt, int B,
-          int Tn, int H, const TokLayout& lay, cudaStream_t st) {
+          int Tn, int H, const TokLayout& lay, void* scratch, cudaStream_t st) {
   DeviceFacts dev;
   if (int e = device_facts(&dev)) return e;
-  return B * H * (N / RV) > dev.sms
-             ? launch_sweep<T, N, BWD, MANY_CTAS<T, N>, MANY_CTAS_ROWS>(dev, in, v, s_in, n_state, out, s_out, ckpt, B, Tn, H, lay, st)
-             : launch_sweep<T, N, BWD, FEW_CTAS<N>, FEW_CTAS_ROWS<N>>(dev, in, v, s_in, n_state, out, s_out, ckpt, B, Tn, H, lay, st);
+  const int units = B * H, NB = (Tn + W - 1) / W;
+  const bool many = units * (N / RV) > dev.sms;
+  if (!scratch || NB < staged_from<N>(units * (N / RV), dev.sms))
+    return many ? launch_inline<T, N, BWD, MANY_CTAS<T, N>, MANY_CTAS_ROWS>(dev, in, v, s_in, n_state, out, s_out, ckpt, B, Tn, H, lay, st)
+                : launch_inline<T, N, BWD, FEW_CTAS<N>, FEW_CTAS_ROWS<N>>(dev, in, v, s_in, n_state, out, s_out, ckpt, B, Tn, H, lay, st);
+  const int stretch = stretch_blocks<N>(units, NB);
+  auto* stages = static_cast<Stage<N, N>*>(scratch);
+  float* between = reinterpret_cast<float*>(stages + (size_t)units * stretch);
+  constexpr int per_cta = PREPARE_THREADS / N, bytes = per_cta * (int)sizeof(PrepareSmem<T, N>);
+  if (allow_smem<r7_prepare_kernel<T, N, BWD>>(dev, bytes)) return RWKVB200_E_CUDA;
+  for (int idx0 = 0; idx0 < NB; idx0 += stretch) {
+    const int nb = NB - idx0 < stretch ? NB - idx0 : stretch, n_items = units * nb;
+    {
+      ProfScope prof("r7_prepare_kernel", st);
+      if (int e = launch(r7_prepare_kernel<T, N, BWD>, (n_items + per_cta - 1) / per_cta, PREPARE_THREADS, bytes, st, 1, in, (const T*)v,
+                         stages, Tn, H, idx0, nb, n_items, lay)) return e;
+    }
+    const bool first = idx0 == 0, last = idx0 + nb == NB;
+    const float* from = first ? s_in : between;
+    float* to = last ? s_out : between;
+    const int n_from = first ? n_state : units;
+    const int e = many ? launch_sweep<T, N, BWD, 4, MANY_CTAS_ROWS, 3>(dev, stages, from, n_from, out, to, ckpt, B, Tn, H, idx0, nb, lay, st)
+                       : launch_sweep<T, N, BWD, FEW_CTAS_SLOTS<N>, FEW_CTAS_ROWS<N>, 1>(dev, stages, from, n_from, out, to, ckpt, B, Tn, H, idx0, nb, lay, st);
+    if (e) return e;
+  }
+  return RWKVB200_OK;
 }
 
 template <typename T, int N>
 int fwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b, const float* h0, int n_state,
-        void* o, float* ht, float* states, int B, int Tn, int H, int head_first, cudaStream_t st) {
+        void* o, float* ht, float* states, void* scratch, int B, int Tn, int H, int head_first, cudaStream_t st) {
   const Vecs<T> in{{(const T*)r, (const T*)w, (const T*)k, (const T*)a, (const T*)b}};
-  return sweep<T, N, false>(in, v, h0, n_state, o, ht, Tn > GT ? states : nullptr, B, Tn, H, TokLayout(Tn, H, head_first, N), st);
+  return sweep<T, N, false>(in, v, h0, n_state, o, ht, Tn > GT ? states : nullptr, B, Tn, H, TokLayout(Tn, H, head_first, N), scratch, st);
 }
 
 template <typename T, int N>
 int bwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b, const float* h0, int n_state,
-        const void* d_o, const float* d_ht, const float* kept, float* ckpt, void* dr, void* dw, void* dk, void* dv, void* da, void* db,
-        float* d_h0, int B, int Tn, int H, int head_first, cudaStream_t st) {
+        const void* d_o, const float* d_ht, const float* kept, float* ckpt, void* scratch, void* dr, void* dw, void* dk, void* dv, void* da,
+        void* db, float* d_h0, int B, int Tn, int H, int head_first, cudaStream_t st) {
   const Vecs<T> in{{(const T*)r, (const T*)w, (const T*)k, (const T*)a, (const T*)b}};
   const TokLayout lay(Tn, H, head_first, N);
   int e = RWKVB200_OK;
@@ -836,9 +1048,9 @@ int bwd(const void* r, const void* w, const void* k, const void* v, const void* 
   if (Tn > GT && !kept) {
     states = ckpt;
     d_states = ckpt + (long long)B * H * ((Tn + GT - 1) / GT - 1) * N * N;
-    e = sweep<T, N, false>(in, v, h0, n_state, nullptr, nullptr, ckpt, B, Tn, H, lay, st);
+    e = sweep<T, N, false>(in, v, h0, n_state, nullptr, nullptr, ckpt, B, Tn, H, lay, scratch, st);
   }
-  if (!e) e = sweep<T, N, true>(in, d_o, d_ht, d_ht ? B * H : 0, dv, d_h0, Tn > GT ? d_states : nullptr, B, Tn, H, lay, st);
+  if (!e) e = sweep<T, N, true>(in, d_o, d_ht, d_ht ? B * H : 0, dv, d_h0, Tn > GT ? d_states : nullptr, B, Tn, H, lay, scratch, st);
   if (e) return e;
   DeviceFacts dev;
   if ((e = device_facts(&dev))) return e;
@@ -863,22 +1075,27 @@ size_t rwkv7_block_states_bytes(int B, int Tn, int H, int dtype, int head_size) 
   return Tn > GT ? (size_t)B * H * ((Tn + GT - 1) / GT - 1) * head_size * head_size * sizeof(float) : 0;
 }
 
+size_t rwkv7_block_scratch_bytes(int B, int Tn, int H, int dtype, int head_size) {
+  if (head_size == 64) return dtype == RWKVB200_BF16 ? 0 : scratch_bytes<64>((long long)B * H, Tn);
+  return scratch_bytes<128>((long long)B * H, Tn);
+}
+
 int launch_rwkv7_block_fwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
                            const float* h0, int n_state, void* o, float* ht, int B, int Tn, int H, int dtype,
-                           int head_first, cudaStream_t st, int head_size, float* states) {
+                           int head_first, cudaStream_t st, int head_size, float* states, void* scratch) {
   if (head_size == 64 && dtype == RWKVB200_BF16)
     return launch_rwkv7_rec_fwd(r, w, k, v, a, b, h0, n_state, o, ht, B, Tn, H, head_first, st);
-  R7_BLOCK_DISPATCH((fwd<T, N>(r, w, k, v, a, b, h0, n_state, o, ht, states, B, Tn, H, head_first, st)))
+  R7_BLOCK_DISPATCH((fwd<T, N>(r, w, k, v, a, b, h0, n_state, o, ht, states, scratch, B, Tn, H, head_first, st)))
 }
 
 int launch_rwkv7_block_bwd(const void* r, const void* w, const void* k, const void* v, const void* a, const void* b,
                            const float* h0, int n_state, const void* d_o, const float* d_ht, float* ckpt,
                            void* dr, void* dw, void* dk, void* dv, void* da, void* db, float* d_h0, int B, int Tn, int H,
-                           int dtype, int head_first, cudaStream_t st, int head_size, const float* states) {
+                           int dtype, int head_first, cudaStream_t st, int head_size, const float* states, void* scratch) {
   if (head_size == 64 && dtype == RWKVB200_BF16)
     return launch_rwkv7_rec_bwd(r, w, k, v, a, b, h0, n_state, d_o, d_ht, ckpt, dr, dw, dk, dv, da, db, d_h0, B, Tn, H,
                                 head_first, st, UnitSel{}, 0);
-  R7_BLOCK_DISPATCH((bwd<T, N>(r, w, k, v, a, b, h0, n_state, d_o, d_ht, states, ckpt, dr, dw, dk, dv, da, db, d_h0, B, Tn, H,
+  R7_BLOCK_DISPATCH((bwd<T, N>(r, w, k, v, a, b, h0, n_state, d_o, d_ht, states, ckpt, scratch, dr, dw, dk, dv, da, db, d_h0, B, Tn, H,
                                head_first, st)))
 }
 

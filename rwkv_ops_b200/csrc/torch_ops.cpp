@@ -217,9 +217,11 @@ Three rwkv7_fwd(const Tensor& r, const Tensor& w, const Tensor& k, const Tensor&
                               d.B, d.H, d.K, code, stream_of(r)), "rwkv7_step");
   } else if (keep && !chunked_rwkv7(d, code, algo)) {
     const size_t n = rwkvb200_rwkv7_states_bytes(d.B, d.T, d.H, d.K, code, (int)algo);
+    const size_t ns = rwkvb200_rwkv7_fwd_workspace_bytes(d.B, d.T, d.H, d.K, code, (int)algo);
+    const Tensor scratch = ns ? bytes(ns, r) : Tensor();
     ws = bytes(n, r);
-    check(rwkvb200_rwkv7_fwd_states(ptr(r), ptr(w), ptr(k), ptr(v), ptr(a), ptr(b), fptr(h0), n_state_of(h0), ptr(o),
-                                    fptr(ht), fptr(ws), n, d.B, d.T, d.H, d.K, code, head_first, (int)algo, stream_of(r)),
+    check(rwkvb200_rwkv7_fwd_states(ptr(r), ptr(w), ptr(k), ptr(v), ptr(a), ptr(b), fptr(h0), n_state_of(h0), ptr(o), fptr(ht),
+                                    fptr(ws), n, ptr(scratch), ns, d.B, d.T, d.H, d.K, code, head_first, (int)algo, stream_of(r)),
           "rwkv7_fwd");
   } else {
     const size_t nws = rwkvb200_rwkv7_fwd_workspace_bytes(d.B, d.T, d.H, d.K, code, flags);
@@ -242,10 +244,10 @@ Seven rwkv7_bwd(const Tensor& r, const Tensor& w, const Tensor& k, const Tensor&
   Tensor dr = fresh_like(r), dw = fresh_like(r), dk = fresh_like(r), dv = fresh_like(r), da = fresh_like(r),
          db = fresh_like(r), dh0 = fresh({d.B, d.H, d.K, d.K}, at::kFloat, r);
   if (have && !chunked_rwkv7(d, code, algo)) {
-    const Tensor ws = fresh_like(kept);
-    const size_t n = (size_t)kept.numel();
+    const size_t n = rwkvb200_rwkv7_bwd_states_workspace_bytes(d.B, d.T, d.H, d.K, code, (int)algo);
+    const Tensor ws = bytes(n, r);
     check(rwkvb200_rwkv7_bwd_states(ptr(r), ptr(w), ptr(k), ptr(v), ptr(a), ptr(b), fptr(h0), n_state_of(h0), ptr(d_o),
-                                    fptr(d_ht), fptr(kept), n, ptr(dr), ptr(dw), ptr(dk), ptr(dv), ptr(da), ptr(db), fptr(dh0),
+                                    fptr(d_ht), fptr(kept), (size_t)kept.numel(), ptr(dr), ptr(dw), ptr(dk), ptr(dv), ptr(da), ptr(db), fptr(dh0),
                                     ptr(ws), n, d.B, d.T, d.H, d.K, code, head_first, (int)algo, stream_of(r)), "rwkv7_bwd");
     return {dr, dw, dk, dv, da, db, dh0};
   }

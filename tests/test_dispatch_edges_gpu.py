@@ -175,3 +175,27 @@ def test_states_kept_for_the_backward(T, K, dtype, monkeypatch):
     again = grads()
     for a, b, c in zip(*kept, again[0]):
         assert torch.equal(a, b) and torch.equal(a, c)
+
+
+@pytest.mark.parametrize("K,dtype", [(64, torch.float32), (64, torch.float16), (128, torch.float32), (128, torch.bfloat16)])
+@pytest.mark.parametrize("few", [False, True])
+def test_blocks_prepared_apart(K, dtype, few):
+    """The sweeps with and without their scratch (C ABI): the same bits, at the block counts from which the scratch is used, and
+    where a unit's blocks take several stretches of it."""
+    lib, dev = _lib.load(), torch.device("cuda")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    code = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}[dtype]
+    H = 3 if few else 2 * sms // (K // 16) + 2
+    for T in ((95, 96, 377, 384, 400) if few else (24, 25, 32, 33, 70)) + (() if few or K == 128 else (2500,)):
+        d = rwkv7_inputs(1, T, H, K, dtype=dtype, seed=T, device="cuda", with_state=True)
+        x = [d[n] for n in "rwkvab"]
+        out = []
+        for scratch in (True, False):
+            o, s = torch.empty_like(x[0]), torch.empty(1, H, K, K, device=dev)
+            n = lib.rwkvb200_rwkv7_fwd_workspace_bytes(1, T, H, K, code, _lib.ALGO_RECURRENT) if scratch else 0
+            ws = torch.empty(n, dtype=torch.uint8, device=dev)
+            _lib.check(lib.rwkvb200_rwkv7_fwd(*(_lib.ptr(t) for t in x), _lib.ptr(d["initial_state"]), 1, _lib.ptr(o), _lib.ptr(s),
+                                              _lib.ptr(ws) if n else None, n, 1, T, H, K, code, 0, _lib.ALGO_RECURRENT,
+                                              _lib.stream_ptr(dev)), "fwd")
+            out.append((o, s))
+        assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1]), T
