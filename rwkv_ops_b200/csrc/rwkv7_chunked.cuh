@@ -136,6 +136,38 @@ struct ChunkWalk {
   }
 };
 
+// The unit of a scan's block in a packed batch: the longest sequences come first, so that the blocks which start when others have ended are
+// short ones.  Up to MAX_SORTED sequences are ranked by length, by the threads of the block.
+constexpr int MAX_SORTED = 256;
+struct SortedSeqs { int len[MAX_SORTED], at; };
+__device__ __forceinline__ int packed_scan_unit(const SeqView& sv, int H, SortedSeqs* sorted, int tid) {
+  const int n_seq = gridDim.x / H, b = blockIdx.x;
+  if (n_seq > MAX_SORTED) return b;
+  if (tid < n_seq) sorted->len[tid] = __ldg(sv.len + tid);
+  __syncthreads();
+  if (tid < n_seq) {
+    const int mine = sorted->len[tid];
+    int rank = 0;
+    for (int i = 0; i < n_seq; ++i) rank += sorted->len[i] > mine || (sorted->len[i] == mine && i < tid);
+    if (rank == b / H) sorted->at = tid;
+  }
+  __syncthreads();
+  return sorted->at * H + b % H;
+}
+// Whether the scans run one block to an SM.  Dense: with at most a sequence and head per SM.  Packed: also where the longest
+// sequence, whose chunks take 3.3 us each with two blocks to an SM and 1.3 alone, would end long after the others; `kb`: KB that a
+// chunk moves, of 6 TB/s that the scans reach.  (8 sequences of 1093 .. 4096 tokens, 32 heads: forward 215 -> 194 us, reverse 115 -> 104;
+// as many equally long ones take 257 and 262.)
+inline bool scans_alone(int n_seq, int Tn, int T_total, int H, int sms, bool packed, float kb) {
+  const int units = n_seq * H;
+  if (units <= sms) return true;
+  if (!packed || n_seq > MAX_SORTED) return false;
+  const float longest = (float)num_chunks(Tn), mean = (float)T_total / n_seq / L + 0.5f, per_sm = mean * units / sms;
+  const float rounds = fmaxf(longest, per_sm + 0.25f * mean);      // chunks in a row on the slowest SM
+  const float memory = units * mean * kb / 6000.f;
+  return fmaxf(rounds * 1.3f, memory * rounds / per_sm) < fmaxf(longest * 3.3f, memory);
+}
+
 // Fused producers (template parameter FUSED of the intra and final kernels).  The three inputs w, a, b of
 // the delta rule are then computed on the fly from pre-activations p, u, q of the same shape,
 //   w = -e^{-1/2} sigmoid(p),   kk = u / max(|u|_2, 1e-12) over the 64 channels of a head,

@@ -42,8 +42,7 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
   extern __shared__ unsigned char smem_raw[];
   BScanSmem& sm = *reinterpret_cast<BScanSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int unit = blockIdx.x, bi = unit / H, hi = unit % H;
-  const size_t ch0 = (size_t)unit * NT_slots;
+  int unit = blockIdx.x, bi = unit / H, hi = unit % H;
   const int wq = warp & 3, hsel = warp >> 2, c0 = 32 * hsel;
   const int row = 16 * wq + (lane & 15);
   const bool state_lane = lane < 16;
@@ -63,6 +62,11 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
   tc_fence_after();
   earlier_kernels_done();
   later_kernels_may_start();
+  if constexpr (PACKED) {
+    unit = packed_scan_unit(sv, H, reinterpret_cast<SortedSeqs*>(sm.dz), tid);
+    bi = unit / H; hi = unit % H;
+  }
+  const size_t ch0 = (size_t)unit * NT_slots;
   const int NT = (sv.length<PACKED>(bi) + L - 1) / L;      // chunks of this sequence
   const int tb = sv.first<PACKED>(bi), brow = sv.row<PACKED>(bi);
   const uint32_t tm = sm.tmem_base;
@@ -220,8 +224,7 @@ r7c_bwd_scan_alone_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned 
   extern __shared__ unsigned char smem_raw[];
   BAloneSmem& sm = *reinterpret_cast<BAloneSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int unit = blockIdx.x, bi = unit / H, hi = unit % H;
-  const size_t ch0 = (size_t)unit * NT_slots;
+  int unit = blockIdx.x, bi = unit / H, hi = unit % H;
   const int wq = warp & 3, c0 = 32 * (warp >> 2);
   const int row = 16 * wq + (lane & 15);
   const bool state_lane = lane < 16;
@@ -239,6 +242,11 @@ r7c_bwd_scan_alone_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned 
   tc_fence_after();
   earlier_kernels_done();
   later_kernels_may_start();
+  if constexpr (PACKED) {
+    unit = packed_scan_unit(sv, H, reinterpret_cast<SortedSeqs*>(sm.dz[0]), tid);
+    bi = unit / H; hi = unit % H;
+  }
+  const size_t ch0 = (size_t)unit * NT_slots;
   const int NT = (sv.length<PACKED>(bi) + L - 1) / L;      // chunks of this sequence
   const int tb = sv.first<PACKED>(bi), brow = sv.row<PACKED>(bi);
   auto chunk_tiles = [&](int n) { return ws_tiles + (ch0 + NT - 1 - n) * (size_t)tiles_per_chunk * TILE_BYTES; };
@@ -941,10 +949,10 @@ int launch_rwkv7_chunked_bwd(const void* r, const void* w, const void* k, const 
     do {                                                                                                          \
       const int smem = (int)sizeof(SMEM) + 1024;                                                                  \
       if (allow_smem<KERNEL<P>>(dev, smem)) return RWKVB200_E_CUDA;                                               \
-      if (int rc = launch(KERNEL<P>, B * H, THREADS, smem, st, 1, tmap_do, ws.tiles, ws.aux, (int)ALL_TILES, d_ht, d_h0, sv, H, \
-                          NT, status)) return rc;                                                                  \
+      if (int rc = launch(KERNEL<P>, B * H, THREADS, smem, st, 1, tmap_do, ws.tiles, ws.aux, (int)ALL_TILES, \
+                          d_ht, d_h0, sv, H, NT, status)) return rc;                                                                  \
     } while (0)
-    if (B * H > dev.sms) {      // two CTAs per SM
+    if (!scans_alone(B, Tn, T_total, H, dev.sms, seq_start != nullptr, 56.f)) {      // two CTAs per SM
       if (seq_start) R7C_LAUNCH_BSCAN(r7c_bwd_scan_kernel, true, 256, BScanSmem);
       else           R7C_LAUNCH_BSCAN(r7c_bwd_scan_kernel, false, 256, BScanSmem);
     } else {

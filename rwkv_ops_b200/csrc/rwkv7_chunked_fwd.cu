@@ -599,9 +599,8 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
   extern __shared__ unsigned char smem_raw[];
   ScanSmem& sm = *reinterpret_cast<ScanSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  int unit = blockIdx.x, bi = unit / H, hi = unit % H;
   const int wq = warp & 3, hsel = warp >> 2, c0 = 32 * hsel;
-  const int unit = blockIdx.x, bi = unit / H, hi = unit % H;
-  const size_t ch0 = (size_t)unit * NT_slots;
   const int row = 16 * wq + (lane & 15);     // state row k (lanes 0-15) or token row i (lanes 16-31)
   const bool state_lane = lane < 16;
   // Single-thread jobs: warp 0 issues the MMAs, ld_warp requests operand tiles, st_warp copies sa, h~0 and X out for the
@@ -621,6 +620,11 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
   tc_fence_after();
   earlier_kernels_done();
   later_kernels_may_start();
+  if constexpr (PACKED) {
+    unit = packed_scan_unit(sv, H, reinterpret_cast<SortedSeqs*>(sm.ot), tid);
+    bi = unit / H; hi = unit % H;
+  }
+  const size_t ch0 = (size_t)unit * NT_slots;
   const int Tn = sv.length<PACKED>(bi), tb = sv.first<PACKED>(bi), brow = sv.row<PACKED>(bi);
   const int NT = (Tn + L - 1) / L;           // chunks of this sequence (at least one)
   const uint32_t tm = sm.tmem_base;
@@ -895,12 +899,10 @@ r7c_scan_fwd_alone_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsi
   extern __shared__ unsigned char smem_raw[];
   AloneSmem& sm = *reinterpret_cast<AloneSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  int unit = blockIdx.x, bi = unit / H, hi = unit % H;
   const int wq = warp & 3, c0 = 32 * (warp >> 2);
-  const int unit = blockIdx.x, bi = unit / H, hi = unit % H;
-  const size_t ch0 = (size_t)unit * NT_slots;
   const int row = 16 * wq + (lane & 15);     // state row k (lanes 0-15) or token row i (lanes 16-31)
   const bool state_lane = lane < 16;
-  auto chunk_tiles = [&](int c) { return ws_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES; };
 
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) { mbar_init(&sm.bar_g1[i], 1); mbar_init(&sm.bar_g2[i], 1); mbar_init(&sm.bar_o[i], 1); }
@@ -915,6 +917,12 @@ r7c_scan_fwd_alone_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsi
   tc_fence_after();
   earlier_kernels_done();
   later_kernels_may_start();
+  if constexpr (PACKED) {
+    unit = packed_scan_unit(sv, H, reinterpret_cast<SortedSeqs*>(sm.ot[0]), tid);
+    bi = unit / H; hi = unit % H;
+  }
+  const size_t ch0 = (size_t)unit * NT_slots;
+  auto chunk_tiles = [&](int c) { return ws_tiles + (ch0 + c) * (size_t)tiles_per_chunk * TILE_BYTES; };
   const int Tn = sv.length<PACKED>(bi), tb = sv.first<PACKED>(bi), brow = sv.row<PACKED>(bi);
   const int NT = (Tn + L - 1) / L;           // chunks of this sequence (at least one)
   // TMEM: columns 0..63 lower lane halves = W h~0; three accumulators in turn: lower halves k~^T v + b~^T sa, upper halves
@@ -1214,7 +1222,7 @@ int launch_rwkv7_chunked_fwd(const void* r, const void* w, const void* k, const 
           keep_for_bwd ? ws.tiles : nullptr, h0, n_state, tmap_o, o ? 1 : 0, ht, (bf16*)o, sv, H, NT, lay, exact,  \
           status, debug_stamp_buffer())) return rc;                                                                \
     } while (0)
-    if (B * H > dev.sms) {
+    if (!scans_alone(B, Tn, T_total, H, dev.sms, seq_start != nullptr, 96.f)) {
       if (seq_start) R7C_LAUNCH_SCAN(r7c_scan_fwd_kernel, true, 256, ScanSmem);
       else           R7C_LAUNCH_SCAN(r7c_scan_fwd_kernel, false, 256, ScanSmem);
     } else {

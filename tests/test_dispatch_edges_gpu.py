@@ -199,3 +199,28 @@ def test_blocks_prepared_apart(K, dtype, few):
                                               _lib.stream_ptr(dev)), "fwd")
             out.append((o, s))
         assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1]), T
+
+
+@pytest.mark.parametrize("lens,H", [([1500, 70, 64, 8, 200, 130, 9, 65, 300, 128], 20), ([8 + i % 70 for i in range(260)], 1)])
+def test_scans_of_a_packed_batch_with_more_units_than_SMs(lens, H):
+    """One sequence much longer than the others (its scans run one block to an SM, longest first), and more sequences than are
+    ranked by length: as each sequence on its own."""
+    assert len(lens) * H > torch.cuda.get_device_properties(0).multi_processor_count
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    d = rwkv7_inputs(1, cu[-1], H, dtype=torch.bfloat16, seed=31, device="cuda", with_grads=True)
+    d_s = 0.1 * torch.randn(len(lens), H, 64, 64, device="cuda")
+
+    def run(fn, x, d_o, d_state):
+        x = [t.clone().requires_grad_(True) for t in x]
+        o, s = fn(*x)
+        return [s.detach(), o.detach(), *torch.autograd.grad([o, s], x, [d_o, d_state])]
+
+    tokens = [d[n] for n in "rwkvab"]
+    out = run(lambda *x: ro.generalized_delta_rule_varlen(*x, cu), tokens, d["d_out"], d_s)
+    for i in list(range(min(len(lens), 10))) + [len(lens) - 1]:
+        at = slice(cu[i], cu[i + 1])
+        ref = run(ro.generalized_delta_rule, [t[:, at].contiguous() for t in tokens], d["d_out"][:, at].contiguous(), d_s[i:i + 1])
+        for m, (a, b) in enumerate(zip(out, ref)):
+            assert rel_l2(a[i:i + 1] if m == 0 else a[:, at], b) < 2e-3, (i, m)
