@@ -1419,7 +1419,8 @@ int launch_wkv6_chunked_bwd(const void* r, const void* k, const void* v, const v
     const int n_units = B * H;
     split = n_units > sms && (Tn + L - 1) / L >= 4;
     const int grid = split ? sms : n_units;
-    if (split && cuda_ok(cudaMemsetAsync(ws.hflags, 0, ((size_t)n_units + 1) * sizeof(int), st))) return RWKVB200_E_CUDA;
+    if (split)
+      if (int rc = launch(w6c_clear_kernel, 1, 256, 0, st, 1, ws.hflags, n_units + 1)) return rc;
     ProfScope prof("wkv6c_bwd_kernel", st);
     RWKVB200_DISPATCH_DTYPE(dtype, W6C_DISPATCH_PACKED(
       if (allow_smem<wkv6c_bwd_kernel<T, P>>(dev, smem)) return RWKVB200_E_CUDA;
