@@ -67,7 +67,17 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
     mbar_init(&sm.bar_m4, 1); mbar_init(&sm.bar_m5, 1);
     fence_mbar_init();
   }
-  if (tid == 32) tma_prefetch_maps(tmap_q, tmap_w, tmap_k, tmap_a, tmap_b, tmap_v);
+  if (tid == 32) {
+    tma_prefetch_maps(tmap_q, tmap_w, tmap_k, tmap_a, tmap_b, tmap_v);
+    if constexpr (!PACKED) {      // the first rows into L2, while the kernel before runs out
+      const ChunkPos p = ChunkWalk<PACKED, true>{sv, dims}.first();
+      tma_prefetch_4d(&tmap_w, 0, p.c * L, p.hi, p.bi);
+      tma_prefetch_4d(&tmap_q, 0, p.c * L, p.hi, p.bi);
+      tma_prefetch_4d(&tmap_k, 0, p.c * L, p.hi, p.bi);
+      tma_prefetch_4d(&tmap_a, 0, p.c * L, p.hi, p.bi);
+      tma_prefetch_4d(&tmap_b, 0, p.c * L, p.hi, p.bi);
+    }
+  }
   if (warp == 0) tmem_alloc(&sm.tmem_base, 256);
   tc_fence_before();
   __syncthreads();
