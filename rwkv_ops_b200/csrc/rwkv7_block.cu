@@ -581,9 +581,10 @@ r7_sweep_kernel(const Stage<N, N>* __restrict__ stages, const float* s_in, int n
 // G_j^T v_i and G_j^T sa_i through the 16 tokens with the scalars sa.do, v.do, sa.dsa, v.dsa (four threads to a
 // channel).  dd_j is summed from the same quantities, positive decay factors throughout, so no term cancels that does not in
 // the token-by-token form.  Bound by shared-memory reads (two 16-byte reads per 16 products).
+template <int N> constexpr bool BOTH_STATES = N == 64;      // both fit; at N = 128 G replaces S and S is fetched again
 template <int N>
 struct GradSmem {
-  float st[N][N + 4];                 // S, then G, then S again
+  float st[BOTH_STATES<N> ? 2 : 1][N][N + 4];      // S, G
   float raw[5][GT][N];                // r, d, k, a, b
   float xs[GT][N + 4];                // a~, then b^
   float cat1[N][36], cat2[N][36];     // [sa v], [do dsa], one row per value channel
@@ -609,12 +610,25 @@ r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, c
   const long long base = bi * lay.sb + hi * lay.sh + (long long)t0 * lay.st;
   const int nt = min(GT, Tn - t0);
   const long long cu = (long long)unit * (NG - 1) + m;      // this unit's boundaries lie between its groups of tokens
+  const float* ckpt_any = reinterpret_cast<const float*>(v);      // (an address for copies of nothing)
   const float* Sg = m > 0 ? states + (cu - 1) * N * N : n_state > 0 ? h0 + (long long)(n_state == 1 ? hi : unit) * N * N : nullptr;
   const float* Gg = m < NG - 1 ? d_states + cu * N * N : d_ht ? d_ht + (long long)unit * N * N : nullptr;
 
-  // ---- tokens and S
+  // ---- tokens and states; everything is requested before anything is waited for
   const int kq = tid % (N / 4), row0 = tid / (N / 4);      // quad of channels, token / state row (16 at a time)
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float (*const S)[N + 4] = sm.st[0];
+  float (*const G)[N + 4] = sm.st[BOTH_STATES<N> ? 1 : 0];
+  auto request_state = [&](float (*to)[N + 4], const float* g) {
+#pragma unroll
+    for (int x = 0; x < N / 16; ++x) {
+      const int rr = row0 + 16 * x;
+      cp_async16(&to[rr][4 * kq], g ? g + (long long)rr * N + 4 * kq : ckpt_any, g != nullptr);
+    }
+  };
+  request_state(S, Sg);
+  if constexpr (BOTH_STATES<N>) request_state(G, Gg);
+  cp_async_commit();
   // four values down a column of an array whose rows are 36 floats long: every second lane starts with another one of
   // them, which leaves two of the eight lanes that would meet on a bank
   auto put_column = [&](const float (&f)[4], auto at) {
@@ -627,25 +641,19 @@ r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, c
   {
     const bool live = row0 < nt;
     const long long off = base + (live ? (long long)row0 * lay.st : 0) + 4 * kq;
+    float4 f[5], fv = zero, fo = zero;
+#pragma unroll
+    for (int i = 0; i < 5; ++i) f[i] = live ? load4(in.p[i] + off) : zero;
+    if (live) { fv = load4(v + off); fo = load4(d_o + off); }
 #pragma unroll
     for (int i = 0; i < 5; ++i) {
-      float4 f = live ? load4(in.p[i] + off) : zero;
-      if (i == VW) f = live ? make_float4(decay_of(f.x), decay_of(f.y), decay_of(f.z), decay_of(f.w)) : make_float4(1.f, 1.f, 1.f, 1.f);
-      *reinterpret_cast<float4*>(&sm.raw[i][row0][4 * kq]) = f;
+      if (i == VW) f[i] = live ? make_float4(decay_of(f[i].x), decay_of(f[i].y), decay_of(f[i].z), decay_of(f[i].w)) : make_float4(1.f, 1.f, 1.f, 1.f);
+      *reinterpret_cast<float4*>(&sm.raw[i][row0][4 * kq]) = f[i];
     }
-    const float4 fv = live ? load4(v + off) : zero, fo = live ? load4(d_o + off) : zero;
     const float ev[4] = {fv.x, fv.y, fv.z, fv.w}, eo[4] = {fo.x, fo.y, fo.z, fo.w};
     put_column(ev, [&](int x) { return &sm.cat1[4 * kq + x][GT + row0]; });
     put_column(eo, [&](int x) { return &sm.cat2[4 * kq + x][row0]; });
   }
-  auto get_state = [&](const float* g) {
-#pragma unroll
-    for (int x = 0; x < N / 16; ++x) {
-      const int rr = row0 + 16 * x;
-      *reinterpret_cast<float4*>(&sm.st[rr][4 * kq]) = g ? __ldg(reinterpret_cast<const float4*>(g + (long long)rr * N + 4 * kq)) : zero;
-    }
-  };
-  get_state(Sg);
   for (int e = tid; e < 4 * GT * GT; e += NTHR) (&sm.sc[0][0][0])[e] = 0.f;
   __syncthreads();
 
@@ -700,10 +708,11 @@ r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, c
     }
   };
   scaled(false);
+  cp_async_wait();
   __syncthreads();
 
   // rows: dst[v][j] = sum_k st[v][k] xs[j][k]; a 4 x 4 tile per thread and a quarter of the channels
-  auto row_product = [&](float (*dst)[36], int j0) {
+  auto row_product = [&](const float (*st)[N + 4], float (*dst)[36], int j0) {
     const int s = (tid >> 2) & 3, tj = (tid & 1) | ((tid >> 3) & 2), tv = ((tid >> 1) & 1) | (tid >> 5 << 1);
     f32x2 acc[16];
 #pragma unroll
@@ -713,7 +722,7 @@ r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, c
       const int c = 4 * (s + 4 * x);
       Quad A[4], B[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) { A[e] = lds4(&sm.st[4 * tv + e][c]); B[e] = lds4(&sm.xs[4 * tj + e][c]); }
+      for (int e = 0; e < 4; ++e) { A[e] = lds4(&st[4 * tv + e][c]); B[e] = lds4(&sm.xs[4 * tj + e][c]); }
 #pragma unroll
       for (int e = 0; e < 16; ++e) acc[e] = fma2(A[e >> 2].hi, B[e & 3].hi, fma2(A[e >> 2].lo, B[e & 3].lo, acc[e]));
     }
@@ -744,16 +753,16 @@ r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, c
       r[j] = lo.x; r[4 + j] = lo.y; r[8 + j] = hi.x; r[12 + j] = hi.y;      // r[4 k + j]
     }
   };
-  auto state_cols = [&](float (*dst)[36], const float (*B)[36]) {
+  auto state_cols = [&](const float (*st)[N + 4], float (*dst)[36], const float (*B)[36]) {
     const int s = (tid >> 2) & 1, tj = (tid & 1) | ((tid >> 2) & 6), tk = ((tid >> 1) & 1) | (tid >> 5 << 1);
     float r[16];
-    col_product(&sm.st[0][0], N + 4, B, tk, tj, s, 2, 4, r);
+    col_product(&st[0][0], N + 4, B, tk, tj, s, 2, 4, r);
     reduce_scatter<16, 4, 4>(r, lane);      // lane s keeps channels 2 s, 2 s + 1
     *reinterpret_cast<float4*>(&dst[4 * tk + 2 * s][4 * tj]) = make_float4(r[0], r[1], r[2], r[3]);
     *reinterpret_cast<float4*>(&dst[4 * tk + 2 * s + 1][4 * tj]) = make_float4(r[4], r[5], r[6], r[7]);
   };
 
-  row_product(sm.cat1, 0);
+  row_product(S, sm.cat1, 0);
   __syncthreads();
   if (tid < N) {      // sa_j, one value row per thread
     float sa[GT], vv[GT];
@@ -783,16 +792,21 @@ r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, c
 #pragma unroll
     for (int j = 0; j < GT; j += 4) *reinterpret_cast<float4*>(&sm.cat1[tid][j]) = make_float4(sa[j], sa[j + 1], sa[j + 2], sa[j + 3]);
   }
-  // ---- G replaces S; sum_v G S on the way (16 partial rows in outS)
+  // ---- sum_v G S (16 partial rows in outS); at N = 128 G replaces S on the way
   {
     float4 z = zero;
 #pragma unroll
     for (int x = 0; x < N / 16; ++x) {
       const int rr = row0 + 16 * x;
-      float4* p = reinterpret_cast<float4*>(&sm.st[rr][4 * kq]);
-      const float4 G = Gg ? __ldg(reinterpret_cast<const float4*>(Gg + (long long)rr * N + 4 * kq)) : zero, S = *p;
-      z.x += G.x * S.x; z.y += G.y * S.y; z.z += G.z * S.z; z.w += G.w * S.w;
-      *p = G;
+      const float4 s4 = *reinterpret_cast<const float4*>(&S[rr][4 * kq]);
+      float4 g4;
+      if constexpr (BOTH_STATES<N>) {
+        g4 = *reinterpret_cast<const float4*>(&G[rr][4 * kq]);
+      } else {
+        g4 = Gg ? __ldg(reinterpret_cast<const float4*>(Gg + (long long)rr * N + 4 * kq)) : zero;
+        *reinterpret_cast<float4*>(&G[rr][4 * kq]) = g4;
+      }
+      z.x += g4.x * s4.x; z.y += g4.y * s4.y; z.z += g4.z * s4.z; z.w += g4.w * s4.w;
     }
     const float ez[4] = {z.x, z.y, z.z, z.w};
     put_column(ez, [&](int x) { return &sm.outS[4 * kq + x][row0]; });
@@ -807,10 +821,13 @@ r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, c
       zsum += (f.x + f.y) + (f.z + f.w);
     }
   }
-  row_product(sm.cat2, GT);
-  state_cols(sm.outG, sm.cat1);
+  row_product(G, sm.cat2, GT);
+  state_cols(G, sm.outG, sm.cat1);
   __syncthreads();
-  get_state(Sg);
+  if constexpr (!BOTH_STATES<N>) {
+    request_state(S, Sg);
+    cp_async_commit();
+  }
   if (tid < N) {      // dsa_j, from the last token to the first
     float ds[GT], dov[GT];
 #pragma unroll
@@ -835,8 +852,9 @@ r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, c
 #pragma unroll
     for (int j = 0; j < GT; j += 4) *reinterpret_cast<float4*>(&sm.cat2[tid][GT + j]) = make_float4(ds[j], ds[j + 1], ds[j + 2], ds[j + 3]);
   }
+  if constexpr (!BOTH_STATES<N>) cp_async_wait();
   __syncthreads();
-  state_cols(sm.outS, sm.cat2);
+  state_cols(S, sm.outS, sm.cat2);
   {
     constexpr int NS = NTHR / 64;      // 4 or 8 lanes per tile
     const int s = (tid >> 2) % NS, high = tid / (4 * NS);      // tj bit 0, ti bit 0, s, then the other two bits of ti and of tj
@@ -938,15 +956,18 @@ r7_grad_kernel(Vecs<T> in, const T* __restrict__ v, const T* __restrict__ d_o, c
       if (j < nt) dst[base + (long long)j * lay.st + c] = from_f32<T>(x[j]);
     }
   }
+  // role 0 has the w rows fetched before it waits (one after the other they took a fifth of the kernel)
+  float ew[GT];
+  if (role == 0) {
+#pragma unroll
+    for (int j = 0; j < GT; ++j) ew[j] = j < nt ? to_f32(__ldg(in.p[VW] + base + (long long)j * lay.st + c)) : 0.f;
+  }
   __syncthreads();
   if (role == 0) {
 #pragma unroll
     for (int j = 0; j < GT; ++j) {
-      if (j < nt) {
-        const long long off = base + (long long)j * lay.st + c;
-        const float s = dd[j] + sm.outS[c][GT + j] + sm.outG[c][GT + j];
-        dw[off] = from_f32<T>(s * d[j] * -expf(to_f32(in.p[VW][off])));
-      }
+      const float s = dd[j] + sm.outS[c][GT + j] + sm.outG[c][GT + j];
+      if (j < nt) dw[base + (long long)j * lay.st + c] = from_f32<T>(s * d[j] * -expf(ew[j]));
     }
   }
 }
