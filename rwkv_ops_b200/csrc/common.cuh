@@ -181,9 +181,9 @@ int need_aligned_smem(const DeviceFacts& f) {
   return n == 1 ? RWKVB200_OK : RWKVB200_E_UNSUPPORTED;
 }
 
-// Every kernel of the library is launched so that its blocks may come onto the SMs while the kernel before it on the stream runs
+// The kernels of the library (but where a launch says why not) are launched so that their blocks may come onto the SMs while the kernel before runs
 // out: what they do before earlier_kernels_done() (barriers, TMEM) overlaps with its last blocks, and so does the launch
-// itself.  No kernel touches global memory before that call, every thread makes it, and it returns when all earlier
+// itself.  No kernel touches global memory before that call but to prefetch into L2, every thread makes it, and it returns when all earlier
 // kernels have completed.  later_kernels_may_start() lets the next kernel's blocks come once all blocks of this one have
 // called it; a kernel that allocates TMEM calls it after the allocation, so that blocks of the next one, which wait for
 // this one, never hold TMEM that a block of this one still needs.

@@ -987,12 +987,17 @@ int launch_rwkv7_chunked_bwd(const void* r, const void* w, const void* k, const 
     const int n_ch = B * H * NT;
     const int sms = dev.sms;
     const int grid = n_ch < 2 * sms ? n_ch : 2 * sms;     // persistent: two CTAs per SM
+    // Blocks that come while the reverse scan runs out save the 2 us between two kernels, but where the CTAs walk over
+    // many chunk-heads the kernel is slower for it (which the launch alone does; why was not isolated).  Forward and backward, us,
+    // with and without, 32 heads: B 1, T 4096 318 and 316; B 2 444 and 441; B 4, T 1024, 48 heads 310 and 303; B 16, T 8192, 64 heads
+    // 11760 and 11665; 8 packed sequences of up to 4096 tokens 952 and 941.
+    const int early = n_ch <= grid ? 1 : 0;
 #define R7C_LAUNCH_FINAL(P, F)                                                                                    \
     do {                                                                                                          \
       if (int rc = need_aligned_smem<r7c_bwd_final_kernel<P, F>>(dev)) return rc;                                 \
       if (allow_smem<r7c_bwd_final_kernel<P, F>>(dev, smem)) \
         return RWKVB200_E_CUDA;                                                                                   \
-      if (int rc = launch(r7c_bwd_final_kernel<P, F>, grid, 256, smem, st, 1, (const bf16*)w, tmap_w, tmap_do, tmap_v, ws.tiles, (int)ALL_TILES, \
+      if (int rc = launch(r7c_bwd_final_kernel<P, F>, grid, 256, smem, st, early, (const bf16*)w, tmap_w, tmap_do, tmap_v, ws.tiles, (int)ALL_TILES, \
           tmap_out[0], tmap_out[1], tmap_out[2], tmap_out[3], tmap_out[4], tmap_out[5], (bf16*)dr, (bf16*)dw,     \
           (bf16*)dk, (bf16*)dv, (bf16*)da, (bf16*)db, sv, WalkDims(H, NT, B, grid), lay, status, debug_stamp_buffer())) return rc; \
     } while (0)
