@@ -19,12 +19,13 @@
 // the token-by-token form would keep, and all arithmetic is float32.
 //
 // The gradient G of the state runs backward in time through the same equations with the roles exchanged
-// (sa -> dsa, o -> dv, v -> do; a <-> b, r <-> k, every A transposed): one kernel serves both directions.  The other
-// five gradients do not feed the chain.  A third kernel computes them for every 16 tokens at once, from the states
-// and state gradients that the two sweeps leave at those boundaries (as much memory as a state every 8 tokens).
+// (sa -> dsa, o -> dv, v -> do; a <-> b, r <-> k, every A transposed): the same code serves both directions.  The other
+// five gradients do not feed the chain.  A kernel of their own computes them for every 16 tokens at once, from the states
+// and state gradients that the two sweeps leave at those boundaries (as much memory as a state every 8 tokens).  The forward
+// of a training call leaves its states for the backward; a backward without them sweeps forward first.
 //
-// B 2, T 1024, 16 heads, float32, against the token-by-token kernels: forward 500 -> 124 us, backward with its forward sweep
-// 1740 -> 415 us.  Head size 128 at T 512: 2800 -> 912 us for both.
+// B 2, T 1024, 16 heads, float32, in kernels: token by token forward 500 us, backward 1740; 106 (20 of preparation) and 235 (24 of
+// preparation, 84 sweep, 127 gradients) here.
 #include <type_traits>
 
 #include "common.cuh"
@@ -580,7 +581,9 @@ r7_sweep_kernel(const Stage<N, N>* __restrict__ stages, const float* s_in, int n
 // dsa; columns: S^T [do dsa], G^T [sa v]), after which every channel is on its own: it steps S_j^T do_i, S_j^T dsa_i,
 // G_j^T v_i and G_j^T sa_i through the 16 tokens with the scalars sa.do, v.do, sa.dsa, v.dsa (four threads to a
 // channel).  dd_j is summed from the same quantities, positive decay factors throughout, so no term cancels that does not in
-// the token-by-token form.  Bound by shared-memory reads (two 16-byte reads per 16 products).
+// the token-by-token form.  At N = 64 a CTA is 31 k warp instructions (1.9 per cycle and SM, of four) and 9.8 k shared-memory
+// wavefronts of 16.8 k cycles, two CTAs to an SM, whose barriers cost as much as either.  B 2, T 1024, 16 heads, float32: 163 us when
+// the lanes that share an operand lay apart, 134 before everything was requested at once and both states kept, 127 now.
 template <int N> constexpr bool BOTH_STATES = N == 64;      // both fit; at N = 128 G replaces S and S is fetched again
 template <int N>
 struct GradSmem {

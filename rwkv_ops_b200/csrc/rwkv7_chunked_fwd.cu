@@ -40,7 +40,7 @@ struct IntraSmem {
 // MMA 1, issue MMA 2 and drain it.
 // What bounds it: 17 tiles per chunk-head through memory (348 us at B 8, T 4096, 32 heads) if two CTAs per SM can
 // overlap their chains of phases well enough: 503 us before the inverse went to two warps and the raw tiles were requested
-// early, 475 us now.  The backward takes the difference of large sums over the tiles made here: a change of their arithmetic in
+// early, 467 us now.  The backward takes the difference of large sums over the tiles made here: a change of their arithmetic in
 // the last bit shows in dw (a 32 x 32 substitution and reciprocals for e^{gref-gi} gave 412 us and were taken back).
 template <bool PACKED, bool FUSED>
 __global__ void __launch_bounds__(256, 2)
