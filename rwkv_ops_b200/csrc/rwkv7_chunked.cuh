@@ -86,9 +86,10 @@ struct ChunkPos { int ch, bi, hi, c; };
 // (a kernel parameter, made on the host: computed in the kernels it would take registers that they do not have)
 struct WalkDims {
   int H, NT, B, n_ch;
-  int dh, db, dc;      // dense: the grid size as heads + H * (sequences + B * chunks)
-  WalkDims(int H_, int NT_, int B_, int grid)
-      : H(H_), NT(NT_), B(B_), n_ch(H_ * NT_ * B_), dh(grid % H_), db(grid / H_ % B_), dc(grid / H_ / B_) {}
+  int dh, db, dc;      // dense: the grid size as heads + H * (sequences + B * chunks), or, by unit, as chunks + NT * (heads + H * sequences)
+  WalkDims(int H_, int NT_, int B_, int grid, bool by_unit = false)
+      : H(H_), NT(NT_), B(B_), n_ch(H_ * NT_ * B_), dh(by_unit ? grid / NT_ % H_ : grid % H_),
+        db(by_unit ? grid / NT_ / H_ : grid / H_ % B_), dc(by_unit ? grid % NT_ : grid / H_ / B_) {}
 };
 template <bool PACKED, bool DOWN>
 struct ChunkWalk {
@@ -132,6 +133,24 @@ struct ChunkWalk {
       if (p.bi >= d.B) { p.bi -= d.B; ++level; }
       place(p, level);
     }
+    return p;
+  }
+};
+
+// Dense: the same list unit by unit, in the order of the workspace (WalkDims by unit).
+struct UnitWalk {
+  const WalkDims& d;
+  __device__ __forceinline__ ChunkPos first() const {
+    const int i = blockIdx.x;
+    return ChunkPos{i, i / d.NT / d.H, i / d.NT % d.H, i % d.NT};
+  }
+  __device__ __forceinline__ ChunkPos after(ChunkPos p) const {
+    p.ch += gridDim.x;
+    p.c += d.dc;
+    p.hi += d.dh;
+    p.bi += d.db;
+    if (p.c >= d.NT) { p.c -= d.NT; ++p.hi; }
+    if (p.hi >= d.H) { p.hi -= d.H; ++p.bi; }
     return p;
   }
 };
