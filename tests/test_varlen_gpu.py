@@ -305,3 +305,28 @@ def test_wkv6_state_map_and_offsets_in_every_accepted_form():
                 call(wrong, offsets)
     y2, s2 = call([0, 2], torch.tensor([cu]))
     assert torch.equal(y2, y) and torch.equal(s2, s)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H", [1, 4])
+def test_wkv6_packed_lengths_of_zero_on_the_device(H, dtype):
+    """The registered operator takes lengths that lie on the device and that it cannot check: an empty sequence hands its state
+    on, whether a unit is one item (100 units), or stretches on persistent CTAs (400), and the others come out as without it."""
+    from rwkv_ops_b200 import _lib, _ops
+    lens = [0] + [n for i in range(33) for n in (0, (520, 40, 129, 7, 300)[i % 5], 64)]
+    full = [n for n in lens if n]
+    T, max_len = sum(lens), max(lens)
+    d = wkv6_inputs(1, T, H, dtype=dtype, seed=12, device="cuda", n_state=1)
+    x = [d[n] for n in "rkvwu"]
+    s0 = 0.1 * torch.randn(len(lens), H, 64, 64, device="cuda").to(dtype)
+    at = torch.tensor(lens).cumsum(0) - torch.tensor(lens)
+    y, s = _ops.load().wkv6_varlen(*x, at.int().cuda(), torch.tensor(lens, dtype=torch.int32, device="cuda"), max_len, s0, None)
+    some = torch.tensor([i for i, n in enumerate(lens) if n])
+    empty = torch.tensor([i for i, n in enumerate(lens) if not n])
+    assert torch.equal(s[empty], s0[empty].to(s.dtype))
+    cu = [0, *torch.tensor(full).cumsum(0).tolist()]
+    y2, s2 = ro.wkv6_varlen(*x, cu, init_state=s0[some].contiguous())
+    # (other batches of units run as other items: the same sums in another order)
+    tol = 1e-4 if dtype == torch.float32 else 5e-3
+    assert rel_l2(y, y2) < tol and rel_l2(s[some], s2) < tol
+    assert _lib.load().rwkvb200_device_status(1) == 0
