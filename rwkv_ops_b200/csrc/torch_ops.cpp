@@ -196,10 +196,13 @@ bool keep_fits(const SymDims& d, int algo, const Tensor& r) {
          keep_limit_bytes(r.device().index());
 }
 
-// The same for the states of the float32 recurrence over blocks (rwkvb200_rwkv7_states_bytes): a length stays a symbol.
+// The same for the states of the float32 recurrence over blocks (rwkvb200_rwkv7_states_bytes; none up to 16 tokens).  Sizes
+// that are symbols stay symbols, without a guard: a traced program serves every length, and keeps the states where they fit
+// at every length that it is declared for.
 bool states_fit(const SymDims& d, const Tensor& r) {
-  return d.T > 16 && d.B * d.H * ((d.T + 15) / 16 - 1) * d.K * d.K * 4 <=
-                         (int64_t)std::min<size_t>(keep_limit_bytes(r.device().index()), std::numeric_limits<int64_t>::max());
+  const auto limit = (int64_t)std::min<size_t>(keep_limit_bytes(r.device().index()), std::numeric_limits<int64_t>::max());
+  return !TORCH_STATICALLY_KNOWN_TRUE(d.T.sym_le(16)) &&
+         TORCH_STATICALLY_KNOWN_TRUE((d.B * d.H * ((d.T + 15) / 16 - 1) * d.K * d.K * 4).sym_le(limit));
 }
 // whether rwkv7_fwd / _bwd take the chunked path, whose kept tensor holds tiles; elsewhere it holds states
 bool chunked_rwkv7(const Dims& d, int code, int64_t algo) {
@@ -212,7 +215,7 @@ Three rwkv7_fwd(const Tensor& r, const Tensor& w, const Tensor& k, const Tensor&
   const Dims d = dims_of(r, head_first);
   const int code = dtype_code(r.scalar_type()), flags = (int)algo | (keep ? RWKVB200_ALGO_KEEP : 0);
   Tensor o = fresh_like(r), ht = fresh({d.B, d.H, d.K, d.K}, at::kFloat, r), ws;
-  if (d.T == 1 && !keep) {
+  if (d.T == 1 && !(keep && chunked_rwkv7(d, code, algo))) {
     check(rwkvb200_rwkv7_step(ptr(r), ptr(w), ptr(k), ptr(v), ptr(a), ptr(b), fptr(h0), n_state_of(h0), fptr(ht), ptr(o),
                               d.B, d.H, d.K, code, stream_of(r)), "rwkv7_step");
   } else if (keep && !chunked_rwkv7(d, code, algo)) {
@@ -229,7 +232,7 @@ Three rwkv7_fwd(const Tensor& r, const Tensor& w, const Tensor& k, const Tensor&
     check(rwkvb200_rwkv7_fwd(ptr(r), ptr(w), ptr(k), ptr(v), ptr(a), ptr(b), fptr(h0), n_state_of(h0), ptr(o), fptr(ht),
                              ptr(ws), nws, d.B, d.T, d.H, d.K, code, head_first, flags, stream_of(r)), "rwkv7_fwd");
   }
-  return {o, ht, keep ? ws : bytes(0, r)};
+  return {o, ht, keep && ws.defined() ? ws : bytes(0, r)};
 }
 
 // `kept` (may be empty): what a forward with keep left; the tiles of the chunked path also serve as scratch, but what the

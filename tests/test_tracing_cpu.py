@@ -5,6 +5,7 @@ import torch
 from torch._dynamo.source import ConstantSource
 from torch._subclasses.fake_tensor import FakeTensorMode
 from torch.fx.experimental.symbolic_shapes import DimDynamic, ShapeEnv
+from torch.utils._python_dispatch import TorchDispatchMode
 
 import rwkv_ops_b200 as ro
 from rwkv_ops_b200 import _ops
@@ -75,17 +76,54 @@ def test_float32_rwkv7_training_keeps_symbolic_sizes():
         assert o.requires_grad and all(_symbolic(o, (0, 1))) and all(_symbolic(s, (0,)))
 
 
-def test_export_with_a_dynamic_length():
-    class Layer(torch.nn.Module):
-        def forward(self, *x):
-            o, s = ro.generalized_delta_rule(*x)
-            return 2 * o, s
+class Layer(torch.nn.Module):
+    def forward(self, *x):
+        o, s = ro.generalized_delta_rule(*x)
+        return 2 * o, s
 
+
+def test_export_with_a_dynamic_length():
     length = torch.export.Dim("length", min=2, max=8192)
     with FakeTensorMode(shape_env=ShapeEnv()), torch.no_grad():
         x = tuple(torch.empty(2, 100, 3, 64, dtype=torch.bfloat16, device="cuda") for _ in range(6))
         program = torch.export.export(Layer(), x, dynamic_shapes=(tuple({1: length} for _ in x),))
     assert any("rwkv_ops_b200" in str(n.target) for n in program.graph.nodes)
+
+
+@pytest.mark.parametrize("longest", [8192, None])
+@pytest.mark.parametrize("traced", [8, 16, 17, 100])
+@pytest.mark.parametrize("dtype,K", [(torch.float32, 64), (torch.float32, 128), (torch.float16, 64), (torch.bfloat16, 128)])
+def test_export_of_the_float32_recurrence_with_gradients(dtype, K, traced, longest):
+    """Whatever length it is traced at, the program serves all that were declared, on either side of 16 tokens, from which on the
+    forward leaves states for its backward, and without a bound from the memory these may take."""
+    length = torch.export.Dim("length", min=2, max=longest)
+    with FakeTensorMode(shape_env=ShapeEnv()):
+        x = tuple(torch.empty(2, traced, 3, K, dtype=dtype, device="cuda", requires_grad=True) for _ in range(6))
+        program = torch.export.export(Layer(), x, dynamic_shapes=(tuple({1: length} for _ in x),))
+    (bounds,) = program.range_constraints.values()
+    assert bounds.lower == 2 and (longest is None or bounds.upper == longest)
+
+
+class _Calls(TorchDispatchMode):
+    def __init__(self):
+        super().__init__()
+        self.keep = []
+
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        if func is torch.ops.rwkv_ops_b200.rwkv7_fwd.default:
+            self.keep.append(args[-1])
+        return func(*args, **(kwargs or {}))
+
+
+@pytest.mark.parametrize("T,limit,keep", [(8, None, False), (16, None, False), (17, None, True), (100, None, True), (100, "0", False)])
+def test_states_are_kept_by_length_and_limit(T, limit, keep, monkeypatch):
+    if limit is not None:
+        monkeypatch.setenv("RWKV_OPS_B200_KEEP_LIMIT_MB", limit)
+    with FakeTensorMode():
+        x = [torch.empty(2, T, 3, 64, device="cuda", requires_grad=True) for _ in range(6)]
+        with _Calls() as calls:
+            ro.generalized_delta_rule(*x)
+    assert calls.keep == [keep]
 
 
 def test_wrong_arguments_still_raise():
