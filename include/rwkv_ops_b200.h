@@ -169,8 +169,8 @@ int rwkvb200_rwkv7_decode_step(const void* r, const void* w, const void* k, cons
                                const void* a, const void* b, void* state, int state_dtype, void* o,
                                int B, int H, int head_size, int dtype, void* stream);
 
-/* The workspace is needed on the chunked path.  The float32 recurrence takes what this asks for to run faster, and takes less,
- * or NULL, too. */
+/* The workspace is needed on the chunked path.  The float32 recurrence takes what this asks for (256 MB at most, nothing where it
+ * would not be used) to run faster, and takes less, or NULL, too. */
 size_t rwkvb200_rwkv7_fwd_workspace_bytes(int B, int T, int H, int head_size, int dtype, int algo);
 
 int rwkvb200_rwkv7_fwd(const void* r, const void* w, const void* k, const void* v,

@@ -474,15 +474,15 @@ constexpr int PREPARE_THREADS = 256;
 
 template <typename T, int N, bool BWD>
 __global__ void __launch_bounds__(PREPARE_THREADS)
-r7_prepare_kernel(Vecs<T> in, const T* __restrict__ v, Stage<N, N>* __restrict__ stages, int Tn, int H, int idx0, int nb, int n_items,
-                  TokLayout lay) {
+r7_prepare_kernel(Vecs<T> in, const T* __restrict__ v, Stage<N, N>* __restrict__ stages, int Tn, int H, int unit0, int idx0, int nb,
+                  int n_items, TokLayout lay) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int g = threadIdx.x / N, q = threadIdx.x % N, item = blockIdx.x * (PREPARE_THREADS / N) + g;
   PrepareSmem<T, N>& sm = reinterpret_cast<PrepareSmem<T, N>*>(smem_raw)[g];
   earlier_kernels_done();
   later_kernels_may_start();
   if (item >= n_items) return;      // the whole group
-  const int unit = item / nb, idx = idx0 + item % nb, NB = (Tn + W - 1) / W;
+  const int unit = unit0 + item / nb, idx = idx0 + item % nb, NB = (Tn + W - 1) / W;
   const int t0 = (BWD ? NB - 1 - idx : idx) * W;
   const long long base = unit / H * lay.sb + unit % H * lay.sh;
   constexpr int EPC = 16 / sizeof(T), CPR = N / EPC;
@@ -524,15 +524,18 @@ struct SweepSmem {
 // With at most one CTA to an SM, slots enough that no two CTAs fit one: they may come while the preparing kernel runs out, and
 // would otherwise share the first SMs that are free (B 2, T 1024, 16 heads: 177 -> 230 us).
 template <int N> constexpr int FEW_CTAS_SLOTS = 116 * 1024 / sizeof(Stage<N, RV>) + 1;
-// Blocks idx0 .. idx0 + nb - 1 in processing order; a warp beside the state warps fetches their stages.
+// What one launch takes through: units from unit0 on and their blocks idx0 .. idx0 + nb - 1 in processing order; the states before
+// and after these (one per unit of the launch), nullptr where they are the sequence's own.
+struct SweepPart { int unit0, idx0, nb; const float* from; float* to; };
+// A warp beside the state warps fetches the stages.
 template <typename T, int N, bool BWD, int SLOTS, int ROWS, int PER_SM>
 __global__ void __launch_bounds__(state_threads<N, ROWS>() + 32, PER_SM)
 r7_sweep_kernel(const Stage<N, N>* __restrict__ stages, const float* s_in, int n_state, T* __restrict__ out, float* s_out,
-                float* __restrict__ ckpt, int Tn, int H, int idx0, int nb, TokLayout lay, int* status) {
+                float* __restrict__ ckpt, int Tn, int H, SweepPart part, TokLayout lay, int* status) {
   constexpr int NCONS = state_threads<N, ROWS>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   auto& sm = *reinterpret_cast<SweepSmem<N, SLOTS>*>(smem_raw);
-  const int unit = blockIdx.x, ys = blockIdx.y, tid = threadIdx.x;
+  const int unit = part.unit0 + blockIdx.x, ys = blockIdx.y, tid = threadIdx.x, nb = part.nb;
   const int bi = unit / H, hi = unit % H;
   if (tid == 0) {
     for (int i = 0; i < SLOTS; ++i) { tc::mbar_init(&sm.full[i], 1); tc::mbar_init(&sm.empty[i], NCONS / 32); }
@@ -545,9 +548,10 @@ r7_sweep_kernel(const Stage<N, N>* __restrict__ stages, const float* s_in, int n
     const int NB = (Tn + W - 1) / W, NG = (Tn + GT - 1) / GT;
     const long long base = bi * lay.sb + hi * lay.sh, rows = (long long)ys * RV * N;
     StateRows<N, ROWS> S(tid);
-    S.get(s_in && n_state > 0 ? s_in + (long long)(n_state == 1 ? hi : unit) * N * N + rows : nullptr);
+    S.get(part.from ? part.from + (long long)blockIdx.x * N * N + rows
+                    : s_in && n_state > 0 ? s_in + (long long)(n_state == 1 ? hi : unit) * N * N + rows : nullptr);
     for (int i = 0, slot = 0, phase = 0; i < nb; ++i) {
-      const int n = BWD ? NB - 1 - idx0 - i : idx0 + i;
+      const int n = BWD ? NB - 1 - part.idx0 - i : part.idx0 + i;
       if (ckpt)
         if (float* p = state_slot<N, BWD>(ckpt, unit, NG, n)) S.put(p + rows);
       if (!tc::mbar_wait(&sm.full[slot], phase, status, 501)) break;
@@ -559,9 +563,10 @@ r7_sweep_kernel(const Stage<N, N>* __restrict__ stages, const float* s_in, int n
       if (out && t < Tn) S.put_out(out + base + (long long)t * lay.st + ys * RV, oo);
       if (++slot == SLOTS) { slot = 0; phase ^= 1; }
     }
-    if (s_out) S.put(s_out + (long long)unit * N * N + rows);
+    if (part.to) S.put(part.to + (long long)blockIdx.x * N * N + rows);
+    else if (s_out) S.put(s_out + (long long)unit * N * N + rows);
   } else if (tc::elect_one()) {
-    const Stage<N, N>* src = stages + (long long)unit * nb;
+    const Stage<N, N>* src = stages + (long long)blockIdx.x * nb;
     for (int i = 0, slot = 0, phase = 1; i < nb; ++i, ++src) {
       if (i >= SLOTS && !tc::mbar_wait(&sm.empty[slot], phase, status, 502)) break;
       tc::mbar_expect_tx(&sm.full[slot], COMMON_BYTES<N> + SLICE_BYTES);
@@ -988,35 +993,49 @@ int launch_inline(const DeviceFacts& dev, const Vecs<T>& in, const void* v, cons
 
 template <typename T, int N, bool BWD, int SLOTS, int ROWS, int PER_SM>
 int launch_sweep(const DeviceFacts& dev, const Stage<N, N>* stages, const float* s_in, int n_state, void* out, float* s_out, float* ckpt,
-                 int B, int Tn, int H, int idx0, int nb, const TokLayout& lay, cudaStream_t st) {
+                 int n_units, int Tn, int H, const SweepPart& part, const TokLayout& lay, cudaStream_t st) {
   constexpr int bytes = (int)sizeof(SweepSmem<N, SLOTS>);
   if (allow_smem<r7_sweep_kernel<T, N, BWD, SLOTS, ROWS, PER_SM>>(dev, bytes)) return RWKVB200_E_CUDA;
   ProfScope prof(BWD ? "r7_sweep_bwd_kernel" : "r7_sweep_fwd_kernel", st);
-  return launch(r7_sweep_kernel<T, N, BWD, SLOTS, ROWS, PER_SM>, dim3(B * H, N / RV), state_threads<N, ROWS>() + 32, bytes, st, PER_SM == 1 ? 1 : 0, stages, s_in,
-                n_state, (T*)out, s_out, ckpt, Tn, H, idx0, nb, lay, dev.status);
+  return launch(r7_sweep_kernel<T, N, BWD, SLOTS, ROWS, PER_SM>, dim3(n_units, N / RV), state_threads<N, ROWS>() + 32, bytes, st,
+                PER_SM == 1 ? 1 : 0, stages, s_in, n_state, (T*)out, s_out, ckpt, Tn, H, part, lay, dev.status);
 }
 
-// Scratch of a sweep: stages of as many blocks of every unit as fit STAGES_BYTES (at least 8), and the units' states between one
-// such stretch and the next.  (More than L2 holds costs little: 1.4 KB per token and head, where the inputs take 1.5.)
-constexpr size_t STAGES_BYTES = (size_t)256 << 20;
 // From how many blocks per unit on they are prepared by a kernel of their own (forward, us; inside the sweep against apart):
 // with at most one CTA per SM the sweep has to be long enough for the other kernel (12 units, T 128 15.8 and 15.0, T 300 32.7 and
 // 29.3, T 1024 101 and 83; 37 units 16.0 and 18.5, 33.0 and 31.6, 101 and 96); at head size 64 two CTAs per SM inside keep up
 // (60 units, T 300 57 and 60); beyond that it pays from the start (128 units, T 32 15.6 and 14.7, T 1024 364 and 227; head size
 // 128, 64 units, T 1024 711 and 375).
 constexpr int STAGED_BLOCKS = 4;
-template <int N> int staged_from(int ctas, int sms) {
-  if (ctas <= sms) return N == 64 ? 48 : 12;
-  return N == 64 && ctas <= 2 * sms ? 1 << 30 : STAGED_BLOCKS;
+template <int N> bool prepared_apart(long long ctas, int NB, int sms) {
+  if (ctas <= sms) return NB >= (N == 64 ? 48 : 12);
+  return (N == 128 || ctas > 2 * sms) && NB >= STAGED_BLOCKS;
 }
-template <int N> int stretch_blocks(long long units, int NB) {
-  const long long fit = (long long)(STAGES_BYTES / sizeof(Stage<N, N>)) / units;
-  return (int)(fit < 8 ? (NB < 8 ? NB : 8) : fit < NB ? fit : NB);
+// Scratch of a sweep whose blocks are prepared apart, STAGES_BYTES at most: stages of `blocks` blocks (a stretch) of `units` units
+// (a pass), and the units' states between one stretch and the next.  As many blocks as fit for all units; with very many units 8,
+// whose 88 KB of stages are worth the 32 KB of a state left and fetched, for as many units as fit, at least 1100, which fill the
+// device.  (More than L2 holds costs little: 1.4 KB per token and head, where the inputs take 1.5.)
+constexpr size_t STAGES_BYTES = (size_t)256 << 20;
+constexpr int STRETCH_BLOCKS = 8;
+struct Staging { int blocks, units; };      // 0: the blocks are prepared inside the sweep, without scratch
+template <int N> size_t unit_bytes(int blocks, int NB) {
+  return blocks * sizeof(Stage<N, N>) + (blocks < NB ? N * N * sizeof(float) : 0);
+}
+template <int N> Staging staging(long long units, int Tn, int sms) {
+  const int NB = (Tn + W - 1) / W;
+  if (!prepared_apart<N>(units * (N / RV), NB, sms)) return Staging{0, 0};
+  int blocks = NB;
+  if (units * unit_bytes<N>(NB, NB) > STAGES_BYTES) {
+    const long long share = STAGES_BYTES / units, fit = (share - (long long)(N * N * sizeof(float))) / (long long)sizeof(Stage<N, N>);
+    blocks = (int)(fit > STRETCH_BLOCKS ? fit : NB < STRETCH_BLOCKS ? NB : STRETCH_BLOCKS);
+  }
+  const long long pass = STAGES_BYTES / unit_bytes<N>(blocks, NB);
+  return Staging{blocks, (int)(pass < units ? pass : units)};
 }
 template <int N> size_t scratch_bytes(long long units, int Tn) {
-  const int NB = (Tn + W - 1) / W;
-  if (NB < STAGED_BLOCKS) return 0;
-  return (size_t)units * (stretch_blocks<N>(units, NB) * sizeof(Stage<N, N>) + N * N * sizeof(float));
+  DeviceFacts dev;
+  const Staging s = staging<N>(units, Tn, device_facts(&dev) ? 148 : dev.sms);      // (asked where there is no device)
+  return s.units * unit_bytes<N>(s.blocks, (Tn + W - 1) / W);
 }
 
 template <typename T, int N, bool BWD>
@@ -1026,29 +1045,30 @@ int sweep(const Vecs<T>& in, const void* v, const float* s_in, int n_state, void
   if (int e = device_facts(&dev)) return e;
   const int units = B * H, NB = (Tn + W - 1) / W;
   const bool many = units * (N / RV) > dev.sms;
-  if (!scratch || NB < staged_from<N>(units * (N / RV), dev.sms))
+  const Staging s = staging<N>(units, Tn, dev.sms);
+  if (!scratch || !s.blocks)
     return many ? launch_inline<T, N, BWD, MANY_CTAS<T, N>, MANY_CTAS_ROWS>(dev, in, v, s_in, n_state, out, s_out, ckpt, B, Tn, H, lay, st)
                 : launch_inline<T, N, BWD, FEW_CTAS<N>, FEW_CTAS_ROWS<N>>(dev, in, v, s_in, n_state, out, s_out, ckpt, B, Tn, H, lay, st);
-  const int stretch = stretch_blocks<N>(units, NB);
   auto* stages = static_cast<Stage<N, N>*>(scratch);
-  float* between = reinterpret_cast<float*>(stages + (size_t)units * stretch);
+  float* between = reinterpret_cast<float*>(stages + (size_t)s.units * s.blocks);
   constexpr int per_cta = PREPARE_THREADS / N, bytes = per_cta * (int)sizeof(PrepareSmem<T, N>);
   if (allow_smem<r7_prepare_kernel<T, N, BWD>>(dev, bytes)) return RWKVB200_E_CUDA;
-  for (int idx0 = 0; idx0 < NB; idx0 += stretch) {
-    const int nb = NB - idx0 < stretch ? NB - idx0 : stretch, n_items = units * nb;
-    {
-      ProfScope prof("r7_prepare_kernel", st);
-      if (int e = launch(r7_prepare_kernel<T, N, BWD>, (n_items + per_cta - 1) / per_cta, PREPARE_THREADS, bytes, st, 1, in, (const T*)v,
-                         stages, Tn, H, idx0, nb, n_items, lay)) return e;
+  for (int unit0 = 0; unit0 < units; unit0 += s.units)
+    for (int idx0 = 0; idx0 < NB; idx0 += s.blocks) {
+      const int n_units = units - unit0 < s.units ? units - unit0 : s.units;
+      const int nb = NB - idx0 < s.blocks ? NB - idx0 : s.blocks, n_items = n_units * nb;
+      {
+        ProfScope prof("r7_prepare_kernel", st);
+        if (int e = launch(r7_prepare_kernel<T, N, BWD>, (n_items + per_cta - 1) / per_cta, PREPARE_THREADS, bytes, st, 1, in,
+                           (const T*)v, stages, Tn, H, unit0, idx0, nb, n_items, lay)) return e;
+      }
+      const float* from = idx0 == 0 ? nullptr : between;
+      float* to = idx0 + nb == NB ? nullptr : between;
+      const SweepPart part{unit0, idx0, nb, from, to};
+      const int e = many ? launch_sweep<T, N, BWD, 4, MANY_CTAS_ROWS, 3>(dev, stages, s_in, n_state, out, s_out, ckpt, n_units, Tn, H, part, lay, st)
+                         : launch_sweep<T, N, BWD, FEW_CTAS_SLOTS<N>, FEW_CTAS_ROWS<N>, 1>(dev, stages, s_in, n_state, out, s_out, ckpt, n_units, Tn, H, part, lay, st);
+      if (e) return e;
     }
-    const bool first = idx0 == 0, last = idx0 + nb == NB;
-    const float* from = first ? s_in : between;
-    float* to = last ? s_out : between;
-    const int n_from = first ? n_state : units;
-    const int e = many ? launch_sweep<T, N, BWD, 4, MANY_CTAS_ROWS, 3>(dev, stages, from, n_from, out, to, ckpt, B, Tn, H, idx0, nb, lay, st)
-                       : launch_sweep<T, N, BWD, FEW_CTAS_SLOTS<N>, FEW_CTAS_ROWS<N>, 1>(dev, stages, from, n_from, out, to, ckpt, B, Tn, H, idx0, nb, lay, st);
-    if (e) return e;
-  }
   return RWKVB200_OK;
 }
 

@@ -127,6 +127,15 @@ Tensor fresh(at::IntArrayRef size, at::ScalarType t, const Tensor& like) {
 }
 Tensor fresh_like(const Tensor& x) { return fresh(x.sizes(), x.scalar_type(), x); }
 Tensor bytes(size_t n, const Tensor& like) { return fresh({(int64_t)n}, at::kByte, like); }
+// Memory that a call only runs faster with: an undefined tensor where it cannot be had.
+Tensor bytes_if_any(size_t n, const Tensor& like) {
+  try {
+    return n ? bytes(n, like) : Tensor();
+  } catch (const c10::OutOfMemoryError&) {
+    return Tensor();
+  }
+}
+size_t size_of(const Tensor& x) { return x.defined() ? (size_t)x.numel() : 0; }
 void* stream_of(const Tensor& x) { return c10::cuda::getCurrentCUDAStream(x.device().index()).stream(); }
 
 bool any_requires_grad(at::ArrayRef<const Tensor*> xs, const OptTensor& s) {
@@ -220,17 +229,20 @@ Three rwkv7_fwd(const Tensor& r, const Tensor& w, const Tensor& k, const Tensor&
                               d.B, d.H, d.K, code, stream_of(r)), "rwkv7_step");
   } else if (keep && !chunked_rwkv7(d, code, algo)) {
     const size_t n = rwkvb200_rwkv7_states_bytes(d.B, d.T, d.H, d.K, code, (int)algo);
-    const size_t ns = rwkvb200_rwkv7_fwd_workspace_bytes(d.B, d.T, d.H, d.K, code, (int)algo);
-    const Tensor scratch = ns ? bytes(ns, r) : Tensor();
-    ws = bytes(n, r);
-    check(rwkvb200_rwkv7_fwd_states(ptr(r), ptr(w), ptr(k), ptr(v), ptr(a), ptr(b), fptr(h0), n_state_of(h0), ptr(o), fptr(ht),
-                                    fptr(ws), n, ptr(scratch), ns, d.B, d.T, d.H, d.K, code, head_first, (int)algo, stream_of(r)),
+    ws = bytes_if_any(n, r);      // (without them the backward sweeps forward once more)
+    const Tensor scratch = bytes_if_any(rwkvb200_rwkv7_fwd_workspace_bytes(d.B, d.T, d.H, d.K, code, (int)algo), r);
+    check(size_of(ws) ? rwkvb200_rwkv7_fwd_states(ptr(r), ptr(w), ptr(k), ptr(v), ptr(a), ptr(b), fptr(h0), n_state_of(h0), ptr(o),
+                                                  fptr(ht), fptr(ws), n, ptr(scratch), size_of(scratch), d.B, d.T, d.H, d.K, code,
+                                                  head_first, (int)algo, stream_of(r))
+                      : rwkvb200_rwkv7_fwd(ptr(r), ptr(w), ptr(k), ptr(v), ptr(a), ptr(b), fptr(h0), n_state_of(h0), ptr(o), fptr(ht),
+                                           ptr(scratch), size_of(scratch), d.B, d.T, d.H, d.K, code, head_first, (int)algo, stream_of(r)),
           "rwkv7_fwd");
   } else {
     const size_t nws = rwkvb200_rwkv7_fwd_workspace_bytes(d.B, d.T, d.H, d.K, code, flags);
-    if (nws) ws = bytes(nws, r);
+    if (chunked_rwkv7(d, code, algo)) ws = bytes(nws, r);
+    else                              ws = bytes_if_any(nws, r);
     check(rwkvb200_rwkv7_fwd(ptr(r), ptr(w), ptr(k), ptr(v), ptr(a), ptr(b), fptr(h0), n_state_of(h0), ptr(o), fptr(ht),
-                             ptr(ws), nws, d.B, d.T, d.H, d.K, code, head_first, flags, stream_of(r)), "rwkv7_fwd");
+                             ptr(ws), size_of(ws), d.B, d.T, d.H, d.K, code, head_first, flags, stream_of(r)), "rwkv7_fwd");
   }
   return {o, ht, keep && ws.defined() ? ws : bytes(0, r)};
 }
@@ -247,17 +259,18 @@ Seven rwkv7_bwd(const Tensor& r, const Tensor& w, const Tensor& k, const Tensor&
   Tensor dr = fresh_like(r), dw = fresh_like(r), dk = fresh_like(r), dv = fresh_like(r), da = fresh_like(r),
          db = fresh_like(r), dh0 = fresh({d.B, d.H, d.K, d.K}, at::kFloat, r);
   if (have && !chunked_rwkv7(d, code, algo)) {
-    const size_t n = rwkvb200_rwkv7_bwd_states_workspace_bytes(d.B, d.T, d.H, d.K, code, (int)algo);
-    const Tensor ws = bytes(n, r);
+    Tensor ws = bytes_if_any(rwkvb200_rwkv7_bwd_states_workspace_bytes(d.B, d.T, d.H, d.K, code, (int)algo), r);
+    if (!ws.defined()) ws = bytes((size_t)kept.numel(), r);      // what is needed: as much as the forward left
     check(rwkvb200_rwkv7_bwd_states(ptr(r), ptr(w), ptr(k), ptr(v), ptr(a), ptr(b), fptr(h0), n_state_of(h0), ptr(d_o),
                                     fptr(d_ht), fptr(kept), (size_t)kept.numel(), ptr(dr), ptr(dw), ptr(dk), ptr(dv), ptr(da), ptr(db), fptr(dh0),
-                                    ptr(ws), n, d.B, d.T, d.H, d.K, code, head_first, (int)algo, stream_of(r)), "rwkv7_bwd");
+                                    ptr(ws), size_of(ws), d.B, d.T, d.H, d.K, code, head_first, (int)algo, stream_of(r)), "rwkv7_bwd");
     return {dr, dw, dk, dv, da, db, dh0};
   }
-  const size_t nws = have ? (size_t)kept.numel() : rwkvb200_rwkv7_bwd_workspace_bytes(d.B, d.T, d.H, d.K, code, (int)algo);
-  const Tensor ws = have ? kept : nws ? bytes(nws, r) : Tensor();
+  const size_t nws = rwkvb200_rwkv7_bwd_workspace_bytes(d.B, d.T, d.H, d.K, code, (int)algo);
+  Tensor ws = have ? kept : chunked_rwkv7(d, code, algo) ? bytes(nws, r) : bytes_if_any(nws, r);
+  if (nws && !ws.defined()) ws = bytes((size_t)d.B * d.H * ((d.T + 7) / 8) * d.K * d.K * sizeof(float) + 255, r);      // what is needed
   check(rwkvb200_rwkv7_bwd(ptr(r), ptr(w), ptr(k), ptr(v), ptr(a), ptr(b), fptr(h0), n_state_of(h0), ptr(d_o), fptr(d_ht),
-                           ptr(dr), ptr(dw), ptr(dk), ptr(dv), ptr(da), ptr(db), fptr(dh0), ptr(ws), nws, d.B, d.T, d.H,
+                           ptr(dr), ptr(dw), ptr(dk), ptr(dv), ptr(da), ptr(db), fptr(dh0), ptr(ws), size_of(ws), d.B, d.T, d.H,
                            d.K, code, head_first, (int)algo | (have ? RWKVB200_ALGO_KEEP : 0), stream_of(r)),
         "rwkv7_bwd");
   return {dr, dw, dk, dv, da, db, dh0};

@@ -115,6 +115,23 @@ def test_python_mirrors_of_the_kept_sizes_match_the_library(lib):
         assert _lib.wkv6_kept_bytes(B, T, H) == lib.rwkvb200_wkv6_bwd_workspace_bytes(B, T, H, 64, _lib.F32, 0)
 
 
+def test_scratch_of_the_float32_recurrence(lib):
+    """Asked for where the sweeps use it (148 SMs), and 256 MB at most however many sequences and heads there are."""
+    def fwd(B, T, H, K):
+        return lib.rwkvb200_rwkv7_fwd_workspace_bytes(B, T, H, K, _lib.F32, _lib.ALGO_AUTO)
+
+    for B, T, H, K in [(2, 1024, 32, 64), (1, 8192, 64, 64), (1, 376, 37, 64), (1, 88, 18, 128), (64, 24, 64, 64), (64, 24, 64, 128)]:
+        assert fwd(B, T, H, K) == 0, (B, T, H, K)
+    for B, T, H, K in [(1, 377, 37, 64), (1, 25, 75, 64), (1, 89, 18, 128), (1, 25, 19, 128), (64, 64, 64, 64), (256, 32, 64, 64),
+                       (512, 128, 64, 128), (1 << 16, 4096, 64, 128), (16, 8192, 64, 64)]:
+        n = fwd(B, T, H, K)
+        assert 0 < n <= 256 << 20, (B, T, H, K, n)
+        checkpoints = (B * H * ((T + 7) // 8) * K * K * 4 + 255) // 256 * 256
+        assert lib.rwkvb200_rwkv7_bwd_workspace_bytes(B, T, H, K, _lib.F32, _lib.ALGO_AUTO) == checkpoints + n
+        left = lib.rwkvb200_rwkv7_states_bytes(B, T, H, K, _lib.F32, _lib.ALGO_AUTO)
+        assert lib.rwkvb200_rwkv7_bwd_states_workspace_bytes(B, T, H, K, _lib.F32, _lib.ALGO_AUTO) == (left + 255) // 256 * 256 + n
+
+
 def test_shared_memory_that_has_to_start_aligned():
     """A kernel without room to align its tiles by hand is refused by its launch, not skipped by its own check, where the
     system's and the kernel's own shared memory do not leave the rest 1024-byte aligned."""

@@ -177,16 +177,19 @@ def test_states_kept_for_the_backward(T, K, dtype, monkeypatch):
         assert torch.equal(a, b) and torch.equal(a, c)
 
 
+def _sizes_prepared_apart(K, sms):
+    """(units, tokens): block counts from which a sweep's blocks are prepared by a kernel of their own with fewer CTAs than SMs and
+    with many; then stretches of blocks, and passes of units, where the scratch does not hold all of them."""
+    return ([(3, T) for T in (95, 96, 377, 384, 400)] + [(2 * sms // (K // 16) + 2, T) for T in (24, 25, 32, 33, 70)]
+            + [(400 if K == 64 else 200, 600), (3100 if K == 64 else 1200, 70)])
+
+
 @pytest.mark.parametrize("K,dtype", [(64, torch.float32), (64, torch.float16), (128, torch.float32), (128, torch.bfloat16)])
-@pytest.mark.parametrize("few", [False, True])
-def test_blocks_prepared_apart(K, dtype, few):
-    """The sweeps with and without their scratch (C ABI): the same bits, at the block counts from which the scratch is used, and
-    where a unit's blocks take several stretches of it."""
+def test_blocks_prepared_apart(K, dtype):
+    """The sweeps with and without their scratch (C ABI): the same bits, whatever part of it a call works with at a time."""
     lib, dev = _lib.load(), torch.device("cuda")
-    sms = torch.cuda.get_device_properties(0).multi_processor_count
     code = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}[dtype]
-    H = 3 if few else 2 * sms // (K // 16) + 2
-    for T in ((95, 96, 377, 384, 400) if few else (24, 25, 32, 33, 70)) + (() if few or K == 128 else (2500,)):
+    for H, T in _sizes_prepared_apart(K, torch.cuda.get_device_properties(0).multi_processor_count):
         d = rwkv7_inputs(1, T, H, K, dtype=dtype, seed=T, device="cuda", with_state=True)
         x = [d[n] for n in "rwkvab"]
         out = []
@@ -198,7 +201,40 @@ def test_blocks_prepared_apart(K, dtype, few):
                                               _lib.ptr(ws) if n else None, n, 1, T, H, K, code, 0, _lib.ALGO_RECURRENT,
                                               _lib.stream_ptr(dev)), "fwd")
             out.append((o, s))
-        assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1]), T
+        assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1]), (H, T)
+
+
+def test_scratch_that_cannot_be_had_is_done_without():
+    """The float32 recurrence's scratch, and the states its forward leaves, are for speed: where the allocator has no room for
+    them, the operator runs without and returns the same bits."""
+    H, T, mb = 600, 512, 1 << 20
+    d = rwkv7_inputs(1, T, H, seed=3, device="cuda", with_grads=True)
+    x = [d[n].requires_grad_(True) for n in "rwkvab"]
+    total = torch.cuda.get_device_properties(0).total_memory
+
+    def room_for(more):      # what is in use, and `more` bytes
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + more) / total)
+
+    tokens, states = x[0].numel() * 4, H * (T // 16 - 1) * 64 * 64 * 4
+    try:
+        o, s = ro.generalized_delta_rule(*x)
+        grads = torch.autograd.grad([o, s], x, [d["d_out"], d["d_state"]], retain_graph=True)
+        room_for(6 * tokens + states + 100 * mb)      # the backward's scratch are 256 MB more
+        grads2 = torch.autograd.grad([o, s], x, [d["d_out"], d["d_state"]])
+        assert all(torch.equal(a, b) for a, b in zip(grads, grads2))
+        del grads2
+        room_for(tokens + 100 * mb)                   # neither states nor scratch
+        o2, s2 = ro.generalized_delta_rule(*x)
+        assert torch.equal(o2, o) and torch.equal(s2, s)
+        with torch.no_grad():
+            del o2, s2
+            room_for(tokens + 100 * mb)
+            o2, s2 = ro.generalized_delta_rule(*x)
+        assert torch.equal(o2, o) and torch.equal(s2, s)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
 
 
 @pytest.mark.parametrize("lens,H", [([1500, 70, 64, 8, 200, 130, 9, 65, 300, 128], 20), ([8 + i % 70 for i in range(260)], 1)])
