@@ -134,7 +134,7 @@ def rwkv7_kept_bytes(n_seq: int, max_len: int, H: int) -> int:
     ``rwkvb200_rwkv7_fwd_workspace_bytes(..., ALGO_KEEP)`` without calling into the library (the shape
     functions of the custom ops must run without a device)."""
     n = n_seq * H * ((max_len + 63) // 64)
-    return _a256(n * 16 * 8192) + _a256(n * 128 * 4) + _a256(n_seq * H * 4) + 1024
+    return _a256(n * 16 * 8192) + _a256(n * 128 * 4) + _a256(n_seq * H * 4) + _a256((n + 1024) * 8) + 1024
 
 
 def rwkv7_states_bytes(B: int, T: int, H: int, K: int) -> int:

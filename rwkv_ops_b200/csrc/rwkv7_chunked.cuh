@@ -75,13 +75,8 @@ struct SeqView {
   }
 };
 
-// The chunk-heads a persistent CTA works on: every gridDim.x-th of a list in which the heads of one chunk of tokens follow
-// each other, so that the CTAs at work at one time read and write whole token rows (H * 128 bytes) between them.  `ch` is the
-// workspace slot.
-// Dense: chunk by chunk through all sequences at once, DOWN from the last chunk to the first or up: what a kernel
-// touches last is what the next one starts with, while it is still in L2 (the forward scan starts at chunk 0, the reverse
-// scan ends there).  Packed: sequence by sequence, without the slots past a sequence's end (skipping those left some CTAs with a
-// fifth more chunk-heads than others: intra / final kernel of 8 sequences of 1093 .. 4096 tokens, 32 heads, 310 / 348 -> 292 / 316 us).
+// The chunk-heads that the persistent CTAs of a kernel work on, and in which order; `ch` is the workspace slot, n_ch after the
+// last one.
 struct ChunkPos { int ch, bi, hi, c; };
 // (a kernel parameter, made on the host: computed in the kernels it would take registers that they do not have)
 struct WalkDims {
@@ -91,60 +86,41 @@ struct WalkDims {
       : H(H_), NT(NT_), B(B_), n_ch(H_ * NT_ * B_), dh(by_unit ? grid / NT_ % H_ : grid % H_),
         db(by_unit ? grid / NT_ / H_ : grid / H_ % B_), dc(by_unit ? grid % NT_ : grid / H_ / B_) {}
 };
-template <bool PACKED, bool DOWN>
-struct ChunkWalk {
-  const SeqView& sv;
+// Dense, by rows: every gridDim.x-th of a list in which the heads of one chunk of tokens follow each other, so that the CTAs at work
+// at one time read and write whole token rows (H * 128 bytes) between them.  It goes through all sequences at once, from the last chunk
+// to the first: what the kernel touches last is what the scan starts with, while it is still in L2.
+struct RowWalk {
   const WalkDims& d;
   __device__ __forceinline__ void place(ChunkPos& p, int level) const {
-    p.c = DOWN ? d.NT - 1 - level : level;
+    p.c = d.NT - 1 - level;
     p.ch = level < d.NT ? (p.bi * d.H + p.hi) * d.NT + p.c : d.n_ch;
-  }
-  // packed: the r-th chunk-head counted from the start of sequence p.bi
-  __device__ __forceinline__ void place_packed(ChunkPos& p, int r) const {
-    for (; p.bi < d.B; ++p.bi) {
-      const int n = d.H * ((sv.template length<true>(p.bi) + L - 1) / L);
-      if (r < n) break;
-      r -= n;
-    }
-    p.c = r / d.H;
-    p.hi = r % d.H;
-    p.ch = p.bi < d.B ? (p.bi * d.H + p.hi) * d.NT + p.c : d.n_ch;
   }
   __device__ __forceinline__ ChunkPos first() const {
     ChunkPos p;
     const int i = blockIdx.x;
-    if constexpr (PACKED) {
-      p.bi = 0;
-      place_packed(p, i);
-    } else {
-      p.hi = i % d.H; p.bi = i / d.H % d.B;
-      place(p, i / d.H / d.B);
-    }
+    p.hi = i % d.H; p.bi = i / d.H % d.B;
+    place(p, i / d.H / d.B);
     return p;
   }
-  __device__ __forceinline__ ChunkPos after(ChunkPos p) const {      // p is in the list
-    if constexpr (PACKED) {
-      place_packed(p, p.c * d.H + p.hi + gridDim.x);
-    } else {
-      int level = (DOWN ? d.NT - 1 - p.c : p.c) + d.dc;
-      p.hi += d.dh;
-      p.bi += d.db;
-      if (p.hi >= d.H) { p.hi -= d.H; ++p.bi; }
-      if (p.bi >= d.B) { p.bi -= d.B; ++level; }
-      place(p, level);
-    }
+  __device__ __forceinline__ ChunkPos after(ChunkPos p, int) const {      // p is in the list
+    int level = d.NT - 1 - p.c + d.dc;
+    p.hi += d.dh;
+    p.bi += d.db;
+    if (p.hi >= d.H) { p.hi -= d.H; ++p.bi; }
+    if (p.bi >= d.B) { p.bi -= d.B; ++level; }
+    place(p, level);
     return p;
   }
 };
 
-// Dense: the same list unit by unit, in the order of the workspace (WalkDims by unit).
+// Dense, by unit: every gridDim.x-th in the order of the workspace (WalkDims by unit).
 struct UnitWalk {
   const WalkDims& d;
   __device__ __forceinline__ ChunkPos first() const {
     const int i = blockIdx.x;
     return ChunkPos{i, i / d.NT / d.H, i / d.NT % d.H, i % d.NT};
   }
-  __device__ __forceinline__ ChunkPos after(ChunkPos p) const {
+  __device__ __forceinline__ ChunkPos after(ChunkPos p, int) const {
     p.ch += gridDim.x;
     p.c += d.dc;
     p.hi += d.dh;
@@ -155,13 +131,60 @@ struct UnitWalk {
   }
 };
 
-// The unit of a scan's block in a packed batch: the longest sequences come first, so that the blocks which start when others have ended are
-// short ones.  Up to MAX_SORTED sequences are ranked by length, by the threads of the block.
+// Packed: the heads of one chunk, then of the next one of its sequence, then the next sequence; no slot past a sequence's end.  Again
+// every gridDim.x-th, which may be many short sequences on: so the intra kernel's CTAs write down which sequence and chunk each of
+// theirs is, once, and both kernels read that.  (A search from one to the next, every thread for itself: 4000 sequences of 8 .. 64
+// tokens, one head, intra / final kernel 412 / 443 us against 127 / 148.  A stretch of neighbours for each CTA instead needs no list, but
+// the CTAs then share no token rows: 8 sequences of up to 4096 tokens, 32 heads, 838 -> 880 us forward and backward.  Slots past a sequence's end left in the
+// list, so that no search is needed: 1000 sequences of 30 .. 500 tokens, 12 heads, 2465 / 2816 us against 1670 / 1825.)
+struct ListWalk {
+  const WalkDims& d;
+  const int2* list;      // of every chunk-head: sequence, chunk; -1 after the last one of each CTA
+  __device__ __forceinline__ ChunkPos at(int i, int hi) const {
+    const int2 e = __ldcg(list + i);
+    return ChunkPos{e.x < 0 ? d.n_ch : (e.x * d.H + hi) * d.NT + e.y, e.x, hi, e.y};
+  }
+  __device__ __forceinline__ ChunkPos first() const { return at(blockIdx.x, blockIdx.x % d.H); }
+  __device__ __forceinline__ ChunkPos after(const ChunkPos& p, int it) const {      // p: the CTA's it-th
+    const int hi = p.hi + d.dh;
+    return at(blockIdx.x + (it + 1) * gridDim.x, hi >= d.H ? hi - d.H : hi);
+  }
+};
+// A CTA's part of the list; all 256 threads.  `sums`: shared memory of 8 ints.
+__device__ __forceinline__ void write_list(int2* list, const SeqView& sv, const WalkDims& d, int* sums, int tid) {
+  auto chunks = [&](int bi) { return min(max((sv.length<true>(bi) + L - 1) / L, 0), d.NT); };
+  const int per = (d.B + 255) / 256, s0 = min(tid * per, d.B), s1 = min(s0 + per, d.B);
+  int mine = 0;      // chunks of the sequences s0 .. s1 - 1
+  for (int s = s0; s < s1; ++s) mine += chunks(s);
+  int upto = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o *= 2) {
+    const int x = __shfl_up_sync(0xffffffffu, upto, o);
+    if ((tid & 31) >= o) upto += x;
+  }
+  if ((tid & 31) == 31) sums[tid >> 5] = upto;
+  __syncthreads();
+  int from = upto - mine;
+  for (int w = 0; w < (tid >> 5); ++w) from += sums[w];
+  const int step = gridDim.x;
+  int i = blockIdx.x;      // the CTA's first chunk-head in these sequences
+  if (from * d.H > i) i += (from * d.H - i + step - 1) / step * step;
+  for (int s = s0; s < s1; ++s) {
+    const int n = chunks(s);
+    for (; i < (from + n) * d.H; i += step) list[i] = make_int2(s, i / d.H - from);
+    from += n;
+  }
+  if (tid == 255) list[i] = make_int2(-1, 0);
+  __syncthreads();
+}
+
+// The unit of a scan's block in a packed batch where the blocks come in more than one round and that pays (scans_sorted): the longest
+// sequences come first, so that the blocks which start when others have ended are short ones.  The sequences (MAX_SORTED at most) are
+// ranked by length, by the threads of the block.
 constexpr int MAX_SORTED = 256;
 struct SortedSeqs { int len[MAX_SORTED], at; };
-__device__ __forceinline__ int packed_scan_unit(const SeqView& sv, int H, SortedSeqs* sorted, int tid) {
+__device__ __forceinline__ int sorted_scan_unit(const SeqView& sv, int H, SortedSeqs* sorted, int tid) {
   const int n_seq = gridDim.x / H, b = blockIdx.x;
-  if (n_seq > MAX_SORTED) return b;
   if (tid < n_seq) sorted->len[tid] = __ldg(sv.len + tid);
   __syncthreads();
   if (tid < n_seq) {
@@ -185,6 +208,17 @@ inline bool scans_alone(int n_seq, int Tn, int T_total, int H, int sms, bool pac
   const float rounds = fmaxf(longest, per_sm + 0.25f * mean);      // chunks in a row on the slowest SM
   const float memory = units * mean * kb / 6000.f;
   return fmaxf(rounds * 1.3f, memory * rounds / per_sm) < fmaxf(longest * 3.3f, memory);
+}
+
+// Whether the blocks of a packed batch's scans come longest sequence first.  Ranking the sequences costs a block 1 us and more (and the
+// kernel its uniform registers), so with two blocks to an SM and several rounds of them it takes one sequence well above the mean
+// (forward scan in order and sorted: 24 sequences of 300 .. 6000 tokens, 16 heads 411 and 358 us, 48 heads 887 and 790; 100 of 50 .. 600,
+// 12 heads 133 and 145; 256 of 64, 12 heads 79 and 136).
+inline bool scans_sorted(int n_seq, int Tn, int T_total, int H, int sms, bool alone) {
+  const int units = n_seq * H;
+  if (n_seq > MAX_SORTED || units <= (alone ? sms : 2 * sms)) return false;
+  const float longest = (float)num_chunks(Tn), mean = (float)T_total / n_seq / L + 0.5f;
+  return alone || longest - mean > (float)units / sms;
 }
 
 // Fused producers (template parameter FUSED of the intra and final kernels).  The three inputs w, a, b of
@@ -216,8 +250,15 @@ struct Workspace {
   float* aux;             // [n_chunks_total][128]
   int* flags;             // [B*H] nonzero: the unit's decay left the range of the scaled operands (DECAY_LIMIT); written by
                           // the forward scan, from the signs of the e^{glast-gref} in aux
+  int2* list;             // [n_chunks_total + MAX_GRID] which sequence and chunk the chunk-heads of a packed batch are (ListWalk)
   int tiles_per_chunk;
 };
+// The intra and the final kernel are persistent, two CTAs per SM; both have the same grid (ListWalk).
+constexpr int MAX_GRID = 1024;
+inline int persistent_grid(int n_ch, int sms) {
+  const int most = 2 * sms < MAX_GRID ? 2 * sms : MAX_GRID;
+  return n_ch < most ? n_ch : most;
+}
 
 // The scaled operands carry e^{+-(gi - gref)}: with the reference point in the middle of the chunk the
 // exponent of a channel reaches the sum of |g| over half a chunk.  Up to DECAY_LIMIT every factor and every
@@ -239,7 +280,7 @@ inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 inline size_t fwd_workspace_bytes(int B, int T, int H, int tiles_per_chunk) {
   const size_t n = (size_t)B * H * num_chunks(T);
   return align256(n * tiles_per_chunk * tc::TILE_BYTES) + align256(n * AUX_FLOATS * sizeof(float)) +
-         align256((size_t)B * H * sizeof(int)) + 1024;
+         align256((size_t)B * H * sizeof(int)) + align256((n + MAX_GRID) * sizeof(int2)) + 1024;
 }
 
 inline Workspace carve(void* ws, int B, int T, int H, int tiles_per_chunk) {
@@ -249,6 +290,7 @@ inline Workspace carve(void* ws, int B, int T, int H, int tiles_per_chunk) {
   w.tiles = reinterpret_cast<unsigned char*>(p);
   w.aux = reinterpret_cast<float*>(p + align256(n * tiles_per_chunk * tc::TILE_BYTES));
   w.flags = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(w.aux) + align256(n * AUX_FLOATS * sizeof(float)));
+  w.list = reinterpret_cast<int2*>(reinterpret_cast<unsigned char*>(w.flags) + align256((size_t)B * H * sizeof(int)));
   w.tiles_per_chunk = tiles_per_chunk;
   return w;
 }

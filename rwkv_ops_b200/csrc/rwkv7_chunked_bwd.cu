@@ -34,7 +34,7 @@ struct BScanSmem {
   uint32_t tmem_base;
 };
 
-template <bool PACKED>
+template <bool PACKED, bool SORTED>
 __global__ void __launch_bounds__(256, 2)
 r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* __restrict__ ws_tiles,
                     const float* __restrict__ ws_aux, int tiles_per_chunk, const float* __restrict__ d_ht,
@@ -42,7 +42,6 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
   extern __shared__ unsigned char smem_raw[];
   BScanSmem& sm = *reinterpret_cast<BScanSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  int unit = blockIdx.x, bi = unit / H, hi = unit % H;
   const int wq = warp & 3, hsel = warp >> 2, c0 = 32 * hsel;
   const int row = 16 * wq + (lane & 15);
   const bool state_lane = lane < 16;
@@ -50,6 +49,14 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
   // bulk-copy groups), ld_warp requests the operand tiles of the chunk after the next
   constexpr int st_warp = 1, ld_warp = 2;
 
+  // A packed batch may have many short sequences, whose blocks come in many rounds: where theirs lies is asked for before the TMEM is
+  // (4000 of up to 64 tokens, 16 heads: 1125 -> 1087 us).
+  if constexpr (PACKED) earlier_kernels_done();
+  int unit = blockIdx.x;
+  if constexpr (SORTED) unit = sorted_scan_unit(sv, H, reinterpret_cast<SortedSeqs*>(sm.dz), tid);
+  const int bi = unit / H, hi = unit % H;
+  const int Tn = sv.length<PACKED>(bi), tb = sv.first<PACKED>(bi), brow = sv.row<PACKED>(bi);
+  const int NT = (Tn + L - 1) / L;           // chunks of this sequence (at least one)
   if (tid == 0) {
     mbar_init(&sm.bar_full[0], 1); mbar_init(&sm.bar_full[1], 1);
     mbar_init(&sm.bar_m1, 1); mbar_init(&sm.bar_m2, 1);
@@ -60,15 +67,9 @@ r7c_bwd_scan_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  earlier_kernels_done();
+  if constexpr (!PACKED) earlier_kernels_done();
   later_kernels_may_start();
-  if constexpr (PACKED) {
-    unit = packed_scan_unit(sv, H, reinterpret_cast<SortedSeqs*>(sm.dz), tid);
-    bi = unit / H; hi = unit % H;
-  }
   const size_t ch0 = (size_t)unit * NT_slots;
-  const int NT = (sv.length<PACKED>(bi) + L - 1) / L;      // chunks of this sequence
-  const int tb = sv.first<PACKED>(bi), brow = sv.row<PACKED>(bi);
   const uint32_t tm = sm.tmem_base;
   // TMEM: columns 64 p .., p = parity of the chunk's place: lower lane halves q~^T do + a~^T dz, upper halves dz
 
@@ -216,7 +217,7 @@ struct BAloneSmem {
 };
 constexpr int BALONE_THREADS = 352;
 
-template <bool PACKED>
+template <bool PACKED, bool SORTED>
 __global__ void __launch_bounds__(BALONE_THREADS, 1)
 r7c_bwd_scan_alone_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned char* __restrict__ ws_tiles,
                           const float* __restrict__ ws_aux, int tiles_per_chunk, const float* __restrict__ d_ht,
@@ -242,8 +243,8 @@ r7c_bwd_scan_alone_kernel(const __grid_constant__ CUtensorMap tmap_do, unsigned 
   tc_fence_after();
   earlier_kernels_done();
   later_kernels_may_start();
-  if constexpr (PACKED) {
-    unit = packed_scan_unit(sv, H, reinterpret_cast<SortedSeqs*>(sm.dz[0]), tid);
+  if constexpr (SORTED) {
+    unit = sorted_scan_unit(sv, H, reinterpret_cast<SortedSeqs*>(sm.dz[0]), tid);
     bi = unit / H; hi = unit % H;
   }
   const size_t ch0 = (size_t)unit * NT_slots;
@@ -421,7 +422,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
                      const __grid_constant__ CUtensorMap tmap_db,
                      bf16* __restrict__ dq_rows, bf16* __restrict__ dw_rows, bf16* __restrict__ dk_rows,
                      bf16* __restrict__ dv_rows, bf16* __restrict__ da_rows, bf16* __restrict__ db_rows,
-                     SeqView sv, const __grid_constant__ WalkDims dims, TokLayout lay, int* status, long long* dbg) {
+                     SeqView sv, const __grid_constant__ WalkDims dims, const int2* list, TokLayout lay, int* status, long long* dbg) {
 #ifdef RWKVB200_DEVTOOLS
 #define R7C_STAMP(n) do { if (dbg && tid == 0 && blockIdx.x == gridDim.x / 2 && it == 15) dbg[n] = clock64(); } while (0)
 #else
@@ -516,7 +517,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
   // Dense: unit by unit, for the 20 tiles that lie side by side in the workspace; by rows of tokens, as the intra kernel goes, this
   // one took 500 us against 489 (B 8, T 4096, 32 heads).
   const auto walk = [&] {
-    if constexpr (PACKED) return ChunkWalk<true, false>{sv, dims}; else return UnitWalk{dims};
+    if constexpr (PACKED) return ListWalk{dims, list}; else return UnitWalk{dims};
   }();
   ChunkPos cur = walk.first();
 
@@ -538,7 +539,7 @@ r7c_bwd_final_kernel(const bf16* __restrict__ w, const __grid_constant__ CUtenso
     const int tt = sv.first<PACKED>(bi) + t0, br = sv.row<PACKED>(bi);
     const unsigned char* tiles = ws_tiles + (size_t)cur.ch * tiles_per_chunk * TILE_BYTES;
     const uint32_t par = it & 1;
-    nxt = walk.after(cur);
+    nxt = walk.after(cur, it);
     const bool more = nxt.ch < dims.n_ch;
     R7C_STAMP(16);
 
@@ -949,20 +950,22 @@ int launch_rwkv7_chunked_bwd(const void* r, const void* w, const void* k, const 
   TokLayout lay(mapT, H, head_first);
   if (phases & PHASE_SCAN) {
     ProfScope prof("r7c_bwd_scan_kernel", st);
-#define R7C_LAUNCH_BSCAN(KERNEL, P, THREADS, SMEM)                                                                \
+#define R7C_LAUNCH_BSCAN(THREADS, SMEM, ...)                                                                       \
     do {                                                                                                          \
       const int smem = (int)sizeof(SMEM) + 1024;                                                                  \
-      if (allow_smem<KERNEL<P>>(dev, smem)) return RWKVB200_E_CUDA;                                               \
-      if (int rc = launch(KERNEL<P>, B * H, THREADS, smem, st, 1, tmap_do, ws.tiles, ws.aux, (int)ALL_TILES, \
-                          d_ht, d_h0, sv, H, NT, status)) return rc;                                                                  \
+      if (allow_smem<__VA_ARGS__>(dev, smem)) return RWKVB200_E_CUDA;                                             \
+      if (int rc = launch(__VA_ARGS__, B * H, THREADS, smem, st, 1, tmap_do, ws.tiles, ws.aux, (int)ALL_TILES,    \
+                          d_ht, d_h0, sv, H, NT, status)) return rc;                                              \
     } while (0)
-    if (!scans_alone(B, Tn, T_total, H, dev.sms, seq_start != nullptr, 56.f)) {      // two CTAs per SM
-      if (seq_start) R7C_LAUNCH_BSCAN(r7c_bwd_scan_kernel, true, 256, BScanSmem);
-      else           R7C_LAUNCH_BSCAN(r7c_bwd_scan_kernel, false, 256, BScanSmem);
-    } else {
-      if (seq_start) R7C_LAUNCH_BSCAN(r7c_bwd_scan_alone_kernel, true, BALONE_THREADS, BAloneSmem);
-      else           R7C_LAUNCH_BSCAN(r7c_bwd_scan_alone_kernel, false, BALONE_THREADS, BAloneSmem);
-    }
+    const bool packed = seq_start != nullptr, alone = scans_alone(B, Tn, T_total, H, dev.sms, packed, 56.f);
+    const bool sorted = packed && scans_sorted(B, Tn, T_total, H, dev.sms, alone);
+    if (!alone) {      // two CTAs per SM
+      if (sorted)      R7C_LAUNCH_BSCAN(256, BScanSmem, r7c_bwd_scan_kernel<true, true>);
+      else if (packed) R7C_LAUNCH_BSCAN(256, BScanSmem, r7c_bwd_scan_kernel<true, false>);
+      else             R7C_LAUNCH_BSCAN(256, BScanSmem, r7c_bwd_scan_kernel<false, false>);
+    } else if (sorted) R7C_LAUNCH_BSCAN(BALONE_THREADS, BAloneSmem, r7c_bwd_scan_alone_kernel<true, true>);
+    else if (packed)   R7C_LAUNCH_BSCAN(BALONE_THREADS, BAloneSmem, r7c_bwd_scan_alone_kernel<true, false>);
+    else               R7C_LAUNCH_BSCAN(BALONE_THREADS, BAloneSmem, r7c_bwd_scan_alone_kernel<false, false>);
 #undef R7C_LAUNCH_BSCAN
   }
   e = check_launch();
@@ -990,7 +993,7 @@ int launch_rwkv7_chunked_bwd(const void* r, const void* w, const void* k, const 
     ProfScope prof("r7c_bwd_final_kernel", st);
     const int n_ch = B * H * NT;
     const int sms = dev.sms;
-    const int grid = n_ch < 2 * sms ? n_ch : 2 * sms;     // persistent: two CTAs per SM
+    const int grid = persistent_grid(n_ch, sms);
     // Blocks that come while the reverse scan runs out save the 2 us between two kernels, but where the CTAs walk over
     // many chunk-heads the kernel is slower for it (which the launch alone does; why was not isolated).  Forward and backward, us,
     // with and without, 32 heads: B 1, T 4096 318 and 316; B 2 444 and 441; B 4, T 1024, 48 heads 310 and 303; B 16, T 8192, 64 heads
@@ -1003,7 +1006,7 @@ int launch_rwkv7_chunked_bwd(const void* r, const void* w, const void* k, const 
         return RWKVB200_E_CUDA;                                                                                   \
       if (int rc = launch(r7c_bwd_final_kernel<P, F>, grid, 256, smem, st, early, (const bf16*)w, tmap_w, tmap_do, tmap_v, ws.tiles, (int)ALL_TILES, \
           tmap_out[0], tmap_out[1], tmap_out[2], tmap_out[3], tmap_out[4], tmap_out[5], (bf16*)dr, (bf16*)dw,     \
-          (bf16*)dk, (bf16*)dv, (bf16*)da, (bf16*)db, sv, WalkDims(H, NT, B, grid, !P), lay, status, debug_stamp_buffer())) return rc; \
+          (bf16*)dk, (bf16*)dv, (bf16*)da, (bf16*)db, sv, WalkDims(H, NT, B, grid, !P), ws.list, lay, status, debug_stamp_buffer())) return rc; \
     } while (0)
     if (seq_start) R7C_LAUNCH_FINAL(true, false);
     else if (fused) R7C_LAUNCH_FINAL(false, true);

@@ -34,7 +34,7 @@ struct IntraSmem {
   uint32_t tmem_base;
 };
 
-// Persistent: CTAs (two per SM) walk over the chunk-heads, the last chunks first (ChunkWalk).
+// Persistent: CTAs (two per SM) walk over the chunk-heads (RowWalk, ListWalk).
 // 256 threads: warp w reads TMEM lanes 32*(w&3).. and the two warps that share a lane window split
 // the columns (hsel = w>>2); warps 6 and 7 invert the diagonal blocks of A_ab while the other warps mask the rest of
 // MMA 1, issue MMA 2 and drain it.
@@ -51,7 +51,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
                      const __grid_constant__ CUtensorMap tmap_b,
                      const __grid_constant__ CUtensorMap tmap_v, unsigned char* __restrict__ ws_tiles,
                      float* __restrict__ ws_aux, int tiles_per_chunk,
-                     int keep_for_bwd, SeqView sv, const __grid_constant__ WalkDims dims, TokLayout lay, int* status, long long* dbg) {
+                     int keep_for_bwd, SeqView sv, const __grid_constant__ WalkDims dims, int2* list, TokLayout lay, int* status, long long* dbg) {
 #ifdef RWKVB200_DEVTOOLS
 #define R7C_STAMP(n) do { if (dbg && tid == 0 && blockIdx.x == gridDim.x / 2 && it == 30) dbg[n] = clock64(); } while (0)
 #else
@@ -70,7 +70,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
   if (tid == 32) {
     tma_prefetch_maps(tmap_q, tmap_w, tmap_k, tmap_a, tmap_b, tmap_v);
     if constexpr (!PACKED) {      // the first rows into L2, while the kernel before runs out
-      const ChunkPos p = ChunkWalk<PACKED, true>{sv, dims}.first();
+      const ChunkPos p = RowWalk{dims}.first();
       tma_prefetch_4d(&tmap_w, 0, p.c * L, p.hi, p.bi);
       tma_prefetch_4d(&tmap_q, 0, p.c * L, p.hi, p.bi);
       tma_prefetch_4d(&tmap_k, 0, p.c * L, p.hi, p.bi);
@@ -113,7 +113,10 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
     tma_prefetch_4d(&tmap_b, 0, tt, p.hi, br);
     tma_prefetch_4d(&tmap_v, 0, tt, p.hi, br);
   };
-  const ChunkWalk<PACKED, true> walk{sv, dims};
+  if constexpr (PACKED) write_list(list, sv, dims, reinterpret_cast<int*>(sm.qtot), tid);
+  const auto walk = [&] {
+    if constexpr (PACKED) return ListWalk{dims, list}; else return RowWalk{dims};
+  }();
   ChunkPos cur = walk.first();
   if (cur.ch < dims.n_ch && warp == 0 && elect_one()) { load_w(cur); load_qka(cur); load_b(cur); }
   // The two CTAs that share an SM would otherwise run their phases in lockstep and compete for the
@@ -129,7 +132,7 @@ r7c_intra_fwd_kernel(const bf16* __restrict__ q, const bf16* __restrict__ w, con
     const int Tn = sv.length<PACKED>(bi);
     unsigned char* out_tiles = ws_tiles + (size_t)ch * tiles_per_chunk * TILE_BYTES;
     const uint32_t par = it & 1;
-    nxt = walk.after(cur);
+    nxt = walk.after(cur, it);
     const int next = nxt.ch;
 
     R7C_STAMP(0);
@@ -593,7 +596,7 @@ __device__ __noinline__ void exact_unit(r7rec::FwdArgs<bf16> args, unsigned char
   r7rec::fwd_rows<bf16, 64, 64, 2, 16, 256>(args, *reinterpret_cast<Smem*>(smem), 0, tid);
 }
 
-template <bool PACKED>
+template <bool PACKED, bool SORTED>
 __global__ void __launch_bounds__(256, 2)
 r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned char* __restrict__ ws_tiles,
                     const float* __restrict__ ws_aux, int* __restrict__ ws_flags, int tiles_per_chunk,
@@ -609,7 +612,6 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
   extern __shared__ unsigned char smem_raw[];
   ScanSmem& sm = *reinterpret_cast<ScanSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  int unit = blockIdx.x, bi = unit / H, hi = unit % H;
   const int wq = warp & 3, hsel = warp >> 2, c0 = 32 * hsel;
   const int row = 16 * wq + (lane & 15);     // state row k (lanes 0-15) or token row i (lanes 16-31)
   const bool state_lane = lane < 16;
@@ -618,6 +620,14 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
   // thread waits for its own copies.
   constexpr int ld_warp = 1, st_warp = 2, out_warp = 3;
 
+  // A packed batch may have many short sequences, whose blocks come in many rounds: where theirs lies is asked for before the TMEM is
+  // (4000 of up to 64 tokens, 16 heads: 1404 -> 1357 us).
+  if constexpr (PACKED) earlier_kernels_done();
+  int unit = blockIdx.x;
+  if constexpr (SORTED) unit = sorted_scan_unit(sv, H, reinterpret_cast<SortedSeqs*>(sm.ot), tid);
+  const int bi = unit / H, hi = unit % H;
+  const int Tn = sv.length<PACKED>(bi), tb = sv.first<PACKED>(bi), brow = sv.row<PACKED>(bi);
+  const int NT = (Tn + L - 1) / L;           // chunks of this sequence (at least one)
   if (tid == 0) {
     mbar_init(&sm.bar_g1, 1); mbar_init(&sm.bar_g2, 1);
     mbar_init(&sm.bar_a, 1); mbar_init(&sm.bar_c, 1); mbar_init(&sm.bar_o, 1);
@@ -628,15 +638,9 @@ r7c_scan_fwd_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned c
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  earlier_kernels_done();
+  if constexpr (!PACKED) earlier_kernels_done();
   later_kernels_may_start();
-  if constexpr (PACKED) {
-    unit = packed_scan_unit(sv, H, reinterpret_cast<SortedSeqs*>(sm.ot), tid);
-    bi = unit / H; hi = unit % H;
-  }
   const size_t ch0 = (size_t)unit * NT_slots;
-  const int Tn = sv.length<PACKED>(bi), tb = sv.first<PACKED>(bi), brow = sv.row<PACKED>(bi);
-  const int NT = (Tn + L - 1) / L;           // chunks of this sequence (at least one)
   const uint32_t tm = sm.tmem_base;
   // TMEM: columns 0..63 lower lane halves = W h~0; columns 64 + 64 p .., p = parity of the chunk: lower halves
   // k~^T v + b~^T sa, upper halves the output rows
@@ -893,7 +897,7 @@ struct AloneSmem {
 };
 constexpr int ALONE_THREADS = 352;
 
-template <bool PACKED>
+template <bool PACKED, bool SORTED>
 __global__ void __launch_bounds__(ALONE_THREADS, 1)
 r7c_scan_fwd_alone_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsigned char* __restrict__ ws_tiles,
                           const float* __restrict__ ws_aux, int* __restrict__ ws_flags, int tiles_per_chunk,
@@ -927,8 +931,8 @@ r7c_scan_fwd_alone_kernel(const __grid_constant__ CUtensorMap tmap_v, const unsi
   tc_fence_after();
   earlier_kernels_done();
   later_kernels_may_start();
-  if constexpr (PACKED) {
-    unit = packed_scan_unit(sv, H, reinterpret_cast<SortedSeqs*>(sm.ot[0]), tid);
+  if constexpr (SORTED) {
+    unit = sorted_scan_unit(sv, H, reinterpret_cast<SortedSeqs*>(sm.ot[0]), tid);
     bi = unit / H; hi = unit % H;
   }
   const size_t ch0 = (size_t)unit * NT_slots;
@@ -1198,14 +1202,14 @@ int launch_rwkv7_chunked_fwd(const void* r, const void* w, const void* k, const 
     ProfScope prof("r7c_intra_fwd_kernel", st);
     const int n_ch = B * H * NT;
     const int sms = dev.sms;
-    const int grid = n_ch < 2 * sms ? n_ch : 2 * sms;     // persistent: two CTAs per SM
+    const int grid = persistent_grid(n_ch, sms);
 #define R7C_LAUNCH_INTRA(P, F)                                                                                     \
     do {                                                                                                           \
       if (allow_smem<r7c_intra_fwd_kernel<P, F>>(dev, smem)) \
         return RWKVB200_E_CUDA;                                                                                    \
       if (int rc = launch(r7c_intra_fwd_kernel<P, F>, grid, 256, smem, st, 1, (const bf16*)r, (const bf16*)w, (const bf16*)k,         \
           (const bf16*)a, (const bf16*)b, tmap_in[0], tmap_in[1], tmap_in[2], tmap_in[3], tmap_in[4], tmap_v,      \
-          ws.tiles, ws.aux, tpc, keep_for_bwd ? 1 : 0, sv, WalkDims(H, NT, B, grid), lay, status,                              \
+          ws.tiles, ws.aux, tpc, keep_for_bwd ? 1 : 0, sv, WalkDims(H, NT, B, grid), ws.list, lay, status,                     \
           debug_stamp_buffer())) return rc;                                                                        \
     } while (0)
     if (seq_start) R7C_LAUNCH_INTRA(true, false);
@@ -1222,23 +1226,24 @@ int launch_rwkv7_chunked_fwd(const void* r, const void* w, const void* k, const 
     if (!fused && (o || ht))
       exact = r7rec::FwdArgs<bf16>{(const bf16*)r, (const bf16*)w, (const bf16*)k, (const bf16*)v, (const bf16*)a, (const bf16*)b,
                                    0, lay.st, 0, nullptr, (bf16*)o, nullptr, nullptr};
-    // more sequences than SMs: two CTAs per SM
-#define R7C_LAUNCH_SCAN(KERNEL, P, THREADS, SMEM)                                                                  \
+#define R7C_LAUNCH_SCAN(THREADS, SMEM, ...)                                                                         \
     do {                                                                                                           \
       const int smem = (int)sizeof(SMEM) + 1024;                                                                   \
-      if (allow_smem<KERNEL<P>>(dev, smem))                                                                        \
+      if (allow_smem<__VA_ARGS__>(dev, smem))                                                                      \
         return RWKVB200_E_CUDA;                                                                                    \
-      if (int rc = launch(KERNEL<P>, B * H, THREADS, smem, st, 1, tmap_v, ws.tiles, ws.aux, ws.flags, tpc,         \
+      if (int rc = launch(__VA_ARGS__, B * H, THREADS, smem, st, 1, tmap_v, ws.tiles, ws.aux, ws.flags, tpc,         \
           keep_for_bwd ? ws.tiles : nullptr, h0, n_state, tmap_o, o ? 1 : 0, ht, (bf16*)o, sv, H, NT, lay, exact,  \
           status, debug_stamp_buffer())) return rc;                                                                \
     } while (0)
-    if (!scans_alone(B, Tn, T_total, H, dev.sms, seq_start != nullptr, 96.f)) {
-      if (seq_start) R7C_LAUNCH_SCAN(r7c_scan_fwd_kernel, true, 256, ScanSmem);
-      else           R7C_LAUNCH_SCAN(r7c_scan_fwd_kernel, false, 256, ScanSmem);
-    } else {
-      if (seq_start) R7C_LAUNCH_SCAN(r7c_scan_fwd_alone_kernel, true, ALONE_THREADS, AloneSmem);
-      else           R7C_LAUNCH_SCAN(r7c_scan_fwd_alone_kernel, false, ALONE_THREADS, AloneSmem);
-    }
+    const bool packed = seq_start != nullptr, alone = scans_alone(B, Tn, T_total, H, dev.sms, packed, 96.f);
+    const bool sorted = packed && scans_sorted(B, Tn, T_total, H, dev.sms, alone);
+    if (!alone) {      // two CTAs per SM
+      if (sorted)      R7C_LAUNCH_SCAN(256, ScanSmem, r7c_scan_fwd_kernel<true, true>);
+      else if (packed) R7C_LAUNCH_SCAN(256, ScanSmem, r7c_scan_fwd_kernel<true, false>);
+      else             R7C_LAUNCH_SCAN(256, ScanSmem, r7c_scan_fwd_kernel<false, false>);
+    } else if (sorted) R7C_LAUNCH_SCAN(ALONE_THREADS, AloneSmem, r7c_scan_fwd_alone_kernel<true, true>);
+    else if (packed)   R7C_LAUNCH_SCAN(ALONE_THREADS, AloneSmem, r7c_scan_fwd_alone_kernel<true, false>);
+    else               R7C_LAUNCH_SCAN(ALONE_THREADS, AloneSmem, r7c_scan_fwd_alone_kernel<false, false>);
 #undef R7C_LAUNCH_SCAN
   }
   return check_launch();

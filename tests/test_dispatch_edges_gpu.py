@@ -237,10 +237,12 @@ def test_scratch_that_cannot_be_had_is_done_without():
         torch.cuda.set_per_process_memory_fraction(1.0)
 
 
-@pytest.mark.parametrize("lens,H", [([1500, 70, 64, 8, 200, 130, 9, 65, 300, 128], 20), ([8 + i % 70 for i in range(260)], 1)])
-def test_scans_of_a_packed_batch_with_more_units_than_SMs(lens, H):
-    """One sequence much longer than the others (its scans run one block to an SM, longest first), and more sequences than are
-    ranked by length: as each sequence on its own."""
+@pytest.mark.parametrize("lens,H", [([1500, 70, 64, 8, 200, 130, 9, 65, 300, 128], 20), ([8 + i % 70 for i in range(260)], 1),
+                                    ([8 + 37 * i % 120 for i in range(700)], 3), ([70] * 255 + [2000], 2), ([1280, 70] * 20, 20)])
+def test_packed_batches_with_more_units_than_SMs(lens, H):
+    """Scans with one block to an SM, longest sequence first (one much longer than the others), with more sequences than are
+    ranked, and with two blocks to an SM, longest first; so many short sequences that a CTA's next chunk-head is a hundred of them
+    on: as each sequence on its own."""
     assert len(lens) * H > torch.cuda.get_device_properties(0).multi_processor_count
     cu = [0]
     for n in lens:
@@ -255,7 +257,7 @@ def test_scans_of_a_packed_batch_with_more_units_than_SMs(lens, H):
 
     tokens = [d[n] for n in "rwkvab"]
     out = run(lambda *x: ro.generalized_delta_rule_varlen(*x, cu), tokens, d["d_out"], d_s)
-    for i in list(range(min(len(lens), 10))) + [len(lens) - 1]:
+    for i in {*range(min(len(lens), 10)), *range(10, len(lens), 97), len(lens) - 1}:
         at = slice(cu[i], cu[i + 1])
         ref = run(ro.generalized_delta_rule, [t[:, at].contiguous() for t in tokens], d["d_out"][:, at].contiguous(), d_s[i:i + 1])
         for m, (a, b) in enumerate(zip(out, ref)):
