@@ -196,18 +196,25 @@ __device__ __forceinline__ int sorted_scan_unit(const SeqView& sv, int H, Sorted
   __syncthreads();
   return sorted->at * H + b % H;
 }
-// Whether the scans run one block to an SM.  Dense: with at most a sequence and head per SM.  Packed: also where the longest
-// sequence, whose chunks take 3.3 us each with two blocks to an SM and 1.3 alone, would end long after the others; `kb`: KB that a
-// chunk moves, of 6 TB/s that the scans reach.  (8 sequences of 1093 .. 4096 tokens, 32 heads: forward 215 -> 194 us, reverse 115 -> 104;
-// as many equally long ones take 257 and 262.)
-inline bool scans_alone(int n_seq, int Tn, int T_total, int H, int sms, bool packed, float kb) {
+// Whether the scans run one block to an SM.  Dense: with at most a sequence and head per SM.  Packed: also where an estimate of the
+// two kernels' times says so (us, from the longest sequence, the mean and the units; the constants of a direction from the times of
+// both on 23 batches, 3 .. 200 sequences of 8 .. 8000 tokens, 2 .. 64 heads; there and on 19 others it cost 7 % at most, 11 % once).  A block
+// alone takes `chunk` per chunk and `block` besides; with two to an SM a chunk takes `free` .. `shared`, by how often an SM has
+// two, but the start and end of one block lie under the other; and both move `kb` KB per chunk, at 6 TB/s at best.
+// Forward / reverse, alone and two: 8 sequences of 1093 .. 4096 tokens, 32 heads 203 and 218 / 113 and 124; 8 of 2048 158 and 138 / 91 and
+// 84; one of 8000 and 60 of 100, 16 heads 196 and 345 / 153 and 166; one of 3000 and 100 of 8, 64 heads 318 and 239 / 267 and 166.
+struct ScanTimes { float kb, alone_memory, chunk, block, free, shared, slope; };
+constexpr ScanTimes SCAN_FWD{96.f, 1.2f, 1.5f, 5.8f, 2.3f, 3.4f, 1.5f}, SCAN_REVERSE{47.f, 1.15f, 1.2f, 5.f, 1.28f, 1.94f, 0.9f};
+inline bool scans_alone(int n_seq, int Tn, int T_total, int H, int sms, bool packed, const ScanTimes& t) {
   const int units = n_seq * H;
   if (units <= sms) return true;
   if (!packed || n_seq > MAX_SORTED) return false;
-  const float longest = (float)num_chunks(Tn), mean = (float)T_total / n_seq / L + 0.5f, per_sm = mean * units / sms;
-  const float rounds = fmaxf(longest, per_sm + 0.25f * mean);      // chunks in a row on the slowest SM
-  const float memory = units * mean * kb / 6000.f;
-  return fmaxf(rounds * 1.3f, memory * rounds / per_sm) < fmaxf(longest * 3.3f, memory);
+  const float longest = (float)num_chunks(Tn), mean = (float)T_total / n_seq / L + 0.5f, blocks = (float)units / sms;
+  const float memory = units * mean * t.kb / 6000.f;
+  const float alone = fmaxf(fmaxf(longest * t.chunk + t.block, memory * t.alone_memory + 3.f * blocks),
+                            (blocks + 0.4f) * mean * t.chunk + blocks * t.block);
+  const float two = fmaxf(longest * fminf(t.shared, t.free + t.slope * (blocks - 1.f)) + 5.f, memory + 2.9f * blocks);
+  return alone < two;
 }
 
 // Whether the blocks of a packed batch's scans come longest sequence first.  Ranking the sequences costs a block 1 us and more (and the

@@ -957,7 +957,7 @@ int launch_rwkv7_chunked_bwd(const void* r, const void* w, const void* k, const 
       if (int rc = launch(__VA_ARGS__, B * H, THREADS, smem, st, 1, tmap_do, ws.tiles, ws.aux, (int)ALL_TILES,    \
                           d_ht, d_h0, sv, H, NT, status)) return rc;                                              \
     } while (0)
-    const bool packed = seq_start != nullptr, alone = scans_alone(B, Tn, T_total, H, dev.sms, packed, 56.f);
+    const bool packed = seq_start != nullptr, alone = scans_alone(B, Tn, T_total, H, dev.sms, packed, SCAN_REVERSE);
     const bool sorted = packed && scans_sorted(B, Tn, T_total, H, dev.sms, alone);
     if (!alone) {      // two CTAs per SM
       if (sorted)      R7C_LAUNCH_BSCAN(256, BScanSmem, r7c_bwd_scan_kernel<true, true>);

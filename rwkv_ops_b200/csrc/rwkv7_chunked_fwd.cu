@@ -1235,7 +1235,7 @@ int launch_rwkv7_chunked_fwd(const void* r, const void* w, const void* k, const 
           keep_for_bwd ? ws.tiles : nullptr, h0, n_state, tmap_o, o ? 1 : 0, ht, (bf16*)o, sv, H, NT, lay, exact,  \
           status, debug_stamp_buffer())) return rc;                                                                \
     } while (0)
-    const bool packed = seq_start != nullptr, alone = scans_alone(B, Tn, T_total, H, dev.sms, packed, 96.f);
+    const bool packed = seq_start != nullptr, alone = scans_alone(B, Tn, T_total, H, dev.sms, packed, SCAN_FWD);
     const bool sorted = packed && scans_sorted(B, Tn, T_total, H, dev.sms, alone);
     if (!alone) {      // two CTAs per SM
       if (sorted)      R7C_LAUNCH_SCAN(256, ScanSmem, r7c_scan_fwd_kernel<true, true>);
