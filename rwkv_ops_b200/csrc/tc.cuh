@@ -55,13 +55,21 @@ __device__ __forceinline__ void fence_mbar_init() {
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
+template <bool CLUSTER = false>      // CLUSTER: acquires what other CTAs of the cluster have released
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  if constexpr (CLUSTER)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
   return ok != 0;
 }
 // Bounded wait; returns false (and records `code`) if the phase never completed.
@@ -70,11 +78,12 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // the vote around it a wait of a single thread took 233 cycles, this way 70.  The polling loop is kept out of it; its
 // result is made uniform over the threads that poll together (a warp sees a barrier in one state), so that the
 // warp-collective TMEM instructions that follow are never executed by part of a warp.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status, int code,
                                           uint32_t limit = WAIT_LIMIT) {
-  if (mbar_try_wait(bar, parity)) return true;
+  if (mbar_try_wait<CLUSTER>(bar, parity)) return true;
   bool done = false;
-  for (uint32_t i = 1; i < limit && !done; ++i) done = mbar_try_wait(bar, parity);
+  for (uint32_t i = 1; i < limit && !done; ++i) done = mbar_try_wait<CLUSTER>(bar, parity);
   if (!done) atomicCAS(status, 0, code);
   return __all_sync(__activemask(), done) != 0;
 }
@@ -93,13 +102,15 @@ __device__ __forceinline__ uint32_t cluster_addr(uint32_t smem_addr, uint32_t ra
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// 16 bytes into another CTA's shared memory; its barrier counts them
+// 16 bytes into another CTA's shared memory; its barrier counts them, and releases them to the cluster: whoever waits for them
+// acquires at that scope (mbar_wait<true>; the time is the same)
 __device__ __forceinline__ void store_async_16(uint32_t addr, float4 f, uint32_t bar) {
   asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
                ::"r"(addr), "f"(f.x), "f"(f.y), "f"(f.z), "f"(f.w), "r"(bar) : "memory");
 }
-// An arrival at another CTA's barrier.  (With the scope of the cluster spelled out it waits for the global stores the thread has in
-// flight, a microsecond: the arrivals here follow reads of shared memory only.)
+// An arrival at another CTA's barrier that hands it nothing but leave to write: what the arriving CTA has read there is in registers
+// or has gone through completed products, which its other threads or a barrier of its own have reported before.  So the scope
+// of the cluster is not spelled out: the release would wait for the global stores the thread has in flight (the wkv6 forward 2-7 % slower).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }

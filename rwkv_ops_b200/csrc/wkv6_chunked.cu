@@ -403,7 +403,7 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   // RELAY: a row piece of the state travels through the 2 x 64 bytes that its S~0 takes up as hi and lo parts
   auto piece = [&](int j) { return tile_chunk_off(srow, 4 * hsel + (j & 3)) + (j >> 2) * TILE_BYTES; };
   auto receive_state = [&]() {
-    if (!mbar_wait(&sm.bar_state, n_fetched & 1, status, 406)) return false;
+    if (!mbar_wait<true>(&sm.bar_state, n_fetched & 1, status, 406)) return false;
     if (!tok_lane) {
 #pragma unroll
       for (int j = 0; j < CW / 4; ++j) {
@@ -560,7 +560,7 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
         tmem_ld<CW>(tm_ys, rr);
         tmem_ld_wait();
         const bool send = RELAY && c + 1 < c_hi;      // (what can be waited for before the state arrives is)
-        if (send) ok = mbar_wait(&sm.bar_free, n_sent & 1, status, 407);
+        if (send) ok = mbar_wait<true>(&sm.bar_free, n_sent & 1, status, 407);
         if (RELAY && need_state) ok = receive_state() && ok;
 #pragma unroll
         for (int j = 0; j < CW; ++j) {
