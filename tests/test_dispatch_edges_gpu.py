@@ -186,22 +186,54 @@ def _sizes_prepared_apart(K, sms):
 
 @pytest.mark.parametrize("K,dtype", [(64, torch.float32), (64, torch.float16), (128, torch.float32), (128, torch.bfloat16)])
 def test_blocks_prepared_apart(K, dtype):
-    """The sweeps with and without their scratch (C ABI): the same bits, whatever part of it a call works with at a time."""
+    """The sweeps of the forward and the backward, with and without states that the forward leaves, with and without their scratch
+    (C ABI): the same bits, whatever part of it a call works with at a time."""
     lib, dev = _lib.load(), torch.device("cuda")
     code = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}[dtype]
     for H, T in _sizes_prepared_apart(K, torch.cuda.get_device_properties(0).multi_processor_count):
-        d = rwkv7_inputs(1, T, H, K, dtype=dtype, seed=T, device="cuda", with_state=True)
-        x = [d[n] for n in "rwkvab"]
-        out = []
-        for scratch in (True, False):
-            o, s = torch.empty_like(x[0]), torch.empty(1, H, K, K, device=dev)
-            n = lib.rwkvb200_rwkv7_fwd_workspace_bytes(1, T, H, K, code, _lib.ALGO_RECURRENT) if scratch else 0
-            ws = torch.empty(n, dtype=torch.uint8, device=dev)
-            _lib.check(lib.rwkvb200_rwkv7_fwd(*(_lib.ptr(t) for t in x), _lib.ptr(d["initial_state"]), 1, _lib.ptr(o), _lib.ptr(s),
-                                              _lib.ptr(ws) if n else None, n, 1, T, H, K, code, 0, _lib.ALGO_RECURRENT,
-                                              _lib.stream_ptr(dev)), "fwd")
-            out.append((o, s))
-        assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1]), (H, T)
+        d = rwkv7_inputs(1, T, H, K, dtype=dtype, seed=T, device="cuda", with_state=True, with_grads=True)
+        x = [_lib.ptr(d[n]) for n in "rwkvab"]
+        h0, d_o, d_ht = (_lib.ptr(d[n]) for n in ("initial_state", "d_out", "d_state"))
+        size, end = (1, T, H, K, code, _lib.ALGO_RECURRENT), (1, T, H, K, code, 0, _lib.ALGO_RECURRENT, _lib.stream_ptr(dev))
+        checkpoints = H * ((T + 7) // 8) * K * K * 4
+        n_states = lib.rwkvb200_rwkv7_states_bytes(*size)
+        assert n_states == _lib.rwkv7_states_bytes(1, T, H, K)
+
+        def memory(n):
+            return torch.empty(n, dtype=torch.uint8, device=dev)
+
+        def run(scratch, kept):
+            out = [torch.empty_like(d["r"]) for _ in range(7)] + [torch.empty(1, H, K, K, device=dev) for _ in range(2)]
+            o, grads, ht, dh0 = _lib.ptr(out[0]), [_lib.ptr(t) for t in out[1:7]], _lib.ptr(out[7]), _lib.ptr(out[8])
+            ws = memory(lib.rwkvb200_rwkv7_fwd_workspace_bytes(*size) if scratch else 0)
+            fwd = (_lib.ptr(ws) if ws.numel() else None, ws.numel(), *end)
+            if kept:
+                states = memory(n_states)
+                _lib.check(lib.rwkvb200_rwkv7_fwd_states(*x, h0, 1, o, ht, _lib.ptr(states), n_states, *fwd), "fwd_states")
+                wb = memory(lib.rwkvb200_rwkv7_bwd_states_workspace_bytes(*size) if scratch else n_states)
+                _lib.check(lib.rwkvb200_rwkv7_bwd_states(*x, h0, 1, d_o, d_ht, _lib.ptr(states), n_states, *grads, dh0, _lib.ptr(wb),
+                                                         wb.numel(), *end), "bwd_states")
+            else:
+                _lib.check(lib.rwkvb200_rwkv7_fwd(*x, h0, 1, o, ht, *fwd), "fwd")
+                wb = memory(lib.rwkvb200_rwkv7_bwd_workspace_bytes(*size) if scratch else (checkpoints + 255) // 256 * 256)
+                _lib.check(lib.rwkvb200_rwkv7_bwd(*x, h0, 1, d_o, d_ht, *grads, dh0, _lib.ptr(wb), wb.numel(), *end), "bwd")
+            return out
+
+        ref = run(False, False)
+        for scratch, kept in ((True, False), (False, True), (True, True)):
+            for i, (got, want) in enumerate(zip(run(scratch, kept), ref)):
+                assert torch.equal(got, want), (H, T, scratch, kept, i)
+
+
+@pytest.mark.parametrize("H,T", [(2, 400), (80, 40)])
+def test_blocks_prepared_apart_against_float64(H, T):
+    """Training through the operator where the blocks are prepared apart: few units from 377 tokens on, many from 25 on."""
+    d = rwkv7_inputs(1, T, H, dtype=torch.float32, seed=T, with_state=True, with_grads=True)
+    ref = _train({n: t.double() for n, t in d.items()}, [d["d_out"].double(), d["d_state"].double()],
+                 lambda *x, **kw: oracle_gdr(*x, **kw, compute_dtype=torch.float64))
+    out = _train({n: t.cuda() for n, t in d.items()}, [d["d_out"].cuda(), d["d_state"].cuda()])
+    for n in ref:
+        assert rel_l2(out[n], ref[n]) < 1e-5, n
 
 
 def test_scratch_that_cannot_be_had_is_done_without():
@@ -262,3 +294,121 @@ def test_packed_batches_with_more_units_than_SMs(lens, H):
         ref = run(ro.generalized_delta_rule, [t[:, at].contiguous() for t in tokens], d["d_out"][:, at].contiguous(), d_s[i:i + 1])
         for m, (a, b) in enumerate(zip(out, ref)):
             assert rel_l2(a[i:i + 1] if m == 0 else a[:, at], b) < 2e-3, (i, m)
+
+
+def _wkv6_train(d, call):
+    x = [d[n].clone().requires_grad_(True) for n in "rkvwu"]
+    y, s = call(*x)
+    return [y.detach(), s.detach(), *torch.autograd.grad([y, s], x, [d["d_y"], d["d_state"].to(s.dtype)])]
+
+
+# (sequences, tokens, heads): clusters of eight CTAs on their third lap and of two on their seventh; stretches on persistent CTAs.
+# Tolerances of this file's other wkv6 tests; float16 rounds eight times finer than bfloat16.
+@pytest.mark.parametrize("B,T,H", [(1, 1100, 2), (4, 777, 32), (5, 520, 64)])
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-4), (torch.bfloat16, 2e-2), (torch.float16, 2.5e-3)])
+def test_wkv6_relays_and_stretches_against_the_recurrence(B, T, H, dtype, tol, monkeypatch):
+    d = wkv6_inputs(B, T, H, dtype=dtype, seed=B + T, device="cuda", n_state=1, with_grads=True)
+    op = ro.RWKV6_OP(64, T)
+
+    def call(*x):
+        return op(*x, with_state=True, init_state=d["init_state"], state_map=torch.zeros(B, dtype=torch.int32, device="cuda"))
+
+    out = _wkv6_train(d, call)
+    with torch.no_grad():
+        y, s = call(*[d[n] for n in "rkvwu"])
+    monkeypatch.setenv("RWKV_OPS_B200_WKV6_ALGO", "recurrent")
+    ref = _wkv6_train(d, call)
+    for i, (a, b) in enumerate(zip([*out, y, s], [*ref, ref[0], ref[1]])):
+        assert rel_l2(a, b) < tol, i
+    assert _lib.load().rwkvb200_device_status(1) == 0
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-4), (torch.bfloat16, 2e-2), (torch.float16, 2.5e-3)])
+def test_wkv6_relay_of_a_packed_batch(dtype, tol, monkeypatch):
+    """Lengths on both sides of a chunk, a CTA's turn and a lap of the cluster; rows past a sequence's end belong to the next one."""
+    lens, H = [512, 513, 63, 1031, 1, 64, 1088, 577], 2
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    d = wkv6_inputs(1, cu[-1], H, dtype=dtype, seed=9, device="cuda", n_state=1, with_grads=True)
+    d["d_state"] = 0.1 * torch.randn(len(lens), H, 64, 64, device="cuda")
+    out = _wkv6_train(d, lambda *x: ro.wkv6_varlen(*x, cu))
+    monkeypatch.setenv("RWKV_OPS_B200_WKV6_ALGO", "recurrent")
+
+    def one_by_one(r, k, v, w, u):
+        ys = [ro.RWKV6_OP(64, n)(*(x[:, i:i + n] for x in (r, k, v, w)), u, with_state=True) for i, n in zip(cu, lens)]
+        return torch.cat([y for y, _ in ys], 1), torch.cat([s for _, s in ys], 0)
+
+    ref = _wkv6_train(d, one_by_one)
+    for i, (a, b) in enumerate(zip(out, ref)):
+        assert rel_l2(a, b) < tol, i
+    assert _lib.load().rwkvb200_device_status(1) == 0
+
+
+def _training_calls():
+    """(name, inputs, call) of every path with more than one kernel: chunked, packed, fused, float32 by blocks, wkv6."""
+    def rwkv7(name, dtype, B, T, H, fn=ro.generalized_delta_rule):
+        d = rwkv7_inputs(B, T, H, dtype=dtype, seed=T, device="cuda", with_grads=True)
+        return name, [d[n] for n in "rwkvab"], fn, [d["d_out"], d["d_state"]]
+
+    yield rwkv7("chunked", torch.bfloat16, 2, 300, 8)
+    yield rwkv7("chunked, many units", torch.bfloat16, 10, 130, 32)
+    yield rwkv7("float32", torch.float32, 1, 400, 4)
+    name, x, _, grads = rwkv7("packed", torch.bfloat16, 1, 700, 4)
+    packed = ro.PackedSequences([0, 300, 310, 700])
+    yield name, x, lambda *x: ro.generalized_delta_rule_varlen(*x, packed), [grads[0], grads[1].expand(3, -1, -1, -1).contiguous()]
+    yield rwkv7("fused", torch.bfloat16, 2, 300, 8, ro.generalized_delta_rule_fused)
+    for name, B, T, H in (("wkv6 relay", 1, 700, 4), ("wkv6 stretches", 5, 520, 64)):
+        d = wkv6_inputs(B, T, H, dtype=torch.bfloat16, seed=T, device="cuda", with_grads=True)
+        op = ro.RWKV6_OP(64, T)
+        yield name, [d[n] for n in "rkvwu"], lambda *x, op=op: op(*x, with_state=True), [d["d_y"], d["d_state"].bfloat16()]
+
+
+def _results(x, fn, grads):
+    x = [t.detach().requires_grad_(True) for t in x]
+    o, s = fn(*x)
+    return [o, s, *torch.autograd.grad([o, s], x, grads)]
+
+
+def _same(got, want, what):
+    for i, (a, b) in enumerate(zip(got, want)):
+        # (wkv6: the gradient of u, the last one, is summed by atomic additions)
+        assert torch.equal(a, b) or (i == len(want) - 1 and "wkv6" in what and rel_l2(a, b) < 1e-2), (what, i)
+
+
+def test_training_replays_from_a_cuda_graph():
+    """Calls of several kernels, whose launches overlap, captured and replayed on other inputs."""
+    for name, x, fn, grads in _training_calls():
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            _results(x, fn, grads)
+        torch.cuda.current_stream().wait_stream(side)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = _results(x, fn, grads)
+        for _ in range(2):
+            for t in x:
+                t.copy_(t.flip(1).contiguous() if t.dim() > 2 else t.flip(0))
+            graph.replay()
+            _same(out, _results(x, fn, grads), name)
+    assert _lib.load().rwkvb200_device_status(1) == 0
+
+
+def test_training_on_two_streams_at_once():
+    """Two calls of every pair of paths in flight at the same time: their kernels share SMs, and each keeps its own workspace."""
+    calls = list(_training_calls())
+    want = [_results(*call[1:]) for call in calls]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    for i in range(len(calls)):
+        for j in range(i, len(calls)):
+            torch.cuda.synchronize()
+            got = []
+            for stream, c in zip(streams, (i, j)):
+                with torch.cuda.stream(stream):
+                    got.append([_results(*calls[c][1:]) for _ in range(3)])
+            torch.cuda.synchronize()
+            for c, results in zip((i, j), got):
+                for r in results:
+                    _same(r, want[c], calls[c][0])
+    assert _lib.load().rwkvb200_device_status(1) == 0
