@@ -336,7 +336,7 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
     const Stretch x = stretch(item);
     if (x.c_lo + rank < x.c_hi) load_in(x, x.c_lo + rank);
   }
-  // an item without a chunk in which to take the next one takes it by itself
+  // an item without a chunk (of a packed batch) takes the next one by itself
   auto take_next = [&]() {
     if (warp == 0 && elect_one()) {
       sm.next_item = atomicAdd(handoff_flags + n_units, 1);
@@ -352,7 +352,7 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
   const long long base = (((long long)cur.brow * Tn_dense + cur.tok0) * H + hi) * HS;   // Tn_dense: rows per batch row
   const size_t nts = PACKED ? (size_t)seqs.nts : (size_t)(cur.NT + 1);
   const bool last_part = c_hi == cur.NT;
-  if (c_lo < c_hi || (part == 0 && c_hi == 0)) {      // (c_hi == 0: an empty sequence, which just hands its state on)
+  if (c_lo < c_hi || (c_hi == 0 && (!PACKED || part == 0))) {      // (c_hi == 0: an empty sequence, which just hands its state on)
   // per-thread slice of u (4 channels) for the diagonal term
   const float4 u4 = load4_as<T>(u, hi * HS + 4 * c4, typed);
   int marked = Tn < SHORT_SEQ;      // thread-wise until the end of the item
@@ -673,9 +673,9 @@ wkv6c_fwd_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __re
       for (int i = 0; i < n_cta; ++i) marked |= sm.marks[i];
     }
     if (tid == 0 && rank == 0) flags[unit] = marked != 0;
-    if (!RELAY && parts > 1 && c_hi == 0) take_next();
+    if (PACKED && !RELAY && parts > 1 && c_hi == 0) take_next();
   }
-  } else if (!RELAY && parts > 1) {
+  } else if (!PACKED || parts > 1) {
     take_next();
   }
   if (parts == 1) break;
