@@ -177,6 +177,30 @@ def test_states_kept_for_the_backward(T, K, dtype, monkeypatch):
         assert torch.equal(a, b) and torch.equal(a, c)
 
 
+@pytest.mark.parametrize("K,dtype", [(64, torch.float32), (64, torch.float16), (128, torch.float32), (128, torch.bfloat16)])
+@pytest.mark.parametrize("few", [False, True])
+def test_blocks_prepared_apart(K, dtype, few):
+    """The sweeps with and without their scratch (C ABI): the same bits, at the block counts from which the scratch is used, and
+    just short of where a unit's blocks take several stretches of it."""
+    lib, dev = _lib.load(), torch.device("cuda")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    code = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}[dtype]
+    H = 3 if few else 2 * sms // (K // 16) + 2
+    for T in ((95, 96, 377, 384, 400) if few else (24, 25, 32, 33, 70)) + (() if few or K == 128 else (2500,)):
+        d = rwkv7_inputs(1, T, H, K, dtype=dtype, seed=T, device="cuda", with_state=True)
+        x = [d[n] for n in "rwkvab"]
+        out = []
+        for scratch in (True, False):
+            o, s = torch.empty_like(x[0]), torch.empty(1, H, K, K, device=dev)
+            n = lib.rwkvb200_rwkv7_fwd_workspace_bytes(1, T, H, K, code, _lib.ALGO_RECURRENT) if scratch else 0
+            ws = torch.empty(n, dtype=torch.uint8, device=dev)
+            _lib.check(lib.rwkvb200_rwkv7_fwd(*(_lib.ptr(t) for t in x), _lib.ptr(d["initial_state"]), 1, _lib.ptr(o), _lib.ptr(s),
+                                              _lib.ptr(ws) if n else None, n, 1, T, H, K, code, 0, _lib.ALGO_RECURRENT,
+                                              _lib.stream_ptr(dev)), "fwd")
+            out.append((o, s))
+        assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1]), T
+
+
 def _sizes_prepared_apart(K, sms):
     """(units, tokens): block counts from which a sweep's blocks are prepared by a kernel of their own with fewer CTAs than SMs and
     with many; then stretches of blocks, and passes of units, where the scratch does not hold all of them."""
@@ -185,7 +209,7 @@ def _sizes_prepared_apart(K, sms):
 
 
 @pytest.mark.parametrize("K,dtype", [(64, torch.float32), (64, torch.float16), (128, torch.float32), (128, torch.bfloat16)])
-def test_blocks_prepared_apart(K, dtype):
+def test_blocks_prepared_apart_forward_and_backward(K, dtype):
     """The sweeps of the forward and the backward, with and without states that the forward leaves, with and without their scratch
     (C ABI): the same bits, whatever part of it a call works with at a time."""
     lib, dev = _lib.load(), torch.device("cuda")
@@ -271,10 +295,10 @@ def test_scratch_that_cannot_be_had_is_done_without():
 
 @pytest.mark.parametrize("lens,H", [([1500, 70, 64, 8, 200, 130, 9, 65, 300, 128], 20), ([8 + i % 70 for i in range(260)], 1),
                                     ([8 + 37 * i % 120 for i in range(700)], 3), ([70] * 255 + [2000], 2), ([1280, 70] * 20, 20)])
-def test_packed_batches_with_more_units_than_SMs(lens, H):
-    """Scans with one block to an SM, longest sequence first (one much longer than the others), with more sequences than are
-    ranked, and with two blocks to an SM, longest first; so many short sequences that a CTA's next chunk-head is a hundred of them
-    on: as each sequence on its own."""
+def test_scans_of_a_packed_batch_with_more_units_than_SMs(lens, H):
+    """One sequence much longer than the others (its scans run one block to an SM, longest first), more sequences than are
+    ranked by length, and two blocks to an SM, longest first; so many short sequences that a CTA's next chunk-head is a hundred of
+    them on: as each sequence on its own."""
     assert len(lens) * H > torch.cuda.get_device_properties(0).multi_processor_count
     cu = [0]
     for n in lens:
